@@ -161,9 +161,9 @@ typedef struct pb_op_params {
     const float* bias;        /* fp32 [K] or NULL */
     const void* residual;     /* same dtype as x, [P][Q][res_Cs], or NULL */
     void* y;                  /* output tensor base (slice offset applied by the kernel) */
-    /* Scratch memory (device, 16-byte aligned, zero-filled before its first use, private to one
-     * in-flight launch).  The tensor-core convolution splits its reduction over several thread
-     * blocks when given at least pb_launch_info.scratch_bytes here; NULL = no split. */
+    /* The tensor-core convolution may spread a long reduction over the thread blocks of a cluster when given at least
+     * pb_launch_info.scratch_bytes here (device memory, 16-byte aligned, private to one in-flight launch); NULL = no
+     * split.  The partial tiles meet in the cluster's shared memory: the memory only states the caller's consent. */
     void* scratch;
     uint64_t scratch_bytes;
     /* Images per launch (0 or 1 = one).  A batch is how a gang of requests of one model runs as one
@@ -183,11 +183,11 @@ PB_API int pb_op_launch(int kind, const pb_op_params* p, void* stream, uint32_t 
 PB_API int64_t pb_op_pack_weights(int kind, const pb_op_params* p, const float* w_oihw, void* dst_host);
 /* 1 if the tcgen05 implicit-GEMM kernel supports this convolution. */
 PB_API int pb_conv_umma_supported(const pb_op_params* p);
-/* The tensor-core convolution splits a long reduction over several thread blocks (partial tiles meet in
- * scratch memory) when its cost model expects to save at least this many microseconds on a lone launch
- * (default 6, or PB_CONV_SPLIT_GAIN_US from the environment; 0 = split whenever it pays at all, a large
- * value = never; negative = back to the default).  Read at every pb_op_info / pb_op_launch, and when a model
- * instance builds its launches for a batch size: instances built before a change keep their split. */
+/* The tensor-core convolution spreads a long reduction over the blocks of a thread-block cluster when its cost model
+ * expects that to pay on a lone launch.  `us` is the reluctance to do so: it has to save a 60th of it (default 6, or
+ * PB_CONV_SPLIT_GAIN_US from the environment; 0 = split whenever it pays at all, above 1e6 = never; negative = back to
+ * the default).  Read at every pb_op_info / pb_op_launch, and when a model instance builds its launches for a batch
+ * size: instances built before a change keep their split. */
 PB_API void pb_set_conv_split_gain_us(double us);
 /* Mean microseconds of one launch of the tensor-core convolution `p` (any batch): 3 warm-up launches, then `iters`
  * launches on a private stream between CUDA events, a write of flush_bytes before each (0 = none).  mode 0 = the
@@ -196,18 +196,11 @@ PB_API int pb_conv_umma_time(const pb_op_params* p, int mode, int iters, size_t 
 /* Tensor-core convolution for callers that must not allocate: code running inside a CUDA memory-pool
  * or allocator callback, a latency-critical thread that may not take the allocator's locks, or a host
  * that pre-partitions all device memory and leaves none to ask for.  It has no counterpart in the
- * reference (which allocates freely); it is the same kernel as pb_op_launch(PB_STAGE_CONV_UMMA) with its
- * split-K scratch taken from a buffer built into the library instead of p->scratch.
+ * reference (which allocates freely); it is the same kernel as pb_op_launch(PB_STAGE_CONV_UMMA), always allowed to
+ * split its reduction (the partial tiles meet in shared memory, so no scratch memory is involved).
  *  - p->scratch / p->scratch_bytes are ignored.  Inputs, weights and outputs are still the caller's.
- *  - Limit: the built-in buffer is 4 MiB (and is held by every GPU that loads the library until the
- *    process exits).  A convolution whose split needs more (pb_launch_info.scratch_bytes) is refused
- *    with PB_ERR_INVALID and a message; nothing is launched.
- *  - The first call on each device looks up the buffer's device address and sets the kernels' shared
- *    memory limit; make that first call outside any stream capture.
- *  - All calls on a device share the one buffer: the tile counters are cleared (stream-ordered) at the
- *    start of every call, the rest keeps the previous call's contents.  Two calls whose kernels can
- *    overlap on the GPU (different streams, no dependency) race on it: keep them on one stream or
- *    order them yourself.
+ *  - The first call on each device looks up a device address and sets the kernels' shared memory limit; make that
+ *    first call outside any stream capture.
  *  - Never calls cudaMalloc, cudaFree or any allocating routine, on the host heap either. */
 PB_API int pb_conv2d_umma_noalloc(const pb_op_params* p, void* stream, uint32_t job_id, void* notifier);
 /* Device-side error flag raised by bounded waits inside kernels (0 = none): the OR of the library's flag and of
@@ -227,6 +220,10 @@ typedef struct pb_instance pb_instance;
 /* precision: -1 = the pack's own hint, 0 = fp32 SIMT kernels, 1 = bf16 (tcgen05 where supported). */
 PB_API int pb_model_load(const char* pack_path, int device, int precision, pb_model** out);
 PB_API void pb_model_destroy(pb_model* m);
+/* Tiling policy of the model's tensor-core launches.  0 (default): a launch has the GPU to itself, so its tiles are cut to
+ * finish it soonest.  1: launches of many other requests run beside it (a server's models), so the tiles are cut to occupy
+ * the GPU least.  Call it before the model's first instance is created; an instance keeps what it was created with. */
+PB_API int pb_model_set_shared_gpu(pb_model* m, int shared);
 PB_API size_t pb_model_input_bytes(const pb_model* m);   /* NCHW fp32 */
 PB_API size_t pb_model_output_bytes(const pb_model* m);  /* fp32 vector */
 PB_API int pb_model_num_stages(const pb_model* m);       /* compute stages (kernels) per request */

@@ -148,6 +148,7 @@ SIGNATURES = {
     "pb_instance_time_stage_batched": (_I, [_VP, _I, _I, _I, _SZ, C.POINTER(C.c_double)]),
     "pb_model_load": (_I, [C.c_char_p, _I, _I, _PP]),
     "pb_model_destroy": (None, [_VP]),
+    "pb_model_set_shared_gpu": (_I, [_VP, _I]),
     "pb_model_input_bytes": (_SZ, [_VP]),
     "pb_model_output_bytes": (_SZ, [_VP]),
     "pb_model_num_stages": (_I, [_VP]),

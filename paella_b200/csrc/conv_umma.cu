@@ -13,8 +13,8 @@
 // tcgen05.ld, adds bias and residual, applies the activation and stores bf16 into the channel
 // slice of the output tensor.
 //
-// CTA = 6 warps: warps 0-3 run the epilogue (thread t owns accumulator lane t), warp 4 is the TMA
-// producer, warp 5 allocates TMEM and issues the MMAs.  Sized for three CTAs per SM.
+// CTA = 6 warps: warps 0-3 run the epilogue (thread t owns accumulator lane t), before it warp 3 loads
+// operand B; warp 4 loads operand A, warp 5 allocates TMEM and issues the MMAs.  Sized for three CTAs per SM.
 // Two entry points share the body (conv_tile_tma): conv_umma_tma_kernel runs one convolution,
 // conv_umma_multi_kernel runs several independent ones as one grid from a descriptor table in
 // device memory.  conv_umma_gather_kernel (PB_CONV_GATHER=1) is the earlier design, kept for
@@ -69,10 +69,10 @@ constexpr uint32_t kSmemBudget = 200u * 1024u;   // one CTA per SM (gather kerne
 #define PB_CONV_SMEM_KB 73
 #endif
 constexpr uint32_t kSmemBudgetTma = PB_CONV_SMEM_KB * 1024u;
-constexpr uint32_t kCounterBytes = 4096;        // split-K tile counters at the head of the scratch buffer
-#ifndef PB_NOALLOC_SCRATCH_BYTES
-#define PB_NOALLOC_SCRATCH_BYTES (4u << 20)      // built-in scratch of pb_conv2d_umma_noalloc: 4 MiB per GPU
-#endif
+constexpr uint32_t kSmemBudgetDeep = 110u * 1024u;      // small launches on a GPU they have to themselves: two CTAs per SM
+// What a split launch asks of pb_op_params.scratch.  The partial tiles meet in the shared memory of a thread-block
+// cluster, so the memory itself is not touched: supplying it is how a caller allows the split (NULL = no split).
+constexpr uint64_t kSplitScratchBytes = 256;
 constexpr int kATileBytes = kBM * kBK * 2;   // 16 KiB
 constexpr uint32_t kWaitLimit = 4u * 1000u * 1000u;  // polls of mbarrier.try_wait before giving up
 constexpr int kThreads = 160;
@@ -98,10 +98,8 @@ struct ConvArgs {
     uint32_t idesc;       // tcgen05 instruction descriptor
     uint32_t tmem_cols;   // power of two >= max(32, BN)
     uint32_t b_stage_bytes;
-    // split-K: blockIdx.z handles k-blocks [z*kb_per_split, ...); partial tiles meet in `ws`
-    int splits, kb_per_split;
-    float* ws;              // [tile][split][128][BN] fp32 partial accumulators
-    unsigned* counters;     // [tile] arrival counters, zero between launches
+    int out_box;          // channels of one TMA store box: 64 or 32 (divides BN); 0 = the epilogue stores directly
+    int splits;           // thread blocks (one cluster) that share a tile's reduction: rank z takes k-blocks [nkb*z/splits, nkb*(z+1)/splits)
 };
 
 // ---- PTX wrappers -----------------------------------------------------------------
@@ -177,6 +175,12 @@ __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorM
         ::"r"(dst), "l"(map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(w_off), "h"(h_off)
         : "memory");
 }
+// Tiled store of a shared-memory box; rows and channels outside the tensor are dropped by the hardware.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -211,6 +215,36 @@ __device__ __forceinline__ void tcgen05_ld16(uint32_t taddr, uint32_t (&r)[16]) 
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
+}
+// One lane of a converged warp, the same one every time.  Loops that issue tensor-core or copy instructions run
+// warp-uniformly and only the instruction itself is predicated on this: under `if (lane == 0)` the compiler cannot
+// know that descriptors and addresses are uniform and moves every operand to the uniform registers each time
+// (a k-block of four MMAs and a commit then took 390 clocks to issue and the loop 640, whatever the tile width).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// A value every lane of the warp agrees on, told to the compiler.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// Thread-block cluster: barrier halves (every thread of every block of the cluster takes part), the address of
+// this block's shared memory word in block `rank`, a 16-byte load from it.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+// Orders nothing: for a rank that has only read.  (A release here would wait for the tile's stores to global memory.)
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 __device__ __forceinline__ void tcgen05_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -303,90 +337,136 @@ __device__ __forceinline__ uint32_t to_bf16x2_act(uint64_t v, float slope_lo = 0
     return d;
 }
 
-// One group of NC (= 16) accumulator columns of this thread's row: TMEM -> registers, (+ split-K
-// partial tiles), + bias (+ residual), activation, bf16, 16-byte stores.  Everything that does not
-// depend on the accumulator is fetched before the TMEM wait.  The four epilogue warps run one per
-// scheduler with nothing to hide instruction latency behind, so the column loop is kept to one
-// packed add and one convert per two columns.
-template <int NC, int ACT>
-__device__ __forceinline__ void epilogue_chunk(const ConvArgs& a, uint32_t lane_addr, int cb, int n0, bool row_valid,
-                                               __nv_bfloat16* yrow, const __nv_bfloat16* rrow, const float* part, size_t tile_floats,
-                                               const float* s_bias) {
-    uint32_t v[NC];
-    static_assert(NC == 16, "16 accumulator columns per step keep the kernel within 112 registers (three CTAs per SM)");
-    tcgen05_ld16(lane_addr + (uint32_t)cb, v);   // warp-collective: all lanes take part
-    const int k0 = n0 + cb;
-    const bool live = row_valid && k0 < a.K;
-    uint4 rv[NC / 8];
+// One group of 16 accumulator columns of this thread's row: + bias (+ residual), activation, bf16, 16-byte
+// stores.  The four epilogue warps run one per scheduler with nothing to hide instruction latency behind, so the
+// column loop is kept to one packed add and one convert per two columns.
+template <int ACT>
+__device__ __forceinline__ uint4 finish8(const ConvArgs& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias8) {
+    const uint4 b0 = *reinterpret_cast<const uint4*>(bias8), b1 = *reinterpret_cast<const uint4*>(bias8 + 4);
+    const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    const uint32_t ru[4] = {res.x, res.y, res.z, res.w};
+    uint32_t o[4];
 #pragma unroll
-    for (int h = 0; h < NC / 8; ++h) rv[h] = make_uint4(0, 0, 0, 0);
-    if (live && rrow) {
-#pragma unroll
-        for (int h = 0; h < NC / 8; ++h)
-            if (k0 + h * 8 + 8 <= a.K) rv[h] = *reinterpret_cast<const uint4*>(rrow + k0 + h * 8);
-    }
-    uint64_t bias2[NC / 2];
-#pragma unroll
-    for (int j = 0; j < NC; j += 4) {
-        const uint4 b4 = *reinterpret_cast<const uint4*>(s_bias + cb + j);
-        bias2[j / 2] = pack_f32x2(b4.x, b4.y);
-        bias2[j / 2 + 1] = pack_f32x2(b4.z, b4.w);
-    }
-    if (live && part) {
-        // every partial tile, this CTA's own included, is read from the workspace in split order, so
-        // the fp32 sum does not depend on which CTA arrived last; it starts from the bias
-        for (int z = 0; z < a.splits; ++z) {
-            const uint4* other = reinterpret_cast<const uint4*>(part + (size_t)z * tile_floats) + threadIdx.x;
-#pragma unroll
-            for (int j = 0; j < NC / 4; ++j) {
-                const uint4 o = __ldcg(other + (size_t)(cb / 4 + j) * kBM);
-                bias2[2 * j] = add_f32x2(bias2[2 * j], pack_f32x2(o.x, o.y));
-                bias2[2 * j + 1] = add_f32x2(bias2[2 * j + 1], pack_f32x2(o.z, o.w));
-            }
+    for (int j = 0; j < 4; ++j) {
+        uint64_t f = add_f32x2(pack_f32x2(v[2 * j], v[2 * j + 1]), pack_f32x2(bw[2 * j], bw[2 * j + 1]));
+        if (has_res) f = add_f32x2(f, pack_f32x2(ru[j] << 16, ru[j] & 0xffff0000u));
+        if constexpr (ACT == 3) {
+            float2 sl = make_float2(0.f, 0.f);
+            if (k < a.K) sl = __ldg(reinterpret_cast<const float2*>(a.bias + a.K + k) + j);   // slopes follow the biases
+            o[j] = to_bf16x2_act<ACT>(f, sl.x, sl.y);
+        } else {
+            o[j] = to_bf16x2_act<ACT>(f);
         }
     }
-    tcgen05_wait_ld();
-    if (!live) return;
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+template <int ACT>
+__device__ __forceinline__ void epilogue_chunk(const ConvArgs& a, const uint32_t (&v)[16], const uint4 (&rv)[2], int cb, int n0, bool row_valid,
+                                               __nv_bfloat16* yrow, bool has_res, const float* s_bias) {
+    if (!row_valid) return;
 #pragma unroll
-    for (int h = 0; h < NC / 8; ++h) {
-        const int kk = k0 + h * 8;
-        if (kk + 8 <= a.K) {
-            const uint32_t ru[4] = {rv[h].x, rv[h].y, rv[h].z, rv[h].w};
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint64_t f = bias2[h * 4 + j];
-                if (!part) f = add_f32x2(pack_f32x2(v[h * 8 + 2 * j], v[h * 8 + 2 * j + 1]), f);
-                if (rrow) f = add_f32x2(f, pack_f32x2(ru[j] << 16, ru[j] & 0xffff0000u));
-                if constexpr (ACT == 3) {
-                    const float2 sl = __ldg(reinterpret_cast<const float2*>(a.bias + a.K + kk) + j);   // slopes follow the biases
-                    o[j] = to_bf16x2_act<ACT>(f, sl.x, sl.y);
-                } else {
-                    o[j] = to_bf16x2_act<ACT>(f);
-                }
-            }
-            *reinterpret_cast<uint4*>(yrow + kk) = make_uint4(o[0], o[1], o[2], o[3]);
-        }
+    for (int h = 0; h < 2; ++h) {
+        const int k = n0 + cb + h * 8;
+        if (k + 8 <= a.K) *reinterpret_cast<uint4*>(yrow + k) = finish8<ACT>(a, v + h * 8, rv[h], has_res, k, s_bias + cb + h * 8);
     }
 }
 
+// The residual of the 16 columns from cb on (zeros where there is none).
+__device__ __forceinline__ void load_residual(const ConvArgs& a, int k0, bool row_valid, const __nv_bfloat16* rrow, uint4 (&rv)[2]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        rv[h] = make_uint4(0, 0, 0, 0);
+        if (row_valid && rrow && k0 + h * 8 + 8 <= a.K) rv[h] = *reinterpret_cast<const uint4*>(rrow + k0 + h * 8);
+    }
+}
+
+// Columns in steps of 16, two steps in flight: the next step leaves tensor memory (and its residual is on its way)
+// while this one is converted and stored.
 template <int ACT>
 __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lane_addr, int n0, bool row_valid, __nv_bfloat16* yrow,
-                                                 const __nv_bfloat16* rrow, const float* part, size_t tile_floats,
-                                                 const float* s_bias) {
-    int cb = 0;
-    for (; cb < a.BN; cb += 16)
-        epilogue_chunk<16, ACT>(a, lane_addr, cb, n0, row_valid, yrow, rrow, part, tile_floats, s_bias);
+                                                 const __nv_bfloat16* rrow, const float* s_bias) {
+    uint32_t v0[16], v1[16];
+    uint4 r0[2], r1[2];
+    const bool has_res = rrow != nullptr;
+    tcgen05_ld16(lane_addr, v0);             // warp-collective: all lanes take part
+    load_residual(a, n0, row_valid, rrow, r0);
+    for (int cb = 0; cb < a.BN; cb += 32) {
+        tcgen05_wait_ld();
+        const bool second = cb + 16 < a.BN;
+        if (second) {
+            tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
+            load_residual(a, n0 + cb + 16, row_valid, rrow, r1);
+        }
+        epilogue_chunk<ACT>(a, v0, r0, cb, n0, row_valid, yrow, has_res, s_bias);
+        if (!second) break;
+        tcgen05_wait_ld();
+        if (cb + 32 < a.BN) {
+            tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
+            load_residual(a, n0 + cb + 32, row_valid, rrow, r0);
+        }
+        epilogue_chunk<ACT>(a, v1, r1, cb + 16, n0, row_valid, yrow, has_res, s_bias);
+    }
+}
+
+// The same with the tile leaving through TMA stores.  A warp's 16-byte stores touch 32 lines each: 128 columns are
+// 16 x 32 line accesses per warp, 2048 clocks of the SM's one store path per tile (1.9 us measured, and co-resident
+// tiles queue behind each other).  So each warp lays its 32 rows out in shared memory, boxes of U columns in the
+// swizzle of their row length (no bank conflicts), and one lane stores a finished box with one instruction.  `buf`: the
+// warp's 32 x BN x 2 bytes of the pipeline memory, free by now.
+template <int ACT>
+__device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t lane_addr, int n0, bool row_valid, const __nv_bfloat16* rrow,
+                                                     const float* s_bias, uint32_t buf, const CUtensorMap* tmap_y, int m_warp) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const int U = a.out_box;
+    const uint32_t swz = U == 64 ? lane & 7u : (lane >> 1) & 3u;
+    const uint32_t row = buf + lane * (uint32_t)(U * 2);
+    const bool has_res = rrow != nullptr;
+    uint32_t v0[16], v1[16];
+    uint4 r0[2], r1[2];
+    auto put = [&](const uint32_t (&v)[16], const uint4 (&rv)[2], int cb) {
+        const int in_box = cb & (U - 1);
+        const uint32_t box = (uint32_t)(cb - in_box) * 64u;      // 32 rows x 2 bytes per column before this box
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint4 o = finish8<ACT>(a, v + h * 8, rv[h], has_res, n0 + cb + h * 8, s_bias + cb + h * 8);
+            st_shared_v4(row + box + ((((uint32_t)(in_box >> 3) + (uint32_t)h) ^ swz) << 4), o.x, o.y, o.z, o.w);
+        }
+        if (in_box + 16 == U) {
+            fence_proxy_async();
+            __syncwarp();
+            const int x = n0 + cb - in_box;
+            if (x < a.K && m_warp < a.M && elect_one()) tma_store_2d(tmap_y, x, m_warp, buf + box);
+            __syncwarp();
+        }
+    };
+    tcgen05_ld16(lane_addr, v0);             // warp-collective: all lanes take part
+    load_residual(a, n0, row_valid, rrow, r0);
+    for (int cb = 0; cb < a.BN; cb += 32) {
+        tcgen05_wait_ld();
+        const bool second = cb + 16 < a.BN;
+        if (second) {
+            tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
+            load_residual(a, n0 + cb + 16, row_valid, rrow, r1);
+        }
+        put(v0, r0, cb);
+        if (!second) break;
+        tcgen05_wait_ld();
+        if (cb + 32 < a.BN) {
+            tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
+            load_residual(a, n0 + cb + 32, row_valid, rrow, r0);
+        }
+        put(v1, r1, cb + 16);
+    }
+    if (elect_one()) tma_store_wait();       // shared memory may go, and the tile is in memory
+    __syncwarp();
 }
 
 // Epilogue, run by warps 0-3 (thread t owns accumulator lane t = tile row t): wait for the
-// accumulator, optionally meet the other split-K CTAs of the tile in the workspace, then
-// bias + residual + activation and bf16 stores into the output channel slice.  (Staging the bf16
-// tile in shared memory for row-contiguous stores was measured slower: the epilogue is bound by its
-// instruction count, not by the scattered 16-byte stores.)
-__device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, bool ok, int m0, int n0, uint32_t tile, uint32_t split,
-                                     const float* s_bias, uint64_t* s_accum_p, volatile uint32_t* s_abort_p, uint32_t* s_is_last_p,
-                                     uint32_t accum_parity = 0u) {
+// accumulator, then bias + residual + activation and bf16 stores into the output channel slice.
+// tmap_y (the one-tile kernels): through TMA stores staged at `buf`.
+__device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, bool ok, int m0, int n0, const float* s_bias,
+                                         uint64_t* s_accum_p, volatile uint32_t* s_abort_p, uint32_t accum_parity = 0u,
+                                         const CUtensorMap* tmap_y = nullptr, uint32_t buf = 0) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int m = m0 + tid;
@@ -396,46 +476,139 @@ __device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, 
     if (tid == 0) PB_T(5);
     tcgen05_fence_after();
     const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-    // Partial tiles in the workspace are stored [BN/4][128 rows] x float4, so consecutive lanes
-    // (= rows) touch consecutive 16-byte words.
-    const size_t tile_floats = (size_t)kBM * a.BN;
-    bool finalize = ok;
-    if (a.splits > 1) {
-        // Park this CTA's partial tile; the CTA that arrives last on the tile's counter adds the
-        // others to its own accumulators and runs the epilogue.
-        float4* mine = reinterpret_cast<float4*>(a.ws + ((size_t)tile * a.splits + split) * tile_floats) + tid;
-        if (ok) {
-            for (int cb = 0; cb < a.BN; cb += 16) {
-                uint32_t v[16];
-                tcgen05_ld16(lane_addr + (uint32_t)cb, v);
-                tcgen05_wait_ld();
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    mine[(size_t)(cb / 4 + j) * kBM] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                                    __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-            }
-        }
-        __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");          // the four epilogue warps only
-        if (tid == 0) {
-            const unsigned prev = atomicAdd(a.counters + tile, 1u);
-            const bool last = prev == (unsigned)a.splits - 1u;
-            if (last) a.counters[tile] = 0;                      // ready for the next launch
-            __threadfence();
-            *s_is_last_p = last ? 1u : 0u;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        finalize = ok && *s_is_last_p != 0;
+    if (!ok) return;
+    const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
+    if (tmap_y) {
+        buf += (uint32_t)warp * (uint32_t)a.BN * 64u;
+        const int m_warp = m0 + warp * 32;
+        if (a.act == 3) epilogue_columns_tma<3>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
+        else if (a.act == 1) epilogue_columns_tma<1>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
+        else if (a.act == 2) epilogue_columns_tma<2>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
+        else epilogue_columns_tma<0>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
+        return;
     }
-    if (finalize) {
+    __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
+    if (a.act == 3) epilogue_columns<3>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    else if (a.act == 1) epilogue_columns<1>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    else if (a.act == 2) epilogue_columns<2>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    else epilogue_columns<0>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+}
+
+// ---- split reduction: the thread blocks of a cluster share one output tile -----------------------------------
+// Rank z of the cluster multiplies its share of the k-blocks; then rank d finishes columns [d*w, (d+1)*w) of the
+// tile, w = BN / splits.  Every rank parks the columns it does not own in its own shared memory (the pipeline
+// buffers, free once its multiplications are done), 16 bytes per lane and consecutive lanes (= rows) side by side;
+// after a cluster barrier the owner reads the other ranks' parts through distributed shared memory, all of them in
+// flight together, and adds them in rank order, so the fp32 result does not depend on timing.  One cluster barrier
+// on the critical path, nothing goes through global memory; a second one, over which the stores run, keeps every
+// rank's memory alive until it has been read.
+// (The partial tiles used to meet in a global workspace under an atomic counter: two fences, an atomic and an L2
+// round trip of BN x 512 bytes per rank, read back by ONE block: +4 to +8 us per launch, so only reductions of 60
+// and more k-blocks gained from it.)
+template <int ACT, int S>
+__device__ __forceinline__ void cluster_finish(const ConvArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
+                                               const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
+    constexpr int kOct = S == 2 ? 2 : 1;      // groups of 8 columns per turn
+    constexpr int kRanks = S < 4 ? S : 4;     // ranks whose loads are in flight together (16-byte loads: up to 8 a thread; more spill)
+    uint32_t active = 0;           // ranks that have k-blocks (all of them unless a grouped launch splits a short reduction)
+#pragma unroll
+    for (int z = 0; z < S; ++z) active |= (a.nkb * (z + 1) / S > a.nkb * z / S ? 1u : 0u) << z;
+    for (int c = 0; c < w; c += 8 * kOct) {
+        uint64_t sum[kOct][4];
+#pragma unroll
+        for (int o = 0; o < kOct; ++o)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[o][j] = 0;        // (+0 is exact; a sum of zeros may lose a -0, which the bias add would too)
+#pragma unroll
+        for (int z0 = 0; z0 < S; z0 += kRanks) {
+            uint4 part[kOct][kRanks][2];
+#pragma unroll
+            for (int o = 0; o < kOct; ++o) {
+                const uint32_t src = buf + ((uint32_t)((rank * w + c + 8 * o) >> 2) * 128u + threadIdx.x) * 16u;
+#pragma unroll
+                for (int z = 0; z < kRanks; ++z) {
+                    part[o][z][0] = part[o][z][1] = make_uint4(0, 0, 0, 0);
+                    if (c + 8 * o >= w || !((active >> (z0 + z)) & 1u)) continue;
+                    const uint32_t at = cluster_addr(src, (uint32_t)(z0 + z));       // this rank's own part too
+                    part[o][z][0] = ld_cluster_v4(at);
+                    part[o][z][1] = ld_cluster_v4(at + 2048u);
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < kOct; ++o)
+#pragma unroll
+                for (int z = 0; z < kRanks; ++z) {
+                    const uint4 lo = part[o][z][0], hi = part[o][z][1];
+                    sum[o][0] = add_f32x2(sum[o][0], pack_f32x2(lo.x, lo.y));
+                    sum[o][1] = add_f32x2(sum[o][1], pack_f32x2(lo.z, lo.w));
+                    sum[o][2] = add_f32x2(sum[o][2], pack_f32x2(hi.x, hi.y));
+                    sum[o][3] = add_f32x2(sum[o][3], pack_f32x2(hi.z, hi.w));
+                }
+        }
+#pragma unroll
+        for (int o = 0; o < kOct; ++o) {
+            const int col = rank * w + c + 8 * o, k = n0 + col;
+            if (c + 8 * o >= w || !row_valid || k >= a.K) continue;
+            uint4 res = make_uint4(0, 0, 0, 0);
+            if (rrow) res = *reinterpret_cast<const uint4*>(rrow + k);
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(sum[o][j]));
+            *reinterpret_cast<uint4*>(yrow + k) = finish8<ACT>(a, v, res, rrow != nullptr, k, s_bias + col);
+        }
+    }
+}
+template <int ACT>
+__device__ __forceinline__ void cluster_finish(const ConvArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
+                                               const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
+    if (a.splits == 2) cluster_finish<ACT, 2>(a, n0, row_valid, yrow, rrow, s_bias, rank, buf, w);
+    else if (a.splits == 4) cluster_finish<ACT, 4>(a, n0, row_valid, yrow, rrow, s_bias, rank, buf, w);
+    else cluster_finish<ACT, 8>(a, n0, row_valid, yrow, rrow, s_bias, rank, buf, w);
+}
+
+// Run by warps 0-3 of every rank.  `mine`: this rank has k-blocks of its own.
+__device__ __forceinline__ void epilogue_cluster(const ConvArgs& a, uint32_t tmem_base, int m0, int n0, int rank, bool mine, uint32_t smem_base,
+                                                 const float* s_bias, uint64_t* s_accum_p, volatile uint32_t* s_abort_p) {
+    const int tid = threadIdx.x;
+    const int warp = tid >> 5;
+    const int m = m0 + tid;
+    const bool row_valid = m < a.M;
+    bool ok = mbar_wait(smem_u32(s_accum_p), 0u, s_abort_p, a.err_flag, 3u);
+    ok = __all_sync(0xffffffffu, ok);
+    if (tid == 0) PB_T(5);
+    tcgen05_fence_after();
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
+    const int w = a.BN / a.splits;
+    if (mine) {
+        uint32_t v0[16], v1[16];
+        uint32_t at = smem_base + (uint32_t)tid * 16u;
+        tcgen05_ld16(lane_addr, v0);
+        for (int cb = 0; cb < a.BN; cb += 32) {
+            tcgen05_wait_ld();
+            if (cb + 16 < a.BN) tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) st_shared_v4(at + (uint32_t)j * 2048u, v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
+            if (cb + 16 >= a.BN) break;
+            tcgen05_wait_ld();
+            if (cb + 32 < a.BN) tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) st_shared_v4(at + 8192u + (uint32_t)j * 2048u, v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
+            at += 16384u;
+        }
+    }
+    cluster_arrive();
+    cluster_wait();                 // every rank's columns are parked
+    if (tid == 0) PB_T(6);
+    if (ok) {
         __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
         const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
-        const float* part = a.splits > 1 ? a.ws + (size_t)tile * a.splits * tile_floats : nullptr;
-        if (a.act == 3) epilogue_columns<3>(a, lane_addr, n0, row_valid, yrow, rrow, part, tile_floats, s_bias);
-        else if (a.act == 1) epilogue_columns<1>(a, lane_addr, n0, row_valid, yrow, rrow, part, tile_floats, s_bias);
-        else if (a.act == 2) epilogue_columns<2>(a, lane_addr, n0, row_valid, yrow, rrow, part, tile_floats, s_bias);
-        else epilogue_columns<0>(a, lane_addr, n0, row_valid, yrow, rrow, part, tile_floats, s_bias);
+        if (a.act == 3) cluster_finish<3>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        else if (a.act == 1) cluster_finish<1>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        else if (a.act == 2) cluster_finish<2>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        else cluster_finish<0>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
     }
+    cluster_arrive_relaxed();
+    cluster_wait();                 // every rank has read what it needs: shared memory may go
 }
 
 template <int kStages>
@@ -447,7 +620,6 @@ conv_umma_gather_kernel(const __grid_constant__ CUtensorMap tmap_w, const ConvAr
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
-    __shared__ uint32_t s_is_last;
     __shared__ __align__(16) float s_bias[128];
     constexpr int kLag = PB_LAG_OF(kStages);
 
@@ -463,9 +635,7 @@ conv_umma_gather_kernel(const __grid_constant__ CUtensorMap tmap_w, const ConvAr
 
     const int m0 = blockIdx.x * kBM;
     const int n0 = blockIdx.y * a.BN;
-    const int kb_begin = blockIdx.z * a.kb_per_split;
-    const int kb_end = min(a.nkb, kb_begin + a.kb_per_split);
-    const int nkb = kb_end - kb_begin;          // >= 1 by construction of the grid
+    const int kb_begin = 0, nkb = a.nkb;         // this kernel never splits the reduction
 
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -567,7 +737,7 @@ conv_umma_gather_kernel(const __grid_constant__ CUtensorMap tmap_w, const ConvAr
             for (int kb = (nkb > kLag ? nkb - kLag : 0); kb < nkb; ++kb) mbar_arrive(smem_u32(&s_full[kb % kStages]));
 
         // ===== epilogue: accumulator lane `tid` = tile row `tid` =====
-        epilogue(a, tmem_base, ok, m0, n0, blockIdx.y * gridDim.x + blockIdx.x, blockIdx.z, s_bias, &s_accum, &s_abort, &s_is_last);
+        epilogue(a, tmem_base, ok, m0, n0, s_bias, &s_accum, &s_abort);
         if (tid == 0) PB_T(6);
     } else {
         // ===== MMA issuer: one thread =====
@@ -614,19 +784,21 @@ conv_umma_gather_kernel(const __grid_constant__ CUtensorMap tmap_w, const ConvAr
 }
 
 // ---- the kernel, operand A by im2col TMA ---------------------------------------------------------
-// CTA = 6 warps.  Warp 4: one thread issues, per k-block, one im2col TMA for A (128 output pixels x
-// 64 channels of one filter tap) and one tiled TMA for B.  Warp 5: allocates TMEM, one thread issues
-// the MMAs.  Warps 0-3 only run the epilogue.  No thread computes an address in the main loop.
+// CTA = 6 warps, each with a short loop of its own: warps 0-3 the epilogue, before it warp 3 operand B (one tiled TMA of
+// weights per k-block), warp 4 operand A (one im2col TMA of 128 output pixels x 64 channels of one filter tap), warp 5
+// tensor memory and the MMAs.  No thread computes an address in the main loop.  (A seventh warp for operand B would
+// leave 80 registers a thread at three CTAs per SM instead of 96.)
 constexpr int kThreadsTma = 192;
+constexpr int kWarpB = 3;
 
-// One CTA's share of one convolution: output tile (bx, by) of a grid gx tiles wide, reduction
-// slice bz, `stages` pipeline buffers.  Shared by the single-convolution kernel and the grouped one.
-__device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const ConvArgs& a, const int stages,
-                                              const int bx, const int by, const int bz, const int gx, uint8_t* smem_raw,
+// One CTA's share of one convolution: output tile (bx, by), rank bz of the cluster that shares the tile's
+// reduction, `stages` pipeline buffers.  Shared by the single-convolution kernel and the grouped one.
+__device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const CUtensorMap* tmap_y, const ConvArgs& a, const int stages,
+                                              const int bx, const int by, const int bz, uint8_t* smem_raw,
                                               uint64_t* s_full, uint64_t* s_empty, uint64_t* s_accum, uint32_t* s_tmem_base,
-                                              volatile uint32_t* s_abort, uint32_t* s_is_last, float* s_bias) {
+                                              volatile uint32_t* s_abort, float* s_bias) {
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = (int)uniform((uint32_t)tid >> 5);
     const int lane = tid & 31;
 #ifdef PB_CONV_STATS
     __shared__ long long s_clk[8];
@@ -647,25 +819,49 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 
     const int m0 = bx * kBM;
     const int n0 = by * a.BN;
-    const int kb_begin = bz * a.kb_per_split;
-    const int kb_end = min(a.nkb, kb_begin + a.kb_per_split);
-    const int nkb = kb_end - kb_begin;
+    const int kb_begin = a.nkb * bz / a.splits;
+    const int nkb = a.nkb * (bz + 1) / a.splits - kb_begin;       // 0 for some ranks of a cluster larger than the k-block count
 
-    // the first copy of each descriptor otherwise pays its fetch into the descriptor cache
-    if (tid == 32) asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_w) : "memory");
-    if (tid == 64) asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
-    if (tid == 0) {
-        for (int s = 0; s < stages; ++s) {
-            mbar_init(smem_u32(&s_full[s]), 1);      // the producer's arrive.expect_tx
-            mbar_init(smem_u32(&s_empty[s]), 1);     // tcgen05.commit
+    // Operand B's warp sets the barriers up and starts at once on the first turn of the pipeline: the weights are
+    // constant, so they need neither the other warps nor the previous kernel.  It also arms each stage's barrier with the
+    // byte count of both operands.  (Operand A's bytes may land before that: the transaction count goes negative for a
+    // moment, and the phase cannot complete before the arrival.)
+    const uint32_t tx_bytes = (uint32_t)kATileBytes + a.b_stage_bytes;
+    if (warp == kWarpB) {
+        if (elect_one()) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_w) : "memory");
+            for (int s = 0; s < stages; ++s) {
+                mbar_init(smem_u32(&s_full[s]), 1);      // this warp's arrive.expect_tx, for the bytes of both operands
+                mbar_init(smem_u32(&s_empty[s]), 1);     // tcgen05.commit
+            }
+            mbar_init(smem_u32(s_accum), 1);
+            *s_abort = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
-        mbar_init(smem_u32(s_accum), 1);
-        *s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
+        for (int q = 0; q < stages && q < nkb; ++q) {
+            if (elect_one()) {
+                mbar_arrive_expect_tx(smem_u32(&s_full[q]), tx_bytes);
+                tma_load_2d(smem_base + (uint32_t)q * stage_bytes + kATileBytes, tmap_w, (kb_begin + q) * kBK, n0, smem_u32(&s_full[q]));
+            }
+            __syncwarp();
+        }
     }
-    for (int j = tid; j < a.BN; j += kThreadsTma) {
-        const int k = n0 + j;
-        s_bias[j] = (a.bias && k < a.K) ? __ldg(a.bias + k) : 0.f;
+    // Where the tile's pixels start is worked out before the wait for the previous kernel.
+    int img = 0, w0 = 0, h0 = 0, tap_r = 0, tap_s = 0, chunk = 0;
+    const int cpt = a.Cp / kBK;               // k-blocks per filter tap
+    if (warp == 4) {
+        if (elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
+        img = m0 / a.PQ;                      // the tile may run on into the next image
+        const int rem = m0 - img * a.PQ;
+        const int p0 = rem / a.Q, q0 = rem - p0 * a.Q;
+        w0 = q0 * a.sw - a.pw;                // filter-window origin of the tile's first pixel
+        h0 = p0 * a.sh - a.ph;
+        const int tap = kb_begin / cpt;
+        chunk = kb_begin - tap * cpt;
+        tap_r = tap / a.S;
+        tap_s = tap - tap_r * a.S;
     }
     if (warp == 5) {
         tcgen05_alloc(smem_u32(s_tmem_base), a.tmem_cols);
@@ -674,124 +870,107 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    const uint32_t tmem_base = *s_tmem_base;
-    if (threadIdx.x == 0) { PB_T(1); PB_S(1); }
-    // Everything above touched only this CTA's shared/tensor memory and constant weights (bias), so it
-    // may overlap the previous kernel's tail.  Activations, the residual, the output and the split-K
-    // workspace may only be touched once the previous kernel has completed.
-    griddep_wait();
-    if (threadIdx.x == 0) PB_S(2);
-
-    // ===== producers: lane 0 of warp 4 and of the four epilogue warps =====
-    // A thread that issues tensor copies one after the other is slow however small the copies: measured with a
-    // copy-only kernel on tiles like these, one thread sustains one 16 KB copy per ~650 clocks (25 B/clk) at any
-    // pipeline depth, four issuing warps of the same CTA 100 B/clk, and the whole GPU saturates near 60 B/clk per
-    // SM.  The tensor cores need a k-block (two copies) every ~270 clocks, so a lone producer thread paced the
-    // whole CTA.  The epilogue warps have nothing to do until the accumulator is complete, so lane 0 of each
-    // joins warp 4: the 2 x stages (stage, operand) pairs are dealt round-robin to the kProducers threads, and a
-    // pair is always refilled by the same thread, in k order.  The thread that loads operand A also arms the
-    // stage's barrier with the byte count of both copies; operand B's bytes may land before that (the
-    // transaction count goes negative for a moment; the phase cannot complete before the arrival).
-    // (Several lanes of ONE warp would not do: they reconverge after each wait, so no copy could be issued
-    // before every stage had been drained.)
-    constexpr int kProducers = 5;
-    const int prod = warp == 4 ? 0 : warp + 1;              // producer index of this warp's lane 0
-    if (warp <= 4 && lane == 0) {
-        const int img = m0 / a.PQ, rem = m0 - img * a.PQ;      // the tile may run on into the next image
-        const int p0 = rem / a.Q, q0 = rem - p0 * a.Q;
-        const int w0 = q0 * a.sw - a.pw;          // filter-window origin of the tile's first pixel
-        const int h0 = p0 * a.sh - a.ph;
-        const int cpt = a.Cp / kBK;               // k-blocks per filter tap
-        bool ok = true;
-        int st = 0;
-        uint32_t parity = 1u;                     // a fresh barrier passes a wait on the "previous" phase
-        // which (stage, operand) pairs are this thread's (bit st), and the filter tap / channel chunk of the k-block,
-        // carried along: a division per k-block is a tenth of what the thread has per copy
-        uint32_t mask_a = 0, mask_b = 0;
-        for (int q = 0; q < stages; ++q) {
-            if ((q * 2) % kProducers == prod) mask_a |= 1u << q;
-            if ((q * 2 + 1) % kProducers == prod) mask_b |= 1u << q;
-        }
-        int tap = kb_begin / cpt, chunk = kb_begin - tap * cpt;
-        int r = tap / a.S, s = tap - r * a.S;
-        uint32_t* const err_flag = a.err_flag;
-        for (int kb = 0; kb < nkb && ok; ++kb) {
-            const bool mine_a = (mask_a >> st) & 1u, mine_b = (mask_b >> st) & 1u;
-            if (mine_a || mine_b) {
-                ok = mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u);
-                if (!ok) break;
-                const uint32_t a_tile = smem_base + (uint32_t)st * stage_bytes;
-                const uint32_t bar = smem_u32(&s_full[st]);
-                const int kbg = kb_begin + kb;
-                if (mine_a) {
-                    mbar_arrive_expect_tx(bar, (uint32_t)kATileBytes + a.b_stage_bytes);
-                    if (a.a_tiled) tma_load_2d(a_tile, tmap_x, chunk * kBK, m0, bar);
-                    else tma_load_im2col_4d(a_tile, tmap_x, chunk * kBK, w0, h0, img, (uint16_t)(s * a.dw), (uint16_t)(r * a.dh), bar);
-                    if (kb == 0) PB_T(2);
-                    PB_TK(kb, 0);
-                }
-                if (mine_b) tma_load_2d(a_tile + kATileBytes, tmap_w, kbg * kBK, n0, bar);
-            }
-            if (++chunk == cpt) {
-                chunk = 0;
-                if (++s == a.S) { s = 0; ++r; }
-            }
-            if (++st == stages) { st = 0; parity ^= 1u; }
-        }
-    }
-    if (warp <= 4) __syncwarp();
+    const uint32_t tmem_base = uniform(*s_tmem_base);
+    if (tid == 0) { PB_T(1); PB_S(1); }
 
     if (warp < 4) {
-        griddep_launch();      // the next kernel's blocks may be scheduled as SM resources free up
-        epilogue(a, tmem_base, true, m0, n0, (uint32_t)(by * gx + bx), (uint32_t)bz, s_bias, s_accum, s_abort, s_is_last);
+        if (warp == kWarpB) {
+            // ===== operand B, from the second turn of the pipeline on =====
+            uint32_t* const err_flag = a.err_flag;
+            uint32_t st = 0, parity = 0u;
+            for (int kb = stages; kb < nkb; ++kb) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u))) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(smem_u32(&s_full[st]), tx_bytes);
+                    tma_load_2d(smem_base + st * stage_bytes + kATileBytes, tmap_w, (kb_begin + kb) * kBK, n0, smem_u32(&s_full[st]));
+                }
+                __syncwarp();
+                if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
+            }
+        } else {
+            // the epilogue's biases
+            for (int j = tid; j < a.BN; j += 32 * kWarpB) {
+                const int k = n0 + j;
+                s_bias[j] = (a.bias && k < a.K) ? __ldg(a.bias + k) : 0.f;
+            }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        // The residual and the output may only be touched once the previous kernel has completed; the next kernel's
+        // blocks may be scheduled as SM resources free up.
+        griddep_wait();
+        if (tid == 0) PB_S(2);
+        griddep_launch();
+        if (a.splits > 1) epilogue_cluster(a, tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
+        else epilogue(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base);
         if (tid == 0) { PB_T(6); PB_S(6); }
     } else if (warp == 4) {
-        __syncwarp();
+        // ===== operand A =====
+        griddep_wait();                           // the activations are the previous kernel's
+        uint32_t* const err_flag = a.err_flag;
+        const int S = a.S, dw = a.dw, dh = a.dh, a_tiled = a.a_tiled;
+        uint32_t st = 0, parity = 1u;             // a fresh barrier passes a wait on the "previous" phase
+        for (int kb = 0; kb < nkb; ++kb) {
+            if (kb >= stages && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u))) break;
+            if (elect_one()) {
+                const uint32_t a_tile = smem_base + st * stage_bytes, bar = smem_u32(&s_full[st]);
+                if (a_tiled) tma_load_2d(a_tile, tmap_x, chunk * kBK, m0, bar);
+                else tma_load_im2col_4d(a_tile, tmap_x, chunk * kBK, w0, h0, img, (uint16_t)(tap_s * dw), (uint16_t)(tap_r * dh), bar);
+                if (kb == 0) PB_T(2);
+                PB_TK(kb, 0);
+            }
+            __syncwarp();
+            if (++chunk == cpt) {
+                chunk = 0;
+                if (++tap_s == S) { tap_s = 0; ++tap_r; }
+            }
+            if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
+        }
         griddep_launch();
+        if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
     } else {
-        // ===== MMA issuer: one thread =====
-        // This thread's own instruction chain per k-block paces the CTA (measured: four MMA issues + commit ~320
-        // clocks, most of it the tensor cores taking the instructions, then ~400 clocks until the next k-block's
-        // barrier had been looked at; an mbarrier wait costs ~170 clocks even when its phase is long complete).
-        // So the NEXT k-block's barrier is probed (test_wait, never blocks) before this k-block's MMAs are issued:
-        // the probe's latency runs under them; and the descriptors are stage 0's plus a stride.
-        if (lane == 0) {
-            uint32_t st = 0, parity = 0u;
-            bool ok = true, have_next = false;
-            uint32_t* const err_flag = a.err_flag;
-            const uint32_t idesc = a.idesc;
-            const uint64_t desc_a0 = umma_desc_sw128(smem_base), desc_b0 = umma_desc_sw128(smem_base + kATileBytes);
-            const uint64_t desc_step = (uint64_t)(stage_bytes >> 4);      // address field counts 16-byte units; no carry out of its 14 bits
-            for (int kb = 0; kb < nkb; ++kb) {
-                if (!have_next) {
-                    ok = mbar_wait(smem_u32(&s_full[st]), parity, s_abort, err_flag, 2u);
-                    if (!ok) break;
-                }
-                if (kb == 0) { PB_T(3); PB_S(3); }
-                PB_TK(kb, 1);
-                tcgen05_fence_after();
-                uint32_t st_n = st + 1, parity_n = parity;
-                if (st_n == (uint32_t)stages) { st_n = 0; parity_n ^= 1u; }
-                have_next = kb + 1 < nkb && mbar_test_wait(smem_u32(&s_full[st_n]), parity_n);
-                const uint64_t da = desc_a0 + (uint64_t)st * desc_step, db = desc_b0 + (uint64_t)st * desc_step;
+        // ===== MMA issuer =====
+        // An mbarrier wait costs ~170 clocks even when its phase is long complete, so the NEXT k-block's barrier is
+        // probed (test_wait, never blocks) before this k-block's MMAs are issued: the probe's latency runs under them;
+        // and the descriptors are stage 0's plus a stride.
+        uint32_t st = 0, parity = 0u;
+        bool ok = true, have_next = false;
+        uint32_t* const err_flag = a.err_flag;
+        const uint32_t idesc = uniform(a.idesc), n_kb = uniform((uint32_t)nkb), n_st = uniform((uint32_t)stages);
+        const uint64_t desc_a0 = umma_desc_sw128(uniform(smem_base)), desc_b0 = umma_desc_sw128(uniform(smem_base) + kATileBytes);
+        const uint32_t desc_step = uniform(stage_bytes) >> 4;      // address field counts 16-byte units; no carry out of its 14 bits
+        for (uint32_t kb = 0; kb < n_kb; ++kb) {
+            if (!__all_sync(0xffffffffu, have_next)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, s_abort, err_flag, 2u));
+                if (!ok) break;
+            }
+            if (lane == 0) { if (kb == 0) { PB_T(3); PB_S(3); } PB_TK(kb, 1); }
+            tcgen05_fence_after();
+            uint32_t st_n = st + 1, parity_n = parity;
+            if (st_n == n_st) { st_n = 0; parity_n ^= 1u; }
+            have_next = kb + 1 < n_kb && mbar_test_wait(smem_u32(&s_full[st_n]), parity_n);
+            const uint64_t da = desc_a0 + st * desc_step, db = desc_b0 + st * desc_step;
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < kBK / 16; ++k)
                     tcgen05_mma_bf16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);   // +32 bytes per K=16 slice
                 tcgen05_commit(smem_u32(&s_empty[st]));
-                PB_TK(kb, 2);
-                st = st_n;
-                parity = parity_n;
             }
-            PB_S(4);
-            if (ok) tcgen05_commit(smem_u32(s_accum));
-            PB_T(4);
-#ifdef PB_CONV_STATS
-            if (ok) mbar_wait(smem_u32(s_accum), 0u, s_abort, a.err_flag, 3u);
-            PB_S(5);
-#endif
+            __syncwarp();
+            if (lane == 0) PB_TK(kb, 2);
+            st = st_n;
+            parity = parity_n;
         }
+        if (lane == 0) PB_S(4);
+        if (ok && elect_one()) tcgen05_commit(smem_u32(s_accum));
+        __syncwarp();
+        if (lane == 0) PB_T(4);
+#ifdef PB_CONV_STATS
+        if (ok) mbar_wait(smem_u32(s_accum), 0u, s_abort, a.err_flag, 3u);
+        if (lane == 0) PB_S(5);
+#endif
         __syncwarp();
         griddep_launch();
+        if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
     }
 
     tcgen05_fence_before();
@@ -824,22 +1003,21 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 }
 
 __global__ void __launch_bounds__(kThreadsTma, 3)
-conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const ConvArgs a,
-                     int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
+conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                     const __grid_constant__ CUtensorMap tmap_y, const ConvArgs a, int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxStages];
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
-    __shared__ uint32_t s_is_last;
     __shared__ __align__(16) float s_bias[kMaxBN];
 
     resolve_slot(job_id, nf);
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
-    conv_tile_tma(&tmap_w, &tmap_x, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.x, smem_raw, s_full,
-                  s_empty, &s_accum, &s_tmem_base, &s_abort, &s_is_last, s_bias);
+    conv_tile_tma(&tmap_w, &tmap_x, &tmap_y, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+                  &s_tmem_base, &s_abort, s_bias);
     if (nf) nf->end(job_id);
 }
 
@@ -864,6 +1042,7 @@ struct PoolSubArgs {
 struct alignas(128) SubConv {
     CUtensorMap tmap_w;
     CUtensorMap tmap_x;
+    CUtensorMap tmap_y;
     union {
         ConvArgs a;
         PoolSubArgs pool;
@@ -948,7 +1127,6 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
-    __shared__ uint32_t s_is_last;
     __shared__ __align__(16) float s_bias[kMaxBN];
     __shared__ __align__(16) ConvArgs s_args;
 
@@ -972,11 +1150,12 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
         if (nf) nf->end(job_id);
         return;
     }
-    const uint32_t gx = sc->gx, gy = sc->gy;
-    const uint32_t bx = local % gx, rest = local / gx;
-    const uint32_t by = rest % gy, bz = rest / gy;
-    conv_tile_tma(&sc->tmap_w, &sc->tmap_x, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, (int)gx, smem_raw, s_full, s_empty,
-                  &s_accum, &s_tmem_base, &s_abort, &s_is_last, s_bias);
+    // the ranks of a cluster are consecutive blocks (every sub-problem of a launch has the same split)
+    const uint32_t S = (uint32_t)s_args.splits, gx = sc->gx;
+    const uint32_t tile = local / S, bz = local - tile * S;
+    const uint32_t by = tile / gx, bx = tile - by * gx;
+    conv_tile_tma(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
+                  &s_tmem_base, &s_abort, s_bias);
     if (nf) nf->end(job_id);
 }
 
@@ -995,8 +1174,8 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
 // pair is always refilled by the same thread).  Sized for two CTAs per SM: <= 108 KB of pipeline, 288 threads
 // of <= 112 registers, 2 x 128 tensor-memory columns.
 // Every tile comes from the launch's table of sub-problems (one entry for a lone convolution, several for the
-// independent convolutions of a grouped launch): tile index -> entry by first_block, then (m tile, n tile,
-// k split) inside it.
+// independent convolutions of a grouped launch): tile index -> entry by first_block, then (m tile, n tile)
+// inside it.  It never splits a reduction.
 constexpr int kPersistProducers = 4;
 constexpr int kThreadsPersist = 32 * (5 + kPersistProducers);
 #ifndef PB_CONV_PERSIST_SMEM_KB
@@ -1014,7 +1193,7 @@ struct SubArgs {
 struct TileRef {
     const SubArgs* sa;
     const SubConv* sc;
-    int bx, by, bz;
+    int bx, by;
 };
 __device__ __forceinline__ TileRef tile_ref(const SubConv* __restrict__ table, const SubArgs* s_sub, int n_sub, uint32_t t) {
     int sub = 0;
@@ -1023,11 +1202,9 @@ __device__ __forceinline__ TileRef tile_ref(const SubConv* __restrict__ table, c
     r.sa = s_sub + sub;
     r.sc = table + sub;
     const uint32_t local = t - r.sa->first_block;
-    const uint32_t gx = r.sa->gx, gy = r.sa->gy;
-    r.bx = (int)(local % gx);
-    const uint32_t rest = local / gx;
-    r.by = (int)(rest % gy);
-    r.bz = (int)(rest / gy);
+    const uint32_t gx = r.sa->gx;
+    r.by = (int)(local / gx);
+    r.bx = (int)(local - (uint32_t)r.by * gx);
     return r;
 }
 
@@ -1041,7 +1218,6 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
     __shared__ __align__(8) uint64_t s_tempty[2];      // accumulator read out (one arrival per epilogue warp)
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
-    __shared__ uint32_t s_is_last;
     __shared__ __align__(16) float s_bias[2][kMaxBN];
     __shared__ __align__(16) SubArgs s_sub[kMaxSubConvs];
 
@@ -1118,8 +1294,7 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (tid == 0) PB_PT(i, 2);
-            epilogue(a, tmem_base + acc * acc_cols, true, tr.bx * kBM, n0, (uint32_t)(tr.by * (int)tr.sa->gx + tr.bx), (uint32_t)tr.bz,
-                     s_bias[acc], &s_tfull[acc], &s_abort, &s_is_last, use & 1u);
+            epilogue(a, tmem_base + acc * acc_cols, true, tr.bx * kBM, n0, s_bias[acc], &s_tfull[acc], &s_abort, use & 1u);
             if (tid == 0) PB_PT(i, 3);
             // this accumulator may be overwritten: every tcgen05.ld of the warp has completed (wait::ld)
             tcgen05_fence_before();
@@ -1148,8 +1323,7 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
                 const uint32_t acc = i & 1u, use = i >> 1;
                 const TileRef tr = tile_ref(table, s_sub, n_sub, t);
                 const ConvArgs& a = tr.sa->a;
-                const int kb_begin = tr.bz * a.kb_per_split;
-                const int nkb = min(a.nkb, kb_begin + a.kb_per_split) - kb_begin;
+                const int nkb = a.nkb;
                 const uint32_t idesc = a.idesc;
 #ifdef PB_CONV_STATS
                 const bool first_tile = i == 0;
@@ -1205,8 +1379,7 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
                 const ConvArgs& a = tr.sa->a;
                 const CUtensorMap* tmap_w = &tr.sc->tmap_w;
                 const CUtensorMap* tmap_x = &tr.sc->tmap_x;
-                const int kb_begin = tr.bz * a.kb_per_split;
-                const int nkb = min(a.nkb, kb_begin + a.kb_per_split) - kb_begin;
+                const int nkb = a.nkb;
                 const int m0 = tr.bx * kBM, n0 = tr.by * a.BN;
                 const int PQ = a.PQ, Q = a.Q;
                 const int img = m0 / PQ, rem = m0 - img * PQ;
@@ -1215,8 +1388,7 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
                 const int cpt = a.Cp / kBK, S = a.S, dw = a.dw, dh = a.dh, a_tiled = a.a_tiled;
                 const uint32_t tx_bytes = (uint32_t)kATileBytes + a.b_stage_bytes;
                 // filter tap (r, s2) and channel chunk of the k-block, carried along
-                int tap = kb_begin / cpt, chunk = kb_begin - tap * cpt;
-                int r = tap / S, s2 = tap - r * S;
+                int chunk = 0, r = 0, s2 = 0;
                 if (prod == 0) PB_PT((t - blockIdx.x) / gridDim.x, 4);
                 for (int kb = 0; kb < nkb; ++kb) {
                     const bool mine_a = (mask_a >> st) & 1u, mine_b = (mask_b >> st) & 1u;
@@ -1233,7 +1405,7 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
                             else tma_load_im2col_4d(a_tile, tmap_x, chunk * kBK, w0, h0, img, (uint16_t)(s2 * dw), (uint16_t)(r * dh), bar);
                             PB_PK(kb, 1);
                         }
-                        if (mine_b) { tma_load_2d(a_tile + kATileBytes, tmap_w, (kb_begin + kb) * kBK, n0, bar); PB_PK(kb, 3); }
+                        if (mine_b) { tma_load_2d(a_tile + kATileBytes, tmap_w, kb * kBK, n0, bar); PB_PK(kb, 3); }
                     }
                     if (++chunk == cpt) {
                         chunk = 0;
@@ -1318,27 +1490,13 @@ bool use_tma_a() {
     return v;
 }
 
-// Widest output-channel tile of the TMA kernel.  A tile of N channels re-reads operand A once per tile,
-// so wide tiles cut the bytes an SM pulls; they also take 2 x 48 KB of pipeline and 256 TMEM columns
-// (two CTAs per SM instead of three) and halve the CTAs of a launch.  Measured (GPU us per request, 1 / 32 /
-// 64 requests in flight, one image per launch): Inception-v3 696 / 46.0 / 43.4 at 128 against 750 / 46.3 / 40.3 at
-// 256; ResNet-50 583 / 39.0 / 34.9 against 737 / 43.1 / 37.5; with 8 images per launch (gangs) and 96 requests in
-// flight 256 gives +3.7 % requests/s.  So the width follows the launch: 128 for a lone image, 256 for launches of at
-// least PB_CONV_WIDE_MIN_BATCH images (default 2: under Poisson arrivals near capacity, where gangs average 3-4
-// requests, the mix met its latency bound at 290k offered requests/s with 2 and not with 4; 0 = never wide).
-// PB_CONV_MAX_BN=128 / 256 fixes the width for every launch.
-int bn_limit(const pb_op_params* p) {
+// Widest output-channel tile: 256 (PB_CONV_MAX_BN=128 caps it; the gather kernel takes 128).
+int bn_limit() {
     static const int fixed = [] {
         const char* e = getenv("PB_CONV_MAX_BN");
-        return e ? (atoi(e) >= 256 ? 256 : 128) : 0;
+        return e && atoi(e) < 256 ? 128 : 256;
     }();
-    static const int wide_from = [] {
-        const char* e = getenv("PB_CONV_WIDE_MIN_BATCH");
-        return e ? atoi(e) : 2;
-    }();
-    if (!use_tma_a()) return 128;
-    if (fixed) return fixed;
-    return (wide_from > 0 && (p->batch > 1 ? p->batch : 1) >= wide_from) ? 256 : 128;
+    return use_tma_a() ? fixed : 128;
 }
 
 // PB_CONV_PERSIST=1: model launches run the persistent kernel (a CTA walks several tiles).  Off by default.
@@ -1358,14 +1516,8 @@ int tiles_per_cta() {
     return n < 1 ? 1 : (n > 64 ? 64 : n);
 }
 
-// A split of the reduction must save at least this much (us) of a lone launch's modelled time.
-// Measured on Inception-v3 (us per request alone / GPU time per request with 32 / 64 in flight):
-// threshold 0 -> 727 / 52.7 / 52.6, 0.5 -> 709 / 46.8 / 45.0, 2 -> 706 / 45.7 / 43.3, never split ->
-// 721 / 45.4 / 42.0: the partial tiles cost load bandwidth that a busy GPU does not have to spare.
-// On the serving mix (MNIST : Inception-v3 = 9 : 1, 48 Inception requests in flight): 2 -> 224k req/s,
-// 6 -> 229k, never -> 230k.  At 6 only the reductions that gain most still split (the 448 -> 384 3x3
-// convolutions on 8x8 maps of Inception-v3, the 512-channel 3x3 ones of a ResNet's last stage).
-// PB_CONV_SPLIT_GAIN_US or pb_set_conv_split_gain_us() overrides it (a large value disables splitting).
+// How reluctant a launch is to split its reduction, in the unit of pb_set_conv_split_gain_us (see choose_tiling, which asks
+// for a 60th of it; above 1e6 nothing splits).  PB_CONV_SPLIT_GAIN_US or the function override the default of 6.
 std::atomic<double> g_split_gain_us{-1.0};      // < 0: not set yet, take PB_CONV_SPLIT_GAIN_US or the default
 double split_gain_us() {
     double v = g_split_gain_us.load(std::memory_order_relaxed);
@@ -1385,65 +1537,114 @@ int dil_w(const pb_op_params* p) { return p->dil_w > 1 ? p->dil_w : 1; }
 struct Geometry {
     int cpt, Cp;                // 64-channel k-blocks per filter tap; Cp = cpt * 64
     int Kdim_pad, nkb;          // k = tap * Cp + c
-    int Kp16, n_tiles, BN, Kout_pad;
+    int Kp16, n_tiles, BN;
     int m_tiles;
-    int stages;                 // 4, 6 or 8
-    int splits, kb_per_split;   // split-K factor the kernel uses when scratch memory is supplied
-    uint64_t scratch_bytes;     // counters + partial tiles for that factor
+    int stages;                 // pipeline buffers
+    int splits;                 // blocks (one cluster) per tile when the caller allows a split
+    int out_box;                // ConvArgs::out_box
+    uint64_t scratch_bytes;     // what the caller has to supply for that
     uint32_t tmem_cols, b_stage_bytes, smem_bytes, idesc;
 };
 
-Geometry geometry(const pb_op_params* p, int bn_max = 0) {
+// Rows of the packed weight matrix: the layout does not depend on how a launch tiles it (a box that reaches past
+// the last row reads zeros).
+int packed_rows(const pb_op_params* p) {
+    const int Kp16 = round_up(p->K, 16), n = ceil_div(Kp16, 128);
+    return n * round_up(ceil_div(Kp16, n), 16);
+}
+
+struct Tiling { int BN, splits; };
+
+// Modelled microseconds of a lone launch inside a stage graph, fitted to 474 measured (layer shape, tile width, split)
+// combinations on B200 - chains of equal layers of 7x7 to 56x56 maps, 64 to 2048 channels, 1x1 and 3x3, 1 to 8 images:
+//   a launch costs 1.6 us outside its k-loop (operand latency, accumulator drain, hand-over to the next launch);
+//   a k-block costs the issue of its copies (0.18 us + 0.8 ns per column) or its bytes at 113 KB/us per SM, shared by
+//   the blocks of the SM;
+//   the epilogue costs 16 ns per column of a block;
+//   a cluster costs its two barriers and the parked tile, and 5 / 8 / 16 ns of placement per block at 2 / 4 / 8 ranks.
+// The tile it picks is within 4 % of the best measured one on average (worst 22 %).
+int tiling_ctas(int m_tiles, int Kp16, const Tiling& t) { return m_tiles * ceil_div(Kp16, t.BN) * t.splits; }
+double tiling_us(int ctas, int nkb, const Tiling& t) {
+    const double per_sm = std::max(1.0, ctas / 148.0);
+    const double kb = std::max(0.183 + 0.00084 * t.BN, per_sm * (16.384 + 0.128 * t.BN) / 113.0);
+    double us = 1.59 + 0.0162 * t.BN / t.splits * (1.0 + 0.56 * (per_sm - 1.0)) + ceil_div(nkb, t.splits) * kb;
+    if (t.splits > 1) us += 0.06 + 0.0174 * t.BN + ctas * (t.splits == 2 ? 0.0048 : t.splits == 4 ? 0.0079 : 0.0164);
+    return us;
+}
+
+// Tile width (output channels) and split of a launch of m_tiles x 128 rows: the combination with the least modelled
+// time, plus a charge for the block slots it takes (444 = 148 SMs x 3): on a GPU that other requests share, what counts is
+// not when a launch ends but what it occupies.  Measured, charge -> 192 requests of MNIST : Inception-v3 = 9 : 1 in flight /
+// 32 of ResNet-18: 0 -> 1893 / 2478 us, 4 -> 1448 / 1581, 8 -> 1337 / 1624, 12 -> 1313 / 1651, 20 -> 1334 / 1727; alone,
+// Inception-v3 / 8 images of ResNet-50: 0 -> 343 / 446 us, 0.5 -> 343 / 438, 5 -> 352 / 481, 20 -> 393 / 556.
+Tiling choose_tiling(int m_tiles, int Kp16, int nkb, int bn_max, int want_splits, double gain_us, bool shared) {
+    const double charge = shared ? 8.0 : 0.5;
+    Tiling best{0, 1};
+    double best_us = 1e30;
+    for (int S = 1; S <= 8; S *= 2) {
+        if (want_splits > 0 ? S != want_splits : (S > 1 && nkb < 2 * S)) continue;
+        const int widest = S > 1 ? std::min(bn_max, 128) : bn_max;
+        for (int n = ceil_div(Kp16, widest); n <= ceil_div(Kp16, 32); ++n) {
+            const Tiling t{round_up(ceil_div(Kp16, n), std::max(16, 8 * S)), S};
+            if (t.BN > widest) continue;
+            const int ctas = tiling_ctas(m_tiles, Kp16, t);
+            double us = tiling_us(ctas, nkb, t) + (S > 1 ? gain_us / 60.0 : 0.0);
+            us += charge * ctas * (1.5 + ceil_div(nkb, S) * 0.2) / 444.0;
+            if (us < best_us - 1e-9) { best_us = us; best = t; }
+        }
+    }
+    return best;
+}
+
+Geometry geometry(const pb_op_params* p, bool allow_split) {
     Geometry g;
-    if (bn_max <= 0) bn_max = bn_limit(p);
     g.cpt = ceil_div(p->Cs, kBK);
     g.Cp = g.cpt * kBK;
     g.nkb = p->R * p->S * g.cpt;
     g.Kdim_pad = g.nkb * kBK;
     g.Kp16 = round_up(p->K, 16);
-    g.n_tiles = ceil_div(g.Kp16, bn_max);
-    g.BN = round_up(ceil_div(g.Kp16, g.n_tiles), 16);
-    g.Kout_pad = g.n_tiles * g.BN;
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM);
+    const double gain = split_gain_us();
+    const int want = p->reserved & kTileSplitMask;       // a grouped launch has one cluster size for all its convolutions (0: not decided)
+    const bool shared = (p->reserved & kTileShared) != 0;
+    Tiling t = choose_tiling(g.m_tiles, g.Kp16, g.nkb, bn_limit(), !use_tma_a() || gain > 1e6 ? 1 : want, gain, shared);
+    g.scratch_bytes = t.splits > 1 ? kSplitScratchBytes : 0;
+    if (t.splits > 1 && !allow_split) t = choose_tiling(g.m_tiles, g.Kp16, g.nkb, bn_limit(), 1, gain, shared);
+    g.BN = t.BN;
+    g.splits = t.splits;
+    g.n_tiles = ceil_div(g.Kp16, g.BN);
     g.tmem_cols = 32;
     while ((int)g.tmem_cols < g.BN) g.tmem_cols <<= 1;
     g.b_stage_bytes = (uint32_t)g.BN * 128u;
-    // Split the reduction over blockIdx.z when that shortens the launch.  Cost model fitted to phase
-    // timings on B200 (microseconds): a k-block costs 0.2 + 0.001*BN in the main loop; a split launch
-    // pays 1.5 for parking the partial tiles plus 0.0088*BN per partial tile the last CTA adds up.
-    const int tiles = g.m_tiles * g.n_tiles;
-    const double per_kb = 0.2 + 0.001 * g.BN, per_partial = 0.0088 * g.BN;
-    int want = 1;
-    double best = g.nkb * per_kb;
-    for (int sp = 2; sp <= 16 && tiles * sp <= 296 && sp * 4 <= g.nkb; ++sp) {
-        const double t = ceil_div(g.nkb, sp) * per_kb + 1.5 + sp * per_partial;
-        if (t < best - split_gain_us()) { best = t; want = sp; }
-    }
-    g.kb_per_split = ceil_div(g.nkb, want);
-    g.splits = ceil_div(g.nkb, g.kb_per_split);
-    g.scratch_bytes = g.splits > 1 ? (uint64_t)kCounterBytes + (uint64_t)tiles * g.splits * kBM * g.BN * 4ull : 0;
-    if ((uint64_t)tiles * 4 > kCounterBytes) { g.splits = 1; g.kb_per_split = g.nkb; g.scratch_bytes = 0; }
-    // Pipeline depth: as many stages as the k-loop can use and the shared-memory budget holds.
+    // Pipeline depth: as many stages as the k-loop can use and the shared-memory budget holds.  On a GPU it has to itself a
+    // launch of up to two blocks per SM gets a deeper pipeline (a refill takes about 1.1 us; 36 k-blocks of 64 columns: 13.6 us
+    // at 73 KB, 12.3 at 110, 11.7 at 150, where the next launch's blocks no longer fit beside it: Inception-v3 402 us
+    // instead of 346).
     const uint32_t stage_bytes = (uint32_t)kATileBytes + g.b_stage_bytes;
-    const uint32_t budget = use_tma_a() ? kSmemBudgetTma : kSmemBudget;
-    static const int kDepths[] = {8, 6, 4, 3, 2};
-    g.stages = 2;
-    for (int d : kDepths) {
-        if (!use_tma_a() && d < 4) break;                       // the gather kernel exists for 4, 6, 8
-        if ((uint32_t)d * stage_bytes + 1024u <= budget && d <= g.kb_per_split + 1) { g.stages = d; break; }
-        if (d == (use_tma_a() ? 2 : 4)) g.stages = d;
+    const bool deep = !shared && g.m_tiles * g.n_tiles * g.splits <= 296;
+    const uint32_t budget = !use_tma_a() ? kSmemBudget : (deep ? kSmemBudgetDeep : kSmemBudgetTma);
+    if (use_tma_a()) {
+        g.stages = (int)std::min<uint32_t>({(uint32_t)kMaxStages, (budget - 1024u) / stage_bytes, (uint32_t)ceil_div(g.nkb, g.splits)});
+        if (g.stages < 2) g.stages = 2;
+    } else {
+        static const int kDepths[] = {8, 6, 4};                     // the gather kernel exists for 4, 6, 8
+        g.stages = 4;
+        for (int d : kDepths)
+            if ((uint32_t)d * stage_bytes + 1024u <= budget && d <= g.nkb + 1) { g.stages = d; break; }
     }
-    g.smem_bytes = (uint32_t)g.stages * stage_bytes + 1024u;
+    // Stores through TMA where blocks share an SM's store path; a block alone on its SM is 0.2 us faster with direct ones
+    // (measured: up to 148 blocks or up to 48 columns direct stores win, above both TMA ones do, by up to 3 us a launch).
+    g.out_box = 0;
+    if (g.splits == 1 && g.BN >= 64 && g.BN % 32 == 0 && (shared || g.m_tiles * g.n_tiles > 148)) g.out_box = g.BN % 64 == 0 ? 64 : 32;
+    const uint32_t exchange = g.splits > 1 ? (uint32_t)g.BN * 512u : 0u;      // a rank's partial tile
+    g.smem_bytes = std::max((uint32_t)g.stages * stage_bytes, exchange) + 1024u;
     // c_format f32 (1 << 4), a/b format bf16 (1 << 7, 1 << 10), K-major both, N >> 3 at bit 17, M >> 4 at bit 24
     g.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
     return g;
 }
-
-// Without (enough) scratch memory the kernel runs the whole reduction in one CTA per tile.
-void drop_split(Geometry* g) {
-    g->splits = 1;
-    g->kb_per_split = g->nkb;
-}
+// The split is the caller's to allow: by the scratch memory that pb_launch_info.scratch_bytes asks for.
+bool split_allowed(const pb_op_params* p) { return p->scratch != nullptr && p->scratch_bytes >= kSplitScratchBytes; }
+Geometry geometry(const pb_op_params* p) { return geometry(p, split_allowed(p)); }
 
 const void* kernel_for(int stages, bool tma) {
     if (tma) return (const void*)conv_umma_tma_kernel;
@@ -1475,12 +1676,9 @@ cudaError_t raise_smem_limits() {
 }  // namespace
 
 struct ConvUmmaPlan {
-    CUtensorMap tmap;        // weights [Kout_pad][Kdim_pad], boxes of g.BN rows (the width a launch of one image uses)
-    CUtensorMap tmap_wide;   // the same weights in boxes of BN_wide rows (launches of a gang)
-    Geometry g;
-    int BN_wide;             // = g.BN when the layer has one column tile either way
+    const void* w_dev;       // packed weights [rows][Kdim_pad]
+    int rows, Kdim_pad;
     int device;
-    const CUtensorMap* map_for(int BN) const { return BN == g.BN ? &tmap : (BN == BN_wide ? &tmap_wide : nullptr); }
 };
 
 #ifdef PB_CONV_STATS
@@ -1520,10 +1718,9 @@ bool conv_umma_supported(const pb_op_params* p) {
 
 int conv_umma_info(const pb_op_params* p, pb_launch_info* out) {
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
-    Geometry g = geometry(p);
+    const Geometry g = geometry(p);
     memset(out, 0, sizeof(*out));
-    out->scratch_bytes = g.scratch_bytes;       // what a split launch needs
-    if (g.splits > 1 && (p->scratch == nullptr || p->scratch_bytes < g.scratch_bytes)) drop_split(&g);
+    out->scratch_bytes = g.scratch_bytes;       // what a split launch asks for
     out->kind = PB_STAGE_CONV_UMMA;
     out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
     out->threads_per_block = use_tma_a() ? kThreadsTma : kThreads;
@@ -1548,10 +1745,8 @@ int conv_umma_info(const pb_op_params* p, pb_launch_info* out) {
 
 int64_t conv_umma_pack_weights(const pb_op_params* p, const float* w, void* dst) {
     if (!conv_umma_supported(p)) { set_error("conv_umma: unsupported convolution"); return PB_ERR_INVALID; }
-    pb_op_params one = *p;      // the layout does not depend on how many images a launch will carry
-    one.batch = 1;
-    const Geometry g = geometry(&one);
-    const size_t n = (size_t)g.Kout_pad * g.Kdim_pad;
+    const Geometry g = geometry(p);
+    const size_t n = (size_t)packed_rows(p) * g.Kdim_pad;
     if (dst) {
         memset(dst, 0, n * 2);
         for (int k = 0; k < p->K; ++k)
@@ -1564,13 +1759,15 @@ int64_t conv_umma_pack_weights(const pb_op_params* p, const float* w, void* dst)
     return (int64_t)(n * 2);
 }
 
-static int make_tmap(const Geometry& g, const void* w_dev, CUtensorMap* out) {
+// Weight map of a launch with tiles of BN output channels.
+static int make_tmap(const ConvUmmaPlan* plan, int BN, CUtensorMap* out) {
+    const void* w_dev = plan->w_dev;
     EncodeTiledFn enc = encode_fn();
     PB_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
     PB_REQUIRE(((uintptr_t)w_dev & 15) == 0, "conv_umma: packed weights must be 16-byte aligned");
-    const cuuint64_t dims[2] = {(cuuint64_t)g.Kdim_pad, (cuuint64_t)g.Kout_pad};
-    const cuuint64_t strides[1] = {(cuuint64_t)g.Kdim_pad * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)g.BN};
+    const cuuint64_t dims[2] = {(cuuint64_t)plan->Kdim_pad, (cuuint64_t)plan->rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)plan->Kdim_pad * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)BN};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w_dev), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1628,6 +1825,27 @@ static int make_xmap(const pb_op_params* p, CUtensorMap* out) {
     return PB_OK;
 }
 
+
+// Output map: [pixels of all images][channels of the slice], boxes of 32 rows.
+static int make_ymap(const pb_op_params* p, int U, CUtensorMap* out) {
+    if (!U) { memset(out, 0, sizeof(*out)); return PB_OK; }
+    EncodeTiledFn enc = encode_fn();
+    PB_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
+    PB_REQUIRE(((uintptr_t)p->y & 15) == 0, "conv_umma: the output must be 16-byte aligned");
+    const cuuint64_t dims[2] = {(cuuint64_t)p->K, (cuuint64_t)batch_of(p) * p->P * p->Q};
+    const cuuint64_t strides[1] = {(cuuint64_t)p->Ks * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)U, 32};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUtensorMapSwizzle sw = U == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, static_cast<__nv_bfloat16*>(p->y) + p->out_c_off, dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled (output) failed with CUresult %d (K %d, stride %d)", (int)r, p->K, p->Ks);
+        return PB_ERR_CUDA;
+    }
+    return PB_OK;
+}
+
 struct alignas(64) ConvUmmaXMap {
     CUtensorMap map;
 };
@@ -1645,22 +1863,12 @@ void conv_umma_xmap_destroy(ConvUmmaXMap* m) { delete m; }
 
 int conv_umma_plan_create(const pb_op_params* p, const void* w_dev, ConvUmmaPlan** out) {
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
+    PB_REQUIRE(((uintptr_t)w_dev & 15) == 0, "conv_umma: packed weights must be 16-byte aligned");
     ConvUmmaPlan* plan = new ConvUmmaPlan();
-    pb_op_params one = *p;
-    one.batch = 1;
-    plan->g = geometry(&one);
+    plan->w_dev = w_dev;
+    plan->rows = packed_rows(p);
+    plan->Kdim_pad = p->R * p->S * ceil_div(p->Cs, kBK) * kBK;
     cudaGetDevice(&plan->device);
-    int rc = make_tmap(plan->g, w_dev, &plan->tmap);
-    if (rc != PB_OK) { delete plan; return rc; }
-    // The weights were packed for plan->g (rows padded to its column tiles); a wider tiling needs at most as many rows.
-    const Geometry gw = geometry(&one, 256);
-    plan->BN_wide = gw.BN;
-    plan->tmap_wide = plan->tmap;
-    if (gw.BN != plan->g.BN) {
-        if (gw.Kout_pad > plan->g.Kout_pad) { delete plan; set_error("conv_umma: wide tiling needs more weight rows than were packed"); return PB_ERR_INVALID; }
-        rc = make_tmap(gw, w_dev, &plan->tmap_wide);
-        if (rc != PB_OK) { delete plan; return rc; }
-    }
     // The shared-memory limit is a per-device function attribute: raise it once on every device used.
     static std::once_flag once[16];
     static cudaError_t attr_errs[16] = {};
@@ -1680,7 +1888,7 @@ int conv_umma_plan_create(const pb_op_params* p, const void* w_dev, ConvUmmaPlan
 
 void conv_umma_plan_destroy(ConvUmmaPlan* plan) { delete plan; }
 
-// Kernel arguments of one convolution; `g` may have had its split dropped for lack of scratch.
+// Kernel arguments of one convolution.
 static int fill_args(const ConvUmmaPlan* plan, const Geometry& g, const pb_op_params* p, uint32_t* err_flag, ConvArgs* out) {
     ConvArgs& a = *out;
     memset(&a, 0, sizeof(a));
@@ -1697,31 +1905,37 @@ static int fill_args(const ConvUmmaPlan* plan, const Geometry& g, const pb_op_pa
     a.act = p->act; a.a_tiled = pointwise(p) ? 1 : 0; a.nkb = g.nkb; a.taps = p->R * p->S; a.Cp = g.Cp; a.BN = g.BN; a.idesc = g.idesc; a.tmem_cols = g.tmem_cols;
     a.b_stage_bytes = g.b_stage_bytes;
     a.splits = g.splits;
-    a.kb_per_split = g.kb_per_split;
-    a.counters = g.splits > 1 ? static_cast<unsigned*>(p->scratch) : nullptr;
-    a.ws = g.splits > 1 ? reinterpret_cast<float*>(static_cast<char*>(p->scratch) + kCounterBytes) : nullptr;
+    a.out_box = g.out_box;
     return PB_OK;
 }
 
 template <typename... Args>
-static cudaError_t launch_pdl(void (*kern)(Args...), dim3 grid, uint32_t smem, cudaStream_t st, bool pdl, Args... args) {
+static cudaError_t launch_pdl(void (*kern)(Args...), dim3 grid, dim3 cluster, uint32_t smem, cudaStream_t st, bool pdl, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreadsTma);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster.x * cluster.y * cluster.z > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster.x;
+        attr[n].val.clusterDim.y = cluster.y;
+        attr[n++].val.clusterDim.z = cluster.z;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap, const pb_op_params* p, cudaStream_t st,
                              uint32_t job_id, void* notifier, uint32_t* err_flag, bool pdl) {
-    Geometry g = geometry(p);       // the plan's own geometry is that of one image; tiles and split follow the batch
-    if (g.splits > 1 && (p->scratch == nullptr || p->scratch_bytes < g.scratch_bytes)) drop_split(&g);
+    const Geometry g = geometry(p);
     if (!use_tma_a()) PB_REQUIRE(batch_of(p) == 1, "conv_umma: the cp.async gather kernel (PB_CONV_GATHER=1) runs one image per launch");
     ConvArgs a;
     const int frc = fill_args(plan, g, p, err_flag, &a);
@@ -1735,16 +1949,22 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
             if (rc != PB_OK) return rc;
             xmap = &local;
         }
-        const CUtensorMap* wmap = plan->map_for(g.BN);
-        PB_REQUIRE(wmap != nullptr, "conv_umma: no weight map for a tile of %d channels", g.BN);
-        const cudaError_t e = launch_pdl(conv_umma_tma_kernel, grid, g.smem_bytes, st, pdl, *wmap, xmap->map, a, g.stages, job_id, nf);
+        CUtensorMap wmap, ymap;
+        int mrc = make_tmap(plan, g.BN, &wmap);
+        if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, &ymap);
+        if (mrc != PB_OK) return mrc;
+        const cudaError_t e = launch_pdl(conv_umma_tma_kernel, grid, dim3(1, 1, (unsigned)g.splits), g.smem_bytes, st, pdl, wmap, xmap->map, ymap, a,
+                                         g.stages, job_id, nf);
         if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_tma_kernel", __FILE__, __LINE__);
         return PB_OK;
     } else {
+        CUtensorMap wmap;
+        const int wrc = make_tmap(plan, g.BN, &wmap);
+        if (wrc != PB_OK) return wrc;
         switch (g.stages) {
-            case 4: conv_umma_gather_kernel<4><<<grid, kThreads, g.smem_bytes, st>>>(plan->tmap, a, job_id, nf); break;
-            case 6: conv_umma_gather_kernel<6><<<grid, kThreads, g.smem_bytes, st>>>(plan->tmap, a, job_id, nf); break;
-            default: conv_umma_gather_kernel<8><<<grid, kThreads, g.smem_bytes, st>>>(plan->tmap, a, job_id, nf); break;
+            case 4: conv_umma_gather_kernel<4><<<grid, kThreads, g.smem_bytes, st>>>(wmap, a, job_id, nf); break;
+            case 6: conv_umma_gather_kernel<6><<<grid, kThreads, g.smem_bytes, st>>>(wmap, a, job_id, nf); break;
+            default: conv_umma_gather_kernel<8><<<grid, kThreads, g.smem_bytes, st>>>(wmap, a, job_id, nf); break;
         }
     }
     return launch_check("conv_umma");
@@ -1757,6 +1977,7 @@ struct ConvUmmaMulti {
     unsigned total_blocks = 0;      // tiles of all sub-problems (= CTAs of the one-tile-per-CTA kernel)
     uint32_t smem = 0;
     uint32_t tmem_cols = 0;
+    unsigned splits = 1;            // cluster size of the launch
     bool has_pool = false;          // pooling layers ride along (one-tile kernel only)
     // persistent kernel
     bool persist = false;
@@ -1766,6 +1987,34 @@ struct ConvUmmaMulti {
 };
 
 bool conv_umma_multi_available() { return use_tma_a(); }
+
+// The cluster size of a grouped launch is one for all its convolutions: the one whose slowest member is modelled fastest.
+int conv_umma_common_splits(const pb_op_params* const* params, int n) {
+    const double gain = split_gain_us();
+    if (!use_tma_a() || persist_enabled() || gain > 1e6) return 1;
+    int best = 1;
+    double best_us = 1e30;
+    for (int S = 1; S <= 8; S *= 2) {
+        std::vector<Tiling> t((size_t)n);
+        std::vector<int> nkb((size_t)n);
+        int ctas = 0, longest = 0;
+        for (int i = 0; i < n; ++i) {
+            const pb_op_params* p = params[i];
+            const int m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM), Kp16 = round_up(p->K, 16);
+            nkb[(size_t)i] = p->R * p->S * ceil_div(p->Cs, kBK);
+            longest = std::max(longest, nkb[(size_t)i]);
+            t[(size_t)i] = choose_tiling(m_tiles, Kp16, nkb[(size_t)i], bn_limit(), S, gain, (p->reserved & kTileShared) != 0);
+            ctas += tiling_ctas(m_tiles, Kp16, t[(size_t)i]);
+        }
+        if (S > 1 && longest < 2 * S) break;
+        double us = 0;
+        for (int i = 0; i < n; ++i) us = std::max(us, tiling_us(ctas, nkb[(size_t)i], t[(size_t)i]));
+        if (S > 1) us += gain / 60.0;
+        if (us < best_us) { best_us = us; best = S; }
+    }
+    return best;
+}
+
 bool conv_umma_persist_enabled() { return persist_enabled(); }
 uint32_t conv_umma_persist_grid(uint32_t total_tiles) {
     const uint32_t g = ceil_div<uint32_t>(total_tiles, (uint32_t)tiles_per_cta());
@@ -1790,34 +2039,22 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
     memset(table.data(), 0, sizeof(SubConv) * (size_t)n);
     ConvUmmaMulti* m = new ConvUmmaMulti();
     m->n = n;
+    auto is_pool = [&](int i) { return kinds && kinds[i] != PB_STAGE_CONV_UMMA; };
+    // the convolutions first: with clusters their blocks have to start on a cluster boundary
+    int at = 0;
     for (int i = 0; i < n; ++i) {
-        if (kinds && kinds[i] != PB_STAGE_CONV_UMMA) {
-            const pb_op_params* p = params[i];
-            if (!p || !conv_umma_pool_fusable(kinds[i], p)) { delete m; set_error("conv_umma_multi_create: entry %d cannot ride along", i); return PB_ERR_INVALID; }
-            SubConv& sc = table[(size_t)i];
-            PoolSubArgs& a = sc.pool;
-            a.x = static_cast<const __nv_bfloat16*>(p->x);
-            a.y = static_cast<__nv_bfloat16*>(p->y);
-            a.C = p->C; a.H = p->H; a.W = p->W; a.Cs = p->Cs; a.P = p->P; a.Q = p->Q; a.Ks = p->Ks; a.out_c_off = p->out_c_off;
-            a.sh = p->stride_h; a.sw = p->stride_w; a.ph = p->pad_h; a.pw = p->pad_w;
-            a.is_max = kinds[i] == PB_STAGE_MAXPOOL; a.count_pad = p->flags & 1; a.batch = batch_of(p);
-            sc.first_block = m->total_blocks;
-            sc.gx = sc.gy = 1;
-            sc.stages = kSubPool;
-            m->total_blocks += conv_umma_pool_blocks(p);
-            m->has_pool = true;
-            continue;
-        }
+        if (is_pool(i)) continue;
         PB_REQUIRE(plans[i] && xmaps[i] && params[i], "conv_umma_multi_create: NULL entry %d", i);
-        Geometry g = geometry(params[i]);
-        if (g.splits > 1 && (params[i]->scratch == nullptr || params[i]->scratch_bytes < g.scratch_bytes)) drop_split(&g);
-        SubConv& sc = table[(size_t)i];
-        const CUtensorMap* wmap = plans[i]->map_for(g.BN);
-        if (!wmap) { delete m; set_error("conv_umma_multi_create: no weight map for a tile of %d channels", g.BN); return PB_ERR_INVALID; }
-        sc.tmap_w = *wmap;
-        sc.tmap_x = xmaps[i]->map;
-        const int rc = fill_args(plans[i], g, params[i], nullptr, &sc.a);
+        const Geometry g = geometry(params[i], split_allowed(params[i]) && !persist_enabled());
+        SubConv& sc = table[(size_t)at++];
+        int rc = make_tmap(plans[i], g.BN, &sc.tmap_w);
+        if (rc == PB_OK) rc = make_ymap(params[i], g.out_box, &sc.tmap_y);
         if (rc != PB_OK) { delete m; return rc; }
+        sc.tmap_x = xmaps[i]->map;
+        rc = fill_args(plans[i], g, params[i], nullptr, &sc.a);
+        if (rc != PB_OK) { delete m; return rc; }
+        if (at > 1 && (unsigned)g.splits != m->splits) { delete m; set_error("conv_umma_multi_create: the entries of a launch must share one split"); return PB_ERR_INVALID; }
+        m->splits = (unsigned)g.splits;
         sc.first_block = m->total_blocks;
         sc.gx = (uint32_t)g.m_tiles;
         sc.gy = (uint32_t)g.n_tiles;
@@ -1827,6 +2064,24 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
         m->tmem_cols = std::max(m->tmem_cols, g.tmem_cols);
         m->stage_bytes = std::max(m->stage_bytes, (uint32_t)kATileBytes + g.b_stage_bytes);
     }
+    for (int i = 0; i < n; ++i) {
+        if (!is_pool(i)) continue;
+        const pb_op_params* p = params[i];
+        if (!p || !conv_umma_pool_fusable(kinds[i], p)) { delete m; set_error("conv_umma_multi_create: entry %d cannot ride along", i); return PB_ERR_INVALID; }
+        SubConv& sc = table[(size_t)at++];
+        PoolSubArgs& a = sc.pool;
+        a.x = static_cast<const __nv_bfloat16*>(p->x);
+        a.y = static_cast<__nv_bfloat16*>(p->y);
+        a.C = p->C; a.H = p->H; a.W = p->W; a.Cs = p->Cs; a.P = p->P; a.Q = p->Q; a.Ks = p->Ks; a.out_c_off = p->out_c_off;
+        a.sh = p->stride_h; a.sw = p->stride_w; a.ph = p->pad_h; a.pw = p->pad_w;
+        a.is_max = kinds[i] == PB_STAGE_MAXPOOL; a.count_pad = p->flags & 1; a.batch = batch_of(p);
+        sc.first_block = m->total_blocks;
+        sc.gx = sc.gy = 1;
+        sc.stages = kSubPool;
+        m->total_blocks += conv_umma_pool_blocks(p);
+        m->has_pool = true;
+    }
+    m->total_blocks = round_up(m->total_blocks, m->splits);      // blocks past the last pooling vector find nothing to do
     if (m->stage_bytes == 0) { delete m; set_error("conv_umma_multi_create: no convolution among the entries"); return PB_ERR_INVALID; }
     // persistent kernel: one pipeline for every sub-problem (stages of the widest), two accumulators
     m->stages = (int)std::min<uint32_t>(kMaxStages, (kSmemBudgetPersist - 1024u) / m->stage_bytes);
@@ -1890,8 +2145,8 @@ int conv_umma_multi_launch(const ConvUmmaMulti* m, cudaStream_t st, uint32_t job
         if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_persist_kernel", __FILE__, __LINE__);
         return PB_OK;
     }
-    const cudaError_t e = launch_pdl(conv_umma_multi_kernel, dim3(m->total_blocks), m->smem, st, pdl, (const SubConv*)m->table_dev, m->n,
-                                     job_id, static_cast<FinishedBlockNotifier*>(notifier));
+    const cudaError_t e = launch_pdl(conv_umma_multi_kernel, dim3(m->total_blocks), dim3(m->splits), m->smem, st, pdl,
+                                     (const SubConv*)m->table_dev, m->n, job_id, static_cast<FinishedBlockNotifier*>(notifier));
     if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_multi_kernel", __FILE__, __LINE__);
     return PB_OK;
 }
@@ -1976,16 +2231,11 @@ int conv_umma_time(const pb_op_params* p, int mode, int iters, size_t flush_byte
 }
 
 // ---- launch without any allocation -----------------------------------------------------------------
-// Scratch for pb_conv2d_umma_noalloc: split-K tile counters (first kCounterBytes) and partial tiles.
-// It lives in the library image, so every GPU that loads the library holds these bytes until exit.
-constexpr size_t kStaticScratchBytes = PB_NOALLOC_SCRATCH_BYTES;
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kStaticScratchBytes];
 static __device__ uint32_t g_noalloc_err_flag;
 
 namespace {
 struct NoAllocDevice {
     bool ready = false;
-    void* scratch = nullptr;      // device address of g_noalloc_scratch on this device
     uint32_t* err_flag = nullptr;
 };
 NoAllocDevice g_noalloc_dev[16];
@@ -2005,37 +2255,23 @@ int conv_umma_launch_noalloc(const pb_op_params* p, cudaStream_t st, uint32_t jo
     PB_REQUIRE(device >= 0 && device < 16, "pb_conv2d_umma_noalloc: device %d out of range", device);
     NoAllocDevice& nd = g_noalloc_dev[device];
     {
-        // First call on this device: resolve the device addresses of the file-scope arrays.  In host
-        // code their names are only stand-ins, not device addresses; the kernel must be given what
+        // First call on this device: resolve the device address of the file-scope flag.  In host
+        // code its name is only a stand-in, not a device address; the kernel must be given what
         // cudaGetSymbolAddress returns, with this device current.
         std::lock_guard<std::mutex> lk(g_noalloc_mu);
         if (!nd.ready) {
-            void* sp = nullptr;
             void* fp = nullptr;
-            PB_CUDA(cudaGetSymbolAddress(&sp, g_noalloc_scratch));
             PB_CUDA(cudaGetSymbolAddress(&fp, g_noalloc_err_flag));
             PB_CUDA(raise_smem_limits());
-            nd.scratch = sp;
             nd.err_flag = static_cast<uint32_t*>(fp);
             nd.ready = true;
         }
     }
-    ConvUmmaPlan plan;            // on the stack: no host allocation either
-    plan.g = geometry(p);
-    plan.device = device;
-    if (plan.g.scratch_bytes > kStaticScratchBytes) {
-        set_error("pb_conv2d_umma_noalloc: this convolution wants %llu bytes of scratch, the built-in buffer holds %llu "
-                  "(use pb_op_launch with caller-provided scratch instead)",
-                  (unsigned long long)plan.g.scratch_bytes, (unsigned long long)kStaticScratchBytes);
-        return PB_ERR_INVALID;
-    }
-    int rc = make_tmap(plan.g, p->w, &plan.tmap);
-    if (rc != PB_OK) return rc;
+    ConvUmmaPlan plan{p->w, packed_rows(p), p->R * p->S * ceil_div(p->Cs, kBK) * kBK, device};      // on the stack: no host allocation either
     pb_op_params q = *p;
-    q.scratch = plan.g.scratch_bytes ? nd.scratch : nullptr;
-    q.scratch_bytes = plan.g.scratch_bytes ? kStaticScratchBytes : 0;
-    // The buffer keeps whatever the previous call left; only the tile counters have to start at zero.
-    if (plan.g.scratch_bytes) PB_CUDA(cudaMemsetAsync(nd.scratch, 0, kCounterBytes, st));
+    q.reserved = 0;
+    q.scratch = (void*)nd.err_flag;         // never touched: allows the split, whose partial tiles meet in shared memory
+    q.scratch_bytes = kSplitScratchBytes;
     return conv_umma_launch_planned(&plan, nullptr, &q, st, job_id, notifier, nd.err_flag);
 }
 

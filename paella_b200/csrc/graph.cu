@@ -54,7 +54,7 @@ struct Stage {
     std::string name;
     int out_tensor;
     int in_tensor = -1, res_tensor = -1;   // tensors read (-1: the request input / none)
-    size_t scratch_off = 0;                // this stage's private slice of the instance's scratch buffer
+    std::vector<int> peers;                // stages whose tensor-core convolutions share a launch with this one (itself included)
 };
 
 }  // namespace
@@ -67,8 +67,6 @@ struct pb_model {
     std::vector<Stage> stages;
     int t_in = 0, t_out = 0;
     size_t arena_bytes = 0;
-    size_t scratch_bytes = 0;     // sum of the stages' scratch requirements: every split-K layer has its own
-                                  // slice, so kernels of parallel branches never share partial tiles
     size_t in_floats = 0, out_floats = 0;
     bool mnist_fused = false;
     // Stage groups: what the job adapter hands to the scheduler as ONE stage.  A group of several
@@ -78,6 +76,7 @@ struct pb_model {
     struct Group { int first, count; pb_launch_info info; std::vector<std::vector<int>> launches; };
     std::vector<Group> groups;
     bool fuse_branches = false;
+    bool shared = false;        // launches of other requests run beside this model's (pb_model_set_shared_gpu)
     bool persist = false;       // tensor-core launches of the stage graphs run the persistent (multi-tile) kernel
     // fused MNIST weights (device)
     float *w1 = nullptr, *b1 = nullptr, *w2 = nullptr, *b2 = nullptr, *wd = nullptr, *bd = nullptr;
@@ -95,7 +94,6 @@ struct Variant {
     std::vector<pb_launch_info> group_info; // per group, for this batch
     std::vector<cudaGraphExec_t> graphs;    // per group; NULL = single kernel, launched directly
     std::vector<std::vector<pb::ConvUmmaMulti*>> multis;   // [group][launch]: descriptor table of a grouped conv launch
-    char* scratch = nullptr;                // split-K scratch, one private slice per stage that splits at this batch
 };
 
 struct pb_instance {
@@ -197,16 +195,62 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
     return out;
 }
 
-// Splits the stage list into groups of at most PB_STAGE_GROUP kernels (default 48; 1 = one kernel per
-// scheduler stage, the reference's granularity) and derives each group's stage declaration.
-void build_groups(pb_model* m) {
-    int gs = 48;      // measured on the headline mix: 24 -> 221k req/s with the host thread 94 % busy, 48 -> 225k at 79 %
-    if (const char* e = getenv("PB_STAGE_GROUP")) gs = atoi(e);
-    if (gs < 1) gs = 1;
-    // Independent tensor-core convolutions of equal dependence depth share one launch, unless the
-    // graphs are captured with parallel branches (PB_GRAPH_BRANCHES=1) or PB_FUSE_BRANCHES=0.
-    m->fuse_branches = env_flag("PB_FUSE_BRANCHES", true) && !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available();
-    m->persist = !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available() && pb::conv_umma_persist_enabled();
+// pb_op_params.reserved of `stage`: the tiling policy of the model and, when the stage's launch is a grouped one, the
+// cluster size of its convolutions.
+int tile_hint(const pb_model* m, int stage, int nb) {
+    const std::vector<int>& l = m->stages[(size_t)stage].peers;
+    const int policy = m->shared ? pb::kTileShared : 0;
+    if (l.size() < 2) return policy;
+    std::vector<pb_op_params> ps;
+    std::vector<const pb_op_params*> pp;
+    for (int s : l) {
+        ps.push_back(m->stages[(size_t)s].p);
+        ps.back().batch = nb;
+        ps.back().reserved = policy;
+    }
+    for (const pb_op_params& p : ps) pp.push_back(&p);
+    return policy | pb::conv_umma_common_splits(pp.data(), (int)pp.size());
+}
+
+int op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
+    if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_info(p, out);
+    if (kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(out);
+    return pb::simple_op_info(kind, p, out);
+}
+
+// Launch geometry of stage `stage` when one launch carries `nb` images (scratch offered without limit).
+int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out) {
+    const Stage& st = m->stages[(size_t)stage];
+    if (st.kind == PB_STAGE_MNIST_FUSED) {
+        const int rc = pb::mnist_fused_info(out);
+        out->num_blocks *= (uint32_t)nb; out->flops *= (uint64_t)nb; out->bytes *= (uint64_t)nb;
+        return rc;
+    }
+    pb_op_params p = st.p;
+    p.batch = nb;
+    p.scratch = (void*)16;
+    p.scratch_bytes = ~0ull;
+    p.reserved = tile_hint(m, stage, nb);
+    return op_info(st.kind, &p, out);
+}
+
+// Launch geometry of the stages and groups for one image.
+void refresh_infos(pb_model* m) {
+    // a stage of a grouped launch has the geometry it has there
+    for (size_t i = 0; i < m->stages.size(); ++i)
+        if (m->stages[i].kind == PB_STAGE_CONV_UMMA) stage_info_batched(m, (int)i, 1, &m->stages[i].info);
+    for (size_t gi = 0; gi < m->groups.size(); ++gi) {
+        std::vector<pb_launch_info> infos(m->stages.size());
+        for (size_t i = 0; i < m->stages.size(); ++i) infos[i] = m->stages[i].info;
+        m->groups[gi].info = group_footprint(m, (int)gi, infos);
+    }
+}
+
+// Splits the stage list into groups of at most `gs` stages and plans each group's launches.  fuse: independent
+// tensor-core convolutions of equal dependence depth share one launch.  fuse_pools: a 3x3 pooling layer joins the grouped
+// launch of the convolutions of its depth (a launch that contains one always starts with a convolution).
+std::vector<pb_model::Group> plan_groups(const pb_model* m, int gs, bool fuse, bool fuse_pools) {
+    std::vector<pb_model::Group> groups;
     const int n = (int)m->stages.size();
     std::vector<std::vector<int>> writers(m->tensors.size());
     for (int first = 0; first < n; first += gs) {
@@ -228,20 +272,14 @@ void build_groups(pb_model* m) {
         }
         std::vector<int> order((size_t)g.count);
         for (int i = 0; i < g.count; ++i) order[(size_t)i] = first + i;
-        if (m->fuse_branches)
-            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return level[(size_t)(a - first)] < level[(size_t)(b - first)]; });
-        // PB_FUSE_POOLS=1 (off by default; not with the persistent kernel): a 3x3 pooling layer joins the grouped launch of
-        // the convolutions of its depth.  A launch that contains a pooling layer always starts with a convolution.
-        // Measured: same bits, a lone Inception-v3 request 885 -> 870 us, but 26.9k -> 17.4k req/s with 96 requests in
-        // flight: a pooling block then holds a whole convolution slot of its SM (the launch's 73 KB of shared memory) while
-        // it waits on loads, and there are 600-900 of them per launch at 8 images.
-        const bool fuse_pools = m->fuse_branches && !m->persist && env_flag("PB_FUSE_POOLS", false);
+        // the convolutions of a depth side by side, the other layers of that depth after them
+        auto rank = [&](int i) { return 2 * level[(size_t)(i - first)] + (m->stages[i].kind == PB_STAGE_CONV_UMMA ? 0 : 1); };
+        if (fuse) std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rank(a) < rank(b); });
         for (int s : order) {
             const Stage& st = m->stages[s];
             const bool conv_ok = st.kind == PB_STAGE_CONV_UMMA && !st.x_is_input && !st.y_is_output;
             const bool pool_ok = fuse_pools && !st.x_is_input && !st.y_is_output && pb::conv_umma_pool_fusable(st.kind, &st.p);
-            const bool fusable = m->fuse_branches && (conv_ok || pool_ok);
-            if (fusable && !g.launches.empty()) {
+            if (fuse && (conv_ok || pool_ok) && !g.launches.empty()) {
                 std::vector<int>& prev = g.launches.back();
                 const Stage& ps = m->stages[prev.front()];
                 const bool prev_fusable = ps.kind == PB_STAGE_CONV_UMMA && !ps.x_is_input && !ps.y_is_output;
@@ -261,28 +299,33 @@ void build_groups(pb_model* m) {
                 if (m->stages[last[k]].kind != PB_STAGE_CONV_UMMA) { out_again.push_back(last[k]); last.erase(last.begin() + (long)k); }
             for (size_t k = out_again.size(); k-- > 0;) g.launches.push_back(std::vector<int>{out_again[k]});
         }
-        m->groups.push_back(g);
+        groups.push_back(g);
     }
-    for (size_t gi = 0; gi < m->groups.size(); ++gi) {
-        std::vector<pb_launch_info> infos(m->stages.size());
-        for (size_t i = 0; i < m->stages.size(); ++i) infos[i] = m->stages[i].info;
-        m->groups[gi].info = group_footprint(m, (int)gi, infos);
-    }
+    return groups;
 }
 
-// Launch geometry of stage `stage` when one launch carries `nb` images (scratch offered without limit).
-int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out) {
-    const Stage& st = m->stages[(size_t)stage];
-    if (st.kind == PB_STAGE_MNIST_FUSED) {
-        const int rc = pb::mnist_fused_info(out);
-        out->num_blocks *= (uint32_t)nb; out->flops *= (uint64_t)nb; out->bytes *= (uint64_t)nb;
-        return rc;
-    }
-    pb_op_params p = st.p;
-    p.batch = nb;
-    p.scratch = (void*)16;
-    p.scratch_bytes = ~0ull;
-    return pb_op_info(st.kind, &p, out);
+// Plans the model's groups (PB_STAGE_GROUP kernels each, default 48; 1 = one kernel per scheduler stage, the reference's
+// granularity) and derives each group's stage declaration.
+void build_groups(pb_model* m) {
+    const int dflt = 48;      // measured on the headline mix: 24 -> 221k req/s with the host thread 94 % busy, 48 -> 225k at 79 %
+    int gs = dflt;
+    if (const char* e = getenv("PB_STAGE_GROUP")) gs = atoi(e);
+    if (gs < 1) gs = 1;
+    // Independent tensor-core convolutions share launches unless the graphs are captured with parallel branches
+    // (PB_GRAPH_BRANCHES=1) or PB_FUSE_BRANCHES=0.
+    m->fuse_branches = env_flag("PB_FUSE_BRANCHES", true) && !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available();
+    m->persist = !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available() && pb::conv_umma_persist_enabled();
+    // PB_FUSE_POOLS=1: off by default; not with the persistent kernel.  Measured: same bits, a lone Inception-v3 request
+    // 885 -> 870 us, but 26.9k -> 17.4k req/s with 96 requests in flight: a pooling block then holds a whole convolution
+    // slot of its SM (the launch's 73 KB of shared memory) while it waits on loads, and there are 600-900 of them per
+    // launch at 8 images.
+    m->groups = plan_groups(m, gs, m->fuse_branches, m->fuse_branches && !m->persist && env_flag("PB_FUSE_POOLS", false));
+    // The convolutions of one grouped launch share a cluster size.  It is decided on the default plan whatever the
+    // switches say, so that they change the scheduling of the model and not its bits.
+    for (const pb_model::Group& g : plan_groups(m, dflt, true, false))
+        for (const std::vector<int>& l : g.launches)
+            for (int s : l) m->stages[(size_t)s].peers = l;
+    refresh_infos(m);
 }
 
 int launch_stage_with(pb_instance* in, const Variant& v, int stage, const pb_op_params* p, cudaStream_t stream, uint32_t job_id, void* notifier,
@@ -470,12 +513,11 @@ void destroy_variant(Variant* v) {
     for (pb::ConvUmmaXMap* x : v->xmaps) pb::conv_umma_xmap_destroy(x);
     for (cudaGraphExec_t g : v->graphs) if (g) cudaGraphExecDestroy(g);
     for (auto& l : v->multis) for (pb::ConvUmmaMulti* mu : l) pb::conv_umma_multi_destroy(mu);
-    if (v->scratch) cudaFree(v->scratch);
     delete v;
 }
 
 // Builds (once) what the instance needs to run batches of `nb` images: resolved parameters, input
-// descriptors, scratch, grouped-launch tables and one executable graph per stage group.
+// descriptors, grouped-launch tables and one executable graph per stage group.
 int ensure_variant(pb_instance* in, int nb, Variant** out) {
     PB_REQUIRE(in && nb >= 1 && nb <= in->cap, "batch %d does not fit this instance (capacity %d)", nb, in ? in->cap : 0);
     if (in->variants[(size_t)nb - 1]) { *out = in->variants[(size_t)nb - 1]; return PB_OK; }
@@ -484,24 +526,13 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
     Variant* v = new Variant();
     v->nb = nb;
     const size_t cap = (size_t)in->cap;
-    // launch geometry and scratch layout of every stage at this batch
+    // launch geometry of every stage at this batch
     std::vector<pb_launch_info> infos(m->stages.size());
-    std::vector<size_t> scratch_off(m->stages.size(), 0);
-    size_t scratch_bytes = 0;
     for (size_t i = 0; i < m->stages.size(); ++i) {
         const int rc = stage_info_batched(m, (int)i, nb, &infos[i]);
         if (rc != PB_OK) { destroy_variant(v); return rc; }
-        if (infos[i].scratch_bytes) {
-            scratch_off[i] = scratch_bytes;
-            scratch_bytes += pb::round_up((size_t)infos[i].scratch_bytes, (size_t)256);
-        }
     }
     cudaError_t e = cudaSuccess;
-    if (scratch_bytes) {
-        e = cudaMalloc((void**)&v->scratch, scratch_bytes);
-        if (e == cudaSuccess) e = cudaMemset(v->scratch, 0, scratch_bytes);
-        if (e != cudaSuccess) { destroy_variant(v); return pb::cuda_fail(e, "split-K scratch", __FILE__, __LINE__); }
-    }
     v->params.resize(m->stages.size());
     v->xmaps.assign(m->stages.size(), nullptr);
     for (size_t i = 0; i < m->stages.size(); ++i) {
@@ -511,8 +542,9 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
         p.x = st.x_is_input ? (const void*)in->in_dev : (const void*)(in->arena + cap * st.x_off);
         p.y = st.y_is_output ? (void*)in->out_dev : (void*)(in->arena + cap * st.y_off);
         p.residual = st.has_res ? (const void*)(in->arena + cap * st.res_off) : nullptr;
-        p.scratch = infos[i].scratch_bytes ? v->scratch + scratch_off[i] : nullptr;
+        p.scratch = infos[i].scratch_bytes ? in->arena : nullptr;      // never touched: allows the split (kSplitScratchBytes)
         p.scratch_bytes = infos[i].scratch_bytes;
+        p.reserved = tile_hint(m, (int)i, nb);
         v->params[i] = p;
         if (st.kind == PB_STAGE_CONV_UMMA) {
             const int rc = pb::conv_umma_xmap_create(&p, &v->xmaps[i]);
@@ -580,14 +612,18 @@ extern "C" {
 
 int pb_op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
     PB_REQUIRE(p && out, "pb_op_info: NULL argument");
-    if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_info(p, out);
-    if (kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(out);
-    return pb::simple_op_info(kind, p, out);
+    pb_op_params q = *p;
+    q.reserved = 0;
+    return op_info(kind, &q, out);
 }
 
 int pb_op_launch(int kind, const pb_op_params* p, void* stream, uint32_t job_id, void* notifier) {
     PB_REQUIRE(p != nullptr, "pb_op_launch: NULL params");
-    if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_launch(p, (cudaStream_t)stream, job_id, notifier);
+    if (kind == PB_STAGE_CONV_UMMA) {
+        pb_op_params q = *p;
+        q.reserved = 0;
+        return pb::conv_umma_launch(&q, (cudaStream_t)stream, job_id, notifier);
+    }
     return pb::simple_op_launch(kind, p, (cudaStream_t)stream, job_id, notifier);
 }
 
@@ -893,14 +929,10 @@ int pb_model_load(const char* pack_path, int device, int precision, pb_model** o
         }
         p.w = st.w_dev;
         p.bias = st.bias_dev;
-        // every instance brings scratch memory of the model's largest requirement: size the launch for it
+        // every instance allows its convolutions to split
         p.scratch = (void*)16;
         p.scratch_bytes = ~0ull;
         PB_FAIL_LOAD(pb_op_info(st.kind, &p, &st.info));
-        if (st.info.scratch_bytes) {
-            st.scratch_off = m->scratch_bytes;
-            m->scratch_bytes += pb::round_up((size_t)st.info.scratch_bytes, (size_t)256);
-        }
         if (st.kind == PB_STAGE_CONV_UMMA) PB_FAIL_LOAD(pb::conv_umma_plan_create(&p, st.w_dev, &st.plan));
         m->stages.push_back(st);
     }
@@ -916,6 +948,13 @@ void pb_model_destroy(pb_model* m) {
     for (auto& st : m->stages) if (st.plan) pb::conv_umma_plan_destroy(st.plan);
     for (void* d : m->allocs) cudaFree(d);
     delete m;
+}
+
+int pb_model_set_shared_gpu(pb_model* m, int shared) {
+    PB_REQUIRE(m != nullptr, "pb_model_set_shared_gpu: NULL model");
+    m->shared = shared != 0;
+    refresh_infos(m);
+    return PB_OK;
 }
 
 size_t pb_model_input_bytes(const pb_model* m) { return m ? m->in_floats * 4 : 0; }

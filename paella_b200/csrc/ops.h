@@ -70,6 +70,11 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
                            int n, ConvUmmaMulti** out);
 bool conv_umma_pool_fusable(int kind, const pb_op_params* p);
 uint32_t conv_umma_pool_blocks(const pb_op_params* p);
+// What pb_op_params.reserved carries inside the library (the public entry points ignore it): the cluster size of the
+// grouped launch the convolution is part of (0 = it decides for itself), and whether other requests' launches run beside it.
+constexpr int kTileSplitMask = 0xff, kTileShared = 0x100;
+// Blocks per tile (cluster size) of a grouped launch of these convolutions.
+int conv_umma_common_splits(const pb_op_params* const* params, int n);
 void conv_umma_multi_destroy(ConvUmmaMulti* m);
 void conv_umma_multi_info(const ConvUmmaMulti* m, pb_launch_info* out);
 int conv_umma_multi_launch(const ConvUmmaMulti* m, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);

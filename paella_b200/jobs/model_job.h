@@ -189,6 +189,7 @@ class ModelJob : public llis::job::Job {
         int precision = -1;
         if (const char* p = std::getenv("PB_PRECISION")) precision = std::atoi(p);
         if (pb_model_load(path.c_str(), device, precision, &m) != PB_OK) return nullptr;
+        pb_model_set_shared_gpu(m, 1);       // many requests in flight: the launches share the GPU
         cache[key] = m;
         return m;
     }

@@ -1,0 +1,355 @@
+// Dense convolution in full precision: an implicit GEMM on the fp32 units.
+//
+//   D[m, n] = sum_k A[m, k] * B[k, n]     m = output pixel (all images back to back), n = output channel,
+//                                          k = (r*S + s)*Cs + c   (filter tap, input channel)
+//
+// No tensor-core format keeps fp32 inputs, so the ceiling is the fused multiply-add rate: 148 SMs x 128 x 2 x 1.9 GHz =
+// 72 TFLOP/s.  The direct kernel this replaces for dense layers (conv_simt_kernel: one output per thread, every operand
+// through L1 for each multiplication) ran at 1.9 TFLOP/s.
+//
+// Block = 256 threads on a tile of 64 pixels x BN channels.  A stage is 32 values of k, three stages deep, brought by
+// cp.async: 64 x 32 activations (zero-filled outside the image), turned to [k][pixel] on the way by 4-byte copies, and
+// 32 x BN weights.  The groups of threads that cover the tile once (64 at BN = 64) split every stage's k between them, so
+// a tile this small still feeds eight warps, and their partial tiles are added in group order at the end.  A layer with
+// few tiles additionally splits its k range over the blocks of a cluster (up to 8), whose sums meet through distributed
+// shared memory, in rank order: results do not depend on timing.
+//
+// This is the fp32 member of the kernel family the reference's TVM adapters launch
+// (jobs/tvm_<model>/tvm_<model>.cpp:24-47; generated fp32 kernels there).
+#include <llis/job/finished_block_notifier.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "launch_slot.cuh"
+#include "ops.h"
+#include "pb_common.h"
+
+using llis::job::FinishedBlockNotifier;
+
+namespace pb {
+
+namespace {
+
+constexpr int kTM = 64, kTK = 32, kDepth = 3;
+constexpr int kBlock = 256;
+
+struct F32Args {
+    OpArgs op;
+    int M, PQ;           // rows of the GEMM (all images), pixels per image
+    int n_stages;        // k stages of the whole reduction
+    int splits;          // cluster size
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <int Bytes>
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, bool ok) {
+    if (Bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4u : 0u) : "memory");
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "r"(addr), "r"(rank)
+        : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// Bias, residual, activation and store of four channels of one output pixel.
+__device__ __forceinline__ void finish4(const OpArgs& a, int m, int k, const float4& s, bool vec) {
+    const float v[4] = {s.x, s.y, s.z, s.w};
+    float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int kk = k + j;
+        if (kk >= a.K) break;
+        float x = v[j] + (a.bias ? __ldg(a.bias + kk) : 0.f);
+        if (a.residual) x += static_cast<const float*>(a.residual)[(size_t)m * a.res_Cs + kk];
+        if (a.act == 3) x = x > 0.f ? x : x * __ldg(a.bias + a.K + kk);      // PReLU: slopes follow the biases
+        else if (a.act == 1) x = fmaxf(x, 0.f);
+        else if (a.act == 2) x = fminf(fmaxf(x, 0.f), 6.f);
+        o[j] = x;
+    }
+    float* y = static_cast<float*>(a.y) + (size_t)m * a.Ks + a.out_c_off + k;
+    if (vec && k + 4 <= a.K) {
+        *reinterpret_cast<float4*>(y) = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (k + j < a.K) y[j] = o[j];
+    }
+}
+
+// VecW: weight rows can be copied 16 bytes at a time (K a multiple of 4).
+//
+// A thread owns 8 pixels x TJ channels and takes, per k, its 8 activations and TJ weights as 16-byte loads and multiplies
+// the outer product.  Operand order matters: with the pixels of one k side by side in registers the compiler can place the
+// accumulators so that the three operands of a multiply-add come from different register banks.  (With the k of one pixel
+// side by side - the layout a 16-byte copy of the activations gives - every other multiply-add conflicts: 37 TFLOP/s on a
+// layer that fills the GPU; the packed two-wide multiply-add has no conflicts, but issues at half the rate or less: 38.)
+template <int BN, bool VecW>
+__global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, uint32_t job_id, FinishedBlockNotifier* nf) {
+    griddep_wait();
+    resolve_slot(job_id, nf);
+    if (nf) nf->start(job_id);
+    constexpr int TJ = BN == 64 ? 8 : 4;           // channels per thread
+    constexpr int kGroupThreads = 8 * BN / TJ, kGroups = kBlock / kGroupThreads, kGroupK = kTK / kGroups;
+    constexpr int kStageFloats = kTK * kTM + kTK * BN;
+    constexpr int kLdR = BN + 4;                   // row of a partial tile
+    extern __shared__ __align__(16) float smem[];
+    const OpArgs& a = f.op;
+    const int tid = threadIdx.x;
+    const int m0 = blockIdx.x * kTM, n0 = blockIdx.y * BN, rank = blockIdx.z;
+    const int s0 = f.n_stages * rank / f.splits, s1 = f.n_stages * (rank + 1) / f.splits;
+
+    // ---- what this thread copies: chunk `tid % 8` (4 channels) of pixels tid/8 and tid/8 + 32 ----
+    const int taps = a.R * a.S, c4n = a.Cs / 4;
+    int ih0[2], iw0[2], row0[2];                   // filter-window origin, first input row of the image
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int m = m0 + (tid >> 3) + 32 * i;
+        const bool in = m < f.M;
+        const int img = in ? m / f.PQ : 0, pix = in ? m - img * f.PQ : 0;
+        const int p = pix / a.Q, q = pix - p * a.Q;
+        ih0[i] = in ? p * a.stride_h - a.pad_h : -(1 << 28);      // fails every bounds check: the row is zero-filled
+        iw0[i] = q * a.stride_w - a.pad_w;
+        row0[i] = img * a.H;
+    }
+    int ta = (s0 * 8 + (tid & 7)) / c4n, ca = (s0 * 8 + (tid & 7)) - ta * c4n;      // filter tap and channel group of the chunk
+    int ra = ta / a.S, sa = ta - ra * a.S;
+    uint32_t src[2];
+    bool ok[2];                                    // the pixels' chunks (in units of 16 bytes) and whether they exist, for this tap
+    auto locate = [&]() {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int ih = ih0[i] + ra * a.dil_h, iw = iw0[i] + sa * a.dil_w;
+            ok[i] = ta < taps && (unsigned)ih < (unsigned)a.H && (unsigned)iw < (unsigned)a.W;
+            src[i] = ok[i] ? ((uint32_t)(row0[i] + ih) * (uint32_t)a.W + (uint32_t)iw) * (uint32_t)c4n + (uint32_t)ca : 0u;
+        }
+    };
+    locate();
+    // ---- and of the weights [tap][C][K]: row kb (of 32), then every kRowStep-th ----
+    constexpr int kCols = VecW ? BN / 4 : BN;                     // copies per row
+    constexpr int kRowStep = kBlock / kCols, kCopies = (kTK + kRowStep - 1) / kRowStep;
+    const int kb = tid / kCols, nb = (tid % kCols) * (VecW ? 4 : 1);
+    int tb[kCopies], cb[kCopies];
+#pragma unroll
+    for (int i = 0; i < kCopies; ++i) {
+        const int k = s0 * kTK + kb + i * kRowStep;
+        tb[i] = k / a.Cs;
+        cb[i] = k - tb[i] * a.Cs;
+    }
+    const bool n_ok = n0 + nb < a.K;
+
+    // Pixel m of k row kk is word kk * 64 + (m ^ (kk / 4 % 8 * 4)): a warp's 4-byte copies (8 chunks x 4 pixels) and the
+    // threads' 16-byte reads of 4 pixels are both free of bank conflicts.
+    const uint32_t chunk = (uint32_t)tid & 7u;
+    const uint32_t da0 = smem_u32(smem) + (chunk * 4u * kTM + (((uint32_t)tid >> 3) ^ (chunk * 4u))) * 4u;
+    const uint32_t db0 = smem_u32(smem) + (uint32_t)(kTK * kTM + kb * BN + nb) * 4u;
+    auto fill = [&](int buf) {
+        const uint32_t da = da0 + (uint32_t)(buf * kStageFloats) * 4u, db = db0 + (uint32_t)(buf * kStageFloats) * 4u;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float* g = static_cast<const float*>(a.x) + (size_t)src[i] * 4;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) cp_async<4>(da + (uint32_t)(j * kTM) * 4u + (uint32_t)(i * 32) * 4u, g + j, ok[i]);      // +32 pixels: the XOR stays below bit 5
+        }
+#pragma unroll
+        for (int i = 0; i < kCopies; ++i) {
+            if (kTK % kRowStep == 0 || kb + i * kRowStep < kTK) {
+                const bool in = n_ok && tb[i] < taps && cb[i] < a.C;      // channels past C have no weights (and zero activations)
+                cp_async<VecW ? 16 : 4>(db + (uint32_t)(i * kRowStep * BN) * 4u, static_cast<const float*>(a.w) + (in ? ((size_t)tb[i] * a.C + cb[i]) * a.K + n0 + nb : 0), in);
+            }
+            cb[i] += kTK;
+            while (cb[i] >= a.Cs) { cb[i] -= a.Cs; ++tb[i]; }
+        }
+        // the next stage's chunk: eight further on, in the same tap or a later one
+        ca += 8;
+        if (ca < c4n) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) src[i] += ok[i] ? 8u : 0u;
+        } else {
+            do {
+                ca -= c4n;
+                ++ta;
+                if (++sa == a.S) { sa = 0; ++ra; }
+            } while (ca >= c4n);
+            locate();
+        }
+    };
+
+    float acc[8][TJ];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < TJ; ++j) acc[i][j] = 0.f;
+    // pixels tm*4 .. +3 and 32 further on; channels tn*4 .. +3 and (TJ == 8) BN/2 further on
+    const int grp = tid / kGroupThreads, tm = tid & 7, tn = (tid % kGroupThreads) >> 3;
+
+#pragma unroll
+    for (int d = 0; d < kDepth - 1; ++d) {
+        if (s0 + d < s1) fill(d);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int buf = 0, fill_buf = kDepth - 1;
+    for (int s = s0; s < s1; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 2) : "memory");
+        __syncthreads();                 // the stage has landed for everyone; everyone is done with the buffer refilled next
+        if (s + kDepth - 1 < s1) fill(fill_buf);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* As = smem + buf * kStageFloats + grp * kGroupK * kTM;
+        const float* Bs = smem + buf * kStageFloats + kTK * kTM + grp * kGroupK * BN + tn * 4;
+#pragma unroll
+        for (int q = 0; q < kGroupK; ++q) {
+            float av[8], bv[TJ];
+            const float* ar = As + q * kTM + ((tm ^ ((grp * kGroupK + q) >> 2 & 7)) << 2);
+            *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(ar);
+            *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(ar + 32);
+            *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(Bs + q * BN);
+            if constexpr (TJ == 8) *reinterpret_cast<float4*>(bv + 4) = *reinterpret_cast<const float4*>(Bs + q * BN + BN / 2);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TJ; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        if (++buf == kDepth) buf = 0;
+        if (++fill_buf == kDepth) fill_buf = 0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    // ---- the groups' partial tiles meet in shared memory ----
+    float* red = smem;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        float* row = red + (grp * kTM + tm * 4 + (i & 3) + (i >> 2) * 32) * kLdR + tn * 4;
+        *reinterpret_cast<float4*>(row) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        if constexpr (TJ == 8) *reinterpret_cast<float4*>(row + BN / 2) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+    }
+    __syncthreads();
+    constexpr int kVecs = kTM * BN / 4;
+    const bool vec = ((a.Ks | a.out_c_off) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
+    for (int v = tid; v < kVecs; v += kBlock) {
+        const int row = v / (BN / 4), col = (v - row * (BN / 4)) * 4;
+        float4 s = *reinterpret_cast<const float4*>(red + row * kLdR + col);
+#pragma unroll
+        for (int g = 1; g < kGroups; ++g) s = add4(s, *reinterpret_cast<const float4*>(red + (g * kTM + row) * kLdR + col));
+        if (f.splits == 1) {
+            if (m0 + row < f.M && n0 + col < a.K) finish4(a, m0 + row, n0 + col, s, vec);
+        } else {
+            *reinterpret_cast<float4*>(red + row * kLdR + col) = s;
+        }
+    }
+    if (f.splits > 1) {
+        // ---- and the ranks' sums through distributed shared memory: rank r finishes rows [r * 64 / splits, ...) ----
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        const int rows = kTM / f.splits, r0 = rank * rows;
+        for (int v = tid; v < rows * (BN / 4); v += kBlock) {
+            const int row = r0 + v / (BN / 4), col = (v % (BN / 4)) * 4;
+            const uint32_t at = smem_u32(red + row * kLdR + col);
+            float4 s = ld_cluster(at, 0);
+            for (int z = 1; z < f.splits; ++z) s = add4(s, ld_cluster(at, (uint32_t)z));
+            if (m0 + row < f.M && n0 + col < a.K) finish4(a, m0 + row, n0 + col, s, vec);
+        }
+        asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait.acquire;" ::: "memory");      // every rank has been read
+    }
+    griddep_launch();
+    if (nf) nf->end(job_id);
+}
+
+struct F32Geometry {
+    int BN, m_tiles, n_tiles, splits, n_stages;
+    uint32_t smem;
+    const void* fn;
+};
+
+int batch_of(const pb_op_params* p) { return p->batch > 1 ? p->batch : 1; }
+
+F32Geometry conv_f32_geometry(const pb_op_params* p) {
+    F32Geometry g;
+    g.BN = p->K > 32 ? 64 : (p->K > 16 ? 32 : 16);
+    g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kTM);
+    g.n_tiles = ceil_div(p->K, g.BN);
+    g.n_stages = ceil_div(p->R * p->S * p->Cs, kTK);
+    // Split: least modelled time of a lone launch.  A stage of a 64-column tile is 1024 clocks of multiply-adds for the
+    // SM, shared by its blocks; a split adds two cluster barriers and the exchange.
+    const int tiles = g.m_tiles * g.n_tiles;
+    g.splits = 1;
+    double best = 1e30;
+    for (int S = 1; S <= 8; S *= 2) {
+        if (S > 1 && (g.n_stages < 2 * S || conv_split_gain_us() > 1e6)) break;
+        const double us = ceil_div(g.n_stages, S) * 0.55 * g.BN / 64.0 * std::max(1.0, tiles * S / 148.0) + (S > 1 ? 1.0 + 0.1 * S : 0.0);
+        if (us < best) { best = us; g.splits = S; }
+    }
+    const int groups = g.BN == 16 ? 8 : 4;
+    const size_t pipe = (size_t)kDepth * (kTK * kTM + kTK * g.BN) * 4, red = (size_t)groups * kTM * (g.BN + 4) * 4;
+    g.smem = (uint32_t)std::max(pipe, red);
+    const bool vec = p->K % 4 == 0 && ((uintptr_t)p->w & 15) == 0;
+#define PB_F32(BN_) (vec ? (const void*)conv_f32_kernel<BN_, true> : (const void*)conv_f32_kernel<BN_, false>)
+    g.fn = g.BN == 64 ? PB_F32(64) : (g.BN == 32 ? PB_F32(32) : PB_F32(16));
+#undef PB_F32
+    return g;
+}
+
+}  // namespace
+
+// Dense fp32 layers; the rest (groups, a handful of outputs) keeps conv_simt_kernel, whose thread per output is the better
+// shape for reductions of a few values.
+bool conv_f32_supported(const pb_op_params* p) {
+    return p->dtype == 0 && p->groups <= 1 && p->Cs % 4 == 0 && p->K >= 8 && p->R * p->S * p->Cs >= 16 &&
+           (uint64_t)batch_of(p) * p->H * p->W * p->Cs / 4 <= 0xffffffffull;
+}
+
+int conv_f32_info(const pb_op_params* p, pb_launch_info* out) {
+    const F32Geometry g = conv_f32_geometry(p);
+    memset(out, 0, sizeof(*out));
+    out->kind = PB_STAGE_CONV_SIMT;
+    out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
+    out->threads_per_block = kBlock;
+    cudaFuncAttributes at;
+    out->regs_per_thread = 128;
+    if (cudaFuncGetAttributes(&at, g.fn) == cudaSuccess) out->regs_per_thread = (uint32_t)at.numRegs;
+    else cudaGetLastError();
+    out->smem_per_block = g.smem;
+    const uint64_t nb = (uint64_t)batch_of(p), y = nb * p->K * p->P * p->Q;
+    out->flops = 2ull * y * p->C * p->R * p->S;
+    out->bytes = 4ull * (nb * p->C * p->H * p->W + (uint64_t)p->K * p->C * p->R * p->S + y + (p->residual ? y : 0)) + 4ull * p->K;
+    return PB_OK;
+}
+
+int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl) {
+    const F32Geometry g = conv_f32_geometry(p);
+    F32Args f;
+    f.op = op;
+    f.PQ = p->P * p->Q;
+    f.M = batch_of(p) * f.PQ;
+    f.n_stages = g.n_stages;
+    f.splits = g.splits;
+    PB_CUDA(cudaFuncSetAttribute(g.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)g.m_tiles, (unsigned)g.n_tiles, (unsigned)g.splits);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (g.splits > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 1;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = (unsigned)g.splits;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, (void (*)(const F32Args, uint32_t, FinishedBlockNotifier*))g.fn, f, job_id, static_cast<FinishedBlockNotifier*>(notifier)));
+    return PB_OK;
+}
+
+}  // namespace pb

@@ -1519,7 +1519,9 @@ int tiles_per_cta() {
 // How reluctant a launch is to split its reduction, in the unit of pb_set_conv_split_gain_us (see choose_tiling, which asks
 // for a 60th of it; above 1e6 nothing splits).  PB_CONV_SPLIT_GAIN_US or the function override the default of 6.
 std::atomic<double> g_split_gain_us{-1.0};      // < 0: not set yet, take PB_CONV_SPLIT_GAIN_US or the default
-double split_gain_us() {
+}  // namespace
+
+double conv_split_gain_us() {
     double v = g_split_gain_us.load(std::memory_order_relaxed);
     if (v < 0) {
         const char* e = getenv("PB_CONV_SPLIT_GAIN_US");
@@ -1529,6 +1531,8 @@ double split_gain_us() {
     }
     return v;
 }
+
+namespace {
 
 int batch_of(const pb_op_params* p) { return p->batch > 1 ? p->batch : 1; }
 int dil_h(const pb_op_params* p) { return p->dil_h > 1 ? p->dil_h : 1; }
@@ -1604,7 +1608,7 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     g.Kdim_pad = g.nkb * kBK;
     g.Kp16 = round_up(p->K, 16);
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM);
-    const double gain = split_gain_us();
+    const double gain = conv_split_gain_us();
     const int want = p->reserved & kTileSplitMask;       // a grouped launch has one cluster size for all its convolutions (0: not decided)
     const bool shared = (p->reserved & kTileShared) != 0;
     Tiling t = choose_tiling(g.m_tiles, g.Kp16, g.nkb, bn_limit(), !use_tma_a() || gain > 1e6 ? 1 : want, gain, shared);
@@ -1990,7 +1994,7 @@ bool conv_umma_multi_available() { return use_tma_a(); }
 
 // The cluster size of a grouped launch is one for all its convolutions: the one whose slowest member is modelled fastest.
 int conv_umma_common_splits(const pb_op_params* const* params, int n) {
-    const double gain = split_gain_us();
+    const double gain = conv_split_gain_us();
     if (!use_tma_a() || persist_enabled() || gain > 1e6) return 1;
     int best = 1;
     double best_us = 1e30;

@@ -1363,6 +1363,7 @@ static int info_one_image(int kind, const pb_op_params* p, pb_launch_info* out) 
 static bool folds_batch(int kind) { return kind == PB_STAGE_ADD || kind == PB_STAGE_AFFINE; }
 
 int simple_op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
+    if (kind == PB_STAGE_CONV_SIMT && conv_f32_supported(p)) return conv_f32_info(p, out);
     const int nb = batch_of(p);
     const int rc = info_one_image(kind, p, out);
     if (rc != PB_OK || nb == 1) return rc;
@@ -1400,6 +1401,7 @@ static void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t
 }
 
 int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl) {
+    if (kind == PB_STAGE_CONV_SIMT && conv_f32_supported(p)) return conv_f32_launch(p, to_args(p), st, job_id, notifier, pdl);
     FinishedBlockNotifier* nf = static_cast<FinishedBlockNotifier*>(notifier);
     pb_launch_info li;
     pb_op_params folded;

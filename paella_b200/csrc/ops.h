@@ -33,6 +33,12 @@ int mnist_fused_info(pb_launch_info* out);
 int mnist_fused_launch(const float* x, const float* w1, const float* b1, const float* w2, const float* b2,
                        const float* wd, const float* bd, float* y, int batch, cudaStream_t st, uint32_t job_id, void* notifier);
 
+// conv_f32.cu: dense fp32 convolution (PB_STAGE_CONV_SIMT) as an implicit GEMM
+bool conv_f32_supported(const pb_op_params* p);
+int conv_f32_info(const pb_op_params* p, pb_launch_info* out);
+int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);
+double conv_split_gain_us();      // see pb_set_conv_split_gain_us
+
 // conv_umma.cu: tcgen05 implicit-GEMM convolution (bf16 operands, fp32 accumulation in TMEM)
 bool conv_umma_supported(const pb_op_params* p);
 int conv_umma_info(const pb_op_params* p, pb_launch_info* out);

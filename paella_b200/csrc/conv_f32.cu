@@ -37,6 +37,7 @@ constexpr int kBlock = 256;
 struct F32Args {
     OpArgs op;
     int M, PQ;           // rows of the GEMM (all images), pixels per image
+    int Kp;              // channels of a row of packed weights (K rounded up to 4)
     int n_stages;        // k stages of the whole reduction
     int splits;          // cluster size
 };
@@ -83,14 +84,14 @@ __device__ __forceinline__ void finish4(const OpArgs& a, int m, int k, const flo
     }
 }
 
-// VecW: weight rows can be copied 16 bytes at a time (K a multiple of 4).
+// Aligned: the weights start on a 16-byte boundary.
 //
 // A thread owns 8 pixels x TJ channels and takes, per k, its 8 activations and TJ weights as 16-byte loads and multiplies
 // the outer product.  Operand order matters: with the pixels of one k side by side in registers the compiler can place the
 // accumulators so that the three operands of a multiply-add come from different register banks.  (With the k of one pixel
 // side by side - the layout a 16-byte copy of the activations gives - every other multiply-add conflicts: 37 TFLOP/s on a
 // layer that fills the GPU; the packed two-wide multiply-add has no conflicts, but issues at half the rate or less: 38.)
-template <int BN, bool VecW>
+template <int BN, bool Aligned>
 __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, uint32_t job_id, FinishedBlockNotifier* nf) {
     griddep_wait();
     resolve_slot(job_id, nf);
@@ -120,29 +121,22 @@ __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, ui
     }
     int ta = (s0 * 8 + (tid & 7)) / c4n, ca = (s0 * 8 + (tid & 7)) - ta * c4n;      // filter tap and channel group of the chunk
     int ra = ta / a.S, sa = ta - ra * a.S;
-    uint32_t src[2];
+    size_t src[2];
     bool ok[2];                                    // the pixels' chunks (in units of 16 bytes) and whether they exist, for this tap
     auto locate = [&]() {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int ih = ih0[i] + ra * a.dil_h, iw = iw0[i] + sa * a.dil_w;
             ok[i] = ta < taps && (unsigned)ih < (unsigned)a.H && (unsigned)iw < (unsigned)a.W;
-            src[i] = ok[i] ? ((uint32_t)(row0[i] + ih) * (uint32_t)a.W + (uint32_t)iw) * (uint32_t)c4n + (uint32_t)ca : 0u;
+            src[i] = ok[i] ? ((size_t)(row0[i] + ih) * a.W + iw) * c4n + ca : 0;
         }
     };
     locate();
-    // ---- and of the weights [tap][C][K]: row kb (of 32), then every kRowStep-th ----
-    constexpr int kCols = VecW ? BN / 4 : BN;                     // copies per row
-    constexpr int kRowStep = kBlock / kCols, kCopies = (kTK + kRowStep - 1) / kRowStep;
-    const int kb = tid / kCols, nb = (tid % kCols) * (VecW ? 4 : 1);
-    int tb[kCopies], cb[kCopies];
-#pragma unroll
-    for (int i = 0; i < kCopies; ++i) {
-        const int k = s0 * kTK + kb + i * kRowStep;
-        tb[i] = k / a.Cs;
-        cb[i] = k - tb[i] * a.Cs;
-    }
-    const bool n_ok = n0 + nb < a.K;
+    // ---- and of the packed weights [tap][Cs][Kp]: row kb (of 32), then every kRowStep-th, four channels each ----
+    constexpr int kCols = BN / 4, kRowStep = kBlock / kCols, kCopies = (kTK + kRowStep - 1) / kRowStep;
+    const int kb = tid / kCols, nb = (tid % kCols) * 4;
+    int rows_left = n0 + nb < f.Kp ? taps * a.Cs - (s0 * kTK + kb) : 0;       // rows from this one to the last
+    uint32_t wsrc = (uint32_t)(s0 * kTK + kb) * (uint32_t)f.Kp + (uint32_t)(n0 + nb);
 
     // Pixel m of k row kk is word kk * 64 + (m ^ (kk / 4 % 8 * 4)): a warp's 4-byte copies (8 chunks x 4 pixels) and the
     // threads' 16-byte reads of 4 pixels are both free of bank conflicts.
@@ -153,19 +147,24 @@ __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, ui
         const uint32_t da = da0 + (uint32_t)(buf * kStageFloats) * 4u, db = db0 + (uint32_t)(buf * kStageFloats) * 4u;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const float* g = static_cast<const float*>(a.x) + (size_t)src[i] * 4;
+            const float* g = static_cast<const float*>(a.x) + src[i] * 4;
 #pragma unroll
             for (int j = 0; j < 4; ++j) cp_async<4>(da + (uint32_t)(j * kTM) * 4u + (uint32_t)(i * 32) * 4u, g + j, ok[i]);      // +32 pixels: the XOR stays below bit 5
         }
 #pragma unroll
-        for (int i = 0; i < kCopies; ++i) {
+        for (int i = 0; i < kCopies; ++i)
             if (kTK % kRowStep == 0 || kb + i * kRowStep < kTK) {
-                const bool in = n_ok && tb[i] < taps && cb[i] < a.C;      // channels past C have no weights (and zero activations)
-                cp_async<VecW ? 16 : 4>(db + (uint32_t)(i * kRowStep * BN) * 4u, static_cast<const float*>(a.w) + (in ? ((size_t)tb[i] * a.C + cb[i]) * a.K + n0 + nb : 0), in);
+                const bool in = i * kRowStep < rows_left;
+                const float* g = static_cast<const float*>(a.w) + (in ? wsrc + (uint32_t)(i * kRowStep) * (uint32_t)f.Kp : 0u);
+                if (Aligned) {
+                    cp_async<16>(db + (uint32_t)(i * kRowStep * BN) * 4u, g, in);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) cp_async<4>(db + (uint32_t)(i * kRowStep * BN + j) * 4u, g + j, in);
+                }
             }
-            cb[i] += kTK;
-            while (cb[i] >= a.Cs) { cb[i] -= a.Cs; ++tb[i]; }
-        }
+        rows_left -= kTK;
+        wsrc += (uint32_t)kTK * (uint32_t)f.Kp;
         // the next stage's chunk: eight further on, in the same tap or a later one
         ca += 8;
         if (ca < c4n) {
@@ -202,18 +201,22 @@ __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, ui
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* As = smem + buf * kStageFloats + grp * kGroupK * kTM;
         const float* Bs = smem + buf * kStageFloats + kTK * kTM + grp * kGroupK * BN + tn * 4;
+        float av[2][8], bv[2][TJ];
+        auto load = [&](int q) {
+            const float* ar = As + q * kTM + ((tm ^ ((grp * kGroupK + q) >> 2 & 7)) << 2);
+            *reinterpret_cast<float4*>(av[q & 1]) = *reinterpret_cast<const float4*>(ar);
+            *reinterpret_cast<float4*>(av[q & 1] + 4) = *reinterpret_cast<const float4*>(ar + 32);
+            *reinterpret_cast<float4*>(bv[q & 1]) = *reinterpret_cast<const float4*>(Bs + q * BN);
+            if constexpr (TJ == 8) *reinterpret_cast<float4*>(bv[q & 1] + 4) = *reinterpret_cast<const float4*>(Bs + q * BN + BN / 2);
+        };
+        load(0);
 #pragma unroll
         for (int q = 0; q < kGroupK; ++q) {
-            float av[8], bv[TJ];
-            const float* ar = As + q * kTM + ((tm ^ ((grp * kGroupK + q) >> 2 & 7)) << 2);
-            *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(ar);
-            *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(ar + 32);
-            *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(Bs + q * BN);
-            if constexpr (TJ == 8) *reinterpret_cast<float4*>(bv + 4) = *reinterpret_cast<const float4*>(Bs + q * BN + BN / 2);
+            if (q + 1 < kGroupK) load(q + 1);          // under this k's multiplications
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < TJ; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < TJ; ++j) acc[i][j] = fmaf(av[q & 1][i], bv[q & 1][j], acc[i][j]);
         }
         if (++buf == kDepth) buf = 0;
         if (++fill_buf == kDepth) fill_buf = 0;
@@ -244,14 +247,20 @@ __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, ui
         }
     }
     if (f.splits > 1) {
-        // ---- and the ranks' sums through distributed shared memory: rank r finishes rows [r * 64 / splits, ...) ----
+        // ---- and the ranks' sums through distributed shared memory: each rank finishes a share of the tile ----
         asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-        const int rows = kTM / f.splits, r0 = rank * rows;
-        for (int v = tid; v < rows * (BN / 4); v += kBlock) {
-            const int row = r0 + v / (BN / 4), col = (v % (BN / 4)) * 4;
+        const int v1 = kVecs * (rank + 1) / f.splits;
+        for (int v = kVecs * rank / f.splits + tid; v < v1; v += kBlock) {
+            const int row = v / (BN / 4), col = (v - row * (BN / 4)) * 4;
             const uint32_t at = smem_u32(red + row * kLdR + col);
-            float4 s = ld_cluster(at, 0);
-            for (int z = 1; z < f.splits; ++z) s = add4(s, ld_cluster(at, (uint32_t)z));
+            float4 part[8];          // every rank's sum on its way before the first is used
+#pragma unroll
+            for (int z = 0; z < 8; ++z)
+                if (z < f.splits) part[z] = ld_cluster(at, (uint32_t)z);
+            float4 s = part[0];
+#pragma unroll
+            for (int z = 1; z < 8; ++z)
+                if (z < f.splits) s = add4(s, part[z]);
             if (m0 + row < f.M && n0 + col < a.K) finish4(a, m0 + row, n0 + col, s, vec);
         }
         asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait.acquire;" ::: "memory");      // every rank has been read
@@ -274,21 +283,27 @@ F32Geometry conv_f32_geometry(const pb_op_params* p) {
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kTM);
     g.n_tiles = ceil_div(p->K, g.BN);
     g.n_stages = ceil_div(p->R * p->S * p->Cs, kTK);
-    // Split: least modelled time of a lone launch.  A stage of a 64-column tile is 1024 clocks of multiply-adds for the
-    // SM, shared by its blocks; a split adds two cluster barriers and the exchange.
+    // Split: least modelled time of a lone launch.  A stage of a 64-column tile takes an SM 1.0 us whether one block runs or
+    // two side by side (measured), so what counts is how many stages the fullest SM gets: one block as long as the launch
+    // fits one per SM, else two, then in waves.  Clusters reach fewer SMs than lone blocks (measured with idle kernels).
+    // A launch costs 5 us besides, a split 1.5 to 2.7 us (two cluster barriers and the exchange).
+    static const int kOnePerSm[9] = {0, 148, 148, 135, 132, 130, 132, 0, 120}, kTwoPerSm[9] = {0, 296, 296, 279, 284, 280, 270, 0, 264};
     const int tiles = g.m_tiles * g.n_tiles;
     g.splits = 1;
     double best = 1e30;
-    for (int S = 1; S <= 8; S *= 2) {
+    for (int S = 1; S <= 8; ++S) {
         if (S > 1 && (g.n_stages < 2 * S || conv_split_gain_us() > 1e6)) break;
-        const double us = ceil_div(g.n_stages, S) * 0.55 * g.BN / 64.0 * std::max(1.0, tiles * S / 148.0) + (S > 1 ? 1.0 + 0.1 * S : 0.0);
+        if (S == 7) continue;      // two clusters of 7 on a GPC's SMs leave the rest idle: 47 us where 5 takes 37
+        const int blocks = tiles * S;
+        const double load = blocks <= kOnePerSm[S] ? 1.0 : (S == 1 ? std::max(2.0, blocks / 148.0) : 2.0 * ceil_div(blocks, kTwoPerSm[S]));
+        const double us = load * ceil_div(g.n_stages, S) * g.BN / 64.0 + (S > 1 ? 1.5 + 0.15 * S : 0.0);
         if (us < best) { best = us; g.splits = S; }
     }
     const int groups = g.BN == 16 ? 8 : 4;
     const size_t pipe = (size_t)kDepth * (kTK * kTM + kTK * g.BN) * 4, red = (size_t)groups * kTM * (g.BN + 4) * 4;
     g.smem = (uint32_t)std::max(pipe, red);
-    const bool vec = p->K % 4 == 0 && ((uintptr_t)p->w & 15) == 0;
-#define PB_F32(BN_) (vec ? (const void*)conv_f32_kernel<BN_, true> : (const void*)conv_f32_kernel<BN_, false>)
+    const bool aligned = ((uintptr_t)p->w & 15) == 0;
+#define PB_F32(BN_) (aligned ? (const void*)conv_f32_kernel<BN_, true> : (const void*)conv_f32_kernel<BN_, false>)
     g.fn = g.BN == 64 ? PB_F32(64) : (g.BN == 32 ? PB_F32(32) : PB_F32(16));
 #undef PB_F32
     return g;
@@ -299,8 +314,21 @@ F32Geometry conv_f32_geometry(const pb_op_params* p) {
 // Dense fp32 layers; the rest (groups, a handful of outputs) keeps conv_simt_kernel, whose thread per output is the better
 // shape for reductions of a few values.
 bool conv_f32_supported(const pb_op_params* p) {
-    return p->dtype == 0 && p->groups <= 1 && p->Cs % 4 == 0 && p->K >= 8 && p->R * p->S * p->Cs >= 16 &&
-           (uint64_t)batch_of(p) * p->H * p->W * p->Cs / 4 <= 0xffffffffull;
+    return p->dtype == 0 && p->groups <= 1 && p->Cs % 4 == 0 && p->K >= 8 && p->R * p->S * p->Cs >= 16 && (uint64_t)p->R * p->S * (p->Cs + 32) * (p->K + 64) <= 0xffffffffull;
+}
+
+// [tap][Cs][K rounded up to 4], zero past C and K.
+int64_t conv_f32_pack_weights(const pb_op_params* p, const float* w, void* dst) {
+    const int taps = p->R * p->S, Kp = round_up(p->K, 4);
+    const size_t n = (size_t)taps * p->Cs * Kp;
+    if (dst) {
+        float* d = static_cast<float*>(dst);
+        memset(d, 0, n * 4);
+        for (int k = 0; k < p->K; ++k)
+            for (int c = 0; c < p->C; ++c)
+                for (int t = 0; t < taps; ++t) d[((size_t)t * p->Cs + c) * Kp + k] = w[((size_t)k * p->C + c) * taps + t];
+    }
+    return (int64_t)(n * 4);
 }
 
 int conv_f32_info(const pb_op_params* p, pb_launch_info* out) {
@@ -326,6 +354,7 @@ int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, ui
     f.op = op;
     f.PQ = p->P * p->Q;
     f.M = batch_of(p) * f.PQ;
+    f.Kp = round_up(p->K, 4);
     f.n_stages = g.n_stages;
     f.splits = g.splits;
     PB_CUDA(cudaFuncSetAttribute(g.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));

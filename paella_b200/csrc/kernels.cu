@@ -1553,6 +1553,7 @@ void store_elem(void* dst, size_t i, float v, int dtype) {
 }
 
 int64_t simple_pack_weights(int kind, const pb_op_params* p, const float* w, void* dst) {
+    if (kind == PB_STAGE_CONV_SIMT && conv_f32_supported(p)) return conv_f32_pack_weights(p, w, dst);
     const size_t es = elem_size(p->dtype);
     const int groups = p->groups > 0 ? p->groups : 1;
     if (kind == PB_STAGE_CONV_SIMT) {

@@ -36,6 +36,7 @@ int mnist_fused_launch(const float* x, const float* w1, const float* b1, const f
 // conv_f32.cu: dense fp32 convolution (PB_STAGE_CONV_SIMT) as an implicit GEMM
 bool conv_f32_supported(const pb_op_params* p);
 int conv_f32_info(const pb_op_params* p, pb_launch_info* out);
+int64_t conv_f32_pack_weights(const pb_op_params* p, const float* w_oihw, void* dst_host);
 int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);
 double conv_split_gain_us();      // see pb_set_conv_split_gain_us
 

@@ -1854,6 +1854,28 @@ struct alignas(64) ConvUmmaXMap {
     CUtensorMap map;
 };
 
+int encode_tiled_bf16(const void* base, int rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, bool nan_fill, CUtensorMap* out) {
+    EncodeTiledFn enc = encode_fn();
+    PB_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
+    PB_REQUIRE(rank >= 1 && rank <= 5 && ((uintptr_t)base & 15) == 0, "tensor map: the tensor must be 16-byte aligned");
+    cuuint64_t d[5], st[5];
+    cuuint32_t bx[5], es[5];
+    for (int i = 0; i < rank; ++i) {
+        d[i] = dims[i];
+        bx[i] = box[i];
+        es[i] = 1;
+        if (i + 1 < rank) st[i] = strides[i];
+    }
+    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           nan_fill ? CU_TENSOR_MAP_FLOAT_OOB_FILL_NAN_REQUEST_ZERO_FMA : CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed with CUresult %d (rank %d, box %u x %u)", (int)r, rank, box[0], box[1]);
+        return PB_ERR_CUDA;
+    }
+    return PB_OK;
+}
+
 int conv_umma_xmap_create(const pb_op_params* p, ConvUmmaXMap** out) {
     if (!use_tma_a()) { *out = nullptr; return PB_OK; }
     ConvUmmaXMap* m = new ConvUmmaXMap();

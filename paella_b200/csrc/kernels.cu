@@ -8,6 +8,7 @@
 // Access pattern: the channel dimension is innermost and padded to a 16-byte vector
 // (4 fp32 / 8 bf16), so one thread moves one 128-bit vector and a warp reads a
 // contiguous 512-byte span whenever Cs >= 32 vectors.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <llis/job/finished_block_notifier.h>
 
@@ -580,239 +581,281 @@ __global__ void __launch_bounds__(256, 2) window3_strip_kernel(OpArgs a, uint32_
     PB_NOTIFY_END();
 }
 
-// ---- 3x3 windows over tensors that fill the GPU many times over -------------------------------------------
-// window3_strip_kernel loads every input row three times (once per output row it belongs to) and converts
-// it to fp32 each time: about 300 instructions per output vector of 8 bf16 channels, which is what bounds
-// it (28 % of the copy bandwidth for the depthwise case; 70 % of the issue slots busy).  window3_tile_kernel
-// below lets a thread own TWO channels (one 32-bit word of bf16) of a strip of output columns and walk down
-// the output rows: each input row is read and converted ONCE and feeds the (up to) three output rows it
-// belongs to, whose accumulators stay in registers, as do the 18 filter values and the 2 biases of the
-// thread's channels.  Max pooling compares the bf16 pairs themselves (a maximum needs no wider type);
-// ReLU / ReLU6 clamp the rounded bf16 pair (rounding is monotonic and 0 and 6 are bf16 values, so clamping
-// after rounding equals rounding after clamping).  Taps outside the tensor contribute the neutral element
-// (0 for sums and products, -inf for max), which leaves every partial result as it is: the additions per
-// output happen in the order of dwconv_kernel / pool_kernel (filter rows, then columns), so the results
-// are theirs bit for bit (finite filter values assumed).  bf16 only.
-constexpr int kTileStrip1 = 4, kTileStrip2 = 2;
-__device__ __forceinline__ f2_t pair_of(uint32_t u) { return f2_pack(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+// ---- 3x3 windows over tensors that fill the GPU, staged through shared memory ------------------------------------
+// window3_strip_kernel loads every input row three times (once per output row it belongs to) and converts it to fp32 each
+// time: about 300 instructions per output vector of 8 bf16 channels, which is what bounds it.  Here a block owns a tile of
+// output rows x columns of ONE slab of 64 channels.  One TMA copy brings the tile's input window into shared memory
+// (zero-filled outside the tensor; NaN for max, which the other operand of a maximum beats), then every half-warp walks down
+// a strip of output columns, its 16 lanes holding four channels each: a row is read with one 8-byte load per input column, converted once, and feeds the
+// (up to) three output rows it belongs to, whose accumulators stay in registers, as do the filter and the biases of the
+// four channels.  Sums and products are packed pairs of fp32 (two IEEE operations per instruction).
+//
+// What bounds it is instruction issue, so the instructions per output are what the layout is chosen for: four channels a
+// lane instead of two halve the loads, stores and address arithmetic, the packed arithmetic halves the rest, and a copy by
+// 16-byte cp.async cost as much as a fifth of the walk in addresses and bounds checks.
+// The activation and how an average counts its padding are template parameters: with all variants in one body the kernel
+// ran out of the instruction cache.  Four or five warps (one per two units) and up to 74 KB of window: three blocks per SM
+// fill and walk in turn.
+//
+// Max pooling compares the bf16 pairs themselves (a maximum needs no wider type); ReLU / ReLU6 clamp the rounded bf16 pair
+// (rounding is monotonic and 0 and 6 are bf16 values).  Taps outside the tensor contribute the neutral element; an
+// output's first tap opens its accumulator, so only the sign of a sum of zeros could show it.  The additions per output happen in the order of dwconv_kernel / pool_kernel (filter
+// rows, then columns), so the results are theirs bit for bit (finite filter values assumed).  bf16 only.
+constexpr int kTileStrip1 = 4, kTileStrip2 = 2;      // output columns per strip at stride 1 / 2
+constexpr int kTileRows1 = 13, kTileRows2 = 6;       // output rows per tile (single images; batches: see win_tile())
+constexpr int kTileSlab = 64;                        // channels per block
+constexpr int kTileMaxThreads = 160;
+
+// Tile geometry of a launch: strips x bands of output rows are the units the half-warps take.
+struct WinTile {
+    int col_tiles, strips, in_cols;      // column tiles per image, strips per tile, window columns
+    int rows, bands, band_rows;          // output rows per tile, split into bands
+    int in_rows, alloc_rows;             // window rows that are copied / that a walk may read
+    int threads, smem;
+};
+
+__device__ __forceinline__ uint64_t p2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t p2_add(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t p2_mul(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t p2_of(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 p2_split(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t p2_bf16(uint32_t u) { return p2_of(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
 __device__ __forceinline__ uint32_t bits_of(__nv_bfloat162 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 __device__ __forceinline__ __nv_bfloat162 bf2_of(uint32_t u) { return *reinterpret_cast<const __nv_bfloat162*>(&u); }
 
-// What a thread keeps per (output, channel pair): fp32 pairs for sums, the bf16 pair itself for a maximum.
-template <int kMode> struct WinAcc { typedef f2_t type; };
+// What a lane keeps per (output, channel pair): fp32 pairs for sums, the bf16 pair itself for a maximum.
+template <int kMode> struct WinAcc { typedef uint64_t type; };
 template <> struct WinAcc<kWinMax> { typedef uint32_t type; };
-template <int kMode> __device__ __forceinline__ typename WinAcc<kMode>::type win_neutral() { return f2_pack(0.f, 0.f); }
-template <> __device__ __forceinline__ uint32_t win_neutral<kWinMax>() { return 0xff80ff80u; }       // (-inf, -inf)
-template <int kMode> __device__ __forceinline__ typename WinAcc<kMode>::type win_value(uint32_t raw) { return pair_of(raw); }
+template <int kMode> __device__ __forceinline__ typename WinAcc<kMode>::type win_value(uint32_t raw) { return p2_bf16(raw); }
 template <> __device__ __forceinline__ uint32_t win_value<kWinMax>(uint32_t raw) { return raw; }
-__device__ __forceinline__ f2_t win_step(f2_t acc, f2_t x, f2_t w, bool dw) { return dw ? f2_fma(x, w, acc) : f2_add(acc, x); }
-__device__ __forceinline__ uint32_t win_step(uint32_t acc, uint32_t x, f2_t, bool) { return bits_of(__hmax2(bf2_of(acc), bf2_of(x))); }
+__device__ __forceinline__ uint64_t win_open(uint64_t x, uint64_t w, bool dw) { return dw ? p2_mul(x, w) : x; }
+__device__ __forceinline__ uint32_t win_open(uint32_t x, uint64_t, bool) { return x; }
+__device__ __forceinline__ uint64_t win_step(uint64_t acc, uint64_t x, uint64_t w, bool dw) { return dw ? p2_fma(x, w, acc) : p2_add(acc, x); }
+__device__ __forceinline__ uint32_t win_step(uint32_t acc, uint32_t x, uint64_t, bool) { return bits_of(__hmax2(bf2_of(acc), bf2_of(x))); }
 
-// One finished output (two channels) -> bf16 pair.  kAct: 0 none, 1 ReLU, 2 ReLU6 (depthwise only).  div / inv: the
-// average pool's divisor and its reciprocal.
+// One finished output (two channels) -> bf16 pair.  kAct: 0 none, 1 ReLU, 2 ReLU6.  div / inv: the average pool's divisor
+// and its reciprocal.  tail: a pooling layer with biases (a convolution that ran before the pooling).
 template <int kMode, int kAct>
-__device__ __forceinline__ uint32_t win_finish(f2_t acc, float b0, float b1, float div, float inv) {
-    float v0, v1;
-    f2_unpack(acc, v0, v1);
+__device__ __forceinline__ uint32_t win_finish(uint64_t v, uint64_t bias, float div, float inv, bool tail) {
     if (kMode == kWinDw) {
-        __nv_bfloat162 h = __floats2bfloat162_rn(v0 + b0, v1 + b1);
-        if (kAct >= 1) h = __hmax2(h, bf2_of(0u));
-        if (kAct == 2) h = __hmin2(h, bf2_of(0x40c040c0u));          // (6, 6)
-        return bits_of(h);
+        v = p2_add(v, bias);
+    } else {
+        // v / div, correctly rounded, without the division sequence: with inv the correctly rounded reciprocal, q = v * inv is
+        // within an ulp, the fused residual v - div * q is exact and q + r * inv rounds to the quotient (Markstein).  An
+        // infinite q makes the residual NaN; clamped to a finite value it leaves q as it is.
+        const uint64_t inv2 = p2_of(inv, inv), q = p2_mul(v, inv2);
+        const float2 r = p2_split(p2_fma(p2_of(-div, -div), q, v));
+        v = p2_fma(p2_of(fmaxf(r.x, -3.402823466e38f), fmaxf(r.y, -3.402823466e38f)), inv2, q);
+        if (tail) v = p2_add(v, bias);
     }
-    // correctly rounded v / div without the division sequence (see window3_strip_kernel)
-    const float q0 = v0 * inv, q1 = v1 * inv;
-    const float r0 = fmaf(-div, q0, v0), r1 = fmaf(-div, q1, v1);
-    v0 = fabsf(q0) <= 3.0e38f ? fmaf(r0, inv, q0) : q0;
-    v1 = fabsf(q1) <= 3.0e38f ? fmaf(r1, inv, q1) : q1;
-    return bits_of(__floats2bfloat162_rn(v0, v1));
+    const float2 f = p2_split(v);
+    uint32_t h;
+    if (kAct >= 1) asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(f.y), "f"(f.x));
+    else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(f.y), "f"(f.x));
+    if (kAct == 2) h = bits_of(__hmin2(bf2_of(h), bf2_of(0x40c040c0u)));          // (6, 6)
+    return h;
 }
 template <int kMode, int kAct>
-__device__ __forceinline__ uint32_t win_finish(uint32_t acc, float, float, float, float) { return acc; }
+__device__ __forceinline__ uint32_t win_finish(uint32_t acc, uint64_t bias, float, float, bool tail) {
+    if (tail) {
+        const float2 f = p2_split(p2_add(p2_bf16(acc), bias));
+        acc = bits_of(__floats2bfloat162_rn(f.x, f.y));
+    }
+    __nv_bfloat162 h = bf2_of(acc);
+    if (kAct >= 1) h = __hmax2(h, bf2_of(0u));
+    if (kAct == 2) h = __hmin2(h, bf2_of(0x40c040c0u));
+    return bits_of(h);
+}
 
-// ---- 3x3 windows over large tensors, staged through shared memory ---------------------------------------
-// Reading the rows with 4-byte global loads spends a third of the instructions on addresses (every load needs
-// its own 64-bit address; measured on a first version that did so).  Here a block of 8 warps owns a tile of kTileRows x (8 * strip) outputs of ONE slab of
-// 64 channels.  It first copies the tile's input window into shared memory with 16-byte cp.async (zero-filled
-// outside the tensor; 65 KB in flight per block, three blocks per SM), then every warp walks down its strip of output columns with
-// lane l holding channels 2l, 2l+1 of the slab: all its shared-memory loads are at compile-time offsets from
-// one pointer that advances once per three rows, and consecutive lanes read consecutive words (no bank
-// conflict).  The results are the bits of every other 3x3 kernel here.
-constexpr int kTileSlab = 64;                       // channels per block
-#ifndef PB_TILE_ROWS1
-#define PB_TILE_ROWS1 13
-#endif
-#ifndef PB_TILE_ROWS2
-#define PB_TILE_ROWS2 6
-#endif
-#ifndef PB_TILE_BLOCKS
-#define PB_TILE_BLOCKS 3
-#endif
-constexpr int kTileRows1 = PB_TILE_ROWS1, kTileRows2 = PB_TILE_ROWS2;      // output rows per block at stride 1 / 2
-
-template <int kStride> struct TileGeom {
-    static constexpr int kStrip = kStride == 1 ? kTileStrip1 : kTileStrip2;
-    static constexpr int kRows = kStride == 1 ? kTileRows1 : kTileRows2;
-    static constexpr int kOutCols = 8 * kStrip;
-    static constexpr int kInCols = (kOutCols - 1) * kStride + 3;
-    static constexpr int kInRows = (kRows - 1) * kStride + 3;
-    static constexpr int kSmemBytes = kInRows * kInCols * kTileSlab * 2;
-};
-
-template <int kMode, int kStride>
-__global__ void __launch_bounds__(256, PB_TILE_BLOCKS) window3_tile_kernel(OpArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
+template <int kMode, int kStride, int kAct, bool kCountPad>
+__global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t* err_flag, uint32_t job_id,
+                                                                        FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
     typedef __nv_bfloat16 T;
-    typedef TileGeom<kStride> G;
     typedef typename WinAcc<kMode>::type Acc;
-    constexpr int kStrip = G::kStrip, kCols = (kStrip - 1) * kStride + 3;
+    constexpr int kStrip = kStride == 1 ? kTileStrip1 : kTileStrip2, kCols = (kStrip - 1) * kStride + 3;
     constexpr bool kDw = kMode == kWinDw;
-    extern __shared__ __align__(16) unsigned char s_tile[];
+    extern __shared__ __align__(128) unsigned char s_tile[];
+    __shared__ __align__(8) uint64_t s_full;
 
     const int slabs = (a.Cs + kTileSlab - 1) / kTileSlab;
-    const int col_tiles = (a.Q + G::kOutCols - 1) / G::kOutCols;
     int b = blockIdx.x;
     const int slab = b % slabs; b /= slabs;
-    const int q_tile = (b % col_tiles) * G::kOutCols;
-    const int p_tile = (b / col_tiles) * G::kRows;
+    const int q_tile = (b % g.col_tiles) * g.strips * kStrip;
+    const int p_tile = (b / g.col_tiles) * g.rows;
+    const int p_end = min(p_tile + g.rows, a.P);
     const int ih0 = p_tile * kStride - a.pad_h, iw0 = q_tile * kStride - a.pad_w;
     const int ch0 = slab * kTileSlab;
 
-    // ---- fill: pixel (r, c) of the window is 8 vectors of 8 channels.  A thread keeps its eighth of the pixel and
-    // moves 32 pixels on per turn (the window is at least 32 pixels wide: at most one row wrap per turn). ----
-    {
-        static_assert(G::kInCols >= 32, "one row wrap per turn of the fill");
-        const T* __restrict__ x = x_img<T>(a);
-        const int ch = ch0 + (threadIdx.x & 7) * 8;
-        const bool ch_ok = ch < a.Cs;
-        int pix = threadIdx.x >> 3;
-        int r = pix / G::kInCols, c = pix - r * G::kInCols;
-        uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tile) + threadIdx.x * 16u;
-        for (; pix < G::kInRows * G::kInCols; pix += 32, dst += 32u * 128u) {
-            const int ih = ih0 + r, iw = iw0 + c;
-            const bool ok = ch_ok && (unsigned)ih < (unsigned)a.H && (unsigned)iw < (unsigned)a.W;
-            if (kMode == kWinMax && !ok) {
-                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0xff80ff80u) : "memory");
-            } else {
-                const T* src = ok ? x + (size_t)(ih * a.W + iw) * a.Cs + ch : x;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
-            }
-            c += 32;
-            if (c >= G::kInCols) { c -= G::kInCols; ++r; }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_full);
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(g.in_rows * g.in_cols * kTileSlab * 2) : "memory");
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(s_tile)), "l"(&tmap), "r"(ch0), "r"(iw0), "r"(ih0), "r"((int)blockIdx.y), "r"(bar)
+                     : "memory");
     }
 
-    // ---- walk: warp = strip of output columns, lane = channel pair ----
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c0 = ch0 + lane * 2;
-    const int q0 = q_tile + warp * kStrip;
-    if (c0 < a.Cs && q0 < a.Q) {
-        const Acc neutral = win_neutral<kMode>();
-        f2_t w[3][3];
-        float b0 = 0.f, b1 = 0.f;
+    const int half = threadIdx.x >> 4, c0 = ch0 + (threadIdx.x & 15) * 4;      // half-warp, first of the lane's four channels
+    const bool ch_in = c0 < a.Cs;
+    const int c_lim = kDw ? a.K : a.C;
+    uint64_t w[3][3][2], bias[2] = {0, 0};
+    if (kDw) {
+        const T* wp = static_cast<const T*>(a.w) + (ch_in ? c0 : 0);
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int s2 = 0; s2 < 3; ++s2) w[r][s2] = f2_pack(0.f, 0.f);
-        if (kDw) {
-            const T* wp = static_cast<const T*>(a.w) + c0;
+            for (int s2 = 0; s2 < 3; ++s2) {
+                const uint2 u = __ldg(reinterpret_cast<const uint2*>(wp + (r * 3 + s2) * a.Cs));
+                w[r][s2][0] = p2_bf16(u.x);
+                w[r][s2][1] = p2_bf16(u.y);
+            }
+    }
+    const bool tail = !kDw && a.bias != nullptr;
+    if (a.bias) {
+        float f[4];
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int s2 = 0; s2 < 3; ++s2) w[r][s2] = pair_of(__ldg(reinterpret_cast<const uint32_t*>(wp + (r * 3 + s2) * a.Cs)));
-            if (a.bias) { b0 = c0 < a.K ? a.bias[c0] : 0.f; b1 = c0 + 1 < a.K ? a.bias[c0 + 1] : 0.f; }
+        for (int j = 0; j < 4; ++j) f[j] = c0 + j < c_lim ? a.bias[c0 + j] : 0.f;
+        bias[0] = p2_of(f[0], f[1]);
+        bias[1] = p2_of(f[2], f[3]);
+    }
+    // channels past the last one are stored as zeros
+    const uint32_t keep0 = c0 + 1 < c_lim ? 0xffffffffu : (c0 < c_lim ? 0x0000ffffu : 0u);
+    const uint32_t keep1 = c0 + 3 < c_lim ? 0xffffffffu : (c0 + 2 < c_lim ? 0x0000ffffu : 0u);
+    const float inv9 = 1.f / 9.f;
+    const int pitch = g.in_cols * (kTileSlab / 4);                             // 8-byte words per window row
+    __syncthreads();                                                           // the barrier exists
+    bool landed = false;
+    for (int i = 0; i < (1 << 22) && !landed; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
+        landed = ok != 0;
+    }
+    if (!landed) {          // the copy is given 50 us more to land before shared memory is released
+        if (threadIdx.x == 0) atomicExch(err_flag, 5u);
+        unsigned long long t0, t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        for (int i = 0; i < (1 << 20); ++i) {
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t - t0 > 50000ull) break;
         }
-        const int nt = min(kStrip, a.Q - q0);
-        const int c_lim = kDw ? a.K : a.C;
-        const uint32_t keep = c0 + 1 < c_lim ? 0xffffffffu : (c0 < c_lim ? 0x0000ffffu : 0u);
-        const int p_end = min(p_tile + G::kRows, a.P);
-        const bool count_pad = (a.flags & 1) != 0;
-        const float inv9 = 1.f / 9.f;
-        T* __restrict__ y = y_img<T>(a) + a.out_c_off + c0;
-        // word (r, col) of this thread: s_row[r * kRowWords + col * 32]
-        constexpr int kRowWords = G::kInCols * (kTileSlab / 2);
-        const uint32_t* s_row = reinterpret_cast<const uint32_t*>(s_tile) + (warp * kStrip * kStride) * (kTileSlab / 2) + lane;
+    }
 
-        auto load_row = [&](int r, Acc (&xv)[kCols]) {
-#pragma unroll
-            for (int col = 0; col < kCols; ++col) xv[col] = win_value<kMode>(s_row[r * kRowWords + col * (kTileSlab / 2)]);
-        };
-        auto row_into = [&](Acc (&acc)[kStrip], const Acc (&xv)[kCols], int r) {
+    // ---- walk ----
+    const int units = landed ? g.strips * g.bands : 0;
+    for (int u0 = 0; u0 + (half & ~1) < units; u0 += blockDim.x / 16) {      // both halves of a warp take the same turns
+        const int unit = min(u0 + half, units - 1);
+        const int band = unit / g.strips, strip = unit - band * g.strips;
+        const int q0 = q_tile + strip * kStrip;
+        const int p0 = p_tile + band * g.band_rows, p1 = min(p0 + g.band_rows, p_end);
+        const int nt = u0 + half < units && ch_in ? min(kStrip, a.Q - q0) : 0;      // outputs this lane stores
+        const bool full = nt == kStrip && (keep0 & keep1) == 0xffffffffu;           // every output of the strip and all four channels exist
+        const uint2* row = reinterpret_cast<const uint2*>(s_tile) + (band * g.band_rows * kStride) * pitch + strip * kStrip * kStride * (kTileSlab / 4) + (threadIdx.x & 15);
+        T* __restrict__ y = y_img<T>(a) + ((size_t)p0 * a.Q + q0) * a.Ks + a.out_c_off + c0;
+
+        auto row_into = [&](Acc (&acc)[kStrip][2], const Acc (&xv)[kCols][2], int r) {
 #pragma unroll
             for (int t = 0; t < kStrip; ++t)
 #pragma unroll
-                for (int s2 = 0; s2 < 3; ++s2) acc[t] = win_step(acc[t], xv[t * kStride + s2], w[r][s2], kDw);
-        };
-        const bool full = nt == kStrip && keep == 0xffffffffu;      // every output of the strip and both channels exist
-        // one output row of the strip; ACT and FULL are literals so that the loop body carries no test of them
-#define PB_TILE_STORE_ROW(ACT, FULL)                                                                                             \
-    do {                                                                                                                         \
-        _Pragma("unroll") for (int t = 0; t < kStrip; ++t) {                                                                     \
-            if (!(FULL) && t >= nt) break;                                                                                       \
-            if (kMode == kWinAvg && !count_pad) {                                                                                \
-                const int cols_in = max(min((q0 + t) * kStride - a.pad_w + 3, a.W) - max((q0 + t) * kStride - a.pad_w, 0), 0);   \
-                const int cnt = rows_in * cols_in;                                                                               \
-                if (cnt != 9) { div = (float)(cnt > 0 ? cnt : 1); inv = 1.f / div; }                                             \
-                else { div = 9.f; inv = inv9; }                                                                                  \
-            }                                                                                                                    \
-            const uint32_t o = win_finish<kMode, ACT>(acc[t], b0, b1, div, inv);                                                \
-            *reinterpret_cast<uint32_t*>(yrow + (size_t)t * a.Ks) = (FULL) ? o : (o & keep);                                     \
-        }                                                                                                                        \
-    } while (0)
-        auto close_row = [&](Acc (&acc)[kStrip], int p) {
-            if (p >= p_tile && p < p_end) {
-                int rows_in = 3;
-                float div = 9.f, inv = inv9;
-                if (kMode == kWinAvg && !count_pad) rows_in = min(p * kStride - a.pad_h + 3, a.H) - max(p * kStride - a.pad_h, 0);
-                T* yrow = y + ((size_t)p * a.Q + q0) * a.Ks;
-                const int act = kDw ? a.act : 0;
-                if (full) {
-                    if (act == 2) PB_TILE_STORE_ROW(2, true);
-                    else if (act == 1) PB_TILE_STORE_ROW(1, true);
-                    else PB_TILE_STORE_ROW(0, true);
-                } else {
-                    if (act == 2) PB_TILE_STORE_ROW(2, false);
-                    else if (act == 1) PB_TILE_STORE_ROW(1, false);
-                    else PB_TILE_STORE_ROW(0, false);
+                for (int s2 = 0; s2 < 3; ++s2) {
+                    if (r == 0 && s2 == 0) {
+                        acc[t][0] = win_open(xv[t * kStride][0], w[0][0][0], kDw);
+                        acc[t][1] = win_open(xv[t * kStride][1], w[0][0][1], kDw);
+                        continue;
+                    }
+                    acc[t][0] = win_step(acc[t][0], xv[t * kStride + s2][0], w[r][s2][0], kDw);
+                    acc[t][1] = win_step(acc[t][1], xv[t * kStride + s2][1], w[r][s2][1], kDw);
                 }
-            }
-#pragma unroll
-            for (int t = 0; t < kStrip; ++t) acc[t] = neutral;
         };
-#undef PB_TILE_STORE_ROW
+        auto load_row = [&](Acc (&xv)[kCols][2]) {
+#pragma unroll
+            for (int col = 0; col < kCols; ++col) {
+                const uint2 v = row[col * (kTileSlab / 4)];
+                xv[col][0] = win_value<kMode>(v.x);
+                xv[col][1] = win_value<kMode>(v.y);
+            }
+            row += pitch;
+        };
+        auto store_row = [&](const Acc (&acc)[kStrip][2], int p, bool all) {
+            float div = 9.f, inv = inv9;
+            int rows_in = 3;
+            if (kMode == kWinAvg && !kCountPad) rows_in = min(p * kStride - a.pad_h + 3, a.H) - max(p * kStride - a.pad_h, 0);
+#pragma unroll
+            for (int t = 0; t < kStrip; ++t) {
+                if (!all && t >= nt) break;
+                if (kMode == kWinAvg && !kCountPad) {
+                    const int cols_in = max(min((q0 + t) * kStride - a.pad_w + 3, a.W) - max((q0 + t) * kStride - a.pad_w, 0), 0);
+                    const int cnt = rows_in * cols_in;
+                    if (cnt != 9) { div = (float)(cnt > 0 ? cnt : 1); inv = 1.f / div; }
+                    else { div = 9.f; inv = inv9; }
+                }
+                uint32_t o0 = win_finish<kMode, kAct>(acc[t][0], bias[0], div, inv, tail);
+                uint32_t o1 = win_finish<kMode, kAct>(acc[t][1], bias[1], div, inv, tail);
+                if (!all) { o0 &= keep0; o1 &= keep1; }
+                *reinterpret_cast<uint2*>(y + (uint32_t)(t * a.Ks)) = make_uint2(o0, o1);
+            }
+            y += (size_t)a.Q * a.Ks;
+        };
+        // output rows are closed in order: p is the one after the last closed, rows before p0 and from p1 on are not stored
+        auto close_row = [&](const Acc (&acc)[kStrip][2], int p) {
+            if (p >= p0 && p < p1) {
+                if (full) store_row(acc, p, true);
+                else store_row(acc, p, false);
+            }
+        };
 
         if (kStride == 1) {
-            // window row r opens output row p_tile + r (filter row 0), continues p_tile + r - 1, closes p_tile + r - 2
-            Acc accA[kStrip], accB[kStrip], accC[kStrip];
+            // window row r opens output row p0 + r (filter row 0), continues p0 + r - 1, closes p0 + r - 2; three window rows per
+            // turn (the last turn may run past the band, into rows that are not stored)
+            Acc accA[kStrip][2], accB[kStrip][2], accC[kStrip][2];
 #pragma unroll
-            for (int t = 0; t < kStrip; ++t) accA[t] = accB[t] = accC[t] = neutral;
-            static_assert(kStride != 1 || G::kInRows % 3 == 0, "the stride-1 walk takes three window rows per turn");
+            for (int t = 0; t < kStrip; ++t)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) accB[t][j] = accC[t][j] = 0;          // (rows before p0: never stored)
 #pragma unroll 1
-            for (int r = 0; r < G::kInRows; r += 3) {
-                Acc xv[kCols];
-                load_row(r, xv);     row_into(accB, xv, 2); row_into(accC, xv, 1); row_into(accA, xv, 0); close_row(accB, p_tile + r - 2);
-                load_row(r + 1, xv); row_into(accC, xv, 2); row_into(accA, xv, 1); row_into(accB, xv, 0); close_row(accC, p_tile + r - 1);
-                load_row(r + 2, xv); row_into(accA, xv, 2); row_into(accB, xv, 1); row_into(accC, xv, 0); close_row(accA, p_tile + r);
+            for (int p = p0; p < p1 + 2; p += 3) {
+                Acc xv[kCols][2];
+                load_row(xv); row_into(accB, xv, 2); row_into(accC, xv, 1); row_into(accA, xv, 0); close_row(accB, p - 2);
+                load_row(xv); row_into(accC, xv, 2); row_into(accA, xv, 1); row_into(accB, xv, 0); close_row(accC, p - 1);
+                load_row(xv); row_into(accA, xv, 2); row_into(accB, xv, 1); row_into(accC, xv, 0); close_row(accA, p);
             }
         } else {
-            // window row r: even r closes output row p_tile + r/2 - 1 (filter row 2) and opens p_tile + r/2 (row 0);
-            // odd r is filter row 1 of p_tile + (r - 1)/2
-            Acc acc[kStrip];
+            // window row 2i closes output row p0 + i - 1 (filter row 2) and opens p0 + i (row 0); row 2i + 1 is filter row 1 of p0 + i
+            Acc acc[kStrip][2];
 #pragma unroll
-            for (int t = 0; t < kStrip; ++t) acc[t] = neutral;
+            for (int t = 0; t < kStrip; ++t) acc[t][0] = acc[t][1] = 0;
 #pragma unroll 1
-            for (int r = 0; r + 1 < G::kInRows; r += 2) {
-                Acc xv[kCols];
-                load_row(r, xv);     row_into(acc, xv, 2); close_row(acc, p_tile + r / 2 - 1); row_into(acc, xv, 0);
-                load_row(r + 1, xv); row_into(acc, xv, 1);
+            for (int p = p0; p < p1; ++p) {
+                Acc xv[kCols][2];
+                load_row(xv); row_into(acc, xv, 2); close_row(acc, p - 1); row_into(acc, xv, 0);
+                load_row(xv); row_into(acc, xv, 1);
             }
-            Acc xv[kCols];
-            load_row(G::kInRows - 1, xv);
+            Acc xv[kCols][2];
+            load_row(xv);
             row_into(acc, xv, 2);
-            close_row(acc, p_tile + (G::kInRows - 1) / 2 - 1);
+            close_row(acc, p1 - 1);
         }
     }
     PB_NOTIFY_END();
@@ -1210,6 +1253,41 @@ static size_t strip_threads(const pb_op_params* p, int strip) {
     return (size_t)p->P * ((p->Q + strip - 1) / strip) * (p->Cs / vec_n(p->dtype));
 }
 
+// Tile of window3_tile_kernel.  A single image is cut into tiles of 8 strips x 13 (stride 2: 6) rows, 65 KB of window.  The
+// images of a batch are mostly small maps, where that tile hangs over the edges (35 columns: a tile of 32 and one of 3, 101 us
+// for 256 images of 35 x 35 x 192 instead of 51), so their tiles are fitted to the map: as few column tiles as hold at most 40 columns
+// each, as many rows as keep the window within 70 KB, and bands of rows where a map has fewer strips than half-warps.
+static WinTile win_tile(const pb_op_params* p) {
+    const int st = p->stride_h, strip = st == 1 ? kTileStrip1 : kTileStrip2;
+    WinTile g;
+    if (batch_of(p) == 1) {
+        g.strips = 8;
+        g.col_tiles = ceil_div(p->Q, g.strips * strip);
+        g.rows = st == 1 ? kTileRows1 : kTileRows2;
+    } else {
+        const int n = ceil_div(p->Q, st == 1 ? 40 : 20);
+        g.strips = ceil_div(ceil_div(p->Q, n), strip);
+        g.col_tiles = ceil_div(p->Q, g.strips * strip);
+    }
+    g.in_cols = (g.strips * strip - 1) * st + 3;
+    if (batch_of(p) > 1) {
+        int fit = ((74 * 1024) / (g.in_cols * kTileSlab * 2) - 3) / st + 1;      // rows of output whose window fits
+        if (fit < 1) fit = 1;
+        g.rows = p->P < fit ? p->P : fit;
+        if (st == 1 && fit < p->P && fit > 3) g.rows = (fit - 1) / 3 * 3 + 1;     // a walk takes three window rows per turn: no turn half used
+    }
+    g.bands = g.strips >= 8 ? 1 : (8 / g.strips < g.rows ? 8 / g.strips : g.rows);
+    g.band_rows = ceil_div(g.rows, g.bands);
+    g.bands = ceil_div(g.rows, g.band_rows);
+    const int walked = st == 1 ? ceil_div(g.band_rows + 2, 3) * 3 : 2 * g.band_rows + 1;      // window rows a unit reads
+    g.alloc_rows = (g.bands - 1) * g.band_rows * st + walked;
+    g.in_rows = (g.rows - 1) * st + 3;
+    g.alloc_rows = g.alloc_rows > g.in_rows ? g.alloc_rows : g.in_rows;
+    g.threads = 32 * ceil_div(g.strips * g.bands < 10 ? g.strips * g.bands : 10, 2);
+    g.smem = g.alloc_rows * g.in_cols * kTileSlab * 2;
+    return g;
+}
+
 // Blocks of window3_tile_kernel for one image, or 0 when the layer keeps the strip kernels: bf16, a 3x3 window of stride 1
 // or 2, and at least 100 blocks in the launch (all images).  Measured on Inception-v3 served in gangs of 8: thresholds of
 // 30, 100 and 300 blocks give the same +2 % requests/s over 592 (its two stem max pools then run here); below 100 a lone
@@ -1217,23 +1295,38 @@ static size_t strip_threads(const pb_op_params* p, int strip) {
 // PB_WINDOW_TILE=0 switches it off; PB_WINDOW_TILE_MIN_BLOCKS sets another threshold (tests use 1).  Read at every call:
 // this runs when a launch is built (graph capture, direct operator calls), never on the replay path.
 static uint32_t tile_blocks(const pb_op_params* p) {
-    if (p->groups <= 1 && (p->bias != nullptr || p->act != 0)) return 0;      // pooling with a bias / activation tail: strip kernels
-    if (p->dtype != 1 || (p->Cs & 7) || (p->Ks & 1) || (p->out_c_off & 1) || strip_of(p) == 0) return 0;
+    if (p->dtype != 1 || (p->Cs & 7) || (p->Ks & 3) || (p->out_c_off & 3) || p->act > 2 || strip_of(p) == 0) return 0;
     const char* e = getenv("PB_WINDOW_TILE");
     if (e && e[0] == '0') return 0;
     size_t least = 100;
     if (const char* m = getenv("PB_WINDOW_TILE_MIN_BLOCKS")) least = (size_t)strtoull(m, nullptr, 10);
-    const int rows = p->stride_h == 1 ? TileGeom<1>::kRows : TileGeom<2>::kRows;
-    const int cols = p->stride_h == 1 ? TileGeom<1>::kOutCols : TileGeom<2>::kOutCols;
-    const size_t n = (size_t)((p->Cs + kTileSlab - 1) / kTileSlab) * ((p->Q + cols - 1) / cols) * ((p->P + rows - 1) / rows);
+    const WinTile g = win_tile(p);
+    const size_t n = (size_t)((p->Cs + kTileSlab - 1) / kTileSlab) * g.col_tiles * ((p->P + g.rows - 1) / g.rows);
     return n * (size_t)batch_of(p) >= least ? (uint32_t)n : 0;
 }
-static const void* tile_fn(int kind, int stride) {
-#define PB_TILE(M) (stride == 1 ? (const void*)window3_tile_kernel<M, 1> : (const void*)window3_tile_kernel<M, 2>)
-    return kind == PB_STAGE_DWCONV ? PB_TILE(kWinDw) : kind == PB_STAGE_MAXPOOL ? PB_TILE(kWinMax) : PB_TILE(kWinAvg);
+// Window map of a launch: boxes of one slab x in_cols x in_rows of the images.
+static int win_map(int kind, const pb_op_params* p, const WinTile& g, CUtensorMap* out, uint32_t** err_flag) {
+    int device = 0;
+    PB_CUDA(cudaGetDevice(&device));
+    *err_flag = device_error_flag_ptr(device);
+    PB_REQUIRE(*err_flag != nullptr, "window kernel: no device error flag");
+    const uint64_t dims[4] = {(uint64_t)p->Cs, (uint64_t)p->W, (uint64_t)p->H, (uint64_t)batch_of(p)};
+    const uint64_t strides[3] = {(uint64_t)p->Cs * 2, (uint64_t)p->W * p->Cs * 2, (uint64_t)p->H * p->W * p->Cs * 2};
+    const uint32_t box[4] = {(uint32_t)kTileSlab, (uint32_t)g.in_cols, (uint32_t)g.in_rows, 1};
+    return encode_tiled_bf16(p->x, 4, dims, strides, box, kind == PB_STAGE_MAXPOOL, out);
+}
+template <int kMode, bool kCountPad>
+static const void* tile_fn(int stride, int act) {
+#define PB_TILE(S) (act == 2 ? (const void*)window3_tile_kernel<kMode, S, 2, kCountPad> : act == 1 ? (const void*)window3_tile_kernel<kMode, S, 1, kCountPad> \
+                                                                                  : (const void*)window3_tile_kernel<kMode, S, 0, kCountPad>)
+    return stride == 1 ? PB_TILE(1) : PB_TILE(2);
 #undef PB_TILE
 }
-static uint32_t tile_smem(int stride) { return stride == 1 ? TileGeom<1>::kSmemBytes : TileGeom<2>::kSmemBytes; }
+static const void* tile_fn(int kind, const pb_op_params* p) {
+    if (kind == PB_STAGE_DWCONV) return tile_fn<kWinDw, true>(p->stride_h, p->act);
+    if (kind == PB_STAGE_MAXPOOL) return tile_fn<kWinMax, true>(p->stride_h, p->act);
+    return (p->flags & 1) ? tile_fn<kWinAvg, true>(p->stride_h, p->act) : tile_fn<kWinAvg, false>(p->stride_h, p->act);
+}
 
 template <int kMode>
 static const void* window3_fn(bool f32, int stride, int strip) {
@@ -1293,8 +1386,9 @@ static int info_one_image(int kind, const pb_op_params* p, pb_launch_info* out) 
             }
             if (const uint32_t nblk = tile_blocks(p)) {
                 out->num_blocks = nblk;
-                out->regs_per_thread = regs_of(tile_fn(kind, p->stride_h));
-                out->smem_per_block = tile_smem(p->stride_h);
+                out->regs_per_thread = regs_of(tile_fn(kind, p));
+                out->smem_per_block = (uint32_t)win_tile(p).smem;
+                out->threads_per_block = (uint32_t)win_tile(p).threads;
             }
             out->flops = 2ull * out_elems * p->R * p->S;
             out->bytes = es * (in_elems + (size_t)p->K * p->R * p->S + out_elems) + 4ull * p->K;
@@ -1312,8 +1406,9 @@ static int info_one_image(int kind, const pb_op_params* p, pb_launch_info* out) 
             }
             if (const uint32_t nblk = tile_blocks(p)) {
                 out->num_blocks = nblk;
-                out->regs_per_thread = regs_of(tile_fn(kind, p->stride_h));
-                out->smem_per_block = tile_smem(p->stride_h);
+                out->regs_per_thread = regs_of(tile_fn(kind, p));
+                out->smem_per_block = (uint32_t)win_tile(p).smem;
+                out->threads_per_block = (uint32_t)win_tile(p).threads;
             }
             out->bytes = es * (in_elems + out_elems) + (p->bias ? 4ull * p->K : 0);
             break;
@@ -1459,10 +1554,15 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
             PB_REQUIRE(a.groups == a.C && a.K == a.C, "dwconv: needs groups == C == K");
             PB_REQUIRE((a.Ks % N) == 0 && (a.out_c_off % N) == 0, "dwconv: output slice must be vector aligned");
             if (tile_blocks(p)) {
-                const void* fn = tile_fn(kind, p->stride_h);
-                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(p->stride_h)));
-                t_launch_smem = tile_smem(p->stride_h);
-                launch_k((void (*)(OpArgs, uint32_t, FinishedBlockNotifier*))fn, grid, block, st, pdl, a, job_id, nf);
+                const WinTile g = win_tile(p);
+                const void* fn = tile_fn(kind, p);
+                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
+                t_launch_smem = (size_t)g.smem;
+                CUtensorMap tmap;
+                uint32_t* err_flag = nullptr;
+                const int mrc = win_map(kind, p, g, &tmap, &err_flag);
+                if (mrc != PB_OK) return mrc;
+                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t*, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, err_flag, job_id, nf);
                 break;
             }
             if (const int strip = strip_of(p)) {
@@ -1475,10 +1575,15 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
         case PB_STAGE_MAXPOOL:
             PB_REQUIRE((a.Ks % N) == 0 && (a.out_c_off % N) == 0, "pool: output slice must be vector aligned");
             if (tile_blocks(p)) {
-                const void* fn = tile_fn(kind, p->stride_h);
-                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(p->stride_h)));
-                t_launch_smem = tile_smem(p->stride_h);
-                launch_k((void (*)(OpArgs, uint32_t, FinishedBlockNotifier*))fn, grid, block, st, pdl, a, job_id, nf);
+                const WinTile g = win_tile(p);
+                const void* fn = tile_fn(kind, p);
+                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
+                t_launch_smem = (size_t)g.smem;
+                CUtensorMap tmap;
+                uint32_t* err_flag = nullptr;
+                const int mrc = win_map(kind, p, g, &tmap, &err_flag);
+                if (mrc != PB_OK) return mrc;
+                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t*, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, err_flag, job_id, nf);
                 break;
             }
             if (const int strip = strip_of(p)) {
@@ -1490,10 +1595,15 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
         case PB_STAGE_AVGPOOL:
             PB_REQUIRE((a.Ks % N) == 0 && (a.out_c_off % N) == 0, "pool: output slice must be vector aligned");
             if (tile_blocks(p)) {
-                const void* fn = tile_fn(kind, p->stride_h);
-                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(p->stride_h)));
-                t_launch_smem = tile_smem(p->stride_h);
-                launch_k((void (*)(OpArgs, uint32_t, FinishedBlockNotifier*))fn, grid, block, st, pdl, a, job_id, nf);
+                const WinTile g = win_tile(p);
+                const void* fn = tile_fn(kind, p);
+                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
+                t_launch_smem = (size_t)g.smem;
+                CUtensorMap tmap;
+                uint32_t* err_flag = nullptr;
+                const int mrc = win_map(kind, p, g, &tmap, &err_flag);
+                if (mrc != PB_OK) return mrc;
+                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t*, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, err_flag, job_id, nf);
                 break;
             }
             if (const int strip = strip_of(p)) {

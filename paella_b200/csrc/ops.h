@@ -1,6 +1,7 @@
 // Internal operator interface shared by the kernel translation units.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -39,6 +40,9 @@ int conv_f32_info(const pb_op_params* p, pb_launch_info* out);
 int64_t conv_f32_pack_weights(const pb_op_params* p, const float* w_oihw, void* dst_host);
 int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);
 double conv_split_gain_us();      // see pb_set_conv_split_gain_us
+
+// Tensor map of a bf16 tensor without swizzle; elements outside read as zeros, or as NaN.
+int encode_tiled_bf16(const void* base, int rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, bool nan_fill, CUtensorMap* out);
 
 // conv_umma.cu: tcgen05 implicit-GEMM convolution (bf16 operands, fp32 accumulation in TMEM)
 bool conv_umma_supported(const pb_op_params* p);

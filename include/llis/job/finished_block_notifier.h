@@ -29,7 +29,7 @@ class FinishedBlockNotifier {
     __device__ __forceinline__ void start(JobId job_id) {
         if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
             const unsigned g = gridDim.x * gridDim.y * gridDim.z;
-            const unsigned total = atomicInc(&agg_counter_start_, g - 1) + 1;
+            const unsigned total = g == 1 ? 1 : atomicInc(&agg_counter_start_, g - 1) + 1;      // a lone block's ticket is always the first
             const unsigned batch = total % noti_batch_size_;
             if (batch == 0) {
                 channel_.write(InstrumentInfo::kStart, 0, (uint8_t)noti_batch_size_, job_id, false);
@@ -44,7 +44,7 @@ class FinishedBlockNotifier {
         if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
             const unsigned g = gridDim.x * gridDim.y * gridDim.z;
             __threadfence();
-            const unsigned total = atomicInc(&agg_counter_end_, g - 1) + 1;
+            const unsigned total = g == 1 ? 1 : atomicInc(&agg_counter_end_, g - 1) + 1;
             const unsigned batch = total % noti_batch_size_;
             if (batch == 0 || total == g) {
                 __threadfence();

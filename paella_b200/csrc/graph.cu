@@ -183,9 +183,12 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
                 lm = lb * pf.tmem_cols_per_block;
             }
         }
-        thr = std::max(thr, lt); smem = std::max(smem, ls); regs = std::max(regs, lr); tmem = std::max(tmem, lm);
+        if (getenv("PB_FOOT")) { thr += lt; smem += ls; regs += lr; tmem += lm; }
+        else {
+        thr = std::max(thr, lt); smem = std::max(smem, ls); regs = std::max(regs, lr); tmem = std::max(tmem, lm); }
         nb = lb;
     }
+    if (getenv("PB_FOOT")) { const double d = grp.launches.size() / atof(getenv("PB_FOOT")); thr = std::max<uint64_t>(nb, thr / d); smem /= d; regs /= d; tmem /= d; }
     out.kind = grp.count == 1 ? infos[(size_t)grp.first].kind : 0xFFFFu;
     out.num_blocks = (uint32_t)nb;
     out.threads_per_block = (uint32_t)pb::ceil_div<uint64_t>(thr, nb);

@@ -1107,8 +1107,14 @@ __global__ void __launch_bounds__(256) detect_kernel(OpArgs a, uint32_t job_id, 
 // ---- whole MNIST-CNN in one launch ---------------------------------------------------
 // conv5x5(1->8)+ReLU, maxpool2, conv5x5(8->16)+ReLU, maxpool3, dense 256->10 for one
 // 28x28 image, fp32, activations in shared memory.  One block of 256 threads: the network
-// is 1.57 MFLOP and 24 KB of weights, so the request is launch-latency bound and one
+// is 1.2 MFLOP (the outer two rows and columns of the second convolution are never pooled) and 24 KB of weights, so one
 // kernel (one start and one end record) replaces six.
+// A lone request is the serial chain of this block, so what counts is multiply-adds per word read from shared memory: a
+// thread owns all eight channels of a 2x2 pooling window of the first convolution (236 words for 800 multiply-adds) and two
+// channels of a 3x3 pooling window of the second, for half of its input channels (396 words for 1800).  With one output per
+// thread, two words per multiply-add, the kernel took 31 us.  Weights are on their way before the request's pointers have
+// been read (they and the image come from the host's memory), and warp 0 reports the block's start while the others fetch
+// the image.
 // Weights: w1 [5][5][1][8], w2 [5][5][8][16], wd [10][4*4*16] (h, w, c order), biases fp32.
 struct MnistArgs {
     const float* x;     // [28][28]
@@ -1118,78 +1124,152 @@ struct MnistArgs {
     float* y;           // [10]
 };
 
-__global__ void __launch_bounds__(256) mnist_fused_kernel(MnistArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
-    PB_NOTIFY_START();
-    // one block per image of the gang
-    a.x = (!a.x && slot_) ? slot_->io_in[blockIdx.x] : a.x + (size_t)blockIdx.x * 784;
-    a.y = (!a.y && slot_) ? slot_->io_out[blockIdx.x] : a.y + (size_t)blockIdx.x * 10;
-    __shared__ float s_in[32][33];          // 28x28 image with a 2-pixel zero border
-    __shared__ float s_w1[25 * 8];
-    __shared__ float s_p1[18][18][8];       // pool1 output 14x14x8 with a 2-pixel zero border
-    __shared__ float s_w2[25 * 8 * 16];
-    __shared__ float s_c2[14 * 14][17];     // conv2 output (padded row to dodge bank conflicts)
+__global__ void __launch_bounds__(256, 2) mnist_fused_kernel(MnistArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
+    constexpr int kInPitch = 34, kP1Pitch = 20, kP1Plane = 18 * kP1Pitch;
+    __shared__ __align__(16) float s_in[32 * kInPitch];       // 28x28 image with a 2-pixel zero border
+    __shared__ __align__(16) float s_w1[25 * 8];
+    __shared__ __align__(16) float s_p1[8 * kP1Plane];        // pool1 output, 8 planes of 14x14 with a 2-pixel zero border
+    __shared__ __align__(16) float s_w2[8 * 25 * 16];         // [channel][tap][16]
+    __shared__ __align__(16) float s_part[128 * 19];          // half of the second convolution's sums
     __shared__ float s_p2[256];
-    const int t = threadIdx.x;
-    for (int i = t; i < 32 * 33; i += 256) (&s_in[0][0])[i] = 0.f;
-    for (int i = t; i < 18 * 18 * 8; i += 256) (&s_p1[0][0][0])[i] = 0.f;
-    for (int i = t; i < 200; i += 256) s_w1[i] = a.w1[i];
-    for (int i = t; i < 3200; i += 256) s_w2[i] = a.w2[i];
-    __syncthreads();
-    for (int i = t; i < 784; i += 256) s_in[i / 28 + 2][i % 28 + 2] = a.x[i];
-    __syncthreads();
-    // conv1 + ReLU + 2x2 max pool: one thread per (pooled pixel, channel): 14*14*8 = 1568
-    for (int i = t; i < 1568; i += 256) {
-        const int k = i & 7, pp = i >> 3;
-        const int py = pp / 14, px = pp % 14;
-        float best = 0.f;  // ReLU output is >= 0
-        const float b = a.b1[k];
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx) {
-                float acc = b;
-                const int oy = 2 * py + dy, ox = 2 * px + dx;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    // the weights do not depend on the previous kernel or the request
+    float w2r[13], wdr[2][8];
 #pragma unroll
-                for (int r = 0; r < 5; ++r)
+    for (int i = 0; i < 13; ++i) w2r[i] = t + 256 * i < 3200 ? __ldg(a.w2 + t + 256 * i) : 0.f;
+    const float w1r = t < 200 ? __ldg(a.w1 + t) : 0.f;
 #pragma unroll
-                    for (int s = 0; s < 5; ++s) acc = fmaf(s_in[oy + r][ox + s], s_w1[(r * 5 + s) * 8 + k], acc);
-                best = fmaxf(best, acc);
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) wdr[h][j] = wid + 8 * h < 10 ? __ldg(a.wd + (wid + 8 * h) * 256 + lane + 32 * j) : 0.f;
+    for (int i = t; i < 32 * kInPitch; i += 256) s_in[i] = 0.f;
+    for (int i = t; i < 8 * kP1Plane; i += 256) s_p1[i] = 0.f;
+    pb::griddep_wait();
+    const pb::LaunchSlot* slot = pb::resolve_slot(job_id, nf);
+    // one block per image of the gang
+    const float* x = (!a.x && slot) ? slot->io_in[blockIdx.x] : a.x + (size_t)blockIdx.x * 784;
+    float* y = (!a.y && slot) ? slot->io_out[blockIdx.x] : a.y + (size_t)blockIdx.x * 10;
+    __syncthreads();                                          // the zeros are down
+    if (wid == 0) {
+        if (nf) nf->start(job_id);
+    } else if ((reinterpret_cast<uintptr_t>(x) & 7) == 0) {
+        for (int i = t - 32; i < 392; i += 224) {
+            const float2 v = reinterpret_cast<const float2*>(x)[i];
+            float* d = s_in + (i / 14 + 2) * kInPitch + (i % 14) * 2 + 2;
+            d[0] = v.x;
+            d[1] = v.y;
+        }
+    } else {
+        for (int i = t - 32; i < 784; i += 224) s_in[(i / 28 + 2) * kInPitch + i % 28 + 2] = x[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 13; ++i) {
+        const int e = t + 256 * i;
+        if (e < 3200) s_w2[((e >> 4 & 7) * 25 + (e >> 7)) * 16 + (e & 15)] = w2r[i];
+    }
+    if (t < 200) s_w1[t] = w1r;
+    __syncthreads();
+    // conv1 + ReLU + 2x2 max pool: one thread per pooled pixel, four channels at a time
+    if (t < 196) {
+        const int py = t / 14, px = t - py * 14;
+        float p[6][6];
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+#pragma unroll
+            for (int c = 0; c < 6; c += 2) {
+                const float2 v = *reinterpret_cast<const float2*>(s_in + (2 * py + r) * kInPitch + 2 * px + c);
+                p[r][c] = v.x;
+                p[r][c + 1] = v.y;
             }
-        s_p1[py + 2][px + 2][k] = best;
+        float* d = s_p1 + (py + 2) * kP1Pitch + px + 2;
+#pragma unroll 1
+        for (int kb = 0; kb < 8; kb += 4) {
+            float acc[4][4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[0][k] = acc[1][k] = acc[2][k] = acc[3][k] = __ldg(a.b1 + kb + k);
+#pragma unroll
+            for (int r = 0; r < 5; ++r)
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    const float4 w = *reinterpret_cast<const float4*>(s_w1 + (r * 5 + c) * 8 + kb);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float v = p[r + (q >> 1)][c + (q & 1)];
+                        acc[q][0] = fmaf(v, w.x, acc[q][0]);
+                        acc[q][1] = fmaf(v, w.y, acc[q][1]);
+                        acc[q][2] = fmaf(v, w.z, acc[q][2]);
+                        acc[q][3] = fmaf(v, w.w, acc[q][3]);
+                    }
+                }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)      // ReLU and pooling in one: the largest of the four and zero
+                d[(kb + k) * kP1Plane] = fmaxf(fmaxf(fmaxf(acc[0][k], acc[1][k]), fmaxf(acc[2][k], acc[3][k])), 0.f);
+        }
     }
     __syncthreads();
-    // conv2 + ReLU: one thread per (pixel, channel): 196*16 = 3136
-    for (int i = t; i < 3136; i += 256) {
-        const int k = i & 15, pp = i >> 4;
-        const int oy = pp / 14, ox = pp % 14;
-        float acc = a.b2[k];
-        for (int r = 0; r < 5; ++r)
-            for (int s = 0; s < 5; ++s) {
-                const float* ip = &s_p1[oy + r][ox + s][0];
-                const float* wp = &s_w2[((r * 5 + s) * 8) * 16 + k];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) acc = fmaf(ip[c], wp[c * 16], acc);
-            }
-        s_c2[pp][k] = fmaxf(acc, 0.f);
-    }
-    __syncthreads();
-    // 3x3/3 max pool (floor: 14 -> 4), output order (h, w, c)
+    // conv2 + ReLU + 3x3 max pool (floor: 14 -> 4): thread = (pooled pixel, pair of channels, half of the input channels)
     {
-        const int k = t & 15, pp = t >> 4;
-        const int py = pp >> 2, px = pp & 3;
-        float best = -INFINITY;
-        for (int dy = 0; dy < 3; ++dy)
-            for (int dx = 0; dx < 3; ++dx) best = fmaxf(best, s_c2[(3 * py + dy) * 14 + 3 * px + dx][k]);
-        s_p2[t] = best;
+        const int kp = t & 7, pix = (t >> 3) & 15, ch = (t >> 7) * 4;
+        const float* ip0 = s_p1 + ch * kP1Plane + (pix >> 2) * 3 * kP1Pitch + (pix & 3) * 3;
+        const float* wp0 = s_w2 + ch * 25 * 16 + kp * 2;
+        float acc[9][2];
+#pragma unroll
+        for (int o = 0; o < 9; ++o) acc[o][0] = acc[o][1] = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            float2 w[25];
+#pragma unroll
+            for (int j = 0; j < 25; ++j) w[j] = *reinterpret_cast<const float2*>(wp0 + c * 25 * 16 + j * 16);
+#pragma unroll
+            for (int r = 0; r < 7; ++r) {
+                float v[7];
+#pragma unroll
+                for (int j = 0; j < 7; ++j) v[j] = ip0[c * kP1Plane + r * kP1Pitch + j];
+#pragma unroll
+                for (int oy = 0; oy < 3; ++oy) {
+                    if (r - oy < 0 || r - oy > 4) continue;
+#pragma unroll
+                    for (int ox = 0; ox < 3; ++ox)
+#pragma unroll
+                        for (int j = 0; j < 5; ++j) {
+                            acc[oy * 3 + ox][0] = fmaf(v[ox + j], w[(r - oy) * 5 + j].x, acc[oy * 3 + ox][0]);
+                            acc[oy * 3 + ox][1] = fmaf(v[ox + j], w[(r - oy) * 5 + j].y, acc[oy * 3 + ox][1]);
+                        }
+                }
+            }
+        }
+        if (t >= 128) {
+#pragma unroll
+            for (int o = 0; o < 9; ++o) {
+                s_part[(t - 128) * 19 + o * 2] = acc[o][0];
+                s_part[(t - 128) * 19 + o * 2 + 1] = acc[o][1];
+            }
+        }
+        __syncthreads();
+        if (t < 128) {
+            float best0 = 0.f, best1 = 0.f;      // ReLU: at least zero
+            const float b0 = __ldg(a.b2 + kp * 2), b1 = __ldg(a.b2 + kp * 2 + 1);
+#pragma unroll
+            for (int o = 0; o < 9; ++o) {
+                best0 = fmaxf(best0, acc[o][0] + s_part[t * 19 + o * 2] + b0);
+                best1 = fmaxf(best1, acc[o][1] + s_part[t * 19 + o * 2 + 1] + b1);
+            }
+            s_p2[pix * 16 + kp * 2] = best0;
+            s_p2[pix * 16 + kp * 2 + 1] = best1;
+        }
     }
     __syncthreads();
     // dense 256 -> 10: warps 0..7 take rows w, w+8
-    {
-        const int lane = t & 31, wid = t >> 5;
-        for (int o = wid; o < 10; o += 8) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int o = wid + 8 * h;
+        if (o < 10) {
             float acc = 0.f;
-            for (int i = lane; i < 256; i += 32) acc = fmaf(s_p2[i], a.wd[o * 256 + i], acc);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc = fmaf(s_p2[lane + 32 * j], wdr[h][j], acc);
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-            if (lane == 0) a.y[o] = acc + a.bd[o];
+            if (lane == 0) y[o] = acc + __ldg(a.bd + o);
         }
     }
     PB_NOTIFY_END();
@@ -1701,7 +1781,7 @@ int mnist_fused_info(pb_launch_info* out) {
     out->threads_per_block = 256;
     out->regs_per_thread = regs_of(mnist_fused_kernel);
     out->smem_per_block = static_smem_of(mnist_fused_kernel);
-    out->flops = 2ull * (156800 + 627200 + 2560);
+    out->flops = 2ull * (156800 + 627200 + 2560);      // the layers as the model states them
     out->bytes = 4ull * (784 + 200 + 8 + 3200 + 16 + 2560 + 10 + 10);
     return PB_OK;
 }

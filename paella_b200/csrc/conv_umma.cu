@@ -180,6 +180,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+// The stores have read their shared memory / are in global memory.
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
@@ -227,6 +229,14 @@ __device__ __forceinline__ bool elect_one() {
 }
 // A value every lane of the warp agrees on, told to the compiler.
 __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
 // Thread-block cluster: barrier halves (every thread of every block of the cluster takes part), the address of
 // this block's shared memory word in block `rank`, a 16-byte load from it.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -242,9 +252,6 @@ __device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
-}
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 __device__ __forceinline__ void tcgen05_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -408,56 +415,54 @@ __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lan
     }
 }
 
-// The same with the tile leaving through TMA stores.  A warp's 16-byte stores touch 32 lines each: 128 columns are
-// 16 x 32 line accesses per warp, 2048 clocks of the SM's one store path per tile (1.9 us measured, and co-resident
-// tiles queue behind each other).  So each warp lays its 32 rows out in shared memory, boxes of U columns in the
-// swizzle of their row length (no bank conflicts), and one lane stores a finished box with one instruction.  `buf`: the
-// warp's 32 x BN x 2 bytes of the pipeline memory, free by now.
+// The same with the tile leaving, and the residual arriving, through TMA.  A warp's 16-byte accesses to its 32 rows touch 32
+// lines each: 128 columns are 16 x 32 line accesses per warp, 2048 clocks of the SM's one load / store path per tile
+// (1.9 us measured, and co-resident tiles queue behind each other; with a residual twice that: half of a ResNet-50 tile's life).
+// So the tile is laid out in shared memory, boxes of 128 rows x U columns in the swizzle of their row length (no bank
+// conflicts): the residual lands there before the accumulator is complete (s_res), each thread replaces its row's part by the
+// result, and one lane of a warp stores the warp's 32 rows of a finished box with one instruction.  `buf`: 128 x BN x 2 bytes
+// of the pipeline memory, free by now.  publish: this launch reports to the host, so the stores have to be in memory when the
+// warp leaves; otherwise they only have to have been read (the next kernel waits for this one's memory operations).
 template <int ACT>
-__device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t lane_addr, int n0, bool row_valid, const __nv_bfloat16* rrow,
-                                                     const float* s_bias, uint32_t buf, const CUtensorMap* tmap_y, int m_warp) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const int U = a.out_box;
-    const uint32_t swz = U == 64 ? lane & 7u : (lane >> 1) & 3u;
-    const uint32_t row = buf + lane * (uint32_t)(U * 2);
-    const bool has_res = rrow != nullptr;
+__device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t lane_addr, int n0, bool has_res, const float* s_bias, uint32_t buf,
+                                                     const CUtensorMap* tmap_y, int m0, bool publish) {
+    const uint32_t r = threadIdx.x;                 // tile row
+    const int U = a.out_box, m_warp = m0 + (int)(r & ~31u);
+    const uint32_t swz = U == 64 ? r & 7u : (r >> 1) & 3u;
+    const uint32_t row = buf + r * (uint32_t)(U * 2), warp_row = buf + (r & ~31u) * (uint32_t)(U * 2);
     uint32_t v0[16], v1[16];
-    uint4 r0[2], r1[2];
-    auto put = [&](const uint32_t (&v)[16], const uint4 (&rv)[2], int cb) {
+    auto put = [&](const uint32_t (&v)[16], int cb) {
         const int in_box = cb & (U - 1);
-        const uint32_t box = (uint32_t)(cb - in_box) * 64u;      // 32 rows x 2 bytes per column before this box
+        const uint32_t box = (uint32_t)(cb - in_box) * 256u;      // 128 rows x 2 bytes per column before this box
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint4 o = finish8<ACT>(a, v + h * 8, rv[h], has_res, n0 + cb + h * 8, s_bias + cb + h * 8);
-            st_shared_v4(row + box + ((((uint32_t)(in_box >> 3) + (uint32_t)h) ^ swz) << 4), o.x, o.y, o.z, o.w);
+            const uint32_t at = row + box + ((((uint32_t)(in_box >> 3) + (uint32_t)h) ^ swz) << 4);
+            uint4 res = make_uint4(0, 0, 0, 0);
+            if (has_res) res = ld_shared_v4(at);
+            const uint4 o = finish8<ACT>(a, v + h * 8, res, has_res, n0 + cb + h * 8, s_bias + cb + h * 8);
+            st_shared_v4(at, o.x, o.y, o.z, o.w);
         }
         if (in_box + 16 == U) {
             fence_proxy_async();
             __syncwarp();
             const int x = n0 + cb - in_box;
-            if (x < a.K && m_warp < a.M && elect_one()) tma_store_2d(tmap_y, x, m_warp, buf + box);
+            if (x < a.K && m_warp < a.M && elect_one()) tma_store_2d(tmap_y, x, m_warp, warp_row + box);
             __syncwarp();
         }
     };
     tcgen05_ld16(lane_addr, v0);             // warp-collective: all lanes take part
-    load_residual(a, n0, row_valid, rrow, r0);
     for (int cb = 0; cb < a.BN; cb += 32) {
         tcgen05_wait_ld();
-        const bool second = cb + 16 < a.BN;
-        if (second) {
-            tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
-            load_residual(a, n0 + cb + 16, row_valid, rrow, r1);
-        }
-        put(v0, r0, cb);
-        if (!second) break;
+        tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
+        put(v0, cb);
         tcgen05_wait_ld();
-        if (cb + 32 < a.BN) {
-            tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
-            load_residual(a, n0 + cb + 32, row_valid, rrow, r0);
-        }
-        put(v1, r1, cb + 16);
+        if (cb + 32 < a.BN) tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
+        put(v1, cb + 16);
     }
-    if (elect_one()) tma_store_wait();       // shared memory may go, and the tile is in memory
+    if (elect_one()) {
+        if (publish) tma_store_wait();
+        else tma_store_wait_read();
+    }
     __syncwarp();
 }
 
@@ -466,7 +471,7 @@ __device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t
 // tmap_y (the one-tile kernels): through TMA stores staged at `buf`.
 __device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, bool ok, int m0, int n0, const float* s_bias,
                                          uint64_t* s_accum_p, volatile uint32_t* s_abort_p, uint32_t accum_parity = 0u,
-                                         const CUtensorMap* tmap_y = nullptr, uint32_t buf = 0) {
+                                         const CUtensorMap* tmap_y = nullptr, uint32_t buf = 0, uint64_t* s_res = nullptr, bool publish = true) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int m = m0 + tid;
@@ -477,16 +482,16 @@ __device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, 
     tcgen05_fence_after();
     const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
     if (!ok) return;
-    const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
     if (tmap_y) {
-        buf += (uint32_t)warp * (uint32_t)a.BN * 64u;
-        const int m_warp = m0 + warp * 32;
-        if (a.act == 3) epilogue_columns_tma<3>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
-        else if (a.act == 1) epilogue_columns_tma<1>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
-        else if (a.act == 2) epilogue_columns_tma<2>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
-        else epilogue_columns_tma<0>(a, lane_addr, n0, row_valid, rrow, s_bias, buf, tmap_y, m_warp);
+        const bool has_res = a.residual != nullptr;
+        if (has_res && !__all_sync(0xffffffffu, mbar_wait(smem_u32(s_res), 0u, s_abort_p, a.err_flag, 6u))) return;
+        if (a.act == 3) epilogue_columns_tma<3>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        else if (a.act == 1) epilogue_columns_tma<1>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        else if (a.act == 2) epilogue_columns_tma<2>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        else epilogue_columns_tma<0>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
         return;
     }
+    const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
     __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
     if (a.act == 3) epilogue_columns<3>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
     else if (a.act == 1) epilogue_columns<1>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
@@ -793,10 +798,11 @@ constexpr int kWarpB = 3;
 
 // One CTA's share of one convolution: output tile (bx, by), rank bz of the cluster that shares the tile's
 // reduction, `stages` pipeline buffers.  Shared by the single-convolution kernel and the grouped one.
-__device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const CUtensorMap* tmap_y, const ConvArgs& a, const int stages,
+__device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const CUtensorMap* tmap_y, const CUtensorMap* tmap_r,
+                                              const ConvArgs& a, const int stages,
                                               const int bx, const int by, const int bz, uint8_t* smem_raw,
                                               uint64_t* s_full, uint64_t* s_empty, uint64_t* s_accum, uint32_t* s_tmem_base,
-                                              volatile uint32_t* s_abort, float* s_bias) {
+                                              volatile uint32_t* s_abort, float* s_bias, uint64_t* s_res, bool publish) {
     const int tid = threadIdx.x;
     const int warp = (int)uniform((uint32_t)tid >> 5);
     const int lane = tid & 31;
@@ -835,6 +841,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
                 mbar_init(smem_u32(&s_empty[s]), 1);     // tcgen05.commit
             }
             mbar_init(smem_u32(s_accum), 1);
+            mbar_init(smem_u32(s_res), 1);
             *s_abort = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -901,7 +908,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         if (tid == 0) PB_S(2);
         griddep_launch();
         if (a.splits > 1) epilogue_cluster(a, tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
-        else epilogue(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base);
+        else epilogue(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
         if (tid == 0) { PB_T(6); PB_S(6); }
     } else if (warp == 4) {
         // ===== operand A =====
@@ -924,6 +931,20 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
                 if (++tap_s == S) { tap_s = 0; ++tap_r; }
             }
             if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
+        }
+        // The residual goes where the tile will be laid out, as soon as the multiplications have read the pipeline buffers there.
+        if (a.residual && a.out_box) {
+            const uint32_t bytes = (uint32_t)a.BN * 256u;
+            bool ok = true;
+            for (uint32_t q = 0; q * stage_bytes < bytes && ok; ++q) {
+                const int uses = nkb > (int)q ? (nkb - (int)q + stages - 1) / stages : 0;
+                if (uses > 0) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[q]), (uint32_t)(uses - 1) & 1u, s_abort, err_flag, 1u));
+            }
+            if (ok && elect_one()) {
+                mbar_arrive_expect_tx(smem_u32(s_res), bytes);
+                for (int c = 0; c < a.BN; c += a.out_box) tma_load_2d(smem_base + (uint32_t)c * 256u, tmap_r, n0 + c, m0, smem_u32(s_res));
+            }
+            __syncwarp();
         }
         griddep_launch();
         if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
@@ -1004,10 +1025,11 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 
 __global__ void __launch_bounds__(kThreadsTma, 3)
 conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                     const __grid_constant__ CUtensorMap tmap_y, const ConvArgs a, int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
+                     const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_r, const ConvArgs a, int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxStages];
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
+    __shared__ __align__(8) uint64_t s_res;
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
@@ -1016,8 +1038,8 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     resolve_slot(job_id, nf);
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
-    conv_tile_tma(&tmap_w, &tmap_x, &tmap_y, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
-                  &s_tmem_base, &s_abort, s_bias);
+    conv_tile_tma(&tmap_w, &tmap_x, &tmap_y, &tmap_r, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+                  &s_tmem_base, &s_abort, s_bias, &s_res, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1043,6 +1065,7 @@ struct alignas(128) SubConv {
     CUtensorMap tmap_w;
     CUtensorMap tmap_x;
     CUtensorMap tmap_y;
+    CUtensorMap tmap_r;
     union {
         ConvArgs a;
         PoolSubArgs pool;
@@ -1124,6 +1147,7 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxStages];
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
+    __shared__ __align__(8) uint64_t s_res;
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
@@ -1154,8 +1178,8 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     const uint32_t S = (uint32_t)s_args.splits, gx = sc->gx;
     const uint32_t tile = local / S, bz = local - tile * S;
     const uint32_t by = tile / gx, bx = tile - by * gx;
-    conv_tile_tma(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
-                  &s_tmem_base, &s_abort, s_bias);
+    conv_tile_tma(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
+                  &s_tmem_base, &s_abort, s_bias, &s_res, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1639,7 +1663,8 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     // Stores through TMA where blocks share an SM's store path; a block alone on its SM is 0.2 us faster with direct ones
     // (measured: up to 148 blocks or up to 48 columns direct stores win, above both TMA ones do, by up to 3 us a launch).
     g.out_box = 0;
-    if (g.splits == 1 && g.BN >= 64 && g.BN % 32 == 0 && (shared || g.m_tiles * g.n_tiles > 148)) g.out_box = g.BN % 64 == 0 ? 64 : 32;
+    static const int rl = getenv("PB_RL") ? atoi(getenv("PB_RL")) : 0;
+    if (g.splits == 1 && g.BN >= 64 && g.BN % 32 == 0 && (shared || g.m_tiles * g.n_tiles > 148 || (rl && p->residual))) g.out_box = g.BN % 64 == 0 ? 64 : 32;
     const uint32_t exchange = g.splits > 1 ? (uint32_t)g.BN * 512u : 0u;      // a rank's partial tile
     g.smem_bytes = std::max((uint32_t)g.stages * stage_bytes, exchange) + 1024u;
     // c_format f32 (1 << 4), a/b format bf16 (1 << 7, 1 << 10), K-major both, N >> 3 at bit 17, M >> 4 at bit 24
@@ -1830,18 +1855,20 @@ static int make_xmap(const pb_op_params* p, CUtensorMap* out) {
 }
 
 
-// Output map: [pixels of all images][channels of the slice], boxes of 32 rows.
-static int make_ymap(const pb_op_params* p, int U, CUtensorMap* out) {
-    if (!U) { memset(out, 0, sizeof(*out)); return PB_OK; }
+// Map of the output slice (boxes of 32 rows) or of the residual (boxes of 128 rows): [pixels of all images][channels].
+static int make_ymap(const pb_op_params* p, int U, bool residual, CUtensorMap* out) {
+    if (!U || (residual && !p->residual)) { memset(out, 0, sizeof(*out)); return PB_OK; }
+    const __nv_bfloat16* base = residual ? static_cast<const __nv_bfloat16*>(p->residual) : static_cast<const __nv_bfloat16*>(p->y) + p->out_c_off;
+    const int stride = residual ? p->res_Cs : p->Ks;
     EncodeTiledFn enc = encode_fn();
     PB_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
-    PB_REQUIRE(((uintptr_t)p->y & 15) == 0, "conv_umma: the output must be 16-byte aligned");
+    PB_REQUIRE(((uintptr_t)base & 15) == 0, "conv_umma: output and residual must be 16-byte aligned");
     const cuuint64_t dims[2] = {(cuuint64_t)p->K, (cuuint64_t)batch_of(p) * p->P * p->Q};
-    const cuuint64_t strides[1] = {(cuuint64_t)p->Ks * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)U, 32};
+    const cuuint64_t strides[1] = {(cuuint64_t)stride * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)U, residual ? 128u : 32u};
     const cuuint32_t estr[2] = {1, 1};
     const CUtensorMapSwizzle sw = U == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, static_cast<__nv_bfloat16*>(p->y) + p->out_c_off, dims, strides, box, estr,
+    const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled (output) failed with CUresult %d (K %d, stride %d)", (int)r, p->K, p->Ks);
@@ -1975,11 +2002,12 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
             if (rc != PB_OK) return rc;
             xmap = &local;
         }
-        CUtensorMap wmap, ymap;
+        CUtensorMap wmap, ymap, rmap;
         int mrc = make_tmap(plan, g.BN, &wmap);
-        if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, &ymap);
+        if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, false, &ymap);
+        if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, true, &rmap);
         if (mrc != PB_OK) return mrc;
-        const cudaError_t e = launch_pdl(conv_umma_tma_kernel, grid, dim3(1, 1, (unsigned)g.splits), g.smem_bytes, st, pdl, wmap, xmap->map, ymap, a,
+        const cudaError_t e = launch_pdl(conv_umma_tma_kernel, grid, dim3(1, 1, (unsigned)g.splits), g.smem_bytes, st, pdl, wmap, xmap->map, ymap, rmap, a,
                                          g.stages, job_id, nf);
         if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_tma_kernel", __FILE__, __LINE__);
         return PB_OK;
@@ -2074,7 +2102,8 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
         const Geometry g = geometry(params[i], split_allowed(params[i]) && !persist_enabled());
         SubConv& sc = table[(size_t)at++];
         int rc = make_tmap(plans[i], g.BN, &sc.tmap_w);
-        if (rc == PB_OK) rc = make_ymap(params[i], g.out_box, &sc.tmap_y);
+        if (rc == PB_OK) rc = make_ymap(params[i], g.out_box, false, &sc.tmap_y);
+        if (rc == PB_OK) rc = make_ymap(params[i], g.out_box, true, &sc.tmap_r);
         if (rc != PB_OK) { delete m; return rc; }
         sc.tmap_x = xmaps[i]->map;
         rc = fill_args(plans[i], g, params[i], nullptr, &sc.a);

@@ -434,14 +434,14 @@ __device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t
     auto put = [&](const uint32_t (&v)[16], int cb) {
         const int in_box = cb & (U - 1);
         const uint32_t box = (uint32_t)(cb - in_box) * 256u;      // 128 rows x 2 bytes per column before this box
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t at = row + box + ((((uint32_t)(in_box >> 3) + (uint32_t)h) ^ swz) << 4);
-            uint4 res = make_uint4(0, 0, 0, 0);
-            if (has_res) res = ld_shared_v4(at);
-            const uint4 o = finish8<ACT>(a, v + h * 8, res, has_res, n0 + cb + h * 8, s_bias + cb + h * 8);
-            st_shared_v4(at, o.x, o.y, o.z, o.w);
-        }
+        // both halves' loads before either's store: a store is a barrier to the compiler
+        const uint32_t at0 = row + box + (((uint32_t)(in_box >> 3) ^ swz) << 4), at1 = row + box + ((((uint32_t)(in_box >> 3) + 1u) ^ swz) << 4);
+        uint4 res0 = make_uint4(0, 0, 0, 0), res1 = res0;
+        if (has_res) { res0 = ld_shared_v4(at0); res1 = ld_shared_v4(at1); }
+        const uint4 o0 = finish8<ACT>(a, v, res0, has_res, n0 + cb, s_bias + cb);
+        const uint4 o1 = finish8<ACT>(a, v + 8, res1, has_res, n0 + cb + 8, s_bias + cb + 8);
+        st_shared_v4(at0, o0.x, o0.y, o0.z, o0.w);
+        st_shared_v4(at1, o1.x, o1.y, o1.z, o1.w);
         if (in_box + 16 == U) {
             fence_proxy_async();
             __syncwarp();
@@ -847,10 +847,12 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         __syncwarp();
-        for (int q = 0; q < stages && q < nkb; ++q) {
+        // The first k-block's weights only: its other copies leave in the main loop (six of them here held every warp at the
+        // barrier below for 0.3 us a tile).
+        if (nkb > 0) {
             if (elect_one()) {
-                mbar_arrive_expect_tx(smem_u32(&s_full[q]), tx_bytes);
-                tma_load_2d(smem_base + (uint32_t)q * stage_bytes + kATileBytes, tmap_w, (kb_begin + q) * kBK, n0, smem_u32(&s_full[q]));
+                mbar_arrive_expect_tx(smem_u32(&s_full[0]), tx_bytes);
+                tma_load_2d(smem_base + kATileBytes, tmap_w, kb_begin * kBK, n0, smem_u32(&s_full[0]));
             }
             __syncwarp();
         }
@@ -882,11 +884,11 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 
     if (warp < 4) {
         if (warp == kWarpB) {
-            // ===== operand B, from the second turn of the pipeline on =====
+            // ===== operand B =====
             uint32_t* const err_flag = a.err_flag;
-            uint32_t st = 0, parity = 0u;
-            for (int kb = stages; kb < nkb; ++kb) {
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u))) break;
+            uint32_t st = stages > 1 ? 1u : 0u, parity = stages > 1 ? 1u : 0u;
+            for (int kb = 1; kb < nkb; ++kb) {
+                if (kb >= stages && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u))) break;
                 if (elect_one()) {
                     mbar_arrive_expect_tx(smem_u32(&s_full[st]), tx_bytes);
                     tma_load_2d(smem_base + st * stage_bytes + kATileBytes, tmap_w, (kb_begin + kb) * kBK, n0, smem_u32(&s_full[st]));
@@ -1663,8 +1665,7 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     // Stores through TMA where blocks share an SM's store path; a block alone on its SM is 0.2 us faster with direct ones
     // (measured: up to 148 blocks or up to 48 columns direct stores win, above both TMA ones do, by up to 3 us a launch).
     g.out_box = 0;
-    static const int rl = getenv("PB_RL") ? atoi(getenv("PB_RL")) : 0;
-    if (g.splits == 1 && g.BN >= 64 && g.BN % 32 == 0 && (shared || g.m_tiles * g.n_tiles > 148 || (rl && p->residual))) g.out_box = g.BN % 64 == 0 ? 64 : 32;
+    if (g.splits == 1 && g.BN >= 64 && g.BN % 32 == 0 && (shared || g.m_tiles * g.n_tiles > 148)) g.out_box = g.BN % 64 == 0 ? 64 : 32;
     const uint32_t exchange = g.splits > 1 ? (uint32_t)g.BN * 512u : 0u;      // a rank's partial tile
     g.smem_bytes = std::max((uint32_t)g.stages * stage_bytes, exchange) + 1024u;
     // c_format f32 (1 << 4), a/b format bf16 (1 << 7, 1 << 10), K-major both, N >> 3 at bit 17, M >> 4 at bit 24

@@ -1583,47 +1583,96 @@ int packed_rows(const pb_op_params* p) {
     return n * round_up(ceil_div(Kp16, n), 16);
 }
 
-struct Tiling { int BN, splits; };
+// How a launch of m_tiles x 128 rows is cut.
+struct Tiling {
+    int BN, splits;             // output channels of a tile, blocks (one cluster) that share its reduction
+    bool tma;                   // the tile leaves (and the residual arrives) through TMA
+};
+struct ConvShape {
+    int m_tiles, Kp16, nkb;
+    bool residual, shared;      // shared: other requests use the GPU too
+};
 
-// Modelled microseconds of a lone launch inside a stage graph, fitted to 474 measured (layer shape, tile width, split)
-// combinations on B200 - chains of equal layers of 7x7 to 56x56 maps, 64 to 2048 channels, 1x1 and 3x3, 1 to 8 images:
-//   a launch costs 1.6 us outside its k-loop (operand latency, accumulator drain, hand-over to the next launch);
-//   a k-block costs the issue of its copies (0.18 us + 0.8 ns per column) or its bytes at 113 KB/us per SM, shared by
-//   the blocks of the SM;
-//   the epilogue costs 16 ns per column of a block;
-//   a cluster costs its two barriers and the parked tile, and 5 / 8 / 16 ns of placement per block at 2 / 4 / 8 ranks.
-// The tile it picks is within 4 % of the best measured one on average (worst 22 %).
-int tiling_ctas(int m_tiles, int Kp16, const Tiling& t) { return m_tiles * ceil_div(Kp16, t.BN) * t.splits; }
-double tiling_us(int ctas, int nkb, const Tiling& t) {
-    const double per_sm = std::max(1.0, ctas / 148.0);
-    const double kb = std::max(0.183 + 0.00084 * t.BN, per_sm * (16.384 + 0.128 * t.BN) / 113.0);
-    double us = 1.59 + 0.0162 * t.BN / t.splits * (1.0 + 0.56 * (per_sm - 1.0)) + ceil_div(nkb, t.splits) * kb;
-    if (t.splits > 1) us += 0.06 + 0.0174 * t.BN + ctas * (t.splits == 2 ? 0.0048 : t.splits == 4 ? 0.0079 : 0.0164);
-    return us;
+// Pipeline depth: as many stages as the k-loop can use and the shared-memory budget holds.  On a GPU it has to itself a
+// launch of up to two blocks per SM gets a deeper pipeline (a refill takes about 1.1 us; 36 k-blocks of 64 columns: 13.6 us
+// at 73 KB, 12.3 at 110, 11.7 at 150, where the next launch's blocks no longer fit beside it: Inception-v3 402 us
+// instead of 346).
+int pipeline_stages(int ctas, int BN, int k_blocks, bool shared) {
+    const int budget = (int)(!shared && ctas <= 296 ? kSmemBudgetDeep : kSmemBudgetTma) - 1024;
+    return std::max(2, std::min({kMaxStages, budget / ((int)kATileBytes + BN * 128), k_blocks}));
 }
 
-// Tile width (output channels) and split of a launch of m_tiles x 128 rows: the combination with the least modelled
-// time, plus a charge for the block slots it takes (444 = 148 SMs x 3): on a GPU that other requests share, what counts is
-// not when a launch ends but what it occupies.  Measured, charge -> 192 requests of MNIST : Inception-v3 = 9 : 1 in flight /
-// 32 of ResNet-18: 0 -> 1893 / 2478 us, 4 -> 1448 / 1581, 8 -> 1337 / 1624, 12 -> 1313 / 1651, 20 -> 1334 / 1727; alone,
-// Inception-v3 / 8 images of ResNet-50: 0 -> 343 / 446 us, 0.5 -> 343 / 438, 5 -> 352 / 481, 20 -> 393 / 556.
-Tiling choose_tiling(int m_tiles, int Kp16, int nkb, int bn_max, int want_splits, double gain_us, bool shared) {
-    const double charge = shared ? 8.0 : 0.5;
-    Tiling best{0, 1};
+// Modelled microseconds of a lone launch inside a stage graph, fitted to 3372 measured (layer shape, tile width, split, way
+// out) combinations on B200 - chains of equal layers of 7x7 to 149x149 maps, 32 to 2048 channels, 1x1 and 3x3, 1 to 8 images,
+// with and without a residual, either pipeline budget:
+//   a launch costs 3.7 us outside its k-loop and epilogue (operand latency, accumulator drain, hand-over to the next launch);
+//   a k-block costs the issue of its copies (0.2 us), its share of a refill's latency, or its bytes at 137 KB/us per SM,
+//   shared by the blocks of the SM (between the mean and the fullest one);
+//   the epilogue costs 11 ns per column of a block with direct stores (24 with a residual), 8 through TMA;
+//   a cluster costs its two barriers and the parked tile, and 2 / 6 / 13 ns of placement per block at 2 / 4 / 8 ranks.
+// Its mean error is 3 %, and what it picks is within 1.5 % of the best measured tiles summed over the layers of a network.
+// (Before, the model knew neither the stores' path nor the residual, and a width of 80 or 176 columns, which TMA cannot
+// store, cost a 14 x 14 layer of 256 -> 1024 channels 8.8 us instead of 6.4 alone and 3.1 instead of 1.7 under load.)
+int tiling_ctas(const ConvShape& c, const Tiling& t) { return c.m_tiles * ceil_div(c.Kp16, t.BN) * t.splits; }
+double tiling_us(int ctas, const ConvShape& c, const Tiling& t) {
+    const int k_blocks = ceil_div(c.nkb, t.splits), stages = pipeline_stages(ctas, t.BN, k_blocks, c.shared);
+    const double mean = std::max(1.0, ctas / 148.0), per_sm = mean + 0.639 * (ceil_div(ctas, 148) - mean);
+    const double crowd = 1.0 + 1.39 * (per_sm - 1.0);
+    double kb = std::max(0.197 + 0.0003 * t.BN, per_sm * (16.384 + 0.128 * t.BN) / 137.0);
+    if (k_blocks > stages) kb = std::max(kb, (0.452 + 0.0015 * t.BN) / stages);
+    double us = 3.68 + k_blocks * kb;
+    if (t.tma) us += 0.164 + 0.0081 * t.BN * crowd + (c.residual ? 0.327 + 0.0006 * t.BN * crowd : 0.0);
+    else us += (c.residual ? 0.0242 : 0.0114) * t.BN / t.splits * crowd;
+    if (t.splits > 1) us += 0.401 + 0.017 * t.BN + ctas * (t.splits == 2 ? 0.0023 : t.splits == 4 ? 0.0055 : 0.0133);
+    return us;
+}
+// Relative length of a block's stay on its SM.
+double tiling_stay(const ConvShape& c, const Tiling& t) {
+    const double column = (t.tma ? 0.012 : 0.0192) * (c.residual ? 1.5 : 1.0);
+    return 1.5 + 0.12 * ceil_div(c.nkb, t.splits) + column * t.BN + (t.splits > 1 ? 1.0 : 0.0);
+}
+
+// Tile width (output channels), split and way out of a launch: the combination with the least modelled time, plus a charge
+// for the block slots it takes (444 = 148 SMs x 3): on a GPU that other requests share, what counts is not when a launch
+// ends but what it occupies.  Measured with eight chains side by side, summed over the layers of ResNet-50 x 8 images /
+// Inception-v3 x 8 / ResNet-18 x 8, charge -> us per chain: 3 -> 155.5 / 147.6 / 60.9, 6 -> 148.7 / 144.3 / 55.0, 8 -> 149.8
+// / 145.1 / 54.4 (best tiles for each layer: 148.2 / 143.9 / 54.0), while alone a chain gets 6 % slower from 3 to 6 and 3 %
+// from 6 to 8; a chain alone: 0 -> 397 / 405 / 163, 0.5 -> 399 / 402 / 164, 1 -> 401 / 404 / 164.
+Tiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
+    const double charge = c.shared ? 6.0 : 0.5;
+    Tiling best{0, 1, false};
     double best_us = 1e30;
     for (int S = 1; S <= 8; S *= 2) {
-        if (want_splits > 0 ? S != want_splits : (S > 1 && nkb < 2 * S)) continue;
+        if (want_splits > 0 ? S != want_splits : (S > 1 && c.nkb < 2 * S)) continue;
         const int widest = S > 1 ? std::min(bn_max, 128) : bn_max;
-        for (int n = ceil_div(Kp16, widest); n <= ceil_div(Kp16, 32); ++n) {
-            const Tiling t{round_up(ceil_div(Kp16, n), std::max(16, 8 * S)), S};
-            if (t.BN > widest) continue;
-            const int ctas = tiling_ctas(m_tiles, Kp16, t);
-            double us = tiling_us(ctas, nkb, t) + (S > 1 ? gain_us / 60.0 : 0.0);
-            us += charge * ctas * (1.5 + ceil_div(nkb, S) * 0.2) / 444.0;
-            if (us < best_us - 1e-9) { best_us = us; best = t; }
+        for (int n = ceil_div(c.Kp16, widest); n <= ceil_div(c.Kp16, 32); ++n) {
+            for (int tma = 0; tma < (S > 1 ? 1 : 2); ++tma) {          // TMA stores boxes of 32 or 64 columns of a whole tile
+                const Tiling t{round_up(ceil_div(c.Kp16, n), tma ? 32 : std::max(16, 8 * S)), S, tma != 0};
+                if (t.BN > widest) continue;
+                const int ctas = tiling_ctas(c, t);
+                double us = tiling_us(ctas, c, t) + (S > 1 ? gain_us / 60.0 : 0.0);
+                us += charge * ctas * tiling_stay(c, t) / 444.0;
+                if (us < best_us - 1e-9) { best_us = us; best = t; }
+            }
         }
     }
     return best;
+}
+
+// The search takes 1 to 6 us, as long as a launch: a thread keeps the tilings of its last few shapes.
+Tiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
+    struct Kept { ConvShape c; int bn_max, want_splits; double gain_us; Tiling t; };
+    static thread_local Kept kept[16] = {};
+    Kept& k = kept[((unsigned)c.m_tiles * 7u + (unsigned)c.Kp16 / 16u + (unsigned)c.nkb * 5u + (unsigned)want_splits + (unsigned)c.residual * 3u) % 16u];
+    if (k.t.BN == 0 || k.c.m_tiles != c.m_tiles || k.c.Kp16 != c.Kp16 || k.c.nkb != c.nkb || k.c.residual != c.residual || k.c.shared != c.shared ||
+        k.bn_max != bn_max || k.want_splits != want_splits || k.gain_us != gain_us)
+        k = {c, bn_max, want_splits, gain_us, best_tiling(c, bn_max, want_splits, gain_us)};
+    return k.t;
+}
+
+ConvShape conv_shape(const pb_op_params* p) {
+    return {ceil_div(batch_of(p) * p->P * p->Q, kBM), round_up(p->K, 16), p->R * p->S * ceil_div(p->Cs, kBK), p->residual != nullptr,
+            (p->reserved & kTileShared) != 0};
 }
 
 Geometry geometry(const pb_op_params* p, bool allow_split) {
@@ -1636,36 +1685,26 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM);
     const double gain = conv_split_gain_us();
     const int want = p->reserved & kTileSplitMask;       // a grouped launch has one cluster size for all its convolutions (0: not decided)
-    const bool shared = (p->reserved & kTileShared) != 0;
-    Tiling t = choose_tiling(g.m_tiles, g.Kp16, g.nkb, bn_limit(), !use_tma_a() || gain > 1e6 ? 1 : want, gain, shared);
+    const ConvShape shape = conv_shape(p);
+    Tiling t = choose_tiling(shape, bn_limit(), !use_tma_a() || gain > 1e6 ? 1 : want, gain);
     g.scratch_bytes = t.splits > 1 ? kSplitScratchBytes : 0;
-    if (t.splits > 1 && !allow_split) t = choose_tiling(g.m_tiles, g.Kp16, g.nkb, bn_limit(), 1, gain, shared);
+    if (t.splits > 1 && !allow_split) t = choose_tiling(shape, bn_limit(), 1, gain);
     g.BN = t.BN;
     g.splits = t.splits;
     g.n_tiles = ceil_div(g.Kp16, g.BN);
     g.tmem_cols = 32;
     while ((int)g.tmem_cols < g.BN) g.tmem_cols <<= 1;
     g.b_stage_bytes = (uint32_t)g.BN * 128u;
-    // Pipeline depth: as many stages as the k-loop can use and the shared-memory budget holds.  On a GPU it has to itself a
-    // launch of up to two blocks per SM gets a deeper pipeline (a refill takes about 1.1 us; 36 k-blocks of 64 columns: 13.6 us
-    // at 73 KB, 12.3 at 110, 11.7 at 150, where the next launch's blocks no longer fit beside it: Inception-v3 402 us
-    // instead of 346).
     const uint32_t stage_bytes = (uint32_t)kATileBytes + g.b_stage_bytes;
-    const bool deep = !shared && g.m_tiles * g.n_tiles * g.splits <= 296;
-    const uint32_t budget = !use_tma_a() ? kSmemBudget : (deep ? kSmemBudgetDeep : kSmemBudgetTma);
     if (use_tma_a()) {
-        g.stages = (int)std::min<uint32_t>({(uint32_t)kMaxStages, (budget - 1024u) / stage_bytes, (uint32_t)ceil_div(g.nkb, g.splits)});
-        if (g.stages < 2) g.stages = 2;
+        g.stages = pipeline_stages(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), shape.shared);
     } else {
         static const int kDepths[] = {8, 6, 4};                     // the gather kernel exists for 4, 6, 8
         g.stages = 4;
         for (int d : kDepths)
-            if ((uint32_t)d * stage_bytes + 1024u <= budget && d <= g.nkb + 1) { g.stages = d; break; }
+            if ((uint32_t)d * stage_bytes + 1024u <= kSmemBudget && d <= g.nkb + 1) { g.stages = d; break; }
     }
-    // Stores through TMA where blocks share an SM's store path; a block alone on its SM is 0.2 us faster with direct ones
-    // (measured: up to 148 blocks or up to 48 columns direct stores win, above both TMA ones do, by up to 3 us a launch).
-    g.out_box = 0;
-    if (g.splits == 1 && g.BN >= 64 && g.BN % 32 == 0 && (shared || g.m_tiles * g.n_tiles > 148)) g.out_box = g.BN % 64 == 0 ? 64 : 32;
+    g.out_box = !t.tma ? 0 : g.BN % 64 == 0 ? 64 : 32;
     const uint32_t exchange = g.splits > 1 ? (uint32_t)g.BN * 512u : 0u;      // a rank's partial tile
     g.smem_bytes = std::max((uint32_t)g.stages * stage_bytes, exchange) + 1024u;
     // c_format f32 (1 << 4), a/b format bf16 (1 << 7, 1 << 10), K-major both, N >> 3 at bit 17, M >> 4 at bit 24
@@ -2051,19 +2090,17 @@ int conv_umma_common_splits(const pb_op_params* const* params, int n) {
     double best_us = 1e30;
     for (int S = 1; S <= 8; S *= 2) {
         std::vector<Tiling> t((size_t)n);
-        std::vector<int> nkb((size_t)n);
+        std::vector<ConvShape> c((size_t)n);
         int ctas = 0, longest = 0;
         for (int i = 0; i < n; ++i) {
-            const pb_op_params* p = params[i];
-            const int m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM), Kp16 = round_up(p->K, 16);
-            nkb[(size_t)i] = p->R * p->S * ceil_div(p->Cs, kBK);
-            longest = std::max(longest, nkb[(size_t)i]);
-            t[(size_t)i] = choose_tiling(m_tiles, Kp16, nkb[(size_t)i], bn_limit(), S, gain, (p->reserved & kTileShared) != 0);
-            ctas += tiling_ctas(m_tiles, Kp16, t[(size_t)i]);
+            c[(size_t)i] = conv_shape(params[i]);
+            longest = std::max(longest, c[(size_t)i].nkb);
+            t[(size_t)i] = choose_tiling(c[(size_t)i], bn_limit(), S, gain);
+            ctas += tiling_ctas(c[(size_t)i], t[(size_t)i]);
         }
         if (S > 1 && longest < 2 * S) break;
         double us = 0;
-        for (int i = 0; i < n; ++i) us = std::max(us, tiling_us(ctas, nkb[(size_t)i], t[(size_t)i]));
+        for (int i = 0; i < n; ++i) us = std::max(us, tiling_us(ctas, c[(size_t)i], t[(size_t)i]));
         if (S > 1) us += gain / 60.0;
         if (us < best_us) { best_us = us; best = S; }
     }

@@ -56,11 +56,13 @@ def test_conv_umma_cluster_split(case, act):
 
 
 WIDE = [
-    # N, C, H, K, R                            launches of more than 148 tiles: the tile leaves through TMA stores
+    # N, C, H, K, R                            the tile leaves through TMA stores
     (13, 64, 40, 64, 1),                       # 163 row tiles, the last one half empty
     (20, 32, 35, 96, 3),                       # 96 columns: three boxes of 32
     (20, 64, 33, 200, 1),                      # 200 columns: the last box is cut
     (40, 16, 29, 136, 3),                      # tiles straddle images
+    (30, 64, 40, 24, 1),                       # the narrowest box: 24 columns of 32
+    (8, 32, 14, 1024, 1),                      # 13 row tiles, wide: no width that only direct stores can take
 ]
 
 

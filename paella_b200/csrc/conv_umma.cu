@@ -1659,11 +1659,14 @@ Tiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_
     return best;
 }
 
-// The search takes 1 to 6 us, as long as a launch: a thread keeps the tilings of its last few shapes.
+// The search takes 1 to 6 us, as long as a launch (and an instance with grouped launches asks for the same tilings several
+// times): a thread keeps the tilings of its last shapes.
 Tiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
     struct Kept { ConvShape c; int bn_max, want_splits; double gain_us; Tiling t; };
-    static thread_local Kept kept[16] = {};
-    Kept& k = kept[((unsigned)c.m_tiles * 7u + (unsigned)c.Kp16 / 16u + (unsigned)c.nkb * 5u + (unsigned)want_splits + (unsigned)c.residual * 3u) % 16u];
+    static thread_local Kept kept[256] = {};
+    unsigned slot = (unsigned)c.m_tiles * 8191u + (unsigned)c.Kp16 * 131u + (unsigned)c.nkb * 8u + (unsigned)want_splits + (c.residual ? 4u : 0u);
+    slot ^= slot >> 8;
+    Kept& k = kept[slot % 256u];
     if (k.t.BN == 0 || k.c.m_tiles != c.m_tiles || k.c.Kp16 != c.Kp16 || k.c.nkb != c.nkb || k.c.residual != c.residual || k.c.shared != c.shared ||
         k.bn_max != bn_max || k.want_splits != want_splits || k.gain_us != gain_us)
         k = {c, bn_max, want_splits, gain_us, best_tiling(c, bn_max, want_splits, gain_us)};

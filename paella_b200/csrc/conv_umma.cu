@@ -1634,12 +1634,13 @@ double tiling_stay(const ConvShape& c, const Tiling& t) {
 
 // Tile width (output channels), split and way out of a launch: the combination with the least modelled time, plus a charge
 // for the block slots it takes (444 = 148 SMs x 3): on a GPU that other requests share, what counts is not when a launch
-// ends but what it occupies.  Measured with eight chains side by side, summed over the layers of ResNet-50 x 8 images /
-// Inception-v3 x 8 / ResNet-18 x 8, charge -> us per chain: 3 -> 155.5 / 147.6 / 60.9, 6 -> 148.7 / 144.3 / 55.0, 8 -> 149.8
-// / 145.1 / 54.4 (best tiles for each layer: 148.2 / 143.9 / 54.0), while alone a chain gets 6 % slower from 3 to 6 and 3 %
-// from 6 to 8; a chain alone: 0 -> 397 / 405 / 163, 0.5 -> 399 / 402 / 164, 1 -> 401 / 404 / 164.
+// ends but what it occupies.  Measured, charge -> 192 requests of MNIST : Inception-v3 = 9 : 1 at once, us / 32 of ResNet-18 /
+// 64 of MobileNet and ResNet-50 / the first mix in a closed loop of 192 clients, thousand requests a second: 6 -> 1309 / 848 /
+// 1679 / 300, 9 -> 1270 / 849 / 1688 / 305, 13 -> 1276 / 845 / 1742 / 317, 16 -> 1243 / 821 / 1730 / 318, 20 -> - / - / - / 312.
+// A chain that has the GPU to itself, ResNet-50 x 8 images / Inception-v3 x 8 / ResNet-18 x 8: 0 -> 397 / 405 / 163 us,
+// 0.5 -> 399 / 402 / 164, 1 -> 401 / 404 / 164.
 Tiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
-    const double charge = c.shared ? 6.0 : 0.5;
+    const double charge = c.shared ? 16.0 : 0.5;
     Tiling best{0, 1, false};
     double best_us = 1e30;
     for (int S = 1; S <= 8; S *= 2) {

@@ -913,8 +913,33 @@ __global__ void __launch_bounds__(256) gap_kernel(OpArgs a, uint32_t job_id, Fin
 // ---- dense: y[k] = act(w[k,:] . x + b[k]); one warp per output row -----------------
 // x has n_in = a.C elements (already in the device's flattened channels-last order, padded
 // entries zero); w is [K][C] with C a multiple of the vector width.
+//
+// A row of weights is streamed once, from HBM, and that is what bounds it.  U raw 128-bit loads per lane are issued before
+// the first is used (cache-streaming, so they do not evict the input vector from L1); the sum keeps the order of the plain
+// loop.  U = 8 with four blocks per SM: fewer rows in flight than eight blocks with U = 4, each in longer runs of DRAM.
+// 16384 -> 8192 in bf16 (268 MB) / 4096 -> 4096 / 25088 -> 512, us: U = 4, eight blocks 49.5 / 10.2 / 28.5; U = 8, eight blocks
+// 46.3; U = 8, four blocks 41.5 (6.5 TB/s) / 9.0 / 18.5; U = 12 42.9 / 9.8 / 18.4; U = 16 (spills) 41.2 / 9.9 / 16.4; U = 16,
+// three blocks 45.4 / 10.5 / 14.6.  What is left of a row takes U = 4 (a classifier of 1024 inputs is one such step), then one.
+template <int U, typename T>
+__device__ __forceinline__ void dense_run(const T* __restrict__ x, const T* __restrict__ w, int C, int& i, float& acc) {
+    constexpr int N = Vec<T>::N, kStep = 32 * N;
+    typedef typename RawVec<T>::type Raw;
+    for (; i + (U - 1) * kStep < C; i += U * kStep) {
+        Raw wr[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) wr[u] = __ldcs(reinterpret_cast<const Raw*>(w + i + u * kStep));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const Vec<T> xv = Vec<T>::load(x + i + u * kStep);
+            const Vec<T> wv = vec_of(wr[u]);
+#pragma unroll
+            for (int j = 0; j < N; ++j) acc = fmaf(xv.v[j], wv.v[j], acc);
+        }
+    }
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) dense_kernel(OpArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
+__global__ void __launch_bounds__(256, 4) dense_kernel(OpArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
     constexpr int N = Vec<T>::N;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -923,30 +948,10 @@ __global__ void __launch_bounds__(256) dense_kernel(OpArgs a, uint32_t job_id, F
         const T* __restrict__ x = x_img<T>(a);
         const T* __restrict__ w = static_cast<const T*>(a.w) + (size_t)warp * a.C;
         float acc = 0.f;
-        // A row of weights is streamed once, from HBM: four raw 128-bit loads per lane are issued before
-        // the first is used (cache-streaming, so they do not evict the input vector from L1); the sum keeps
-        // the order of the plain loop.
-        typedef typename RawVec<T>::type Raw;
-        constexpr int kStep = 32 * N;
         int i = lane * N;
-        for (; i + 3 * kStep < a.C; i += 4 * kStep) {
-            Raw wr[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) wr[u] = __ldcs(reinterpret_cast<const Raw*>(w + i + u * kStep));
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const Vec<T> xv = Vec<T>::load(x + i + u * kStep);
-                const Vec<T> wv = vec_of(wr[u]);
-#pragma unroll
-                for (int j = 0; j < N; ++j) acc = fmaf(xv.v[j], wv.v[j], acc);
-            }
-        }
-        for (; i < a.C; i += kStep) {
-            const Vec<T> xv = Vec<T>::load(x + i);
-            const Vec<T> wv = vec_of(__ldcs(reinterpret_cast<const Raw*>(w + i)));
-#pragma unroll
-            for (int j = 0; j < N; ++j) acc = fmaf(xv.v[j], wv.v[j], acc);
-        }
+        dense_run<8>(x, w, a.C, i, acc);
+        dense_run<4>(x, w, a.C, i, acc);
+        dense_run<1>(x, w, a.C, i, acc);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) {

@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "launch_slot.cuh"
@@ -252,7 +253,9 @@ void refresh_infos(pb_model* m) {
 
 // Splits the stage list into groups of at most `gs` stages and plans each group's launches.  fuse: independent
 // tensor-core convolutions of equal dependence depth share one launch.  fuse_pools: a 3x3 pooling layer joins the grouped
-// launch of the convolutions of its depth (a launch that contains one always starts with a convolution).
+// launch of the convolutions of its depth (a launch that contains one always starts with a convolution).  Only convolutions
+// with the same `peers` meet in a launch: those of other sets may have another cluster size (groups of another length restart
+// the depth at other stages, so convolutions of two sets can come out equally deep).
 std::vector<pb_model::Group> plan_groups(const pb_model* m, int gs, bool fuse, bool fuse_pools) {
     std::vector<pb_model::Group> groups;
     const int n = (int)m->stages.size();
@@ -276,8 +279,12 @@ std::vector<pb_model::Group> plan_groups(const pb_model* m, int gs, bool fuse, b
         }
         std::vector<int> order((size_t)g.count);
         for (int i = 0; i < g.count; ++i) order[(size_t)i] = first + i;
-        // the convolutions of a depth side by side, the other layers of that depth after them
-        auto rank = [&](int i) { return 2 * level[(size_t)(i - first)] + (m->stages[i].kind == PB_STAGE_CONV_UMMA ? 0 : 1); };
+        // the convolutions of a depth side by side, set by set, the other layers of that depth after them
+        auto rank = [&](int i) {
+            const bool conv = m->stages[(size_t)i].kind == PB_STAGE_CONV_UMMA;
+            const std::vector<int>& peers = m->stages[(size_t)i].peers;
+            return std::make_tuple(level[(size_t)(i - first)], conv ? 0 : 1, conv && !peers.empty() ? peers.front() : 0);
+        };
         if (fuse) std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rank(a) < rank(b); });
         for (int s : order) {
             const Stage& st = m->stages[s];
@@ -287,7 +294,8 @@ std::vector<pb_model::Group> plan_groups(const pb_model* m, int gs, bool fuse, b
                 std::vector<int>& prev = g.launches.back();
                 const Stage& ps = m->stages[prev.front()];
                 const bool prev_fusable = ps.kind == PB_STAGE_CONV_UMMA && !ps.x_is_input && !ps.y_is_output;
-                if (prev_fusable && level[(size_t)(prev.front() - first)] == level[(size_t)(s - first)] && (int)prev.size() < 8) {
+                const bool same_set = !conv_ok || ps.peers == st.peers;
+                if (prev_fusable && same_set && level[(size_t)(prev.front() - first)] == level[(size_t)(s - first)] && (int)prev.size() < 8) {
                     prev.push_back(s);
                     continue;
                 }
@@ -319,16 +327,16 @@ void build_groups(pb_model* m) {
     // (PB_GRAPH_BRANCHES=1) or PB_FUSE_BRANCHES=0.
     m->fuse_branches = env_flag("PB_FUSE_BRANCHES", true) && !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available();
     m->persist = !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available() && pb::conv_umma_persist_enabled();
-    // PB_FUSE_POOLS=1: off by default; not with the persistent kernel.  Measured: same bits, a lone Inception-v3 request
-    // 885 -> 870 us, but 26.9k -> 17.4k req/s with 96 requests in flight: a pooling block then holds a whole convolution
-    // slot of its SM (the launch's 73 KB of shared memory) while it waits on loads, and there are 600-900 of them per
-    // launch at 8 images.
-    m->groups = plan_groups(m, gs, m->fuse_branches, m->fuse_branches && !m->persist && env_flag("PB_FUSE_POOLS", false));
     // The convolutions of one grouped launch share a cluster size.  It is decided on the default plan whatever the
     // switches say, so that they change the scheduling of the model and not its bits.
     for (const pb_model::Group& g : plan_groups(m, dflt, true, false))
         for (const std::vector<int>& l : g.launches)
             for (int s : l) m->stages[(size_t)s].peers = l;
+    // PB_FUSE_POOLS=1: off by default; not with the persistent kernel.  Measured: same bits, a lone Inception-v3 request
+    // 885 -> 870 us, but 26.9k -> 17.4k req/s with 96 requests in flight: a pooling block then holds a whole convolution
+    // slot of its SM (the launch's 73 KB of shared memory) while it waits on loads, and there are 600-900 of them per
+    // launch at 8 images.
+    m->groups = plan_groups(m, gs, m->fuse_branches, m->fuse_branches && !m->persist && env_flag("PB_FUSE_POOLS", false));
     refresh_infos(m);
 }
 

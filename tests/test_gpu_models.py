@@ -200,6 +200,36 @@ def test_graph_capture_options_give_the_same_bits(models_dir, monkeypatch, env):
     m.close()
 
 
+@pytest.mark.parametrize("group", ["4", "12", "24", "64"])
+@pytest.mark.parametrize("model", ["inception_v3", "googlenet"])
+def test_any_stage_granularity_gives_the_same_bits(models_dir, monkeypatch, model, group):
+    """PB_STAGE_GROUP restarts the dependence depth at other stages, so convolutions that do not share a launch (nor a cluster
+    size) by default come out equally deep: the models load, and give the bits of the default granularity, for one image and
+    a gang of eight, under either tiling policy."""
+    L = capi.load()
+    path = os.path.join(models_dir, packer.pack_file_name(model))
+    xs = np.stack([make_input(model, seed) for seed in range(5, 13)]).astype(np.float32)
+    for shared in (0, 1):
+        outs = []
+        for env in (None, group):
+            if env is None:
+                monkeypatch.delenv("PB_STAGE_GROUP", raising=False)
+            else:
+                monkeypatch.setenv("PB_STAGE_GROUP", env)
+            m, inst = C.c_void_p(), C.c_void_p()
+            capi.check(L.pb_model_load(path.encode(), 0, 1, C.byref(m)), "pb_model_load")
+            capi.check(L.pb_model_set_shared_gpu(m, shared), "pb_model_set_shared_gpu")
+            capi.check(L.pb_instance_create_batched(m, 8, 0, C.byref(inst)), "pb_instance_create_batched")
+            y = np.zeros((9, L.pb_model_output_bytes(m) // 4), np.float32)
+            capi.check(L.pb_instance_run_batch_sync(inst, 1, 1, xs.ctypes.data, y.ctypes.data), "one image")
+            capi.check(L.pb_instance_run_batch_sync(inst, 8, 1, xs.ctypes.data, y[1:].ctypes.data), "eight images")
+            assert gu.error_flag() == 0
+            outs.append(y)
+            L.pb_instance_destroy(inst)
+            L.pb_model_destroy(m)
+        np.testing.assert_array_equal(outs[1], outs[0])
+
+
 def test_arcface_embedding(models_dir):
     """ArcFace LResNet100E-IR: 100 convolutions deep, PReLU, a 512-d embedding out (no class scores, so no
     argmax).  bf16 STORAGE through 49 residual units drifts by 1.3 % of the largest component from fp32 - the

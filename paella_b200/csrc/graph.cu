@@ -204,8 +204,8 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
 // cluster size of its convolutions.
 int tile_hint(const pb_model* m, int stage, int nb) {
     const std::vector<int>& l = m->stages[(size_t)stage].peers;
-    const int policy = m->shared ? pb::kTileShared : 0;
-    if (l.size() < 2) return policy;
+    const int policy = (m->shared ? pb::kTileShared : 0) | (m->persist ? 1 : 0);      // the persistent kernel never splits
+    if (l.size() < 2 || m->persist) return policy;
     std::vector<pb_op_params> ps;
     std::vector<const pb_op_params*> pp;
     for (int s : l) {

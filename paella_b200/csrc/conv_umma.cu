@@ -1570,9 +1570,8 @@ struct Geometry {
     int Kp16, n_tiles, BN;
     int m_tiles;
     int stages;                 // pipeline buffers
-    int splits;                 // blocks (one cluster) per tile when the caller allows a split
+    int splits;                 // blocks (one cluster) per tile
     int out_box;                // ConvArgs::out_box
-    uint64_t scratch_bytes;     // what the caller has to supply for that
     uint32_t tmem_cols, b_stage_bytes, smem_bytes, idesc;
 };
 
@@ -1583,11 +1582,7 @@ int packed_rows(const pb_op_params* p) {
     return n * round_up(ceil_div(Kp16, n), 16);
 }
 
-// How a launch of m_tiles x 128 rows is cut.
-struct Tiling {
-    int BN, splits;             // output channels of a tile, blocks (one cluster) that share its reduction
-    bool tma;                   // the tile leaves (and the residual arrives) through TMA
-};
+// What the tiling of a launch of m_tiles x 128 rows depends on.
 struct ConvShape {
     int m_tiles, Kp16, nkb;
     bool residual, shared;      // shared: other requests use the GPU too
@@ -1613,8 +1608,8 @@ int pipeline_stages(int ctas, int BN, int k_blocks, bool shared) {
 // Its mean error is 3 %, and what it picks is within 1.5 % of the best measured tiles summed over the layers of a network.
 // (Before, the model knew neither the stores' path nor the residual, and a width of 80 or 176 columns, which TMA cannot
 // store, cost a 14 x 14 layer of 256 -> 1024 channels 8.8 us instead of 6.4 alone and 3.1 instead of 1.7 under load.)
-int tiling_ctas(const ConvShape& c, const Tiling& t) { return c.m_tiles * ceil_div(c.Kp16, t.BN) * t.splits; }
-double tiling_us(int ctas, const ConvShape& c, const Tiling& t) {
+int tiling_ctas(const ConvShape& c, const ConvTiling& t) { return c.m_tiles * ceil_div(c.Kp16, t.BN) * t.splits; }
+double tiling_us(int ctas, const ConvShape& c, const ConvTiling& t) {
     const int k_blocks = ceil_div(c.nkb, t.splits), stages = pipeline_stages(ctas, t.BN, k_blocks, c.shared);
     const double mean = std::max(1.0, ctas / 148.0), per_sm = mean + 0.639 * (ceil_div(ctas, 148) - mean);
     const double crowd = 1.0 + 1.39 * (per_sm - 1.0);
@@ -1627,7 +1622,7 @@ double tiling_us(int ctas, const ConvShape& c, const Tiling& t) {
     return us;
 }
 // Relative length of a block's stay on its SM.
-double tiling_stay(const ConvShape& c, const Tiling& t) {
+double tiling_stay(const ConvShape& c, const ConvTiling& t) {
     const double column = (t.tma ? 0.012 : 0.0192) * (c.residual ? 1.5 : 1.0);
     return 1.5 + 0.12 * ceil_div(c.nkb, t.splits) + column * t.BN + (t.splits > 1 ? 1.0 : 0.0);
 }
@@ -1639,16 +1634,16 @@ double tiling_stay(const ConvShape& c, const Tiling& t) {
 // 1679 / 300, 9 -> 1270 / 849 / 1688 / 305, 13 -> 1276 / 845 / 1742 / 317, 16 -> 1243 / 821 / 1730 / 318, 20 -> - / - / - / 312.
 // A chain that has the GPU to itself, ResNet-50 x 8 images / Inception-v3 x 8 / ResNet-18 x 8: 0 -> 397 / 405 / 163 us,
 // 0.5 -> 399 / 402 / 164, 1 -> 401 / 404 / 164.
-Tiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
+ConvTiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
     const double charge = c.shared ? 16.0 : 0.5;
-    Tiling best{0, 1, false};
+    ConvTiling best{0, 1, false, c.shared};
     double best_us = 1e30;
     for (int S = 1; S <= 8; S *= 2) {
         if (want_splits > 0 ? S != want_splits : (S > 1 && c.nkb < 2 * S)) continue;
         const int widest = S > 1 ? std::min(bn_max, 128) : bn_max;
         for (int n = ceil_div(c.Kp16, widest); n <= ceil_div(c.Kp16, 32); ++n) {
             for (int tma = 0; tma < (S > 1 ? 1 : 2); ++tma) {          // TMA stores boxes of 32 or 64 columns of a whole tile
-                const Tiling t{round_up(ceil_div(c.Kp16, n), tma ? 32 : std::max(16, 8 * S)), S, tma != 0};
+                const ConvTiling t{round_up(ceil_div(c.Kp16, n), tma ? 32 : std::max(16, 8 * S)), S, tma != 0, c.shared};
                 if (t.BN > widest) continue;
                 const int ctas = tiling_ctas(c, t);
                 double us = tiling_us(ctas, c, t) + (S > 1 ? gain_us / 60.0 : 0.0);
@@ -1662,8 +1657,8 @@ Tiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_
 
 // The search takes 1 to 6 us, as long as a launch (and an instance with grouped launches asks for the same tilings several
 // times): a thread keeps the tilings of its last shapes.
-Tiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
-    struct Kept { ConvShape c; int bn_max, want_splits; double gain_us; Tiling t; };
+ConvTiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
+    struct Kept { ConvShape c; int bn_max, want_splits; double gain_us; ConvTiling t; };
     static thread_local Kept kept[256] = {};
     unsigned slot = (unsigned)c.m_tiles * 8191u + (unsigned)c.Kp16 * 131u + (unsigned)c.nkb * 8u + (unsigned)want_splits + (c.residual ? 4u : 0u);
     slot ^= slot >> 8;
@@ -1674,12 +1669,19 @@ Tiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double gai
     return k.t;
 }
 
-ConvShape conv_shape(const pb_op_params* p) {
-    return {ceil_div(batch_of(p) * p->P * p->Q, kBM), round_up(p->K, 16), p->R * p->S * ceil_div(p->Cs, kBK), p->residual != nullptr,
-            (p->reserved & kTileShared) != 0};
+ConvShape conv_shape(const pb_op_params* p, bool shared) {
+    return {ceil_div(batch_of(p) * p->P * p->Q, kBM), round_up(p->K, 16), p->R * p->S * ceil_div(p->Cs, kBK), p->residual != nullptr, shared};
 }
+bool splits_off() { return !use_tma_a() || conv_split_gain_us() > 1e6; }
+// want_splits: the cluster size (0: the fastest).
+ConvTiling tiling_for(const pb_op_params* p, bool shared, int want_splits) {
+    return choose_tiling(conv_shape(p, shared), bn_limit(), splits_off() ? 1 : want_splits, conv_split_gain_us());
+}
+// The split is the caller's to allow: by the scratch memory that pb_launch_info.scratch_bytes asks for.
+bool split_allowed(const pb_op_params* p) { return p->scratch != nullptr && p->scratch_bytes >= kSplitScratchBytes; }
+ConvTiling tiling_or(const ConvTiling* given, const pb_op_params* p) { return given ? *given : tiling_for(p, false, split_allowed(p) ? 0 : 1); }
 
-Geometry geometry(const pb_op_params* p, bool allow_split) {
+Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     Geometry g;
     g.cpt = ceil_div(p->Cs, kBK);
     g.Cp = g.cpt * kBK;
@@ -1687,12 +1689,6 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     g.Kdim_pad = g.nkb * kBK;
     g.Kp16 = round_up(p->K, 16);
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM);
-    const double gain = conv_split_gain_us();
-    const int want = p->reserved & kTileSplitMask;       // a grouped launch has one cluster size for all its convolutions (0: not decided)
-    const ConvShape shape = conv_shape(p);
-    Tiling t = choose_tiling(shape, bn_limit(), !use_tma_a() || gain > 1e6 ? 1 : want, gain);
-    g.scratch_bytes = t.splits > 1 ? kSplitScratchBytes : 0;
-    if (t.splits > 1 && !allow_split) t = choose_tiling(shape, bn_limit(), 1, gain);
     g.BN = t.BN;
     g.splits = t.splits;
     g.n_tiles = ceil_div(g.Kp16, g.BN);
@@ -1701,7 +1697,7 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     g.b_stage_bytes = (uint32_t)g.BN * 128u;
     const uint32_t stage_bytes = (uint32_t)kATileBytes + g.b_stage_bytes;
     if (use_tma_a()) {
-        g.stages = pipeline_stages(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), shape.shared);
+        g.stages = pipeline_stages(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), t.shared);
     } else {
         static const int kDepths[] = {8, 6, 4};                     // the gather kernel exists for 4, 6, 8
         g.stages = 4;
@@ -1715,9 +1711,6 @@ Geometry geometry(const pb_op_params* p, bool allow_split) {
     g.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
     return g;
 }
-// The split is the caller's to allow: by the scratch memory that pb_launch_info.scratch_bytes asks for.
-bool split_allowed(const pb_op_params* p) { return p->scratch != nullptr && p->scratch_bytes >= kSplitScratchBytes; }
-Geometry geometry(const pb_op_params* p) { return geometry(p, split_allowed(p)); }
 
 const void* kernel_for(int stages, bool tma) {
     if (tma) return (const void*)conv_umma_tma_kernel;
@@ -1789,11 +1782,14 @@ bool conv_umma_supported(const pb_op_params* p) {
            !(p->flags & 2);
 }
 
-int conv_umma_info(const pb_op_params* p, pb_launch_info* out) {
+ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split) { return tiling_for(p, shared, may_split ? 0 : 1); }
+
+int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling) {
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
-    const Geometry g = geometry(p);
+    const Geometry g = geometry(p, tiling_or(tiling, p));
     memset(out, 0, sizeof(*out));
-    out->scratch_bytes = g.scratch_bytes;       // what a split launch asks for
+    // what a split launch asks for
+    out->scratch_bytes = (tiling ? g.splits : tiling_for(p, false, 0).splits) > 1 ? kSplitScratchBytes : 0;
     out->kind = PB_STAGE_CONV_UMMA;
     out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
     out->threads_per_block = use_tma_a() ? kThreadsTma : kThreads;
@@ -1818,15 +1814,15 @@ int conv_umma_info(const pb_op_params* p, pb_launch_info* out) {
 
 int64_t conv_umma_pack_weights(const pb_op_params* p, const float* w, void* dst) {
     if (!conv_umma_supported(p)) { set_error("conv_umma: unsupported convolution"); return PB_ERR_INVALID; }
-    const Geometry g = geometry(p);
-    const size_t n = (size_t)packed_rows(p) * g.Kdim_pad;
+    const int Cp = round_up(p->Cs, kBK), Kdim_pad = p->R * p->S * Cp;
+    const size_t n = (size_t)packed_rows(p) * Kdim_pad;
     if (dst) {
         memset(dst, 0, n * 2);
         for (int k = 0; k < p->K; ++k)
             for (int c = 0; c < p->C; ++c)
                 for (int r = 0; r < p->R; ++r)
                     for (int s = 0; s < p->S; ++s)
-                        store_elem(dst, (size_t)k * g.Kdim_pad + (size_t)(r * p->S + s) * g.Cp + c,
+                        store_elem(dst, (size_t)k * Kdim_pad + (size_t)(r * p->S + s) * Cp + c,
                                    w[(((size_t)k * p->C + c) * p->R + r) * p->S + s], 1);
     }
     return (int64_t)(n * 2);
@@ -2031,8 +2027,8 @@ static cudaError_t launch_pdl(void (*kern)(Args...), dim3 grid, dim3 cluster, ui
 }
 
 int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap, const pb_op_params* p, cudaStream_t st,
-                             uint32_t job_id, void* notifier, uint32_t* err_flag, bool pdl) {
-    const Geometry g = geometry(p);
+                             uint32_t job_id, void* notifier, uint32_t* err_flag, bool pdl, const ConvTiling* tiling) {
+    const Geometry g = geometry(p, tiling_or(tiling, p));
     if (!use_tma_a()) PB_REQUIRE(batch_of(p) == 1, "conv_umma: the cp.async gather kernel (PB_CONV_GATHER=1) runs one image per launch");
     ConvArgs a;
     const int frc = fill_args(plan, g, p, err_flag, &a);
@@ -2087,28 +2083,23 @@ struct ConvUmmaMulti {
 bool conv_umma_multi_available() { return use_tma_a(); }
 
 // The cluster size of a grouped launch is one for all its convolutions: the one whose slowest member is modelled fastest.
-int conv_umma_common_splits(const pb_op_params* const* params, int n) {
-    const double gain = conv_split_gain_us();
-    if (!use_tma_a() || persist_enabled() || gain > 1e6) return 1;
-    int best = 1;
+void conv_umma_group_tilings(const pb_op_params* const* params, int n, bool shared, bool may_split, ConvTiling* out) {
+    const int most = may_split && !splits_off() ? 8 : 1;
+    int longest = 0;
+    for (int i = 0; i < n; ++i) longest = std::max(longest, conv_shape(params[i], shared).nkb);
     double best_us = 1e30;
-    for (int S = 1; S <= 8; S *= 2) {
-        std::vector<Tiling> t((size_t)n);
-        std::vector<ConvShape> c((size_t)n);
-        int ctas = 0, longest = 0;
+    std::vector<ConvTiling> t((size_t)n);
+    for (int S = 1; S <= most && (S == 1 || longest >= 2 * S); S *= 2) {
+        int ctas = 0;
         for (int i = 0; i < n; ++i) {
-            c[(size_t)i] = conv_shape(params[i]);
-            longest = std::max(longest, c[(size_t)i].nkb);
-            t[(size_t)i] = choose_tiling(c[(size_t)i], bn_limit(), S, gain);
-            ctas += tiling_ctas(c[(size_t)i], t[(size_t)i]);
+            t[(size_t)i] = tiling_for(params[i], shared, S);
+            ctas += tiling_ctas(conv_shape(params[i], shared), t[(size_t)i]);
         }
-        if (S > 1 && longest < 2 * S) break;
-        double us = 0;
-        for (int i = 0; i < n; ++i) us = std::max(us, tiling_us(ctas, c[(size_t)i], t[(size_t)i]));
-        if (S > 1) us += gain / 60.0;
-        if (us < best_us) { best_us = us; best = S; }
+        double us = S > 1 ? conv_split_gain_us() / 60.0 : 0.0, slowest = 0;
+        for (int i = 0; i < n; ++i) slowest = std::max(slowest, tiling_us(ctas, conv_shape(params[i], shared), t[(size_t)i]));
+        us += slowest;
+        if (us < best_us) { best_us = us; std::copy(t.begin(), t.end(), out); }
     }
-    return best;
 }
 
 bool conv_umma_persist_enabled() { return persist_enabled(); }
@@ -2128,7 +2119,7 @@ uint32_t conv_umma_pool_blocks(const pb_op_params* p) {
 }
 
 int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap* const* xmaps, const pb_op_params* const* params, const int* kinds,
-                           int n, ConvUmmaMulti** out) {
+                           const ConvTiling* tilings, int n, ConvUmmaMulti** out) {
     PB_REQUIRE(out && plans && xmaps && params && n >= 1 && n <= kMaxSubConvs, "conv_umma_multi_create: 1..%d entries", kMaxSubConvs);
     PB_REQUIRE(use_tma_a(), "conv_umma_multi_create: needs the TMA operand path");
     std::vector<SubConv> table((size_t)n);
@@ -2141,7 +2132,8 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
     for (int i = 0; i < n; ++i) {
         if (is_pool(i)) continue;
         PB_REQUIRE(plans[i] && xmaps[i] && params[i], "conv_umma_multi_create: NULL entry %d", i);
-        const Geometry g = geometry(params[i], split_allowed(params[i]) && !persist_enabled());
+        const bool split = split_allowed(params[i]) && !persist_enabled();
+        const Geometry g = geometry(params[i], tilings ? tilings[i] : tiling_for(params[i], false, split ? 0 : 1));
         SubConv& sc = table[(size_t)at++];
         int rc = make_tmap(plans[i], g.BN, &sc.tmap_w);
         if (rc == PB_OK) rc = make_ymap(params[i], g.out_box, false, &sc.tmap_y);
@@ -2184,7 +2176,7 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
     m->stages = (int)std::min<uint32_t>(kMaxStages, (kSmemBudgetPersist - 1024u) / m->stage_bytes);
     m->persist_smem = (uint32_t)m->stages * m->stage_bytes + 1024u;
     m->grid = conv_umma_persist_grid(m->total_blocks);
-    m->persist = persist_enabled() && m->stages >= 2 && 2u * m->tmem_cols <= 512u && !m->has_pool;
+    m->persist = persist_enabled() && m->splits == 1 && m->stages >= 2 && 2u * m->tmem_cols <= 512u && !m->has_pool;
     cudaError_t e = cudaMalloc((void**)&m->table_dev, sizeof(SubConv) * (size_t)n);
     if (e == cudaSuccess) e = cudaMemcpy(m->table_dev, table.data(), sizeof(SubConv) * (size_t)n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { conv_umma_multi_destroy(m); return cuda_fail(e, "conv_umma_multi_create", __FILE__, __LINE__); }
@@ -2263,7 +2255,7 @@ int conv_umma_launch(const pb_op_params* p, cudaStream_t st, uint32_t job_id, vo
             const ConvUmmaPlan* plans[1] = {plan};
             const ConvUmmaXMap* xms[1] = {xm};
             const pb_op_params* pp[1] = {p};
-            rc = conv_umma_multi_create(plans, xms, pp, nullptr, 1, &mu);
+            rc = conv_umma_multi_create(plans, xms, pp, nullptr, nullptr, 1, &mu);
         }
         if (rc == PB_OK && !mu->persist) { set_error("conv_umma: this shape does not fit the persistent kernel"); rc = PB_ERR_INVALID; }
         if (rc == PB_OK) rc = conv_umma_multi_launch(mu, st, job_id, notifier, false);
@@ -2294,7 +2286,7 @@ int conv_umma_time(const pb_op_params* p, int mode, int iters, size_t flush_byte
         const ConvUmmaPlan* plans[1] = {plan};
         const ConvUmmaXMap* xms[1] = {xm};
         const pb_op_params* pp[1] = {p};
-        rc = conv_umma_multi_create(plans, xms, pp, nullptr, 1, &mu);
+        rc = conv_umma_multi_create(plans, xms, pp, nullptr, nullptr, 1, &mu);
         if (rc == PB_OK && !mu->persist) { set_error("pb_conv_umma_time: the persistent kernel is off or does not fit this shape"); rc = PB_ERR_INVALID; }
     }
     cudaError_t e = cudaSuccess;
@@ -2366,7 +2358,6 @@ int conv_umma_launch_noalloc(const pb_op_params* p, cudaStream_t st, uint32_t jo
     }
     ConvUmmaPlan plan{p->w, packed_rows(p), p->R * p->S * ceil_div(p->Cs, kBK) * kBK, device};      // on the stack: no host allocation either
     pb_op_params q = *p;
-    q.reserved = 0;
     q.scratch = (void*)nd.err_flag;         // never touched: allows the split, whose partial tiles meet in shared memory
     q.scratch_bytes = kSplitScratchBytes;
     return conv_umma_launch_planned(&plan, nullptr, &q, st, job_id, notifier, nd.err_flag);

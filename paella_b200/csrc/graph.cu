@@ -91,6 +91,7 @@ struct pb_model {
 struct Variant {
     int nb = 1;
     std::vector<pb_op_params> params;       // per stage, pointers resolved
+    std::vector<pb::ConvTiling> tilings;    // per stage: how its convolution is cut (tensor-core convs)
     std::vector<pb::ConvUmmaXMap*> xmaps;   // per stage: im2col descriptor of the stage's input (tensor-core convs)
     std::vector<pb_launch_info> group_info; // per group, for this batch
     std::vector<cudaGraphExec_t> graphs;    // per group; NULL = single kernel, launched directly
@@ -200,30 +201,24 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
     return out;
 }
 
-// pb_op_params.reserved of `stage`: the tiling policy of the model and, when the stage's launch is a grouped one, the
-// cluster size of its convolutions.
-int tile_hint(const pb_model* m, int stage, int nb) {
+// How the tensor-core convolution of `stage` is cut for `nb` images: as a member of the grouped launch it shares by default.
+pb::ConvTiling stage_tiling(const pb_model* m, int stage, int nb) {
     const std::vector<int>& l = m->stages[(size_t)stage].peers;
-    const int policy = (m->shared ? pb::kTileShared : 0) | (m->persist ? 1 : 0);      // the persistent kernel never splits
-    if (l.size() < 2 || m->persist) return policy;
     std::vector<pb_op_params> ps;
     std::vector<const pb_op_params*> pp;
     for (int s : l) {
         ps.push_back(m->stages[(size_t)s].p);
         ps.back().batch = nb;
-        ps.back().reserved = policy;
     }
     for (const pb_op_params& p : ps) pp.push_back(&p);
-    return policy | pb::conv_umma_common_splits(pp.data(), (int)pp.size());
+    const bool may_split = !m->persist;      // the persistent kernel never splits
+    if (l.size() < 2) return pb::conv_umma_tiling(pp[0], m->shared, may_split);
+    std::vector<pb::ConvTiling> t(l.size());
+    pb::conv_umma_group_tilings(pp.data(), (int)l.size(), m->shared, may_split, t.data());
+    return t[(size_t)(std::find(l.begin(), l.end(), stage) - l.begin())];
 }
 
-int op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
-    if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_info(p, out);
-    if (kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(out);
-    return pb::simple_op_info(kind, p, out);
-}
-
-// Launch geometry of stage `stage` when one launch carries `nb` images (scratch offered without limit).
+// Launch geometry of stage `stage` when one launch carries `nb` images.
 int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out) {
     const Stage& st = m->stages[(size_t)stage];
     if (st.kind == PB_STAGE_MNIST_FUSED) {
@@ -233,10 +228,9 @@ int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out
     }
     pb_op_params p = st.p;
     p.batch = nb;
-    p.scratch = (void*)16;
-    p.scratch_bytes = ~0ull;
-    p.reserved = tile_hint(m, stage, nb);
-    return op_info(st.kind, &p, out);
+    if (st.kind != PB_STAGE_CONV_UMMA) return pb_op_info(st.kind, &p, out);
+    const pb::ConvTiling t = stage_tiling(m, stage, nb);
+    return pb::conv_umma_info(&p, out, &t);
 }
 
 // Launch geometry of the stages and groups for one image.
@@ -349,7 +343,7 @@ int launch_stage_with(pb_instance* in, const Variant& v, int stage, const pb_op_
             return pb::mnist_fused_launch(mnist_x, m->w1, m->b1, m->w2, m->b2, m->wd, m->bd, mnist_y, v.nb, stream, job_id, notifier);
         }
         case PB_STAGE_CONV_UMMA:
-            return pb::conv_umma_launch_planned(st.plan, v.xmaps[stage], p, stream, job_id, notifier, nullptr, pdl);
+            return pb::conv_umma_launch_planned(st.plan, v.xmaps[stage], p, stream, job_id, notifier, nullptr, pdl, &v.tilings[stage]);
         default:
             return pb::simple_op_launch(st.kind, p, stream, job_id, notifier, pdl);
     }
@@ -547,6 +541,7 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
     cudaError_t e = cudaSuccess;
     v->params.resize(m->stages.size());
     v->xmaps.assign(m->stages.size(), nullptr);
+    v->tilings.resize(m->stages.size());
     for (size_t i = 0; i < m->stages.size(); ++i) {
         const Stage& st = m->stages[i];
         pb_op_params p = st.p;
@@ -556,9 +551,9 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
         p.residual = st.has_res ? (const void*)(in->arena + cap * st.res_off) : nullptr;
         p.scratch = infos[i].scratch_bytes ? in->arena : nullptr;      // never touched: allows the split (kSplitScratchBytes)
         p.scratch_bytes = infos[i].scratch_bytes;
-        p.reserved = tile_hint(m, (int)i, nb);
         v->params[i] = p;
         if (st.kind == PB_STAGE_CONV_UMMA) {
+            v->tilings[i] = stage_tiling(m, (int)i, nb);
             const int rc = pb::conv_umma_xmap_create(&p, &v->xmaps[i]);
             if (rc != PB_OK) { destroy_variant(v); return rc; }
         }
@@ -579,8 +574,9 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
             std::vector<const pb::ConvUmmaXMap*> xm;
             std::vector<const pb_op_params*> pp;
             std::vector<int> kinds;
-            for (int s : l) { plans.push_back(m->stages[s].plan); xm.push_back(v->xmaps[s]); pp.push_back(&v->params[s]); kinds.push_back(m->stages[s].kind); }
-            const int rc = pb::conv_umma_multi_create(plans.data(), xm.data(), pp.data(), kinds.data(), (int)l.size(), &v->multis[g][li]);
+            std::vector<pb::ConvTiling> tilings;
+            for (int s : l) { plans.push_back(m->stages[s].plan); xm.push_back(v->xmaps[s]); pp.push_back(&v->params[s]); kinds.push_back(m->stages[s].kind); tilings.push_back(v->tilings[(size_t)s]); }
+            const int rc = pb::conv_umma_multi_create(plans.data(), xm.data(), pp.data(), kinds.data(), tilings.data(), (int)l.size(), &v->multis[g][li]);
             if (rc != PB_OK) { destroy_variant(v); return rc; }
         }
     }
@@ -624,18 +620,14 @@ extern "C" {
 
 int pb_op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
     PB_REQUIRE(p && out, "pb_op_info: NULL argument");
-    pb_op_params q = *p;
-    q.reserved = 0;
-    return op_info(kind, &q, out);
+    if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_info(p, out);
+    if (kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(out);
+    return pb::simple_op_info(kind, p, out);
 }
 
 int pb_op_launch(int kind, const pb_op_params* p, void* stream, uint32_t job_id, void* notifier) {
     PB_REQUIRE(p != nullptr, "pb_op_launch: NULL params");
-    if (kind == PB_STAGE_CONV_UMMA) {
-        pb_op_params q = *p;
-        q.reserved = 0;
-        return pb::conv_umma_launch(&q, (cudaStream_t)stream, job_id, notifier);
-    }
+    if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_launch(p, (cudaStream_t)stream, job_id, notifier);
     return pb::simple_op_launch(kind, p, (cudaStream_t)stream, job_id, notifier);
 }
 

@@ -46,7 +46,17 @@ int encode_tiled_bf16(const void* base, int rank, const uint64_t* dims, const ui
 
 // conv_umma.cu: tcgen05 implicit-GEMM convolution (bf16 operands, fp32 accumulation in TMEM)
 bool conv_umma_supported(const pb_op_params* p);
-int conv_umma_info(const pb_op_params* p, pb_launch_info* out);
+// How a launch is cut.  It travels beside pb_op_params: a launch that is given none (NULL below) has the GPU to itself and
+// chooses its own, split only where the caller's scratch memory allows it.
+struct ConvTiling {
+    int BN, splits;        // output channels of a tile, blocks (one cluster) that share its reduction
+    bool tma;              // the tile leaves (and the residual arrives) through TMA
+    bool shared;           // other requests' launches run beside it
+};
+ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split);
+// Tilings of the convolutions of one grouped launch: they share a cluster size.
+void conv_umma_group_tilings(const pb_op_params* const* params, int n, bool shared, bool may_split, ConvTiling* out);
+int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling = nullptr);
 int conv_umma_launch(const pb_op_params* p, cudaStream_t st, uint32_t job_id, void* notifier);
 int64_t conv_umma_pack_weights(const pb_op_params* p, const float* w_oihw, void* dst_host);
 // Per-layer state the tensor-core path needs beyond pb_op_params (the TMA descriptor of the
@@ -63,7 +73,7 @@ void conv_umma_xmap_destroy(ConvUmmaXMap* m);
 // pdl: launch with the programmatic-serialization attribute (the kernel waits for its predecessor
 // itself, after its set-up); only meaningful when the previous operation in `st` is a kernel.
 int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap, const pb_op_params* p, cudaStream_t st,
-                             uint32_t job_id, void* notifier, uint32_t* err_flag = nullptr, bool pdl = false);
+                             uint32_t job_id, void* notifier, uint32_t* err_flag = nullptr, bool pdl = false, const ConvTiling* tiling = nullptr);
 // Grouped launch: up to 8 independent convolutions (their plans, input descriptors and resolved
 // parameters) run as ONE grid; the table of descriptors is copied to device memory here.
 struct ConvUmmaMulti;
@@ -76,16 +86,12 @@ uint32_t conv_umma_persist_grid(uint32_t total_tiles);
 // Footprint of a persistent launch over `total_tiles` tiles whose widest accumulator has `max_tmem_cols` columns.
 void conv_umma_persist_footprint(uint32_t total_tiles, uint32_t max_tmem_cols, pb_launch_info* out);
 // kinds[i] (NULL = all convolutions): PB_STAGE_CONV_UMMA, or PB_STAGE_MAXPOOL / PB_STAGE_AVGPOOL for a 3x3 pooling layer that rides
-// along (conv_umma_pool_fusable; its plan and map entries are NULL).  At least one entry is a convolution.
+// along (conv_umma_pool_fusable; its plan and map entries are NULL).  At least one entry is a convolution.  tilings: one per entry
+// (those of pooling layers are not read), or NULL.
 int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap* const* xmaps, const pb_op_params* const* params, const int* kinds,
-                           int n, ConvUmmaMulti** out);
+                           const ConvTiling* tilings, int n, ConvUmmaMulti** out);
 bool conv_umma_pool_fusable(int kind, const pb_op_params* p);
 uint32_t conv_umma_pool_blocks(const pb_op_params* p);
-// What pb_op_params.reserved carries inside the library (the public entry points ignore it): the cluster size of the
-// grouped launch the convolution is part of (0 = it decides for itself), and whether other requests' launches run beside it.
-constexpr int kTileSplitMask = 0xff, kTileShared = 0x100;
-// Blocks per tile (cluster size) of a grouped launch of these convolutions.
-int conv_umma_common_splits(const pb_op_params* const* params, int n);
 void conv_umma_multi_destroy(ConvUmmaMulti* m);
 void conv_umma_multi_info(const ConvUmmaMulti* m, pb_launch_info* out);
 int conv_umma_multi_launch(const ConvUmmaMulti* m, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);

@@ -670,13 +670,14 @@ __device__ __forceinline__ uint32_t win_finish(uint64_t v, uint64_t bias, float 
     }
     const float2 f = p2_split(v);
     uint32_t h;
-    if (kAct >= 1) asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(f.y), "f"(f.x));
-    else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(f.y), "f"(f.x));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(f.y), "f"(f.x));
+    if (kAct >= 1) h = bits_of(__hmax2(bf2_of(h), bf2_of(0u)));                   // zero for NaN, which cvt.rn.relu would keep
     if (kAct == 2) h = bits_of(__hmin2(bf2_of(h), bf2_of(0x40c040c0u)));          // (6, 6)
     return h;
 }
 template <int kMode, int kAct>
 __device__ __forceinline__ uint32_t win_finish(uint32_t acc, uint64_t bias, float, float, bool tail) {
+    acc = bits_of(__hmax2(bf2_of(acc), bf2_of(0xff80ff80u)));      // a window with nothing but NaN and padding: -infinity
     if (tail) {
         const float2 f = p2_split(p2_add(p2_bf16(acc), bias));
         acc = bits_of(__floats2bfloat162_rn(f.x, f.y));

@@ -1,0 +1,72 @@
+"""The tiled 3x3 window kernel where its values, pointers or surroundings are unusual.  Bit for bit the strip kernels
+(PB_WINDOW_TILE=0), which it stands in for on launches that fill the GPU."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from paella_b200 import capi
+from tests import gpu_util as gu
+from tests.test_gpu_ops import _params
+
+pytestmark = pytest.mark.gpu
+
+KINDS = [(kind, flags, act, bias) for kind, flags, biases in ((capi.STAGE_DWCONV, 0, (True, False)), (capi.STAGE_MAXPOOL, 0, (True, False)),
+                                                              (capi.STAGE_AVGPOOL, 1, (True, False)), (capi.STAGE_AVGPOOL, 0, (True, False)))
+         for act in (0, 1, 2) for bias in biases]
+
+
+def _both(monkeypatch, L, kind, p, y):
+    """Output of the strip kernels and of the tiled kernel for the same parameters, as raw 16-bit words."""
+    import torch
+    outs = []
+    for tile in ("0", "1"):
+        monkeypatch.setenv("PB_WINDOW_TILE", tile)
+        monkeypatch.setenv("PB_WINDOW_TILE_MIN_BLOCKS", "1")
+        y.fill_(3.0)
+        li = capi.LaunchInfo()
+        capi.check(L.pb_op_info(kind, C.byref(p), C.byref(li)), "pb_op_info")
+        assert (li.threads_per_block == 256) == (tile == "0")
+        capi.check(L.pb_op_launch(kind, C.byref(p), None, 0, None), "pb_op_launch")
+        gu.sync()
+        assert gu.error_flag() == 0
+        outs.append(y.view(torch.int16).cpu().numpy().view(np.uint16).copy())
+    return outs
+
+
+def _same_values(a, b, what):
+    """Equal words, any NaN equal to any other, and -0 equal to +0 (the sign of a zero sum is not specified)."""
+    fa, fb = ((v.astype(np.uint32) << 16).view(np.float32) for v in (a, b))
+    np.testing.assert_array_equal(fa, fb, err_msg=str(what))
+
+
+@pytest.mark.parametrize("stride,pad", [(1, 1), (2, 1), (1, 0)])
+@pytest.mark.parametrize("nb", [1, 3])
+def test_special_values_give_what_the_strip_kernels_give(monkeypatch, nb, stride, pad):
+    """NaN, infinities, the largest finite values and whole windows of NaN: a maximum passes over NaN, ReLU makes zero of it,
+    an average keeps it."""
+    import torch
+    L = capi.load()
+    c, h, w = 72, 21, 19
+    P, Q = (h + 2 * pad - 3) // stride + 1, (w + 2 * pad - 3) // stride + 1
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((nb, h, w, c)).astype(np.float32)
+    pick = rng.random(x.shape)
+    for lo, v in ((0.00, np.nan), (0.02, np.inf), (0.04, -np.inf), (0.06, 3.3e38), (0.08, -3.3e38), (0.10, 0.0), (0.13, -0.0)):
+        x[(pick >= lo) & (pick < lo + 0.02)] = v
+    x[:, 4:10, 4:12, :20] = np.nan                        # windows with nothing but NaN
+    x[:, 12:18, 4:12, 8:30] = -np.inf
+    xd = torch.from_numpy(x).cuda().to(torch.bfloat16)
+    wt = rng.standard_normal((c, 1, 3, 3)).astype(np.float32)
+    bd = torch.randn(c, device="cuda")
+    y = torch.zeros((nb, P, Q, c + 16), device="cuda", dtype=torch.bfloat16)
+    for kind, flags, act, bias in KINDS:
+        p = _params(1, (c, h, w), c, P, Q, c + 16, 3, 3, stride, stride, pad, pad, groups=c if kind == capi.STAGE_DWCONV else 1, act=act, flags=flags,
+                    out_c_off=8, Cs=c)
+        p.batch = nb
+        if kind == capi.STAGE_DWCONV:
+            wd = gu.pack_weights(kind, p, wt)
+            p.w = wd.data_ptr()
+        p.x, p.bias, p.y = xd.data_ptr(), bd.data_ptr() if bias else None, y.data_ptr()
+        strip, tile = _both(monkeypatch, L, kind, p, y)
+        _same_values(tile, strip, (kind, flags, act, bias))

@@ -70,3 +70,36 @@ def test_special_values_give_what_the_strip_kernels_give(monkeypatch, nb, stride
         p.x, p.bias, p.y = xd.data_ptr(), bd.data_ptr() if bias else None, y.data_ptr()
         strip, tile = _both(monkeypatch, L, kind, p, y)
         _same_values(tile, strip, (kind, flags, act, bias))
+
+
+@pytest.mark.parametrize("nb", [1, 2])
+def test_pointers_aligned_to_a_pair_of_channels(monkeypatch, nb):
+    """Output and filter that start on a 4-byte boundary give the bits of aligned ones, and nothing beside the output is touched."""
+    import torch
+    L = capi.load()
+    c, h, w = 72, 20, 37
+    x = torch.randn((nb, h, w, c), device="cuda").to(torch.bfloat16)
+    wt = np.random.default_rng(9).standard_normal((c, 1, 3, 3)).astype(np.float32)
+    bd = torch.randn(c, device="cuda")
+    monkeypatch.setenv("PB_WINDOW_TILE_MIN_BLOCKS", "1")
+    for kind, flags in ((capi.STAGE_DWCONV, 0), (capi.STAGE_MAXPOOL, 0), (capi.STAGE_AVGPOOL, 0)):
+        outs = []
+        for shift in (0, 2):                              # elements of two bytes
+            p = _params(1, (c, h, w), c, h, w, c, 3, 3, 1, 1, 1, 1, groups=c if kind == capi.STAGE_DWCONV else 1, act=1, flags=flags, Cs=c)
+            p.batch = nb
+            if kind == capi.STAGE_DWCONV:
+                packed = gu.pack_weights(kind, p, wt).view(torch.bfloat16)
+                wd = torch.zeros(packed.numel() + 8, device="cuda", dtype=torch.bfloat16)
+                wd[shift: shift + packed.numel()] = packed
+                p.w = wd.data_ptr() + 2 * shift
+            y = torch.full((nb * h * w * c + 8,), 3.0, device="cuda", dtype=torch.bfloat16)
+            p.x, p.bias, p.y = x.data_ptr(), bd.data_ptr(), y.data_ptr() + 2 * shift
+            li = capi.LaunchInfo()
+            capi.check(L.pb_op_info(kind, C.byref(p), C.byref(li)), "pb_op_info")
+            assert li.threads_per_block <= 160
+            capi.check(L.pb_op_launch(kind, C.byref(p), None, 0, None), "pb_op_launch")
+            gu.sync()
+            assert gu.error_flag() == 0
+            assert (y[:shift] == 3.0).all() and (y[shift + nb * h * w * c:] == 3.0).all()
+            outs.append(y[shift: shift + nb * h * w * c].clone())
+        assert torch.equal(outs[0], outs[1]), kind

@@ -688,9 +688,13 @@ __device__ __forceinline__ uint32_t win_finish(uint32_t acc, uint64_t bias, floa
     return bits_of(h);
 }
 
+// Raised when the window's copy does not land.  In the module, not allocated: a program's first launch may be inside a stream
+// capture, where nothing may be.
+static __device__ uint32_t g_window_err_flag;
+
 // kWide: output and filter start on an 8-byte boundary, so a lane's four channels are one access; otherwise two of 4 bytes.
 template <int kMode, int kStride, int kAct, bool kCountPad, bool kWide>
-__global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t* err_flag, uint32_t job_id,
+__global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
                                                                         FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
     typedef __nv_bfloat16 T;
@@ -758,7 +762,7 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
         landed = ok != 0;
     }
     if (!landed) {          // the copy is given 50 us more to land before shared memory is released
-        if (threadIdx.x == 0) atomicExch(err_flag, 5u);
+        if (threadIdx.x == 0) atomicExch(&g_window_err_flag, 5u);
         unsigned long long t0, t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
         for (int i = 0; i < (1 << 20); ++i) {
@@ -1399,12 +1403,14 @@ static uint32_t tile_blocks(const pb_op_params* p) {
     const size_t n = (size_t)((p->Cs + kTileSlab - 1) / kTileSlab) * g.col_tiles * ((p->P + g.rows - 1) / g.rows);
     return n * (size_t)batch_of(p) >= least ? (uint32_t)n : 0;
 }
+uint32_t* window_error_flag_ptr() {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_window_err_flag) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return static_cast<uint32_t*>(p);
+}
+
 // Window map of a launch: boxes of one slab x in_cols x in_rows of the images.
-static int win_map(int kind, const pb_op_params* p, const WinTile& g, CUtensorMap* out, uint32_t** err_flag) {
-    int device = 0;
-    PB_CUDA(cudaGetDevice(&device));
-    *err_flag = device_error_flag_ptr(device);
-    PB_REQUIRE(*err_flag != nullptr, "window kernel: no device error flag");
+static int win_map(int kind, const pb_op_params* p, const WinTile& g, CUtensorMap* out) {
     const uint64_t dims[4] = {(uint64_t)p->Cs, (uint64_t)p->W, (uint64_t)p->H, (uint64_t)batch_of(p)};
     const uint64_t strides[3] = {(uint64_t)p->Cs * 2, (uint64_t)p->W * p->Cs * 2, (uint64_t)p->H * p->W * p->Cs * 2};
     const uint32_t box[4] = {(uint32_t)kTileSlab, (uint32_t)g.in_cols, (uint32_t)g.in_rows, 1};
@@ -1661,10 +1667,9 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
                 PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
                 t_launch_smem = (size_t)g.smem;
                 CUtensorMap tmap;
-                uint32_t* err_flag = nullptr;
-                const int mrc = win_map(kind, p, g, &tmap, &err_flag);
+                const int mrc = win_map(kind, p, g, &tmap);
                 if (mrc != PB_OK) return mrc;
-                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t*, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, err_flag, job_id, nf);
+                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, job_id, nf);
                 break;
             }
             if (const int strip = strip_of(p)) {
@@ -1682,10 +1687,9 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
                 PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
                 t_launch_smem = (size_t)g.smem;
                 CUtensorMap tmap;
-                uint32_t* err_flag = nullptr;
-                const int mrc = win_map(kind, p, g, &tmap, &err_flag);
+                const int mrc = win_map(kind, p, g, &tmap);
                 if (mrc != PB_OK) return mrc;
-                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t*, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, err_flag, job_id, nf);
+                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, job_id, nf);
                 break;
             }
             if (const int strip = strip_of(p)) {
@@ -1702,10 +1706,9 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
                 PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
                 t_launch_smem = (size_t)g.smem;
                 CUtensorMap tmap;
-                uint32_t* err_flag = nullptr;
-                const int mrc = win_map(kind, p, g, &tmap, &err_flag);
+                const int mrc = win_map(kind, p, g, &tmap);
                 if (mrc != PB_OK) return mrc;
-                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t*, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, err_flag, job_id, nf);
+                launch_k((void (*)(OpArgs, WinTile, const CUtensorMap, uint32_t, FinishedBlockNotifier*))fn, grid, dim3((unsigned)g.threads), st, pdl, a, g, tmap, job_id, nf);
                 break;
             }
             if (const int strip = strip_of(p)) {

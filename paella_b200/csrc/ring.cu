@@ -188,8 +188,9 @@ int pb_device_error_flag(int device, uint32_t* flag_out, int reset) {
     PB_CUDA(cudaSetDevice(device));
     if (flag_out) PB_CUDA(cudaMemcpy(flag_out, p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     if (reset) PB_CUDA(cudaMemset(p, 0, sizeof(uint32_t)));
-    // the no-allocation convolution path keeps its own flag (it may not share one that was cudaMalloc'ed)
-    if (uint32_t* q = pb::noalloc_error_flag_ptr(device)) {
+    // the no-allocation convolution path and the window kernels keep flags of their own (they may not share one that was cudaMalloc'ed)
+    for (uint32_t* q : {pb::noalloc_error_flag_ptr(device), pb::window_error_flag_ptr()}) {
+        if (!q) continue;
         uint32_t v = 0;
         PB_CUDA(cudaMemcpy(&v, q, sizeof(uint32_t), cudaMemcpyDeviceToHost));
         if (flag_out) *flag_out |= v;      // both flags are reported: neither hides the other

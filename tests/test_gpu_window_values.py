@@ -1,6 +1,9 @@
 """The tiled 3x3 window kernel where its values, pointers or surroundings are unusual.  Bit for bit the strip kernels
 (PB_WINDOW_TILE=0), which it stands in for on launches that fill the GPU."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -103,3 +106,40 @@ def test_pointers_aligned_to_a_pair_of_channels(monkeypatch, nb):
             assert (y[:shift] == 3.0).all() and (y[shift + nb * h * w * c:] == 3.0).all()
             outs.append(y[shift: shift + nb * h * w * c].clone())
         assert torch.equal(outs[0], outs[1]), kind
+
+
+CAPTURED = """
+import ctypes as C, torch
+from paella_b200 import capi
+L = capi.load()
+torch.manual_seed(1)
+x = torch.randn((1, 128, 64, 512), device="cuda").to(torch.bfloat16)
+y = torch.zeros((1, 128, 64, 512), device="cuda", dtype=torch.bfloat16)
+p = capi.OpParams()
+p.dtype, p.C, p.H, p.W, p.Cs, p.K, p.P, p.Q, p.Ks = 1, 512, 128, 64, 512, 512, 128, 64, 512
+p.R, p.S, p.stride_h, p.stride_w, p.pad_h, p.pad_w, p.groups, p.batch = 3, 3, 1, 1, 1, 1, 1, 1
+p.x, p.y = x.data_ptr(), y.data_ptr()
+li = capi.LaunchInfo()
+capi.check(L.pb_op_info(capi.STAGE_MAXPOOL, C.byref(p), C.byref(li)), "pb_op_info")
+assert li.threads_per_block <= 160, "the tiled kernel"
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    rc = L.pb_op_launch(capi.STAGE_MAXPOOL, C.byref(p), torch.cuda.current_stream().cuda_stream, 0, None)
+assert rc == 0, L.pb_last_error()
+g.replay()
+torch.cuda.synchronize()
+want = torch.nn.functional.max_pool2d(x.float().permute(0, 3, 1, 2), 3, 1, 1).permute(0, 2, 3, 1)
+assert torch.equal(y.float(), want)
+flag = C.c_uint32(7)
+capi.check(L.pb_device_error_flag(0, C.byref(flag), 1), "flag")
+assert flag.value == 0
+print("captured")
+"""
+
+
+def test_a_first_launch_may_be_captured():
+    """A program whose first call into the library is a pooling launch inside a stream capture: nothing may be allocated there."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CAPTURED], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]

@@ -1355,7 +1355,9 @@ static size_t strip_threads(const pb_op_params* p, int strip) {
 // Tile of window3_tile_kernel.  A single image is cut into tiles of 8 strips x 13 (stride 2: 6) rows, 65 KB of window.  The
 // images of a batch are mostly small maps, where that tile hangs over the edges (35 columns: a tile of 32 and one of 3, 101 us
 // for 256 images of 35 x 35 x 192 instead of 51), so their tiles are fitted to the map: as few column tiles as hold at most 40 columns
-// each, as many rows as keep the window within 70 KB, and bands of rows where a map has fewer strips than half-warps.
+// each, as many rows as keep the window (the rows a walk runs past the tile included) within 74 KB, so that three blocks fit an SM,
+// and bands of rows where a map has fewer strips than half-warps.
+constexpr int kTileWindowBytes = 74 * 1024;
 static WinTile win_tile(const pb_op_params* p) {
     const int st = p->stride_h, strip = st == 1 ? kTileStrip1 : kTileStrip2;
     WinTile g;
@@ -1370,20 +1372,24 @@ static WinTile win_tile(const pb_op_params* p) {
     }
     g.in_cols = (g.strips * strip - 1) * st + 3;
     if (batch_of(p) > 1) {
-        int fit = ((74 * 1024) / (g.in_cols * kTileSlab * 2) - 3) / st + 1;      // rows of output whose window fits
+        int fit = (kTileWindowBytes / (g.in_cols * kTileSlab * 2) - 3) / st + 1;      // rows of output whose window fits
         if (fit < 1) fit = 1;
         g.rows = p->P < fit ? p->P : fit;
         if (st == 1 && fit < p->P && fit > 3) g.rows = (fit - 1) / 3 * 3 + 1;     // a walk takes three window rows per turn: no turn half used
     }
-    g.bands = g.strips >= 8 ? 1 : (8 / g.strips < g.rows ? 8 / g.strips : g.rows);
-    g.band_rows = ceil_div(g.rows, g.bands);
-    g.bands = ceil_div(g.rows, g.band_rows);
-    const int walked = st == 1 ? ceil_div(g.band_rows + 2, 3) * 3 : 2 * g.band_rows + 1;      // window rows a unit reads
-    g.alloc_rows = (g.bands - 1) * g.band_rows * st + walked;
-    g.in_rows = (g.rows - 1) * st + 3;
-    g.alloc_rows = g.alloc_rows > g.in_rows ? g.alloc_rows : g.in_rows;
+    for (;;) {
+        g.bands = g.strips >= 8 ? 1 : (8 / g.strips < g.rows ? 8 / g.strips : g.rows);
+        g.band_rows = ceil_div(g.rows, g.bands);
+        g.bands = ceil_div(g.rows, g.band_rows);
+        const int walked = st == 1 ? ceil_div(g.band_rows + 2, 3) * 3 : 2 * g.band_rows + 1;      // window rows a unit reads
+        g.alloc_rows = (g.bands - 1) * g.band_rows * st + walked;
+        g.in_rows = (g.rows - 1) * st + 3;
+        g.alloc_rows = g.alloc_rows > g.in_rows ? g.alloc_rows : g.in_rows;
+        g.smem = g.alloc_rows * g.in_cols * kTileSlab * 2;
+        if (g.smem <= kTileWindowBytes || g.rows == 1) break;
+        g.rows = ceil_div(p->P, ceil_div(p->P, g.rows) + 1) < g.rows ? ceil_div(p->P, ceil_div(p->P, g.rows) + 1) : g.rows - 1;      // one more row tile
+    }
     g.threads = 32 * ceil_div(g.strips * g.bands < 10 ? g.strips * g.bands : 10, 2);
-    g.smem = g.alloc_rows * g.in_cols * kTileSlab * 2;
     return g;
 }
 

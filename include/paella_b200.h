@@ -222,7 +222,8 @@ PB_API int pb_model_load(const char* pack_path, int device, int precision, pb_mo
 PB_API void pb_model_destroy(pb_model* m);
 /* Tiling policy of the model's tensor-core launches.  0 (default): a launch has the GPU to itself, so its tiles are cut to
  * finish it soonest.  1: launches of many other requests run beside it (a server's models), so the tiles are cut to occupy
- * the GPU least.  Call it before the model's first instance is created; an instance keeps what it was created with. */
+ * the GPU least.  Call it before the model's first instance is created: after that a change is refused with PB_ERR_INVALID
+ * (what the model declares for a batch size and what its instances launch have to agree). */
 PB_API int pb_model_set_shared_gpu(pb_model* m, int shared);
 PB_API size_t pb_model_input_bytes(const pb_model* m);   /* NCHW fp32 */
 PB_API size_t pb_model_output_bytes(const pb_model* m);  /* fp32 vector */

@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -78,6 +79,7 @@ struct pb_model {
     std::vector<Group> groups;
     bool fuse_branches = false;
     bool shared = false;        // launches of other requests run beside this model's (pb_model_set_shared_gpu)
+    std::atomic<bool> instantiated{false};      // an instance has been created: `shared` is settled
     bool persist = false;       // tensor-core launches of the stage graphs run the persistent (multi-tile) kernel
     // fused MNIST weights (device)
     float *w1 = nullptr, *b1 = nullptr, *w2 = nullptr, *b2 = nullptr, *wd = nullptr, *bd = nullptr;
@@ -956,6 +958,8 @@ void pb_model_destroy(pb_model* m) {
 
 int pb_model_set_shared_gpu(pb_model* m, int shared) {
     PB_REQUIRE(m != nullptr, "pb_model_set_shared_gpu: NULL model");
+    if (m->shared == (shared != 0)) return PB_OK;
+    PB_REQUIRE(!m->instantiated.load(), "pb_model_set_shared_gpu: the model's first instance has been created already");
     m->shared = shared != 0;
     refresh_infos(m);
     return PB_OK;
@@ -982,6 +986,7 @@ int pb_instance_create_batched(pb_model* m, int capacity, int prepare_all, pb_in
     PB_CUDA(cudaSetDevice(m->device));
     pb_instance* in = new pb_instance();
     in->m = m;
+    m->instantiated = true;
     in->cap = capacity;
     in->variants.assign((size_t)capacity, nullptr);
     const size_t cap = (size_t)capacity;

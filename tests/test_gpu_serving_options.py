@@ -44,3 +44,28 @@ def test_persistent_kernel_launches_report_every_block(tmp_path, monkeypatch):
     ref = og.run(og.Pack(packer.MODELS["resnet18"](seed=1234).to_bytes()), x)
     assert float(np.abs(y - ref).max()) <= 1e-2 * float(np.abs(ref).max())
     L.pb_server_destroy(s)
+
+
+def test_tiling_policy_is_fixed_by_the_first_instance(models_dir):
+    """pb_model_set_shared_gpu after an instance exists is refused, unless it changes nothing: batch sizes the instance builds
+    later, and what the model declares for them, keep the policy it was created with."""
+    L = capi.load()
+    path = os.path.join(models_dir, packer.pack_file_name("resnet18"))
+    m, inst, twin = C.c_void_p(), C.c_void_p(), C.c_void_p()
+    capi.check(L.pb_model_load(path.encode(), 0, 1, C.byref(m)), "pb_model_load")
+    capi.check(L.pb_model_set_shared_gpu(m, 1), "before the first instance")
+    capi.check(L.pb_instance_create_batched(m, 8, 0, C.byref(inst)), "instance")
+    assert L.pb_model_set_shared_gpu(m, 0) == -2 and b"instance" in L.pb_last_error()
+    capi.check(L.pb_model_set_shared_gpu(m, 1), "no change")
+    capi.check(L.pb_instance_create_batched(m, 8, 1, C.byref(twin)), "every batch size built at creation")
+    x = np.random.default_rng(2).standard_normal((8, 3, 224, 224), dtype=np.float32)
+    ys = []
+    for i in (inst, twin):
+        y = np.zeros((8, 1000), np.float32)
+        capi.check(L.pb_instance_run_batch_sync(i, 8, 1, x.ctypes.data, y.ctypes.data), "run")
+        ys.append(y)
+    np.testing.assert_array_equal(ys[0], ys[1])
+    for i in (inst, twin):
+        L.pb_instance_destroy(i)
+    assert L.pb_model_set_shared_gpu(m, 0) == -2          # (launch geometry has been handed out for it)
+    L.pb_model_destroy(m)

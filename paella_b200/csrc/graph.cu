@@ -19,6 +19,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -79,6 +81,9 @@ struct pb_model {
     std::vector<Group> groups;
     bool fuse_branches = false;
     bool shared = false;        // launches of other requests run beside this model's (pb_model_set_shared_gpu)
+    struct Tilings { double gain_us; bool shared; std::shared_ptr<const std::vector<pb::ConvTiling>> by_stage; };
+    mutable std::mutex tilings_mu;
+    mutable Tilings tilings[pb::kMaxGang + 1];      // by batch size: see tilings_for()
     std::atomic<bool> instantiated{false};      // an instance has been created: `shared` is settled
     bool persist = false;       // tensor-core launches of the stage graphs run the persistent (multi-tile) kernel
     // fused MNIST weights (device)
@@ -203,21 +208,33 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
     return out;
 }
 
-// How the tensor-core convolution of `stage` is cut for `nb` images: as a member of the grouped launch it shares by default.
-pb::ConvTiling stage_tiling(const pb_model* m, int stage, int nb) {
-    const std::vector<int>& l = m->stages[(size_t)stage].peers;
-    std::vector<pb_op_params> ps;
-    std::vector<const pb_op_params*> pp;
-    for (int s : l) {
-        ps.push_back(m->stages[(size_t)s].p);
-        ps.back().batch = nb;
-    }
-    for (const pb_op_params& p : ps) pp.push_back(&p);
+// How the tensor-core convolutions of the model are cut for `nb` images, by stage: as members of the grouped launches they share
+// by default.  A search takes microseconds per convolution and cluster size, and every instance, stage declaration and gang size
+// asks, so the model keeps the last answer per batch size.
+std::shared_ptr<const std::vector<pb::ConvTiling>> tilings_for(const pb_model* m, int nb) {
+    std::lock_guard<std::mutex> lk(m->tilings_mu);
+    pb_model::Tilings& kept = m->tilings[nb];
+    const double gain = pb::conv_split_gain_us();
+    if (kept.by_stage && kept.gain_us == gain && kept.shared == m->shared) return kept.by_stage;
+    auto by_stage = std::make_shared<std::vector<pb::ConvTiling>>(m->stages.size());
     const bool may_split = !m->persist;      // the persistent kernel never splits
-    if (l.size() < 2) return pb::conv_umma_tiling(pp[0], m->shared, may_split);
-    std::vector<pb::ConvTiling> t(l.size());
-    pb::conv_umma_group_tilings(pp.data(), (int)l.size(), m->shared, may_split, t.data());
-    return t[(size_t)(std::find(l.begin(), l.end(), stage) - l.begin())];
+    for (size_t i = 0; i < m->stages.size(); ++i) {
+        const std::vector<int>& l = m->stages[i].peers;
+        if (m->stages[i].kind != PB_STAGE_CONV_UMMA || l.front() != (int)i) continue;
+        std::vector<pb_op_params> ps;
+        std::vector<const pb_op_params*> pp;
+        for (int s : l) {
+            ps.push_back(m->stages[(size_t)s].p);
+            ps.back().batch = nb;
+        }
+        for (const pb_op_params& p : ps) pp.push_back(&p);
+        std::vector<pb::ConvTiling> t(l.size());
+        if (l.size() == 1) t[0] = pb::conv_umma_tiling(pp[0], m->shared, may_split);
+        else pb::conv_umma_group_tilings(pp.data(), (int)l.size(), m->shared, may_split, t.data());
+        for (size_t k = 0; k < l.size(); ++k) (*by_stage)[(size_t)l[k]] = t[k];
+    }
+    kept = {gain, m->shared, by_stage};
+    return by_stage;
 }
 
 // Launch geometry of stage `stage` when one launch carries `nb` images.
@@ -231,8 +248,7 @@ int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out
     pb_op_params p = st.p;
     p.batch = nb;
     if (st.kind != PB_STAGE_CONV_UMMA) return pb_op_info(st.kind, &p, out);
-    const pb::ConvTiling t = stage_tiling(m, stage, nb);
-    return pb::conv_umma_info(&p, out, &t);
+    return pb::conv_umma_info(&p, out, &(*tilings_for(m, nb))[(size_t)stage]);
 }
 
 // Launch geometry of the stages and groups for one image.
@@ -543,7 +559,7 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
     cudaError_t e = cudaSuccess;
     v->params.resize(m->stages.size());
     v->xmaps.assign(m->stages.size(), nullptr);
-    v->tilings.resize(m->stages.size());
+    v->tilings = *tilings_for(m, nb);
     for (size_t i = 0; i < m->stages.size(); ++i) {
         const Stage& st = m->stages[i];
         pb_op_params p = st.p;
@@ -555,7 +571,6 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
         p.scratch_bytes = infos[i].scratch_bytes;
         v->params[i] = p;
         if (st.kind == PB_STAGE_CONV_UMMA) {
-            v->tilings[i] = stage_tiling(m, (int)i, nb);
             const int rc = pb::conv_umma_xmap_create(&p, &v->xmaps[i]);
             if (rc != PB_OK) { destroy_variant(v); return rc; }
         }

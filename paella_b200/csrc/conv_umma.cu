@@ -1655,18 +1655,29 @@ ConvTiling best_tiling(const ConvShape& c, int bn_max, int want_splits, double g
     return best;
 }
 
-// The search takes 1 to 6 us, as long as a launch (and an instance with grouped launches asks for the same tilings several
-// times): a thread keeps the tilings of its last shapes.
+// The search takes 1 to 6 us, as long as a launch: the tilings of the last shapes that operator calls asked for are kept.  The
+// table is the library's and not a thread's (thread-local storage is allocated when a thread first touches it, which
+// pb_conv2d_umma_noalloc may not do); a thread that finds it in use searches for itself.
 ConvTiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double gain_us) {
     struct Kept { ConvShape c; int bn_max, want_splits; double gain_us; ConvTiling t; };
-    static thread_local Kept kept[256] = {};
+    static Kept kept[256];                       // BN 0: empty
+    static std::atomic_flag busy = ATOMIC_FLAG_INIT;
     unsigned slot = (unsigned)c.m_tiles * 8191u + (unsigned)c.Kp16 * 131u + (unsigned)c.nkb * 8u + (unsigned)want_splits + (c.residual ? 4u : 0u);
     slot ^= slot >> 8;
     Kept& k = kept[slot % 256u];
-    if (k.t.BN == 0 || k.c.m_tiles != c.m_tiles || k.c.Kp16 != c.Kp16 || k.c.nkb != c.nkb || k.c.residual != c.residual || k.c.shared != c.shared ||
-        k.bn_max != bn_max || k.want_splits != want_splits || k.gain_us != gain_us)
-        k = {c, bn_max, want_splits, gain_us, best_tiling(c, bn_max, want_splits, gain_us)};
-    return k.t;
+    if (!busy.test_and_set(std::memory_order_acquire)) {
+        const Kept found = k;
+        busy.clear(std::memory_order_release);
+        if (found.t.BN != 0 && found.c.m_tiles == c.m_tiles && found.c.Kp16 == c.Kp16 && found.c.nkb == c.nkb && found.c.residual == c.residual &&
+            found.c.shared == c.shared && found.bn_max == bn_max && found.want_splits == want_splits && found.gain_us == gain_us)
+            return found.t;
+    }
+    const ConvTiling t = best_tiling(c, bn_max, want_splits, gain_us);
+    if (!busy.test_and_set(std::memory_order_acquire)) {
+        k = {c, bn_max, want_splits, gain_us, t};
+        busy.clear(std::memory_order_release);
+    }
+    return t;
 }
 
 ConvShape conv_shape(const pb_op_params* p, bool shared) {

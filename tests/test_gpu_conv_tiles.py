@@ -18,7 +18,7 @@ F32_CASES = [
     (16, 8, 8, 8, 1, 1, 1, 1, 0, 0),          # smallest layer it takes: one tile, one half-filled stage, half a 16-column tile
     (32, 13, 5, 64, 1, 1, 1, 1, 0, 0),        # 65 rows: one row in the second tile; exactly one stage
     (33, 9, 7, 65, 1, 1, 1, 1, 0, 0),         # 63 rows, channels past a stage (36 with padding), one column in the second tile
-    (7, 12, 12, 30, 3, 3, 1, 1, 1, 1),        # channel padding inside every tap; 30 columns: weights not 16-byte aligned
+    (7, 12, 12, 30, 3, 3, 1, 1, 1, 1),        # channel padding inside every tap; 30 columns: rows of weights padded to 32
     (20, 11, 11, 17, 3, 3, 2, 2, 0, 0),       # 17 columns of a 32-column tile, stride 2
     (3, 40, 40, 64, 7, 7, 2, 2, 3, 3),        # stem: a tap per chunk of four channels
     (256, 7, 7, 512, 3, 3, 1, 1, 1, 1),       # 49 rows, 72 stages: split over a cluster of 8
@@ -38,13 +38,42 @@ def test_conv_f32_slice_and_dilation():
     _run_conv(capi.STAGE_CONV_SIMT, 0, 16, 19, 23, 16, 3, 3, 1, 1, 2, 3, dilation=(2, 3))
 
 
+@pytest.mark.parametrize("cols", [16, 24, 72])
+def test_conv_f32_weights_on_a_4_byte_boundary(cols):
+    """Weights that do not start on a 16-byte boundary take another instance of each of the three tile widths (16, 32, 64
+    columns): same order of additions, so the bits of the aligned ones."""
+    import torch
+    L = capi.load()
+    c, h = 20, 11
+    x = torch.randn((h, h, c), device="cuda")
+    w = RNG.standard_normal((cols, c, 3, 3), dtype=np.float32)
+    p = _params(0, (c, h, h), cols, h, h, cols, 3, 3, 1, 1, 1, 1, 1, 1, 0, 0, c)
+    packed = gu.pack_weights(capi.STAGE_CONV_SIMT, p, w).view(torch.float32)
+    outs = []
+    for shift in (0, 1, 3):
+        wd = torch.full((packed.numel() + 4,), float("nan"), device="cuda")
+        wd[shift: shift + packed.numel()] = packed
+        y = torch.full((h, h, cols), 7.0, device="cuda")
+        p.x, p.w, p.y = x.data_ptr(), wd.data_ptr() + 4 * shift, y.data_ptr()
+        capi.check(L.pb_op_launch(capi.STAGE_CONV_SIMT, C.byref(p), None, 0, None), "pb_op_launch")
+        gu.sync()
+        outs.append(y)
+    ref = og.conv2d(np.ascontiguousarray(x.permute(2, 0, 1).cpu().numpy()), w, None, (1, 1), (1, 1), 1, 1, None)
+    _assert_close(gu.from_device_cl(outs[0], cols), ref, 0)
+    assert torch.equal(outs[1], outs[0]) and torch.equal(outs[2], outs[0])
+
+
 UMMA_SPLITS = [
-    # C, H, W, K, R, S, sh, sw, ph, pw        (tiles of 128 rows; a k-block is 64 channels of one tap)
-    (256, 8, 16, 32, 1, 1, 1, 1, 0, 0),       # exactly one row tile, four k-blocks
-    (128, 3, 43, 40, 3, 3, 1, 1, 1, 1),       # 129 rows, 40 columns: the last tile is mostly outside
-    (448, 8, 8, 384, 3, 3, 1, 1, 1, 1),       # 63 k-blocks: ranks with unequal shares
-    (512, 7, 7, 512, 3, 3, 1, 1, 1, 1),       # 72 k-blocks on half a row tile
-    (192, 17, 17, 200, 1, 7, 1, 1, 0, 3),     # 21 k-blocks, 200 columns
+    # C, H, W, K, R, S, sh, sw, ph, pw, blocks     (tiles of 128 rows; a k-block is 64 channels of one tap)
+    (64, 28, 28, 16, 3, 3, 1, 1, 1, 1, 14),       # 2 ranks on each of 7 row tiles, 8 columns each; 9 k-blocks: 4 and 5
+    (128, 70, 70, 40, 3, 3, 1, 1, 1, 1, 78),      # 2 ranks on 39 row tiles, 24 columns each: an odd number of octets
+    (64, 8, 16, 16, 3, 3, 1, 1, 1, 1, 4),         # 4 ranks on exactly one row tile; 9 k-blocks
+    (192, 56, 56, 80, 3, 3, 1, 1, 1, 1, 100),     # 4 ranks on 25 row tiles, 24 columns each
+    (256, 7, 7, 16, 3, 3, 1, 1, 1, 1, 8),         # 8 ranks on one tile, 8 columns each
+    (128, 3, 43, 40, 3, 3, 1, 1, 1, 1, 16),       # 129 rows, 40 columns: the last tile is mostly outside
+    (448, 8, 8, 384, 3, 3, 1, 1, 1, 1, 48),       # 63 k-blocks: ranks with unequal shares
+    (512, 7, 7, 512, 3, 3, 1, 1, 1, 1, 64),       # 72 k-blocks on half a row tile
+    (192, 17, 17, 200, 1, 7, 1, 1, 0, 3, 84),     # 21 k-blocks, 200 columns
 ]
 
 
@@ -52,7 +81,12 @@ UMMA_SPLITS = [
 @pytest.mark.parametrize("case", UMMA_SPLITS)
 def test_conv_umma_cluster_split(case, act):
     """Split over a cluster (scratch allows it), with a residual and an output slice."""
-    _run_conv(capi.STAGE_CONV_UMMA, 1, *case, act=act, residual=True, scratch=True, out_total=case[3] + 24, off=16)
+    L = capi.load()
+    L.pb_set_conv_split_gain_us(0.0)
+    try:
+        _run_conv(capi.STAGE_CONV_UMMA, 1, *case[:10], act=act, residual=True, scratch=True, split_blocks=case[10], out_total=case[3] + 24, off=16)
+    finally:
+        L.pb_set_conv_split_gain_us(-1.0)
 
 
 WIDE = [

@@ -1,5 +1,5 @@
 """The tiled 3x3 window kernel on batches, whose tiles are fitted to the map: widths and heights around a strip, a band and a
-tile, channel counts off the slab and the vector, pooling with the bias + activation tail.  Bit for bit the strip kernels
+tile, channel counts off the slab and off the vector, pooling with the bias + activation tail.  Bit for bit the strip kernels
 (PB_WINDOW_TILE=0) on the same launch."""
 import ctypes as C
 
@@ -16,6 +16,8 @@ CASES = [
     # N, C, H, W, stride, pad
     (2, 64, 35, 35, 1, 1), (3, 72, 17, 17, 1, 1), (2, 8, 8, 8, 1, 1), (2, 200, 4, 3, 1, 1), (2, 64, 41, 81, 1, 1), (2, 128, 14, 1, 1, 1),
     (2, 64, 71, 71, 2, 0), (3, 40, 35, 36, 2, 1), (2, 64, 7, 7, 2, 1), (2, 24, 3, 90, 2, 1), (2, 16, 64, 40, 1, 0),
+    # channels past the last vector (stored as zeros): one, two and three of four missing, past a slab
+    (2, 20, 9, 10, 1, 1), (3, 69, 17, 17, 1, 1), (2, 131, 12, 40, 1, 1), (2, 67, 15, 15, 2, 1), (1, 133, 40, 33, 1, 1),
 ]
 
 
@@ -57,4 +59,4 @@ def test_tiles_of_a_batch_equal_the_strip_kernels(case, monkeypatch):
             outs.append(y.float().cpu().numpy())
         assert blocks[0] <= 160 and blocks[1] == 256
         np.testing.assert_array_equal(outs[0], outs[1], err_msg=str((kind, flags, act, bias)))
-        assert (outs[0][..., :8] == 3.0).all() and (outs[0][..., 8 + cs:] == 3.0).all()
+        assert (outs[0][..., :8] == 3.0).all() and (outs[0][..., 8 + cs:] == 3.0).all() and (outs[0][..., 8 + c: 8 + cs] == 0.0).all()

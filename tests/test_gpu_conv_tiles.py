@@ -126,3 +126,28 @@ def test_conv_umma_many_tiles(case, residual):
     for i in (0, nb // 2, nb - 1):
         _assert_close(got[i, off:off + K], og.conv2d(x[i], w, b, (1, 1), (R // 2, R // 2), 1, 1, res[i] if residual else None), 1)
     assert (got[:, :off] == 7.0).all() and (got[:, off + K:] == 7.0).all()
+
+
+@pytest.mark.parametrize("c,cs,k,r", [(7, 8, 16, 3), (24, 40, 24, 3), (33, 36, 72, 1), (5, 32, 64, 5)])
+def test_conv_f32_reads_its_own_channels_only(c, cs, k, r):
+    """Channels from C to the stride Cs belong to nobody (padding) or to another layer (a prefix of a concatenation): whatever they
+    hold, NaN included, the result is that of zeros there."""
+    import torch
+    L = capi.load()
+    h = 9
+    gen = torch.Generator(device="cuda").manual_seed(c)
+    x = torch.full((h, h, cs), float("nan"), device="cuda")
+    x[..., :c] = torch.randn((h, h, c), generator=gen, device="cuda")
+    w = RNG.standard_normal((k, c, r, r), dtype=np.float32) * np.float32(np.sqrt(2.0 / (c * r * r)))
+    p = _params(0, (c, h, h), k, h, h, k, r, r, 1, 1, r // 2, r // 2, 1, 0, 0, 0, cs)
+    wd = gu.pack_weights(capi.STAGE_CONV_SIMT, p, w)
+    outs = []
+    for t in (x, torch.nan_to_num(x)):
+        y = torch.full((h, h, k), 7.0, device="cuda")
+        p.x, p.w, p.y = t.data_ptr(), wd.data_ptr(), y.data_ptr()
+        capi.check(L.pb_op_launch(capi.STAGE_CONV_SIMT, C.byref(p), None, 0, None), "pb_op_launch")
+        gu.sync()
+        outs.append(y)
+    ref = og.conv2d(np.ascontiguousarray(x[..., :c].permute(2, 0, 1).cpu().numpy()), w, None, (1, 1), (r // 2, r // 2), 1, 0, None)
+    _assert_close(gu.from_device_cl(outs[1], k), ref, 0)
+    assert torch.equal(outs[0], outs[1])

@@ -1795,6 +1795,11 @@ bool conv_umma_supported(const pb_op_params* p) {
 
 ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split) { return tiling_for(p, shared, may_split ? 0 : 1); }
 
+double conv_umma_us(const pb_op_params* p, const ConvTiling& t) {
+    const ConvShape c = conv_shape(p, t.shared);
+    return tiling_us(tiling_ctas(c, t), c, t);
+}
+
 int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling) {
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
     const Geometry g = geometry(p, tiling_or(tiling, p));

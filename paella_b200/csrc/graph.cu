@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -157,57 +158,6 @@ bool uses_multi(const pb_model* m, const std::vector<int>& l) {
     return m->persist && m->stages[(size_t)l[0]].kind == PB_STAGE_CONV_UMMA;
 }
 
-// What group `g` declares to the scheduler, from its stages' launch geometry `infos` (per stage): only the
-// LAST launch of a group reports block start/end, so the declared block count is that launch's grid; the
-// per-block resources are scaled so that blocks x per-block equals the mean footprint of the group's launches, which
-// run one after the other: what the stage occupies on average while it is in flight.  (With the LARGEST footprint, a
-// ResNet-18 request - one stage - held what its 98-block stem convolution needs from start to end: four requests filled
-// the GPU's shared memory and 32 of them took 1620 us instead of 970.)
-pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_launch_info>& infos) {
-    const pb_model::Group& grp = m->groups[(size_t)g];
-    pb_launch_info out;
-    memset(&out, 0, sizeof(out));
-    uint64_t thr = 0, smem = 0, regs = 0, tmem = 0, nb = 0;
-    for (const std::vector<int>& l : grp.launches) {
-        uint64_t lt = 0, ls = 0, lr = 0, lm = 0, lb = 0;
-        uint32_t max_tmem = 0;
-        for (int i : l) {
-            const pb_launch_info& li = infos[(size_t)i];
-            lb += li.num_blocks;
-            lt += (uint64_t)li.num_blocks * li.threads_per_block;
-            ls += (uint64_t)li.num_blocks * li.smem_per_block;
-            lr += (uint64_t)li.num_blocks * li.threads_per_block * li.regs_per_thread;
-            lm += (uint64_t)li.num_blocks * li.tmem_cols_per_block;
-            max_tmem = std::max(max_tmem, li.tmem_cols_per_block);
-            out.flops += li.flops;
-            out.bytes += li.bytes;
-        }
-        if (uses_multi(m, l)) {
-            // the launch's tiles (lb) are walked by fewer, longer-lived CTAs
-            pb_launch_info pf;
-            pb::conv_umma_persist_footprint((uint32_t)lb, max_tmem, &pf);
-            if (m->persist && 2u * max_tmem <= 512u) {
-                lb = pf.num_blocks;
-                lt = lb * pf.threads_per_block;
-                ls = lb * pf.smem_per_block;
-                lr = lt * pf.regs_per_thread;
-                lm = lb * pf.tmem_cols_per_block;
-            }
-        }
-        thr += lt; smem += ls; regs += lr; tmem += lm;
-        nb = lb;
-    }
-    const uint64_t n = grp.launches.size();
-    thr = std::max(pb::ceil_div(thr, n), nb); smem /= n; regs /= n; tmem /= n;
-    out.kind = grp.count == 1 ? infos[(size_t)grp.first].kind : 0xFFFFu;
-    out.num_blocks = (uint32_t)nb;
-    out.threads_per_block = (uint32_t)pb::ceil_div<uint64_t>(thr, nb);
-    out.smem_per_block = (uint32_t)pb::ceil_div<uint64_t>(smem, nb);
-    out.regs_per_thread = (uint32_t)pb::ceil_div<uint64_t>(regs, (uint64_t)out.threads_per_block * nb);
-    out.tmem_cols_per_block = (uint32_t)pb::ceil_div<uint64_t>(tmem, nb);
-    return out;
-}
-
 // How the tensor-core convolutions of the model are cut for `nb` images, by stage: as members of the grouped launches they share
 // by default.  A search takes microseconds per convolution and cluster size, and every instance, stage declaration and gang size
 // asks, so the model keeps the last answer per batch size.
@@ -237,6 +187,74 @@ std::shared_ptr<const std::vector<pb::ConvTiling>> tilings_for(const pb_model* m
     return by_stage;
 }
 
+// What group `g` declares to the scheduler, from its stages' launch geometry `infos` (per stage) for `nb` images: only the
+// LAST launch of a group reports block start/end, so the declared block count is that launch's grid; the
+// per-block resources are scaled so that blocks x per-block equals the mean footprint of the group's launches over the time
+// they take, one after the other: what the stage occupies on average while it is in flight.  Times are modelled: convolutions
+// by what their tiles are chosen with, other kernels as 2.5 us and the longer of their bytes at 3 TB/s and their operations at
+// 30 TFLOP/s.
+// Measured, largest footprint / plain mean over launches / mean over time: 32 ResNet-18 requests 1492 / 812 / 795 us (with the
+// largest a ResNet-18 request - one stage - holds what its 98-block stem needs from start to end, and four fill the GPU);
+// 64 of MobileNet and ResNet-50 1700 / 1692 / 1738 us; MNIST : Inception-v3 = 9 : 1 under Poisson arrivals, thousand requests a
+// second inside the latency bounds 301 / 291 / 303 (with launches of 4 and 40 us alike too many requests get in, and gangs stay
+// small).
+pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_launch_info>& infos, int nb) {
+    const pb_model::Group& grp = m->groups[(size_t)g];
+    const auto tilings = tilings_for(m, nb);
+    pb_launch_info out;
+    memset(&out, 0, sizeof(out));
+    double us = 0, thr = 0, smem = 0, regs = 0, tmem = 0;      // sums over launches of time x footprint
+    uint64_t blocks = 0;
+    for (const std::vector<int>& l : grp.launches) {
+        uint64_t lt = 0, ls = 0, lr = 0, lm = 0, lb = 0;
+        uint32_t max_tmem = 0;
+        for (int i : l) {
+            const pb_launch_info& li = infos[(size_t)i];
+            lb += li.num_blocks;
+            lt += (uint64_t)li.num_blocks * li.threads_per_block;
+            ls += (uint64_t)li.num_blocks * li.smem_per_block;
+            lr += (uint64_t)li.num_blocks * li.threads_per_block * li.regs_per_thread;
+            lm += (uint64_t)li.num_blocks * li.tmem_cols_per_block;
+            max_tmem = std::max(max_tmem, li.tmem_cols_per_block);
+            out.flops += li.flops;
+            out.bytes += li.bytes;
+        }
+        if (uses_multi(m, l)) {
+            // the launch's tiles (lb) are walked by fewer, longer-lived CTAs
+            pb_launch_info pf;
+            pb::conv_umma_persist_footprint((uint32_t)lb, max_tmem, &pf);
+            if (m->persist && 2u * max_tmem <= 512u) {
+                lb = pf.num_blocks;
+                lt = lb * pf.threads_per_block;
+                ls = lb * pf.smem_per_block;
+                lr = lt * pf.regs_per_thread;
+                lm = lb * pf.tmem_cols_per_block;
+            }
+        }
+        double t = 0;
+        for (int i : l) {
+            const Stage& st = m->stages[(size_t)i];
+            double one = 2.5 + std::max((double)infos[(size_t)i].bytes / 3e6, (double)infos[(size_t)i].flops / 30e6);
+            if (st.kind == PB_STAGE_CONV_UMMA) {
+                pb_op_params p = st.p;
+                p.batch = nb;
+                one = pb::conv_umma_us(&p, (*tilings)[(size_t)i]);
+            }
+            t = std::max(t, one);
+        }
+        us += t; thr += t * (double)lt; smem += t * (double)ls; regs += t * (double)lr; tmem += t * (double)lm;
+        blocks = lb;
+    }
+    out.kind = grp.count == 1 ? infos[(size_t)grp.first].kind : 0xFFFFu;
+    const auto per_block = [&](double sum) { return (uint32_t)std::ceil(sum / us / (double)blocks); };
+    out.num_blocks = (uint32_t)blocks;
+    out.threads_per_block = std::max(per_block(thr), 1u);
+    out.smem_per_block = per_block(smem);
+    out.regs_per_thread = (uint32_t)std::ceil(regs / us / ((double)out.threads_per_block * (double)blocks));
+    out.tmem_cols_per_block = per_block(tmem);
+    return out;
+}
+
 // Launch geometry of stage `stage` when one launch carries `nb` images.
 int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out) {
     const Stage& st = m->stages[(size_t)stage];
@@ -259,7 +277,7 @@ void refresh_infos(pb_model* m) {
     for (size_t gi = 0; gi < m->groups.size(); ++gi) {
         std::vector<pb_launch_info> infos(m->stages.size());
         for (size_t i = 0; i < m->stages.size(); ++i) infos[i] = m->stages[i].info;
-        m->groups[gi].info = group_footprint(m, (int)gi, infos);
+        m->groups[gi].info = group_footprint(m, (int)gi, infos, 1);
     }
 }
 
@@ -576,7 +594,7 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
         }
     }
     v->group_info.resize(m->groups.size());
-    for (size_t g = 0; g < m->groups.size(); ++g) v->group_info[g] = group_footprint(m, (int)g, infos);
+    for (size_t g = 0; g < m->groups.size(); ++g) v->group_info[g] = group_footprint(m, (int)g, infos, nb);
     v->graphs.assign(m->groups.size(), nullptr);
     v->multis.resize(m->groups.size());
     // descriptor tables of the launches that go through one (grouped convolutions; with the persistent kernel
@@ -1076,7 +1094,7 @@ int pb_model_group_info_batched(const pb_model* m, int group, int batch, pb_laun
         const int rc = stage_info_batched(m, i, batch, &infos[(size_t)i]);
         if (rc != PB_OK) return rc;
     }
-    *out = group_footprint(m, group, infos);
+    *out = group_footprint(m, group, infos, batch);
     return PB_OK;
 }
 

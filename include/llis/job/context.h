@@ -33,10 +33,6 @@ class Context {
     // may free what its jobs of that server hold on the device.
     static void* get_owner();
     static void set_owner(void* owner);
-    // Stream of the calling server on which a plugin may start a request's input copy when the request is admitted, long
-    // before its first stage is dispatched (in admission order; NULL = the server has none: copy with the first stage).
-    static cudaStream_t get_input_stream();
-    static void set_input_stream(cudaStream_t stream);
     static unsigned max_gang();
     static void set_max_gang(unsigned n);
     static Job* const* get_gang(unsigned* num_followers);

@@ -25,7 +25,6 @@ pb_server::~pb_server() {
         if (release_t fn = (release_t)dlsym(t->dl_handle, "pb_plugin_release")) fn(this);
     }
     for (cudaStream_t s : streams) cudaStreamDestroy(s);
-    if (input_stream) cudaStreamDestroy(input_stream);
     if (notifiers_raw) llis::job::FinishedBlockNotifier::free_array(notifiers_raw);
     // Plugin instances are never destroyed (their class has no virtual destructor in the
     // plugin ABI); device memory they hold goes away with the context.
@@ -97,7 +96,6 @@ int pb_server::init(const pb_server_config& c) {
         return PB_ERR_CUDA;
     }
     Context::set_gpu2sched_channel(&channel);
-    PB_CUDA(cudaStreamCreateWithFlags(&input_stream, cudaStreamNonBlocking));
     streams.resize(sc.num_streams);
     std::vector<llis::job::FinishedBlockNotifier*> nfs(sc.num_streams);
     for (unsigned i = 0; i < sc.num_streams; ++i) {
@@ -142,7 +140,6 @@ int pb_server::launch(uint32_t job_ref_id, void* io_ptr, uint64_t cookie, llis::
     Context::set_device_resident(cfg.device_resident != 0);
     Context::set_max_gang(cfg.max_gang > 1 ? cfg.max_gang : 1);
     Context::set_owner(this);
-    Context::set_input_stream(input_stream);
     job->set_remote_ptr((void*)(uintptr_t)cookie);
     if (fresh) {
         job->set_client_details(client_id, t.id);

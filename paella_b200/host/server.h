@@ -92,7 +92,6 @@ struct pb_server final : public llis::server::SchedulerHost {
     int device = 0;
     llis::ipc::Gpu2SchedChannel channel;
     std::vector<cudaStream_t> streams;
-    cudaStream_t input_stream = nullptr;       // input copies of admitted requests, one after the other
     llis::job::FinishedBlockNotifier* notifiers_raw = nullptr;
     std::unique_ptr<llis::server::Scheduler> scheduler;
     std::vector<std::unique_ptr<llis::server::JobType>> types;

@@ -59,8 +59,7 @@ class ModelJob : public llis::job::Job {
         if (cap_ < 1) cap_ = 1;
         // every gang size is prepared now (descriptors, graphs): nothing is built on the serving path
         if (pb_instance_create_batched(model, cap_, 1, &inst_) != PB_OK) { set_error(PB_ERR_CUDA); return; }
-        check(cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming));
-        remember(llis::job::Context::get_owner(), Held{inst_, copied_});
+        remember(llis::job::Context::get_owner(), inst_);
         const int n = pb_model_num_groups(model);
         decls_.resize((size_t)n * (size_t)cap_);          // [group][gang size - 1]
         for (int i = 0; i < n; ++i)
@@ -83,7 +82,6 @@ class ModelJob : public llis::job::Job {
         next_ = 0;
         gang_n_ = 1;
         resident_ = llis::job::Context::device_resident();
-        start_input_copy();
         declare();
     }
 
@@ -109,12 +107,15 @@ class ModelJob : public llis::job::Job {
             for (int i = 0; i < gang_n_; ++i) {
                 char* io = i == 0 ? io_ptr_ : static_cast<ModelJob*>(follow[i - 1])->io_ptr_;     // followers are jobs of this type
                 ins[i] = direct_io ? io : nullptr;
-                outs[i] = direct_io ? io + get_output_offset() : nullptr;
+                // Loads issued by SMs keep few PCIe reads in flight (about 11 GB/s measured); a copy engine
+                // streams several times faster.  Large inputs therefore go through the instance's device
+                // input buffer (image i), enqueued on the same stream right before the first kernel group.
                 if (direct_io && cur == lead && in_bytes_ >= kDmaInputBytes) {
-                    if (copy_started_) check(cudaStreamWaitEvent(st, copied_, 0));
-                    else check(cudaMemcpyAsync(input_dev() + (size_t)i * in_bytes_, io, in_bytes_, cudaMemcpyHostToDevice, st));
+                    check(cudaMemcpyAsync(static_cast<char*>(pb_instance_input_dev(inst_)) + (size_t)i * in_bytes_, io, in_bytes_,
+                                          cudaMemcpyHostToDevice, st));
                     ins[i] = nullptr;
                 }
+                outs[i] = direct_io ? io + get_output_offset() : nullptr;
             }
             if (pb_instance_launch_group_batched(inst_, cur - lead, gang_n_, st, get_id(), get_finished_block_notifier(), ins, outs) != PB_OK)
                 set_error(PB_ERR_CUDA);
@@ -127,22 +128,6 @@ class ModelJob : public llis::job::Job {
 
   private:
     static constexpr size_t kDmaInputBytes = 64 * 1024;
-    char* input_dev() { return static_cast<char*>(pb_instance_input_dev(inst_)); }
-    // Loads issued by SMs keep few PCIe reads in flight (about 11 GB/s measured); a copy engine streams several times
-    // faster, so large inputs go through the instance's device input buffer.  On a server that runs one request per launch
-    // the copy starts when the request is admitted and runs while the request waits for its turn on the GPU (enqueued with
-    // its first stage, a dispatched request held its share of the GPU while its input, and those of the requests dispatched
-    // before it, crossed PCIe: 32 ResNet-18 requests 838 us instead of 800).  A gang needs all its members' inputs, so theirs
-    // should follow one another: they are copied when the gang is dispatched (in the order of admission, 64 requests of
-    // MobileNet and ResNet-50 took 1784 us instead of 1730: the first gang of either waited for the inputs of both).
-    void start_input_copy() {
-        copy_started_ = false;
-        cudaStream_t st = llis::job::Context::get_input_stream();
-        if (!st || !inst_ || cap_ > 1 || copy_stages_ || resident_ || in_bytes_ < kDmaInputBytes) return;
-        check(cudaMemcpyAsync(input_dev(), io_ptr_, in_bytes_, cudaMemcpyHostToDevice, st));
-        check(cudaEventRecord(copied_, st));
-        copy_started_ = true;
-    }
     void check(cudaError_t e) { if (e != cudaSuccess) set_error(PB_ERR_CUDA); }
 
     // Declares stage `next_` (resources, copy or compute, pre-notify on the last one).
@@ -166,26 +151,22 @@ class ModelJob : public llis::job::Job {
     // Instances by the server that owns them: the job objects themselves are never destroyed (the plugin ABI has no
     // virtual destructor and the reference pools instances for ever, src/server/registered_job.cpp:91-93), but a
     // server that goes away gives the device memory of its instances back through pb_plugin_release().
-    struct Held {
-        pb_instance* inst;
-        cudaEvent_t copied;
-    };
-    static std::map<void*, std::vector<Held>>& registry() {
-        static std::map<void*, std::vector<Held>> r;
+    static std::map<void*, std::vector<pb_instance*>>& registry() {
+        static std::map<void*, std::vector<pb_instance*>> r;
         return r;
     }
     static std::mutex& registry_mu() {
         static std::mutex mu;
         return mu;
     }
-    static void remember(void* owner, const Held& held) {
+    static void remember(void* owner, pb_instance* inst) {
         std::lock_guard<std::mutex> lk(registry_mu());
-        registry()[owner].push_back(held);
+        registry()[owner].push_back(inst);
     }
 
   public:
     static void release_all(void* owner) {
-        std::vector<Held> mine;
+        std::vector<pb_instance*> mine;
         {
             std::lock_guard<std::mutex> lk(registry_mu());
             auto it = registry().find(owner);
@@ -193,10 +174,7 @@ class ModelJob : public llis::job::Job {
             mine.swap(it->second);
             registry().erase(it);
         }
-        for (const Held& h : mine) {
-            pb_instance_destroy(h.inst);
-            if (h.copied) cudaEventDestroy(h.copied);
-        }
+        for (pb_instance* i : mine) pb_instance_destroy(i);
     }
 
   private:
@@ -219,8 +197,6 @@ class ModelJob : public llis::job::Job {
     std::string name_;
     size_t in_bytes_, out_bytes_;
     pb_instance* inst_ = nullptr;
-    cudaEvent_t copied_ = nullptr;                 // recorded behind the request's input copy
-    bool copy_started_ = false;
     std::vector<llis::job::StageDecl> decls_;      // [group][gang size - 1]
     int num_groups_ = 0;
     int cap_ = 1;          // images the instance holds = largest gang this job can lead

@@ -544,8 +544,8 @@ def main():
     ap.add_argument("--replicas-per-gpu", type=int, default=1,
                     help="independent scheduler+pool replicas (one busy-polling host thread each) sharing every GPU")
     ap.add_argument("--extra-kernels", type=int, default=0,
-                    help="scheduler: over-subscribed stages allowed in flight (--extra_kernels); default 18 for the headline mix (under Poisson "
-                         "arrivals the gate makes requests queue into gangs when the GPU is busy: measured best of 6..64), 64 otherwise")
+                    help="scheduler: over-subscribed stages allowed in flight (--extra_kernels); default 14 for the headline mix (under Poisson "
+                         "arrivals the gate makes requests queue into gangs when the GPU is busy: measured best of 7..18), 64 otherwise")
     ap.add_argument("--sched", default="full3", choices=["full3", "fifo", "fifo2"],
                     help="full3 = the kernel-level scheduler; fifo (job by job) and fifo2 (stage by stage, arrival order) are the ablations")
     ap.add_argument("--streams", type=int, default=500, help="scheduler stream pool (--num_streams); 1 with --sched fifo = single-stream baseline")
@@ -577,7 +577,7 @@ def main():
         args.batch = {"mix": 12000, "mnist": 20000, "fig11": 8000, "fig12": 8000}.get(args.workload, 1500)
     paper = PAPER_MIXES.get(args.workload)
     if args.extra_kernels <= 0:
-        args.extra_kernels = 18 if args.workload == "mix" else 64
+        args.extra_kernels = 14 if args.workload == "mix" else 64
     if args.concurrency <= 0:
         args.concurrency = paper["concurrency"] if paper else 192
     global MIX, GANG, DEFERRED

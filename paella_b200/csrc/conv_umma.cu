@@ -18,7 +18,8 @@
 // Two entry points share the body (conv_tile_tma): conv_umma_tma_kernel runs one convolution,
 // conv_umma_multi_kernel runs several independent ones as one grid from a descriptor table in
 // device memory.  conv_umma_gather_kernel (PB_CONV_GATHER=1) is the earlier design, kept for
-// comparison: 128 producer threads gather A with 16-byte cp.async copies.
+// comparison: 128 producer threads gather A with 16-byte cp.async copies (a lone Inception-v3 request
+// takes 1656 us with it, 342 without).
 //
 // Every wait is bounded: when a wait runs out the CTA raises a device-global error flag,
 // sets a shared abort flag that releases all other waits of the CTA, skips the epilogue,
@@ -1526,10 +1527,10 @@ int bn_limit() {
 }
 
 // PB_CONV_PERSIST=1: model launches run the persistent kernel (a CTA walks several tiles).  Off by default.
-// Measured on B200: a lone Inception-v3 request 723 -> 604 us (3 tiles per CTA: 868 us), Inception-v3 alone with 96
-// requests in flight 26.5k -> 27.4k req/s, but the headline mix (MNIST : Inception-v3 = 9 : 1, 96 clients, gangs of 4)
-// 242k -> 221k req/s: its 108 KB CTAs leave an SM no room for anything else, and fewer, longer CTAs per launch lengthen
-// every request's chain of launches, which is what the mix runs out of first.
+// Measured on B200 with 3 tiles per CTA: a lone Inception-v3 request 342 -> 1119 us, the mix MNIST : Inception-v3 = 9 : 1 in a closed
+// loop of 192 clients 317 -> 166 thousand requests a second.  It has not followed the one-tile kernel: no split reductions, no
+// stores through TMA, multiplications and copies issued under `lane == 0` (390 clocks a k-block), and the tiles it walks are cut
+// for one tile per CTA.  (Against the one-tile kernel of its time it had a lone request at 604 us instead of 723.)
 bool persist_enabled() {
     const char* e = getenv("PB_CONV_PERSIST");      // read at every use: a model keeps what it was loaded with
     return e && e[0] == '1' && use_tma_a();
@@ -1605,7 +1606,9 @@ int pipeline_stages(int ctas, int BN, int k_blocks, bool shared) {
 //   shared by the blocks of the SM (between the mean and the fullest one);
 //   the epilogue costs 11 ns per column of a block with direct stores (24 with a residual), 8 through TMA;
 //   a cluster costs its two barriers and the parked tile, and 2 / 6 / 13 ns of placement per block at 2 / 4 / 8 ranks.
-// Its mean error is 3 %, and what it picks is within 1.5 % of the best measured tiles summed over the layers of a network.
+// Its mean error there is 3 %, and what it picks is within 1.5 % of the best measured tiles summed over the layers of a network.
+// A layer repeated 40 times in one graph, all launches alike, takes 1.8 us less than modelled (0.3 us spread over 19 layers of 7x7 to
+// 56x56 maps, 1 and 8 images); the tiles picked for those 19 take 91.6 us in all, the best of 6 to 33 measured for each 90.4.
 // (Before, the model knew neither the stores' path nor the residual, and a width of 80 or 176 columns, which TMA cannot
 // store, cost a 14 x 14 layer of 256 -> 1024 channels 8.8 us instead of 6.4 alone and 3.1 instead of 1.7 under load.)
 int tiling_ctas(const ConvShape& c, const ConvTiling& t) { return c.m_tiles * ceil_div(c.Kp16, t.BN) * t.splits; }

@@ -363,9 +363,9 @@ void build_groups(pb_model* m) {
         for (const std::vector<int>& l : g.launches)
             for (int s : l) m->stages[(size_t)s].peers = l;
     // PB_FUSE_POOLS=1: off by default; not with the persistent kernel.  Measured: same bits, a lone Inception-v3 request
-    // 885 -> 870 us, but 26.9k -> 17.4k req/s with 96 requests in flight: a pooling block then holds a whole convolution
-    // slot of its SM (the launch's 73 KB of shared memory) while it waits on loads, and there are 600-900 of them per
-    // launch at 8 images.
+    // 342 -> 330 us, but 317 -> 313 thousand requests a second of MNIST : Inception-v3 = 9 : 1 in a closed loop of 192 clients: a
+    // pooling block then holds a whole convolution slot of its SM (the launch's 73 KB of shared memory) while it waits on
+    // loads, and there are 600-900 of them per launch at 8 images.
     m->groups = plan_groups(m, gs, m->fuse_branches, m->fuse_branches && !m->persist && env_flag("PB_FUSE_POOLS", false));
     refresh_infos(m);
 }

@@ -164,12 +164,23 @@ __global__ void __launch_bounds__(256) input_patch_kernel(OpArgs a, uint32_t job
 // scattered 4-byte loads per output vector (each value about 2.25 times, with the index arithmetic of its filter tap
 // every time) and holds a block slot for 256 output vectors; under serving load that costs more than its share of a
 // lone request (6.7 % of the Inception-v3 throughput, measured by leaving it out).  Here a block first copies the
-// window of its kPatchTileP x kPatchTileQ output pixels into shared memory with coalesced loads that are all in flight
-// together (fp32, zero outside the image), then writes its output vectors from there; the offset of every k in the
-// window is looked up in a table (up to 256 values of k) built once per block.  Same values, same rounding: identical bits.
+// window of its kPatchTileP x kPatchTileQ output pixels into shared memory, as T (zero outside the image): a warp takes rows
+// of the window and has twelve coalesced loads in flight.  Then it writes its output vectors from there.  A thread keeps
+// ONE vector position k0 for all its pixels, so the eight offsets of its values in the window are registers; consecutive
+// threads write consecutive vectors.  Bound by those 2-byte reads of shared memory (a value is read R*S / stride^2 times).
+// (Offsets looked up in a table in shared memory for every value, and fp32 values there: the table's reads alone were 8-way
+// bank conflicts; 8 images of 224 x 224, 7 x 7 stride 2: 25 us.)  Same values, same rounding: identical bits.
 constexpr int kPatchTileP = 8, kPatchTileQ = 32;
 __host__ __device__ __forceinline__ int patch_tile_rows(int R, int sh) { return (kPatchTileP - 1) * sh + R; }
 __host__ __device__ __forceinline__ int patch_tile_cols(int S, int sw) { return (kPatchTileQ - 1) * sw + S; }
+
+__device__ __forceinline__ void patch_store(float* y, const float (&v)[4]) { *reinterpret_cast<float4*>(y) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void patch_store(__nv_bfloat16* y, const __nv_bfloat16 (&v)[8]) {
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = (uint32_t)__bfloat16_as_ushort(v[2 * i]) | (uint32_t)__bfloat16_as_ushort(v[2 * i + 1]) << 16;
+    *reinterpret_cast<uint4*>(y) = make_uint4(u[0], u[1], u[2], u[3]);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) input_patch_tile_kernel(OpArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
@@ -179,44 +190,65 @@ __global__ void __launch_bounds__(256) input_patch_tile_kernel(OpArgs a, uint32_
                                                   : static_cast<const float*>(a.x) + (size_t)blockIdx.y * a.C * a.H * a.W;
     constexpr int N = Vec<T>::N;
     const int rows = patch_tile_rows(a.R, a.stride_h), cols = patch_tile_cols(a.S, a.stride_w);
-    int* s_off = reinterpret_cast<int*>(s_patch);                 // [Ks] offset of k in the window, -1 = zero
-    float* s_win = reinterpret_cast<float*>(s_patch + 1024);      // [C][rows][cols]
+    T* s_win = reinterpret_cast<T*>(s_patch);                     // [C][rows][cols]
     const int tiles_q = (a.Q + kPatchTileQ - 1) / kPatchTileQ;
     const int p0 = (blockIdx.x / tiles_q) * kPatchTileP, q0 = (blockIdx.x % tiles_q) * kPatchTileQ;
     const int ih0 = p0 * a.stride_h - a.pad_h, iw0 = q0 * a.stride_w - a.pad_w;
-    if (threadIdx.x < a.Ks) {
-        const int k = threadIdx.x, taps_c = a.R * a.S * a.C;
-        int off = -1;
-        if (k < taps_c) {
-            const int tap = k / a.C, c = k - tap * a.C;
-            const int r = tap / a.S, s2 = tap - r * a.S;
-            off = (c * rows + r) * cols + s2;
+
+    const int lane = threadIdx.x & 31, n_rows = a.C * rows;
+    for (int row0 = threadIdx.x >> 5; row0 < n_rows; row0 += 32) {
+        for (int col0 = lane; col0 < cols; col0 += 96) {
+            float v[4][3];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int row = row0 + 8 * u, c = row / rows, ih = ih0 + row - c * rows;
+                const bool row_ok = row < n_rows && (unsigned)ih < (unsigned)a.H;
+                const float* __restrict__ g = x + ((ptrdiff_t)c * a.H + ih) * a.W + iw0;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    const int col = col0 + 32 * t;
+                    v[u][t] = row_ok && col < cols && (unsigned)(iw0 + col) < (unsigned)a.W ? __ldg(g + col) : 0.f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int t = 0; t < 3; ++t)
+                    if (row0 + 8 * u < n_rows && col0 + 32 * t < cols) s_win[(row0 + 8 * u) * cols + col0 + 32 * t] = from_f<T>(v[u][t]);
         }
-        s_off[k] = off;
     }
-    const int n_win = a.C * rows * cols;
-    for (int i = threadIdx.x; i < n_win; i += 256) {
-        const int col = i % cols, rest = i / cols;
-        const int r = rest % rows, c = rest / rows;
-        const int ih = ih0 + r, iw = iw0 + col;
-        s_win[i] = (ih >= 0 && ih < a.H && iw >= 0 && iw < a.W) ? __ldg(x + ((size_t)c * a.H + ih) * a.W + iw) : 0.f;
-    }
-    __syncthreads();
-    const int kv = a.Ks / N;
-    T* __restrict__ y = y_img<T>(a);
-    for (int v = threadIdx.x; v < kPatchTileP * kPatchTileQ * kv; v += 256) {
-        const int k0 = (v % kv) * N, pl = v / kv;
-        const int pr = pl / kPatchTileQ, pc = pl - pr * kPatchTileQ;
-        const int p = p0 + pr, q = q0 + pc;
-        if (p >= a.P || q >= a.Q) continue;
-        const int base = pr * a.stride_h * cols + pc * a.stride_w;
-        Vec<T> o;
+    // this thread's vector of k, where its values lie in a pixel's window, and its first pixel
+    const int kv = a.Ks / N, groups = 256 / kv;
+    const int grp = threadIdx.x / kv, k0 = (threadIdx.x - grp * kv) * N;
+    int off[N];
+    uint32_t real = 0;                       // values of the filter window; the others are zeros
+    {
+        int c = k0 % a.C, s2 = k0 / a.C % a.S, r = k0 / (a.C * a.S);
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-            const int off = s_off[k0 + j];
-            o.v[j] = off >= 0 ? s_win[base + off] : 0.f;
+            real |= (r < a.R ? 1u : 0u) << j;
+            off[j] = r < a.R ? (c * rows + r) * cols + s2 : 0;
+            if (++c == a.C) {
+                c = 0;
+                if (++s2 == a.S) { s2 = 0; ++r; }
+            }
         }
-        o.store(y + ((size_t)p * a.Q + q) * a.Ks + k0);
+    }
+    __syncthreads();
+    if constexpr (sizeof(T) == 2) pb::griddep_launch();      // the window has arrived: what is left is short
+    if (grp < groups) {
+        T* __restrict__ y = y_img<T>(a) + k0;
+#pragma unroll 2
+        for (int px = grp; px < kPatchTileP * kPatchTileQ; px += groups) {
+            const int pr = px / kPatchTileQ, pc = px % kPatchTileQ;
+            const int p = p0 + pr, q = q0 + pc;
+            if (p >= a.P || q >= a.Q) continue;
+            const T* __restrict__ w = s_win + pr * a.stride_h * cols + pc * a.stride_w;
+            T o[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) o[j] = (real >> j) & 1u ? w[off[j]] : from_f<T>(0.f);
+            patch_store(y + ((size_t)p * a.Q + q) * a.Ks, o);
+        }
     }
     PB_NOTIFY_END();
 }
@@ -224,7 +256,7 @@ __global__ void __launch_bounds__(256) input_patch_tile_kernel(OpArgs a, uint32_
 // not fit, more than 256 values of k).
 static size_t patch_tile_smem(const pb_op_params* p) {
     if (p->Ks > 256 || p->R * p->S <= 1) return 0;
-    const size_t n = 1024 + (size_t)p->C * patch_tile_rows(p->R, p->stride_h) * patch_tile_cols(p->S, p->stride_w) * 4;
+    const size_t n = (size_t)p->C * patch_tile_rows(p->R, p->stride_h) * patch_tile_cols(p->S, p->stride_w) * (p->dtype == 0 ? 4 : 2);
     return n <= 40 * 1024 ? n : 0;
 }
 static uint32_t patch_tile_blocks(const pb_op_params* p) {

@@ -327,55 +327,73 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t x, uint64_t y) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return r;
 }
-template <int ACT>
-__device__ __forceinline__ uint32_t to_bf16x2_act(uint64_t v, float slope_lo = 0.f, float slope_hi = 0.f) {
-    uint32_t lo, hi, d;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
-    if constexpr (ACT == 3) {       // PReLU: v > 0 ? v : slope * v, per channel
-        const float a = __uint_as_float(lo), b = __uint_as_float(hi);
-        lo = __float_as_uint(a > 0.f ? a : a * slope_lo);
-        hi = __float_as_uint(b > 0.f ? b : b * slope_hi);
-    }
-    if constexpr (ACT == 0 || ACT == 3) {
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
-    } else {
-        asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
-        if constexpr (ACT == 2) asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(d), "r"(0x40C040C0u));
-    }
-    return d;
+// The activation is chosen at run time, by branches all threads take alike: as a template parameter of the epilogues it made four
+// copies of each (and of each cluster size), 124 KB of code per kernel, and a launch whose copy had not run on its SM lately
+// spent 0.5 to 1.6 us of its epilogue fetching it.  The loops below are kept rolled for the same reason.
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+    uint32_t l, h;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(l), "=r"(h) : "l"(v));
+    lo = __uint_as_float(l);
+    hi = __uint_as_float(h);
 }
 
-// One group of 16 accumulator columns of this thread's row: + bias (+ residual), activation, bf16, 16-byte
-// stores.  The four epilogue warps run one per scheduler with nothing to hide instruction latency behind, so the
-// column loop is kept to one packed add and one convert per two columns.
-template <int ACT>
-__device__ __forceinline__ uint4 finish8(const ConvArgs& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias8) {
-    const uint4 b0 = *reinterpret_cast<const uint4*>(bias8), b1 = *reinterpret_cast<const uint4*>(bias8 + 4);
-    const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-    const uint32_t ru[4] = {res.x, res.y, res.z, res.w};
-    uint32_t o[4];
+// Eight accumulator columns of this thread's row, from channel k on: + bias (+ residual), activation, bf16.  The four epilogue
+// warps run one per scheduler with nothing to hide instruction latency behind, so this is kept to one packed add and one
+// convert per two columns.
+__device__ __forceinline__ uint4 finish8(const ConvArgs& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias) {
+    uint64_t f[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint64_t f = add_f32x2(pack_f32x2(v[2 * j], v[2 * j + 1]), pack_f32x2(bw[2 * j], bw[2 * j + 1]));
-        if (has_res) f = add_f32x2(f, pack_f32x2(ru[j] << 16, ru[j] & 0xffff0000u));
-        if constexpr (ACT == 3) {
-            float2 sl = make_float2(0.f, 0.f);
-            if (k < a.K) sl = __ldg(reinterpret_cast<const float2*>(a.bias + a.K + k) + j);   // slopes follow the biases
-            o[j] = to_bf16x2_act<ACT>(f, sl.x, sl.y);
-        } else {
-            o[j] = to_bf16x2_act<ACT>(f);
+    for (int h = 0; h < 2; ++h) {
+        const uint4 b = *reinterpret_cast<const uint4*>(bias + 4 * h);
+        f[2 * h] = add_f32x2(pack_f32x2(v[4 * h], v[4 * h + 1]), pack_f32x2(b.x, b.y));
+        f[2 * h + 1] = add_f32x2(pack_f32x2(v[4 * h + 2], v[4 * h + 3]), pack_f32x2(b.z, b.w));
+    }
+    if (has_res) {
+        const uint32_t ru[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = add_f32x2(f[j], pack_f32x2(ru[j] << 16, ru[j] & 0xffff0000u));
+    }
+    uint32_t o[4];
+    if (a.act == 1 || a.act == 2) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float lo, hi;
+            unpack_f32x2(f[j], lo, hi);
+            asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(o[j]) : "f"(hi), "f"(lo));
+        }
+        if (a.act == 2) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) asm("min.bf16x2 %0, %1, %2;" : "=r"(o[j]) : "r"(o[j]), "r"(0x40C040C0u));
+        }
+    } else {
+        if (a.act == 3) {           // PReLU: v > 0 ? v : slope * v, per channel; the slopes follow the biases
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float lo, hi;
+                unpack_f32x2(f[j], lo, hi);
+                float2 sl = make_float2(0.f, 0.f);
+                if (k + 2 * j < a.K) sl = __ldg(reinterpret_cast<const float2*>(a.bias + a.K + k) + j);
+                lo = lo > 0.f ? lo : lo * sl.x;
+                hi = hi > 0.f ? hi : hi * sl.y;
+                f[j] = pack_f32x2(__float_as_uint(lo), __float_as_uint(hi));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float lo, hi;
+            unpack_f32x2(f[j], lo, hi);
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[j]) : "f"(hi), "f"(lo));
         }
     }
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
-template <int ACT>
 __device__ __forceinline__ void epilogue_chunk(const ConvArgs& a, const uint32_t (&v)[16], const uint4 (&rv)[2], int cb, int n0, bool row_valid,
                                                __nv_bfloat16* yrow, bool has_res, const float* s_bias) {
     if (!row_valid) return;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int k = n0 + cb + h * 8;
-        if (k + 8 <= a.K) *reinterpret_cast<uint4*>(yrow + k) = finish8<ACT>(a, v + h * 8, rv[h], has_res, k, s_bias + cb + h * 8);
+        if (k + 8 <= a.K) *reinterpret_cast<uint4*>(yrow + k) = finish8(a, v + h * 8, rv[h], has_res, k, s_bias + cb + h * 8);
     }
 }
 
@@ -390,7 +408,6 @@ __device__ __forceinline__ void load_residual(const ConvArgs& a, int k0, bool ro
 
 // Columns in steps of 16, two steps in flight: the next step leaves tensor memory (and its residual is on its way)
 // while this one is converted and stored.
-template <int ACT>
 __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lane_addr, int n0, bool row_valid, __nv_bfloat16* yrow,
                                                  const __nv_bfloat16* rrow, const float* s_bias) {
     uint32_t v0[16], v1[16];
@@ -398,6 +415,7 @@ __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lan
     const bool has_res = rrow != nullptr;
     tcgen05_ld16(lane_addr, v0);             // warp-collective: all lanes take part
     load_residual(a, n0, row_valid, rrow, r0);
+#pragma unroll 1
     for (int cb = 0; cb < a.BN; cb += 32) {
         tcgen05_wait_ld();
         const bool second = cb + 16 < a.BN;
@@ -405,14 +423,14 @@ __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lan
             tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
             load_residual(a, n0 + cb + 16, row_valid, rrow, r1);
         }
-        epilogue_chunk<ACT>(a, v0, r0, cb, n0, row_valid, yrow, has_res, s_bias);
+        epilogue_chunk(a, v0, r0, cb, n0, row_valid, yrow, has_res, s_bias);
         if (!second) break;
         tcgen05_wait_ld();
         if (cb + 32 < a.BN) {
             tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
             load_residual(a, n0 + cb + 32, row_valid, rrow, r0);
         }
-        epilogue_chunk<ACT>(a, v1, r1, cb + 16, n0, row_valid, yrow, has_res, s_bias);
+        epilogue_chunk(a, v1, r1, cb + 16, n0, row_valid, yrow, has_res, s_bias);
     }
 }
 
@@ -424,7 +442,6 @@ __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lan
 // result, and one lane of a warp stores the warp's 32 rows of a finished box with one instruction.  `buf`: 128 x BN x 2 bytes
 // of the pipeline memory, free by now.  publish: this launch reports to the host, so the stores have to be in memory when the
 // warp leaves; otherwise they only have to have been read (the next kernel waits for this one's memory operations).
-template <int ACT>
 __device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t lane_addr, int n0, bool has_res, const float* s_bias, uint32_t buf,
                                                      const CUtensorMap* tmap_y, int m0, bool publish) {
     const uint32_t r = threadIdx.x;                 // tile row
@@ -439,8 +456,8 @@ __device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t
         const uint32_t at0 = row + box + (((uint32_t)(in_box >> 3) ^ swz) << 4), at1 = row + box + ((((uint32_t)(in_box >> 3) + 1u) ^ swz) << 4);
         uint4 res0 = make_uint4(0, 0, 0, 0), res1 = res0;
         if (has_res) { res0 = ld_shared_v4(at0); res1 = ld_shared_v4(at1); }
-        const uint4 o0 = finish8<ACT>(a, v, res0, has_res, n0 + cb, s_bias + cb);
-        const uint4 o1 = finish8<ACT>(a, v + 8, res1, has_res, n0 + cb + 8, s_bias + cb + 8);
+        const uint4 o0 = finish8(a, v, res0, has_res, n0 + cb, s_bias + cb);
+        const uint4 o1 = finish8(a, v + 8, res1, has_res, n0 + cb + 8, s_bias + cb + 8);
         st_shared_v4(at0, o0.x, o0.y, o0.z, o0.w);
         st_shared_v4(at1, o1.x, o1.y, o1.z, o1.w);
         if (in_box + 16 == U) {
@@ -452,6 +469,7 @@ __device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t
         }
     };
     tcgen05_ld16(lane_addr, v0);             // warp-collective: all lanes take part
+#pragma unroll 1
     for (int cb = 0; cb < a.BN; cb += 32) {
         tcgen05_wait_ld();
         tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
@@ -486,18 +504,12 @@ __device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, 
     if (tmap_y) {
         const bool has_res = a.residual != nullptr;
         if (has_res && !__all_sync(0xffffffffu, mbar_wait(smem_u32(s_res), 0u, s_abort_p, a.err_flag, 6u))) return;
-        if (a.act == 3) epilogue_columns_tma<3>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
-        else if (a.act == 1) epilogue_columns_tma<1>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
-        else if (a.act == 2) epilogue_columns_tma<2>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
-        else epilogue_columns_tma<0>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        epilogue_columns_tma(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
         return;
     }
     const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
     __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
-    if (a.act == 3) epilogue_columns<3>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
-    else if (a.act == 1) epilogue_columns<1>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
-    else if (a.act == 2) epilogue_columns<2>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
-    else epilogue_columns<0>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    epilogue_columns(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
 }
 
 // ---- split reduction: the thread blocks of a cluster share one output tile -----------------------------------
@@ -511,65 +523,65 @@ __device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, 
 // (The partial tiles used to meet in a global workspace under an atomic counter: two fences, an atomic and an L2
 // round trip of BN x 512 bytes per rank, read back by ONE block: +4 to +8 us per launch, so only reductions of 60
 // and more k-blocks gained from it.)
-template <int ACT, int S>
 __device__ __forceinline__ void cluster_finish(const ConvArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
                                                const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
-    constexpr int kOct = S == 2 ? 2 : 1;      // groups of 8 columns per turn
-    constexpr int kRanks = S < 4 ? S : 4;     // ranks whose loads are in flight together (16-byte loads: up to 8 a thread; more spill)
-    uint32_t active = 0;           // ranks that have k-blocks (all of them unless a grouped launch splits a short reduction)
+    const int S = a.splits;
+    uint32_t active = (1u << S) - 1u;      // ranks that have k-blocks (all of them unless a grouped launch splits a short reduction)
+    if (a.nkb < S) {
+        active = 0;
+#pragma unroll 1
+        for (int z = 0; z < S; ++z) active |= (a.nkb * (z + 1) / S > a.nkb * z / S ? 1u : 0u) << z;
+    }
+    // Four partial sums of 8 columns in flight per turn (16-byte loads: 8 a thread; more spill): four ranks', or with two ranks
+    // those of 16 columns.
+    const int step = S == 2 ? 16 : 8;
+#pragma unroll 1
+    for (int c = 0; c < w; c += step) {
+        uint64_t sum[2][4];
 #pragma unroll
-    for (int z = 0; z < S; ++z) active |= (a.nkb * (z + 1) / S > a.nkb * z / S ? 1u : 0u) << z;
-    for (int c = 0; c < w; c += 8 * kOct) {
-        uint64_t sum[kOct][4];
-#pragma unroll
-        for (int o = 0; o < kOct; ++o)
+        for (int o = 0; o < 2; ++o)
 #pragma unroll
             for (int j = 0; j < 4; ++j) sum[o][j] = 0;        // (+0 is exact; a sum of zeros may lose a -0, which the bias add would too)
+#pragma unroll 1
+        for (int z0 = 0; z0 < S; z0 += 4) {
+            uint4 part[4][2];
 #pragma unroll
-        for (int z0 = 0; z0 < S; z0 += kRanks) {
-            uint4 part[kOct][kRanks][2];
-#pragma unroll
-            for (int o = 0; o < kOct; ++o) {
-                const uint32_t src = buf + ((uint32_t)((rank * w + c + 8 * o) >> 2) * 128u + threadIdx.x) * 16u;
-#pragma unroll
-                for (int z = 0; z < kRanks; ++z) {
-                    part[o][z][0] = part[o][z][1] = make_uint4(0, 0, 0, 0);
-                    if (c + 8 * o >= w || !((active >> (z0 + z)) & 1u)) continue;
-                    const uint32_t at = cluster_addr(src, (uint32_t)(z0 + z));       // this rank's own part too
-                    part[o][z][0] = ld_cluster_v4(at);
-                    part[o][z][1] = ld_cluster_v4(at + 2048u);
-                }
+            for (int i = 0; i < 4; ++i) {
+                const int z = S == 2 ? i & 1 : z0 + i, col = S == 2 ? c + (i >> 1) * 8 : c;
+                part[i][0] = part[i][1] = make_uint4(0, 0, 0, 0);
+                if (col >= w || !((active >> z) & 1u)) continue;
+                const uint32_t at = cluster_addr(buf + ((uint32_t)((rank * w + col) >> 2) * 128u + threadIdx.x) * 16u, (uint32_t)z);       // this rank's own part too
+                part[i][0] = ld_cluster_v4(at);
+                part[i][1] = ld_cluster_v4(at + 2048u);
             }
-#pragma unroll
-            for (int o = 0; o < kOct; ++o)
-#pragma unroll
-                for (int z = 0; z < kRanks; ++z) {
-                    const uint4 lo = part[o][z][0], hi = part[o][z][1];
-                    sum[o][0] = add_f32x2(sum[o][0], pack_f32x2(lo.x, lo.y));
-                    sum[o][1] = add_f32x2(sum[o][1], pack_f32x2(lo.z, lo.w));
-                    sum[o][2] = add_f32x2(sum[o][2], pack_f32x2(hi.x, hi.y));
-                    sum[o][3] = add_f32x2(sum[o][3], pack_f32x2(hi.z, hi.w));
-                }
+            auto add = [&](uint64_t (&s)[4], const uint4 (&q)[2]) {
+                s[0] = add_f32x2(s[0], pack_f32x2(q[0].x, q[0].y));
+                s[1] = add_f32x2(s[1], pack_f32x2(q[0].z, q[0].w));
+                s[2] = add_f32x2(s[2], pack_f32x2(q[1].x, q[1].y));
+                s[3] = add_f32x2(s[3], pack_f32x2(q[1].z, q[1].w));
+            };
+            add(sum[0], part[0]);
+            add(sum[0], part[1]);
+            if (S == 2) {
+                add(sum[1], part[2]);
+                add(sum[1], part[3]);
+            } else {
+                add(sum[0], part[2]);
+                add(sum[0], part[3]);
+            }
         }
 #pragma unroll
-        for (int o = 0; o < kOct; ++o) {
-            const int col = rank * w + c + 8 * o, k = n0 + col;
-            if (c + 8 * o >= w || !row_valid || k >= a.K) continue;
+        for (int o = 0; o < 2; ++o) {
+            const int at = c + 8 * o, col = rank * w + at, k = n0 + col;
+            if ((o && S != 2) || at >= w || !row_valid || k >= a.K) continue;
             uint4 res = make_uint4(0, 0, 0, 0);
             if (rrow) res = *reinterpret_cast<const uint4*>(rrow + k);
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(sum[o][j]));
-            *reinterpret_cast<uint4*>(yrow + k) = finish8<ACT>(a, v, res, rrow != nullptr, k, s_bias + col);
+            *reinterpret_cast<uint4*>(yrow + k) = finish8(a, v, res, rrow != nullptr, k, s_bias + col);
         }
     }
-}
-template <int ACT>
-__device__ __forceinline__ void cluster_finish(const ConvArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
-                                               const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
-    if (a.splits == 2) cluster_finish<ACT, 2>(a, n0, row_valid, yrow, rrow, s_bias, rank, buf, w);
-    else if (a.splits == 4) cluster_finish<ACT, 4>(a, n0, row_valid, yrow, rrow, s_bias, rank, buf, w);
-    else cluster_finish<ACT, 8>(a, n0, row_valid, yrow, rrow, s_bias, rank, buf, w);
 }
 
 // Run by warps 0-3 of every rank.  `mine`: this rank has k-blocks of its own.
@@ -589,6 +601,7 @@ __device__ __forceinline__ void epilogue_cluster(const ConvArgs& a, uint32_t tme
         uint32_t v0[16], v1[16];
         uint32_t at = smem_base + (uint32_t)tid * 16u;
         tcgen05_ld16(lane_addr, v0);
+#pragma unroll 1
         for (int cb = 0; cb < a.BN; cb += 32) {
             tcgen05_wait_ld();
             if (cb + 16 < a.BN) tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
@@ -608,10 +621,7 @@ __device__ __forceinline__ void epilogue_cluster(const ConvArgs& a, uint32_t tme
     if (ok) {
         __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
         const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
-        if (a.act == 3) cluster_finish<3>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
-        else if (a.act == 1) cluster_finish<1>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
-        else if (a.act == 2) cluster_finish<2>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
-        else cluster_finish<0>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        cluster_finish(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
     }
     cluster_arrive_relaxed();
     cluster_wait();                 // every rank has read what it needs: shared memory may go
@@ -953,25 +963,22 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
     } else {
         // ===== MMA issuer =====
-        // An mbarrier wait costs ~170 clocks even when its phase is long complete, so the NEXT k-block's barrier is
-        // probed (test_wait, never blocks) before this k-block's MMAs are issued: the probe's latency runs under them;
-        // and the descriptors are stage 0's plus a stride.
+        // A wait on a complete barrier costs about 130 clocks and the tensor pipe holds few instructions, so it drains meanwhile:
+        // four multiplications of 32 columns take 160 clocks, a k-block 325.  Probing the next barrier before the multiplications
+        // are issued only puts the probe's latency in front of them (360).  The descriptors are stage 0's plus a stride.
         uint32_t st = 0, parity = 0u;
-        bool ok = true, have_next = false;
+        bool ok = true;
         uint32_t* const err_flag = a.err_flag;
         const uint32_t idesc = uniform(a.idesc), n_kb = uniform((uint32_t)nkb), n_st = uniform((uint32_t)stages);
         const uint64_t desc_a0 = umma_desc_sw128(uniform(smem_base)), desc_b0 = umma_desc_sw128(uniform(smem_base) + kATileBytes);
         const uint32_t desc_step = uniform(stage_bytes) >> 4;      // address field counts 16-byte units; no carry out of its 14 bits
         for (uint32_t kb = 0; kb < n_kb; ++kb) {
-            if (!__all_sync(0xffffffffu, have_next)) {
-                ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, s_abort, err_flag, 2u));
-                if (!ok) break;
-            }
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, s_abort, err_flag, 2u));
+            if (!ok) break;
             if (lane == 0) { if (kb == 0) { PB_T(3); PB_S(3); } PB_TK(kb, 1); }
             tcgen05_fence_after();
             uint32_t st_n = st + 1, parity_n = parity;
             if (st_n == n_st) { st_n = 0; parity_n ^= 1u; }
-            have_next = kb + 1 < n_kb && mbar_test_wait(smem_u32(&s_full[st_n]), parity_n);
             const uint64_t da = desc_a0 + st * desc_step, db = desc_b0 + st * desc_step;
             if (elect_one()) {
 #pragma unroll

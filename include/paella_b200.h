@@ -249,7 +249,8 @@ PB_API int pb_model_group_stages(const pb_model* m, int group, int* first_stage,
 /* The group's launch plan: its stages in launch order (dependence depth first, then program order) and,
  * for each, the index of the launch it belongs to.  Stages that share a launch index are independent
  * tensor-core convolutions issued as ONE grid (the parallel branches of an Inception block, a ResNet
- * shortcut beside the block's first convolution); the group's last launch is the one that notifies, so
+ * shortcut beside the block's first convolution), or an affine layer followed by the pointwise convolution that
+ * applies it to its input tiles itself (never in the group's last launch); the group's last launch is the one that notifies, so
  * pb_model_group_info's block count is the sum of its stages' grids.  Returns the number of stages
  * written (<= max_stages).  PB_FUSE_BRANCHES=0 at load time: program order, one stage per launch.
  * No counterpart in the reference (it launches one TVM kernel at a time). */

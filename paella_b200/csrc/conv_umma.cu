@@ -101,6 +101,11 @@ struct ConvArgs {
     uint32_t b_stage_bytes;
     int out_box;          // channels of one TMA store box: 64 or 32 (divides BN); 0 = the epilogue stores directly
     int splits;           // thread blocks (one cluster) that share a tile's reduction: rank z takes k-blocks [nkb*z/splits, nkb*(z+1)/splits)
+    // A pointwise layer may take act(x * pre_scale + pre_bias), per input channel, instead of x (pre_scale NULL: x itself).
+    const float* pre_scale;
+    const float* pre_bias;
+    int pre_act;
+    uint32_t pre_offset;  // where their part of shared memory begins
 };
 
 // ---- PTX wrappers -----------------------------------------------------------------
@@ -799,21 +804,96 @@ conv_umma_gather_kernel(const __grid_constant__ CUtensorMap tmap_w, const ConvAr
     if (nf) nf->end(job_id);
 }
 
+constexpr int kThreadsTma = 192;
+constexpr int kWarpB = 3;          // issues operand B's copies
+
+// ---- a batch-norm in front of a pointwise convolution -----------------------------------------------------------
+// DenseNet normalises the concatenated features before each 1x1 convolution, each time with other constants, so no earlier
+// epilogue can do it.  As a launch of its own that is 2.5 us and a hand-over of 0.75 us for a few hundred KB.  Here the tile of
+// raw features is normalised where it landed: the epilogue's warps, idle until the accumulator is complete, rewrite each stage of
+// operand A in shared memory and then let the MMA warp have it (operand A's warp loads operand B too).  Two warps take a stage, so
+// that one pair's wait and fence lie beside the other's arithmetic; a thread has one vector of 8 channels of sixteen rows, eight in
+// flight.
+// The arithmetic is affine_kernel's - fp32 multiply-add, ReLU, one rounding to bf16 - and so are the bits (the maximum with
+// zero may follow the rounding: rounding is monotonic and keeps zeros; NaN gives zero either way).
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
+// consts: [k-block][64 scales, 64 biases] of this rank's k-blocks, in shared memory.
+__device__ __forceinline__ void normalise_constants(const ConvArgs& a, float* consts, int kb_begin, int nkb) {
+    for (int i = threadIdx.x; i < nkb * 32; i += 128) {
+        const int c = (i & 15) * 4, from = (kb_begin + (i >> 5)) * kBK + c;
+        const float* src = (i & 16 ? a.pre_bias : a.pre_scale) + from;
+        *reinterpret_cast<float4*>(consts + i * 4) = from < a.Cs ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+}
+__device__ __forceinline__ void normalise_stages(const ConvArgs& a, uint32_t smem_base, uint32_t stage_bytes, int stages, int nkb, const float* consts,
+                                                 uint64_t* s_full, uint64_t* s_ready, volatile uint32_t* s_abort) {
+    const uint32_t vec = threadIdx.x & 7u, row = threadIdx.x >> 3 & 7u;      // rows row + 8 i: the swizzle is the same for all
+    const uint32_t pair = uniform(threadIdx.x >> 6);
+    const uint32_t at = smem_base + row * 128u + ((vec ^ (row & 7u)) << 4);
+    uint32_t st = pair, parity = 0;              // (a pipeline has two stages at least)
+    const bool relu = a.pre_act == 1;
+#pragma unroll 1
+    for (int kb = (int)pair; kb < nkb; kb += 2) {
+        uint64_t sc[4], bi[4];
+        const ulonglong2* k = reinterpret_cast<const ulonglong2*>(consts + kb * 128 + vec * 8);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const ulonglong2 s = k[h], b = k[h + 16];
+            sc[2 * h] = s.x; sc[2 * h + 1] = s.y;
+            bi[2 * h] = b.x; bi[2 * h + 1] = b.y;
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, s_abort, a.err_flag, 7u))) return;
+#pragma unroll 1
+        for (uint32_t half = 0; half < 2; ++half) {
+            const uint32_t tile = at + st * stage_bytes + half * 8192u;
+            uint4 v[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) v[i] = ld_shared_v4(tile + i * 1024u);
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+                uint32_t o[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float lo, hi;
+                    unpack_f32x2(fma_f32x2(pack_f32x2(u[j] << 16, u[j] & 0xffff0000u), sc[j], bi[j]), lo, hi);
+                    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[j]) : "f"(hi), "f"(lo));
+                }
+                if (relu) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) asm("max.bf16x2 %0, %1, %2;" : "=r"(o[j]) : "r"(o[j]), "r"(0u));
+                }
+                st_shared_v4(tile + i * 1024u, o[0], o[1], o[2], o[3]);
+            }
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (elect_one()) mbar_arrive(smem_u32(&s_ready[st]));
+        __syncwarp();
+        if ((st += 2u) >= (uint32_t)stages) { st -= (uint32_t)stages; parity ^= 1u; }
+    }
+}
+
 // ---- the kernel, operand A by im2col TMA ---------------------------------------------------------
 // CTA = 6 warps, each with a short loop of its own: warps 0-3 the epilogue, before it warp 3 operand B (one tiled TMA of
 // weights per k-block), warp 4 operand A (one im2col TMA of 128 output pixels x 64 channels of one filter tap), warp 5
 // tensor memory and the MMAs.  No thread computes an address in the main loop.  (A seventh warp for operand B would
 // leave 80 registers a thread at three CTAs per SM instead of 96.)
-constexpr int kThreadsTma = 192;
-constexpr int kWarpB = 3;
 
 // One CTA's share of one convolution: output tile (bx, by), rank bz of the cluster that shares the tile's
 // reduction, `stages` pipeline buffers.  Shared by the single-convolution kernel and the grouped one.
+// kPre: the tile's input is normalised first (see above; a kernel of its own: the others' code and registers stay as they are).
+template <bool kPre>
 __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const CUtensorMap* tmap_y, const CUtensorMap* tmap_r,
                                               const ConvArgs& a, const int stages,
                                               const int bx, const int by, const int bz, uint8_t* smem_raw,
                                               uint64_t* s_full, uint64_t* s_empty, uint64_t* s_accum, uint32_t* s_tmem_base,
-                                              volatile uint32_t* s_abort, float* s_bias, uint64_t* s_res, bool publish) {
+                                              volatile uint32_t* s_abort, float* s_bias, uint64_t* s_res, uint64_t* s_ready, bool publish) {
     const int tid = threadIdx.x;
     const int warp = (int)uniform((uint32_t)tid >> 5);
     const int lane = tid & 31;
@@ -850,6 +930,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
             for (int s = 0; s < stages; ++s) {
                 mbar_init(smem_u32(&s_full[s]), 1);      // this warp's arrive.expect_tx, for the bytes of both operands
                 mbar_init(smem_u32(&s_empty[s]), 1);     // tcgen05.commit
+                if (kPre) mbar_init(smem_u32(&s_ready[s]), 2);     // normalised: one arrival of each of two warps
             }
             mbar_init(smem_u32(s_accum), 1);
             mbar_init(smem_u32(s_res), 1);
@@ -894,7 +975,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
     if (tid == 0) { PB_T(1); PB_S(1); }
 
     if (warp < 4) {
-        if (warp == kWarpB) {
+        if (warp == kWarpB && !kPre) {
             // ===== operand B =====
             uint32_t* const err_flag = a.err_flag;
             uint32_t st = stages > 1 ? 1u : 0u, parity = stages > 1 ? 1u : 0u;
@@ -907,12 +988,19 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
                 __syncwarp();
                 if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
             }
-        } else {
+        } else if (warp != kWarpB) {
             // the epilogue's biases
             for (int j = tid; j < a.BN; j += 32 * kWarpB) {
                 const int k = n0 + j;
                 s_bias[j] = (a.bias && k < a.K) ? __ldg(a.bias + k) : 0.f;
             }
+        }
+        if (kPre) {
+            float* const consts = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + a.pre_offset);
+            normalise_constants(a, consts, kb_begin, nkb);
+            griddep_wait();
+            griddep_launch();
+            normalise_stages(a, smem_base, stage_bytes, stages, nkb, consts, s_full, s_ready, s_abort);
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         // The residual and the output may only be touched once the previous kernel has completed; the next kernel's
@@ -925,14 +1013,25 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         if (tid == 0) { PB_T(6); PB_S(6); }
     } else if (warp == 4) {
         // ===== operand A =====
-        griddep_wait();                           // the activations are the previous kernel's
         uint32_t* const err_flag = a.err_flag;
+        for (int kb = 1; kPre && kb < min(stages, nkb); ++kb) {      // operand B's warp normalises
+            if (elect_one()) {
+                mbar_arrive_expect_tx(smem_u32(&s_full[kb]), tx_bytes);
+                tma_load_2d(smem_base + kb * stage_bytes + kATileBytes, tmap_w, (kb_begin + kb) * kBK, n0, smem_u32(&s_full[kb]));
+            }
+            __syncwarp();
+        }
+        griddep_wait();                           // the activations are the previous kernel's
         const int S = a.S, dw = a.dw, dh = a.dh, a_tiled = a.a_tiled;
         uint32_t st = 0, parity = 1u;             // a fresh barrier passes a wait on the "previous" phase
         for (int kb = 0; kb < nkb; ++kb) {
             if (kb >= stages && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u))) break;
             if (elect_one()) {
                 const uint32_t a_tile = smem_base + st * stage_bytes, bar = smem_u32(&s_full[st]);
+                if (kPre && kb >= stages) {
+                    mbar_arrive_expect_tx(bar, tx_bytes);
+                    tma_load_2d(a_tile + kATileBytes, tmap_w, (kb_begin + kb) * kBK, n0, bar);
+                }
                 if (a_tiled) tma_load_2d(a_tile, tmap_x, chunk * kBK, m0, bar);
                 else tma_load_im2col_4d(a_tile, tmap_x, chunk * kBK, w0, h0, img, (uint16_t)(tap_s * dw), (uint16_t)(tap_r * dh), bar);
                 if (kb == 0) PB_T(2);
@@ -972,8 +1071,9 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         const uint32_t idesc = uniform(a.idesc), n_kb = uniform((uint32_t)nkb), n_st = uniform((uint32_t)stages);
         const uint64_t desc_a0 = umma_desc_sw128(uniform(smem_base)), desc_b0 = umma_desc_sw128(uniform(smem_base) + kATileBytes);
         const uint32_t desc_step = uniform(stage_bytes) >> 4;      // address field counts 16-byte units; no carry out of its 14 bits
+        uint64_t* const s_operands = kPre ? s_ready : s_full;
         for (uint32_t kb = 0; kb < n_kb; ++kb) {
-            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, s_abort, err_flag, 2u));
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_operands[st]), parity, s_abort, err_flag, 2u));
             if (!ok) break;
             if (lane == 0) { if (kb == 0) { PB_T(3); PB_S(3); } PB_TK(kb, 1); }
             tcgen05_fence_after();
@@ -1033,12 +1133,14 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 #endif
 }
 
+template <bool kPre>
 __global__ void __launch_bounds__(kThreadsTma, 3)
 conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                      const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_r, const ConvArgs a, int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxStages];
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
+    __shared__ __align__(8) uint64_t s_ready[kPre ? kMaxStages : 1];
     __shared__ __align__(8) uint64_t s_res;
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
@@ -1048,8 +1150,8 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     resolve_slot(job_id, nf);
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
-    conv_tile_tma(&tmap_w, &tmap_x, &tmap_y, &tmap_r, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
-                  &s_tmem_base, &s_abort, s_bias, &s_res, nf != nullptr);
+    conv_tile_tma<kPre>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+                  &s_tmem_base, &s_abort, s_bias, &s_res, s_ready, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1188,8 +1290,8 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     const uint32_t S = (uint32_t)s_args.splits, gx = sc->gx;
     const uint32_t tile = local / S, bz = local - tile * S;
     const uint32_t by = tile / gx, bx = tile - by * gx;
-    conv_tile_tma(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
-                  &s_tmem_base, &s_abort, s_bias, &s_res, nf != nullptr);
+    conv_tile_tma<false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
+                  &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1734,7 +1836,7 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
 }
 
 const void* kernel_for(int stages, bool tma) {
-    if (tma) return (const void*)conv_umma_tma_kernel;
+    if (tma) return (const void*)conv_umma_tma_kernel<false>;
     switch (stages) {
         case 4: return (const void*)conv_umma_gather_kernel<4>;
         case 6: return (const void*)conv_umma_gather_kernel<6>;
@@ -1744,7 +1846,7 @@ const void* kernel_for(int stages, bool tma) {
 
 // Raises the dynamic shared-memory limit of every kernel of this file on the current device.
 cudaError_t raise_smem_limits() {
-    const void* kernels[] = {(const void*)conv_umma_tma_kernel, (const void*)conv_umma_multi_kernel, (const void*)conv_umma_persist_kernel,
+    const void* kernels[] = {(const void*)conv_umma_tma_kernel<false>, (const void*)conv_umma_tma_kernel<true>, (const void*)conv_umma_multi_kernel, (const void*)conv_umma_persist_kernel,
                              (const void*)conv_umma_gather_kernel<4>, (const void*)conv_umma_gather_kernel<6>,
                              (const void*)conv_umma_gather_kernel<8>};
     for (const void* k : kernels) {
@@ -1883,16 +1985,17 @@ static bool pointwise(const pb_op_params* p) {
     return p->R == 1 && p->S == 1 && p->stride_h == 1 && p->stride_w == 1 && p->pad_h == 0 && p->pad_w == 0;      // any batch: images are contiguous
 }
 
-static int make_xmap(const pb_op_params* p, CUtensorMap* out) {
+static int make_xmap(const pb_op_params* p, const ConvPre* pre, CUtensorMap* out) {
     if (pointwise(p)) {
         EncodeTiledFn enc2 = encode_fn();
         PB_REQUIRE(enc2 != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
-        PB_REQUIRE(((uintptr_t)p->x & 15) == 0, "conv_umma: activations must be 16-byte aligned");
+        const void* const x = pre ? pre->x : p->x;
+        PB_REQUIRE(((uintptr_t)x & 15) == 0, "conv_umma: activations must be 16-byte aligned");
         const cuuint64_t dims2[2] = {(cuuint64_t)p->Cs, (cuuint64_t)batch_of(p) * p->H * p->W};
-        const cuuint64_t strides2[1] = {(cuuint64_t)p->Cs * 2};
+        const cuuint64_t strides2[1] = {(cuuint64_t)(pre ? pre->x_Cs : p->Cs) * 2};
         const cuuint32_t box2[2] = {(cuuint32_t)kBK, (cuuint32_t)kBM};
         const cuuint32_t estr2[2] = {1, 1};
-        const CUresult r2 = enc2(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p->x), dims2, strides2, box2, estr2,
+        const CUresult r2 = enc2(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims2, strides2, box2, estr2,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r2 != CUDA_SUCCESS) {
@@ -1943,6 +2046,12 @@ static int make_ymap(const pb_op_params* p, int U, bool residual, CUtensorMap* o
     return PB_OK;
 }
 
+// The affine's channels are the layer's input channels, in whole vectors (x_Cs apart from pixel to pixel).
+bool conv_umma_pre_supported(const pb_op_params* p, const ConvPre& pre) {
+    return use_tma_a() && pointwise(p) && p->C == p->Cs && p->C % 8 == 0 && pre.x_Cs % 8 == 0 && (pre.act == 0 || pre.act == 1) &&
+           (((uintptr_t)pre.scale | (uintptr_t)pre.bias) & 15) == 0;
+}
+
 struct alignas(64) ConvUmmaXMap {
     CUtensorMap map;
 };
@@ -1969,10 +2078,10 @@ int encode_tiled_bf16(const void* base, int rank, const uint64_t* dims, const ui
     return PB_OK;
 }
 
-int conv_umma_xmap_create(const pb_op_params* p, ConvUmmaXMap** out) {
+int conv_umma_xmap_create(const pb_op_params* p, ConvUmmaXMap** out, const ConvPre* pre) {
     if (!use_tma_a()) { *out = nullptr; return PB_OK; }
     ConvUmmaXMap* m = new ConvUmmaXMap();
-    const int rc = make_xmap(p, &m->map);
+    const int rc = make_xmap(p, pre, &m->map);
     if (rc != PB_OK) { delete m; return rc; }
     *out = m;
     return PB_OK;
@@ -2053,18 +2162,23 @@ static cudaError_t launch_pdl(void (*kern)(Args...), dim3 grid, dim3 cluster, ui
 }
 
 int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap, const pb_op_params* p, cudaStream_t st,
-                             uint32_t job_id, void* notifier, uint32_t* err_flag, bool pdl, const ConvTiling* tiling) {
+                             uint32_t job_id, void* notifier, uint32_t* err_flag, bool pdl, const ConvTiling* tiling, const ConvPre* pre) {
     const Geometry g = geometry(p, tiling_or(tiling, p));
     if (!use_tma_a()) PB_REQUIRE(batch_of(p) == 1, "conv_umma: the cp.async gather kernel (PB_CONV_GATHER=1) runs one image per launch");
     ConvArgs a;
     const int frc = fill_args(plan, g, p, err_flag, &a);
     if (frc != PB_OK) return frc;
+    if (pre) {
+        PB_REQUIRE(use_tma_a() && conv_umma_pre_supported(p, *pre), "conv_umma: this layer cannot take an input affine");
+        a.pre_scale = pre->scale; a.pre_bias = pre->bias; a.pre_act = pre->act; a.pre_offset = g.smem_bytes - 1024u;
+    }
+    const uint32_t smem = g.smem_bytes + (pre ? (uint32_t)ceil_div(g.nkb, g.splits) * 512u : 0u);
     const dim3 grid((unsigned)g.m_tiles, (unsigned)g.n_tiles, (unsigned)g.splits);
     FinishedBlockNotifier* nf = static_cast<FinishedBlockNotifier*>(notifier);
     if (use_tma_a()) {
         ConvUmmaXMap local;
         if (!xmap) {
-            const int rc = make_xmap(p, &local.map);
+            const int rc = make_xmap(p, pre, &local.map);
             if (rc != PB_OK) return rc;
             xmap = &local;
         }
@@ -2073,7 +2187,7 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
         if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, false, &ymap);
         if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, true, &rmap);
         if (mrc != PB_OK) return mrc;
-        const cudaError_t e = launch_pdl(conv_umma_tma_kernel, grid, dim3(1, 1, (unsigned)g.splits), g.smem_bytes, st, pdl, wmap, xmap->map, ymap, rmap, a,
+        const cudaError_t e = launch_pdl(pre ? conv_umma_tma_kernel<true> : conv_umma_tma_kernel<false>, grid, dim3(1, 1, (unsigned)g.splits), smem, st, pdl, wmap, xmap->map, ymap, rmap, a,
                                          g.stages, job_id, nf);
         if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_tma_kernel", __FILE__, __LINE__);
         return PB_OK;

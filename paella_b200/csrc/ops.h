@@ -68,14 +68,24 @@ int conv_umma_plan_create(const pb_op_params* p, const void* w_dev, ConvUmmaPlan
 void conv_umma_plan_destroy(ConvUmmaPlan* plan);
 // Per-instance state: the im2col TMA descriptor of one layer's INPUT tensor (`p->x`).
 struct ConvUmmaXMap;
-int conv_umma_xmap_create(const pb_op_params* p, ConvUmmaXMap** out);
+// An affine (+ ReLU) in front of a pointwise convolution: it reads act(x * scale + bias), per channel, where p->x would have been.
+struct ConvPre {
+    const void* x;
+    int x_Cs;                  // channel stride of x
+    const float* scale;
+    const float* bias;
+    int act;                   // 0 or 1
+};
+bool conv_umma_pre_supported(const pb_op_params* p, const ConvPre& pre);
+int conv_umma_xmap_create(const pb_op_params* p, ConvUmmaXMap** out, const ConvPre* pre = nullptr);
 void conv_umma_xmap_destroy(ConvUmmaXMap* m);
 // xmap may be NULL: the descriptor is then encoded for this one launch.
 // err_flag: device word raised when a bounded wait runs out (NULL = the library's per-device flag).
 // pdl: launch with the programmatic-serialization attribute (the kernel waits for its predecessor
 // itself, after its set-up); only meaningful when the previous operation in `st` is a kernel.
 int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap, const pb_op_params* p, cudaStream_t st,
-                             uint32_t job_id, void* notifier, uint32_t* err_flag = nullptr, bool pdl = false, const ConvTiling* tiling = nullptr);
+                             uint32_t job_id, void* notifier, uint32_t* err_flag = nullptr, bool pdl = false, const ConvTiling* tiling = nullptr,
+                             const ConvPre* pre = nullptr);
 // Grouped launch: up to 8 independent convolutions (their plans, input descriptors and resolved
 // parameters) run as ONE grid; the table of descriptors is copied to device memory here.
 struct ConvUmmaMulti;

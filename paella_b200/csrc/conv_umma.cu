@@ -813,7 +813,8 @@ constexpr int kWarpB = 3;          // issues operand B's copies
 // raw features is normalised where it landed: the epilogue's warps, idle until the accumulator is complete, rewrite each stage of
 // operand A in shared memory and then let the MMA warp have it (operand A's warp loads operand B too).  Two warps take a stage, so
 // that one pair's wait and fence lie beside the other's arithmetic; a thread has one vector of 8 channels of sixteen rows, eight in
-// flight.
+// flight.  Bound by these warps' instructions: about 0.35 us a k-block, where a layer without it takes 0.2 (all four warps on one
+// stage: 0.37; three warps: 0.48; constants read from global memory per k-block: 1.0, slower than the launch it replaces).
 // The arithmetic is affine_kernel's - fp32 multiply-add, ReLU, one rounding to bf16 - and so are the bits (the maximum with
 // zero may follow the rounding: rounding is monotonic and keeps zeros; NaN gives zero either way).
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z) {

@@ -342,10 +342,23 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
     hi = __uint_as_float(h);
 }
 
+// What the epilogues need of a convolution's arguments, in registers before they wait for the accumulator.  (A grouped launch has
+// its arguments in shared memory, and a compiler that sees a memory barrier reads them again behind each.)
+struct EpiArgs {
+    const __nv_bfloat16* residual;
+    const float* bias;
+    __nv_bfloat16* y;
+    uint32_t* err_flag;
+    int M, K, Ks, out_c_off, res_Cs, act, BN, out_box, splits, nkb;
+};
+__device__ __forceinline__ EpiArgs epi_args(const ConvArgs& a) {
+    return {a.residual, a.bias, a.y, a.err_flag, a.M, a.K, a.Ks, a.out_c_off, a.res_Cs, a.act, a.BN, a.out_box, a.splits, a.nkb};
+}
+
 // Eight accumulator columns of this thread's row, from channel k on: + bias (+ residual), activation, bf16.  The four epilogue
 // warps run one per scheduler with nothing to hide instruction latency behind, so this is kept to one packed add and one
 // convert per two columns.
-__device__ __forceinline__ uint4 finish8(const ConvArgs& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias) {
+__device__ __forceinline__ uint4 finish8(const EpiArgs& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias) {
     uint64_t f[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -392,7 +405,7 @@ __device__ __forceinline__ uint4 finish8(const ConvArgs& a, const uint32_t* v, c
     }
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
-__device__ __forceinline__ void epilogue_chunk(const ConvArgs& a, const uint32_t (&v)[16], const uint4 (&rv)[2], int cb, int n0, bool row_valid,
+__device__ __forceinline__ void epilogue_chunk(const EpiArgs& a, const uint32_t (&v)[16], const uint4 (&rv)[2], int cb, int n0, bool row_valid,
                                                __nv_bfloat16* yrow, bool has_res, const float* s_bias) {
     if (!row_valid) return;
 #pragma unroll
@@ -403,7 +416,7 @@ __device__ __forceinline__ void epilogue_chunk(const ConvArgs& a, const uint32_t
 }
 
 // The residual of the 16 columns from cb on (zeros where there is none).
-__device__ __forceinline__ void load_residual(const ConvArgs& a, int k0, bool row_valid, const __nv_bfloat16* rrow, uint4 (&rv)[2]) {
+__device__ __forceinline__ void load_residual(const EpiArgs& a, int k0, bool row_valid, const __nv_bfloat16* rrow, uint4 (&rv)[2]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         rv[h] = make_uint4(0, 0, 0, 0);
@@ -413,7 +426,7 @@ __device__ __forceinline__ void load_residual(const ConvArgs& a, int k0, bool ro
 
 // Columns in steps of 16, two steps in flight: the next step leaves tensor memory (and its residual is on its way)
 // while this one is converted and stored.
-__device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lane_addr, int n0, bool row_valid, __nv_bfloat16* yrow,
+__device__ __forceinline__ void epilogue_columns(const EpiArgs& a, uint32_t lane_addr, int n0, bool row_valid, __nv_bfloat16* yrow,
                                                  const __nv_bfloat16* rrow, const float* s_bias) {
     uint32_t v0[16], v1[16];
     uint4 r0[2], r1[2];
@@ -447,7 +460,7 @@ __device__ __forceinline__ void epilogue_columns(const ConvArgs& a, uint32_t lan
 // result, and one lane of a warp stores the warp's 32 rows of a finished box with one instruction.  `buf`: 128 x BN x 2 bytes
 // of the pipeline memory, free by now.  publish: this launch reports to the host, so the stores have to be in memory when the
 // warp leaves; otherwise they only have to have been read (the next kernel waits for this one's memory operations).
-__device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t lane_addr, int n0, bool has_res, const float* s_bias, uint32_t buf,
+__device__ __forceinline__ void epilogue_columns_tma(const EpiArgs& a, uint32_t lane_addr, int n0, bool has_res, const float* s_bias, uint32_t buf,
                                                      const CUtensorMap* tmap_y, int m0, bool publish) {
     const uint32_t r = threadIdx.x;                 // tile row
     const int U = a.out_box, m_warp = m0 + (int)(r & ~31u);
@@ -493,9 +506,10 @@ __device__ __forceinline__ void epilogue_columns_tma(const ConvArgs& a, uint32_t
 // Epilogue, run by warps 0-3 (thread t owns accumulator lane t = tile row t): wait for the
 // accumulator, then bias + residual + activation and bf16 stores into the output channel slice.
 // tmap_y (the one-tile kernels): through TMA stores staged at `buf`.
-__device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, bool ok, int m0, int n0, const float* s_bias,
+__device__ __forceinline__ void epilogue(const ConvArgs& args, uint32_t tmem_base, bool ok, int m0, int n0, const float* s_bias,
                                          uint64_t* s_accum_p, volatile uint32_t* s_abort_p, uint32_t accum_parity = 0u,
                                          const CUtensorMap* tmap_y = nullptr, uint32_t buf = 0, uint64_t* s_res = nullptr, bool publish = true) {
+    const EpiArgs a = epi_args(args);
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int m = m0 + tid;
@@ -528,7 +542,7 @@ __device__ __forceinline__ void epilogue(const ConvArgs& a, uint32_t tmem_base, 
 // (The partial tiles used to meet in a global workspace under an atomic counter: two fences, an atomic and an L2
 // round trip of BN x 512 bytes per rank, read back by ONE block: +4 to +8 us per launch, so only reductions of 60
 // and more k-blocks gained from it.)
-__device__ __forceinline__ void cluster_finish(const ConvArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
+__device__ __forceinline__ void cluster_finish(const EpiArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
                                                const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
     const int S = a.splits;
     uint32_t active = (1u << S) - 1u;      // ranks that have k-blocks (all of them unless a grouped launch splits a short reduction)
@@ -590,8 +604,9 @@ __device__ __forceinline__ void cluster_finish(const ConvArgs& a, int n0, bool r
 }
 
 // Run by warps 0-3 of every rank.  `mine`: this rank has k-blocks of its own.
-__device__ __forceinline__ void epilogue_cluster(const ConvArgs& a, uint32_t tmem_base, int m0, int n0, int rank, bool mine, uint32_t smem_base,
+__device__ __forceinline__ void epilogue_cluster(const ConvArgs& args, uint32_t tmem_base, int m0, int n0, int rank, bool mine, uint32_t smem_base,
                                                  const float* s_bias, uint64_t* s_accum_p, volatile uint32_t* s_abort_p) {
+    const EpiArgs a = epi_args(args);
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int m = m0 + tid;

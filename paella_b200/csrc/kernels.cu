@@ -1040,6 +1040,8 @@ __global__ void __launch_bounds__(256) add_kernel(OpArgs a, uint32_t job_id, Fin
 // y[pix][c] = act(x[pix][c] * scale[c] + bias[c]) for the first a.C channels: the folded batch-norm +
 // ReLU that DenseNet applies to the concatenated features BEFORE each convolution.
 constexpr int kAffinePer = 4;      // vectors per thread
+// Threads of a launch over `pixels` pixels of `cv` vectors: a quarter of the pixels, rounded up.
+__host__ __device__ __forceinline__ size_t affine_threads(size_t pixels, int cv) { return (pixels + kAffinePer - 1) / kAffinePer * cv; }
 
 template <typename T>
 __global__ void __launch_bounds__(256) affine_kernel(OpArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
@@ -1047,47 +1049,49 @@ __global__ void __launch_bounds__(256) affine_kernel(OpArgs a, uint32_t job_id, 
     constexpr int N = Vec<T>::N;
     typedef typename RawVec<T>::type Raw;
     const int cv = (a.C + N - 1) / N;
-    const size_t total = (size_t)a.H * a.W * cv;
-    // kAffinePer vectors per thread, a quarter of the tensor apart, all loads issued (as raw 128-bit words)
-    // before any is used: with one load in flight per thread the kernel ran at 54 % of the copy bandwidth
-    // on a tensor larger than L2, which needs about 50 KB in flight per SM.
-    const size_t part = (total + kAffinePer - 1) / kAffinePer;
+    // A thread takes the same kAffinePer channels' vector of kAffinePer pixels, a quarter of the tensor apart: all loads are issued
+    // (as raw 128-bit words) before any is used - with one load in flight per thread the kernel ran at 54 % of the copy
+    // bandwidth on a tensor larger than L2, which needs about 50 KB in flight per SM - and scale and bias are loaded once.
+    // (Loaded for every vector they were two thirds of the bytes through L1, whose data pipe was 76 % busy: 16 x 256 x 256 x 128 in
+    // bf16 108.4 us, 86.3 now: 95 % of the copy bandwidth.)
+    const size_t pixels = (size_t)a.H * a.W, part = affine_threads(pixels, cv), step = part / cv;
     const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i0 < part) {
-        size_t pix[kAffinePer];
-        int c0[kAffinePer];
+        // 32-bit division whenever the index fits (always, short of a 64 GB tensor)
+        const size_t pix0 = part <= 0xffffffffull ? (size_t)((uint32_t)i0 / (uint32_t)cv) : i0 / cv;
+        const int c0 = (int)(i0 - pix0 * cv) * N;
+        const T* __restrict__ x = static_cast<const T*>(a.x) + c0;
         Raw raw[kAffinePer];
 #pragma unroll
         for (int h = 0; h < kAffinePer; ++h) {
-            const size_t i = (i0 + h * part < total) ? i0 + h * part : i0;
-            // 32-bit division whenever the index fits (always, short of a 64 GB tensor)
-            pix[h] = total <= 0xffffffffull ? (size_t)((uint32_t)i / (uint32_t)cv) : i / cv;
-            c0[h] = (int)(i - pix[h] * cv) * N;
-            raw[h] = *reinterpret_cast<const Raw*>(static_cast<const T*>(a.x) + pix[h] * a.Cs + c0[h]);
+            const size_t pix = pix0 + h * step;
+            raw[h] = *reinterpret_cast<const Raw*>(x + (pix < pixels ? pix : pix0) * a.Cs);
         }
-        const float* __restrict__ sc = static_cast<const float*>(a.w);
-        const bool aligned = ((reinterpret_cast<uintptr_t>(sc) | reinterpret_cast<uintptr_t>(a.bias)) & 15) == 0;
+        const float* __restrict__ sc = static_cast<const float*>(a.w) + c0;
+        const float* __restrict__ bi = a.bias + c0;
+        float scv[N], biv[N];
+        if (c0 + N <= a.C && ((reinterpret_cast<uintptr_t>(sc) | reinterpret_cast<uintptr_t>(bi)) & 15) == 0) {
+#pragma unroll
+            for (int j = 0; j < N; j += 4) {
+                *reinterpret_cast<float4*>(scv + j) = __ldg(reinterpret_cast<const float4*>(sc + j));
+                *reinterpret_cast<float4*>(biv + j) = __ldg(reinterpret_cast<const float4*>(bi + j));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                scv[j] = c0 + j < a.C ? __ldg(sc + j) : 0.f;
+                biv[j] = c0 + j < a.C ? __ldg(bi + j) : 0.f;
+            }
+        }
 #pragma unroll
         for (int h = 0; h < kAffinePer; ++h) {
-            if (h > 0 && i0 + h * part >= total) break;
+            const size_t pix = pix0 + h * step;
+            if (pix >= pixels) break;
             const Vec<T> u = vec_of(raw[h]);
             Vec<T> o;
-            if (c0[h] + N <= a.C && aligned) {
-                // whole vector inside the tensor: scale and bias as 128-bit loads instead of 2 x N scalar ones
-                float scv[N], biv[N];
 #pragma unroll
-                for (int j = 0; j < N; j += 4) {
-                    *reinterpret_cast<float4*>(scv + j) = __ldg(reinterpret_cast<const float4*>(sc + c0[h] + j));
-                    *reinterpret_cast<float4*>(biv + j) = __ldg(reinterpret_cast<const float4*>(a.bias + c0[h] + j));
-                }
-#pragma unroll
-                for (int j = 0; j < N; ++j) o.v[j] = act_fn(u.v[j] * scv[j] + biv[j], a.act);
-            } else {
-#pragma unroll
-                for (int j = 0; j < N; ++j)
-                    o.v[j] = (c0[h] + j < a.C) ? act_fn(u.v[j] * __ldg(sc + c0[h] + j) + __ldg(a.bias + c0[h] + j), a.act) : 0.f;
-            }
-            o.store(static_cast<T*>(a.y) + pix[h] * a.Ks + a.out_c_off + c0[h]);
+            for (int j = 0; j < N; ++j) o.v[j] = c0 + j < a.C ? act_fn(u.v[j] * scv[j] + biv[j], a.act) : 0.f;
+            o.store(static_cast<T*>(a.y) + pix * a.Ks + a.out_c_off + c0);
         }
     }
     PB_NOTIFY_END();
@@ -1585,7 +1589,7 @@ static int info_one_image(int kind, const pb_op_params* p, pb_launch_info* out) 
             out->bytes = es * 3 * in_elems;
             break;
         case PB_STAGE_AFFINE:
-            out->num_blocks = blocks_for(((size_t)p->H * p->W * pb::ceil_div(p->C, N) + kAffinePer - 1) / kAffinePer);
+            out->num_blocks = blocks_for(affine_threads((size_t)p->H * p->W, pb::ceil_div(p->C, N)));
             out->regs_per_thread = f32 ? regs_of(affine_kernel<float>) : regs_of(affine_kernel<__nv_bfloat16>);
             out->flops = 2ull * p->C * p->H * p->W;
             out->bytes = es * 2ull * p->C * p->H * p->W + 8ull * p->C;

@@ -1207,7 +1207,7 @@ constexpr int kPoolVecsPerThread = 2;                 // output vectors (8 chann
 
 // One block's share of a 3x3 pooling layer: thread t takes output vectors base + t and base + 192 + t.  All nine
 // loads of a window are issued before the first use (addresses clamped into the tensor, taps outside dropped
-// afterwards).  Arithmetic and its order are those of pool_kernel / window3_strip_kernel (rows, then columns, fp32
+// afterwards).  Arithmetic and its order are those of pool_kernel / window3_strip_kernel (the columns of a row, then the rows, fp32
 // sums from +0, IEEE division; fmaxf from -inf), so the bits are theirs.
 __device__ __forceinline__ void pool_sub_block(const PoolSubArgs& a, uint32_t local_block) {
     const int cv = a.Cs >> 3;
@@ -1242,7 +1242,10 @@ __device__ __forceinline__ void pool_sub_block(const PoolSubArgs& a, uint32_t lo
         for (int j = 0; j < 8; ++j) acc[j] = a.is_max ? -INFINITY : 0.f;
         int cnt = 0;
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+        for (int r = 0; r < 3; ++r) {
+            float row[8];                     // sums: the columns of a row first, as in the pooling kernels
+#pragma unroll
+            for (int j = 0; j < 8; ++j) row[j] = 0.f;
 #pragma unroll
             for (int s2 = 0; s2 < 3; ++s2) {
                 if (!((ok >> (r * 3 + s2)) & 1u)) continue;
@@ -1250,11 +1253,21 @@ __device__ __forceinline__ void pool_sub_block(const PoolSubArgs& a, uint32_t lo
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xffff0000u);
-                    acc[2 * j] = a.is_max ? fmaxf(acc[2 * j], lo) : acc[2 * j] + lo;
-                    acc[2 * j + 1] = a.is_max ? fmaxf(acc[2 * j + 1], hi) : acc[2 * j + 1] + hi;
+                    if (a.is_max) {
+                        acc[2 * j] = fmaxf(acc[2 * j], lo);
+                        acc[2 * j + 1] = fmaxf(acc[2 * j + 1], hi);
+                    } else {
+                        row[2 * j] += lo;
+                        row[2 * j + 1] += hi;
+                    }
                 }
                 ++cnt;
             }
+            if (!a.is_max) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j] += row[j];
+            }
+        }
         const float div = a.count_pad ? 9.f : (float)(cnt > 0 ? cnt : 1);
         uint32_t o[4];
 #pragma unroll

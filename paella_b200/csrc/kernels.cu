@@ -361,13 +361,23 @@ __global__ void __launch_bounds__(256, 6) pool_kernel(OpArgs a, uint32_t job_id,
         for (int r = 0; r < a.R; ++r) {
             const int ih = p * a.stride_h + r - a.pad_h;
             if (ih < 0 || ih >= a.H) continue;
+            float row[N];                     // average pooling: the columns of a row first
+#pragma unroll
+            for (int j = 0; j < N; ++j) row[j] = 0.f;
             for (int s = 0; s < a.S; ++s) {
                 const int iw = q * a.stride_w + s - a.pad_w;
                 if (iw < 0 || iw >= a.W) continue;
                 const Vec<T> xv = Vec<T>::load(x + ((size_t)ih * a.W + iw) * a.Cs + c0);
 #pragma unroll
-                for (int j = 0; j < N; ++j) acc[j] = kMax ? fmaxf(acc[j], xv.v[j]) : acc[j] + xv.v[j];
+                for (int j = 0; j < N; ++j) {
+                    if (kMax) acc[j] = fmaxf(acc[j], xv.v[j]);
+                    else row[j] += xv.v[j];
+                }
                 ++cnt;
+            }
+            if (!kMax) {
+#pragma unroll
+                for (int j = 0; j < N; ++j) acc[j] += row[j];
             }
         }
         Vec<T> o;
@@ -392,8 +402,8 @@ __global__ void __launch_bounds__(256, 6) pool_kernel(OpArgs a, uint32_t job_id,
 // ALL loads of the strip's window back to back, unconditionally (addresses clamped into the tensor, the
 // taps that fall outside are dropped afterwards), so 6-9 loads per thread are in flight; each loaded
 // vector feeds every output it belongs to, and a row of weights is loaded once per thread.
-// The order of the additions per output is the one of dwconv_kernel / pool_kernel (rows, then columns),
-// so results are bit-identical to theirs.  Used when the strips alone fill the GPU (strip_threads()).
+// The order of the additions per output is the one of dwconv_kernel / pool_kernel (depthwise: rows, then columns; average:
+// the columns of each row, then the rows), so results are bit-identical to theirs.  Used when the strips alone fill the GPU (strip_threads()).
 // With kStrip = 1 (every other 3x3 layer of stride 1 or 2, i.e. the batch-1 layers of the served models)
 // the thread owns one output vector as in dwconv_kernel / pool_kernel, but its nine loads are
 // unconditional and in flight together instead of one guarded load after the other.
@@ -541,6 +551,11 @@ __global__ void __launch_bounds__(256, 2) window3_strip_kernel(OpArgs a, uint32_
 #pragma unroll
                 for (int s = 0; s < 3; ++s) unpack_pairs(*reinterpret_cast<const Raw*>(w + (r * 3 + s) * a.Cs), wv[s]);
             }
+            f2_t row_sum[kStrip][NP];         // average pooling: the columns of a row first
+#pragma unroll
+            for (int t = 0; t < kStrip; ++t)
+#pragma unroll
+                for (int j = 0; j < NP; ++j) row_sum[t][j] = f2_pack(0.f, 0.f);
 #pragma unroll
             for (int col = 0; col < kCols; ++col) {
                 if (!((ok[r] >> col) & 1u)) continue;
@@ -555,9 +570,15 @@ __global__ void __launch_bounds__(256, 2) window3_strip_kernel(OpArgs a, uint32_
                     for (int j = 0; j < NP; ++j) {
                         if (kMode == kWinDw) acc[t][j] = f2_fma(xv[j], wv[s][j], acc[t][j]);
                         else if (kMode == kWinMax) acc[t][j] = f2_max(acc[t][j], xv[j]);
-                        else acc[t][j] = f2_add(acc[t][j], xv[j]);
+                        else row_sum[t][j] = f2_add(row_sum[t][j], xv[j]);
                     }
                 }
+            }
+            if (kMode == kWinAvg) {
+#pragma unroll
+                for (int t = 0; t < kStrip; ++t)
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) acc[t][j] = f2_add(acc[t][j], row_sum[t][j]);
             }
         }
         T* yrow = y_img<T>(a) + ((size_t)p * a.Q + q0) * a.Ks + a.out_c_off + c0;
@@ -640,8 +661,10 @@ __global__ void __launch_bounds__(256, 2) window3_strip_kernel(OpArgs a, uint32_
 //
 // Max pooling compares the bf16 pairs themselves (a maximum needs no wider type); ReLU / ReLU6 clamp the rounded bf16 pair
 // (rounding is monotonic and 0 and 6 are bf16 values).  Taps outside the tensor contribute the neutral element; an
-// output's first tap opens its accumulator, so only the sign of a sum of zeros could show it.  The additions per output happen in the order of dwconv_kernel / pool_kernel (filter
-// rows, then columns), so the results are theirs bit for bit (finite filter values assumed).  bf16 only.
+// output's first tap opens its accumulator, so only the sign of a sum of zeros could show it.  The additions per output happen in the order of dwconv_kernel / pool_kernel (depthwise: filter
+// rows, then columns; average: the columns of each row, then the rows, so that a row's three columns are added once for the three
+// output rows they belong to: 4 additions instead of 9 a channel, 256 maps of 35 x 35 x 192 54.4 -> 49.2 us), so the results are theirs bit for bit (finite filter values
+// assumed).  bf16 only.
 constexpr int kTileStrip1 = 4, kTileStrip2 = 2;      // output columns per strip at stride 1 / 2
 constexpr int kTileRows1 = 13, kTileRows2 = 6;       // output rows per tile (single images; batches: see win_tile())
 constexpr int kTileSlab = 64;                        // channels per block
@@ -824,27 +847,44 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
         const uint2* row = reinterpret_cast<const uint2*>(s_tile) + (band * g.band_rows * kStride) * pitch + strip * kStrip * kStride * (kTileSlab / 4) + (threadIdx.x & 15);
         T* __restrict__ y = y_img<T>(a) + ((size_t)p0 * a.Q + q0) * a.Ks + a.out_c_off + c0;
 
-        auto row_into = [&](Acc (&acc)[kStrip][2], const Acc (&xv)[kCols][2], int r) {
+        // A window row as the walk wants it: its columns (depthwise), or for pooling each output's three columns already reduced, once
+        // for the three output rows the window row belongs to.
+        constexpr int kRow = kDw ? kCols : kStrip;
+        auto row_into = [&](Acc (&acc)[kStrip][2], const Acc (&xv)[kRow][2], int r) {
 #pragma unroll
-            for (int t = 0; t < kStrip; ++t)
+            for (int t = 0; t < kStrip; ++t) {
+                if constexpr (!kDw) {
 #pragma unroll
-                for (int s2 = 0; s2 < 3; ++s2) {
-                    if (r == 0 && s2 == 0) {
-                        acc[t][0] = win_open(xv[t * kStride][0], w[0][0][0], kDw);
-                        acc[t][1] = win_open(xv[t * kStride][1], w[0][0][1], kDw);
-                        continue;
+                    for (int j = 0; j < 2; ++j) acc[t][j] = r == 0 ? xv[t][j] : win_step(acc[t][j], xv[t][j], 0, false);
+                } else {
+#pragma unroll
+                    for (int s2 = 0; s2 < 3; ++s2) {
+                        if (r == 0 && s2 == 0) {
+                            acc[t][0] = win_open(xv[t * kStride][0], w[0][0][0], true);
+                            acc[t][1] = win_open(xv[t * kStride][1], w[0][0][1], true);
+                            continue;
+                        }
+                        acc[t][0] = win_step(acc[t][0], xv[t * kStride + s2][0], w[r][s2][0], true);
+                        acc[t][1] = win_step(acc[t][1], xv[t * kStride + s2][1], w[r][s2][1], true);
                     }
-                    acc[t][0] = win_step(acc[t][0], xv[t * kStride + s2][0], w[r][s2][0], kDw);
-                    acc[t][1] = win_step(acc[t][1], xv[t * kStride + s2][1], w[r][s2][1], kDw);
                 }
+            }
         };
-        auto load_row = [&](Acc (&xv)[kCols][2]) {
+        auto load_row = [&](Acc (&xv)[kRow][2]) {
+            Acc col_v[kCols][2];
 #pragma unroll
             for (int col = 0; col < kCols; ++col) {
                 const uint2 v = row[col * (kTileSlab / 4)];
-                xv[col][0] = win_value<kMode>(v.x);
-                xv[col][1] = win_value<kMode>(v.y);
+                col_v[col][0] = win_value<kMode>(v.x);
+                col_v[col][1] = win_value<kMode>(v.y);
             }
+#pragma unroll
+            for (int t = 0; t < kRow; ++t)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if constexpr (kDw) xv[t][j] = col_v[t][j];
+                    else xv[t][j] = win_step(win_step(col_v[t * kStride][j], col_v[t * kStride + 1][j], 0, false), col_v[t * kStride + 2][j], 0, false);
+                }
             row += pitch;
         };
         auto store_row = [&](const Acc (&acc)[kStrip][2], int p, bool all) {
@@ -891,7 +931,7 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
                 for (int j = 0; j < 2; ++j) accB[t][j] = accC[t][j] = 0;          // (rows before p0: never stored)
 #pragma unroll 1
             for (int p = p0; p < p1 + 2; p += 3) {
-                Acc xv[kCols][2];
+                Acc xv[kRow][2];
                 load_row(xv); row_into(accB, xv, 2); row_into(accC, xv, 1); row_into(accA, xv, 0); close_row(accB, p - 2);
                 load_row(xv); row_into(accC, xv, 2); row_into(accA, xv, 1); row_into(accB, xv, 0); close_row(accC, p - 1);
                 load_row(xv); row_into(accA, xv, 2); row_into(accB, xv, 1); row_into(accC, xv, 0); close_row(accA, p);
@@ -903,11 +943,11 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
             for (int t = 0; t < kStrip; ++t) acc[t][0] = acc[t][1] = 0;
 #pragma unroll 1
             for (int p = p0; p < p1; ++p) {
-                Acc xv[kCols][2];
+                Acc xv[kRow][2];
                 load_row(xv); row_into(acc, xv, 2); close_row(acc, p - 1); row_into(acc, xv, 0);
                 load_row(xv); row_into(acc, xv, 1);
             }
-            Acc xv[kCols][2];
+            Acc xv[kRow][2];
             load_row(xv);
             row_into(acc, xv, 2);
             close_row(acc, p1 - 1);

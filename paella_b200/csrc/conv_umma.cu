@@ -1171,6 +1171,200 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     if (nf) nf->end(job_id);
 }
 
+// ---- a pair of blocks on one tile of 256 rows ---------------------------------------------------------------------
+// A lone block of 128 rows loads 16 KB of activations and BN x 128 bytes of weights for each k-block, and its tensor core reads both
+// from shared memory again: 40 KB each way at 192 columns against 384 clocks of multiplications, where an SM loads 60 bytes a
+// clock and its shared memory moves 128.  Here two SMs share a tile of 256 x BN (tcgen05 with cta_group::2): each holds 128 rows of
+// operand A and HALF of operand B's columns, so the weights cross each SM's load path and shared memory once for 256 rows.
+// Each block loads its own halves; the copies of both count on the barriers of the first (its "full" barriers), whose MMA warp
+// issues for the pair and commits to the barriers of both ("empty", "accumulator complete").  Each block has its own rows of
+// the accumulator in its tensor memory and finishes them as a lone block does.  Two pairs share a pair of SMs, so one's epilogue
+// and barrier latencies lie under the other's multiplications.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_4d_pair(uint32_t dst, const CUtensorMap* map, int c, int w, int h, int n, uint16_t w_off, uint16_t h_off,
+                                                        uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
+        ::"r"(dst), "l"(map), "r"(leader_bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(w_off), "h"(h_off)
+        : "memory");
+}
+__device__ __forceinline__ void tcgen05_mma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Arrives on the barrier at this offset in both blocks once the pair's multiplications so far are complete.
+__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+
+__global__ void __launch_bounds__(kThreadsTma, 2)
+conv_umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
+                      const __grid_constant__ CUtensorMap tmap_r, const ConvArgs a, int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t s_full[kMaxStages];
+    __shared__ __align__(8) uint64_t s_empty[kMaxStages];
+    __shared__ __align__(8) uint64_t s_res;
+    __shared__ __align__(8) uint64_t s_accum;
+    __shared__ uint32_t s_tmem_base;
+    __shared__ volatile uint32_t s_abort;
+    __shared__ __align__(16) float s_bias[kMaxBN];
+
+    resolve_slot(job_id, nf);
+    if (nf) nf->start(job_id);
+    const int tid = threadIdx.x;
+    const int warp = (int)uniform((uint32_t)tid >> 5);
+    const int rank = (int)(blockIdx.x & 1u);                       // in the pair (clusters are two blocks along x)
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t stage_bytes = (uint32_t)kATileBytes + a.b_stage_bytes;      // b_stage_bytes: this block's half
+    const int m0 = (int)blockIdx.x * kBM, n0 = (int)blockIdx.y * a.BN, half = a.BN / 2;
+    const int nkb = a.nkb;
+
+    if (warp == kWarpB) {
+        if (elect_one()) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+            for (int s = 0; s < stages; ++s) {
+                mbar_init(smem_u32(&s_full[s]), 1);
+                mbar_init(smem_u32(&s_empty[s]), 1);
+            }
+            mbar_init(smem_u32(&s_accum), 1);
+            mbar_init(smem_u32(&s_res), 1);
+            s_abort = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncwarp();
+    }
+    const int cpt = a.Cp / kBK;
+    const int img = m0 / a.PQ, rem = m0 - img * a.PQ;
+    const int p0 = rem / a.Q, q0 = rem - p0 * a.Q;
+    const int w0 = q0 * a.sw - a.pw, h0 = p0 * a.sh - a.ph;
+    if (warp == 4 && elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)), "r"(a.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();                     // both blocks' barriers and tensor memory are set up
+    tcgen05_fence_after();
+    const uint32_t tmem_base = uniform(s_tmem_base);
+
+    if (warp < 4) {
+        if (warp == kWarpB) {
+            // ===== operand B: this block's half of the columns =====
+            uint32_t* const err_flag = a.err_flag;
+            uint32_t st = 0, parity = 1u;
+            for (int kb = 0; kb < nkb; ++kb) {
+                if (kb >= stages && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, &s_abort, err_flag, 1u))) break;
+                if (elect_one()) {
+                    const uint32_t bar = smem_u32(&s_full[st]);
+                    if (rank == 0) mbar_arrive_expect_tx(bar, 2u * stage_bytes);       // both blocks' copies
+                    tma_load_2d_pair(smem_base + st * stage_bytes + kATileBytes, &tmap_w, kb * kBK, n0 + rank * half, cluster_addr(bar, 0u));
+                }
+                __syncwarp();
+                if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
+            }
+        } else {
+            for (int j = tid; j < a.BN; j += 32 * kWarpB) {
+                const int k = n0 + j;
+                s_bias[j] = (a.bias && k < a.K) ? __ldg(a.bias + k) : 0.f;
+            }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        griddep_wait();
+        griddep_launch();
+        epilogue(a, tmem_base, true, m0, n0, s_bias, &s_accum, &s_abort, 0u, a.out_box ? &tmap_y : nullptr, smem_base, &s_res, nf != nullptr);
+    } else if (warp == 4) {
+        // ===== operand A: this block's 128 rows =====
+        griddep_wait();
+        uint32_t* const err_flag = a.err_flag;
+        uint32_t st = 0, parity = 1u;
+        int tap_r = 0, tap_s = 0, chunk = 0;
+        for (int kb = 0; kb < nkb; ++kb) {
+            if (kb >= stages && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, &s_abort, err_flag, 1u))) break;
+            if (elect_one()) {
+                const uint32_t a_tile = smem_base + st * stage_bytes, bar = cluster_addr(smem_u32(&s_full[st]), 0u);
+                if (a.a_tiled) tma_load_2d_pair(a_tile, &tmap_x, chunk * kBK, m0, bar);
+                else tma_load_im2col_4d_pair(a_tile, &tmap_x, chunk * kBK, w0, h0, img, (uint16_t)(tap_s * a.dw), (uint16_t)(tap_r * a.dh), bar);
+            }
+            __syncwarp();
+            if (++chunk == cpt) {
+                chunk = 0;
+                if (++tap_s == a.S) { tap_s = 0; ++tap_r; }
+            }
+            if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
+        }
+        if (a.residual && a.out_box) {      // as in conv_tile_tma
+            const uint32_t bytes = (uint32_t)a.BN * 256u;
+            bool ok = true;
+            for (uint32_t q = 0; q * stage_bytes < bytes && ok; ++q) {
+                const int uses = q < (uint32_t)stages && nkb > (int)q ? (nkb - (int)q + stages - 1) / stages : 0;
+                if (uses > 0) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[q]), (uint32_t)(uses - 1) & 1u, &s_abort, err_flag, 1u));
+            }
+            if (ok && elect_one()) {
+                mbar_arrive_expect_tx(smem_u32(&s_res), bytes);
+                for (int c = 0; c < a.BN; c += a.out_box) tma_load_2d(smem_base + (uint32_t)c * 256u, &tmap_r, n0 + c, m0, smem_u32(&s_res));
+            }
+            __syncwarp();
+        }
+        griddep_launch();
+    } else if (rank == 0) {
+        // ===== the pair's multiplications =====
+        uint32_t st = 0, parity = 0u;
+        bool ok = true;
+        uint32_t* const err_flag = a.err_flag;
+        const uint32_t idesc = uniform(a.idesc), n_kb = uniform((uint32_t)nkb), n_st = uniform((uint32_t)stages);
+        const uint64_t desc_a0 = umma_desc_sw128(uniform(smem_base)), desc_b0 = umma_desc_sw128(uniform(smem_base) + kATileBytes);
+        const uint32_t desc_step = uniform(stage_bytes) >> 4;
+        for (uint32_t kb = 0; kb < n_kb; ++kb) {
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err_flag, 2u));
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint64_t da = desc_a0 + st * desc_step, db = desc_b0 + st * desc_step;
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < kBK / 16; ++k)
+                    tcgen05_mma_bf16_pair(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                tcgen05_commit_pair(smem_u32(&s_empty[st]));
+            }
+            __syncwarp();
+            if (++st == n_st) { st = 0; parity ^= 1u; }
+        }
+        if (ok && elect_one()) tcgen05_commit_pair(smem_u32(&s_accum));
+        __syncwarp();
+        griddep_launch();
+    } else {
+        griddep_launch();
+    }
+
+    tcgen05_fence_before();
+    __syncthreads();
+    if (s_abort) {
+        const unsigned long long t0 = globaltimer_ns();
+        for (uint32_t i = 0; i < (1u << 20); ++i) {
+            if (globaltimer_ns() - t0 > 50000ull) break;
+        }
+    }
+    cluster_arrive();
+    cluster_wait();                     // neither block's memory goes before both have finished
+    if (warp == 5) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(a.tmem_cols) : "memory");
+    }
+    if (nf) nf->end(job_id);
+}
+
 // Grouped launch: several independent convolutions (the parallel branches of an Inception block at the
 // same depth, a ResNet block's shortcut beside its first convolution) in ONE grid.  Kernel-level
 // concurrency on a GPU is capped by its hardware queues, and a batch-1 convolution rarely has more
@@ -1710,6 +1904,7 @@ struct Geometry {
     int m_tiles;
     int stages;                 // pipeline buffers
     int splits;                 // blocks (one cluster) per tile
+    bool pair;                  // two blocks on a tile of 256 rows
     int out_box;                // ConvArgs::out_box
     uint32_t tmem_cols, b_stage_bytes, smem_bytes, idesc;
 };
@@ -1824,14 +2019,36 @@ ConvTiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double
 ConvShape conv_shape(const pb_op_params* p, bool shared) {
     return {ceil_div(batch_of(p) * p->P * p->Q, kBM), round_up(p->K, 16), p->R * p->S * ceil_div(p->Cs, kBK), p->residual != nullptr, shared};
 }
+// When a launch runs on pairs of blocks: wide tiles (the weights are what is shared), a k-loop long enough to carry the pair's
+// set-up, and tiles that fill the 74 pairs of SMs evenly - one each, or (nearly) two and more, which share a pair of SMs and are
+// replaced as they finish.  Measured, lone blocks / pairs, us: 288 -> 384 3x3 35 x 35 x 64 images (614 pairs, 192 columns) 142 / 131, the
+// same with stride 2 (146) 32.6 / 31.4, 256 -> 256 3x3 56 x 56 x 16 (196) 56.4 / 48.0, 1024 -> 256 1x1 56 x 56 x 16 (196, 16 k-blocks)
+// 41.6 / 39.5, 1024 -> 1024 3x3 14 x 14 x 16 (52) 64.2 / 52.1, 256 -> 256 3x3 28 x 28 x 16 with a residual (49) 25.2 / 21.2; and outside:
+// 512 -> 512 3x3 28 x 28 x 16 (98 pairs) 46.4 / 52.9, 128 columns 62.5 / 69.7, 96 columns 28.6 / 37.4, 4 k-blocks 52.7 / 56.5.
+// Not on a GPU that other requests share, where three lone blocks an SM do better.
+// PB_CONV_PAIR (read at every use; for tests and comparisons): 0 = no pairs, 1 = pairs wherever their kernel can run.
+ConvTiling pair_tiling(const ConvShape& c) {
+    ConvTiling none{0, 1, false, c.shared};
+    const char* e = getenv("PB_CONV_PAIR");
+    const int force = e && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : -1;
+    if (force == 0 || !use_tma_a() || persist_enabled() || bn_limit() < 256) return none;
+    const int n = ceil_div(c.Kp16, 256), BN = round_up(ceil_div(c.Kp16, n), 32);
+    const int pairs = ceil_div(c.m_tiles, 2) * n;
+    if (force < 0 && (c.shared || BN < 192 || c.nkb < 16 || pairs < 48 || (pairs > 74 && pairs < 140))) return none;
+    return {BN, 1, true, c.shared, true};
+}
 bool splits_off() { return !use_tma_a() || conv_split_gain_us() > 1e6; }
 // want_splits: the cluster size (0: the fastest).
-ConvTiling tiling_for(const pb_op_params* p, bool shared, int want_splits) {
+ConvTiling tiling_for(const pb_op_params* p, bool shared, int want_splits, bool may_pair = false) {
+    if (may_pair) {
+        const ConvTiling t = pair_tiling(conv_shape(p, shared));
+        if (t.BN) return t;
+    }
     return choose_tiling(conv_shape(p, shared), bn_limit(), splits_off() ? 1 : want_splits, conv_split_gain_us());
 }
 // The split is the caller's to allow: by the scratch memory that pb_launch_info.scratch_bytes asks for.
 bool split_allowed(const pb_op_params* p) { return p->scratch != nullptr && p->scratch_bytes >= kSplitScratchBytes; }
-ConvTiling tiling_or(const ConvTiling* given, const pb_op_params* p) { return given ? *given : tiling_for(p, false, split_allowed(p) ? 0 : 1); }
+ConvTiling tiling_or(const ConvTiling* given, const pb_op_params* p) { return given ? *given : tiling_for(p, false, split_allowed(p) ? 0 : 1, true); }
 
 Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     Geometry g;
@@ -1841,15 +2058,18 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     g.Kdim_pad = g.nkb * kBK;
     g.Kp16 = round_up(p->K, 16);
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kBM);
+    g.pair = t.pair;
+    if (g.pair) g.m_tiles = round_up(g.m_tiles, 2);
     g.BN = t.BN;
     g.splits = t.splits;
     g.n_tiles = ceil_div(g.Kp16, g.BN);
     g.tmem_cols = 32;
     while ((int)g.tmem_cols < g.BN) g.tmem_cols <<= 1;
-    g.b_stage_bytes = (uint32_t)g.BN * 128u;
+    g.b_stage_bytes = (uint32_t)(g.pair ? g.BN / 2 : g.BN) * 128u;
     const uint32_t stage_bytes = (uint32_t)kATileBytes + g.b_stage_bytes;
     if (use_tma_a()) {
-        g.stages = pipeline_stages(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), t.shared);
+        g.stages = g.pair ? std::min(kMaxStages, (int)((kSmemBudgetDeep - 1024u) / stage_bytes))
+                          : pipeline_stages(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), t.shared);
     } else {
         static const int kDepths[] = {8, 6, 4};                     // the gather kernel exists for 4, 6, 8
         g.stages = 4;
@@ -1860,11 +2080,12 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     const uint32_t exchange = g.splits > 1 ? (uint32_t)g.BN * 512u : 0u;      // a rank's partial tile
     g.smem_bytes = std::max((uint32_t)g.stages * stage_bytes, exchange) + 1024u;
     // c_format f32 (1 << 4), a/b format bf16 (1 << 7, 1 << 10), K-major both, N >> 3 at bit 17, M >> 4 at bit 24
-    g.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+    g.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)((g.pair ? 2 * kBM : kBM) >> 4) << 24);
     return g;
 }
 
-const void* kernel_for(int stages, bool tma) {
+const void* kernel_for(int stages, bool tma, bool pair = false) {
+    if (pair) return (const void*)conv_umma_pair_kernel;
     if (tma) return (const void*)conv_umma_tma_kernel<false>;
     switch (stages) {
         case 4: return (const void*)conv_umma_gather_kernel<4>;
@@ -1875,7 +2096,7 @@ const void* kernel_for(int stages, bool tma) {
 
 // Raises the dynamic shared-memory limit of every kernel of this file on the current device.
 cudaError_t raise_smem_limits() {
-    const void* kernels[] = {(const void*)conv_umma_tma_kernel<false>, (const void*)conv_umma_tma_kernel<true>, (const void*)conv_umma_multi_kernel, (const void*)conv_umma_persist_kernel,
+    const void* kernels[] = {(const void*)conv_umma_pair_kernel, (const void*)conv_umma_tma_kernel<false>, (const void*)conv_umma_tma_kernel<true>, (const void*)conv_umma_multi_kernel, (const void*)conv_umma_persist_kernel,
                              (const void*)conv_umma_gather_kernel<4>, (const void*)conv_umma_gather_kernel<6>,
                              (const void*)conv_umma_gather_kernel<8>};
     for (const void* k : kernels) {
@@ -1934,7 +2155,7 @@ bool conv_umma_supported(const pb_op_params* p) {
            !(p->flags & 2);
 }
 
-ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split) { return tiling_for(p, shared, may_split ? 0 : 1); }
+ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split, bool may_pair) { return tiling_for(p, shared, may_split ? 0 : 1, may_pair); }
 
 double conv_umma_us(const pb_op_params* p, const ConvTiling& t) {
     const ConvShape c = conv_shape(p, t.shared);
@@ -1952,7 +2173,7 @@ int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling*
     out->threads_per_block = use_tma_a() ? kThreadsTma : kThreads;
     cudaFuncAttributes at;
     uint32_t regs = 64, sstatic = 128;
-    if (cudaFuncGetAttributes(&at, kernel_for(g.stages, use_tma_a())) == cudaSuccess) {
+    if (cudaFuncGetAttributes(&at, kernel_for(g.stages, use_tma_a(), g.pair)) == cudaSuccess) {
         regs = (uint32_t)at.numRegs;
         sstatic = (uint32_t)at.sharedSizeBytes;
     } else {
@@ -1986,6 +2207,7 @@ int64_t conv_umma_pack_weights(const pb_op_params* p, const float* w, void* dst)
 }
 
 // Weight map of a launch with tiles of BN output channels.
+// (BN: rows of a box, half a tile's columns for a pair of blocks)
 static int make_tmap(const ConvUmmaPlan* plan, int BN, CUtensorMap* out) {
     const void* w_dev = plan->w_dev;
     EncodeTiledFn enc = encode_fn();
@@ -2212,11 +2434,12 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
             xmap = &local;
         }
         CUtensorMap wmap, ymap, rmap;
-        int mrc = make_tmap(plan, g.BN, &wmap);
+        int mrc = make_tmap(plan, g.pair ? g.BN / 2 : g.BN, &wmap);
         if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, false, &ymap);
         if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, true, &rmap);
         if (mrc != PB_OK) return mrc;
-        const cudaError_t e = launch_pdl(pre ? conv_umma_tma_kernel<true> : conv_umma_tma_kernel<false>, grid, dim3(1, 1, (unsigned)g.splits), smem, st, pdl, wmap, xmap->map, ymap, rmap, a,
+        const dim3 cluster = g.pair ? dim3(2, 1, 1) : dim3(1, 1, (unsigned)g.splits);
+        const cudaError_t e = launch_pdl(g.pair ? conv_umma_pair_kernel : pre ? conv_umma_tma_kernel<true> : conv_umma_tma_kernel<false>, grid, cluster, smem, st, pdl, wmap, xmap->map, ymap, rmap, a,
                                          g.stages, job_id, nf);
         if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_tma_kernel", __FILE__, __LINE__);
         return PB_OK;

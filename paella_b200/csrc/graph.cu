@@ -160,6 +160,15 @@ bool uses_multi(const pb_model* m, const std::vector<int>& l) {
     return m->persist && m->stages[(size_t)l[0]].kind == PB_STAGE_CONV_UMMA;
 }
 
+// Has the convolution a launch to itself wherever it runs in the stage graphs (no riders, no affine of its own)?
+bool launched_alone(const pb_model* m, int stage) {
+    for (const pb_model::Group& g : m->groups)
+        for (size_t li = 0; li < g.launches.size(); ++li)
+            for (int s : g.launches[li])
+                if (s == stage && (g.launches[li].size() > 1 || g.pre[li] >= 0)) return false;
+    return true;
+}
+
 // How the tensor-core convolutions of the model are cut for `nb` images, by stage: as members of the grouped launches they share
 // by default.  A search takes microseconds per convolution and cluster size, and every instance, stage declaration and gang size
 // asks, so the model keeps the last answer per batch size.
@@ -181,7 +190,7 @@ std::shared_ptr<const std::vector<pb::ConvTiling>> tilings_for(const pb_model* m
         }
         for (const pb_op_params& p : ps) pp.push_back(&p);
         std::vector<pb::ConvTiling> t(l.size());
-        if (l.size() == 1) t[0] = pb::conv_umma_tiling(pp[0], m->shared, may_split);
+        if (l.size() == 1) t[0] = pb::conv_umma_tiling(pp[0], m->shared, may_split, may_split && launched_alone(m, (int)i));
         else pb::conv_umma_group_tilings(pp.data(), (int)l.size(), m->shared, may_split, t.data());
         for (size_t k = 0; k < l.size(); ++k) (*by_stage)[(size_t)l[k]] = t[k];
     }

@@ -53,8 +53,10 @@ struct ConvTiling {
     int BN, splits;        // output channels of a tile, blocks (one cluster) that share its reduction
     bool tma;              // the tile leaves (and the residual arrives) through TMA
     bool shared;           // other requests' launches run beside it
+    bool pair = false;     // two blocks (a cluster) on a tile of 256 rows
 };
-ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split);
+// may_pair: the launch is conv_umma_launch_planned's, without an input affine.
+ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split, bool may_pair);
 // Tilings of the convolutions of one grouped launch: they share a cluster size.
 void conv_umma_group_tilings(const pb_op_params* const* params, int n, bool shared, bool may_split, ConvTiling* out);
 double conv_umma_us(const pb_op_params* p, const ConvTiling& tiling);      // modelled microseconds of a lone launch

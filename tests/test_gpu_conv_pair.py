@@ -1,0 +1,74 @@
+"""Tiles of 256 rows on a pair of blocks, at the sizes where they can go wrong: fewer rows than one block's, rows that end in the first or
+the second block, one k-block, more k-blocks than stages, ragged output channels, strides, images that straddle a tile, slices
+and residuals, stores through TMA and direct.
+
+Reference: the convolution of the bf16 operands in 64 bits.  Products of bf16 values are exact in fp32; n = C*R*S of them summed
+in fp32 in any order differ from the exact sum by at most n * 2^-23 * sum |products| (every addition truncating, in the worst
+order); one rounding to bf16 (2^-8 relative) follows."""
+import ctypes as C
+
+import pytest
+
+from paella_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # C, H, W, K, R, S, stride, pad_h, pad_w, images, act, residual, slice offset, out channels
+    (8, 3, 3, 8, 1, 1, 1, 0, 0, 1, 0, False, 0, 8),               # nine rows: the second block has none; one k-block
+    (64, 16, 8, 32, 1, 1, 1, 0, 0, 1, 1, True, 0, 32),            # exactly the first block's rows
+    (64, 43, 3, 96, 1, 1, 1, 0, 0, 1, 1, False, 0, 96),           # one row in the second block
+    (64, 16, 16, 64, 3, 3, 1, 1, 1, 1, 2, True, 0, 64),           # exactly one pair
+    (72, 257, 1, 40, 1, 1, 1, 0, 0, 1, 1, False, 24, 80),         # one row of a second pair; 40 of 64 columns; a slice
+    (288, 35, 35, 384, 3, 3, 1, 1, 1, 2, 1, False, 0, 384),       # two tiles of 192 columns, 45 k-blocks
+    (128, 17, 17, 200, 1, 7, 1, 0, 3, 3, 1, True, 0, 200),        # 224 columns, 200 of them real
+    (96, 31, 29, 256, 3, 3, 2, 0, 0, 5, 1, False, 0, 256),        # stride 2, images straddle tiles
+    (64, 14, 14, 512, 1, 1, 1, 0, 0, 4, 3, False, 0, 512),        # PReLU
+]
+
+
+@pytest.mark.parametrize("mode", ["0", "1"])
+@pytest.mark.parametrize("case", CASES)
+def test_pairs_of_blocks(case, mode, monkeypatch):
+    import torch
+    L = capi.load()
+    monkeypatch.setenv("PB_CONV_PAIR", mode)
+    c, h, w, k, r, s, stride, ph, pw, n, act, residual, off, total = case
+    P, Q = (h + 2 * ph - r) // stride + 1, (w + 2 * pw - s) // stride + 1
+    gen = torch.Generator(device="cuda").manual_seed(c * 131 + h)
+    cs = (c + 7) // 8 * 8
+    x = torch.relu(torch.randn((n, h, w, cs), generator=gen, device="cuda")).to(torch.bfloat16)
+    wt = (torch.randn((k, c, r, s), generator=gen, device="cuda") * (2.0 / (c * r * s)) ** 0.5).to(torch.bfloat16)
+    bias = torch.randn(2 * k, generator=gen, device="cuda") * 0.1          # PReLU: the slopes follow
+    res = torch.randn((n, P, Q, k), generator=gen, device="cuda").to(torch.bfloat16)
+    y = torch.full((n, P, Q, total), 7.0, device="cuda", dtype=torch.bfloat16)
+    p = capi.OpParams()
+    p.dtype, p.C, p.H, p.W, p.Cs, p.K, p.P, p.Q, p.Ks, p.out_c_off = 1, c, h, w, cs, k, P, Q, total, off
+    p.R, p.S, p.stride_h, p.stride_w, p.pad_h, p.pad_w, p.groups, p.act, p.batch, p.dil_h, p.dil_w = r, s, stride, stride, ph, pw, 1, act, n, 1, 1
+    host = wt.float().cpu().contiguous()
+    size = L.pb_op_pack_weights(capi.STAGE_CONV_UMMA, C.byref(p), host.data_ptr(), None)
+    packed = torch.zeros(size, dtype=torch.uint8)
+    L.pb_op_pack_weights(capi.STAGE_CONV_UMMA, C.byref(p), host.data_ptr(), packed.data_ptr())
+    packed = packed.cuda()
+    p.x, p.w, p.bias, p.y = x.data_ptr(), packed.data_ptr(), bias.data_ptr(), y.data_ptr()
+    if residual:
+        p.residual, p.res_Cs = res.data_ptr(), k
+    xd, wd = x[..., :c].permute(0, 3, 1, 2).double().cpu(), wt.double().cpu()
+    conv = lambda a, b: torch.nn.functional.conv2d(a, b, padding=(ph, pw), stride=stride).permute(0, 2, 3, 1)
+    want = conv(xd, wd) + bias[:k].double().cpu()
+    if residual:
+        want = want + res.double().cpu()
+    want = torch.relu(want) if act in (1, 2) else want
+    want = torch.where(want > 0, want, want * bias[k:].double().cpu()) if act == 3 else want
+    want = want.clamp(max=6.0) if act == 2 else want
+    bound = c * r * s * 2.0 ** -23 * conv(xd.abs(), wd.abs()) + 2.0 ** -8 * want.abs() + 1e-6
+    capi.check(L.pb_op_launch(capi.STAGE_CONV_UMMA, C.byref(p), None, 0, None), "pb_op_launch")
+    torch.cuda.synchronize()
+    flag = C.c_uint32(0)
+    capi.check(L.pb_device_error_flag(0, C.byref(flag), 1), "pb_device_error_flag")
+    assert flag.value == 0
+    got = y[..., off:off + k].double().cpu()
+    assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
+    untouched = torch.ones(total, dtype=torch.bool)
+    untouched[off:off + k] = False
+    assert bool((y[..., untouched.cuda()] == 7.0).all())

@@ -17,7 +17,8 @@
 // operand B; warp 4 loads operand A, warp 5 allocates TMEM and issues the MMAs.  Sized for three CTAs per SM.
 // Two entry points share the body (conv_tile_tma): conv_umma_tma_kernel runs one convolution,
 // conv_umma_multi_kernel runs several independent ones as one grid from a descriptor table in
-// device memory.  conv_umma_gather_kernel (PB_CONV_GATHER=1) is the earlier design, kept for
+// device memory; conv_umma_tma_kernel<true> also normalises its input tiles.  conv_umma_pair_kernel puts two blocks (cta_group::2)
+// on a tile of 256 rows where a lone launch is large.  conv_umma_gather_kernel (PB_CONV_GATHER=1) is the earlier design, kept for
 // comparison: 128 producer threads gather A with 16-byte cp.async copies (a lone Inception-v3 request
 // takes 1656 us with it, 342 without).
 //

@@ -17,7 +17,7 @@
 // operand B; warp 4 loads operand A, warp 5 allocates TMEM and issues the MMAs.  Sized for three CTAs per SM.
 // Two entry points share the body (conv_tile_tma): conv_umma_tma_kernel runs one convolution,
 // conv_umma_multi_kernel runs several independent ones as one grid from a descriptor table in
-// device memory; conv_umma_tma_kernel<true> also normalises its input tiles.  conv_umma_pair_kernel puts two blocks (cta_group::2)
+// device memory; conv_umma_pre_kernel also normalises its input tiles.  conv_umma_pair_kernel puts two blocks (cta_group::2)
 // on a tile of 256 rows where a lone launch is large.  conv_umma_gather_kernel (PB_CONV_GATHER=1) is the earlier design, kept for
 // comparison: 128 producer threads gather A with 16-byte cp.async copies (a lone Inception-v3 request
 // takes 1656 us with it, 342 without).
@@ -833,6 +833,10 @@ constexpr int kWarpB = 3;          // issues operand B's copies
 // stage: 0.37; three warps: 0.48; constants read from global memory per k-block: 1.0, slower than the launch it replaces).
 // The arithmetic is affine_kernel's - fp32 multiply-add, ReLU, one rounding to bf16 - and so are the bits (the maximum with
 // zero may follow the rounding: rounding is monotonic and keeps zeros; NaN gives zero either way).
+// The normalised tiles also go to the affine's own tensor, where whoever launches or reads single stages afterwards looks for them:
+// operand A's warp stores a stage through TMA before it loads the next tile there, and the blocks of a row tile, which normalise the same
+// k-blocks, take turns at that.  (DenseNet-121 of three images: 622 us without these stores, 637 with them, 670 when the normalising
+// threads store.)
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z) {
     uint64_t r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
@@ -907,7 +911,7 @@ __device__ __forceinline__ void normalise_stages(const ConvArgs& a, uint32_t sme
 // kPre: the tile's input is normalised first (see above; a kernel of its own: the others' code and registers stay as they are).
 template <bool kPre>
 __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const CUtensorMap* tmap_y, const CUtensorMap* tmap_r,
-                                              const ConvArgs& a, const int stages,
+                                              const CUtensorMap* tmap_n, const ConvArgs& a, const int stages,
                                               const int bx, const int by, const int bz, uint8_t* smem_raw,
                                               uint64_t* s_full, uint64_t* s_empty, uint64_t* s_accum, uint32_t* s_tmem_base,
                                               volatile uint32_t* s_abort, float* s_bias, uint64_t* s_res, uint64_t* s_ready, bool publish) {
@@ -949,7 +953,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
                 mbar_init(smem_u32(&s_empty[s]), 1);     // tcgen05.commit
                 if (kPre) mbar_init(smem_u32(&s_ready[s]), 2);     // normalised: one arrival of each of two warps
             }
-            mbar_init(smem_u32(s_accum), 1);
+            mbar_init(smem_u32(s_accum), kPre ? 2 : 1);                // normalised: its memory is free, too
             mbar_init(smem_u32(s_res), 1);
             *s_abort = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1040,9 +1044,22 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         }
         griddep_wait();                           // the activations are the previous kernel's
         const int S = a.S, dw = a.dw, dh = a.dh, a_tiled = a.a_tiled;
+        // The normalised k-block kb, in stage st, to its tensor (by one lane: it waits for its own stores).
+        auto store_normalised = [&](int kb, uint32_t st, uint32_t parity) {
+            if ((unsigned)(kb_begin + kb) % gridDim.y != (unsigned)by) return true;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_ready[st]), parity, s_abort, err_flag, 8u))) return false;
+            if (lane == 0) tma_store_2d(tmap_n, (kb_begin + kb) * kBK, m0, smem_base + st * stage_bytes);
+            __syncwarp();
+            return true;
+        };
         uint32_t st = 0, parity = 1u;             // a fresh barrier passes a wait on the "previous" phase
         for (int kb = 0; kb < nkb; ++kb) {
+            if (kPre && kb >= stages && !store_normalised(kb - stages, st, parity)) break;
             if (kb >= stages && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, s_abort, err_flag, 1u))) break;
+            if (kPre && kb >= stages) {
+                if (lane == 0) tma_store_wait_read();
+                __syncwarp();
+            }
             if (elect_one()) {
                 const uint32_t a_tile = smem_base + st * stage_bytes, bar = smem_u32(&s_full[st]);
                 if (kPre && kb >= stages) {
@@ -1061,6 +1078,25 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
             }
             if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
         }
+        if (kPre) {
+            // The epilogue may start once the stages whose memory it uses (for the partial or the finished tile) have been stored; the
+            // others leave beside it.
+            const uint32_t bytes = a.splits > 1 ? (uint32_t)a.BN * 512u : a.out_box ? (uint32_t)a.BN * 256u : 0u;
+            const int used = (int)((bytes + stage_bytes - 1) / stage_bytes), last_st = nkb > 0 ? (nkb - 1) % stages : 0;
+            const int until = used > 0 ? nkb - 1 - max(0, last_st - (used - 1)) : -1;        // the last k-block in one of them
+            auto let_epilogue = [&]() {
+                if (lane == 0) {
+                    tma_store_wait_read();
+                    mbar_arrive(smem_u32(s_accum));
+                }
+                __syncwarp();
+            };
+            if (until < 0) let_epilogue();
+            for (int kb = max(0, nkb - stages); kb < nkb; ++kb) {
+                if (!store_normalised(kb, (uint32_t)(kb % stages), (uint32_t)(kb / stages) & 1u)) break;
+                if (kb == until) let_epilogue();
+            }
+        }
         // The residual goes where the tile will be laid out, as soon as the multiplications have read the pipeline buffers there.
         if (a.residual && a.out_box) {
             const uint32_t bytes = (uint32_t)a.BN * 256u;
@@ -1077,6 +1113,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         }
         griddep_launch();
         if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
+        if (kPre && lane == 0) tma_store_wait_read();
     } else {
         // ===== MMA issuer =====
         // A wait on a complete barrier costs about 130 clocks and the tensor pipe holds few instructions, so it drains meanwhile:
@@ -1150,14 +1187,12 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 #endif
 }
 
-template <bool kPre>
 __global__ void __launch_bounds__(kThreadsTma, 3)
 conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                      const __grid_constant__ CUtensorMap tmap_y, const __grid_constant__ CUtensorMap tmap_r, const ConvArgs a, int stages, uint32_t job_id, FinishedBlockNotifier* nf) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxStages];
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
-    __shared__ __align__(8) uint64_t s_ready[kPre ? kMaxStages : 1];
     __shared__ __align__(8) uint64_t s_res;
     __shared__ __align__(8) uint64_t s_accum;
     __shared__ uint32_t s_tmem_base;
@@ -1167,8 +1202,31 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     resolve_slot(job_id, nf);
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
-    conv_tile_tma<kPre>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
-                  &s_tmem_base, &s_abort, s_bias, &s_res, s_ready, nf != nullptr);
+    conv_tile_tma<false>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, nullptr, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+                         &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
+    if (nf) nf->end(job_id);
+}
+
+// The same with the input normalised; tmap_n: the normalised input's own tensor.
+__global__ void __launch_bounds__(kThreadsTma, 3)
+conv_umma_pre_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
+                     const __grid_constant__ CUtensorMap tmap_r, const __grid_constant__ CUtensorMap tmap_n, const ConvArgs a, int stages, uint32_t job_id,
+                     FinishedBlockNotifier* nf) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t s_full[kMaxStages];
+    __shared__ __align__(8) uint64_t s_empty[kMaxStages];
+    __shared__ __align__(8) uint64_t s_ready[kMaxStages];
+    __shared__ __align__(8) uint64_t s_res;
+    __shared__ __align__(8) uint64_t s_accum;
+    __shared__ uint32_t s_tmem_base;
+    __shared__ volatile uint32_t s_abort;
+    __shared__ __align__(16) float s_bias[kMaxBN];
+
+    resolve_slot(job_id, nf);
+    if (nf) nf->start(job_id);
+    if (threadIdx.x == 0) PB_T(0);
+    conv_tile_tma<true>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, &tmap_n, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+                        &s_tmem_base, &s_abort, s_bias, &s_res, s_ready, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1514,7 +1572,7 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     const uint32_t S = (uint32_t)s_args.splits, gx = sc->gx;
     const uint32_t tile = local / S, bz = local - tile * S;
     const uint32_t by = tile / gx, bx = tile - by * gx;
-    conv_tile_tma<false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
+    conv_tile_tma<false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, nullptr, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
                   &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
     if (nf) nf->end(job_id);
 }
@@ -2087,7 +2145,7 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
 
 const void* kernel_for(int stages, bool tma, bool pair = false) {
     if (pair) return (const void*)conv_umma_pair_kernel;
-    if (tma) return (const void*)conv_umma_tma_kernel<false>;
+    if (tma) return (const void*)conv_umma_tma_kernel;
     switch (stages) {
         case 4: return (const void*)conv_umma_gather_kernel<4>;
         case 6: return (const void*)conv_umma_gather_kernel<6>;
@@ -2097,7 +2155,7 @@ const void* kernel_for(int stages, bool tma, bool pair = false) {
 
 // Raises the dynamic shared-memory limit of every kernel of this file on the current device.
 cudaError_t raise_smem_limits() {
-    const void* kernels[] = {(const void*)conv_umma_pair_kernel, (const void*)conv_umma_tma_kernel<false>, (const void*)conv_umma_tma_kernel<true>, (const void*)conv_umma_multi_kernel, (const void*)conv_umma_persist_kernel,
+    const void* kernels[] = {(const void*)conv_umma_pair_kernel, (const void*)conv_umma_tma_kernel, (const void*)conv_umma_pre_kernel, (const void*)conv_umma_multi_kernel, (const void*)conv_umma_persist_kernel,
                              (const void*)conv_umma_gather_kernel<4>, (const void*)conv_umma_gather_kernel<6>,
                              (const void*)conv_umma_gather_kernel<8>};
     for (const void* k : kernels) {
@@ -2276,37 +2334,49 @@ static int make_xmap(const pb_op_params* p, const ConvPre* pre, CUtensorMap* out
 }
 
 
-// Map of the output slice (boxes of 32 rows) or of the residual (boxes of 128 rows): [pixels of all images][channels].
-static int make_ymap(const pb_op_params* p, int U, bool residual, CUtensorMap* out) {
-    if (!U || (residual && !p->residual)) { memset(out, 0, sizeof(*out)); return PB_OK; }
-    const __nv_bfloat16* base = residual ? static_cast<const __nv_bfloat16*>(p->residual) : static_cast<const __nv_bfloat16*>(p->y) + p->out_c_off;
-    const int stride = residual ? p->res_Cs : p->Ks;
+// Map of [pixels of all images][channels] in boxes of U channels and so many rows.
+static int make_rows_map(const pb_op_params* p, const __nv_bfloat16* base, int channels, int stride, int U, uint32_t rows, CUtensorMap* out) {
     EncodeTiledFn enc = encode_fn();
     PB_REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
     PB_REQUIRE(((uintptr_t)base & 15) == 0, "conv_umma: output and residual must be 16-byte aligned");
-    const cuuint64_t dims[2] = {(cuuint64_t)p->K, (cuuint64_t)batch_of(p) * p->P * p->Q};
+    const cuuint64_t dims[2] = {(cuuint64_t)channels, (cuuint64_t)batch_of(p) * p->P * p->Q};
     const cuuint64_t strides[1] = {(cuuint64_t)stride * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)U, residual ? 128u : 32u};
+    const cuuint32_t box[2] = {(cuuint32_t)U, rows};
     const cuuint32_t estr[2] = {1, 1};
     const CUtensorMapSwizzle sw = U == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled (output) failed with CUresult %d (K %d, stride %d)", (int)r, p->K, p->Ks);
+        set_error("cuTensorMapEncodeTiled (output) failed with CUresult %d (%d channels, stride %d)", (int)r, channels, stride);
         return PB_ERR_CUDA;
     }
     return PB_OK;
 }
 
+// Map of the output slice (boxes of 32 rows) or of the residual (boxes of 128 rows).
+static int make_ymap(const pb_op_params* p, int U, bool residual, CUtensorMap* out) {
+    if (!U || (residual && !p->residual)) { memset(out, 0, sizeof(*out)); return PB_OK; }
+    if (residual) return make_rows_map(p, static_cast<const __nv_bfloat16*>(p->residual), p->K, p->res_Cs, U, 128u, out);
+    return make_rows_map(p, static_cast<const __nv_bfloat16*>(p->y) + p->out_c_off, p->K, p->Ks, U, 32u, out);
+}
+
 // The affine's channels are the layer's input channels, in whole vectors (x_Cs apart from pixel to pixel).
 bool conv_umma_pre_supported(const pb_op_params* p, const ConvPre& pre) {
-    return use_tma_a() && pointwise(p) && p->C == p->Cs && p->C % 8 == 0 && pre.x_Cs % 8 == 0 && (pre.act == 0 || pre.act == 1) &&
+    return use_tma_a() && pointwise(p) && p->C == p->Cs && p->C % 8 == 0 && pre.x_Cs % 8 == 0 && pre.y_Cs % 8 == 0 && (pre.act == 0 || pre.act == 1) &&
            (((uintptr_t)pre.scale | (uintptr_t)pre.bias) & 15) == 0;
 }
 
 struct alignas(64) ConvUmmaXMap {
     CUtensorMap map;
+    CUtensorMap normalised;      // of a launch with an input affine: the affine's tensor, in tiles of operand A
 };
+
+// Descriptors of a launch's input.
+static int make_input_maps(const pb_op_params* p, const ConvPre* pre, ConvUmmaXMap* m) {
+    const int rc = make_xmap(p, pre, &m->map);
+    if (rc != PB_OK || !pre) return rc;
+    return make_rows_map(p, static_cast<const __nv_bfloat16*>(pre->y), p->C, pre->y_Cs, kBK, (uint32_t)kBM, &m->normalised);
+}
 
 int encode_tiled_bf16(const void* base, int rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box, bool nan_fill, CUtensorMap* out) {
     EncodeTiledFn enc = encode_fn();
@@ -2333,7 +2403,7 @@ int encode_tiled_bf16(const void* base, int rank, const uint64_t* dims, const ui
 int conv_umma_xmap_create(const pb_op_params* p, ConvUmmaXMap** out, const ConvPre* pre) {
     if (!use_tma_a()) { *out = nullptr; return PB_OK; }
     ConvUmmaXMap* m = new ConvUmmaXMap();
-    const int rc = make_xmap(p, pre, &m->map);
+    const int rc = make_input_maps(p, pre, m);
     if (rc != PB_OK) { delete m; return rc; }
     *out = m;
     return PB_OK;
@@ -2430,7 +2500,7 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
     if (use_tma_a()) {
         ConvUmmaXMap local;
         if (!xmap) {
-            const int rc = make_xmap(p, pre, &local.map);
+            const int rc = make_input_maps(p, pre, &local);
             if (rc != PB_OK) return rc;
             xmap = &local;
         }
@@ -2440,9 +2510,11 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
         if (mrc == PB_OK) mrc = make_ymap(p, g.out_box, true, &rmap);
         if (mrc != PB_OK) return mrc;
         const dim3 cluster = g.pair ? dim3(2, 1, 1) : dim3(1, 1, (unsigned)g.splits);
-        const cudaError_t e = launch_pdl(g.pair ? conv_umma_pair_kernel : pre ? conv_umma_tma_kernel<true> : conv_umma_tma_kernel<false>, grid, cluster, smem, st, pdl, wmap, xmap->map, ymap, rmap, a,
-                                         g.stages, job_id, nf);
-        if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_tma_kernel", __FILE__, __LINE__);
+        const cudaError_t e =
+            pre ? launch_pdl(conv_umma_pre_kernel, grid, cluster, smem, st, pdl, wmap, xmap->map, ymap, rmap, xmap->normalised, a, g.stages, job_id, nf)
+                : launch_pdl(g.pair ? conv_umma_pair_kernel : conv_umma_tma_kernel, grid, cluster, smem, st, pdl, wmap, xmap->map, ymap, rmap, a, g.stages, job_id, nf);
+        if (e != cudaSuccess)
+            return cuda_fail(e, pre ? "launch of conv_umma_pre_kernel" : g.pair ? "launch of conv_umma_pair_kernel" : "launch of conv_umma_tma_kernel", __FILE__, __LINE__);
         return PB_OK;
     } else {
         CUtensorMap wmap;

@@ -363,14 +363,18 @@ std::vector<pb_model::Group> plan_groups(const pb_model* m, int gs, bool fuse, b
     return groups;
 }
 
-// What convolution stage `conv` needs of affine stage `pre` to apply it itself; x is the affine's input.
-pb::ConvPre conv_pre(const Stage& pre, const void* x) {
-    return {x, pre.p.Cs, static_cast<const float*>(pre.p.w), pre.p.bias, pre.p.act};
+// What a convolution needs of affine stage `pre` to apply it itself; x and y are the affine's.
+pb::ConvPre conv_pre(const Stage& pre, const void* x, void* y) {
+    return {x, y, pre.p.Cs, pre.p.Ks, static_cast<const float*>(pre.p.w), pre.p.bias, pre.p.act};
+}
+pb::ConvPre conv_pre(const pb_model* m, const Variant& v, int pre) {
+    const pb_op_params& p = v.params[(size_t)pre];
+    return conv_pre(m->stages[(size_t)pre], p.x, p.y);
 }
 
 // An affine layer whose only reader is the pointwise tensor-core convolution right behind it in the chain has no launch: the
-// convolution normalises its tiles itself (same bits).  DenseNet-121 has 58 such pairs, each saving a launch of 2.5 us and its
-// hand-over; three images: 721 -> 632 us.
+// convolution normalises its tiles itself and stores them to the affine's tensor on the way (same bits).  DenseNet-121 has 58 such pairs, each saving a launch of 2.5 us and its
+// hand-over; three images: 721 -> 637 us.
 void fuse_affines(const pb_model* m, pb_model::Group& g) {
     std::vector<int> readers(m->tensors.size(), 0), writers(m->tensors.size(), 0);
     for (const Stage& st : m->stages) {
@@ -385,7 +389,7 @@ void fuse_affines(const pb_model* m, pb_model::Group& g) {
         const Stage &sa = m->stages[(size_t)a], &sc = m->stages[(size_t)c];
         if (sa.kind != PB_STAGE_AFFINE || sc.kind != PB_STAGE_CONV_UMMA || sc.in_tensor != sa.out_tensor || sc.res_tensor == sa.out_tensor || sa.x_is_input ||
             readers[(size_t)sa.out_tensor] != 1 || writers[(size_t)sa.out_tensor] != 1 || sa.p.out_c_off != 0 || sa.p.C != sc.p.C || sc.y_is_output ||
-            sa.in_tensor == sc.out_tensor || !pb::conv_umma_pre_supported(&sc.p, conv_pre(sa, nullptr)))
+            sa.in_tensor == sc.out_tensor || !pb::conv_umma_pre_supported(&sc.p, conv_pre(sa, nullptr, nullptr)))
             continue;
         g.launches.erase(g.launches.begin() + (long)li);
         g.pre.erase(g.pre.begin() + (long)li);
@@ -430,7 +434,7 @@ int launch_stage_with(pb_instance* in, const Variant& v, int stage, const pb_op_
         }
         case PB_STAGE_CONV_UMMA:
             if (pre >= 0) {
-                const pb::ConvPre cp = conv_pre(in->m->stages[(size_t)pre], v.params[(size_t)pre].x);
+                const pb::ConvPre cp = conv_pre(in->m, v, pre);
                 return pb::conv_umma_launch_planned(st.plan, v.pre_xmaps[stage], p, stream, job_id, notifier, nullptr, pdl, &v.tilings[stage], &cp);
             }
             return pb::conv_umma_launch_planned(st.plan, v.xmaps[stage], p, stream, job_id, notifier, nullptr, pdl, &v.tilings[stage]);
@@ -653,7 +657,7 @@ int ensure_variant(pb_instance* in, int nb, Variant** out) {
         for (size_t li = 0; li < g.launches.size(); ++li) {
             if (g.pre[li] < 0) continue;
             const int c = g.launches[li][0];
-            const pb::ConvPre cp = conv_pre(m->stages[(size_t)g.pre[li]], v->params[(size_t)g.pre[li]].x);
+            const pb::ConvPre cp = conv_pre(m, *v, g.pre[li]);
             const int rc = pb::conv_umma_xmap_create(&v->params[(size_t)c], &v->pre_xmaps[(size_t)c], &cp);
             if (rc != PB_OK) { destroy_variant(v); return rc; }
         }
@@ -1277,18 +1281,6 @@ int pb_instance_read_tensor(pb_instance* in, int tensor, float* dst, size_t dst_
         return PB_OK;
     }
     if (m->mnist_fused) { pb::set_error("intermediate tensors do not exist in the fused MNIST kernel"); return PB_ERR_INVALID; }
-    // the stage graphs do not write the tensor of an affine that its convolution applies itself: it is computed now, from its
-    // input, which is still there (every tensor has memory of its own)
-    for (const pb_model::Group& g : m->groups)
-        for (int a : g.pre) {
-            if (a < 0 || m->stages[(size_t)a].out_tensor != tensor) continue;
-            Variant* v = nullptr;
-            const int rc = ensure_variant(in, 1, &v);
-            if (rc != PB_OK) return rc;
-            const int lrc = launch_stage_with(in, *v, a, &v->params[(size_t)a], nullptr, 0, nullptr, nullptr, nullptr);
-            if (lrc != PB_OK) return lrc;
-            PB_CUDA(cudaDeviceSynchronize());
-        }
     const size_t es = m->dtype == 0 ? 4 : 2;
     std::vector<uint8_t> raw((size_t)t.H * t.W * t.Cs * es);
     PB_CUDA(cudaMemcpy(raw.data(), in->arena + (size_t)in->cap * t.offset, raw.size(), cudaMemcpyDeviceToHost));   // image 0

@@ -70,10 +70,12 @@ int conv_umma_plan_create(const pb_op_params* p, const void* w_dev, ConvUmmaPlan
 void conv_umma_plan_destroy(ConvUmmaPlan* plan);
 // Per-instance state: the im2col TMA descriptor of one layer's INPUT tensor (`p->x`).
 struct ConvUmmaXMap;
-// An affine (+ ReLU) in front of a pointwise convolution: it reads act(x * scale + bias), per channel, where p->x would have been.
+// An affine (+ ReLU) in front of a pointwise convolution, which applies it itself: it reads x and leaves act(x * scale + bias), per
+// channel, in y (p->x, the tensor it would have read).
 struct ConvPre {
     const void* x;
-    int x_Cs;                  // channel stride of x
+    void* y;
+    int x_Cs, y_Cs;            // channel strides
     const float* scale;
     const float* bias;
     int act;                   // 0 or 1

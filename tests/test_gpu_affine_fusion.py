@@ -65,6 +65,43 @@ def test_affine_in_the_convolution_has_the_bits_of_two_launches(tmp_path, monkey
     assert launches["1"] == launches["0"] - 1
 
 
+@pytest.mark.parametrize("case", CASES)
+def test_single_stages_after_the_groups_see_the_affine(tmp_path, monkeypatch, case):
+    """The affine's tensor is this request's after the stage groups ran, for a single stage launched from it: by stage, and as an
+    operator with the stage's parameters for a batch."""
+    import torch
+    monkeypatch.setenv("PB_FUSE_AFFINE", "1")
+    g, _ = _graph(case)
+    m = Model(g.save(str(tmp_path / "affine.bin")), 1)
+    names = [m.L.pb_model_stage_name(m.m, s).decode() for s in range(m.L.pb_model_num_stages(m.m))]
+    conv = names.index("conv")
+    t = next(o.out for o in g.ops if o.name == "conv")
+    xs = np.random.default_rng(1).standard_normal((3, 16) + case[3], dtype=np.float32)
+    m.run(xs[0])                                            # another request was there before
+    m.run_groups(xs[1])
+    want = m.tensor(t, g.tensors[t])
+    capi.check(m.L.pb_instance_launch_stage(m.i, conv, None, 0, None), "pb_instance_launch_stage")
+    np.testing.assert_array_equal(m.tensor(t, g.tensors[t]), want)
+
+    inst, out = C.c_void_p(), np.zeros((3, 10), np.float32)
+    capi.check(m.L.pb_instance_create_batched(m.m, 3, 0, C.byref(inst)), "pb_instance_create_batched")
+    p, got = capi.OpParams(), {}
+    for by_groups in (0, 1):
+        first = np.ascontiguousarray(xs[::-1]) if by_groups else xs
+        capi.check(m.L.pb_instance_run_batch_sync(inst, 3, 0, first.ctypes.data, out.ctypes.data), "run batch")
+        if by_groups:
+            capi.check(m.L.pb_instance_run_batch_sync(inst, 3, 1, xs.ctypes.data, out.ctypes.data), "run batch")
+        capi.check(m.L.pb_instance_stage_params(inst, conv, 3, C.byref(p)), "pb_instance_stage_params")
+        y = torch.zeros((3, p.P, p.Q, p.Ks), device="cuda", dtype=torch.bfloat16)
+        p.y = y.data_ptr()
+        capi.check(m.L.pb_op_launch(capi.STAGE_CONV_UMMA, C.byref(p), None, 0, None), "pb_op_launch")
+        torch.cuda.synchronize()
+        got[by_groups] = y
+    assert torch.equal(got[0], got[1])
+    m.L.pb_instance_destroy(inst)
+    m.close()
+
+
 def test_densenet_gang_with_and_without_fused_affines(models_dir, monkeypatch):
     path = os.path.join(models_dir, packer.pack_file_name("densenet121"))
     xs = np.random.default_rng(2).standard_normal((3, 3, 224, 224), dtype=np.float32)

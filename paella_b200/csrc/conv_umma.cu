@@ -72,6 +72,8 @@ constexpr uint32_t kSmemBudget = 200u * 1024u;   // one CTA per SM (gather kerne
 #endif
 constexpr uint32_t kSmemBudgetTma = PB_CONV_SMEM_KB * 1024u;
 constexpr uint32_t kSmemBudgetDeep = 110u * 1024u;      // small launches on a GPU they have to themselves: two CTAs per SM
+constexpr uint32_t kSmemLimit = kSmemBudget + 2048u;    // dynamic shared memory the kernels are allowed
+constexpr uint32_t kPreBytes = 512u;                    // scales and biases of a k-block of a normalising convolution
 // What a split launch asks of pb_op_params.scratch.  The partial tiles meet in the shared memory of a thread-block
 // cluster, so the memory itself is not touched: supplying it is how a caller allows the split (NULL = no split).
 constexpr uint64_t kSplitScratchBytes = 256;
@@ -2159,7 +2161,7 @@ cudaError_t raise_smem_limits() {
                              (const void*)conv_umma_gather_kernel<4>, (const void*)conv_umma_gather_kernel<6>,
                              (const void*)conv_umma_gather_kernel<8>};
     for (const void* k : kernels) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget + 2048);
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
         if (e != cudaSuccess) return e;
         // An SM's split between shared memory and L1 is fixed while blocks are resident.  Left to the default, the
         // first block to land on an idle SM sizes the split for itself alone and the SM then holds one or two blocks
@@ -2360,9 +2362,10 @@ static int make_ymap(const pb_op_params* p, int U, bool residual, CUtensorMap* o
     return make_rows_map(p, static_cast<const __nv_bfloat16*>(p->y) + p->out_c_off, p->K, p->Ks, U, 32u, out);
 }
 
-// The affine's channels are the layer's input channels, in whole vectors (x_Cs apart from pixel to pixel).
+// The affine's channels are the layer's input channels, in whole vectors (x_Cs apart from pixel to pixel), and their constants fit
+// beside the deepest pipeline even if the reduction is not split: 184 k-blocks, 11776 channels.
 bool conv_umma_pre_supported(const pb_op_params* p, const ConvPre& pre) {
-    return use_tma_a() && pointwise(p) && p->C == p->Cs && p->C % 8 == 0 && pre.x_Cs % 8 == 0 && pre.y_Cs % 8 == 0 && (pre.act == 0 || pre.act == 1) &&
+    return use_tma_a() && pointwise(p) && p->C == p->Cs && (uint32_t)ceil_div(p->Cs, kBK) * kPreBytes <= kSmemLimit - kSmemBudgetDeep && p->C % 8 == 0 && pre.x_Cs % 8 == 0 && pre.y_Cs % 8 == 0 && (pre.act == 0 || pre.act == 1) &&
            (((uintptr_t)pre.scale | (uintptr_t)pre.bias) & 15) == 0;
 }
 
@@ -2494,7 +2497,7 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
         PB_REQUIRE(use_tma_a() && conv_umma_pre_supported(p, *pre), "conv_umma: this layer cannot take an input affine");
         a.pre_scale = pre->scale; a.pre_bias = pre->bias; a.pre_act = pre->act; a.pre_offset = g.smem_bytes - 1024u;
     }
-    const uint32_t smem = g.smem_bytes + (pre ? (uint32_t)ceil_div(g.nkb, g.splits) * 512u : 0u);
+    const uint32_t smem = g.smem_bytes + (pre ? (uint32_t)ceil_div(g.nkb, g.splits) * kPreBytes : 0u);
     const dim3 grid((unsigned)g.m_tiles, (unsigned)g.n_tiles, (unsigned)g.splits);
     FinishedBlockNotifier* nf = static_cast<FinishedBlockNotifier*>(notifier);
     if (use_tma_a()) {

@@ -102,6 +102,27 @@ def test_single_stages_after_the_groups_see_the_affine(tmp_path, monkeypatch, ca
     m.close()
 
 
+@pytest.mark.parametrize("channels", [11776, 11784, 16384])
+def test_as_many_channels_as_the_constants_have_room_for(tmp_path, monkeypatch, channels):
+    """The constants of an unsplit reduction lie in one block's shared memory beside its pipeline: 184 k-blocks' at most.  Wider
+    affines have a launch of their own."""
+    g, _ = _graph((channels, channels, 16, (2, 2), True))
+    path = g.save(str(tmp_path / "affine.bin"))
+    x = np.random.default_rng(5).standard_normal((16, 2, 2), dtype=np.float32)
+    outs, launches = {}, {}
+    capi.load().pb_set_conv_split_gain_us(1e7)              # nothing splits
+    try:
+        for flag in ("0", "1"):
+            monkeypatch.setenv("PB_FUSE_AFFINE", flag)
+            m = Model(path, 1)
+            outs[flag], launches[flag] = m.run_groups(x), _launches(m)
+            m.close()
+    finally:
+        capi.load().pb_set_conv_split_gain_us(-1.0)
+    np.testing.assert_array_equal(outs["0"], outs["1"])
+    assert launches["1"] == launches["0"] - (1 if channels <= 11776 else 0)
+
+
 def test_densenet_gang_with_and_without_fused_affines(models_dir, monkeypatch):
     path = os.path.join(models_dir, packer.pack_file_name("densenet121"))
     xs = np.random.default_rng(2).standard_normal((3, 3, 224, 224), dtype=np.float32)

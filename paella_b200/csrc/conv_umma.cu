@@ -2145,8 +2145,12 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     return g;
 }
 
-const void* kernel_for(int stages, bool tma, bool pair = false) {
+// Dynamic shared memory of a launch; pre: it normalises its input.
+uint32_t dynamic_smem(const Geometry& g, bool pre) { return g.smem_bytes + (pre ? (uint32_t)ceil_div(g.nkb, g.splits) * kPreBytes : 0u); }
+
+const void* kernel_for(int stages, bool tma, bool pair, bool pre) {
     if (pair) return (const void*)conv_umma_pair_kernel;
+    if (pre) return (const void*)conv_umma_pre_kernel;
     if (tma) return (const void*)conv_umma_tma_kernel;
     switch (stages) {
         case 4: return (const void*)conv_umma_gather_kernel<4>;
@@ -2223,7 +2227,7 @@ double conv_umma_us(const pb_op_params* p, const ConvTiling& t) {
     return tiling_us(tiling_ctas(c, t), c, t);
 }
 
-int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling) {
+int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling, bool pre) {
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
     const Geometry g = geometry(p, tiling_or(tiling, p));
     memset(out, 0, sizeof(*out));
@@ -2234,14 +2238,14 @@ int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling*
     out->threads_per_block = use_tma_a() ? kThreadsTma : kThreads;
     cudaFuncAttributes at;
     uint32_t regs = 64, sstatic = 128;
-    if (cudaFuncGetAttributes(&at, kernel_for(g.stages, use_tma_a(), g.pair)) == cudaSuccess) {
+    if (cudaFuncGetAttributes(&at, kernel_for(g.stages, use_tma_a(), g.pair, pre)) == cudaSuccess) {
         regs = (uint32_t)at.numRegs;
         sstatic = (uint32_t)at.sharedSizeBytes;
     } else {
         cudaGetLastError();
     }
     out->regs_per_thread = regs;
-    out->smem_per_block = g.smem_bytes + sstatic;
+    out->smem_per_block = dynamic_smem(g, pre) + sstatic;
     out->tmem_cols_per_block = g.tmem_cols;
     const uint64_t nb = (uint64_t)batch_of(p);
     const uint64_t out_elems = nb * p->K * p->P * p->Q;
@@ -2497,7 +2501,7 @@ int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap,
         PB_REQUIRE(use_tma_a() && conv_umma_pre_supported(p, *pre), "conv_umma: this layer cannot take an input affine");
         a.pre_scale = pre->scale; a.pre_bias = pre->bias; a.pre_act = pre->act; a.pre_offset = g.smem_bytes - 1024u;
     }
-    const uint32_t smem = g.smem_bytes + (pre ? (uint32_t)ceil_div(g.nkb, g.splits) * kPreBytes : 0u);
+    const uint32_t smem = dynamic_smem(g, pre != nullptr);
     const dim3 grid((unsigned)g.m_tiles, (unsigned)g.n_tiles, (unsigned)g.splits);
     FinishedBlockNotifier* nf = static_cast<FinishedBlockNotifier*>(notifier);
     if (use_tma_a()) {

@@ -59,6 +59,7 @@ struct Stage {
     std::string name;
     int out_tensor;
     int in_tensor = -1, res_tensor = -1;   // tensors read (-1: the request input / none)
+    int pre = -1;                          // the affine stage that this convolution applies itself in the stage graphs (-1: none)
     std::vector<int> peers;                // stages whose tensor-core convolutions share a launch with this one (itself included)
 };
 
@@ -218,9 +219,10 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
     uint64_t blocks = 0;
     for (size_t k = 0; k < grp.launches.size(); ++k) {
         const std::vector<int>& l = grp.launches[k];
-        if (grp.pre[k] >= 0) {
+        if (grp.pre[k] >= 0) {                 // reads what the affine reads and writes its tensor, which is not read back
+            const pb_op_params& p = m->stages[(size_t)l[0]].p;
             out.flops += infos[(size_t)grp.pre[k]].flops;
-            out.bytes += infos[(size_t)grp.pre[k]].bytes;
+            out.bytes += infos[(size_t)grp.pre[k]].bytes - 2ull * (uint64_t)nb * p.C * p.H * p.W;
         }
         uint64_t lt = 0, ls = 0, lr = 0, lm = 0, lb = 0;
         uint32_t max_tmem = 0;
@@ -282,7 +284,7 @@ int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out
     pb_op_params p = st.p;
     p.batch = nb;
     if (st.kind != PB_STAGE_CONV_UMMA) return pb_op_info(st.kind, &p, out);
-    return pb::conv_umma_info(&p, out, &(*tilings_for(m, nb))[(size_t)stage]);
+    return pb::conv_umma_info(&p, out, &(*tilings_for(m, nb))[(size_t)stage], st.pre >= 0);
 }
 
 // Launch geometry of the stages and groups for one image.
@@ -421,6 +423,8 @@ void build_groups(pb_model* m) {
     // PB_FUSE_AFFINE=0: affine layers in front of pointwise convolutions keep launches of their own (same bits).
     if (m->fuse_branches && !m->persist && env_flag("PB_FUSE_AFFINE", true))
         for (pb_model::Group& g : m->groups) fuse_affines(m, g);
+    for (const pb_model::Group& g : m->groups)
+        for (size_t li = 0; li < g.launches.size(); ++li) m->stages[(size_t)g.launches[li][0]].pre = g.pre[li];
     refresh_infos(m);
 }
 

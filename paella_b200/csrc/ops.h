@@ -60,7 +60,8 @@ ConvTiling conv_umma_tiling(const pb_op_params* p, bool shared, bool may_split, 
 // Tilings of the convolutions of one grouped launch: they share a cluster size.
 void conv_umma_group_tilings(const pb_op_params* const* params, int n, bool shared, bool may_split, ConvTiling* out);
 double conv_umma_us(const pb_op_params* p, const ConvTiling& tiling);      // modelled microseconds of a lone launch
-int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling = nullptr);
+// pre: the launch applies an affine to its input (ConvPre).
+int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling = nullptr, bool pre = false);
 int conv_umma_launch(const pb_op_params* p, cudaStream_t st, uint32_t job_id, void* notifier);
 int64_t conv_umma_pack_weights(const pb_op_params* p, const float* w_oihw, void* dst_host);
 // Per-layer state the tensor-core path needs beyond pb_op_params (the TMA descriptor of the

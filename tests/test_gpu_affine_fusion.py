@@ -102,6 +102,32 @@ def test_single_stages_after_the_groups_see_the_affine(tmp_path, monkeypatch, ca
     m.close()
 
 
+@pytest.mark.parametrize("case", CASES)
+def test_the_launch_is_declared_with_its_constants(tmp_path, monkeypatch, case):
+    """An unsplit normalising convolution holds 512 bytes for each k-block beside its pipeline (and a few more barriers); the group
+    moves the affine's and the convolution's bytes less the convolution's input, which is not read back."""
+    g, _ = _graph(case)
+    path = g.save(str(tmp_path / "affine.bin"))
+    smem, blocks, moved, li = {}, {}, {}, capi.LaunchInfo()
+    capi.load().pb_set_conv_split_gain_us(1e7)              # nothing splits
+    try:
+        for flag in ("0", "1"):
+            monkeypatch.setenv("PB_FUSE_AFFINE", flag)
+            m = Model(path, 1)
+            names = [m.L.pb_model_stage_name(m.m, s).decode() for s in range(m.L.pb_model_num_stages(m.m))]
+            capi.check(m.L.pb_model_stage_info(m.m, names.index("conv"), C.byref(li)), "stage info")
+            smem[flag], blocks[flag] = li.smem_per_block, li.num_blocks
+            capi.check(m.L.pb_model_group_info(m.m, 0, C.byref(li)), "group info")
+            moved[flag] = li.bytes
+            m.close()
+    finally:
+        capi.load().pb_set_conv_split_gain_us(-1.0)
+    cin, _, _, (h, w), _ = case
+    assert blocks["1"] == blocks["0"]
+    assert 0 <= smem["1"] - smem["0"] - 512 * -(-cin // 64) <= 64
+    assert moved["0"] - moved["1"] == 2 * cin * h * w
+
+
 @pytest.mark.parametrize("channels", [11776, 11784, 16384])
 def test_as_many_channels_as_the_constants_have_room_for(tmp_path, monkeypatch, channels):
     """The constants of an unsplit reduction lie in one block's shared memory beside its pipeline: 184 k-blocks' at most.  Wider

@@ -60,6 +60,7 @@ struct Stage {
     int out_tensor;
     int in_tensor = -1, res_tensor = -1;   // tensors read (-1: the request input / none)
     int pre = -1;                          // the affine stage that this convolution applies itself in the stage graphs (-1: none)
+    bool may_pair = false;                 // the convolution has a launch of its own in the default plan, without an affine
     std::vector<int> peers;                // stages whose tensor-core convolutions share a launch with this one (itself included)
 };
 
@@ -161,7 +162,7 @@ bool uses_multi(const pb_model* m, const std::vector<int>& l) {
     return m->persist && m->stages[(size_t)l[0]].kind == PB_STAGE_CONV_UMMA;
 }
 
-// Has the convolution a launch to itself wherever it runs in the stage graphs (no riders, no affine of its own)?
+// Has the convolution a launch to itself in the stage graphs (no riders, no affine of its own)?
 bool launched_alone(const pb_model* m, int stage) {
     for (const pb_model::Group& g : m->groups)
         for (size_t li = 0; li < g.launches.size(); ++li)
@@ -191,8 +192,13 @@ std::shared_ptr<const std::vector<pb::ConvTiling>> tilings_for(const pb_model* m
         }
         for (const pb_op_params& p : ps) pp.push_back(&p);
         std::vector<pb::ConvTiling> t(l.size());
-        if (l.size() == 1) t[0] = pb::conv_umma_tiling(pp[0], m->shared, may_split, may_split && launched_alone(m, (int)i));
-        else pb::conv_umma_group_tilings(pp.data(), (int)l.size(), m->shared, may_split, t.data());
+        if (l.size() == 1) {
+            t[0] = pb::conv_umma_tiling(pp[0], m->shared, may_split, may_split && m->stages[i].may_pair);
+            // beside a rider, or with an affine, there are no pairs: whole tiles have their bits
+            if (t[0].pair && !launched_alone(m, (int)i)) t[0] = pb::conv_umma_tiling(pp[0], m->shared, false, false);
+        } else {
+            pb::conv_umma_group_tilings(pp.data(), (int)l.size(), m->shared, may_split, t.data());
+        }
         for (size_t k = 0; k < l.size(); ++k) (*by_stage)[(size_t)l[k]] = t[k];
     }
     kept = {gain, m->shared, by_stage};
@@ -410,11 +416,16 @@ void build_groups(pb_model* m) {
     // (PB_GRAPH_BRANCHES=1) or PB_FUSE_BRANCHES=0.
     m->fuse_branches = env_flag("PB_FUSE_BRANCHES", true) && !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available();
     m->persist = !env_flag("PB_GRAPH_BRANCHES", false) && pb::conv_umma_multi_available() && pb::conv_umma_persist_enabled();
-    // The convolutions of one grouped launch share a cluster size.  It is decided on the default plan whatever the
-    // switches say, so that they change the scheduling of the model and not its bits.
-    for (const pb_model::Group& g : plan_groups(m, dflt, true, false))
+    // The convolutions of one grouped launch share a cluster size, and one that has a launch of its own may run on pairs of blocks
+    // instead of splitting its reduction.  Both are decided on the default plan whatever the switches say, so that they change
+    // the scheduling of the model and not its bits.
+    for (pb_model::Group& g : plan_groups(m, dflt, true, false)) {
         for (const std::vector<int>& l : g.launches)
             for (int s : l) m->stages[(size_t)s].peers = l;
+        fuse_affines(m, g);
+        for (size_t li = 0; li < g.launches.size(); ++li)
+            if (g.launches[li].size() == 1) m->stages[(size_t)g.launches[li][0]].may_pair = g.pre[li] < 0;
+    }
     // PB_FUSE_POOLS=1: off by default; not with the persistent kernel.  Measured: same bits, a lone Inception-v3 request
     // 342 -> 330 us, but 317 -> 313 thousand requests a second of MNIST : Inception-v3 = 9 : 1 in a closed loop of 192 clients: a
     // pooling block then holds a whole convolution slot of its SM (the launch's 73 KB of shared memory) while it waits on

@@ -7,9 +7,11 @@ in fp32 in any order differ from the exact sum by at most n * 2^-23 * sum |produ
 order); one rounding to bf16 (2^-8 relative) follows."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
-from paella_b200 import capi
+from paella_b200 import capi, packer
+from tests.test_gpu_models import Model
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +74,37 @@ def test_pairs_of_blocks(case, mode, monkeypatch):
     untouched = torch.ones(total, dtype=torch.bool)
     untouched[off:off + k] = False
     assert bool((y[..., untouched.cuda()] == 7.0).all())
+
+
+def test_the_plan_of_a_model_does_not_change_its_bits(tmp_path, monkeypatch):
+    """A convolution that runs on pairs of blocks in the default plan (and whose reduction lone blocks would split), with a pooling
+    layer in its launch, and in launches of other groupings: the same bits."""
+    g = packer.Graph("pairs", (16, 40, 40), seed=3, precision=1, round_weights_bf16=True)
+    x = g.conv(g.input, 1024, 1, name="wide")
+    cat = g.tensor(192 + 1024, 40, 40)
+    g.conv(x, 192, 3, 1, 1, name="big", out=cat, out_c_off=0)
+    g.maxpool(x, 3, 1, 1, out=cat, out_c_off=192, name="pool")
+    g.dense(g.gap(g.conv(cat, 32, 1, name="next"), name="gap"), 10, name="fc")
+    path = g.save(str(tmp_path / "pairs.bin"))
+    xs = np.random.default_rng(4).standard_normal((8, 16, 40, 40), dtype=np.float32)
+    switches = ["PB_CONV_PAIR", "PB_FUSE_POOLS", "PB_STAGE_GROUP", "PB_FUSE_BRANCHES"]
+    outs, smem, split, li = {}, {}, {}, capi.LaunchInfo()
+    for name, value in [(None, None), ("PB_CONV_PAIR", "0"), ("PB_FUSE_POOLS", "1"), ("PB_STAGE_GROUP", "2"), ("PB_FUSE_BRANCHES", "0")]:
+        for sw in switches:
+            monkeypatch.delenv(sw, raising=False)
+        if name:
+            monkeypatch.setenv(name, value)
+        m = Model(path, 1)
+        names = [m.L.pb_model_stage_name(m.m, s).decode() for s in range(m.L.pb_model_num_stages(m.m))]
+        capi.check(m.L.pb_model_stage_info_batched(m.m, names.index("big"), 8, C.byref(li)), "stage info")
+        smem[name], split[name] = li.smem_per_block, li.num_blocks > 100
+        inst, y = C.c_void_p(), np.zeros((8, 10), np.float32)
+        capi.check(m.L.pb_instance_create_batched(m.m, 8, 0, C.byref(inst)), "pb_instance_create_batched")
+        capi.check(m.L.pb_instance_run_batch_sync(inst, 8, 1, xs.ctypes.data, y.ctypes.data), "run batch")
+        outs[name] = y
+        m.L.pb_instance_destroy(inst)
+        m.close()
+    assert split["PB_CONV_PAIR"] and not split[None]       # 100 row tiles: lone blocks split them, pairs do not
+    assert smem[None] == smem["PB_STAGE_GROUP"] == smem["PB_FUSE_BRANCHES"] != smem["PB_FUSE_POOLS"]
+    for name in ("PB_FUSE_POOLS", "PB_STAGE_GROUP", "PB_FUSE_BRANCHES"):
+        np.testing.assert_array_equal(outs[name], outs[None], err_msg=name)

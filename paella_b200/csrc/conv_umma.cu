@@ -2080,12 +2080,33 @@ ConvTiling choose_tiling(const ConvShape& c, int bn_max, int want_splits, double
 ConvShape conv_shape(const pb_op_params* p, bool shared) {
     return {ceil_div(batch_of(p) * p->P * p->Q, kBM), round_up(p->K, 16), p->R * p->S * ceil_div(p->Cs, kBK), p->residual != nullptr, shared};
 }
+// Would lone blocks have less to do on the fullest SM than pairs, with n tiles of BN columns?
+// - In fewer waves (148 pairs, two on a pair of SMs, against 296 blocks): with an odd m_tiles the last pair holds one real row tile.
+//   Measured, lone blocks / pairs, 768 columns at 16 / 36 / 72 k-blocks: 297 pairs 0.83 / 0.84 / 0.88, 741 0.99 / 0.97 / 0.94, 1185 1.04 / 0.97 / 1.00;
+//   half a wave more is none (519 pairs 1.06 / 1.02 / 1.06).
+// - In as many rounds of one block an SM, with tiles of three quarters of the columns.  One round: 384 columns on 48 row tiles (128 wide
+//   against 192) 0.86 to 0.91 at 16 to 72 k-blocks, 640 on 31 (160 / 224) 0.83 to 0.89, 576 on 31 (144 / 192) 0.92 to 0.95, 512 on 48
+//   (176 / 256) 0.97 at 16, 1.07 at 36, 1.13 at 72, 768 on 31 (192 / 256) 0.97 / 1.05 / 1.11.  Three rounds, 99 row tiles, at 16 / 36 / 72 k-blocks:
+//   640 columns 0.89 / 0.96 / 1.01, 768 columns 0.90 / 0.92 to 0.97 / 1.00, 576 columns (144 wide, which TMA does not store) 1.00 / 1.10 / 1.13.
+//   Four fifths of the columns are no match: 1024 on 25 row tiles (208 / 256) 1.04 / 1.12 / 1.20.
+bool lone_is_lighter(const ConvShape& c, int n, int BN, int pairs) {
+    const int waves = ceil_div(pairs, 148), rounds = ceil_div(pairs, 74);
+    if (waves <= 6 && ceil_div(c.m_tiles * n, 296) < waves) return true;
+    for (int k = n + 1; ceil_div(c.m_tiles * k, 148) <= rounds; ++k) {
+        const int w = round_up(ceil_div(c.Kp16, k), 16);
+        if (4 * w > 3 * BN) continue;
+        if (c.nkb < 36 || (rounds == 1 ? BN < 256 : c.nkb < 64 && w % 32 == 0)) return true;
+    }
+    return false;
+}
 // When a launch runs on pairs of blocks: wide tiles (the weights are what is shared), a k-loop long enough to carry the pair's
-// set-up, and tiles that fill the 74 pairs of SMs evenly - one each, or (nearly) two and more, which share a pair of SMs and are
-// replaced as they finish.  Measured, lone blocks / pairs, us: 288 -> 384 3x3 35 x 35 x 64 images (614 pairs, 192 columns) 142 / 131, the
-// same with stride 2 (146) 32.6 / 31.4, 256 -> 256 3x3 56 x 56 x 16 (196) 56.4 / 48.0, 1024 -> 256 1x1 56 x 56 x 16 (196, 16 k-blocks)
-// 41.6 / 39.5, 1024 -> 1024 3x3 14 x 14 x 16 (52) 64.2 / 52.1, 256 -> 256 3x3 28 x 28 x 16 with a residual (49) 25.2 / 21.2; and outside:
-// 512 -> 512 3x3 28 x 28 x 16 (98 pairs) 46.4 / 52.9, 128 columns 62.5 / 69.7, 96 columns 28.6 / 37.4, 4 k-blocks 52.7 / 56.5.
+// set-up, and 48 to 74 pairs, one for each pair of SMs, or 140 and more, where two share a pair of SMs and are replaced as they finish -
+// where lone blocks do not come out lighter.  Measured, lone blocks / pairs, us: 288 -> 384 3x3 35 x 35 x 64 images (614 pairs, 192
+// columns) 143.8 / 132.8, 1024 -> 1024 3x3 14 x 14 x 16 (52) 61.3 / 49.4, 512 -> 512 3x3 28 x 28 x 8 (50) 32.9 / 29.3, 256 -> 256 3x3
+// 28 x 28 x 16 with a residual (49) 22.7 / 19.1; 256 and 512 columns on maps of 16 x 32 by pairs, lone / pairs, at 18 / 36 / 72 k-blocks: 48 to
+// 72 pairs 1.09 to 1.11 / 1.18 to 1.20 / 1.13 to 1.27, 140 to 148 0.99 to 1.01 / 1.00 / 1.01, 152 to 176 1.05 / 1.06 to 1.11 / 1.11 to 1.22, 184
+// to 208 1.10 / 1.00 / 1.00, 220 to 296 1.00 / 1.00 to 1.02 / 1.00 to 1.02, 304 and more 1.00 to 1.06 / 1.01 to 1.12 / 1.01 to 1.05.  Outside: 76 to
+// 96 pairs 0.98 / 0.99 / 0.88, 32 pairs 0.76, 4 k-blocks (196 pairs) 0.97.
 // Not on a GPU that other requests share, where three lone blocks an SM do better.
 // PB_CONV_PAIR (read at every use; for tests and comparisons): 0 = no pairs, 1 = pairs wherever their kernel can run.
 ConvTiling pair_tiling(const ConvShape& c) {
@@ -2095,7 +2116,7 @@ ConvTiling pair_tiling(const ConvShape& c) {
     if (force == 0 || !use_tma_a() || persist_enabled() || bn_limit() < 256) return none;
     const int n = ceil_div(c.Kp16, 256), BN = round_up(ceil_div(c.Kp16, n), 32);
     const int pairs = ceil_div(c.m_tiles, 2) * n;
-    if (force < 0 && (c.shared || BN < 192 || c.nkb < 16 || pairs < 48 || (pairs > 74 && pairs < 140))) return none;
+    if (force < 0 && (c.shared || BN < 192 || c.nkb < 16 || pairs < 48 || (pairs > 74 && pairs < 140) || lone_is_lighter(c, n, BN, pairs))) return none;
     return {BN, 1, true, c.shared, true};
 }
 bool splits_off() { return !use_tma_a() || conv_split_gain_us() > 1e6; }

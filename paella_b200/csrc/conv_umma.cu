@@ -2252,8 +2252,8 @@ int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling*
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
     const Geometry g = geometry(p, tiling_or(tiling, p));
     memset(out, 0, sizeof(*out));
-    // what a split launch asks for
-    out->scratch_bytes = (tiling ? g.splits : tiling_for(p, false, 0).splits) > 1 ? kSplitScratchBytes : 0;
+    // what a split launch asks for, if it may split
+    out->scratch_bytes = (tiling ? g.splits : tiling_for(p, false, 0, true).splits) > 1 ? kSplitScratchBytes : 0;
     out->kind = PB_STAGE_CONV_UMMA;
     out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
     out->threads_per_block = use_tma_a() ? kThreadsTma : kThreads;

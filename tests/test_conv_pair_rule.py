@@ -41,3 +41,12 @@ def test_which_launches_are_pairs(monkeypatch, pair, c, k, r, row_tiles):
     lone, forced, got = (_info(monkeypatch, mode, c, k, r, row_tiles) for mode in ("0", "1", ""))
     assert forced[:2] != lone[:2]
     assert got[:2] == (forced if pair else lone)[:2]
+
+
+def test_pairs_ask_for_no_scratch(monkeypatch):
+    """A reduction that lone blocks would split (144 k-blocks on 100 row tiles) and pairs do not: the scratch memory
+    that allows the split is asked for only where it would be used."""
+    lone, forced, got = (_info(monkeypatch, mode, 1024, 192, 3, 100) for mode in ("0", "1", ""))
+    assert lone[2] > 0 and lone[0] > 100
+    assert got == forced and got[2] == 0
+    assert _info(monkeypatch, "", 1024, 192, 3, 100, scratch=False) == got

@@ -2130,7 +2130,9 @@ ConvTiling tiling_for(const pb_op_params* p, bool shared, int want_splits, bool 
 }
 // The split is the caller's to allow: by the scratch memory that pb_launch_info.scratch_bytes asks for.
 bool split_allowed(const pb_op_params* p) { return p->scratch != nullptr && p->scratch_bytes >= kSplitScratchBytes; }
-ConvTiling tiling_or(const ConvTiling* given, const pb_op_params* p) { return given ? *given : tiling_for(p, false, split_allowed(p) ? 0 : 1, true); }
+ConvTiling tiling_or(const ConvTiling* given, const pb_op_params* p, bool pre) {
+    return given ? *given : tiling_for(p, false, split_allowed(p) ? 0 : 1, !pre);      // the pair kernel does not normalise
+}
 
 Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     Geometry g;
@@ -2250,10 +2252,10 @@ double conv_umma_us(const pb_op_params* p, const ConvTiling& t) {
 
 int conv_umma_info(const pb_op_params* p, pb_launch_info* out, const ConvTiling* tiling, bool pre) {
     PB_REQUIRE(conv_umma_supported(p), "conv_umma: unsupported convolution");
-    const Geometry g = geometry(p, tiling_or(tiling, p));
+    const Geometry g = geometry(p, tiling_or(tiling, p, pre));
     memset(out, 0, sizeof(*out));
     // what a split launch asks for, if it may split
-    out->scratch_bytes = (tiling ? g.splits : tiling_for(p, false, 0, true).splits) > 1 ? kSplitScratchBytes : 0;
+    out->scratch_bytes = (tiling ? g.splits : tiling_for(p, false, 0, !pre).splits) > 1 ? kSplitScratchBytes : 0;
     out->kind = PB_STAGE_CONV_UMMA;
     out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
     out->threads_per_block = use_tma_a() ? kThreadsTma : kThreads;
@@ -2513,13 +2515,13 @@ static cudaError_t launch_pdl(void (*kern)(Args...), dim3 grid, dim3 cluster, ui
 
 int conv_umma_launch_planned(const ConvUmmaPlan* plan, const ConvUmmaXMap* xmap, const pb_op_params* p, cudaStream_t st,
                              uint32_t job_id, void* notifier, uint32_t* err_flag, bool pdl, const ConvTiling* tiling, const ConvPre* pre) {
-    const Geometry g = geometry(p, tiling_or(tiling, p));
+    const Geometry g = geometry(p, tiling_or(tiling, p, pre != nullptr));
     if (!use_tma_a()) PB_REQUIRE(batch_of(p) == 1, "conv_umma: the cp.async gather kernel (PB_CONV_GATHER=1) runs one image per launch");
     ConvArgs a;
     const int frc = fill_args(plan, g, p, err_flag, &a);
     if (frc != PB_OK) return frc;
     if (pre) {
-        PB_REQUIRE(use_tma_a() && conv_umma_pre_supported(p, *pre), "conv_umma: this layer cannot take an input affine");
+        PB_REQUIRE(use_tma_a() && !g.pair && conv_umma_pre_supported(p, *pre), "conv_umma: this layer cannot take an input affine");
         a.pre_scale = pre->scale; a.pre_bias = pre->bias; a.pre_act = pre->act; a.pre_offset = g.smem_bytes - 1024u;
     }
     const uint32_t smem = dynamic_smem(g, pre != nullptr);

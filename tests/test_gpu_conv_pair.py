@@ -6,12 +6,17 @@ Reference: the convolution of the bf16 operands in 64 bits.  Products of bf16 va
 in fp32 in any order differ from the exact sum by at most n * 2^-23 * sum |products| (every addition truncating, in the worst
 order); one rounding to bf16 (2^-8 relative) follows."""
 import ctypes as C
+import os
 
 import numpy as np
 import pytest
 
+from oracle import graph as og
 from paella_b200 import capi, packer
+from tests import gpu_util as gu
+from tests.test_gpu_gang import _pinned, _run_until, _server
 from tests.test_gpu_models import Model
+from tests.test_gpu_serving_options import _register
 
 pytestmark = pytest.mark.gpu
 
@@ -29,12 +34,10 @@ CASES = [
 ]
 
 
-@pytest.mark.parametrize("mode", ["0", "1"])
-@pytest.mark.parametrize("case", CASES)
-def test_pairs_of_blocks(case, mode, monkeypatch):
+def _problem(case):
+    """Operator parameters on the GPU (with what they point to) and the 64-bit result with its error bound."""
     import torch
     L = capi.load()
-    monkeypatch.setenv("PB_CONV_PAIR", mode)
     c, h, w, k, r, s, stride, ph, pw, n, act, residual, off, total = case
     P, Q = (h + 2 * ph - r) // stride + 1, (w + 2 * pw - s) // stride + 1
     gen = torch.Generator(device="cuda").manual_seed(c * 131 + h)
@@ -43,7 +46,6 @@ def test_pairs_of_blocks(case, mode, monkeypatch):
     wt = (torch.randn((k, c, r, s), generator=gen, device="cuda") * (2.0 / (c * r * s)) ** 0.5).to(torch.bfloat16)
     bias = torch.randn(2 * k, generator=gen, device="cuda") * 0.1          # PReLU: the slopes follow
     res = torch.randn((n, P, Q, k), generator=gen, device="cuda").to(torch.bfloat16)
-    y = torch.full((n, P, Q, total), 7.0, device="cuda", dtype=torch.bfloat16)
     p = capi.OpParams()
     p.dtype, p.C, p.H, p.W, p.Cs, p.K, p.P, p.Q, p.Ks, p.out_c_off = 1, c, h, w, cs, k, P, Q, total, off
     p.R, p.S, p.stride_h, p.stride_w, p.pad_h, p.pad_w, p.groups, p.act, p.batch, p.dil_h, p.dil_w = r, s, stride, stride, ph, pw, 1, act, n, 1, 1
@@ -52,7 +54,7 @@ def test_pairs_of_blocks(case, mode, monkeypatch):
     packed = torch.zeros(size, dtype=torch.uint8)
     L.pb_op_pack_weights(capi.STAGE_CONV_UMMA, C.byref(p), host.data_ptr(), packed.data_ptr())
     packed = packed.cuda()
-    p.x, p.w, p.bias, p.y = x.data_ptr(), packed.data_ptr(), bias.data_ptr(), y.data_ptr()
+    p.x, p.w, p.bias = x.data_ptr(), packed.data_ptr(), bias.data_ptr()
     if residual:
         p.residual, p.res_Cs = res.data_ptr(), k
     xd, wd = x[..., :c].permute(0, 3, 1, 2).double().cpu(), wt.double().cpu()
@@ -64,16 +66,95 @@ def test_pairs_of_blocks(case, mode, monkeypatch):
     want = torch.where(want > 0, want, want * bias[k:].double().cpu()) if act == 3 else want
     want = want.clamp(max=6.0) if act == 2 else want
     bound = c * r * s * 2.0 ** -23 * conv(xd.abs(), wd.abs()) + 2.0 ** -8 * want.abs() + 1e-6
+    return p, (x, packed, bias, res), want, bound
+
+
+def _launch(p):
+    """The output of one launch, every channel of the destination."""
+    import torch
+    L = capi.load()
+    y = torch.full((p.batch, p.P, p.Q, p.Ks), 7.0, device="cuda", dtype=torch.bfloat16)
+    p.y = y.data_ptr()
     capi.check(L.pb_op_launch(capi.STAGE_CONV_UMMA, C.byref(p), None, 0, None), "pb_op_launch")
     torch.cuda.synchronize()
-    flag = C.c_uint32(0)
-    capi.check(L.pb_device_error_flag(0, C.byref(flag), 1), "pb_device_error_flag")
-    assert flag.value == 0
-    got = y[..., off:off + k].double().cpu()
-    assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound).max())
-    untouched = torch.ones(total, dtype=torch.bool)
-    untouched[off:off + k] = False
-    assert bool((y[..., untouched.cuda()] == 7.0).all())
+    assert gu.error_flag() == 0
+    return y
+
+
+def _geometry(p):
+    li = capi.LaunchInfo()
+    capi.check(capi.load().pb_op_info(capi.STAGE_CONV_UMMA, C.byref(p), C.byref(li)), "pb_op_info")
+    return li.num_blocks, li.smem_per_block
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_pairs_of_blocks(case, monkeypatch):
+    """Both ways within the bound, and with the same bits: neither splits its reduction (no scratch memory is given)."""
+    import torch
+    p, keep, want, bound = _problem(case)
+    k, off = case[3], case[12]
+    got, geometry = {}, {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("PB_CONV_PAIR", mode)
+        geometry[mode] = _geometry(p)
+        got[mode] = _launch(p)
+        y = got[mode][..., off:off + k].double().cpu()
+        assert bool(((y - want).abs() <= bound).all()), float(((y - want).abs() / bound).max())
+        untouched = torch.ones(p.Ks, dtype=torch.bool)
+        untouched[off:off + k] = False
+        assert bool((got[mode][..., untouched.cuda()] == 7.0).all())
+    row_tiles, col_tiles = -(-p.batch * p.P * p.Q // 128), -(-k // 256)
+    assert geometry["1"] != geometry["0"] and geometry["1"][0] == (row_tiles + 1) // 2 * 2 * col_tiles
+    assert torch.equal(got["0"], got["1"])
+
+
+def test_pairs_by_the_default_rule(monkeypatch):
+    """50 pairs of 224 columns, 36 k-blocks: taken without the switch."""
+    import torch
+    p, keep, want, bound = _problem((256, 40, 40, 224, 3, 3, 1, 1, 1, 8, 1, True, 0, 224))
+    got, geometry = {}, {}
+    for mode in ("0", "1", ""):
+        monkeypatch.setenv("PB_CONV_PAIR", mode)
+        geometry[mode], got[mode] = _geometry(p), _launch(p)
+    assert geometry[""] == geometry["1"] != geometry["0"]
+    assert torch.equal(got[""], got["0"])
+    assert bool(((got[""].double().cpu() - want).abs() <= bound).all())
+
+
+def test_pairs_report_every_block_beside_other_requests(tmp_path, monkeypatch):
+    """PB_CONV_PAIR=1 on a server, three launches a stage: stages end in a pair launch, behind a programmatic predecessor, which
+    reports the blocks it was declared with while other requests' convolutions run on other streams."""
+    d = tmp_path / "models_pairs_served"
+    d.mkdir()
+    packer.write_all(str(d), ["resnet18"])
+    monkeypatch.delenv("PB_PRECISION", raising=False)
+    monkeypatch.setenv("PB_CONV_PAIR", "1")
+    monkeypatch.setenv("PB_STAGE_GROUP", "3")
+    L, s = _server(str(d), monkeypatch, 1)
+    job, ib, ob, sb = _register(L, s, "tvm_resnet18")
+    n = 6
+    t, xs = _pinned(sb * n), np.random.default_rng(3).standard_normal((n, 3, 224, 224), dtype=np.float32)
+    for i in range(n):
+        t.numpy()[i * sb:i * sb + ib] = np.frombuffer(xs[i].tobytes(), np.uint8)
+        capi.check(L.pb_server_launch(s, job, t.data_ptr() + i * sb, i), "launch")
+    done = _run_until(L, s, n, timeout=20.0)
+    assert done == {i: 0 for i in range(n)}, "a request was not answered"
+    assert gu.error_flag() == 0
+    pack, off = og.Pack(packer.MODELS["resnet18"](seed=1234).to_bytes()), (ib + 7) // 8 * 8
+    ys = [np.frombuffer(t.numpy()[i * sb + off:i * sb + off + ob].tobytes(), np.float32) for i in range(n)]
+    for i in (0, n - 1):
+        ref = og.run(pack, xs[i])
+        assert float(np.abs(ys[i] - ref).max()) <= 1e-2 * float(np.abs(ref).max())
+    L.pb_server_destroy(s)
+    # the stages do end in pair launches: their declared geometry is not the lone blocks'
+    path, li, ends = os.path.join(str(d), packer.pack_file_name("resnet18")), capi.LaunchInfo(), {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("PB_CONV_PAIR", mode)
+        m = Model(path, 1)
+        capi.check(L.pb_model_group_info(m.m, 1, C.byref(li)), "group info")
+        ends[mode] = li.num_blocks
+        m.close()
+    assert ends["1"] != ends["0"] and ends["1"] % 2 == 0
 
 
 def test_the_plan_of_a_model_does_not_change_its_bits(tmp_path, monkeypatch):

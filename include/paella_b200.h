@@ -191,7 +191,7 @@ PB_API int pb_conv_umma_supported(const pb_op_params* p);
 PB_API void pb_set_conv_split_gain_us(double us);
 /* Mean microseconds of one launch of the tensor-core convolution `p` (any batch): 3 warm-up launches, then `iters`
  * launches on a private stream between CUDA events, a write of flush_bytes before each (0 = none).  mode 0 = the
- * one-tile-per-CTA kernel pb_op_launch uses, 1 = the persistent kernel the model stage graphs use. */
+ * kernel pb_op_launch uses, 1 = the persistent kernel of the stage graphs (PB_CONV_PERSIST=1). */
 PB_API int pb_conv_umma_time(const pb_op_params* p, int mode, int iters, size_t flush_bytes, double* us_out);
 /* Tensor-core convolution for callers that must not allocate: code running inside a CUDA memory-pool
  * or allocator callback, a latency-critical thread that may not take the allocator's locks, or a host
@@ -239,7 +239,7 @@ PB_API int pb_instance_launch_stage(pb_instance* inst, int stage, void* stream, 
  * (default up to 48 kernels, PB_STAGE_GROUP=1 gives the reference's one-kernel-per-stage granularity).
  * A multi-kernel group is replayed as a CUDA graph - one driver call instead of one per kernel - and
  * only its last kernel reports block start/end on the notifier, so pb_model_group_info's block count
- * is that kernel's grid and its per-block resources are the group's largest footprint spread over
+ * is that kernel's grid and its per-block resources are the mean footprint over the group's time spread over
  * those blocks.  io_in / io_out: this request's input (NCHW fp32) and output buffers, device memory
  * or host-mapped pinned memory; the first kernel reads io_in and the last writes io_out directly
  * (no separate copy stages).  NULL = the instance's own device buffers. */
@@ -250,7 +250,7 @@ PB_API int pb_model_group_stages(const pb_model* m, int group, int* first_stage,
  * for each, the index of the launch it belongs to.  Stages that share a launch index are independent
  * tensor-core convolutions issued as ONE grid (the parallel branches of an Inception block, a ResNet
  * shortcut beside the block's first convolution), or an affine layer followed by the pointwise convolution that
- * applies it to its input tiles itself (never in the group's last launch); the group's last launch is the one that notifies, so
+ * applies it to its input tiles itself and stores the affine's tensor (never in the group's last launch); the group's last launch is the one that notifies, so
  * pb_model_group_info's block count is the sum of its stages' grids.  Returns the number of stages
  * written (<= max_stages).  PB_FUSE_BRANCHES=0 at load time: program order, one stage per launch.
  * No counterpart in the reference (it launches one TVM kernel at a time). */

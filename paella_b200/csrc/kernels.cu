@@ -1182,7 +1182,7 @@ __global__ void __launch_bounds__(256) affine_kernel(OpArgs a, uint32_t job_id, 
     const size_t pixels = (size_t)a.H * a.W, part = affine_threads(pixels, cv), step = part / cv;
     const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i0 < part) {
-        // 32-bit division whenever the index fits (always, short of a 64 GB tensor)
+        // 32-bit division whenever the index fits (always, short of a 256 GB tensor)
         const size_t pix0 = part <= 0xffffffffull ? (size_t)((uint32_t)i0 / (uint32_t)cv) : i0 / cv;
         const int c0 = (int)(i0 - pix0 * cv) * N;
         const T* __restrict__ x = static_cast<const T*>(a.x) + c0;
@@ -1493,13 +1493,13 @@ static uint32_t static_smem_of(F fn) {
     return (uint32_t)at.sharedSizeBytes;
 }
 
-// Threads of work -> blocks of 256.
 // Does a pooling layer run pool2_kernel?  Rows of less than 192 vectors leave most of a block idle: they keep pool_kernel.
 static bool pool2(const pb_op_params* p) {
     const int N = p->dtype == 0 ? 4 : 8;
     return p->R == 2 && p->S == 2 && p->stride_h == 2 && p->stride_w == 2 && p->pad_h == 0 && p->pad_w == 0 && 2 * p->P <= p->H && 2 * p->Q <= p->W &&
            p->Cs % N == 0 && (int64_t)p->Q * (p->Cs / N) >= 192 && (int64_t)p->Q * p->Cs < (1 << 30);
 }
+// Threads of work -> blocks of 256.
 static uint32_t blocks_for(size_t work) { return (uint32_t)((work + 255) / 256 > 0 ? (work + 255) / 256 : 1); }
 
 // Output pixels per thread of window3_strip_kernel for a depthwise convolution or pooling layer: 0 when the

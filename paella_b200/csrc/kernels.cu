@@ -74,7 +74,8 @@ __device__ __forceinline__ float act_fn(float v, int act) {
 // Every kernel here may be launched as a programmatic dependent of the previous kernel of its stage
 // graph: it waits for that kernel on the device before touching memory (a no-op otherwise).  PB_NOTIFY_START_EARLY then lets
 // the next kernel's blocks in, which set themselves up (tensor memory, barriers, first weights) while this one runs: 2.0 us
-// from this kernel's end to the next one's first instruction after its wait without that trigger, 0.75 us with it.
+// from this kernel's end to the next one's first instruction after its wait without that trigger, 0.75 us with it (window3_tile_kernel
+// has none: not measured there).
 // Only where this kernel is short, so that the blocks that wait hold their SM slots for a microsecond or two (the input kernels
 // take 8 to 25 us: triggered at their start, 32 ResNet-18 requests took 833 instead of 808 us), and only in bf16: the
 // full-precision convolution's blocks, when they come in beside other blocks, are dealt two to an SM while others idle

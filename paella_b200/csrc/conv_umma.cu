@@ -337,7 +337,8 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t x, uint64_t y) {
 }
 // The activation is chosen at run time, by branches all threads take alike: as a template parameter of the epilogues it made four
 // copies of each (and of each cluster size), 124 KB of code per kernel, and a launch whose copy had not run on its SM lately
-// spent 0.5 to 1.6 us of its epilogue fetching it.  The loops below are kept rolled for the same reason.
+// spent 0.5 to 1.6 us of its epilogue fetching it.  The loops below are kept rolled for the same reason.  Two copies, ReLU and ReLU6 /
+// the others, are as fast as four where the arguments are constants (the lone launches): see EpiArgs.
 __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
     uint32_t l, h;
     asm("mov.b64 {%0, %1}, %2;" : "=r"(l), "=r"(h) : "l"(v));
@@ -345,8 +346,13 @@ __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
     hi = __uint_as_float(h);
 }
 
-// What the epilogues need of a convolution's arguments, in registers before they wait for the accumulator.  (A grouped launch has
-// its arguments in shared memory, and a compiler that sees a memory barrier reads them again behind each.)
+// What the epilogues of grouped and normalising launches need of a convolution's arguments, in registers before they wait for the
+// accumulator.  (A grouped launch has its arguments in shared memory, and a compiler that sees a memory barrier reads them again behind
+// each.)  Lone launches read their arguments where they are, in the constant bank, so that the compiler knows every branch on
+// them to be taken alike, and have the activation's branch outside of the column loops (kAct).  Measured, a launch in a row of equal ones, us,
+// registers and a branch per 8 columns / this: 64 -> 256 channels 1x1 on 8 maps of 56 x 56 7.04 / 6.39, 256 -> 1024 at 14 x 14
+// with a residual 5.92 / 5.58, 184 -> 120 at 112 x 112, stride 2, with a residual 5.25 / 5.11; ResNet-50 x 8 images 373 / 359.  (For grouped and
+// normalising launches this is the slower way: Inception-v3 alone 298.7 / 300.2, DenseNet-121 x 3 images 641 / 650.)
 struct EpiArgs {
     const __nv_bfloat16* residual;
     const float* bias;
@@ -358,10 +364,12 @@ __device__ __forceinline__ EpiArgs epi_args(const ConvArgs& a) {
     return {a.residual, a.bias, a.y, a.err_flag, a.M, a.K, a.Ks, a.out_c_off, a.res_Cs, a.act, a.BN, a.out_box, a.splits, a.nkb};
 }
 
+// kAct: 0 = the activation is chosen here, 1 = it is ReLU or ReLU6, 2 = it is neither.
 // Eight accumulator columns of this thread's row, from channel k on: + bias (+ residual), activation, bf16.  The four epilogue
 // warps run one per scheduler with nothing to hide instruction latency behind, so this is kept to one packed add and one
 // convert per two columns.
-__device__ __forceinline__ uint4 finish8(const EpiArgs& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias) {
+template <int kAct, class Args>
+__device__ __forceinline__ uint4 finish8(const Args& a, const uint32_t* v, const uint4& res, bool has_res, int k, const float* bias) {
     uint64_t f[4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -375,7 +383,7 @@ __device__ __forceinline__ uint4 finish8(const EpiArgs& a, const uint32_t* v, co
         for (int j = 0; j < 4; ++j) f[j] = add_f32x2(f[j], pack_f32x2(ru[j] << 16, ru[j] & 0xffff0000u));
     }
     uint32_t o[4];
-    if (a.act == 1 || a.act == 2) {
+    if (kAct == 1 || (kAct == 0 && (a.act == 1 || a.act == 2))) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float lo, hi;
@@ -408,18 +416,20 @@ __device__ __forceinline__ uint4 finish8(const EpiArgs& a, const uint32_t* v, co
     }
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
-__device__ __forceinline__ void epilogue_chunk(const EpiArgs& a, const uint32_t (&v)[16], const uint4 (&rv)[2], int cb, int n0, bool row_valid,
+template <int kAct, class Args>
+__device__ __forceinline__ void epilogue_chunk(const Args& a, const uint32_t (&v)[16], const uint4 (&rv)[2], int cb, int n0, bool row_valid,
                                                __nv_bfloat16* yrow, bool has_res, const float* s_bias) {
     if (!row_valid) return;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int k = n0 + cb + h * 8;
-        if (k + 8 <= a.K) *reinterpret_cast<uint4*>(yrow + k) = finish8(a, v + h * 8, rv[h], has_res, k, s_bias + cb + h * 8);
+        if (k + 8 <= a.K) *reinterpret_cast<uint4*>(yrow + k) = finish8<kAct>(a, v + h * 8, rv[h], has_res, k, s_bias + cb + h * 8);
     }
 }
 
 // The residual of the 16 columns from cb on (zeros where there is none).
-__device__ __forceinline__ void load_residual(const EpiArgs& a, int k0, bool row_valid, const __nv_bfloat16* rrow, uint4 (&rv)[2]) {
+template <class Args>
+__device__ __forceinline__ void load_residual(const Args& a, int k0, bool row_valid, const __nv_bfloat16* rrow, uint4 (&rv)[2]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         rv[h] = make_uint4(0, 0, 0, 0);
@@ -429,7 +439,8 @@ __device__ __forceinline__ void load_residual(const EpiArgs& a, int k0, bool row
 
 // Columns in steps of 16, two steps in flight: the next step leaves tensor memory (and its residual is on its way)
 // while this one is converted and stored.
-__device__ __forceinline__ void epilogue_columns(const EpiArgs& a, uint32_t lane_addr, int n0, bool row_valid, __nv_bfloat16* yrow,
+template <int kAct, class Args>
+__device__ __forceinline__ void epilogue_columns(const Args& a, uint32_t lane_addr, int n0, bool row_valid, __nv_bfloat16* yrow,
                                                  const __nv_bfloat16* rrow, const float* s_bias) {
     uint32_t v0[16], v1[16];
     uint4 r0[2], r1[2];
@@ -444,14 +455,14 @@ __device__ __forceinline__ void epilogue_columns(const EpiArgs& a, uint32_t lane
             tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
             load_residual(a, n0 + cb + 16, row_valid, rrow, r1);
         }
-        epilogue_chunk(a, v0, r0, cb, n0, row_valid, yrow, has_res, s_bias);
+        epilogue_chunk<kAct>(a, v0, r0, cb, n0, row_valid, yrow, has_res, s_bias);
         if (!second) break;
         tcgen05_wait_ld();
         if (cb + 32 < a.BN) {
             tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
             load_residual(a, n0 + cb + 32, row_valid, rrow, r0);
         }
-        epilogue_chunk(a, v1, r1, cb + 16, n0, row_valid, yrow, has_res, s_bias);
+        epilogue_chunk<kAct>(a, v1, r1, cb + 16, n0, row_valid, yrow, has_res, s_bias);
     }
 }
 
@@ -463,7 +474,8 @@ __device__ __forceinline__ void epilogue_columns(const EpiArgs& a, uint32_t lane
 // result, and one lane of a warp stores the warp's 32 rows of a finished box with one instruction.  `buf`: 128 x BN x 2 bytes
 // of the pipeline memory, free by now.  publish: this launch reports to the host, so the stores have to be in memory when the
 // warp leaves; otherwise they only have to have been read (the next kernel waits for this one's memory operations).
-__device__ __forceinline__ void epilogue_columns_tma(const EpiArgs& a, uint32_t lane_addr, int n0, bool has_res, const float* s_bias, uint32_t buf,
+template <int kAct, class Args>
+__device__ __forceinline__ void epilogue_columns_tma(const Args& a, uint32_t lane_addr, int n0, bool has_res, const float* s_bias, uint32_t buf,
                                                      const CUtensorMap* tmap_y, int m0, bool publish) {
     const uint32_t r = threadIdx.x;                 // tile row
     const int U = a.out_box, m_warp = m0 + (int)(r & ~31u);
@@ -477,8 +489,8 @@ __device__ __forceinline__ void epilogue_columns_tma(const EpiArgs& a, uint32_t 
         const uint32_t at0 = row + box + (((uint32_t)(in_box >> 3) ^ swz) << 4), at1 = row + box + ((((uint32_t)(in_box >> 3) + 1u) ^ swz) << 4);
         uint4 res0 = make_uint4(0, 0, 0, 0), res1 = res0;
         if (has_res) { res0 = ld_shared_v4(at0); res1 = ld_shared_v4(at1); }
-        const uint4 o0 = finish8(a, v, res0, has_res, n0 + cb, s_bias + cb);
-        const uint4 o1 = finish8(a, v + 8, res1, has_res, n0 + cb + 8, s_bias + cb + 8);
+        const uint4 o0 = finish8<kAct>(a, v, res0, has_res, n0 + cb, s_bias + cb);
+        const uint4 o1 = finish8<kAct>(a, v + 8, res1, has_res, n0 + cb + 8, s_bias + cb + 8);
         st_shared_v4(at0, o0.x, o0.y, o0.z, o0.w);
         st_shared_v4(at1, o1.x, o1.y, o1.z, o1.w);
         if (in_box + 16 == U) {
@@ -509,10 +521,11 @@ __device__ __forceinline__ void epilogue_columns_tma(const EpiArgs& a, uint32_t 
 // Epilogue, run by warps 0-3 (thread t owns accumulator lane t = tile row t): wait for the
 // accumulator, then bias + residual + activation and bf16 stores into the output channel slice.
 // tmap_y (the one-tile kernels): through TMA stores staged at `buf`.
-__device__ __forceinline__ void epilogue(const ConvArgs& args, uint32_t tmem_base, bool ok, int m0, int n0, const float* s_bias,
+// kByAct: a copy of the column loops for either kind of activation.
+template <bool kByAct, class Args>
+__device__ __forceinline__ void epilogue(const Args& a, uint32_t tmem_base, bool ok, int m0, int n0, const float* s_bias,
                                          uint64_t* s_accum_p, volatile uint32_t* s_abort_p, uint32_t accum_parity = 0u,
                                          const CUtensorMap* tmap_y = nullptr, uint32_t buf = 0, uint64_t* s_res = nullptr, bool publish = true) {
-    const EpiArgs a = epi_args(args);
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int m = m0 + tid;
@@ -526,12 +539,16 @@ __device__ __forceinline__ void epilogue(const ConvArgs& args, uint32_t tmem_bas
     if (tmap_y) {
         const bool has_res = a.residual != nullptr;
         if (has_res && !__all_sync(0xffffffffu, mbar_wait(smem_u32(s_res), 0u, s_abort_p, a.err_flag, 6u))) return;
-        epilogue_columns_tma(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        if constexpr (!kByAct) epilogue_columns_tma<0>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        else if (a.act == 1 || a.act == 2) epilogue_columns_tma<1>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
+        else epilogue_columns_tma<2>(a, lane_addr, n0, has_res, s_bias, buf, tmap_y, m0, publish);
         return;
     }
     const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
     __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
-    epilogue_columns(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    if constexpr (!kByAct) epilogue_columns<0>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    else if (a.act == 1 || a.act == 2) epilogue_columns<1>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
+    else epilogue_columns<2>(a, lane_addr, n0, row_valid, yrow, rrow, s_bias);
 }
 
 // ---- split reduction: the thread blocks of a cluster share one output tile -----------------------------------
@@ -545,7 +562,8 @@ __device__ __forceinline__ void epilogue(const ConvArgs& args, uint32_t tmem_bas
 // (The partial tiles used to meet in a global workspace under an atomic counter: two fences, an atomic and an L2
 // round trip of BN x 512 bytes per rank, read back by ONE block: +4 to +8 us per launch, so only reductions of 60
 // and more k-blocks gained from it.)
-__device__ __forceinline__ void cluster_finish(const EpiArgs& a, int n0, bool row_valid, __nv_bfloat16* yrow,
+template <int kAct, class Args>
+__device__ __forceinline__ void cluster_finish(const Args& a, int n0, bool row_valid, __nv_bfloat16* yrow,
                                                const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
     const int S = a.splits;
     uint32_t active = (1u << S) - 1u;      // ranks that have k-blocks (all of them unless a grouped launch splits a short reduction)
@@ -601,15 +619,15 @@ __device__ __forceinline__ void cluster_finish(const EpiArgs& a, int n0, bool ro
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(sum[o][j]));
-            *reinterpret_cast<uint4*>(yrow + k) = finish8(a, v, res, rrow != nullptr, k, s_bias + col);
+            *reinterpret_cast<uint4*>(yrow + k) = finish8<kAct>(a, v, res, rrow != nullptr, k, s_bias + col);
         }
     }
 }
 
 // Run by warps 0-3 of every rank.  `mine`: this rank has k-blocks of its own.
-__device__ __forceinline__ void epilogue_cluster(const ConvArgs& args, uint32_t tmem_base, int m0, int n0, int rank, bool mine, uint32_t smem_base,
+template <bool kByAct, class Args>
+__device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_base, int m0, int n0, int rank, bool mine, uint32_t smem_base,
                                                  const float* s_bias, uint64_t* s_accum_p, volatile uint32_t* s_abort_p) {
-    const EpiArgs a = epi_args(args);
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int m = m0 + tid;
@@ -644,7 +662,9 @@ __device__ __forceinline__ void epilogue_cluster(const ConvArgs& args, uint32_t 
     if (ok) {
         __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
         const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
-        cluster_finish(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        if constexpr (!kByAct) cluster_finish<0>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        else if (a.act == 1 || a.act == 2) cluster_finish<1>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        else cluster_finish<2>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
     }
     cluster_arrive_relaxed();
     cluster_wait();                 // every rank has read what it needs: shared memory may go
@@ -776,7 +796,7 @@ conv_umma_gather_kernel(const __grid_constant__ CUtensorMap tmap_w, const ConvAr
             for (int kb = (nkb > kLag ? nkb - kLag : 0); kb < nkb; ++kb) mbar_arrive(smem_u32(&s_full[kb % kStages]));
 
         // ===== epilogue: accumulator lane `tid` = tile row `tid` =====
-        epilogue(a, tmem_base, ok, m0, n0, s_bias, &s_accum, &s_abort);
+        epilogue<true>(a, tmem_base, ok, m0, n0, s_bias, &s_accum, &s_abort);
         if (tid == 0) PB_T(6);
     } else {
         // ===== MMA issuer: one thread =====
@@ -911,7 +931,8 @@ __device__ __forceinline__ void normalise_stages(const ConvArgs& a, uint32_t sme
 // One CTA's share of one convolution: output tile (bx, by), rank bz of the cluster that shares the tile's
 // reduction, `stages` pipeline buffers.  Shared by the single-convolution kernel and the grouped one.
 // kPre: the tile's input is normalised first (see above; a kernel of its own: the others' code and registers stay as they are).
-template <bool kPre>
+// kLone: the launch has this convolution only and does not normalise.
+template <bool kPre, bool kLone>
 __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const CUtensorMap* tmap_x, const CUtensorMap* tmap_y, const CUtensorMap* tmap_r,
                                               const CUtensorMap* tmap_n, const ConvArgs& a, const int stages,
                                               const int bx, const int by, const int bz, uint8_t* smem_raw,
@@ -1031,8 +1052,13 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         griddep_wait();
         if (tid == 0) PB_S(2);
         griddep_launch();
-        if (a.splits > 1) epilogue_cluster(a, tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
-        else epilogue(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
+        if constexpr (kLone) {
+            if (a.splits > 1) epilogue_cluster<true>(a, tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
+            else epilogue<true>(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
+        } else {
+            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
+            else epilogue<false>(epi_args(a), tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
+        }
         if (tid == 0) { PB_T(6); PB_S(6); }
     } else if (warp == 4) {
         // ===== operand A =====
@@ -1204,7 +1230,7 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     resolve_slot(job_id, nf);
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
-    conv_tile_tma<false>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, nullptr, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+    conv_tile_tma<false, true>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, nullptr, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
                          &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
     if (nf) nf->end(job_id);
 }
@@ -1227,7 +1253,7 @@ conv_umma_pre_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     resolve_slot(job_id, nf);
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
-    conv_tile_tma<true>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, &tmap_n, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
+    conv_tile_tma<true, false>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, &tmap_n, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
                         &s_tmem_base, &s_abort, s_bias, &s_res, s_ready, nf != nullptr);
     if (nf) nf->end(job_id);
 }
@@ -1345,7 +1371,7 @@ conv_umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         asm volatile("bar.sync 1, 128;" ::: "memory");
         griddep_wait();
         griddep_launch();
-        epilogue(a, tmem_base, true, m0, n0, s_bias, &s_accum, &s_abort, 0u, a.out_box ? &tmap_y : nullptr, smem_base, &s_res, nf != nullptr);
+        epilogue<true>(a, tmem_base, true, m0, n0, s_bias, &s_accum, &s_abort, 0u, a.out_box ? &tmap_y : nullptr, smem_base, &s_res, nf != nullptr);
     } else if (warp == 4) {
         // ===== operand A: this block's 128 rows =====
         griddep_wait();
@@ -1574,7 +1600,7 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     const uint32_t S = (uint32_t)s_args.splits, gx = sc->gx;
     const uint32_t tile = local / S, bz = local - tile * S;
     const uint32_t by = tile / gx, bx = tile - by * gx;
-    conv_tile_tma<false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, nullptr, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
+    conv_tile_tma<false, false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, nullptr, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
                   &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
     if (nf) nf->end(job_id);
 }
@@ -1714,7 +1740,7 @@ conv_umma_persist_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t 
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (tid == 0) PB_PT(i, 2);
-            epilogue(a, tmem_base + acc * acc_cols, true, tr.bx * kBM, n0, s_bias[acc], &s_tfull[acc], &s_abort, use & 1u);
+            epilogue<false>(epi_args(a), tmem_base + acc * acc_cols, true, tr.bx * kBM, n0, s_bias[acc], &s_tfull[acc], &s_abort, use & 1u);
             if (tid == 0) PB_PT(i, 3);
             // this accumulator may be overwritten: every tcgen05.ld of the warp has completed (wait::ld)
             tcgen05_fence_before();

@@ -1053,7 +1053,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         if (tid == 0) PB_S(2);
         griddep_launch();
         if constexpr (kLone) {
-            if (a.splits > 1) epilogue_cluster<true>(a, tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
+            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
             else epilogue<true>(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
         } else {
             if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);

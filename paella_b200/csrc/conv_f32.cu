@@ -3,8 +3,8 @@
 //   D[m, n] = sum_k A[m, k] * B[k, n]     m = output pixel (all images back to back), n = output channel,
 //                                          k = (r*S + s)*Cs + c   (filter tap, input channel)
 //
-// No tensor-core format keeps fp32 inputs, so the ceiling is the fused multiply-add rate: 148 SMs x 128 x 2 x 1.9 GHz =
-// 72 TFLOP/s.  The direct kernel this replaces for dense layers (conv_simt_kernel: one output per thread, every operand
+// The layers that conv_f32_umma.cu leaves: few input channels, narrow 1x1 layers, unaligned tensors, output sizes of the caller's own.
+// The ceiling is the fused multiply-add rate: 148 SMs x 128 x 2 x 1.9 GHz = 72 TFLOP/s.  The direct kernel this replaces for dense layers (conv_simt_kernel: one output per thread, every operand
 // through L1 for each multiplication) ran at 1.9 TFLOP/s.
 //
 // Block = 256 threads on a tile of 64 pixels x BN channels.  A stage is 32 values of k, three stages deep, brought by
@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "conv_f32.h"
 #include "launch_slot.cuh"
 #include "ops.h"
 #include "pb_common.h"
@@ -345,6 +346,7 @@ int conv_f32_info(const pb_op_params* p, pb_launch_info* out) {
     if (cudaFuncGetAttributes(&at, g.fn) == cudaSuccess) out->regs_per_thread = (uint32_t)at.numRegs;
     else cudaGetLastError();
     out->smem_per_block = g.smem;
+    if (conv_f32_split_takes(p)) conv_f32_split_info(p, out);
     const uint64_t nb = (uint64_t)batch_of(p), y = nb * p->K * p->P * p->Q;
     out->flops = 2ull * y * p->C * p->R * p->S;
     out->bytes = 4ull * (nb * p->C * p->H * p->W + (uint64_t)p->K * p->C * p->R * p->S + y + (p->residual ? y : 0)) + 4ull * p->K;
@@ -352,6 +354,7 @@ int conv_f32_info(const pb_op_params* p, pb_launch_info* out) {
 }
 
 int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl) {
+    if (conv_f32_split_takes(p)) return conv_f32_split_launch(p, op, st, job_id, notifier, pdl);
     const F32Geometry g = conv_f32_geometry(p);
     F32Args f;
     f.op = op;

@@ -1,0 +1,680 @@
+// Dense fp32 convolution on the tensor cores, without giving up a bit of fp32: an implicit GEMM of operands that are split into three
+// bf16 parts each.
+//
+//   D[m, n] = sum_k A[m, k] * B[k, n]     m = output pixel (all images back to back), n = output channel,
+//                                          k = (tap, input channel), taps of 32-channel chunks
+//
+// A = a0 + a1 + a2 and B = b0 + b1 + b2 exactly (8 bits of mantissa each, rounded to nearest, so 24 and the signs), and of the nine
+// products the six of weight 2^-18 and more are multiplied: what is left out is 2^-26 of a product at most and has no preferred sign.
+// Products of bf16 values are exact in fp32.  The tensor core's own additions do not round to nearest, so its sums are kept
+// short: an accumulator holds 64 values of k, and the products a0 b0 have one of their own, apart from the five small ones (whose
+// roundings are 2^-8 of theirs).  After every 64 k both are read from tensor memory and added to the sums in registers, which are
+// ordinary fp32.
+//
+// Block = 26 warps on a tile of 128 pixels x BN channels, in steps of 64 k:
+//   warp 24      copies, three or four steps ahead: two im2col boxes of 128 pixels x 32 channels and two of 32 x BN weights, fp32
+//   warps 8-15   split them: a thread has one box of a pixel, and leaves its three rows of bf16 in TENSOR memory, from where the tensor core
+//                takes operand A (shared memory then moves operand B only: six multiplications per 16 k read 6 x 2 KB there, not 6 x 6 KB)
+//   warps 16-23  split the weights, into shared memory
+//   warp 25      multiplies: 4 x 6 instructions of 128 x BN x 16 a step
+//   warps 0-7    add up, half of the columns each, and finish the tile: bias, residual, activation
+// Tensor memory: two steps of operand A (192 columns) and two pairs of accumulators (4 BN).  A layer with few tiles splits its k range over
+// the blocks of a cluster, whose sums meet through distributed shared memory, in rank order: results do not depend on timing.
+//
+// Bound by the instructions of the splitting warps (about 1250 issue slots a scheduler and step) and, where a launch has few steps, by the
+// latency of a step's chain: 0.74 us at 64 columns, 0.66 at 32.  Measured against the kernel on the fp32 units, us a launch in a chain:
+// 64 -> 64 3x3 on 2 maps of 56 x 56 23.1 -> 9.3, 128 -> 128 on 2 of 28 x 28 21.7 -> 10.1, 512 -> 512 on 2 of 7 x 7 29.2 -> 13.0, 256 -> 256 on 16 of
+// 28 x 28 408 -> 98 (151 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 235.  Error against 64 bits, relative, fp32 units / here:
+// 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
+//
+// Infinities, NaN and values that round to infinity in bf16 make 0 x inf of the parts: an output that is not finite is computed again,
+// as a plain fp32 sum.
+//
+// This is the fp32 member of the kernel family the reference's TVM adapters launch
+// (jobs/tvm_<model>/tvm_<model>.cpp:24-47; generated fp32 kernels there).
+#include <cuda.h>
+#include <llis/job/finished_block_notifier.h>
+
+#include <algorithm>
+#include <cfloat>
+#include <cstdlib>
+#include <type_traits>
+
+#include "conv_f32.h"
+#include "launch_slot.cuh"
+#include "ops.h"
+#include "pb_common.h"
+#include "umma.cuh"
+
+using llis::job::FinishedBlockNotifier;
+
+namespace pb {
+
+__device__ uint32_t g_f32_err_flag;      // raised when a bounded wait runs out
+
+namespace {
+
+constexpr int kRows = 128, kChunk = 32;             // pixels of a tile, channels of a copy box
+constexpr int kMaxRing = 4;
+constexpr uint32_t kBox = kRows * kChunk * 4;       // 16 KB
+constexpr int kWarpA = 8, kWarpB = 16, kWarpCopy = 24, kWarpMma = 25;
+constexpr int kThreadsF = 26 * 32;
+constexpr uint32_t kTmemCols = 512;
+
+struct SplitArgs {
+    OpArgs op;
+    int M, PQ, Kp;       // rows of the GEMM, pixels per image, channels of a row of packed weights
+    int cpt, chunks;     // chunks of 32 channels per tap, and of the whole reduction
+    int splits;          // cluster size
+    int a_tiled;         // pointwise: operand A is a plain matrix
+};
+
+// Shared memory: the ring of raw operands (two boxes of pixels, two of weights a step), the split weights of two steps, and where the sums
+// of a tile meet.  Tensor memory columns: accumulators [buffer][large, small][BN], then operand A [step][part][32].
+template <int BN>
+struct Layout {
+    static constexpr uint32_t ring = BN == 64 ? 3 : 4;
+    static constexpr uint32_t raw_w = 2 * kBox, w_box = kChunk * BN * 4, stage = raw_w + 2 * w_box;
+    static constexpr uint32_t part = BN * 128, parts = ring * stage, parts_step = 3 * part;
+    static constexpr uint32_t meet = parts + 2 * parts_step, bytes = meet + kRows * BN * 4;
+    static constexpr uint32_t acc = 0, a = 4 * BN;
+};
+
+__device__ __forceinline__ void mma_ta(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void tcgen05_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ uint64_t sub_f32x2(uint64_t x, uint64_t y) {
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
+// 16 bytes into another block's shared memory, counted by its barrier.
+__device__ __forceinline__ void st_async_v4(uint32_t addr, const float4& v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void tcgen05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Two values to three pairs of bf16 that add up to them (the first in the low halves).
+__device__ __forceinline__ void split2(uint32_t x0, uint32_t x1, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    uint64_t v = pack_f32x2(x0, x1);
+    float lo = __uint_as_float(x0), hi = __uint_as_float(x1);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p0) : "f"(hi), "f"(lo));
+    v = sub_f32x2(v, pack_f32x2(p0 << 16, p0 & 0xffff0000u));
+    unpack_f32x2(v, lo, hi);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(hi), "f"(lo));
+    v = sub_f32x2(v, pack_f32x2(p1 << 16, p1 & 0xffff0000u));
+    unpack_f32x2(v, lo, hi);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(hi), "f"(lo));
+}
+
+// One output as a plain fp32 sum.
+__device__ __forceinline__ float plain_dot(const SplitArgs& f, int m, int k) {
+    const OpArgs& a = f.op;
+    const int img = m / f.PQ, pix = m - img * f.PQ, p = pix / a.Q, q = pix - p * a.Q;
+    float sum = 0.f;
+    for (int r = 0; r < a.R; ++r)
+        for (int s = 0; s < a.S; ++s) {
+            const int ih = p * a.stride_h - a.pad_h + r * a.dil_h, iw = q * a.stride_w - a.pad_w + s * a.dil_w;
+            if (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) continue;
+            const float* x = static_cast<const float*>(a.x) + (((size_t)img * a.H + ih) * a.W + iw) * a.Cs;
+            const float* w = static_cast<const float*>(a.w) + (size_t)(r * a.S + s) * a.Cs * f.Kp + k;
+            for (int c = 0; c < a.C; ++c) sum = fmaf(x[c], w[(size_t)c * f.Kp], sum);
+        }
+    return sum;
+}
+
+__device__ __forceinline__ bool finite4(const float4& v) {
+    return (fabsf(v.x) <= FLT_MAX) & (fabsf(v.y) <= FLT_MAX) & (fabsf(v.z) <= FLT_MAX) & (fabsf(v.w) <= FLT_MAX);
+}
+// Four outputs of row m, from channel k on: bias, residual, activation, whatever the alignment.
+__device__ __forceinline__ void finish4(const OpArgs& a, int m, int k, float4 v, const float4& b, const float4& s, bool vec, bool vec_r) {
+    v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+    if (a.residual) {
+        const float* res = static_cast<const float*>(a.residual) + (size_t)m * a.res_Cs + k;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vec_r && k + 4 <= a.K) q = *reinterpret_cast<const float4*>(res);
+        else {
+            q.x = res[0];
+            if (k + 1 < a.K) q.y = res[1];
+            if (k + 2 < a.K) q.z = res[2];
+            if (k + 3 < a.K) q.w = res[3];
+        }
+        v = make_float4(v.x + q.x, v.y + q.y, v.z + q.z, v.w + q.w);
+    }
+    if (a.act == 3) {           // PReLU
+        v = make_float4(v.x > 0.f ? v.x : v.x * s.x, v.y > 0.f ? v.y : v.y * s.y, v.z > 0.f ? v.z : v.z * s.z, v.w > 0.f ? v.w : v.w * s.w);
+    } else if (a.act == 1 || a.act == 2) {
+        v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+        if (a.act == 2) v = make_float4(fminf(v.x, 6.f), fminf(v.y, 6.f), fminf(v.z, 6.f), fminf(v.w, 6.f));
+    }
+    float* y = static_cast<float*>(a.y) + (size_t)m * a.Ks + a.out_c_off + k;
+    if (vec && k + 4 <= a.K) {
+        *reinterpret_cast<float4*>(y) = v;
+    } else {
+        y[0] = v.x;
+        if (k + 1 < a.K) y[1] = v.y;
+        if (k + 2 < a.K) y[2] = v.z;
+        if (k + 3 < a.K) y[3] = v.w;
+    }
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kThreadsF, 1)
+conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ SplitArgs f, uint32_t job_id, FinishedBlockNotifier* nf) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t s_full[kMaxRing], s_empty[kMaxRing];      // raw operands
+    __shared__ __align__(8) uint64_t s_ready[2], s_done[2], s_free[2];   // operands split; multiplied; accumulators read
+    __shared__ __align__(8) uint64_t s_sums;                             // the other ranks' sums have arrived
+    __shared__ uint32_t s_tmem_base;
+    __shared__ volatile uint32_t s_abort;
+    __shared__ __align__(16) float s_bias[BN], s_slope[BN];
+    using L = Layout<BN>;
+
+    resolve_slot(job_id, nf);
+    if (nf) nf->start(job_id);
+    const OpArgs& a = f.op;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = (int)uniform((uint32_t)tid >> 5);
+    const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int m0 = (int)blockIdx.x * kRows, n0 = (int)blockIdx.y * BN, rank = (int)blockIdx.z;
+    const int steps = (f.chunks + 1) / 2;                          // of 64 k
+    const int kb0 = steps * rank / f.splits, n_kb = steps * (rank + 1) / f.splits - kb0;
+    constexpr uint32_t ring = L::ring;
+    uint32_t* const err = &g_f32_err_flag;
+
+    if (warp == kWarpCopy) {
+        if (elect_one()) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+            for (uint32_t i = 0; i < ring; ++i) {
+                mbar_init(smem_u32(&s_full[i]), 1);
+                mbar_init(smem_u32(&s_empty[i]), 16);
+            }
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(smem_u32(&s_ready[i]), 16);
+                mbar_init(smem_u32(&s_done[i]), 1);
+                mbar_init(smem_u32(&s_free[i]), 8);
+            }
+            mbar_init(smem_u32(&s_sums), 1);
+            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(&s_sums), (uint32_t)((f.splits - 1) * (kRows / f.splits) * BN * 4));
+            s_abort = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            fence_proxy_async();
+        }
+        __syncwarp();
+    }
+    if (warp == kWarpMma) {
+        tcgen05_alloc(smem_u32(&s_tmem_base), kTmemCols);
+        tcgen05_relinquish();
+    }
+    // Where the tile's pixels and this rank's k begin (worked out before the previous launch has to be waited for).
+    int c_chunk = 2 * kb0, c_tap = c_chunk / f.cpt, c_c = c_chunk - c_tap * f.cpt, c_r = 0, c_s = 0, img = 0, w_org = 0, h_org = 0;
+    if (warp == kWarpCopy) {
+        c_r = c_tap / a.S;
+        c_s = c_tap - c_r * a.S;
+        img = m0 / f.PQ;
+        const int rem = m0 - img * f.PQ, p = rem / a.Q, q = rem - p * a.Q;
+        w_org = q * a.stride_w - a.pad_w;
+        h_org = p * a.stride_h - a.pad_h;
+    }
+    // The weights are constants: those of the first steps are on their way before the previous launch has to be waited for.  (A stage's barrier
+    // is armed with the bytes of both operands.)
+    auto copy_weights = [&](int kb, uint32_t st, int chunk, int& tap, int& cc) {
+        const int have = min(2, f.chunks - chunk);
+        const uint32_t bar = smem_u32(&s_full[st]), to = smem + st * L::stage + L::raw_w;
+        if (elect_one()) mbar_arrive_expect_tx(bar, (uint32_t)have * (kBox + L::w_box));
+        for (int h = 0; h < have; ++h) {
+            if (elect_one()) tma_load_3d(to + (uint32_t)h * L::w_box, &tmap_w, n0, cc * kChunk, tap, bar);
+            __syncwarp();
+            if (++cc == f.cpt) { cc = 0; ++tap; }
+        }
+    };
+    int w_tap = c_tap, w_c = c_c, w_ahead = min((int)ring, n_kb);
+    if (warp == kWarpCopy)
+        for (int kb = 0; kb < w_ahead; ++kb) copy_weights(kb, (uint32_t)kb, c_chunk + 2 * kb, w_tap, w_c);
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    if (f.splits > 1) cluster_arrive();        // the sums' barrier is set up (the one wait for it: where sums are sent)
+    const uint32_t tmem = uniform(s_tmem_base);
+
+    if (warp >= kWarpA) griddep_launch();       // the next launch's blocks may have the SMs that this one leaves idle
+    if (warp < kWarpA) {
+        // ===== sums =====
+        griddep_wait();
+        griddep_launch();
+        constexpr int kCols = BN / 2;                  // of this thread, of one row
+        const int row = tid & 127, col0 = (tid >> 7) * kCols;
+        if (tid < BN) {
+            const int k = n0 + tid;
+            s_bias[tid] = a.bias && k < a.K ? __ldg(a.bias + k) : 0.f;
+            s_slope[tid] = a.act == 3 && k < a.K ? __ldg(a.bias + a.K + k) : 0.f;      // the slopes follow the biases
+        }
+        uint64_t acc[kCols / 2];
+#pragma unroll
+        for (int j = 0; j < kCols / 2; ++j) acc[j] = 0;
+        const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + L::acc + (uint32_t)col0;
+        bool ok = true;
+        for (int kb = 0; kb < n_kb; ++kb) {
+            const int t = kb & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_done[t]), (uint32_t)(kb >> 1) & 1u, &s_abort, err, 0x21u));
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t d = lanes + (uint32_t)(t * 2 * BN);
+#pragma unroll
+            for (int c = 0; c < kCols; c += 16) {
+                uint32_t big[16], small[16];
+                tcgen05_ld16(d + (uint32_t)c, big);
+                tcgen05_ld16(d + (uint32_t)(BN + c), small);
+                tcgen05_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 16; j += 2)
+                    acc[(c + j) / 2] = add_f32x2(acc[(c + j) / 2], add_f32x2(pack_f32x2(big[j], big[j + 1]), pack_f32x2(small[j], small[j + 1])));
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (elect_one()) mbar_arrive(smem_u32(&s_free[t]));
+            __syncwarp();
+        }
+        // Rank z finishes rows [z, z + 1) x 128 / splits of the tile: every rank sends it its sums (st.async: the sums go from registers into the
+        // owner's shared memory and count on its barrier), laid out as [rank][row][channel], 16-byte chunks in an order that keeps both the
+        // writers (a row each) and the readers (a chunk each) free of bank conflicts.
+        const uint32_t meet = smem + L::meet;
+        const int share = kRows / f.splits;
+        {
+            const int owner = row / share, rl = row - owner * share;
+            const uint32_t at = meet + (uint32_t)((rank * share + rl) * (BN * 4)), mix = (uint32_t)rl & 7u;
+            uint32_t to = at, bar = 0;
+            if (f.splits > 1) {
+                cluster_wait();                 // every block of the cluster is running
+                to = cluster_addr(at, (uint32_t)owner);
+                bar = cluster_addr(smem_u32(&s_sums), (uint32_t)owner);
+            }
+#pragma unroll
+            for (int c = 0; c < kCols; c += 4) {
+                float4 v;
+                unpack_f32x2(acc[c / 2], v.x, v.y);
+                unpack_f32x2(acc[c / 2 + 1], v.z, v.w);
+                const uint32_t off = (((uint32_t)(col0 + c) >> 2) ^ mix) << 4;
+                if (owner == rank) st_shared_v4(at + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+                else st_async_v4(to + off, v, bar);
+            }
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (f.splits > 1) {       // (also when this block gives up: it stays until the others have written to it)
+            bool here = false;
+            for (uint32_t i = 0; i < kWaitLimit && !here; ++i) here = mbar_try_wait(smem_u32(&s_sums), 0u);
+            if (!here) atomicExch(err, 0x28u);
+            ok = __all_sync(0xffffffffu, here) && ok;
+        }
+        if (ok) {
+            const bool vec = ((a.Ks | a.out_c_off) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
+            const bool vec_r = (a.res_Cs & 3) == 0 && (reinterpret_cast<uintptr_t>(a.residual) & 15) == 0;
+            // this rank's share of the tile's rows; a thread has four columns of every kStepR-th
+            constexpr int kStepR = 256 / (BN / 4);
+            const int r1 = min(share, f.M - m0 - rank * share), c = tid % (BN / 4) * 4, k = n0 + c, m_share = m0 + rank * share;
+            int r = tid / (BN / 4);                             // in the share
+            auto sum4 = [&](int row) {
+                const uint32_t at = meet + (uint32_t)row * (BN * 4) + ((((uint32_t)c >> 2) ^ ((uint32_t)row & 7u)) << 4);
+                uint4 q = ld_shared_v4(at);
+                float4 v = make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w));
+#pragma unroll 1
+                for (int z = 1; z < f.splits; ++z) {             // in rank order
+                    q = ld_shared_v4(at + (uint32_t)(z * share) * (BN * 4));
+                    v = make_float4(v.x + __uint_as_float(q.x), v.y + __uint_as_float(q.y), v.z + __uint_as_float(q.z), v.w + __uint_as_float(q.w));
+                }
+                return v;
+            };
+            const float4 bias = *reinterpret_cast<const float4*>(s_bias + c), slope = *reinterpret_cast<const float4*>(s_slope + c);
+            // Row by row, whatever the alignment and the activation, and with values that are not finite.
+            auto any_row = [&](int row) {
+                float4 x = sum4(row);
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {      // one of the four at a time, in x.x
+                    if (!(fabsf(x.x) <= FLT_MAX) && k + j < a.K) x.x = plain_dot(f, m_share + row, k + j);
+                    x = make_float4(x.y, x.z, x.w, x.x);
+                }
+                finish4(a, m_share + row, k, x, bias, slope, vec, vec_r);
+            };
+            // Branches cost a lone warp more than the arithmetic: rows four at a time, their loads together, nothing left to decide.
+            auto rows4 = [&](auto with_residual, auto with_clamp) {
+                constexpr bool residual = decltype(with_residual)::value, clamp = decltype(with_clamp)::value;
+                const float top = a.act == 2 ? 6.f : INFINITY;
+                const float* res = static_cast<const float*>(a.residual) + (size_t)(m_share + r) * a.res_Cs + k;
+                float* y = static_cast<float*>(a.y) + (size_t)(m_share + r) * a.Ks + a.out_c_off + k;
+#pragma unroll 1
+                for (; r < r1; r += 4 * kStepR) {
+                    float4 v[4], q[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (residual && r + u * kStepR < r1) q[u] = *reinterpret_cast<const float4*>(res + (size_t)(u * kStepR) * a.res_Cs);
+                    bool plain = false;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (r + u * kStepR < r1) v[u] = sum4(r + u * kStepR);
+                        plain = plain | !finite4(v[u]);
+                    }
+                    if (plain) {
+#pragma unroll 1
+                        for (int u = 0; u < 4; ++u)
+                            if (r + u * kStepR < r1) any_row(r + u * kStepR);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            float4 x = make_float4(v[u].x + bias.x, v[u].y + bias.y, v[u].z + bias.z, v[u].w + bias.w);
+                            if (residual) x = make_float4(x.x + q[u].x, x.y + q[u].y, x.z + q[u].z, x.w + q[u].w);
+                            if (clamp) x = make_float4(fminf(fmaxf(x.x, 0.f), top), fminf(fmaxf(x.y, 0.f), top), fminf(fmaxf(x.z, 0.f), top), fminf(fmaxf(x.w, 0.f), top));
+                            if (r + u * kStepR < r1) *reinterpret_cast<float4*>(y + (size_t)(u * kStepR) * a.Ks) = x;
+                        }
+                    }
+                    res += (size_t)(4 * kStepR) * a.res_Cs;
+                    y += (size_t)(4 * kStepR) * a.Ks;
+                }
+            };
+            const bool has_res = a.residual != nullptr;
+            if (k >= a.K) {
+            } else if (!vec || (has_res && !vec_r) || k + 4 > a.K || a.act == 3) {
+#pragma unroll 1
+                for (; r < r1; r += kStepR) any_row(r);
+            } else if (a.act == 1 || a.act == 2) {
+                if (has_res) rows4(std::true_type{}, std::true_type{});
+                else rows4(std::false_type{}, std::true_type{});
+            } else {
+                if (has_res) rows4(std::true_type{}, std::false_type{});
+                else rows4(std::false_type{}, std::false_type{});
+            }
+        }
+    } else if (warp < kWarpB) {
+        // ===== pixels to three parts, in tensor memory =====
+        const uint32_t row = (uint32_t)tid & 127u, swz = row & 7u;
+        const int h = (warp >> 2) & 1;                             // this thread's box
+        const uint32_t at0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + L::a + (uint32_t)(h * 16);
+        uint32_t st = 0, parity = 0;
+        for (int kb = 0; kb < n_kb; ++kb) {
+            const int t = kb & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err, 0x22u))) break;
+            const bool have = 2 * (kb0 + kb) + h < f.chunks;       // an odd number of chunks ends with half a step
+            const uint32_t from = smem + st * L::stage + (uint32_t)h * kBox + row * 128u;
+            uint4 v[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = ld_shared_v4(from + (((uint32_t)c ^ swz) << 4));      // (without a second box: not used)
+            bool ok = true;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                uint32_t p[3][8];
+                if (have) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint4& x = v[q * 4 + c];
+                        split2(x.x, x.y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
+                        split2(x.z, x.w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) p[0][c] = p[1][c] = p[2][c] = 0u;
+                }
+                if (q == 0 && kb >= 2) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_done[t]), (uint32_t)((kb >> 1) - 1) & 1u, &s_abort, err, 0x23u));
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) tcgen05_st8(at0 + (uint32_t)(t * 96 + i * 32 + q * 8), p[i]);
+            }
+            if (!ok) break;
+            tcgen05_wait_st();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (elect_one()) {
+                mbar_arrive(smem_u32(&s_ready[t]));
+                mbar_arrive(smem_u32(&s_empty[st]));
+            }
+            __syncwarp();
+            if (++st == ring) { st = 0; parity ^= 1u; }
+        }
+    } else if (warp < kWarpCopy) {
+        // ===== weights to three parts, in shared memory: eight k of one channel at a time, lanes along the channels =====
+        const int bw = warp - kWarpB, n = lane + (BN == 64 ? 32 * (bw & 1) : 0), kg0 = BN == 64 ? bw >> 1 : bw;
+        constexpr int kTasks = BN == 64 ? 2 : 1;
+        uint32_t st = 0, parity = 0;
+        for (int kb = 0; kb < n_kb; ++kb) {
+            const int t = kb & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err, 0x29u))) break;
+            uint32_t p[kTasks][3][4];
+            uint32_t v[kTasks][8];
+#pragma unroll
+            for (int j = 0; j < kTasks; ++j) {
+                const uint32_t from = smem + st * L::stage + L::raw_w + (uint32_t)((kg0 + 4 * j) * 8 * BN + n) * 4u;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v[j][i]) : "r"(from + (uint32_t)(i * BN) * 4u) : "memory");
+            }
+#pragma unroll
+            for (int j = 0; j < kTasks; ++j) {
+                if (2 * (kb0 + kb) + ((kg0 + 4 * j) >> 2) < f.chunks) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) split2(v[j][2 * i], v[j][2 * i + 1], p[j][0][i], p[j][1][i], p[j][2][i]);
+                } else {      // (no second box)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) p[j][0][i] = p[j][1][i] = p[j][2][i] = 0u;
+                }
+            }
+            if (kb >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_done[t]), (uint32_t)((kb >> 1) - 1) & 1u, &s_abort, err, 0x24u))) break;
+            const uint32_t to = smem + L::parts + (uint32_t)t * L::parts_step + (uint32_t)n * 128u;
+#pragma unroll
+            for (int j = 0; j < kTasks; ++j)
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    st_shared_v4(to + (uint32_t)q * L::part + ((uint32_t)((kg0 + 4 * j) ^ (n & 7)) << 4), p[j][q][0], p[j][q][1], p[j][q][2], p[j][q][3]);
+            fence_proxy_async();
+            __syncwarp();
+            if (elect_one()) {
+                mbar_arrive(smem_u32(&s_ready[t]));
+                mbar_arrive(smem_u32(&s_empty[st]));
+            }
+            __syncwarp();
+            if (++st == ring) { st = 0; parity ^= 1u; }
+        }
+    } else if (warp == kWarpCopy) {
+        // ===== copies =====
+        griddep_wait();                            // the pixels are the previous launch's
+        int r = c_r, s = c_s, c = c_c, chunk = c_chunk;
+        uint32_t st = 0, parity = 1u;
+        for (int kb = 0; kb < n_kb; ++kb) {
+            if (kb >= (int)ring) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, &s_abort, err, 0x25u))) break;
+                copy_weights(kb, st, chunk, w_tap, w_c);
+            }
+            const int have = min(2, f.chunks - chunk);
+            const uint32_t bar = smem_u32(&s_full[st]);
+            for (int h = 0; h < have; ++h) {
+                if (elect_one()) {
+                    const uint32_t to = smem + st * L::stage + (uint32_t)h * kBox;
+                    if (f.a_tiled) tma_load_2d(to, &tmap_x, c * kChunk, m0, bar);
+                    else tma_load_im2col_4d(to, &tmap_x, c * kChunk, w_org, h_org, img, (uint16_t)(s * a.dil_w), (uint16_t)(r * a.dil_h), bar);
+                }
+                __syncwarp();
+                if (++c == f.cpt) {
+                    c = 0;
+                    if (++s == a.S) { s = 0; ++r; }
+                }
+            }
+            chunk += 2;
+            if (++st == ring) { st = 0; parity ^= 1u; }
+        }
+    } else {
+        // ===== multiplications =====
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+        const uint64_t b0 = umma_desc_sw128(uniform(smem) + L::parts);
+        bool ok = true;
+        for (int kb = 0; kb < n_kb && ok; ++kb) {
+            const int t = kb & 1;
+            if (kb >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_free[t]), (uint32_t)((kb >> 1) - 1) & 1u, &s_abort, err, 0x27u));
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_ready[t]), (uint32_t)(kb >> 1) & 1u, &s_abort, err, 0x26u));
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t big = tmem + L::acc + (uint32_t)(t * 2 * BN), small = big + BN, at = tmem + L::a + (uint32_t)(t * 96);
+            const uint64_t bt = b0 + (uint64_t)((uint32_t)t * (L::parts_step >> 4));
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t a0 = at + (uint32_t)(k * 8), a1 = a0 + 32u, a2 = a0 + 64u;
+                    const uint64_t w0 = bt + (uint64_t)(k * 2), w1 = w0 + (L::part >> 4), w2 = w1 + (L::part >> 4);
+                    mma_ta(small, a0, w2, idesc, k > 0 ? 1u : 0u);
+                    mma_ta(small, a2, w0, idesc, 1u);
+                    mma_ta(small, a1, w1, idesc, 1u);
+                    mma_ta(small, a0, w1, idesc, 1u);
+                    mma_ta(small, a1, w0, idesc, 1u);
+                    mma_ta(big, a0, w0, idesc, k > 0 ? 1u : 0u);
+                }
+                tcgen05_commit(smem_u32(&s_done[t]));
+            }
+            __syncwarp();
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (s_abort) {          // copies and multiplications in flight finish before their memory goes
+        const unsigned long long t0 = globaltimer_ns();
+        for (uint32_t i = 0; i < (1u << 20); ++i)
+            if (globaltimer_ns() - t0 > 50000ull) break;
+        __syncthreads();
+    }
+    if (warp == kWarpMma) {
+        tcgen05_fence_after();
+        tcgen05_dealloc(tmem, kTmemCols);
+    }
+    if (nf) nf->end(job_id);
+}
+
+int batch_of(const pb_op_params* p) { return p->batch > 1 ? p->batch : 1; }
+int dil(int d) { return d > 1 ? d : 1; }
+bool pointwise(const pb_op_params* p) { return p->R == 1 && p->S == 1 && p->stride_h == 1 && p->stride_w == 1 && p->pad_h == 0 && p->pad_w == 0; }
+
+struct SplitGeometry {
+    int BN, m_tiles, n_tiles, splits, cpt, chunks;
+    uint32_t smem;
+    const void* fn;
+};
+
+SplitGeometry split_geometry(const pb_op_params* p) {
+    SplitGeometry g;
+    g.cpt = ceil_div(p->C, kChunk);
+    g.chunks = p->R * p->S * g.cpt;
+    g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kRows);
+    const int steps = ceil_div(g.chunks, 2);
+    // Least modelled time: waves of one block an SM, each a block's fixed time (operand latency, the meeting of the ranks' sums, stores) and
+    // its steps.  Measured in chains of equal launches, tile width / ranks -> us: 256 -> 256 channels 3x3 on 2 maps of 14 x 14 64/1 31.3, 64/2 18.2,
+    // 64/4 12.0, 64/8 18.4 (two waves), 32/1 27.7, 32/2 16.1, 32/4 11.9; 64 -> 64 on 2 of 56 x 56 11.1, 9.3, 15.9, -, 10.2, 15.4, 22.1;
+    // 512 -> 512 on 2 of 7 x 7 58.2, 31.7, 18.7, 13.0, 52.3, 28.1, 16.2, 21.6.
+    static const struct { int splits, blocks; double fixed[2]; } kRanks[] = {{1, 148, {4.4, 4.8}}, {2, 148, {4.8, 5.2}}, {4, 132, {5.0, 5.4}}, {8, 120, {5.3, 6.2}}};
+    double best = 1e30;
+    for (int wide = 0; wide < (p->K > 32 ? 2 : 1); ++wide)
+        for (const auto& c : kRanks) {
+            if (c.splits > 1 && (steps < 2 * c.splits || conv_split_gain_us() > 1e6)) break;
+            const int BN = wide ? 64 : 32, blocks = g.m_tiles * ceil_div(p->K, BN) * c.splits;
+            const double us = ceil_div(blocks, c.blocks) * (c.fixed[wide] + ceil_div(steps, c.splits) * (wide ? 0.74 : 0.66));
+            if (us < best) { best = us; g.BN = BN; g.splits = c.splits; }
+        }
+    g.n_tiles = ceil_div(p->K, g.BN);
+    g.smem = (g.BN == 64 ? Layout<64>::bytes : Layout<32>::bytes) + 1024u;
+    g.fn = g.BN == 64 ? (const void*)conv_f32_split_kernel<64> : (const void*)conv_f32_split_kernel<32>;
+    return g;
+}
+
+}  // namespace
+
+uint32_t* conv_f32_error_flag_ptr() {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_f32_err_flag) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return static_cast<uint32_t*>(p);
+}
+
+// The layers that run here: what the copies can express - pixels and weights on 16-byte boundaries, the output size that follows from
+// padding, filter and stride (im2col boxes walk exactly those pixels), offsets within the descriptor's fields - and what gains.
+// - A box is 32 channels of one tap, so a layer of fewer than 24 would multiply zeros: 56 x 56, 3x3, 8 images, 8 / 16 / 24 / 32 channels -> 64 the
+//   fp32 units 18.7 / 24.5 / 30.7 / 36.1 us, here 19.1 / 19.1 / 19.2 / 19.1; one image 8.2 / 8.9 / 10.1 / 11.2 and 8.2 / 8.0 / 8.2 / 8.1.
+// - 1x1 layers of up to 32 output channels are short and store little: 256 -> 24 at 14 x 14 5.6 and 7.3, 128 -> 24 at 28 x 28 x 8 6.2 and 6.4 (36
+//   columns: 7.2 and 7.2, 9.1 and 6.7); 3x3 layers gain at any width (64 -> 8 at 56 x 56 8.5 and 8.6, x 8 images 28.5 and 23.1).
+// PB_F32_SPLIT=0 (read at every use; for tests and comparisons) keeps every layer on the fp32 units.
+bool conv_f32_split_takes(const pb_op_params* p) {
+    const char* e = getenv("PB_F32_SPLIT");
+    if (e && e[0] == '0') return false;
+    const int reach_h = (p->R - 1) * dil(p->dil_h), reach_w = (p->S - 1) * dil(p->dil_w);
+    return p->C >= 24 && (p->K > 32 || p->R * p->S > 1) && (((uintptr_t)p->x | (uintptr_t)p->w) & 15) == 0 && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
+           p->pad_w <= 100 && reach_h <= 100 && reach_w <= 100 && p->stride_h >= 1 && p->stride_w >= 1 && p->stride_h <= 8 && p->stride_w <= 8 &&
+           p->P == (p->H + 2 * p->pad_h - reach_h - 1) / p->stride_h + 1 && p->Q == (p->W + 2 * p->pad_w - reach_w - 1) / p->stride_w + 1;
+}
+
+int conv_f32_split_info(const pb_op_params* p, pb_launch_info* out) {
+    const SplitGeometry g = split_geometry(p);
+    out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
+    out->threads_per_block = kThreadsF;
+    cudaFuncAttributes at;
+    out->regs_per_thread = 144;
+    if (cudaFuncGetAttributes(&at, g.fn) == cudaSuccess) out->regs_per_thread = (uint32_t)at.numRegs;
+    else cudaGetLastError();
+    out->smem_per_block = g.smem;
+    out->tmem_cols_per_block = kTmemCols;
+    return PB_OK;
+}
+
+int conv_f32_split_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl) {
+    const SplitGeometry g = split_geometry(p);
+    SplitArgs f;
+    f.op = op;
+    f.PQ = p->P * p->Q;
+    f.M = batch_of(p) * f.PQ;
+    f.Kp = round_up(p->K, 4);
+    f.cpt = g.cpt;
+    f.chunks = g.chunks;
+    f.splits = g.splits;
+    f.a_tiled = pointwise(p) ? 1 : 0;
+    CUtensorMap map, wmap;
+    int rc = encode_pixels_f32(p->x, p->C, p->Cs, p->W, p->H, batch_of(p), p->pad_w, p->pad_h, (p->S - 1) * dil(p->dil_w), (p->R - 1) * dil(p->dil_h),
+                                     p->stride_w, p->stride_h, f.a_tiled != 0, kChunk, kRows, &map);
+    if (rc == PB_OK) rc = encode_weights_f32(p->w, f.Kp, p->Cs, p->R * p->S, g.BN, kChunk, &wmap);
+    if (rc != PB_OK) return rc;
+    PB_CUDA(cudaFuncSetAttribute(g.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)g.m_tiles, (unsigned)g.n_tiles, (unsigned)g.splits);
+    cfg.blockDim = dim3(kThreadsF);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (g.splits > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 1;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = (unsigned)g.splits;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, (void (*)(const CUtensorMap, const CUtensorMap, const SplitArgs, uint32_t, FinishedBlockNotifier*))g.fn, map, wmap, f, job_id,
+                               static_cast<FinishedBlockNotifier*>(notifier)));
+    return PB_OK;
+}
+
+}  // namespace pb

@@ -40,6 +40,7 @@ bool conv_f32_supported(const pb_op_params* p);
 int conv_f32_info(const pb_op_params* p, pb_launch_info* out);
 int64_t conv_f32_pack_weights(const pb_op_params* p, const float* w_oihw, void* dst_host);
 int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);
+uint32_t* conv_f32_error_flag_ptr();    // their error flag on the current device
 double conv_split_gain_us();      // see pb_set_conv_split_gain_us
 
 // Tensor map of a bf16 tensor without swizzle; elements outside read as zeros, or as NaN.

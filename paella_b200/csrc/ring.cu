@@ -188,8 +188,8 @@ int pb_device_error_flag(int device, uint32_t* flag_out, int reset) {
     PB_CUDA(cudaSetDevice(device));
     if (flag_out) PB_CUDA(cudaMemcpy(flag_out, p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     if (reset) PB_CUDA(cudaMemset(p, 0, sizeof(uint32_t)));
-    // the no-allocation convolution path and the window kernels keep flags of their own (they may not share one that was cudaMalloc'ed)
-    for (uint32_t* q : {pb::noalloc_error_flag_ptr(device), pb::window_error_flag_ptr()}) {
+    // the no-allocation convolution path and the window and fp32 convolution kernels keep flags of their own (they may not share one that was cudaMalloc'ed)
+    for (uint32_t* q : {pb::noalloc_error_flag_ptr(device), pb::window_error_flag_ptr(), pb::conv_f32_error_flag_ptr()}) {
         if (!q) continue;
         uint32_t v = 0;
         PB_CUDA(cudaMemcpy(&v, q, sizeof(uint32_t), cudaMemcpyDeviceToHost));

@@ -1,0 +1,162 @@
+"""Dense fp32 convolutions on the tensor cores (operands split into three bf16 parts) at the sizes where they can go wrong, against
+torch in 64 bits.
+
+Bound: an output is sum(x w) over n = C*R*S products.  The parts reproduce the operands exactly; the products left out are at most
+3 * 2^-26 of each product.  A step of 64 products is four additions of 16 exact products each to an fp32 accumulator, every one of which
+may truncate (2^-23 of a partial sum, itself at most sum|x w| of the step), and one rounding to nearest adds it to the sums of the steps
+before it: together at most (8 + n / 64) * 2^-23 * sum|x w|.  Bias, residual and result add one rounding each."""
+import ctypes as C
+import os
+
+import pytest
+
+from paella_b200 import capi
+from tests import gpu_util as gu
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # N, C, H, W, K, R, S, stride, pad_h, pad_w, dilation    (tiles of 128 rows x 64 or 32 columns, steps of two boxes of 32 channels)
+    (1, 24, 8, 16, 40, 1, 1, 1, 0, 0, 1),          # the fewest channels: one box, cut; exactly one row tile
+    (1, 24, 3, 43, 8, 3, 3, 1, 1, 1, 1),           # 129 rows; 8 of 32 columns; nine boxes: the last step has one
+    (1, 31, 1, 127, 33, 1, 3, 1, 0, 1, 1),         # 127 rows, 33 columns of 64, rows of weights padded to 36
+    (1, 32, 9, 7, 64, 1, 1, 1, 0, 0, 1),           # exactly a box and a tile's columns
+    (2, 33, 9, 7, 65, 1, 1, 1, 0, 0, 1),           # a second box of one channel, a second column tile of one column, images in one tile
+    (3, 63, 11, 13, 96, 3, 3, 1, 1, 1, 1),         # tiles straddle images, odd maps
+    (1, 64, 20, 20, 36, 5, 5, 2, 2, 2, 1),         # stride 2, 36 columns
+    (2, 65, 15, 9, 64, 3, 3, 2, 0, 0, 1),          # three boxes a tap
+    (1, 48, 19, 23, 40, 3, 3, 1, 3, 2, 2),         # dilated, unequal padding
+    (1, 200, 7, 7, 48, 1, 1, 1, 0, 0, 1),          # 4 steps: two ranks
+    (1, 128, 14, 14, 128, 3, 3, 1, 1, 1, 1),       # 18 steps: four ranks
+    (2, 512, 7, 7, 512, 3, 3, 1, 1, 1, 1),         # 72 steps: eight ranks, 98 rows
+    (1, 320, 4, 8, 64, 3, 3, 1, 1, 1, 1),          # 45 steps on 32 rows: most ranks finish rows that do not exist
+    (4, 96, 56, 56, 64, 3, 3, 1, 1, 1, 1),         # the operands' ring goes round
+    (16, 32, 61, 59, 64, 1, 1, 1, 0, 0, 1),        # several waves of one step each
+]
+
+
+def _prepare(case, act=1, residual=False, cs=None, total=None, off=0, seed=0, x=None):
+    import torch
+    n, c, h, w, k, r, s, stride, ph, pw, d = case
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    cs, total = cs or (c + 3) // 4 * 4, total or (k + 3) // 4 * 4
+    P, Q = (h + 2 * ph - (r - 1) * d - 1) // stride + 1, (w + 2 * pw - (s - 1) * d - 1) // stride + 1
+    p = capi.OpParams()
+    p.dtype, p.C, p.H, p.W, p.Cs, p.K, p.P, p.Q, p.Ks = 0, c, h, w, cs, k, P, Q, total
+    p.R, p.S, p.stride_h, p.stride_w, p.pad_h, p.pad_w, p.dil_h, p.dil_w = r, s, stride, stride, ph, pw, d, d
+    p.groups, p.act, p.batch, p.out_c_off = 1, act, n, off
+    t = {"x": torch.full((n, h, w, cs), float("nan"), device="cuda"), "w": rnd(k, c, r, s) * (2.0 / (c * r * s)) ** 0.5,
+         "b": rnd(2 * k) * 0.1, "res": rnd(n, P, Q, k), "y": torch.full((n, P, Q, total), 7.0, device="cuda")}
+    t["x"][..., :c] = rnd(n, h, w, c) if x is None else x
+    t["wd"] = gu.pack_weights(capi.STAGE_CONV_SIMT, p, t["w"].cpu().numpy())
+    p.x, p.w, p.bias, p.y = t["x"].data_ptr(), t["wd"].data_ptr(), t["b"].data_ptr(), t["y"].data_ptr()
+    if residual:
+        t["res"] = torch.nn.functional.pad(t["res"], (0, -k % 4)).contiguous()
+        p.residual, p.res_Cs = t["res"].data_ptr(), t["res"].shape[-1]
+    return p, t
+
+
+def _launch(p):
+    capi.check(capi.load().pb_op_launch(capi.STAGE_CONV_SIMT, C.byref(p), None, 0, None), "pb_op_launch")
+    gu.sync()
+    assert gu.error_flag() == 0
+
+
+def _reference(p, t, residual):
+    """The result in 64 bits, the bound on its error, and that on a chain of fp32 multiply-adds."""
+    import torch
+    x, w = t["x"][..., :p.C].permute(0, 3, 1, 2).double(), t["w"].double()
+    conv = lambda a, b: torch.nn.functional.conv2d(a, b, None, (p.stride_h, p.stride_w), (p.pad_h, p.pad_w), (p.dil_h, p.dil_w)).permute(0, 2, 3, 1)
+    y, mass = conv(x, w), conv(x.abs(), w.abs())
+    y = y + t["b"][:p.K].double()
+    if residual:
+        y = y + t["res"][..., :p.K].double()
+    n, last = p.C * p.R * p.S, 4 * 2.0 ** -24 * (y.abs() + mass)
+    bound, chain = (8 + n / 64) * 2.0 ** -23 * mass + last, n * 2.0 ** -24 * mass + last
+    if p.act == 3:
+        slope = t["b"][p.K:].double()
+        y, bound = torch.where(y > 0, y, y * slope), bound * torch.clamp(slope.abs(), min=1.0)
+    elif p.act:
+        y = torch.clamp(y, min=0.0, max=6.0 if p.act == 2 else None)
+    return y, bound, chain
+
+
+def _kernel_threads(p):
+    li = capi.LaunchInfo()
+    capi.check(capi.load().pb_op_info(capi.STAGE_CONV_SIMT, C.byref(p), C.byref(li)), "pb_op_info")
+    return li.threads_per_block
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("case", CASES)
+def test_within_the_bound(case, residual):
+    p, t = _prepare(case, act=CASES.index(case) % 4, residual=residual)
+    assert _kernel_threads(p) == 832
+    _launch(p)
+    y, bound, _ = _reference(p, t, residual)
+    assert ((t["y"][..., :p.K].double() - y).abs() <= bound).all()
+    assert (t["y"][..., p.K:] == 7.0).all()
+
+
+@pytest.mark.parametrize("total,off", [(72, 8), (47, 3)])
+def test_slice_of_a_wider_output(total, off):
+    p, t = _prepare((1, 40, 9, 11, 36, 3, 3, 1, 1, 1, 1), residual=True, total=total, off=off)
+    _launch(p)
+    y, bound, _ = _reference(p, t, True)
+    assert ((t["y"][..., off:off + 36].double() - y).abs() <= bound).all()
+    assert (t["y"][..., :off] == 7.0).all() and (t["y"][..., off + 36:] == 7.0).all()
+
+
+@pytest.mark.parametrize("case", [CASES[5], CASES[9], CASES[11]])
+def test_no_further_off_than_the_fp32_units(case, monkeypatch):
+    errors = []
+    for on in "10":
+        monkeypatch.setenv("PB_F32_SPLIT", on)
+        p, t = _prepare(case, act=0)
+        assert _kernel_threads(p) == (832 if on == "1" else 256)
+        _launch(p)
+        y = _reference(p, t, False)[0]
+        errors.append(((t["y"][..., :p.K].double() - y).norm() / y.norm()).item())
+    assert errors[0] <= errors[1]
+
+
+@pytest.mark.parametrize("case", [(1, 40, 13, 11, 72, 3, 3, 1, 1, 1, 1), (1, 512, 7, 7, 64, 1, 1, 1, 0, 0, 1)])
+def test_values_that_are_not_finite(case, monkeypatch):
+    """Infinities, NaN, and finite values whose rounding to bf16 or whose sum is not: as on the fp32 units."""
+    import torch
+    n, c, h, w = case[:4]
+    x = torch.randn((n, h, w, c), generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    x[0, 1, 2, 3], x[0, 2, 5, 0], x[0, 4, 4, 5], x[0, 5, 1, 7], x[0, 6, 6, 1] = float("inf"), -float("inf"), float("nan"), 3.4e38, -3.4e38
+    outs = []
+    for on in "10":
+        monkeypatch.setenv("PB_F32_SPLIT", on)
+        p, t = _prepare(case, act=0, x=x)
+        _launch(p)
+        outs.append(t["y"][..., :p.K])
+    a, b = outs
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isposinf(a), torch.isposinf(b)) and torch.equal(torch.isneginf(a), torch.isneginf(b))
+    ok = torch.isfinite(b)
+    assert 0 < ok.sum() < ok.numel()
+    assert ((a[ok] - b[ok]).double().norm() <= 1e-5 * b[ok].double().norm())
+
+
+@pytest.mark.parametrize("what", ["x", "w", "size", "narrow", "few"])
+def test_what_stays_on_the_fp32_units(what):
+    import torch
+    case = {"narrow": (1, 64, 9, 9, 32, 1, 1, 1, 0, 0, 1), "few": (1, 23, 9, 9, 64, 3, 3, 1, 1, 1, 1)}.get(what, (1, 64, 9, 9, 64, 3, 3, 1, 1, 1, 1))
+    p, t = _prepare(case)
+    rows = p.P
+    if what in ("x", "w"):
+        old = t["x"] if what == "x" else t["wd"].view(torch.float32)
+        t["moved"] = torch.zeros(old.numel() + 1, device="cuda")
+        t["moved"][1:] = old.reshape(-1)
+        setattr(p, what, t["moved"].data_ptr() + 4)
+    if what == "size":
+        p.P = rows = 8                       # fewer rows than padding and filter give
+        t["y"] = torch.full((1, 8, p.Q, p.Ks), 7.0, device="cuda")
+        p.y = t["y"].data_ptr()
+    assert _kernel_threads(p) == 256
+    _launch(p)
+    y, _, chain = _reference(p, t, False)
+    assert ((t["y"][..., :p.K].double() - y[:, :rows]).abs() <= chain[:, :rows]).all()

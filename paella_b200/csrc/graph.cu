@@ -282,11 +282,7 @@ pb_launch_info group_footprint(const pb_model* m, int g, const std::vector<pb_la
 // Launch geometry of stage `stage` when one launch carries `nb` images.
 int stage_info_batched(const pb_model* m, int stage, int nb, pb_launch_info* out) {
     const Stage& st = m->stages[(size_t)stage];
-    if (st.kind == PB_STAGE_MNIST_FUSED) {
-        const int rc = pb::mnist_fused_info(out);
-        out->num_blocks *= (uint32_t)nb; out->flops *= (uint64_t)nb; out->bytes *= (uint64_t)nb;
-        return rc;
-    }
+    if (st.kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(nb, out);
     pb_op_params p = st.p;
     p.batch = nb;
     if (st.kind != PB_STAGE_CONV_UMMA) return pb_op_info(st.kind, &p, out);
@@ -739,7 +735,7 @@ extern "C" {
 int pb_op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
     PB_REQUIRE(p && out, "pb_op_info: NULL argument");
     if (kind == PB_STAGE_CONV_UMMA) return pb::conv_umma_info(p, out);
-    if (kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(out);
+    if (kind == PB_STAGE_MNIST_FUSED) return pb::mnist_fused_info(p->batch, out);
     return pb::simple_op_info(kind, p, out);
 }
 
@@ -852,7 +848,7 @@ int pb_model_load(const char* pack_path, int device, int precision, pb_model** o
         st.x_is_input = true; st.y_is_output = true; st.has_res = false;
         st.out_tensor = m->t_out;
         memset(&st.p, 0, sizeof(st.p));
-        pb::mnist_fused_info(&st.info);
+        pb::mnist_fused_info(1, &st.info);
         m->stages.push_back(st);
         build_groups(m);
         *out = m;

@@ -1295,16 +1295,16 @@ __global__ void __launch_bounds__(256) detect_kernel(OpArgs a, uint32_t job_id, 
 }
 
 // ---- whole MNIST-CNN in one launch ---------------------------------------------------
-// conv5x5(1->8)+ReLU, maxpool2, conv5x5(8->16)+ReLU, maxpool3, dense 256->10 for one
-// 28x28 image, fp32, activations in shared memory.  One block of 256 threads: the network
-// is 1.2 MFLOP (the outer two rows and columns of the second convolution are never pooled) and 24 KB of weights, so one
-// kernel (one start and one end record) replaces six.
-// A lone request is the serial chain of this block, so what counts is multiply-adds per word read from shared memory: a
-// thread owns all eight channels of a 2x2 pooling window of the first convolution (236 words for 800 multiply-adds) and two
-// channels of a 3x3 pooling window of the second, for half of its input channels (396 words for 1800).  With one output per
-// thread, two words per multiply-add, the kernel took 31 us.  Weights are on their way before the request's pointers have
-// been read (they and the image come from the host's memory), and warp 0 reports the block's start while the others fetch
-// the image.
+// conv5x5(1->8)+ReLU, maxpool2, conv5x5(8->16)+ReLU, maxpool3, dense 256->10 for 28x28 images, fp32, activations in shared
+// memory.  The network is 1.2 MFLOP (the outer two rows and columns of the second convolution are never pooled) and 24 KB of
+// weights, so one kernel (one start and one end record) replaces six.
+// A lone request is the serial chain of its blocks, so what counts is multiply-adds per word read from shared memory and how many SMs
+// share them.  A lone image has a cluster of four blocks, and rank r row r of the pooled 4x4 result: its rows of the second convolution need
+// seven rows of the pooled first one (five at the borders), which it works out itself - twice the multiply-adds of a quarter of that
+// layer, but nothing is exchanged before the ten partial sums of the classifier, which meet in rank 0's shared memory.  In the second
+// convolution a warp has one input channel and a thread its 25 weights of two output channels, in registers since before the
+// request's pointers have been read (they and the image come from the host's memory); warp 0 reports the start while the others
+// fetch the image.  (All of it in one block of 256 threads: about 9 us of arithmetic, a lone request 19.2 us; this: 16.1.)
 // Weights: w1 [5][5][1][8], w2 [5][5][8][16], wd [10][4*4*16] (h, w, c order), biases fp32.
 struct MnistArgs {
     const float* x;     // [28][28]
@@ -1314,7 +1314,174 @@ struct MnistArgs {
     float* y;           // [10]
 };
 
-__global__ void __launch_bounds__(256, 2) mnist_fused_kernel(MnistArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
+constexpr int kMnistRanks = 4;
+__global__ void __launch_bounds__(256, 1) mnist_fused_kernel(MnistArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
+    constexpr int kInRows = 18, kInPitch = 34, kP1Rows = 7, kP1Pitch = 20, kP1Plane = kP1Rows * kP1Pitch, kPartPitch = 16;
+    __shared__ __align__(16) float s_in[kInRows * kInPitch];  // image rows 6 r - 6 on, with a 2-pixel zero border
+    __shared__ __align__(16) float s_w1[25 * 8];
+    __shared__ __align__(16) float s_p1[8 * kP1Plane];        // pool1 rows 3 r - 2 on, 8 planes with a 2-pixel zero border
+    __shared__ __align__(16) float s_part[8 * 36 * kPartPitch];      // [input channel][pooled pixel][position][16]
+    __shared__ float s_max[3 * 64];
+    __shared__ float s_p2[64];
+    __shared__ float s_sum[kMnistRanks][12];                  // rank 0: the ranks' shares of the classifier's sums
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, rank = (int)blockIdx.x;
+    const int kp = t & 7, px = (t >> 3) & 3;                  // second convolution: channel pair, pooled pixel
+    // every block of the cluster is running before its shared memory is written to
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    // the weights do not depend on the request
+    float2 w2r[25];
+#pragma unroll
+    for (int j = 0; j < 25; ++j) w2r[j] = __ldg(reinterpret_cast<const float2*>(a.w2 + j * 128 + wid * 16 + kp * 2));
+    float wdr[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) wdr[h][j] = wid + 8 * h < 10 ? __ldg(a.wd + (wid + 8 * h) * 256 + rank * 64 + lane + 32 * j) : 0.f;
+    const float b2r = __ldg(a.b2 + (t & 15)), bdr = t < 10 ? __ldg(a.bd + t) : 0.f;
+    if (t < 200) s_w1[t] = __ldg(a.w1 + t);
+    for (int i = t; i < kInRows * kInPitch; i += 256) s_in[i] = 0.f;
+    for (int i = t; i < 8 * kP1Plane; i += 256) s_p1[i] = 0.f;
+    pb::griddep_wait();
+    const pb::LaunchSlot* slot = pb::resolve_slot(job_id, nf);
+    const float* const x = (!a.x && slot) ? slot->io_in[0] : a.x;
+    float* const y = (!a.y && slot) ? slot->io_out[0] : a.y;
+    __syncthreads();                                          // the zeros are down
+    if (wid == 0) {
+        // the cluster is declared, and reports, as one block of 1024 threads
+        if (nf && rank == 0 && t == 0) nf->channel_.write(llis::job::InstrumentInfo::kStart, 0, 1, job_id, false);
+    } else {
+        const int top = 6 * rank - 6, lo = max(top, 0), n = min(top + kInRows, 28) - lo;
+        if ((reinterpret_cast<uintptr_t>(x) & 7) == 0) {
+            for (int i = t - 32; i < n * 14; i += 224) {
+                const float2 v = reinterpret_cast<const float2*>(x)[lo * 14 + i];
+                float* d = s_in + (lo - top + i / 14) * kInPitch + (i % 14) * 2 + 2;
+                d[0] = v.x;
+                d[1] = v.y;
+            }
+        } else {
+            for (int i = t - 32; i < n * 28; i += 224) s_in[(lo - top + i / 28) * kInPitch + i % 28 + 2] = x[lo * 28 + i];
+        }
+    }
+    __syncthreads();
+    // conv1 + ReLU + 2x2 max pool: thread = (pooled pixel, four channels)
+    {
+        const int half = t >= 98 ? 1 : 0, pix = t - 98 * half, row = pix / 14, col = pix - row * 14;
+        if (t < 196 && 3 * rank - 2 + row >= 0) {             // (the last rank's rows end with the map)
+            float p[6][6];
+#pragma unroll
+            for (int r = 0; r < 6; ++r)
+#pragma unroll
+                for (int c = 0; c < 6; c += 2) {
+                    const float2 v = *reinterpret_cast<const float2*>(s_in + (2 * row + r) * kInPitch + 2 * col + c);
+                    p[r][c] = v.x;
+                    p[r][c + 1] = v.y;
+                }
+            float acc[4][4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[0][k] = acc[1][k] = acc[2][k] = acc[3][k] = __ldg(a.b1 + half * 4 + k);
+#pragma unroll
+            for (int r = 0; r < 5; ++r)
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    const float4 w = *reinterpret_cast<const float4*>(s_w1 + (r * 5 + c) * 8 + half * 4);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float v = p[r + (q >> 1)][c + (q & 1)];
+                        acc[q][0] = fmaf(v, w.x, acc[q][0]);
+                        acc[q][1] = fmaf(v, w.y, acc[q][1]);
+                        acc[q][2] = fmaf(v, w.z, acc[q][2]);
+                        acc[q][3] = fmaf(v, w.w, acc[q][3]);
+                    }
+                }
+            float* d = s_p1 + half * 4 * kP1Plane + row * kP1Pitch + col + 2;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)      // ReLU and pooling in one: the largest of the four and zero
+                d[k * kP1Plane] = fmaxf(fmaxf(fmaxf(acc[0][k], acc[1][k]), fmaxf(acc[2][k], acc[3][k])), 0.f);
+        }
+    }
+    __syncthreads();
+    // conv2: thread = (input channel, pooled pixel, pair of output channels), the nine positions of the pooling window
+    {
+        const float* ip = s_p1 + wid * kP1Plane + px * 3;
+        float acc[9][2];
+#pragma unroll
+        for (int o = 0; o < 9; ++o) acc[o][0] = acc[o][1] = 0.f;
+#pragma unroll
+        for (int r = 0; r < 7; ++r) {
+            float v[7];
+#pragma unroll
+            for (int j = 0; j < 7; ++j) v[j] = ip[r * kP1Pitch + j];
+#pragma unroll
+            for (int oy = 0; oy < 3; ++oy) {
+                if (r - oy < 0 || r - oy > 4) continue;
+#pragma unroll
+                for (int ox = 0; ox < 3; ++ox)
+#pragma unroll
+                    for (int j = 0; j < 5; ++j) {
+                        acc[oy * 3 + ox][0] = fmaf(v[ox + j], w2r[(r - oy) * 5 + j].x, acc[oy * 3 + ox][0]);
+                        acc[oy * 3 + ox][1] = fmaf(v[ox + j], w2r[(r - oy) * 5 + j].y, acc[oy * 3 + ox][1]);
+                    }
+            }
+        }
+        float* d = s_part + (wid * 36 + px * 9) * kPartPitch + kp * 2;
+#pragma unroll
+        for (int o = 0; o < 9; ++o) *reinterpret_cast<float2*>(d + o * kPartPitch) = make_float2(acc[o][0], acc[o][1]);
+    }
+    __syncthreads();
+    // the channels' sums in channel order, + bias, ReLU, 3x3 max pool: thread = (row of the window, pooled pixel, channel), then its rows
+    if (t < 192) {
+        const int oy = t >> 6, f = t & 63;
+        const float* s = s_part + ((f >> 4) * 9 + oy * 3) * kPartPitch + (f & 15);
+        float best = 0.f;
+#pragma unroll
+        for (int ox = 0; ox < 3; ++ox) {
+            float sum[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                sum[h] = s[(h * 144 + ox) * kPartPitch];
+#pragma unroll
+                for (int c = 1; c < 4; ++c) sum[h] += s[(h * 144 + c * 36 + ox) * kPartPitch];
+            }
+            best = fmaxf(best, sum[0] + sum[1] + b2r);
+        }
+        s_max[t] = best;
+    }
+    __syncthreads();
+    if (t < 64) s_p2[t] = fmaxf(fmaxf(s_max[t], s_max[t + 64]), s_max[t + 128]);
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    // dense 256 -> 10, this rank's 64 values: warps 0..7 take rows w, w+8
+    const uint32_t sum0 = (uint32_t)__cvta_generic_to_shared(&s_sum[0][0]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int o = wid + 8 * h;
+        if (o < 10) {
+            float acc = s_p2[lane] * wdr[h][0];
+            acc = fmaf(s_p2[lane + 32], wdr[h][1], acc);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+            if (lane == 0)
+                asm volatile("{\n\t.reg .b32 at;\n\tmapa.shared::cluster.u32 at, %0, 0;\n\tst.shared::cluster.f32 [at], %1;\n\t}" ::"r"(sum0 + (uint32_t)(rank * 12 + o) * 4u), "f"(acc)
+                             : "memory");
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    if (rank != 0) return;                                    // nobody reads or writes this block's memory any more
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    if (wid == 0) {
+        if (t < 10) y[t] = ((s_sum[0][t] + s_sum[1][t]) + (s_sum[2][t] + s_sum[3][t])) + bdr;
+        __syncwarp();
+        if (nf && t == 0) {
+            __threadfence();
+            nf->channel_.write(llis::job::InstrumentInfo::kEnd, 0, 1, job_id, true);
+        }
+    }
+}
+
+// The images of a gang, one block each, the same sums in the same order.  On a GPU full of other requests' blocks four free places on one
+// GPC are longer in coming than one (192 requests of MNIST : Inception-v3 = 9 : 1 with clusters for gangs, too, 1197 us; with these blocks
+// 1175), and the images of a gang are side by side anyway.
+__global__ void __launch_bounds__(256, 2) mnist_gang_kernel(MnistArgs a, uint32_t job_id, FinishedBlockNotifier* nf) {
     constexpr int kInPitch = 34, kP1Pitch = 20, kP1Plane = 18 * kP1Pitch;
     __shared__ __align__(16) float s_in[32 * kInPitch];       // 28x28 image with a 2-pixel zero border
     __shared__ __align__(16) float s_w1[25 * 8];
@@ -1402,11 +1569,14 @@ __global__ void __launch_bounds__(256, 2) mnist_fused_kernel(MnistArgs a, uint32
         const int kp = t & 7, pix = (t >> 3) & 15, ch = (t >> 7) * 4;
         const float* ip0 = s_p1 + ch * kP1Plane + (pix >> 2) * 3 * kP1Pitch + (pix & 3) * 3;
         const float* wp0 = s_w2 + ch * 25 * 16 + kp * 2;
-        float acc[9][2];
+        float sum[9][2];                          // the channels' sums, each complete, are added in order, as the cluster does
 #pragma unroll
-        for (int o = 0; o < 9; ++o) acc[o][0] = acc[o][1] = 0.f;
+        for (int o = 0; o < 9; ++o) sum[o][0] = sum[o][1] = 0.f;
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
+            float acc[9][2];
+#pragma unroll
+            for (int o = 0; o < 9; ++o) acc[o][0] = acc[o][1] = 0.f;
             float2 w[25];
 #pragma unroll
             for (int j = 0; j < 25; ++j) w[j] = *reinterpret_cast<const float2*>(wp0 + c * 25 * 16 + j * 16);
@@ -1427,12 +1597,17 @@ __global__ void __launch_bounds__(256, 2) mnist_fused_kernel(MnistArgs a, uint32
                         }
                 }
             }
+#pragma unroll
+            for (int o = 0; o < 9; ++o) {
+                sum[o][0] += acc[o][0];
+                sum[o][1] += acc[o][1];
+            }
         }
         if (t >= 128) {
 #pragma unroll
             for (int o = 0; o < 9; ++o) {
-                s_part[(t - 128) * 19 + o * 2] = acc[o][0];
-                s_part[(t - 128) * 19 + o * 2 + 1] = acc[o][1];
+                s_part[(t - 128) * 19 + o * 2] = sum[o][0];
+                s_part[(t - 128) * 19 + o * 2 + 1] = sum[o][1];
             }
         }
         __syncthreads();
@@ -1441,8 +1616,8 @@ __global__ void __launch_bounds__(256, 2) mnist_fused_kernel(MnistArgs a, uint32
             const float b0 = __ldg(a.b2 + kp * 2), b1 = __ldg(a.b2 + kp * 2 + 1);
 #pragma unroll
             for (int o = 0; o < 9; ++o) {
-                best0 = fmaxf(best0, acc[o][0] + s_part[t * 19 + o * 2] + b0);
-                best1 = fmaxf(best1, acc[o][1] + s_part[t * 19 + o * 2 + 1] + b1);
+                best0 = fmaxf(best0, sum[o][0] + s_part[t * 19 + o * 2] + b0);
+                best1 = fmaxf(best1, sum[o][1] + s_part[t * 19 + o * 2 + 1] + b1);
             }
             s_p2[pix * 16 + kp * 2] = best0;
             s_p2[pix * 16 + kp * 2 + 1] = best1;
@@ -1454,12 +1629,14 @@ __global__ void __launch_bounds__(256, 2) mnist_fused_kernel(MnistArgs a, uint32
     for (int h = 0; h < 2; ++h) {
         const int o = wid + 8 * h;
         if (o < 10) {
-            float acc = 0.f;
+            float acc[kMnistRanks];              // a rank's 64 values at a time
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc = fmaf(s_p2[lane + 32 * j], wdr[h][j], acc);
+            for (int r = 0; r < kMnistRanks; ++r) acc[r] = fmaf(s_p2[lane + 64 * r + 32], wdr[h][2 * r + 1], s_p2[lane + 64 * r] * wdr[h][2 * r]);
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-            if (lane == 0) y[o] = acc + __ldg(a.bd + o);
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int r = 0; r < kMnistRanks; ++r) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], off);
+            if (lane == 0) y[o] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + __ldg(a.bd + o);
         }
     }
     PB_NOTIFY_END();
@@ -1995,23 +2172,41 @@ int64_t simple_pack_weights(int kind, const pb_op_params* p, const float* w, voi
     return PB_ERR_INVALID;
 }
 
-int mnist_fused_info(pb_launch_info* out) {
+int mnist_fused_info(int batch, pb_launch_info* out) {
+    const bool gang = batch > 1;
+    const uint32_t nb = gang ? (uint32_t)batch : 1u;
     memset(out, 0, sizeof(*out));
     out->kind = PB_STAGE_MNIST_FUSED;
-    out->num_blocks = 1;
-    out->threads_per_block = 256;
-    out->regs_per_thread = regs_of(mnist_fused_kernel);
-    out->smem_per_block = static_smem_of(mnist_fused_kernel);
-    out->flops = 2ull * (156800 + 627200 + 2560);      // the layers as the model states them
-    out->bytes = 4ull * (784 + 200 + 8 + 3200 + 16 + 2560 + 10 + 10);
+    out->num_blocks = nb;
+    out->threads_per_block = gang ? 256 : 256 * kMnistRanks;      // a lone image's cluster counts as one block
+    out->regs_per_thread = gang ? regs_of(mnist_gang_kernel) : regs_of(mnist_fused_kernel);
+    out->smem_per_block = gang ? static_smem_of(mnist_gang_kernel) : kMnistRanks * static_smem_of(mnist_fused_kernel);
+    out->flops = nb * 2ull * (156800 + 627200 + 2560);      // the layers as the model states them
+    out->bytes = nb * 4ull * (784 + 200 + 8 + 3200 + 16 + 2560 + 10 + 10);
     return PB_OK;
 }
 
 int mnist_fused_launch(const float* x, const float* w1, const float* b1, const float* w2, const float* b2,
                        const float* wd, const float* bd, float* y, int batch, cudaStream_t st, uint32_t job_id, void* notifier) {
     MnistArgs a{x, w1, b1, w2, b2, wd, bd, y};
-    mnist_fused_kernel<<<batch > 1 ? batch : 1, 256, 0, st>>>(a, job_id, static_cast<FinishedBlockNotifier*>(notifier));
-    return launch_check("mnist_fused");
+    FinishedBlockNotifier* const nf = static_cast<FinishedBlockNotifier*>(notifier);
+    if (batch > 1) {
+        mnist_gang_kernel<<<batch, 256, 0, st>>>(a, job_id, nf);
+        return launch_check("mnist_gang");
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kMnistRanks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kMnistRanks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, mnist_fused_kernel, a, job_id, nf));
+    return PB_OK;
 }
 
 }  // namespace pb

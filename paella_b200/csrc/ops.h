@@ -31,7 +31,7 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
 int64_t simple_pack_weights(int kind, const pb_op_params* p, const float* w_oihw, void* dst_host);
 void store_elem(void* dst, size_t i, float v, int dtype);
 uint32_t* window_error_flag_ptr();      // the window kernels' error flag on the current device
-int mnist_fused_info(pb_launch_info* out);
+int mnist_fused_info(int batch, pb_launch_info* out);
 int mnist_fused_launch(const float* x, const float* w1, const float* b1, const float* w2, const float* b2,
                        const float* wd, const float* bd, float* y, int batch, cudaStream_t st, uint32_t job_id, void* notifier);
 

@@ -105,6 +105,7 @@ struct ConvArgs {
     uint32_t b_stage_bytes;
     int out_box;          // channels of one TMA store box: 64 or 32 (divides BN); 0 = the epilogue stores directly
     int splits;           // thread blocks (one cluster) that share a tile's reduction: rank z takes k-blocks [nkb*z/splits, nkb*(z+1)/splits)
+    uint32_t meet;        // where the other ranks' sums arrive in shared memory (0: in the pipeline buffers, once their multiplications are done)
     // A pointwise layer may take act(x * pre_scale + pre_bias), per input channel, instead of x (pre_scale NULL: x itself).
     const float* pre_scale;
     const float* pre_bias;
@@ -183,9 +184,10 @@ struct EpiArgs {
     __nv_bfloat16* y;
     uint32_t* err_flag;
     int M, K, Ks, out_c_off, res_Cs, act, BN, out_box, splits, nkb;
+    uint32_t meet;
 };
 __device__ __forceinline__ EpiArgs epi_args(const ConvArgs& a) {
-    return {a.residual, a.bias, a.y, a.err_flag, a.M, a.K, a.Ks, a.out_c_off, a.res_Cs, a.act, a.BN, a.out_box, a.splits, a.nkb};
+    return {a.residual, a.bias, a.y, a.err_flag, a.M, a.K, a.Ks, a.out_c_off, a.res_Cs, a.act, a.BN, a.out_box, a.splits, a.nkb, a.meet};
 }
 
 // kAct: 0 = the activation is chosen here, 1 = it is ReLU or ReLU6, 2 = it is neither.
@@ -377,121 +379,188 @@ __device__ __forceinline__ void epilogue(const Args& a, uint32_t tmem_base, bool
 
 // ---- split reduction: the thread blocks of a cluster share one output tile -----------------------------------
 // Rank z of the cluster multiplies its share of the k-blocks; then rank d finishes columns [d*w, (d+1)*w) of the
-// tile, w = BN / splits.  Every rank parks the columns it does not own in its own shared memory (the pipeline
-// buffers, free once its multiplications are done), 16 bytes per lane and consecutive lanes (= rows) side by side;
-// after a cluster barrier the owner reads the other ranks' parts through distributed shared memory, all of them in
-// flight together, and adds them in rank order, so the fp32 result does not depend on timing.  One cluster barrier
-// on the critical path, nothing goes through global memory; a second one, over which the stores run, keeps every
-// rank's memory alive until it has been read.
-// (The partial tiles used to meet in a global workspace under an atomic counter: two fences, an atomic and an L2
-// round trip of BN x 512 bytes per rank, read back by ONE block: +4 to +8 us per launch, so only reductions of 60
-// and more k-blocks gained from it.)
-template <int kAct, class Args>
-__device__ __forceinline__ void cluster_finish(const Args& a, int n0, bool row_valid, __nv_bfloat16* yrow,
-                                               const __nv_bfloat16* rrow, const float* s_bias, int rank, uint32_t buf, int w) {
+// tile, w = BN / splits.  Every rank sends each owner its part straight from tensor memory (st.async: registers into the owner's
+// shared memory, counted by the owner's barrier), 16 bytes per lane and consecutive lanes (= rows) side by side; the owner adds the
+// parts in rank order, its own from its tensor memory, so the fp32 result does not depend on timing.  Where the pipeline leaves
+// room the parts have a place of their own and a rank sends as soon as its accumulator is complete; else they land in
+// the owner's pipeline buffers, and every rank first tells the others that its multiplications are done with them.
+// Nobody waits for having been read: a block ends when the others' parts, and before them their messages, have arrived.
+// Bound by the way between SMs: with development probes 800 clocks and 20 bytes a clock per SM, however it is used; owners that pulled parked
+// tiles with loads saw 8 to 10 (48 KB at four ranks 5080 clocks, 28 KB at eight 5070; st.async 3110 and 2410), and two cluster barriers
+// besides.  (A global workspace under an atomic counter, before: +4 to +8 us per launch.)
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar)
+                 : "memory");
+}
+// (Relaxed: it says that memory has been read, and a release takes 1500 clocks.)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tcgen05_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Ranks that have k-blocks: all of them unless a grouped launch splits a short reduction.
+template <class Args>
+__device__ __forceinline__ uint32_t active_ranks(const Args& a) {
     const int S = a.splits;
-    uint32_t active = (1u << S) - 1u;      // ranks that have k-blocks (all of them unless a grouped launch splits a short reduction)
-    if (a.nkb < S) {
-        active = 0;
+    if (a.nkb >= S) return (1u << S) - 1u;
+    uint32_t active = 0;
 #pragma unroll 1
-        for (int z = 0; z < S; ++z) active |= (a.nkb * (z + 1) / S > a.nkb * z / S ? 1u : 0u) << z;
-    }
-    // Four partial sums of 8 columns in flight per turn (16-byte loads: 8 a thread; more spill): four ranks', or with two ranks
-    // those of 16 columns.
-    const int step = S == 2 ? 16 : 8;
+    for (int z = 0; z < S; ++z) active |= (a.nkb * (z + 1) / S > a.nkb * z / S ? 1u : 0u) << z;
+    return active;
+}
+// What arrives at a rank, in bytes.
+template <class Args>
+__device__ __forceinline__ uint32_t meet_bytes(const Args& a, int rank) {
+    return (uint32_t)__popc(active_ranks(a) & ~(1u << rank)) * (uint32_t)(a.BN / a.splits) * 512u;
+}
+
+// The columns of this rank: its own part, then the others' in rank order.  `at` is this thread's row of those, [rank but this][4 columns][row].
+template <int kAct, class Args>
+__device__ __forceinline__ void cluster_finish(const Args& a, uint32_t own_addr, int k0, bool row_valid, __nv_bfloat16* yrow, const __nv_bfloat16* rrow,
+                                               const float* bias, uint32_t others, uint32_t at, int w, bool mine, uint32_t (&own)[8], uint4 res) {
+    const uint32_t step = (uint32_t)(w >> 2) * 2048u;      // between two ranks' parts
+    const int n = a.splits - 1;
+    const bool all = others == (1u << n) - 1u;
 #pragma unroll 1
-    for (int c = 0; c < w; c += step) {
-        uint64_t sum[2][4];
+    for (int c = 0; c < w; c += 8) {
+        const int k = k0 + c;
+        uint64_t sum[4];
 #pragma unroll
-        for (int o = 0; o < 2; ++o)
+        for (int j = 0; j < 4; ++j) sum[j] = pack_f32x2(own[2 * j], own[2 * j + 1]);
+        uint4 next = make_uint4(0, 0, 0, 0);      // the residual and this rank's part of the next turn
+        if (c + 8 < w) {
+            tcgen05_ld8(own_addr + (uint32_t)c + 8u, own);
+            if (rrow && row_valid && k + 8 < a.K) next = *reinterpret_cast<const uint4*>(rrow + k + 8);
+        }
+        auto add = [&](const uint4& p, const uint4& q) {
+            sum[0] = add_f32x2(sum[0], pack_f32x2(p.x, p.y));
+            sum[1] = add_f32x2(sum[1], pack_f32x2(p.z, p.w));
+            sum[2] = add_f32x2(sum[2], pack_f32x2(q.x, q.y));
+            sum[3] = add_f32x2(sum[3], pack_f32x2(q.z, q.w));
+        };
+        const uint32_t from = at + (uint32_t)(c >> 2) * 2048u;
+        if (all && n == 3) {
+            uint4 p[3], q[3];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sum[o][j] = 0;        // (+0 is exact; a sum of zeros may lose a -0, which the bias add would too)
-#pragma unroll 1
-        for (int z0 = 0; z0 < S; z0 += 4) {
-            uint4 part[4][2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int z = S == 2 ? i & 1 : z0 + i, col = S == 2 ? c + (i >> 1) * 8 : c;
-                part[i][0] = part[i][1] = make_uint4(0, 0, 0, 0);
-                if (col >= w || !((active >> z) & 1u)) continue;
-                const uint32_t at = cluster_addr(buf + ((uint32_t)((rank * w + col) >> 2) * 128u + threadIdx.x) * 16u, (uint32_t)z);       // this rank's own part too
-                part[i][0] = ld_cluster_v4(at);
-                part[i][1] = ld_cluster_v4(at + 2048u);
+            for (int i = 0; i < 3; ++i) {
+                p[i] = ld_shared_v4(from + (uint32_t)i * step);
+                q[i] = ld_shared_v4(from + (uint32_t)i * step + 2048u);
             }
-            auto add = [&](uint64_t (&s)[4], const uint4 (&q)[2]) {
-                s[0] = add_f32x2(s[0], pack_f32x2(q[0].x, q[0].y));
-                s[1] = add_f32x2(s[1], pack_f32x2(q[0].z, q[0].w));
-                s[2] = add_f32x2(s[2], pack_f32x2(q[1].x, q[1].y));
-                s[3] = add_f32x2(s[3], pack_f32x2(q[1].z, q[1].w));
-            };
-            add(sum[0], part[0]);
-            add(sum[0], part[1]);
-            if (S == 2) {
-                add(sum[1], part[2]);
-                add(sum[1], part[3]);
-            } else {
-                add(sum[0], part[2]);
-                add(sum[0], part[3]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) add(p[i], q[i]);
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < n; ++i) {
+                if (!((others >> i) & 1u)) continue;
+                const uint4 p = ld_shared_v4(from + (uint32_t)i * step), q = ld_shared_v4(from + (uint32_t)i * step + 2048u);
+                add(p, q);
             }
         }
-#pragma unroll
-        for (int o = 0; o < 2; ++o) {
-            const int at = c + 8 * o, col = rank * w + at, k = n0 + col;
-            if ((o && S != 2) || at >= w || !row_valid || k >= a.K) continue;
-            uint4 res = make_uint4(0, 0, 0, 0);
-            if (rrow) res = *reinterpret_cast<const uint4*>(rrow + k);
+        if (row_valid && k < a.K) {
             uint32_t v[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(sum[o][j]));
-            *reinterpret_cast<uint4*>(yrow + k) = finish8<kAct>(a, v, res, rrow != nullptr, k, s_bias + col);
+            for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(sum[j]));
+            *reinterpret_cast<uint4*>(yrow + k) = finish8<kAct>(a, v, res, rrow != nullptr, k, bias + c);
+        }
+        res = next;
+        tcgen05_wait_ld();
+        if (!mine) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) own[j] = 0;
         }
     }
 }
 
-// Run by warps 0-3 of every rank.  `mine`: this rank has k-blocks of its own.
+// Run by warps 0-3 of every rank.  s_go: the other ranks' pipelines are free (splits - 1 arrivals); s_parts: their parts are here.
 template <bool kByAct, class Args>
-__device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_base, int m0, int n0, int rank, bool mine, uint32_t smem_base,
-                                                 const float* s_bias, uint64_t* s_accum_p, volatile uint32_t* s_abort_p) {
+__device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_base, int m0, int n0, int rank, uint32_t smem_base, const float* s_bias,
+                                                 uint64_t* s_accum_p, uint64_t* s_go, uint64_t* s_parts, volatile uint32_t* s_abort_p) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
-    const int m = m0 + tid;
+    const int m = m0 + tid, S = a.splits, w = a.BN / S, k0 = n0 + rank * w;
     const bool row_valid = m < a.M;
+    const uint32_t active = active_ranks(a);
+    const bool mine = (active >> rank) & 1u;
+    // What can be had before the accumulator is waited for: the residual's first part, the other ranks' arrival.
+    const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
+    uint4 res = make_uint4(0, 0, 0, 0);
+    if (rrow && row_valid && k0 < a.K) res = *reinterpret_cast<const uint4*>(rrow + k0);
+    cluster_wait();                 // every rank is running and has set its barriers up
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
+    const uint32_t at = smem_base + a.meet + (uint32_t)tid * 16u, parts = smem_u32(s_parts);
+    // Columns in steps of 8 from the next rank's on, so that not everybody sends to the same one at once.
+    int d = rank + 1 < S ? rank + 1 : 0, c = d * w, left = w;
+    uint32_t to = 0, bar = 0;
+    auto address = [&]() {
+        to = cluster_addr(at + (uint32_t)((rank - (rank > d ? 1 : 0)) * (w >> 2)) * 2048u, (uint32_t)d);
+        bar = cluster_addr(parts, (uint32_t)d);
+    };
+    address();
     bool ok = mbar_wait(smem_u32(s_accum_p), 0u, s_abort_p, a.err_flag, 3u);
     ok = __all_sync(0xffffffffu, ok);
     if (tid == 0) PB_T(5);
     tcgen05_fence_after();
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
-    const int w = a.BN / a.splits;
-    if (mine) {
-        uint32_t v0[16], v1[16];
-        uint32_t at = smem_base + (uint32_t)tid * 16u;
-        tcgen05_ld16(lane_addr, v0);
+    bool go = true;
+    if (a.meet == 0) {
+        if (tid > 0 && tid < S) mbar_arrive_cluster(cluster_addr(smem_u32(s_go), (uint32_t)((rank + tid) % S)));
+        __syncwarp();
+    }
+    uint32_t v0[8], v1[8];
+    tcgen05_ld8(lane_addr + (uint32_t)c, v0);
+    if (a.meet == 0) go = __all_sync(0xffffffffu, mbar_wait(smem_u32(s_go), 0u, s_abort_p, a.err_flag, 9u));
+    if (mine && go) {
+        auto send = [&](const uint32_t (&v)[8]) {
+            st_async_v4(to, v[0], v[1], v[2], v[3], bar);
+            st_async_v4(to + 2048u, v[4], v[5], v[6], v[7], bar);
+            to += 4096u;
+            if ((left -= 8) == 0) {
+                left = w;
+                d = d + 1 < S ? d + 1 : 0;
+                address();
+            }
+        };
 #pragma unroll 1
-        for (int cb = 0; cb < a.BN; cb += 32) {
+        for (int g = (a.BN - w) >> 3; g > 0; g -= 2) {
+            c = c + 8 < a.BN ? c + 8 : 0;
             tcgen05_wait_ld();
-            if (cb + 16 < a.BN) tcgen05_ld16(lane_addr + (uint32_t)(cb + 16), v1);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) st_shared_v4(at + (uint32_t)j * 2048u, v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
-            if (cb + 16 >= a.BN) break;
+            if (g > 1) tcgen05_ld8(lane_addr + (uint32_t)c, v1);
+            send(v0);
+            if (g == 1) break;
+            c = c + 8 < a.BN ? c + 8 : 0;
             tcgen05_wait_ld();
-            if (cb + 32 < a.BN) tcgen05_ld16(lane_addr + (uint32_t)(cb + 32), v0);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) st_shared_v4(at + 8192u + (uint32_t)j * 2048u, v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
-            at += 16384u;
+            if (g > 2) tcgen05_ld8(lane_addr + (uint32_t)c, v0);
+            send(v1);
         }
     }
-    cluster_arrive();
-    cluster_wait();                 // every rank's columns are parked
-    if (tid == 0) PB_T(6);
+    if (tid == 0) PB_T(10);
+    // This rank's own first columns (zeros if it had no k-blocks), under the wait for the others' parts.
+    tcgen05_wait_ld();
+    const uint32_t own_addr = lane_addr + (uint32_t)(rank * w);
+    tcgen05_ld8(own_addr, v0);
+    // (Also when this block gives up: it stays until the others have written to it.)
+    bool here = false;
+    for (uint32_t i = 0; i < kWaitLimit && !here; ++i) here = mbar_try_wait(parts, 0u);
+    if (!here) { *s_abort_p = 1; atomicExch(a.err_flag, 10u); }
+    ok = __all_sync(0xffffffffu, here) && ok;
+    tcgen05_wait_ld();
+    if (!mine) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v0[j] = 0;
+    }
+    if (tid == 0) PB_T(11);
     if (ok) {
         __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
-        const __nv_bfloat16* rrow = a.residual ? a.residual + (size_t)m * a.res_Cs : nullptr;
-        if constexpr (!kByAct) cluster_finish<0>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
-        else if (a.act == 1 || a.act == 2) cluster_finish<1>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
-        else cluster_finish<2>(a, n0, row_valid, yrow, rrow, s_bias, rank, smem_base, w);
+        const uint32_t others = (active & ((1u << rank) - 1u)) | ((active >> (rank + 1)) << rank);
+        const float* bias = s_bias + rank * w;
+        if constexpr (!kByAct) cluster_finish<0>(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
+        else if (a.act == 1 || a.act == 2) cluster_finish<1>(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
+        else cluster_finish<2>(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
     }
-    cluster_arrive_relaxed();
-    cluster_wait();                 // every rank has read what it needs: shared memory may go
 }
 
 template <int kStages>
@@ -761,7 +830,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
                                               const CUtensorMap* tmap_n, const ConvArgs& a, const int stages,
                                               const int bx, const int by, const int bz, uint8_t* smem_raw,
                                               uint64_t* s_full, uint64_t* s_empty, uint64_t* s_accum, uint32_t* s_tmem_base,
-                                              volatile uint32_t* s_abort, float* s_bias, uint64_t* s_res, uint64_t* s_ready, bool publish) {
+                                              volatile uint32_t* s_abort, float* s_bias, uint64_t* s_res, uint64_t* s_ready, uint64_t* s_go, uint64_t* s_parts, bool publish) {
     const int tid = threadIdx.x;
     const int warp = (int)uniform((uint32_t)tid >> 5);
     const int lane = tid & 31;
@@ -802,6 +871,11 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
             }
             mbar_init(smem_u32(s_accum), kPre ? 2 : 1);                // normalised: its memory is free, too
             mbar_init(smem_u32(s_res), 1);
+            if (a.splits > 1) {
+                mbar_init(smem_u32(s_go), (uint32_t)(a.splits - 1));
+                mbar_init(smem_u32(s_parts), 1);
+                mbar_arrive_expect_tx(smem_u32(s_parts), meet_bytes(a, bz));
+            }
             *s_abort = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -839,6 +913,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    if (a.splits > 1) cluster_arrive_relaxed();      // (the barriers' fence has released them) the epilogue waits for the other ranks before it sends them anything
     const uint32_t tmem_base = uniform(*s_tmem_base);
     if (tid == 0) { PB_T(1); PB_S(1); }
 
@@ -877,10 +952,10 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         if (tid == 0) PB_S(2);
         griddep_launch();
         if constexpr (kLone) {
-            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
+            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, smem_base, s_bias, s_accum, s_go, s_parts, s_abort);
             else epilogue<true>(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
         } else {
-            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, nkb > 0, smem_base, s_bias, s_accum, s_abort);
+            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, smem_base, s_bias, s_accum, s_go, s_parts, s_abort);
             else epilogue<false>(epi_args(a), tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
         }
         if (tid == 0) { PB_T(6); PB_S(6); }
@@ -931,9 +1006,9 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
             if (++st == (uint32_t)stages) { st = 0; parity ^= 1u; }
         }
         if (kPre) {
-            // The epilogue may start once the stages whose memory it uses (for the partial or the finished tile) have been stored; the
+            // The epilogue may start once the stages whose memory it uses (for the others' parts or the finished tile) have been stored; the
             // others leave beside it.
-            const uint32_t bytes = a.splits > 1 ? (uint32_t)a.BN * 512u : a.out_box ? (uint32_t)a.BN * 256u : 0u;
+            const uint32_t bytes = a.splits > 1 ? (a.meet ? 0u : (uint32_t)(a.BN - a.BN / a.splits) * 512u) : a.out_box ? (uint32_t)a.BN * 256u : 0u;
             const int used = (int)((bytes + stage_bytes - 1) / stage_bytes), last_st = nkb > 0 ? (nkb - 1) % stages : 0;
             const int until = used > 0 ? nkb - 1 - max(0, last_st - (used - 1)) : -1;        // the last k-block in one of them
             auto let_epilogue = [&]() {
@@ -964,7 +1039,6 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
             __syncwarp();
         }
         griddep_launch();
-        if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
         if (kPre && lane == 0) tma_store_wait_read();
     } else {
         // ===== MMA issuer =====
@@ -1007,7 +1081,6 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 #endif
         __syncwarp();
         griddep_launch();
-        if (a.splits > 1) { cluster_arrive_relaxed(); cluster_wait(); cluster_arrive_relaxed(); cluster_wait(); }
     }
 
     tcgen05_fence_before();
@@ -1047,6 +1120,8 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
     __shared__ __align__(8) uint64_t s_res;
     __shared__ __align__(8) uint64_t s_accum;
+    __shared__ __align__(8) uint64_t s_go;
+    __shared__ __align__(8) uint64_t s_parts;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
     __shared__ __align__(16) float s_bias[kMaxBN];
@@ -1055,7 +1130,7 @@ conv_umma_tma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
     conv_tile_tma<false, true>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, nullptr, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
-                         &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
+                         &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, &s_go, &s_parts, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1070,6 +1145,8 @@ conv_umma_pre_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     __shared__ __align__(8) uint64_t s_ready[kMaxStages];
     __shared__ __align__(8) uint64_t s_res;
     __shared__ __align__(8) uint64_t s_accum;
+    __shared__ __align__(8) uint64_t s_go;
+    __shared__ __align__(8) uint64_t s_parts;
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
     __shared__ __align__(16) float s_bias[kMaxBN];
@@ -1078,7 +1155,7 @@ conv_umma_pre_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
     conv_tile_tma<true, false>(&tmap_w, &tmap_x, &tmap_y, &tmap_r, &tmap_n, a, stages, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, smem_raw, s_full, s_empty, &s_accum,
-                        &s_tmem_base, &s_abort, s_bias, &s_res, s_ready, nf != nullptr);
+                        &s_tmem_base, &s_abort, s_bias, &s_res, s_ready, &s_go, &s_parts, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1398,6 +1475,8 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile uint32_t s_abort;
     __shared__ __align__(16) float s_bias[kMaxBN];
+    __shared__ __align__(8) uint64_t s_go;
+    __shared__ __align__(8) uint64_t s_parts;
     __shared__ __align__(16) ConvArgs s_args;
 
     resolve_slot(job_id, nf);
@@ -1425,7 +1504,7 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     const uint32_t tile = local / S, bz = local - tile * S;
     const uint32_t by = tile / gx, bx = tile - by * gx;
     conv_tile_tma<false, false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, nullptr, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
-                  &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, nf != nullptr);
+                  &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, &s_go, &s_parts, nf != nullptr);
     if (nf) nf->end(job_id);
 }
 
@@ -1818,6 +1897,7 @@ struct Geometry {
     bool pair;                  // two blocks on a tile of 256 rows
     int out_box;                // ConvArgs::out_box
     uint32_t tmem_cols, b_stage_bytes, smem_bytes, idesc;
+    uint32_t meet;              // ConvArgs::meet
 };
 
 // Rows of the packed weight matrix: the layout does not depend on how a launch tiles it (a box that reaches past
@@ -1837,9 +1917,18 @@ struct ConvShape {
 // launch of up to two blocks per SM gets a deeper pipeline (a refill takes about 1.1 us; 36 k-blocks of 64 columns: 13.6 us
 // at 73 KB, 12.3 at 110, 11.7 at 150, where the next launch's blocks no longer fit beside it: Inception-v3 402 us
 // instead of 346).
-int pipeline_stages(int ctas, int BN, int k_blocks, bool shared) {
-    const int budget = (int)(!shared && ctas <= 296 ? kSmemBudgetDeep : kSmemBudgetTma) - 1024;
-    return std::max(2, std::min({kMaxStages, budget / ((int)kATileBytes + BN * 128), k_blocks}));
+// Where the other ranks' parts of a split tile arrive: beside the pipeline where that leaves it three stages (or as many as there are
+// k-blocks), else in its buffers.
+struct Pipeline { int stages; uint32_t meet, bytes; };        // meet: offset of that place, 0 = in the buffers
+Pipeline pipeline(int ctas, int BN, int k_blocks, int splits, bool shared) {
+    const int budget = (int)(!shared && ctas <= 296 ? kSmemBudgetDeep : kSmemBudgetTma) - 1024, stage = (int)kATileBytes + BN * 128;
+    const int parts = splits > 1 ? (BN - BN / splits) * 512 : 0, most = std::min(kMaxStages, k_blocks);
+    if (parts && (budget - parts) / stage >= std::max(2, std::min(3, k_blocks))) {
+        const int stages = std::max(2, std::min(most, (budget - parts) / stage));
+        return {stages, (uint32_t)(stages * stage), (uint32_t)(stages * stage + parts)};
+    }
+    const int stages = std::max(2, std::min(most, budget / stage));
+    return {stages, 0u, (uint32_t)std::max(stages * stage, parts)};
 }
 
 // Modelled microseconds of a lone launch inside a stage graph, fitted to 3372 measured (layer shape, tile width, split, way
@@ -1857,7 +1946,7 @@ int pipeline_stages(int ctas, int BN, int k_blocks, bool shared) {
 // store, cost a 14 x 14 layer of 256 -> 1024 channels 8.8 us instead of 6.4 alone and 3.1 instead of 1.7 under load.)
 int tiling_ctas(const ConvShape& c, const ConvTiling& t) { return c.m_tiles * ceil_div(c.Kp16, t.BN) * t.splits; }
 double tiling_us(int ctas, const ConvShape& c, const ConvTiling& t) {
-    const int k_blocks = ceil_div(c.nkb, t.splits), stages = pipeline_stages(ctas, t.BN, k_blocks, c.shared);
+    const int k_blocks = ceil_div(c.nkb, t.splits), stages = pipeline(ctas, t.BN, k_blocks, t.splits, c.shared).stages;
     const double mean = std::max(1.0, ctas / 148.0), per_sm = mean + 0.639 * (ceil_div(ctas, 148) - mean);
     const double crowd = 1.0 + 1.39 * (per_sm - 1.0);
     double kb = std::max(0.197 + 0.0003 * t.BN, per_sm * (16.384 + 0.128 * t.BN) / 137.0);
@@ -2001,9 +2090,17 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
     while ((int)g.tmem_cols < g.BN) g.tmem_cols <<= 1;
     g.b_stage_bytes = (uint32_t)(g.pair ? g.BN / 2 : g.BN) * 128u;
     const uint32_t stage_bytes = (uint32_t)kATileBytes + g.b_stage_bytes;
+    uint32_t pipe_bytes = 0;
+    g.meet = 0;
     if (use_tma_a()) {
-        g.stages = g.pair ? std::min(kMaxStages, (int)((kSmemBudgetDeep - 1024u) / stage_bytes))
-                          : pipeline_stages(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), t.shared);
+        if (g.pair) {
+            g.stages = std::min(kMaxStages, (int)((kSmemBudgetDeep - 1024u) / stage_bytes));
+        } else {
+            const Pipeline pipe = pipeline(g.m_tiles * g.n_tiles * g.splits, g.BN, ceil_div(g.nkb, g.splits), g.splits, t.shared);
+            g.stages = pipe.stages;
+            g.meet = pipe.meet;
+            pipe_bytes = pipe.bytes;
+        }
     } else {
         static const int kDepths[] = {8, 6, 4};                     // the gather kernel exists for 4, 6, 8
         g.stages = 4;
@@ -2011,8 +2108,7 @@ Geometry geometry(const pb_op_params* p, const ConvTiling& t) {
             if ((uint32_t)d * stage_bytes + 1024u <= kSmemBudget && d <= g.nkb + 1) { g.stages = d; break; }
     }
     g.out_box = !t.tma ? 0 : g.BN % 64 == 0 ? 64 : 32;
-    const uint32_t exchange = g.splits > 1 ? (uint32_t)g.BN * 512u : 0u;      // a rank's partial tile
-    g.smem_bytes = std::max((uint32_t)g.stages * stage_bytes, exchange) + 1024u;
+    g.smem_bytes = (pipe_bytes ? pipe_bytes : (uint32_t)g.stages * stage_bytes) + 1024u;
     // c_format f32 (1 << 4), a/b format bf16 (1 << 7, 1 << 10), K-major both, N >> 3 at bit 17, M >> 4 at bit 24
     g.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.BN >> 3) << 17) | ((uint32_t)((g.pair ? 2 * kBM : kBM) >> 4) << 24);
     return g;
@@ -2379,6 +2475,7 @@ static int fill_args(const ConvUmmaPlan* plan, const Geometry& g, const pb_op_pa
     a.act = p->act; a.a_tiled = pointwise(p) ? 1 : 0; a.nkb = g.nkb; a.taps = p->R * p->S; a.Cp = g.Cp; a.BN = g.BN; a.idesc = g.idesc; a.tmem_cols = g.tmem_cols;
     a.b_stage_bytes = g.b_stage_bytes;
     a.splits = g.splits;
+    a.meet = g.meet;
     a.out_box = g.out_box;
     return PB_OK;
 }

@@ -1938,7 +1938,11 @@ Pipeline pipeline(int ctas, int BN, int k_blocks, int splits, bool shared) {
 //   a k-block costs the issue of its copies (0.2 us), its share of a refill's latency, or its bytes at 137 KB/us per SM,
 //   shared by the blocks of the SM (between the mean and the fullest one);
 //   the epilogue costs 11 ns per column of a block with direct stores (24 with a residual), 8 through TMA;
-//   a cluster costs its two barriers and the parked tile, and 2 / 6 / 13 ns of placement per block at 2 / 4 / 8 ranks.
+//   a cluster costs 21 ns per column that a rank sends, 4 / 4 / 6 ns of placement per block at 2 / 4 / 8 ranks, and a message to and fro
+//   where the parts land in the pipeline's buffers (fitted to 912 combinations of 66 shapes, launches with st.async; the tiles it
+//   picks for the shapes take 391.5 us in all, the best measured 386.8).
+// On a GPU that other requests share, the costs that a cluster had with barriers and pulled parts stay: with these, clusters win where
+// lone blocks serve the mixes better (192 requests of MNIST : Inception-v3 = 9 : 1 1144 and 1195 us, 64 of MobileNet and ResNet-50 1633 and 1679).
 // Its mean error there is 3 %, and what it picks is within 1.5 % of the best measured tiles summed over the layers of a network.
 // A layer repeated 40 times in one graph, all launches alike, takes 1.8 us less than modelled (0.3 us spread over 19 layers of 7x7 to
 // 56x56 maps, 1 and 8 images); the tiles picked for those 19 take 91.6 us in all, the best of 6 to 33 measured for each 90.4.
@@ -1946,7 +1950,9 @@ Pipeline pipeline(int ctas, int BN, int k_blocks, int splits, bool shared) {
 // store, cost a 14 x 14 layer of 256 -> 1024 channels 8.8 us instead of 6.4 alone and 3.1 instead of 1.7 under load.)
 int tiling_ctas(const ConvShape& c, const ConvTiling& t) { return c.m_tiles * ceil_div(c.Kp16, t.BN) * t.splits; }
 double tiling_us(int ctas, const ConvShape& c, const ConvTiling& t) {
-    const int k_blocks = ceil_div(c.nkb, t.splits), stages = pipeline(ctas, t.BN, k_blocks, t.splits, c.shared).stages;
+    const int k_blocks = ceil_div(c.nkb, t.splits);
+    const Pipeline pipe = pipeline(ctas, t.BN, k_blocks, t.splits, c.shared);
+    const int stages = pipe.stages;
     const double mean = std::max(1.0, ctas / 148.0), per_sm = mean + 0.639 * (ceil_div(ctas, 148) - mean);
     const double crowd = 1.0 + 1.39 * (per_sm - 1.0);
     double kb = std::max(0.197 + 0.0003 * t.BN, per_sm * (16.384 + 0.128 * t.BN) / 137.0);
@@ -1954,7 +1960,10 @@ double tiling_us(int ctas, const ConvShape& c, const ConvTiling& t) {
     double us = 3.68 + k_blocks * kb;
     if (t.tma) us += 0.164 + 0.0081 * t.BN * crowd + (c.residual ? 0.327 + 0.0006 * t.BN * crowd : 0.0);
     else us += (c.residual ? 0.0242 : 0.0114) * t.BN / t.splits * crowd;
-    if (t.splits > 1) us += 0.401 + 0.017 * t.BN + ctas * (t.splits == 2 ? 0.0023 : t.splits == 4 ? 0.0055 : 0.0133);
+    if (t.splits > 1) {
+        if (c.shared) us += 0.401 + 0.017 * t.BN + ctas * (t.splits == 2 ? 0.0023 : t.splits == 4 ? 0.0055 : 0.0133);
+        else us += 0.021 * (t.BN - t.BN / t.splits) + ctas * (t.splits == 2 ? 0.0044 : t.splits == 4 ? 0.0042 : 0.0062) + (pipe.meet ? 0.0 : 0.17);
+    }
     return us;
 }
 // Relative length of a block's stay on its SM.

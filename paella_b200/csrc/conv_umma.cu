@@ -1315,15 +1315,22 @@ conv_umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         const uint32_t idesc = uniform(a.idesc), n_kb = uniform((uint32_t)nkb), n_st = uniform((uint32_t)stages);
         const uint64_t desc_a0 = umma_desc_sw128(uniform(smem_base)), desc_b0 = umma_desc_sw128(uniform(smem_base) + kATileBytes);
         const uint32_t desc_step = uniform(stage_bytes) >> 4;
+        // The last channels of a tap may fill less than a k-block: what is past them are zeros, which need no multiplying (288 -> 384 channels
+        // 3x3 on 64 maps of 35 x 35 150.9 -> 144.5 us; in conv_tile_tma, whose launches the tensor pipe does not bound, the choice costs more than it
+        // saves: ResNet-50 x 8 images 347 -> 352).
+        const uint32_t n_cpt = uniform((uint32_t)cpt), last_slices = uniform((uint32_t)(a.Cs - (cpt - 1) * kBK + 15) >> 4);
+        uint32_t chunk_k = 0;
         for (uint32_t kb = 0; kb < n_kb; ++kb) {
             ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err_flag, 2u));
             if (!ok) break;
             tcgen05_fence_after();
             const uint64_t da = desc_a0 + st * desc_step, db = desc_b0 + st * desc_step;
+            uint32_t slices = kBK / 16;
+            if (++chunk_k == n_cpt) { chunk_k = 0; slices = last_slices; }
             if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < kBK / 16; ++k)
-                    tcgen05_mma_bf16_pair(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                for (uint32_t k = 0; k < kBK / 16; ++k)
+                    if (k < slices) tcgen05_mma_bf16_pair(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
                 tcgen05_commit_pair(smem_u32(&s_empty[st]));
             }
             __syncwarp();

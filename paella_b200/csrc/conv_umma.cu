@@ -111,6 +111,7 @@ struct ConvArgs {
     const float* pre_bias;
     int pre_act;
     uint32_t pre_offset;  // where their part of shared memory begins
+    float inv_PQ, inv_Q, inv_cpt, inv_S;      // reciprocals of the divisors of a block's set-up
 };
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
@@ -171,6 +172,18 @@ __device__ unsigned long long g_conv_ns;             // sum of the CTAs' lifetim
 // copies of each (and of each cluster size), 124 KB of code per kernel, and a launch whose copy had not run on its SM lately
 // spent 0.5 to 1.6 us of its epilogue fetching it.  The loops below are kept rolled for the same reason.  Two copies, ReLU and ReLU6 /
 // the others, are as fast as four where the arguments are constants (the lone launches): see EpiArgs.
+// n / d for n >= 0, with d's reciprocal: a few instructions where the integer division is a chain of twenty to forty (a block's set-up had five
+// of them in a row).  The estimate is off by one at most while the quotient is below 2^22; the loops make it right whatever it is.
+__device__ __forceinline__ int quotient(int n, int d, float inv, int& rem) {
+    int q = (int)((float)n * inv);
+    rem = n - q * d;
+    while (rem < 0) { --q; rem += d; }
+    while (rem >= d) { ++q; rem -= d; }
+    return q;
+}
+// Cluster sizes are powers of two.
+__device__ __forceinline__ int log2_of(int splits) { return 31 - __clz(splits); }
+
 // What the epilogues of grouped and normalising launches need of a convolution's arguments, in registers before they wait for the
 // accumulator.  (A grouped launch has its arguments in shared memory, and a compiler that sees a memory barrier reads them again behind
 // each.)  Lone launches read their arguments where they are, in the constant bank, so that the compiler knows every branch on
@@ -410,13 +423,13 @@ __device__ __forceinline__ uint32_t active_ranks(const Args& a) {
     if (a.nkb >= S) return (1u << S) - 1u;
     uint32_t active = 0;
 #pragma unroll 1
-    for (int z = 0; z < S; ++z) active |= (a.nkb * (z + 1) / S > a.nkb * z / S ? 1u : 0u) << z;
+    for (int z = 0; z < S; ++z) active |= ((a.nkb * (z + 1)) >> log2_of(S) > (a.nkb * z) >> log2_of(S) ? 1u : 0u) << z;
     return active;
 }
 // What arrives at a rank, in bytes.
 template <class Args>
 __device__ __forceinline__ uint32_t meet_bytes(const Args& a, int rank) {
-    return (uint32_t)__popc(active_ranks(a) & ~(1u << rank)) * (uint32_t)(a.BN / a.splits) * 512u;
+    return (uint32_t)__popc(active_ranks(a) & ~(1u << rank)) * (uint32_t)(a.BN >> log2_of(a.splits)) * 512u;
 }
 
 // The columns of this rank: its own part, then the others' in rank order.  `at` is this thread's row of those, [rank but this][4 columns][row].
@@ -482,7 +495,7 @@ __device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_ba
                                                  uint64_t* s_accum_p, uint64_t* s_go, uint64_t* s_parts, volatile uint32_t* s_abort_p) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
-    const int m = m0 + tid, S = a.splits, w = a.BN / S, k0 = n0 + rank * w;
+    const int m = m0 + tid, S = a.splits, w = a.BN >> log2_of(S), k0 = n0 + rank * w;
     const bool row_valid = m < a.M;
     const uint32_t active = active_ranks(a);
     const bool mine = (active >> rank) & 1u;
@@ -507,7 +520,7 @@ __device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_ba
     tcgen05_fence_after();
     bool go = true;
     if (a.meet == 0) {
-        if (tid > 0 && tid < S) mbar_arrive_cluster(cluster_addr(smem_u32(s_go), (uint32_t)((rank + tid) % S)));
+        if (tid > 0 && tid < S) mbar_arrive_cluster(cluster_addr(smem_u32(s_go), (uint32_t)((rank + tid) & (S - 1))));
         __syncwarp();
     }
     uint32_t v0[8], v1[8];
@@ -853,8 +866,9 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
 
     const int m0 = bx * kBM;
     const int n0 = by * a.BN;
-    const int kb_begin = a.nkb * bz / a.splits;
-    const int nkb = a.nkb * (bz + 1) / a.splits - kb_begin;       // 0 for some ranks of a cluster larger than the k-block count
+    const int ranks_log2 = log2_of(a.splits);
+    const int kb_begin = (a.nkb * bz) >> ranks_log2;
+    const int nkb = ((a.nkb * (bz + 1)) >> ranks_log2) - kb_begin;       // 0 for some ranks of a cluster larger than the k-block count
 
     // Operand B's warp sets the barriers up and starts at once on the first turn of the pipeline: the weights are
     // constant, so they need neither the other warps nor the previous kernel.  It also arms each stage's barrier with the
@@ -862,24 +876,24 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
     // moment, and the phase cannot complete before the arrival.)
     const uint32_t tx_bytes = (uint32_t)kATileBytes + a.b_stage_bytes;
     if (warp == kWarpB) {
-        if (elect_one()) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_w) : "memory");
-            for (int s = 0; s < stages; ++s) {
-                mbar_init(smem_u32(&s_full[s]), 1);      // this warp's arrive.expect_tx, for the bytes of both operands
-                mbar_init(smem_u32(&s_empty[s]), 1);     // tcgen05.commit
-                if (kPre) mbar_init(smem_u32(&s_ready[s]), 2);     // normalised: one arrival of each of two warps
-            }
+        // a lane per barrier: one thread took 20 initialisations in a row
+        if (lane < stages) {
+            mbar_init(smem_u32(&s_full[lane]), 1);      // this warp's arrive.expect_tx, for the bytes of both operands
+            mbar_init(smem_u32(&s_empty[lane]), 1);     // tcgen05.commit
+            if (kPre) mbar_init(smem_u32(&s_ready[lane]), 2);     // normalised: one arrival of each of two warps
+        } else if (lane == kMaxStages) {
             mbar_init(smem_u32(s_accum), kPre ? 2 : 1);                // normalised: its memory is free, too
             mbar_init(smem_u32(s_res), 1);
-            if (a.splits > 1) {
-                mbar_init(smem_u32(s_go), (uint32_t)(a.splits - 1));
-                mbar_init(smem_u32(s_parts), 1);
-                mbar_arrive_expect_tx(smem_u32(s_parts), meet_bytes(a, bz));
-            }
             *s_abort = 0;
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        } else if (lane == kMaxStages + 1 && a.splits > 1) {
+            mbar_init(smem_u32(s_go), (uint32_t)(a.splits - 1));
+            mbar_init(smem_u32(s_parts), 1);
+            mbar_arrive_expect_tx(smem_u32(s_parts), meet_bytes(a, bz));
+        } else if (lane == kMaxStages + 2) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_w) : "memory");
         }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         // The first k-block's weights only: its other copies leave in the main loop (six of them here held every warp at the
         // barrier below for 0.3 us a tile).
@@ -896,15 +910,14 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
     const int cpt = a.Cp / kBK;               // k-blocks per filter tap
     if (warp == 4) {
         if (elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(tmap_x) : "memory");
-        img = m0 / a.PQ;                      // the tile may run on into the next image
-        const int rem = m0 - img * a.PQ;
-        const int p0 = rem / a.Q, q0 = rem - p0 * a.Q;
-        w0 = q0 * a.sw - a.pw;                // filter-window origin of the tile's first pixel
-        h0 = p0 * a.sh - a.ph;
-        const int tap = kb_begin / cpt;
-        chunk = kb_begin - tap * cpt;
-        tap_r = tap / a.S;
-        tap_s = tap - tap_r * a.S;
+        if (!a.a_tiled) {
+            int rem, q0;
+            img = quotient(m0, a.PQ, a.inv_PQ, rem);      // the tile may run on into the next image
+            const int p0 = quotient(rem, a.Q, a.inv_Q, q0);
+            w0 = q0 * a.sw - a.pw;                // filter-window origin of the tile's first pixel
+            h0 = p0 * a.sh - a.ph;
+        }
+        if (kb_begin > 0) tap_r = quotient(quotient(kb_begin, cpt, a.inv_cpt, chunk), a.S, a.inv_S, tap_s);
     }
     if (warp == 5) {
         tcgen05_alloc(smem_u32(s_tmem_base), a.tmem_cols);
@@ -1008,7 +1021,7 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         if (kPre) {
             // The epilogue may start once the stages whose memory it uses (for the others' parts or the finished tile) have been stored; the
             // others leave beside it.
-            const uint32_t bytes = a.splits > 1 ? (a.meet ? 0u : (uint32_t)(a.BN - a.BN / a.splits) * 512u) : a.out_box ? (uint32_t)a.BN * 256u : 0u;
+            const uint32_t bytes = a.splits > 1 ? (a.meet ? 0u : (uint32_t)(a.BN - (a.BN >> ranks_log2)) * 512u) : a.out_box ? (uint32_t)a.BN * 256u : 0u;
             const int used = (int)((bytes + stage_bytes - 1) / stage_bytes), last_st = nkb > 0 ? (nkb - 1) % stages : 0;
             const int until = used > 0 ? nkb - 1 - max(0, last_st - (used - 1)) : -1;        // the last k-block in one of them
             auto let_epilogue = [&]() {
@@ -1233,8 +1246,8 @@ conv_umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         __syncwarp();
     }
     const int cpt = a.Cp / kBK;
-    const int img = m0 / a.PQ, rem = m0 - img * a.PQ;
-    const int p0 = rem / a.Q, q0 = rem - p0 * a.Q;
+    int rem, q0;
+    const int img = quotient(m0, a.PQ, a.inv_PQ, rem), p0 = quotient(rem, a.Q, a.inv_Q, q0);
     const int w0 = q0 * a.sw - a.pw, h0 = p0 * a.sh - a.ph;
     if (warp == 4 && elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
     if (warp == 5) {
@@ -1388,9 +1401,11 @@ struct alignas(128) SubConv {
         PoolSubArgs pool;
     };
     uint32_t first_block, gx, gy, stages;
+    float inv_gx;
 };
 static_assert(sizeof(PoolSubArgs) <= sizeof(ConvArgs), "a pooling entry fits where a convolution's arguments are");
 constexpr int kMaxSubConvs = 8;
+struct SubStarts { uint32_t first[kMaxSubConvs]; };      // first block of each entry; past the last entry, of none
 constexpr uint32_t kSubPool = 0xffffffffu;
 constexpr int kPoolVecsPerThread = 2;                 // output vectors (8 channels) per thread of a pooling block
 
@@ -1473,7 +1488,7 @@ __device__ __forceinline__ void pool_sub_block(const PoolSubArgs& a, uint32_t lo
 }
 
 __global__ void __launch_bounds__(kThreadsTma, 3)
-conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t job_id, FinishedBlockNotifier* nf) {
+conv_umma_multi_kernel(const SubConv* __restrict__ table, const SubStarts starts, uint32_t job_id, FinishedBlockNotifier* nf) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxStages];
     __shared__ __align__(8) uint64_t s_empty[kMaxStages];
@@ -1490,16 +1505,22 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
     if (nf) nf->start(job_id);
     if (threadIdx.x == 0) PB_T(0);
 
+    // Which sub-problem: its first block is in the constant bank (looked up in the table it took a chain of up to seven loads from L2).
     int sub = 0;
-    while (sub + 1 < n_sub && blockIdx.x >= table[sub + 1].first_block) ++sub;
+    uint32_t first = 0;
+#pragma unroll
+    for (int i = 1; i < kMaxSubConvs; ++i)
+        if (blockIdx.x >= starts.first[i]) { sub = i; first = starts.first[i]; }
     const SubConv* sc = table + sub;
+    const uint32_t gx = __ldg(&sc->gx), stages = __ldg(&sc->stages);
+    const float inv_gx = __ldg(&sc->inv_gx);
     // the table is constant for the life of the instance: it may be read before griddepcontrol.wait
     static_assert(sizeof(ConvArgs) % 4 == 0, "ConvArgs is copied word by word");
     if (threadIdx.x < sizeof(ConvArgs) / 4)
         reinterpret_cast<uint32_t*>(&s_args)[threadIdx.x] = reinterpret_cast<const uint32_t*>(&sc->a)[threadIdx.x];
     __syncthreads();
-    const uint32_t local = blockIdx.x - sc->first_block;
-    if (sc->stages == kSubPool) {        // a pooling layer riding along: no tensor memory, no pipeline
+    const uint32_t local = blockIdx.x - first;
+    if (stages == kSubPool) {        // a pooling layer riding along: no tensor memory, no pipeline
         griddep_wait();
         griddep_launch();
         pool_sub_block(*reinterpret_cast<const PoolSubArgs*>(&s_args), local);
@@ -1507,10 +1528,10 @@ conv_umma_multi_kernel(const SubConv* __restrict__ table, int n_sub, uint32_t jo
         return;
     }
     // the ranks of a cluster are consecutive blocks (every sub-problem of a launch has the same split)
-    const uint32_t S = (uint32_t)s_args.splits, gx = sc->gx;
-    const uint32_t tile = local / S, bz = local - tile * S;
-    const uint32_t by = tile / gx, bx = tile - by * gx;
-    conv_tile_tma<false, false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, nullptr, s_args, (int)sc->stages, (int)bx, (int)by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
+    const uint32_t S = (uint32_t)s_args.splits, tile = local >> log2_of((int)S), bz = local & (S - 1u);
+    int bx;
+    const int by = quotient((int)tile, (int)gx, inv_gx, bx);
+    conv_tile_tma<false, false>(&sc->tmap_w, &sc->tmap_x, &sc->tmap_y, &sc->tmap_r, nullptr, s_args, (int)stages, bx, by, (int)bz, smem_raw, s_full, s_empty, &s_accum,
                   &s_tmem_base, &s_abort, s_bias, &s_res, nullptr, &s_go, &s_parts, nf != nullptr);
     if (nf) nf->end(job_id);
 }
@@ -2492,6 +2513,7 @@ static int fill_args(const ConvUmmaPlan* plan, const Geometry& g, const pb_op_pa
     a.b_stage_bytes = g.b_stage_bytes;
     a.splits = g.splits;
     a.meet = g.meet;
+    a.inv_PQ = 1.f / (float)a.PQ; a.inv_Q = 1.f / (float)a.Q; a.inv_cpt = 1.f / (float)g.cpt; a.inv_S = 1.f / (float)a.S;
     a.out_box = g.out_box;
     return PB_OK;
 }
@@ -2573,6 +2595,7 @@ struct ConvUmmaMulti {
     unsigned total_blocks = 0;      // tiles of all sub-problems (= CTAs of the one-tile-per-CTA kernel)
     uint32_t smem = 0;
     uint32_t tmem_cols = 0;
+    SubStarts starts;
     unsigned splits = 1;            // cluster size of the launch
     bool has_pool = false;          // pooling layers ride along (one-tile kernel only)
     // persistent kernel
@@ -2648,6 +2671,7 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
         m->splits = (unsigned)g.splits;
         sc.first_block = m->total_blocks;
         sc.gx = (uint32_t)g.m_tiles;
+        sc.inv_gx = 1.f / (float)g.m_tiles;
         sc.gy = (uint32_t)g.n_tiles;
         sc.stages = (uint32_t)g.stages;
         m->total_blocks += (unsigned)(g.m_tiles * g.n_tiles * g.splits);
@@ -2668,6 +2692,7 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
         a.is_max = kinds[i] == PB_STAGE_MAXPOOL; a.count_pad = p->flags & 1; a.batch = batch_of(p);
         sc.first_block = m->total_blocks;
         sc.gx = sc.gy = 1;
+        sc.inv_gx = 1.f;
         sc.stages = kSubPool;
         m->total_blocks += conv_umma_pool_blocks(p);
         m->has_pool = true;
@@ -2679,6 +2704,7 @@ int conv_umma_multi_create(const ConvUmmaPlan* const* plans, const ConvUmmaXMap*
     m->persist_smem = (uint32_t)m->stages * m->stage_bytes + 1024u;
     m->grid = conv_umma_persist_grid(m->total_blocks);
     m->persist = persist_enabled() && m->splits == 1 && m->stages >= 2 && 2u * m->tmem_cols <= 512u && !m->has_pool;
+    for (int i = 0; i < kMaxSubConvs; ++i) m->starts.first[i] = i < n ? table[(size_t)i].first_block : 0xffffffffu;
     cudaError_t e = cudaMalloc((void**)&m->table_dev, sizeof(SubConv) * (size_t)n);
     if (e == cudaSuccess) e = cudaMemcpy(m->table_dev, table.data(), sizeof(SubConv) * (size_t)n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { conv_umma_multi_destroy(m); return cuda_fail(e, "conv_umma_multi_create", __FILE__, __LINE__); }
@@ -2737,7 +2763,7 @@ int conv_umma_multi_launch(const ConvUmmaMulti* m, cudaStream_t st, uint32_t job
         return PB_OK;
     }
     const cudaError_t e = launch_pdl(conv_umma_multi_kernel, dim3(m->total_blocks), dim3(m->splits), m->smem, st, pdl,
-                                     (const SubConv*)m->table_dev, m->n, job_id, static_cast<FinishedBlockNotifier*>(notifier));
+                                     (const SubConv*)m->table_dev, m->starts, job_id, static_cast<FinishedBlockNotifier*>(notifier));
     if (e != cudaSuccess) return cuda_fail(e, "launch of conv_umma_multi_kernel", __FILE__, __LINE__);
     return PB_OK;
 }

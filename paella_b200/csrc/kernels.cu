@@ -757,15 +757,123 @@ __device__ __forceinline__ uint32_t win_finish(uint32_t acc, uint64_t bias, floa
 // capture, where nothing may be.
 static __device__ uint32_t g_window_err_flag;
 
+// What a lane knows of its four channels (from c0 on), and the steps of a walk down the window's rows.
 // kWide: output and filter start on an 8-byte boundary, so a lane's four channels are one access; otherwise two of 4 bytes.
+template <int kMode, int kStride, int kAct, bool kCountPad, bool kWide>
+struct WinLane {
+    typedef __nv_bfloat16 T;
+    typedef typename WinAcc<kMode>::type Acc;
+    static constexpr bool kDw = kMode == kWinDw;
+    static constexpr int kStrip = kStride == 1 ? kTileStrip1 : kTileStrip2, kCols = (kStrip - 1) * kStride + 3;
+    // A window row as the walk wants it: its columns (depthwise), or for pooling each output's three columns already reduced, once
+    // for the three output rows the window row belongs to.
+    static constexpr int kRow = kDw ? kCols : kStrip;
+    uint64_t w[3][3][2], bias[2];
+    uint32_t keep0, keep1;
+    bool tail;
+
+    __device__ __forceinline__ void channels(const OpArgs& a, int c0) {
+        const int c_lim = kDw ? a.K : a.C;
+        if (kDw) {
+            const T* wp = static_cast<const T*>(a.w) + (c0 < a.Cs ? c0 : 0);
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int s2 = 0; s2 < 3; ++s2) {
+                    const T* tap = wp + (r * 3 + s2) * a.Cs;
+                    const uint2 u = kWide ? __ldg(reinterpret_cast<const uint2*>(tap))
+                                          : make_uint2(__ldg(reinterpret_cast<const uint32_t*>(tap)), __ldg(reinterpret_cast<const uint32_t*>(tap) + 1));
+                    w[r][s2][0] = p2_bf16(u.x);
+                    w[r][s2][1] = p2_bf16(u.y);
+                }
+        }
+        bias[0] = bias[1] = 0;
+        tail = !kDw && a.bias != nullptr;
+        if (a.bias) {
+            float f[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) f[j] = c0 + j < c_lim ? a.bias[c0 + j] : 0.f;
+            bias[0] = p2_of(f[0], f[1]);
+            bias[1] = p2_of(f[2], f[3]);
+        }
+        // channels past the last one are stored as zeros
+        keep0 = c0 + 1 < c_lim ? 0xffffffffu : (c0 < c_lim ? 0x0000ffffu : 0u);
+        keep1 = c0 + 3 < c_lim ? 0xffffffffu : (c0 + 2 < c_lim ? 0x0000ffffu : 0u);
+    }
+    __device__ __forceinline__ void row_into(Acc (&acc)[kStrip][2], const Acc (&xv)[kRow][2], int r) const {
+#pragma unroll
+        for (int t = 0; t < kStrip; ++t) {
+            if constexpr (!kDw) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) acc[t][j] = r == 0 ? xv[t][j] : win_step(acc[t][j], xv[t][j], 0, false);
+            } else {
+#pragma unroll
+                for (int s2 = 0; s2 < 3; ++s2) {
+                    if (r == 0 && s2 == 0) {
+                        acc[t][0] = win_open(xv[t * kStride][0], w[0][0][0], true);
+                        acc[t][1] = win_open(xv[t * kStride][1], w[0][0][1], true);
+                        continue;
+                    }
+                    acc[t][0] = win_step(acc[t][0], xv[t * kStride + s2][0], w[r][s2][0], true);
+                    acc[t][1] = win_step(acc[t][1], xv[t * kStride + s2][1], w[r][s2][1], true);
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ void load_row(const uint2* row, Acc (&xv)[kRow][2]) const {
+        Acc col_v[kCols][2];
+#pragma unroll
+        for (int col = 0; col < kCols; ++col) {
+            const uint2 v = row[col * (kTileSlab / 4)];
+            col_v[col][0] = win_value<kMode>(v.x);
+            col_v[col][1] = win_value<kMode>(v.y);
+        }
+#pragma unroll
+        for (int t = 0; t < kRow; ++t)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if constexpr (kDw) xv[t][j] = col_v[t][j];
+                else xv[t][j] = win_step(win_step(col_v[t * kStride][j], col_v[t * kStride + 1][j], 0, false), col_v[t * kStride + 2][j], 0, false);
+            }
+    }
+    // The strip's outputs of row p (nt of them, from column q0 on), finished and stored at y.
+    __device__ __forceinline__ void store_row(const OpArgs& a, const Acc (&acc)[kStrip][2], T* __restrict__ y, int p, int q0, int nt, bool all) const {
+        const float inv9 = 1.f / 9.f;
+        float div = 9.f, inv = inv9;
+        int rows_in = 3;
+        if (kMode == kWinAvg && !kCountPad) rows_in = min(p * kStride - a.pad_h + 3, a.H) - max(p * kStride - a.pad_h, 0);
+#pragma unroll
+        for (int t = 0; t < kStrip; ++t) {
+            if (!all && t >= nt) break;
+            if (kMode == kWinAvg && !kCountPad) {
+                const int cols_in = max(min((q0 + t) * kStride - a.pad_w + 3, a.W) - max((q0 + t) * kStride - a.pad_w, 0), 0);
+                const int cnt = rows_in * cols_in;
+                if (cnt != 9) { div = (float)(cnt > 0 ? cnt : 1); inv = 1.f / div; }
+                else { div = 9.f; inv = inv9; }
+            }
+            uint32_t o0 = win_finish<kMode, kAct>(acc[t][0], bias[0], div, inv, tail);
+            uint32_t o1 = win_finish<kMode, kAct>(acc[t][1], bias[1], div, inv, tail);
+            if (!all) { o0 &= keep0; o1 &= keep1; }
+            if (kWide) {
+                *reinterpret_cast<uint2*>(y + (uint32_t)(t * a.Ks)) = make_uint2(o0, o1);
+            } else {
+                uint32_t* const out = reinterpret_cast<uint32_t*>(y + (uint32_t)(t * a.Ks));
+                out[0] = o0;
+                out[1] = o1;
+            }
+        }
+    }
+    __device__ __forceinline__ bool whole(int nt) const { return nt == kStrip && (keep0 & keep1) == 0xffffffffu; }      // every output of the strip and all four channels exist
+};
+
 template <int kMode, int kStride, int kAct, bool kCountPad, bool kWide>
 __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
                                                                         FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
-    typedef __nv_bfloat16 T;
-    typedef typename WinAcc<kMode>::type Acc;
-    constexpr int kStrip = kStride == 1 ? kTileStrip1 : kTileStrip2, kCols = (kStrip - 1) * kStride + 3;
-    constexpr bool kDw = kMode == kWinDw;
+    typedef WinLane<kMode, kStride, kAct, kCountPad, kWide> Lane;
+    typedef typename Lane::T T;
+    typedef typename Lane::Acc Acc;
+    constexpr int kStrip = Lane::kStrip, kRow = Lane::kRow;
     extern __shared__ __align__(128) unsigned char s_tile[];
     __shared__ __align__(8) uint64_t s_full;
 
@@ -791,33 +899,8 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
 
     const int half = threadIdx.x >> 4, c0 = ch0 + (threadIdx.x & 15) * 4;      // half-warp, first of the lane's four channels
     const bool ch_in = c0 < a.Cs;
-    const int c_lim = kDw ? a.K : a.C;
-    uint64_t w[3][3][2], bias[2] = {0, 0};
-    if (kDw) {
-        const T* wp = static_cast<const T*>(a.w) + (ch_in ? c0 : 0);
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int s2 = 0; s2 < 3; ++s2) {
-                const T* tap = wp + (r * 3 + s2) * a.Cs;
-                const uint2 u = kWide ? __ldg(reinterpret_cast<const uint2*>(tap))
-                                      : make_uint2(__ldg(reinterpret_cast<const uint32_t*>(tap)), __ldg(reinterpret_cast<const uint32_t*>(tap) + 1));
-                w[r][s2][0] = p2_bf16(u.x);
-                w[r][s2][1] = p2_bf16(u.y);
-            }
-    }
-    const bool tail = !kDw && a.bias != nullptr;
-    if (a.bias) {
-        float f[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) f[j] = c0 + j < c_lim ? a.bias[c0 + j] : 0.f;
-        bias[0] = p2_of(f[0], f[1]);
-        bias[1] = p2_of(f[2], f[3]);
-    }
-    // channels past the last one are stored as zeros
-    const uint32_t keep0 = c0 + 1 < c_lim ? 0xffffffffu : (c0 < c_lim ? 0x0000ffffu : 0u);
-    const uint32_t keep1 = c0 + 3 < c_lim ? 0xffffffffu : (c0 + 2 < c_lim ? 0x0000ffffu : 0u);
-    const float inv9 = 1.f / 9.f;
+    Lane lane;
+    lane.channels(a, c0);
     const int pitch = g.in_cols * (kTileSlab / 4);                             // 8-byte words per window row
     __syncthreads();                                                           // the barrier exists
     bool landed = false;
@@ -844,74 +927,17 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
         const int q0 = q_tile + strip * kStrip;
         const int p0 = p_tile + band * g.band_rows, p1 = min(p0 + g.band_rows, p_end);
         const int nt = u0 + half < units && ch_in ? min(kStrip, a.Q - q0) : 0;      // outputs this lane stores
-        const bool full = nt == kStrip && (keep0 & keep1) == 0xffffffffu;           // every output of the strip and all four channels exist
+        const bool full = lane.whole(nt);
         const uint2* row = reinterpret_cast<const uint2*>(s_tile) + (band * g.band_rows * kStride) * pitch + strip * kStrip * kStride * (kTileSlab / 4) + (threadIdx.x & 15);
         T* __restrict__ y = y_img<T>(a) + ((size_t)p0 * a.Q + q0) * a.Ks + a.out_c_off + c0;
 
-        // A window row as the walk wants it: its columns (depthwise), or for pooling each output's three columns already reduced, once
-        // for the three output rows the window row belongs to.
-        constexpr int kRow = kDw ? kCols : kStrip;
-        auto row_into = [&](Acc (&acc)[kStrip][2], const Acc (&xv)[kRow][2], int r) {
-#pragma unroll
-            for (int t = 0; t < kStrip; ++t) {
-                if constexpr (!kDw) {
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) acc[t][j] = r == 0 ? xv[t][j] : win_step(acc[t][j], xv[t][j], 0, false);
-                } else {
-#pragma unroll
-                    for (int s2 = 0; s2 < 3; ++s2) {
-                        if (r == 0 && s2 == 0) {
-                            acc[t][0] = win_open(xv[t * kStride][0], w[0][0][0], true);
-                            acc[t][1] = win_open(xv[t * kStride][1], w[0][0][1], true);
-                            continue;
-                        }
-                        acc[t][0] = win_step(acc[t][0], xv[t * kStride + s2][0], w[r][s2][0], true);
-                        acc[t][1] = win_step(acc[t][1], xv[t * kStride + s2][1], w[r][s2][1], true);
-                    }
-                }
-            }
-        };
+        auto row_into = [&](Acc (&acc)[kStrip][2], const Acc (&xv)[kRow][2], int r) { lane.row_into(acc, xv, r); };
         auto load_row = [&](Acc (&xv)[kRow][2]) {
-            Acc col_v[kCols][2];
-#pragma unroll
-            for (int col = 0; col < kCols; ++col) {
-                const uint2 v = row[col * (kTileSlab / 4)];
-                col_v[col][0] = win_value<kMode>(v.x);
-                col_v[col][1] = win_value<kMode>(v.y);
-            }
-#pragma unroll
-            for (int t = 0; t < kRow; ++t)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    if constexpr (kDw) xv[t][j] = col_v[t][j];
-                    else xv[t][j] = win_step(win_step(col_v[t * kStride][j], col_v[t * kStride + 1][j], 0, false), col_v[t * kStride + 2][j], 0, false);
-                }
+            lane.load_row(row, xv);
             row += pitch;
         };
         auto store_row = [&](const Acc (&acc)[kStrip][2], int p, bool all) {
-            float div = 9.f, inv = inv9;
-            int rows_in = 3;
-            if (kMode == kWinAvg && !kCountPad) rows_in = min(p * kStride - a.pad_h + 3, a.H) - max(p * kStride - a.pad_h, 0);
-#pragma unroll
-            for (int t = 0; t < kStrip; ++t) {
-                if (!all && t >= nt) break;
-                if (kMode == kWinAvg && !kCountPad) {
-                    const int cols_in = max(min((q0 + t) * kStride - a.pad_w + 3, a.W) - max((q0 + t) * kStride - a.pad_w, 0), 0);
-                    const int cnt = rows_in * cols_in;
-                    if (cnt != 9) { div = (float)(cnt > 0 ? cnt : 1); inv = 1.f / div; }
-                    else { div = 9.f; inv = inv9; }
-                }
-                uint32_t o0 = win_finish<kMode, kAct>(acc[t][0], bias[0], div, inv, tail);
-                uint32_t o1 = win_finish<kMode, kAct>(acc[t][1], bias[1], div, inv, tail);
-                if (!all) { o0 &= keep0; o1 &= keep1; }
-                if (kWide) {
-                    *reinterpret_cast<uint2*>(y + (uint32_t)(t * a.Ks)) = make_uint2(o0, o1);
-                } else {
-                    uint32_t* const out = reinterpret_cast<uint32_t*>(y + (uint32_t)(t * a.Ks));
-                    out[0] = o0;
-                    out[1] = o1;
-                }
-            }
+            lane.store_row(a, acc, y, p, q0, nt, all);
             y += (size_t)a.Q * a.Ks;
         };
         // output rows are closed in order: p is the one after the last closed, rows before p0 and from p1 on are not stored
@@ -953,6 +979,153 @@ __global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs
             row_into(acc, xv, 2);
             close_row(acc, p1 - 1);
         }
+    }
+    PB_NOTIFY_END();
+}
+
+// The depthwise walk (stride 1) over tensors of many rows, with the window in a ring: a fixed number of blocks share all rows of all
+// (image, column tile) units of their slab between them, each a contiguous range, and walk down it while one warp copies the next three window
+// rows.  A tile of window3_tile_kernel reads two rows more than the thirteen it writes; here that is once per unit or range, and the blocks
+// neither fill and walk in turn nor end in waves.  Bound by DRAM with reads and writes mixed: 128 x 1024 x 1024 104 -> 95.5 us (86 % of the copy
+// rate), and 98, 104 and 108 with rings of three, four and five stages - more rows under way are more places open at once; with the slabs of
+// a pixel in different ranges 113.  Average pooling gains nothing here (256 maps of 35 x 35 x 192: tiles 49.2, rings 49.4 to 55 us).
+constexpr int kRingStages = 2;
+struct WinRing {
+    int col_tiles, strips, in_cols, slabs;
+    int rows;                       // output rows of a slab, all images and column tiles
+    int blocks, threads;            // no blocks: the launch keeps its tiles
+    int stage_bytes, smem;
+};
+// A block's next piece of work: rows [p0, p1) of one unit.
+struct WinPiece {
+    int img, col, p0, p1;
+    __device__ __forceinline__ void at(const WinRing& g, int P, int row, int end) {
+        const int unit = row / P;
+        p0 = row - unit * P;
+        p1 = min(P, p0 + end - row);
+        img = unit / g.col_tiles;
+        col = unit - img * g.col_tiles;
+    }
+};
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, volatile uint32_t* s_abort) {
+    for (int i = 0; i < (1 << 22); ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((i & 63) == 63 && *s_abort) return false;
+    }
+    *s_abort = 1;
+    atomicExch(&g_window_err_flag, 6u);
+    return false;
+}
+
+// (128 registers: at most four walking warps.)
+template <int kAct, bool kWide>
+__global__ void __launch_bounds__(160, 3) window3_ring_kernel(OpArgs a, const WinRing g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
+                                                                                FinishedBlockNotifier* nf) {
+    PB_NOTIFY_START();
+    typedef WinLane<kWinDw, 1, kAct, true, kWide> Lane;
+    typedef typename Lane::T T;
+    typedef typename Lane::Acc Acc;
+    constexpr int kStrip = Lane::kStrip, kRow = Lane::kRow;
+    extern __shared__ __align__(128) unsigned char s_ring[];
+    __shared__ __align__(8) uint64_t s_full[kRingStages], s_empty[kRingStages];
+    __shared__ volatile uint32_t s_abort;
+
+    const int warp = threadIdx.x >> 5, walkers = (blockDim.x >> 5) - 1;
+    const uint32_t full = (uint32_t)__cvta_generic_to_shared(s_full), empty = (uint32_t)__cvta_generic_to_shared(s_empty);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kRingStages; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8u * i));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty + 8u * i), "r"(walkers));
+        }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    // neighbouring blocks take the slabs of the same rows: together they read whole pixels
+    const int range = (int)blockIdx.x / g.slabs, slab = (int)blockIdx.x - range * g.slabs, ranges = (int)gridDim.x / g.slabs;
+    const int begin = (int)((long long)g.rows * range / ranges), end = (int)((long long)g.rows * (range + 1) / ranges);
+    WinPiece piece;
+    int st = 0;
+    uint32_t parity = 0;
+
+    if (warp == walkers) {
+        // ===== copies: three window rows a stage =====
+        if ((threadIdx.x & 31) == 0) {
+            int turn = 0;
+            bool ok = true;
+            for (int row = begin; row < end && ok; row += piece.p1 - piece.p0) {
+                piece.at(g, a.P, row, end);
+                const int ch0 = slab * kTileSlab, iw0 = piece.col * g.strips * kStrip - a.pad_w;
+                for (int p = piece.p0; p < piece.p1 + 2 && ok; p += 3) {
+                    if (turn >= kRingStages) ok = ring_wait(empty + 8u * st, parity ^ 1u, &s_abort);
+                    if (!ok) break;
+                    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(full + 8u * st), "r"(g.stage_bytes) : "memory");
+                    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(s_ring) + (uint32_t)(st * g.stage_bytes)), "l"(&tmap), "r"(ch0), "r"(iw0), "r"(p - a.pad_h), "r"(piece.img),
+                                 "r"(full + 8u * st)
+                                 : "memory");
+                    ++turn;
+                    if (++st == kRingStages) { st = 0; parity ^= 1u; }
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ===== walks =====
+        const int half = threadIdx.x >> 4, strip = min(half, g.strips - 1);        // (a last half-warp without a strip repeats one and stores nothing)
+        const int pitch = g.in_cols * (kTileSlab / 4);                             // 8-byte words per window row
+        const uint2* const ring0 = reinterpret_cast<const uint2*>(s_ring) + strip * kStrip * (kTileSlab / 4) + (threadIdx.x & 15);
+        const int c0 = slab * kTileSlab + (threadIdx.x & 15) * 4;
+        Lane lane;
+        lane.channels(a, c0);
+        bool ok = true;
+        for (int at = begin; at < end && ok; at += piece.p1 - piece.p0) {
+            piece.at(g, a.P, at, end);
+            const int q0 = (piece.col * g.strips + strip) * kStrip, p0 = piece.p0, p1 = piece.p1;
+            const int nt = half < g.strips && c0 < a.Cs ? min(kStrip, a.Q - q0) : 0;      // outputs this lane stores
+            const bool whole = lane.whole(nt);
+            T* __restrict__ y = static_cast<T*>(a.y) + (((size_t)piece.img * a.P + p0) * a.Q + q0) * a.Ks + a.out_c_off + c0;
+            auto close_row = [&](const Acc (&acc)[kStrip][2], int p) {
+                if (p >= p0 && p < p1) {
+                    if (whole) lane.store_row(a, acc, y, p, q0, nt, true);
+                    else lane.store_row(a, acc, y, p, q0, nt, false);
+                    y += (size_t)a.Q * a.Ks;
+                }
+            };
+            // window row r opens output row p0 + r (filter row 0), continues p0 + r - 1, closes p0 + r - 2; three window rows per turn
+            Acc accA[kStrip][2], accB[kStrip][2], accC[kStrip][2];
+#pragma unroll
+            for (int t = 0; t < kStrip; ++t)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) accB[t][j] = accC[t][j] = 0;          // (rows before p0: never stored)
+#pragma unroll 1
+            for (int p = p0; p < p1 + 2; p += 3) {
+                ok = __all_sync(0xffffffffu, ring_wait(full + 8u * st, parity, &s_abort));
+                if (!ok) break;
+                const uint2* row = ring0 + (size_t)st * (g.stage_bytes / 8);
+                Acc xv[kRow][2];
+                lane.load_row(row, xv); lane.row_into(accB, xv, 2); lane.row_into(accC, xv, 1); lane.row_into(accA, xv, 0); close_row(accB, p - 2);
+                lane.load_row(row + pitch, xv); lane.row_into(accC, xv, 2); lane.row_into(accA, xv, 1); lane.row_into(accB, xv, 0); close_row(accC, p - 1);
+                lane.load_row(row + 2 * pitch, xv); lane.row_into(accA, xv, 2); lane.row_into(accB, xv, 1); lane.row_into(accC, xv, 0);
+                __syncwarp();
+                if ((threadIdx.x & 31) == 0) asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.shared::cta.b64 s, [%0];\n\t}" ::"r"(empty + 8u * st) : "memory");
+                close_row(accA, p);
+                if (++st == kRingStages) { st = 0; parity ^= 1u; }
+            }
+        }
+    }
+    __syncthreads();
+    if (s_abort) {          // copies are given 50 us more to land before shared memory is released
+        unsigned long long t0, t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        for (int i = 0; i < (1 << 20); ++i) {
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t - t0 > 50000ull) break;
+        }
+        __syncthreads();
     }
     PB_NOTIFY_END();
 }
@@ -1796,6 +1969,39 @@ static const void* tile_fn(int kind, const pb_op_params* p) {
     return (at & 7) == 0 ? tile_fn<true>(kind, p) : tile_fn<false>(kind, p);
 }
 
+// Ring of a launch's window: depthwise windows of stride 1 whose column tiles have seven or eight strips (four walking warps; with five
+// strips, 256 maps of 64 x 40 x 16, 37 us become 47) and whose rows give every block 24 and more (a block's range starts with two rows of
+// no output; fewer blocks than the GPU holds lose more than the ring gains).  Tiles / ring: 64 maps of 112 x 112 x 128 86.0 / 82.0 us, 32 of
+// 224 x 224 x 64 83.6 / 71.9, 4 of 300 x 500 x 96 63.4 / 55.5, 64 of 57 x 57 x 200 50.6 / 45.7, 2 of 200 x 200 x 640 45.3 / 44.8.
+static WinRing win_ring(int kind, const pb_op_params* p) {
+    WinRing g = {};
+    if (kind != PB_STAGE_DWCONV || p->stride_h != 1 || p->stride_w != 1 || tile_blocks(p) == 0) return g;
+    g.strips = ceil_div(ceil_div(p->Q, ceil_div(p->Q, 32)), kTileStrip1);
+    g.col_tiles = ceil_div(p->Q, g.strips * kTileStrip1);
+    g.slabs = ceil_div(p->Cs, kTileSlab);
+    g.in_cols = g.strips * kTileStrip1 + 2;
+    g.stage_bytes = 3 * g.in_cols * kTileSlab * 2;
+    g.smem = kRingStages * g.stage_bytes;
+    g.threads = 32 * (ceil_div(g.strips, 2) + 1);
+    const int ranges = 3 * 148 / g.slabs;
+    const long long rows = (long long)batch_of(p) * g.col_tiles * p->P;      // of a slab
+    if (g.strips < 7 || ranges < 1 || rows < 24ll * ranges || rows > 0x3fffffff) return g;
+    g.rows = (int)rows;
+    g.blocks = ranges * g.slabs;
+    return g;
+}
+static int ring_map(const pb_op_params* p, const WinRing& g, CUtensorMap* out) {
+    const uint64_t dims[4] = {(uint64_t)p->Cs, (uint64_t)p->W, (uint64_t)p->H, (uint64_t)batch_of(p)};
+    const uint64_t strides[3] = {(uint64_t)p->Cs * 2, (uint64_t)p->W * p->Cs * 2, (uint64_t)p->H * p->W * p->Cs * 2};
+    const uint32_t box[4] = {(uint32_t)kTileSlab, (uint32_t)g.in_cols, 3, 1};
+    return encode_tiled_bf16(p->x, 4, dims, strides, box, false, out);
+}
+static const void* ring_fn(const pb_op_params* p) {
+#define PB_RING(W) (p->act == 2 ? (const void*)window3_ring_kernel<2, W> : p->act == 1 ? (const void*)window3_ring_kernel<1, W> : (const void*)window3_ring_kernel<0, W>)
+    return ((reinterpret_cast<uintptr_t>(p->y) | reinterpret_cast<uintptr_t>(p->w)) & 7) == 0 ? PB_RING(true) : PB_RING(false);
+#undef PB_RING
+}
+
 template <int kMode>
 static const void* window3_fn(bool f32, int stride, int strip) {
 #define PB_W3(T) (stride == 1 ? (strip == 1 ? (const void*)window3_strip_kernel<T, kMode, 1, 1> : (const void*)window3_strip_kernel<T, kMode, 1, kStripWide1>) \
@@ -1934,13 +2140,22 @@ int simple_op_info(int kind, const pb_op_params* p, pb_launch_info* out) {
     if (kind == PB_STAGE_CONV_SIMT && conv_f32_supported(p)) return conv_f32_info(p, out);
     const int nb = batch_of(p);
     const int rc = info_one_image(kind, p, out);
-    if (rc != PB_OK || nb == 1) return rc;
+    if (rc != PB_OK) return rc;
+    const WinRing ring = win_ring(kind, p);
+    if (ring.blocks) {          // the blocks share all images
+        out->num_blocks = (uint32_t)ring.blocks;
+        out->regs_per_thread = regs_of(ring_fn(p));
+        out->smem_per_block = (uint32_t)ring.smem;
+        out->threads_per_block = (uint32_t)ring.threads;
+    }
+    if (nb == 1) return rc;
     if (folds_batch(kind)) {
         pb_op_params q = *p;
         q.H *= nb;
         return info_one_image(kind, &q, out);
     }
     out->num_blocks *= (uint32_t)nb;
+    if (ring.blocks) out->num_blocks = (uint32_t)ring.blocks;
     out->flops *= (uint64_t)nb;
     // the weights are read once per launch whatever the batch
     const uint64_t es = p->dtype == 0 ? 4 : 2;
@@ -2026,6 +2241,16 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
         case PB_STAGE_DWCONV:
             PB_REQUIRE(a.groups == a.C && a.K == a.C, "dwconv: needs groups == C == K");
             PB_REQUIRE((a.Ks % N) == 0 && (a.out_c_off % N) == 0, "dwconv: output slice must be vector aligned");
+            if (const WinRing r = win_ring(kind, p); r.blocks) {
+                const void* fn = ring_fn(p);
+                PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, r.smem));
+                t_launch_smem = (size_t)r.smem;
+                CUtensorMap tmap;
+                const int mrc = ring_map(p, r, &tmap);
+                if (mrc != PB_OK) return mrc;
+                launch_k((void (*)(OpArgs, const WinRing, const CUtensorMap, uint32_t, FinishedBlockNotifier*))fn, dim3((unsigned)r.blocks), dim3((unsigned)r.threads), st, pdl, a, r, tmap, job_id, nf);
+                break;
+            }
             if (tile_blocks(p)) {
                 const WinTile g = win_tile(p);
                 const void* fn = tile_fn(kind, p);

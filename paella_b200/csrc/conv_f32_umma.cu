@@ -195,64 +195,39 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int m0 = (int)blockIdx.x * kRows, n0 = (int)blockIdx.y * BN, rank = (int)blockIdx.z;
     const int steps = (f.chunks + 1) / 2;                          // of 64 k
-    const int kb0 = steps * rank / f.splits, n_kb = steps * (rank + 1) / f.splits - kb0;
+    const int ranks_log2 = 31 - __clz(f.splits);                   // (a power of two)
+    const int kb0 = (steps * rank) >> ranks_log2, n_kb = ((steps * (rank + 1)) >> ranks_log2) - kb0;
     constexpr uint32_t ring = L::ring;
     uint32_t* const err = &g_f32_err_flag;
 
-    if (warp == kWarpCopy) {
-        if (elect_one()) {
+    if (warp == kWarpCopy) {            // a lane per barrier
+        if (lane < (int)ring) {
+            mbar_init(smem_u32(&s_full[lane]), 1);
+            mbar_init(smem_u32(&s_empty[lane]), 16);
+        } else if (lane >= 8 && lane < 10) {
+            mbar_init(smem_u32(&s_ready[lane - 8]), 16);
+            mbar_init(smem_u32(&s_done[lane - 8]), 1);
+            mbar_init(smem_u32(&s_free[lane - 8]), 8);
+        } else if (lane == 16) {
+            mbar_init(smem_u32(&s_sums), 1);
+            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(&s_sums), (uint32_t)((f.splits - 1) * (kRows >> ranks_log2) * BN * 4));
+            s_abort = 0;
+        } else if (lane == 24) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-            for (uint32_t i = 0; i < ring; ++i) {
-                mbar_init(smem_u32(&s_full[i]), 1);
-                mbar_init(smem_u32(&s_empty[i]), 16);
-            }
-            for (int i = 0; i < 2; ++i) {
-                mbar_init(smem_u32(&s_ready[i]), 16);
-                mbar_init(smem_u32(&s_done[i]), 1);
-                mbar_init(smem_u32(&s_free[i]), 8);
-            }
-            mbar_init(smem_u32(&s_sums), 1);
-            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(&s_sums), (uint32_t)((f.splits - 1) * (kRows / f.splits) * BN * 4));
-            s_abort = 0;
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            fence_proxy_async();
         }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async();
         __syncwarp();
     }
     if (warp == kWarpMma) {
         tcgen05_alloc(smem_u32(&s_tmem_base), kTmemCols);
         tcgen05_relinquish();
     }
-    // Where the tile's pixels and this rank's k begin (worked out before the previous launch has to be waited for).
-    int c_chunk = 2 * kb0, c_tap = c_chunk / f.cpt, c_c = c_chunk - c_tap * f.cpt, c_r = 0, c_s = 0, img = 0, w_org = 0, h_org = 0;
-    if (warp == kWarpCopy) {
-        c_r = c_tap / a.S;
-        c_s = c_tap - c_r * a.S;
-        img = m0 / f.PQ;
-        const int rem = m0 - img * f.PQ, p = rem / a.Q, q = rem - p * a.Q;
-        w_org = q * a.stride_w - a.pad_w;
-        h_org = p * a.stride_h - a.pad_h;
-    }
-    // The weights are constants: those of the first steps are on their way before the previous launch has to be waited for.  (A stage's barrier
-    // is armed with the bytes of both operands.)
-    auto copy_weights = [&](int kb, uint32_t st, int chunk, int& tap, int& cc) {
-        const int have = min(2, f.chunks - chunk);
-        const uint32_t bar = smem_u32(&s_full[st]), to = smem + st * L::stage + L::raw_w;
-        if (elect_one()) mbar_arrive_expect_tx(bar, (uint32_t)have * (kBox + L::w_box));
-        for (int h = 0; h < have; ++h) {
-            if (elect_one()) tma_load_3d(to + (uint32_t)h * L::w_box, &tmap_w, n0, cc * kChunk, tap, bar);
-            __syncwarp();
-            if (++cc == f.cpt) { cc = 0; ++tap; }
-        }
-    };
-    int w_tap = c_tap, w_c = c_c, w_ahead = min((int)ring, n_kb);
-    if (warp == kWarpCopy)
-        for (int kb = 0; kb < w_ahead; ++kb) copy_weights(kb, (uint32_t)kb, c_chunk + 2 * kb, w_tap, w_c);
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    if (f.splits > 1) cluster_arrive();        // the sums' barrier is set up (the one wait for it: where sums are sent)
+    if (f.splits > 1) cluster_arrive_relaxed();        // (the barriers' fence has released them; a release here takes 1100 clocks)
     const uint32_t tmem = uniform(s_tmem_base);
 
     if (warp >= kWarpA) griddep_launch();       // the next launch's blocks may have the SMs that this one leaves idle
@@ -260,6 +235,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         // ===== sums =====
         griddep_wait();
         griddep_launch();
+        if (f.splits > 1) cluster_wait();              // every block of the cluster is running and has set its barriers up
         constexpr int kCols = BN / 2;                  // of this thread, of one row
         const int row = tid & 127, col0 = (tid >> 7) * kCols;
         if (tid < BN) {
@@ -297,13 +273,12 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         // owner's shared memory and count on its barrier), laid out as [rank][row][channel], 16-byte chunks in an order that keeps both the
         // writers (a row each) and the readers (a chunk each) free of bank conflicts.
         const uint32_t meet = smem + L::meet;
-        const int share = kRows / f.splits;
+        const int share = kRows >> ranks_log2;
         {
-            const int owner = row / share, rl = row - owner * share;
+            const int owner = row >> (7 - ranks_log2), rl = row & (share - 1);
             const uint32_t at = meet + (uint32_t)((rank * share + rl) * (BN * 4)), mix = (uint32_t)rl & 7u;
             uint32_t to = at, bar = 0;
             if (f.splits > 1) {
-                cluster_wait();                 // every block of the cluster is running
                 to = cluster_addr(at, (uint32_t)owner);
                 bar = cluster_addr(smem_u32(&s_sums), (uint32_t)owner);
             }
@@ -494,13 +469,41 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         }
     } else if (warp == kWarpCopy) {
         // ===== copies =====
+        // The weights are constants: those of the first steps are on their way before the previous launch has to be waited for.  (A stage's barrier
+        // is armed with the bytes of both operands.)
+        int chunk = 2 * kb0, c = chunk, r = 0, s = 0, tap = 0;
+        if (kb0 > 0) {
+            tap = chunk / f.cpt;
+            c = chunk - tap * f.cpt;
+            r = tap / a.S;
+            s = tap - r * a.S;
+        }
+        int w_tap = tap, w_c = c;
+        auto copy_weights = [&](uint32_t st, int chunk_w) {
+            const int have = min(2, f.chunks - chunk_w);
+            const uint32_t bar = smem_u32(&s_full[st]), to = smem + st * L::stage + L::raw_w;
+            if (elect_one()) mbar_arrive_expect_tx(bar, (uint32_t)have * (kBox + L::w_box));
+            for (int h = 0; h < have; ++h) {
+                if (elect_one()) tma_load_3d(to + (uint32_t)h * L::w_box, &tmap_w, n0, w_c * kChunk, w_tap, bar);
+                __syncwarp();
+                if (++w_c == f.cpt) { w_c = 0; ++w_tap; }
+            }
+        };
+        const int ahead = min((int)ring, n_kb);
+        for (int kb = 0; kb < ahead; ++kb) copy_weights((uint32_t)kb, chunk + 2 * kb);
+        int img = 0, w_org = 0, h_org = 0;
+        if (!f.a_tiled) {
+            img = m0 / f.PQ;
+            const int rem = m0 - img * f.PQ, p = rem / a.Q, q = rem - p * a.Q;
+            w_org = q * a.stride_w - a.pad_w;
+            h_org = p * a.stride_h - a.pad_h;
+        }
         griddep_wait();                            // the pixels are the previous launch's
-        int r = c_r, s = c_s, c = c_c, chunk = c_chunk;
         uint32_t st = 0, parity = 1u;
         for (int kb = 0; kb < n_kb; ++kb) {
             if (kb >= (int)ring) {
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, &s_abort, err, 0x25u))) break;
-                copy_weights(kb, st, chunk, w_tap, w_c);
+                copy_weights(st, chunk);
             }
             const int have = min(2, f.chunks - chunk);
             const uint32_t bar = smem_u32(&s_full[st]);

@@ -22,9 +22,9 @@
 // the blocks of a cluster, whose sums meet through distributed shared memory, in rank order: results do not depend on timing.
 //
 // Bound by the instructions of the splitting warps (about 1250 issue slots a scheduler and step) and, where a launch has few steps, by the
-// latency of a step's chain: 0.74 us at 64 columns, 0.66 at 32.  Measured against the kernel on the fp32 units, us a launch in a chain:
-// 64 -> 64 3x3 on 2 maps of 56 x 56 23.1 -> 9.3, 128 -> 128 on 2 of 28 x 28 21.7 -> 10.1, 512 -> 512 on 2 of 7 x 7 29.2 -> 13.0, 256 -> 256 on 16 of
-// 28 x 28 408 -> 98 (151 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 235.  Error against 64 bits, relative, fp32 units / here:
+// latency of a step's chain: 0.76 us at 64 columns, 0.68 at 32.  Measured against the kernel on the fp32 units, us a launch in a chain:
+// 64 -> 64 3x3 on 2 maps of 56 x 56 23.1 -> 8.8, 128 -> 128 on 2 of 28 x 28 21.7 -> 9.5, 512 -> 512 on 2 of 7 x 7 29.2 -> 12.5, 256 -> 256 on 16 of
+// 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 223.  Error against 64 bits, relative, fp32 units / here:
 // 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
 //
 // Infinities, NaN and values that round to infinity in bf16 make 0 x inf of the parts: an output that is not finite is computed again,
@@ -584,16 +584,16 @@ SplitGeometry split_geometry(const pb_op_params* p) {
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kRows);
     const int steps = ceil_div(g.chunks, 2);
     // Least modelled time: waves of one block an SM, each a block's fixed time (operand latency, the meeting of the ranks' sums, stores) and
-    // its steps.  Measured in chains of equal launches, tile width / ranks -> us: 256 -> 256 channels 3x3 on 2 maps of 14 x 14 64/1 31.3, 64/2 18.2,
-    // 64/4 12.0, 64/8 18.4 (two waves), 32/1 27.7, 32/2 16.1, 32/4 11.9; 64 -> 64 on 2 of 56 x 56 11.1, 9.3, 15.9, -, 10.2, 15.4, 22.1;
-    // 512 -> 512 on 2 of 7 x 7 58.2, 31.7, 18.7, 13.0, 52.3, 28.1, 16.2, 21.6.
-    static const struct { int splits, blocks; double fixed[2]; } kRanks[] = {{1, 148, {4.4, 4.8}}, {2, 148, {4.8, 5.2}}, {4, 132, {5.0, 5.4}}, {8, 120, {5.3, 6.2}}};
+    // its steps.  Measured in chains of equal launches, tile width / ranks -> us: 256 -> 256 channels 3x3 on 2 maps of 14 x 14 64/1 31.4, 64/2 18.2,
+    // 64/4 11.9, 64/8 17.5 (two waves), 32/1 27.6, 32/2 15.9, 32/4 11.1; 512 -> 512 on 2 of 7 x 7 58.6, 31.8, 18.6, 12.5, 52.2, 28.0, 16.1, 20.6; 512 -> 512
+    // 1x1 on one of 14 x 14 9.9, 7.4, 6.2, -, 8.5, 6.2, 5.9.
+    static const struct { int splits, blocks; double fixed[2]; } kRanks[] = {{1, 148, {3.2, 4.0}}, {2, 148, {3.7, 4.6}}, {4, 132, {4.2, 5.1}}, {8, 120, {4.6, 5.6}}};
     double best = 1e30;
     for (int wide = 0; wide < (p->K > 32 ? 2 : 1); ++wide)
         for (const auto& c : kRanks) {
             if (c.splits > 1 && (steps < 2 * c.splits || conv_split_gain_us() > 1e6)) break;
             const int BN = wide ? 64 : 32, blocks = g.m_tiles * ceil_div(p->K, BN) * c.splits;
-            const double us = ceil_div(blocks, c.blocks) * (c.fixed[wide] + ceil_div(steps, c.splits) * (wide ? 0.74 : 0.66));
+            const double us = ceil_div(blocks, c.blocks) * (c.fixed[wide] + ceil_div(steps, c.splits) * (wide ? 0.755 : 0.683));
             if (us < best) { best = us; g.BN = BN; g.splits = c.splits; }
         }
     g.n_tiles = ceil_div(p->K, g.BN);

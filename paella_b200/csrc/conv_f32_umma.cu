@@ -24,7 +24,7 @@
 // Bound by the instructions of the splitting warps (about 1250 issue slots a scheduler and step) and, where a launch has few steps, by the
 // latency of a step's chain: 0.76 us at 64 columns, 0.68 at 32.  Measured against the kernel on the fp32 units, us a launch in a chain:
 // 64 -> 64 3x3 on 2 maps of 56 x 56 23.1 -> 8.8, 128 -> 128 on 2 of 28 x 28 21.7 -> 9.5, 512 -> 512 on 2 of 7 x 7 29.2 -> 12.5, 256 -> 256 on 16 of
-// 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 223.  Error against 64 bits, relative, fp32 units / here:
+// 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 212.  Error against 64 bits, relative, fp32 units / here:
 // 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
 //
 // Infinities, NaN and values that round to infinity in bf16 make 0 x inf of the parts: an output that is not finite is computed again,
@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstdlib>
+#include <cstring>
 #include <type_traits>
 
 #include "conv_f32.h"
@@ -54,9 +55,9 @@ __device__ uint32_t g_f32_err_flag;      // raised when a bounded wait runs out
 
 namespace {
 
-constexpr int kRows = 128, kChunk = 32;             // pixels of a tile, channels of a copy box
+constexpr int kTileRows = 128, kChunk = 32;             // pixels of a tile, channels of a copy box
 constexpr int kMaxRing = 4;
-constexpr uint32_t kBox = kRows * kChunk * 4;       // 16 KB
+constexpr uint32_t kBox = kTileRows * kChunk * 4;       // 16 KB
 constexpr int kWarpA = 8, kWarpB = 16, kWarpCopy = 24, kWarpMma = 25;
 constexpr int kThreadsF = 26 * 32;
 constexpr uint32_t kTmemCols = 512;
@@ -76,7 +77,7 @@ struct Layout {
     static constexpr uint32_t ring = BN == 64 ? 3 : 4;
     static constexpr uint32_t raw_w = 2 * kBox, w_box = kChunk * BN * 4, stage = raw_w + 2 * w_box;
     static constexpr uint32_t part = BN * 128, parts = ring * stage, parts_step = 3 * part;
-    static constexpr uint32_t meet = parts + 2 * parts_step, bytes = meet + kRows * BN * 4;
+    static constexpr uint32_t meet = parts + 2 * parts_step, bytes = meet + kTileRows * BN * 4;
     static constexpr uint32_t acc = 0, a = 4 * BN;
 };
 
@@ -175,7 +176,10 @@ __device__ __forceinline__ void finish4(const OpArgs& a, int m, int k, float4 v,
     }
 }
 
-template <int BN>
+// kRows: a stem, whose pixels have four channels (up to four of them real).  There a chunk is a row of the filter - up to eight pixels side by
+// side, 32 values - and the splitting warps read the pixels themselves: a tap of its own would fill an eighth of a chunk.  (7 x 7, stride 2, 64
+// channels on 2 maps of 224 x 224: 32.3 us on the fp32 units, 17.9 here.)
+template <int BN, bool kRows>
 __global__ void __launch_bounds__(kThreadsF, 1)
 conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ SplitArgs f, uint32_t job_id, FinishedBlockNotifier* nf) {
     extern __shared__ uint8_t smem_raw[];
@@ -193,7 +197,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = (int)uniform((uint32_t)tid >> 5);
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int m0 = (int)blockIdx.x * kRows, n0 = (int)blockIdx.y * BN, rank = (int)blockIdx.z;
+    const int m0 = (int)blockIdx.x * kTileRows, n0 = (int)blockIdx.y * BN, rank = (int)blockIdx.z;
     const int steps = (f.chunks + 1) / 2;                          // of 64 k
     const int ranks_log2 = 31 - __clz(f.splits);                   // (a power of two)
     const int kb0 = (steps * rank) >> ranks_log2, n_kb = ((steps * (rank + 1)) >> ranks_log2) - kb0;
@@ -203,17 +207,17 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     if (warp == kWarpCopy) {            // a lane per barrier
         if (lane < (int)ring) {
             mbar_init(smem_u32(&s_full[lane]), 1);
-            mbar_init(smem_u32(&s_empty[lane]), 16);
+            mbar_init(smem_u32(&s_empty[lane]), kRows ? 8 : 16);
         } else if (lane >= 8 && lane < 10) {
             mbar_init(smem_u32(&s_ready[lane - 8]), 16);
             mbar_init(smem_u32(&s_done[lane - 8]), 1);
             mbar_init(smem_u32(&s_free[lane - 8]), 8);
         } else if (lane == 16) {
             mbar_init(smem_u32(&s_sums), 1);
-            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(&s_sums), (uint32_t)((f.splits - 1) * (kRows >> ranks_log2) * BN * 4));
+            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(&s_sums), (uint32_t)((f.splits - 1) * (kTileRows >> ranks_log2) * BN * 4));
             s_abort = 0;
         } else if (lane == 24) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+            if (!kRows) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -273,7 +277,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         // owner's shared memory and count on its barrier), laid out as [rank][row][channel], 16-byte chunks in an order that keeps both the
         // writers (a row each) and the readers (a chunk each) free of bank conflicts.
         const uint32_t meet = smem + L::meet;
-        const int share = kRows >> ranks_log2;
+        const int share = kTileRows >> ranks_log2;
         {
             const int owner = row >> (7 - ranks_log2), rl = row & (share - 1);
             const uint32_t at = meet + (uint32_t)((rank * share + rl) * (BN * 4)), mix = (uint32_t)rl & 7u;
@@ -383,14 +387,41 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         const int h = (warp >> 2) & 1;                             // this thread's box
         const uint32_t at0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + L::a + (uint32_t)(h * 16);
         uint32_t st = 0, parity = 0;
+        // kRows: where this thread's filter window begins
+        int ih0 = 0, iw0 = 0;
+        const float4* image = nullptr;
+        if constexpr (kRows) {
+            const int m = m0 + (int)row, img = m / f.PQ, rem = m - img * f.PQ, p = rem / a.Q, q = rem - p * a.Q;
+            ih0 = m < f.M ? p * a.stride_h - a.pad_h : -(1 << 28);      // fails every bounds check
+            iw0 = q * a.stride_w - a.pad_w;
+            image = static_cast<const float4*>(a.x) + (size_t)(m < f.M ? img : 0) * a.H * a.W;
+            griddep_wait();                        // the pixels are the previous launch's
+        }
         for (int kb = 0; kb < n_kb; ++kb) {
             const int t = kb & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err, 0x22u))) break;
             const bool have = 2 * (kb0 + kb) + h < f.chunks;       // an odd number of chunks ends with half a step
-            const uint32_t from = smem + st * L::stage + (uint32_t)h * kBox + row * 128u;
             uint4 v[8];
+            if constexpr (kRows) {
+                const int ih = ih0 + (2 * (kb0 + kb) + h) * a.dil_h;
+                const bool row_ok = have && ih >= 0 && ih < a.H;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) v[c] = ld_shared_v4(from + (((uint32_t)c ^ swz) << 4));      // (without a second box: not used)
+                for (int c = 0; c < 8; ++c) {
+                    const int iw = iw0 + c;
+                    v[c] = make_uint4(0, 0, 0, 0);
+                    if (row_ok && c < a.S && iw >= 0 && iw < a.W) v[c] = *reinterpret_cast<const uint4*>(image + (size_t)ih * a.W + iw);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    if (a.C < 4) v[c].w = 0;
+                    if (a.C < 3) v[c].z = 0;
+                    if (a.C < 2) v[c].y = 0;
+                }
+            } else {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err, 0x22u))) break;
+                const uint32_t from = smem + st * L::stage + (uint32_t)h * kBox + row * 128u;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) v[c] = ld_shared_v4(from + (((uint32_t)c ^ swz) << 4));      // (without a second box: not used)
+            }
             bool ok = true;
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
@@ -420,7 +451,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             __syncwarp();
             if (elect_one()) {
                 mbar_arrive(smem_u32(&s_ready[t]));
-                mbar_arrive(smem_u32(&s_empty[st]));
+                if (!kRows) mbar_arrive(smem_u32(&s_empty[st]));
             }
             __syncwarp();
             if (++st == ring) { st = 0; parity ^= 1u; }
@@ -482,7 +513,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         auto copy_weights = [&](uint32_t st, int chunk_w) {
             const int have = min(2, f.chunks - chunk_w);
             const uint32_t bar = smem_u32(&s_full[st]), to = smem + st * L::stage + L::raw_w;
-            if (elect_one()) mbar_arrive_expect_tx(bar, (uint32_t)have * (kBox + L::w_box));
+            if (elect_one()) mbar_arrive_expect_tx(bar, (uint32_t)have * ((kRows ? 0u : kBox) + L::w_box));
             for (int h = 0; h < have; ++h) {
                 if (elect_one()) tma_load_3d(to + (uint32_t)h * L::w_box, &tmap_w, n0, w_c * kChunk, w_tap, bar);
                 __syncwarp();
@@ -505,7 +536,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), parity, &s_abort, err, 0x25u))) break;
                 copy_weights(st, chunk);
             }
-            const int have = min(2, f.chunks - chunk);
+            const int have = kRows ? 0 : min(2, f.chunks - chunk);
             const uint32_t bar = smem_u32(&s_full[st]);
             for (int h = 0; h < have; ++h) {
                 if (elect_one()) {
@@ -524,7 +555,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         }
     } else {
         // ===== multiplications =====
-        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
         const uint64_t b0 = umma_desc_sw128(uniform(smem) + L::parts);
         bool ok = true;
         for (int kb = 0; kb < n_kb && ok; ++kb) {
@@ -571,17 +602,22 @@ int batch_of(const pb_op_params* p) { return p->batch > 1 ? p->batch : 1; }
 int dil(int d) { return d > 1 ? d : 1; }
 bool pointwise(const pb_op_params* p) { return p->R == 1 && p->S == 1 && p->stride_h == 1 && p->stride_w == 1 && p->pad_h == 0 && p->pad_w == 0; }
 
+// A filter row of such a layer is one chunk.
+bool stem(const pb_op_params* p) { return p->Cs == 4 && p->S <= 8 && dil(p->dil_w) == 1 && p->R * p->S > 1 && p->K >= 16; }
+
 struct SplitGeometry {
     int BN, m_tiles, n_tiles, splits, cpt, chunks;
+    bool rows;                  // chunks are rows of the filter
     uint32_t smem;
     const void* fn;
 };
 
 SplitGeometry split_geometry(const pb_op_params* p) {
     SplitGeometry g;
-    g.cpt = ceil_div(p->C, kChunk);
-    g.chunks = p->R * p->S * g.cpt;
-    g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kRows);
+    g.rows = stem(p);
+    g.cpt = g.rows ? 1 : ceil_div(p->C, kChunk);
+    g.chunks = g.rows ? p->R : p->R * p->S * g.cpt;
+    g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kTileRows);
     const int steps = ceil_div(g.chunks, 2);
     // Least modelled time: waves of one block an SM, each a block's fixed time (operand latency, the meeting of the ranks' sums, stores) and
     // its steps.  Measured in chains of equal launches, tile width / ranks -> us: 256 -> 256 channels 3x3 on 2 maps of 14 x 14 64/1 31.4, 64/2 18.2,
@@ -598,7 +634,8 @@ SplitGeometry split_geometry(const pb_op_params* p) {
         }
     g.n_tiles = ceil_div(p->K, g.BN);
     g.smem = (g.BN == 64 ? Layout<64>::bytes : Layout<32>::bytes) + 1024u;
-    g.fn = g.BN == 64 ? (const void*)conv_f32_split_kernel<64> : (const void*)conv_f32_split_kernel<32>;
+    g.fn = g.BN == 64 ? (g.rows ? (const void*)conv_f32_split_kernel<64, true> : (const void*)conv_f32_split_kernel<64, false>)
+                      : (g.rows ? (const void*)conv_f32_split_kernel<32, true> : (const void*)conv_f32_split_kernel<32, false>);
     return g;
 }
 
@@ -616,12 +653,14 @@ uint32_t* conv_f32_error_flag_ptr() {
 //   fp32 units 18.7 / 24.5 / 30.7 / 36.1 us, here 19.1 / 19.1 / 19.2 / 19.1; one image 8.2 / 8.9 / 10.1 / 11.2 and 8.2 / 8.0 / 8.2 / 8.1.
 // - 1x1 layers of up to 32 output channels are short and store little: 256 -> 24 at 14 x 14 5.6 and 7.3, 128 -> 24 at 28 x 28 x 8 6.2 and 6.4 (36
 //   columns: 7.2 and 7.2, 9.1 and 6.7); 3x3 layers gain at any width (64 -> 8 at 56 x 56 8.5 and 8.6, x 8 images 28.5 and 23.1).
+// - Stems: 7 x 7, stride 2, 64 channels on 1 / 2 / 8 images of 224 x 224 22.4 / 32.3 / 110 and 9.7 / 17.9 / 51 us; 3 x 3, stride 2, 32 channels on 2
+//   and 8 10.6 / 31.2 and 10.1 / 28.1, 16 channels on 8 of 320 x 320 51.3 and 51.4, 8 channels 5 x 5 on one of 28 x 28 5.8 and 6.4.
 // PB_F32_SPLIT=0 (read at every use; for tests and comparisons) keeps every layer on the fp32 units.
 bool conv_f32_split_takes(const pb_op_params* p) {
     const char* e = getenv("PB_F32_SPLIT");
     if (e && e[0] == '0') return false;
     const int reach_h = (p->R - 1) * dil(p->dil_h), reach_w = (p->S - 1) * dil(p->dil_w);
-    return p->C >= 24 && (p->K > 32 || p->R * p->S > 1) && (((uintptr_t)p->x | (uintptr_t)p->w) & 15) == 0 && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
+    return (p->C >= 24 || stem(p)) && (p->K > 32 || p->R * p->S > 1) && (((uintptr_t)p->x | (uintptr_t)p->w) & 15) == 0 && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
            p->pad_w <= 100 && reach_h <= 100 && reach_w <= 100 && p->stride_h >= 1 && p->stride_w >= 1 && p->stride_h <= 8 && p->stride_w <= 8 &&
            p->P == (p->H + 2 * p->pad_h - reach_h - 1) / p->stride_h + 1 && p->Q == (p->W + 2 * p->pad_w - reach_w - 1) / p->stride_w + 1;
 }
@@ -651,9 +690,11 @@ int conv_f32_split_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t 
     f.splits = g.splits;
     f.a_tiled = pointwise(p) ? 1 : 0;
     CUtensorMap map, wmap;
-    int rc = encode_pixels_f32(p->x, p->C, p->Cs, p->W, p->H, batch_of(p), p->pad_w, p->pad_h, (p->S - 1) * dil(p->dil_w), (p->R - 1) * dil(p->dil_h),
-                                     p->stride_w, p->stride_h, f.a_tiled != 0, kChunk, kRows, &map);
-    if (rc == PB_OK) rc = encode_weights_f32(p->w, f.Kp, p->Cs, p->R * p->S, g.BN, kChunk, &wmap);
+    memset(&map, 0, sizeof(map));
+    int rc = g.rows ? PB_OK
+                    : encode_pixels_f32(p->x, p->C, p->Cs, p->W, p->H, batch_of(p), p->pad_w, p->pad_h, (p->S - 1) * dil(p->dil_w), (p->R - 1) * dil(p->dil_h),
+                                        p->stride_w, p->stride_h, f.a_tiled != 0, kChunk, kTileRows, &map);
+    if (rc == PB_OK) rc = g.rows ? encode_weights_f32(p->w, f.Kp, p->S * p->Cs, p->R, g.BN, kChunk, &wmap) : encode_weights_f32(p->w, f.Kp, p->Cs, p->R * p->S, g.BN, kChunk, &wmap);
     if (rc != PB_OK) return rc;
     PB_CUDA(cudaFuncSetAttribute(g.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
     cudaLaunchConfig_t cfg = {};

@@ -32,6 +32,13 @@ CASES = [
     (1, 320, 4, 8, 64, 3, 3, 1, 1, 1, 1),          # 45 steps on 32 rows: most ranks finish rows that do not exist
     (4, 96, 56, 56, 64, 3, 3, 1, 1, 1, 1),         # the operands' ring goes round
     (16, 32, 61, 59, 64, 1, 1, 1, 0, 0, 1),        # several waves of one step each
+    # four channels a pixel: a row of the filter is a chunk
+    (2, 3, 41, 39, 64, 7, 7, 2, 3, 3, 1),          # seven chunks, tiles straddle images
+    (1, 4, 16, 8, 33, 3, 8, 1, 1, 4, 1),           # eight taps a row
+    (1, 1, 3, 43, 40, 3, 3, 1, 1, 1, 1),           # one channel, 129 rows
+    (1, 2, 9, 9, 64, 1, 5, 1, 0, 2, 1),            # one chunk
+    (3, 3, 30, 30, 16, 3, 3, 2, 0, 0, 1),          # 16 columns
+    (1, 3, 64, 5, 64, 16, 3, 1, 8, 1, 1),          # sixteen chunks: eight steps, two ranks or more
 ]
 
 
@@ -141,10 +148,11 @@ def test_values_that_are_not_finite(case, monkeypatch):
     assert ((a[ok] - b[ok]).double().norm() <= 1e-5 * b[ok].double().norm())
 
 
-@pytest.mark.parametrize("what", ["x", "w", "size", "narrow", "few"])
+@pytest.mark.parametrize("what", ["x", "w", "size", "narrow", "few", "stem"])
 def test_what_stays_on_the_fp32_units(what):
     import torch
-    case = {"narrow": (1, 64, 9, 9, 32, 1, 1, 1, 0, 0, 1), "few": (1, 23, 9, 9, 64, 3, 3, 1, 1, 1, 1)}.get(what, (1, 64, 9, 9, 64, 3, 3, 1, 1, 1, 1))
+    case = {"narrow": (1, 64, 9, 9, 32, 1, 1, 1, 0, 0, 1), "few": (1, 23, 9, 9, 64, 3, 3, 1, 1, 1, 1),
+            "stem": (1, 3, 20, 20, 15, 3, 3, 2, 1, 1, 1)}.get(what, (1, 64, 9, 9, 64, 3, 3, 1, 1, 1, 1))
     p, t = _prepare(case)
     rows = p.P
     if what in ("x", "w"):

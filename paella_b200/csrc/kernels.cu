@@ -867,7 +867,7 @@ struct WinLane {
 };
 
 template <int kMode, int kStride, int kAct, bool kCountPad, bool kWide>
-__global__ void __launch_bounds__(kTileMaxThreads, 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
+__global__ void __launch_bounds__(kTileMaxThreads, kMode == kWinAvg ? 4 : 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
                                                                         FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
     typedef WinLane<kMode, kStride, kAct, kCountPad, kWide> Lane;
@@ -1884,8 +1884,11 @@ static size_t strip_threads(const pb_op_params* p, int strip) {
 // for 256 images of 35 x 35 x 192 instead of 51), so their tiles are fitted to the map: as few column tiles as hold at most 40 columns
 // each, as many rows as keep the window (the rows a walk runs past the tile included) within 74 KB, so that three blocks fit an SM,
 // and bands of rows where a map has fewer strips than half-warps.
-constexpr int kTileWindowBytes = 74 * 1024;
-static WinTile win_tile(const pb_op_params* p) {
+// An average's lane holds no filter, so four of its blocks fit an SM's registers, and a batch's windows are cut for four (256 maps of 35 x 35 x
+// 192 49.2 -> 47.2 us; the smaller windows alone 53.1, five blocks 47.2).
+constexpr int kTileWindowBytes = 74 * 1024, kTileWindowBytesAvg = 54 * 1024;
+static WinTile win_tile(int kind, const pb_op_params* p) {
+    const int limit = kind == PB_STAGE_AVGPOOL && batch_of(p) > 1 ? kTileWindowBytesAvg : kTileWindowBytes;
     const int st = p->stride_h, strip = st == 1 ? kTileStrip1 : kTileStrip2;
     WinTile g;
     if (batch_of(p) == 1) {
@@ -1899,7 +1902,7 @@ static WinTile win_tile(const pb_op_params* p) {
     }
     g.in_cols = (g.strips * strip - 1) * st + 3;
     if (batch_of(p) > 1) {
-        int fit = (kTileWindowBytes / (g.in_cols * kTileSlab * 2) - 3) / st + 1;      // rows of output whose window fits
+        int fit = (limit / (g.in_cols * kTileSlab * 2) - 3) / st + 1;      // rows of output whose window fits
         if (fit < 1) fit = 1;
         g.rows = p->P < fit ? p->P : fit;
         if (st == 1 && fit < p->P && fit > 3) g.rows = (fit - 1) / 3 * 3 + 1;     // a walk takes three window rows per turn: no turn half used
@@ -1913,7 +1916,7 @@ static WinTile win_tile(const pb_op_params* p) {
         g.in_rows = (g.rows - 1) * st + 3;
         g.alloc_rows = g.alloc_rows > g.in_rows ? g.alloc_rows : g.in_rows;
         g.smem = g.alloc_rows * g.in_cols * kTileSlab * 2;
-        if (g.smem <= kTileWindowBytes || g.rows == 1) break;
+        if (g.smem <= limit || g.rows == 1) break;
         g.rows = ceil_div(p->P, ceil_div(p->P, g.rows) + 1) < g.rows ? ceil_div(p->P, ceil_div(p->P, g.rows) + 1) : g.rows - 1;      // one more row tile
     }
     g.threads = 32 * ceil_div(g.strips * g.bands < 10 ? g.strips * g.bands : 10, 2);
@@ -1926,13 +1929,13 @@ static WinTile win_tile(const pb_op_params* p) {
 // request's pooling layers are a few dozen blocks and keep the strip kernels, which finish sooner on an idle GPU.
 // PB_WINDOW_TILE=0 switches it off; PB_WINDOW_TILE_MIN_BLOCKS sets another threshold (tests use 1).  Read at every call:
 // this runs when a launch is built (graph capture, direct operator calls), never on the replay path.
-static uint32_t tile_blocks(const pb_op_params* p) {
+static uint32_t tile_blocks(int kind, const pb_op_params* p) {
     if (p->dtype != 1 || (p->Cs & 7) || (p->Ks & 3) || (p->out_c_off & 3) || p->act > 2 || strip_of(p) == 0) return 0;
     const char* e = getenv("PB_WINDOW_TILE");
     if (e && e[0] == '0') return 0;
     size_t least = 100;
     if (const char* m = getenv("PB_WINDOW_TILE_MIN_BLOCKS")) least = (size_t)strtoull(m, nullptr, 10);
-    const WinTile g = win_tile(p);
+    const WinTile g = win_tile(kind, p);
     const size_t n = (size_t)((p->Cs + kTileSlab - 1) / kTileSlab) * g.col_tiles * ((p->P + g.rows - 1) / g.rows);
     return n * (size_t)batch_of(p) >= least ? (uint32_t)n : 0;
 }
@@ -1975,7 +1978,7 @@ static const void* tile_fn(int kind, const pb_op_params* p) {
 // 224 x 224 x 64 83.6 / 71.9, 4 of 300 x 500 x 96 63.4 / 55.5, 64 of 57 x 57 x 200 50.6 / 45.7, 2 of 200 x 200 x 640 45.3 / 44.8.
 static WinRing win_ring(int kind, const pb_op_params* p) {
     WinRing g = {};
-    if (kind != PB_STAGE_DWCONV || p->stride_h != 1 || p->stride_w != 1 || tile_blocks(p) == 0) return g;
+    if (kind != PB_STAGE_DWCONV || p->stride_h != 1 || p->stride_w != 1 || tile_blocks(kind, p) == 0) return g;
     g.strips = ceil_div(ceil_div(p->Q, ceil_div(p->Q, 32)), kTileStrip1);
     g.col_tiles = ceil_div(p->Q, g.strips * kTileStrip1);
     g.slabs = ceil_div(p->Cs, kTileSlab);
@@ -2058,11 +2061,11 @@ static int info_one_image(int kind, const pb_op_params* p, pb_launch_info* out) 
                 out->regs_per_thread = regs_of(window3_fn(kind, f32, p->stride_h, strip));
                 out->smem_per_block = strip > 1 ? (uint32_t)window3_smem_bytes(p->Cs, f32 ? 4 : 2) : 0;
             }
-            if (const uint32_t nblk = tile_blocks(p)) {
+            if (const uint32_t nblk = tile_blocks(kind, p)) {
                 out->num_blocks = nblk;
                 out->regs_per_thread = regs_of(tile_fn(kind, p));
-                out->smem_per_block = (uint32_t)win_tile(p).smem;
-                out->threads_per_block = (uint32_t)win_tile(p).threads;
+                out->smem_per_block = (uint32_t)win_tile(kind, p).smem;
+                out->threads_per_block = (uint32_t)win_tile(kind, p).threads;
             }
             out->flops = 2ull * out_elems * p->R * p->S;
             out->bytes = es * (in_elems + (size_t)p->K * p->R * p->S + out_elems) + 4ull * p->K;
@@ -2083,11 +2086,11 @@ static int info_one_image(int kind, const pb_op_params* p, pb_launch_info* out) 
                 out->num_blocks = blocks_for(strip_threads(p, strip));
                 out->regs_per_thread = regs_of(window3_fn(kind, f32, p->stride_h, strip));
             }
-            if (const uint32_t nblk = tile_blocks(p)) {
+            if (const uint32_t nblk = tile_blocks(kind, p)) {
                 out->num_blocks = nblk;
                 out->regs_per_thread = regs_of(tile_fn(kind, p));
-                out->smem_per_block = (uint32_t)win_tile(p).smem;
-                out->threads_per_block = (uint32_t)win_tile(p).threads;
+                out->smem_per_block = (uint32_t)win_tile(kind, p).smem;
+                out->threads_per_block = (uint32_t)win_tile(kind, p).threads;
             }
             out->bytes = es * (in_elems + out_elems) + (p->bias ? 4ull * p->K : 0);
             break;
@@ -2251,8 +2254,8 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
                 launch_k((void (*)(OpArgs, const WinRing, const CUtensorMap, uint32_t, FinishedBlockNotifier*))fn, dim3((unsigned)r.blocks), dim3((unsigned)r.threads), st, pdl, a, r, tmap, job_id, nf);
                 break;
             }
-            if (tile_blocks(p)) {
-                const WinTile g = win_tile(p);
+            if (tile_blocks(kind, p)) {
+                const WinTile g = win_tile(kind, p);
                 const void* fn = tile_fn(kind, p);
                 PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
                 t_launch_smem = (size_t)g.smem;
@@ -2271,8 +2274,8 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
             break;
         case PB_STAGE_MAXPOOL:
             PB_REQUIRE((a.Ks % N) == 0 && (a.out_c_off % N) == 0, "pool: output slice must be vector aligned");
-            if (tile_blocks(p)) {
-                const WinTile g = win_tile(p);
+            if (tile_blocks(kind, p)) {
+                const WinTile g = win_tile(kind, p);
                 const void* fn = tile_fn(kind, p);
                 PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
                 t_launch_smem = (size_t)g.smem;
@@ -2294,8 +2297,8 @@ int simple_op_launch(int kind, const pb_op_params* p, cudaStream_t st, uint32_t 
             break;
         case PB_STAGE_AVGPOOL:
             PB_REQUIRE((a.Ks % N) == 0 && (a.out_c_off % N) == 0, "pool: output slice must be vector aligned");
-            if (tile_blocks(p)) {
-                const WinTile g = win_tile(p);
+            if (tile_blocks(kind, p)) {
+                const WinTile g = win_tile(kind, p);
                 const void* fn = tile_fn(kind, p);
                 PB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g.smem));
                 t_launch_smem = (size_t)g.smem;

@@ -867,7 +867,7 @@ struct WinLane {
 };
 
 template <int kMode, int kStride, int kAct, bool kCountPad, bool kWide>
-__global__ void __launch_bounds__(kTileMaxThreads, kMode == kWinAvg ? 4 : 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
+__global__ void __launch_bounds__(kTileMaxThreads, kMode == kWinDw ? 3 : 4) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
                                                                         FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
     typedef WinLane<kMode, kStride, kAct, kCountPad, kWide> Lane;
@@ -1884,11 +1884,11 @@ static size_t strip_threads(const pb_op_params* p, int strip) {
 // for 256 images of 35 x 35 x 192 instead of 51), so their tiles are fitted to the map: as few column tiles as hold at most 40 columns
 // each, as many rows as keep the window (the rows a walk runs past the tile included) within 74 KB, so that three blocks fit an SM,
 // and bands of rows where a map has fewer strips than half-warps.
-// An average's lane holds no filter, so four of its blocks fit an SM's registers, and a batch's windows are cut for four (256 maps of 35 x 35 x
-// 192 49.2 -> 47.2 us; the smaller windows alone 53.1, five blocks 47.2).
-constexpr int kTileWindowBytes = 74 * 1024, kTileWindowBytesAvg = 54 * 1024;
-static WinTile win_tile(int kind, const pb_op_params* p) {
-    const int limit = kind == PB_STAGE_AVGPOOL && batch_of(p) > 1 ? kTileWindowBytesAvg : kTileWindowBytes;
+// A pooling lane holds no filter, so four of its blocks fit an SM's registers, and a batch's windows are cut for four (average, 256 maps of
+// 35 x 35 x 192 49.2 -> 47.2 us, the smaller windows alone 53.1, five blocks 47.2; 256 of 17 x 17 x 256 25.0 -> 20.7; maximum 20.7 -> 17.5, stride 2 on
+// 64 of 35 x 35 x 288 14.3 -> 12.6).  Depthwise blocks, whose registers allow three, lose with them (256 of 35 x 35 x 192 55.7 -> 59.8).
+constexpr int kTileWindowBytes = 74 * 1024, kTileWindowBytesPool = 54 * 1024;
+static WinTile win_tile_within(const pb_op_params* p, int limit) {
     const int st = p->stride_h, strip = st == 1 ? kTileStrip1 : kTileStrip2;
     WinTile g;
     if (batch_of(p) == 1) {
@@ -1922,6 +1922,12 @@ static WinTile win_tile(int kind, const pb_op_params* p) {
     g.threads = 32 * ceil_div(g.strips * g.bands < 10 ? g.strips * g.bands : 10, 2);
     return g;
 }
+static size_t win_blocks(const pb_op_params* p, const WinTile& g) { return (size_t)ceil_div(p->Cs, kTileSlab) * g.col_tiles * ceil_div(p->P, g.rows); }
+static WinTile win_tile(int kind, const pb_op_params* p) {
+    const WinTile g = win_tile_within(p, kTileWindowBytes);
+    const bool fills = win_blocks(p, g) * batch_of(p) >= 3 * 148;      // else more blocks are only more halo: 8 of 147 x 147 x 64 4.4 -> 4.8
+    return kind != PB_STAGE_DWCONV && batch_of(p) > 1 && fills ? win_tile_within(p, kTileWindowBytesPool) : g;
+}
 
 // Blocks of window3_tile_kernel for one image, or 0 when the layer keeps the strip kernels: bf16, a 3x3 window of stride 1
 // or 2, and at least 100 blocks in the launch (all images).  Measured on Inception-v3 served in gangs of 8: thresholds of
@@ -1936,7 +1942,7 @@ static uint32_t tile_blocks(int kind, const pb_op_params* p) {
     size_t least = 100;
     if (const char* m = getenv("PB_WINDOW_TILE_MIN_BLOCKS")) least = (size_t)strtoull(m, nullptr, 10);
     const WinTile g = win_tile(kind, p);
-    const size_t n = (size_t)((p->Cs + kTileSlab - 1) / kTileSlab) * g.col_tiles * ((p->P + g.rows - 1) / g.rows);
+    const size_t n = win_blocks(p, g);
     return n * (size_t)batch_of(p) >= least ? (uint32_t)n : 0;
 }
 uint32_t* window_error_flag_ptr() {

@@ -24,11 +24,13 @@
 // Bound by the instructions of the splitting warps (about 1250 issue slots a scheduler and step) and, where a launch has few steps, by the
 // latency of a step's chain: 0.76 us at 64 columns, 0.68 at 32.  Measured against the kernel on the fp32 units, us a launch in a chain:
 // 64 -> 64 3x3 on 2 maps of 56 x 56 23.1 -> 8.8, 128 -> 128 on 2 of 28 x 28 21.7 -> 9.5, 512 -> 512 on 2 of 7 x 7 29.2 -> 12.5, 256 -> 256 on 16 of
-// 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 212.  Error against 64 bits, relative, fp32 units / here:
+// 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 214.  Error against 64 bits, relative, fp32 units / here:
 // 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
 //
 // Infinities, NaN and values that round to infinity in bf16 make 0 x inf of the parts: an output that is not finite is computed again,
-// as a plain fp32 sum.
+// as a plain fp32 sum.  So are outputs below 2^-100 whose neighbours (four channels of up to four pixels) are no larger: an operand below 2^-110
+// loses the ends that bf16 cannot hold, 2^-134 at most each, which shows where all is that small (64 -> 64 3x3, inputs of 2^-114 / 2^-118 /
+// 2^-122: relative error 5.6e-7 / 8.7e-6 / 1.4e-4 without the second sum, 1.3e-7 with it, 1.1e-7 on the fp32 units) and nowhere else.
 //
 // This is the fp32 member of the kernel family the reference's TVM adapters launch
 // (jobs/tvm_<model>/tvm_<model>.cpp:24-47; generated fp32 kernels there).
@@ -136,13 +138,23 @@ __device__ __forceinline__ float plain_dot(const SplitArgs& f, int m, int k) {
             if (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) continue;
             const float* x = static_cast<const float*>(a.x) + (((size_t)img * a.H + ih) * a.W + iw) * a.Cs;
             const float* w = static_cast<const float*>(a.w) + (size_t)(r * a.S + s) * a.Cs * f.Kp + k;
-            for (int c = 0; c < a.C; ++c) sum = fmaf(x[c], w[(size_t)c * f.Kp], sum);
+            for (int c0 = 0; c0 < a.C; c0 += 16) {      // shorter chains round less
+                float part = 0.f;
+                for (int c = c0; c < min(c0 + 16, a.C); ++c) part = fmaf(x[c], w[(size_t)c * f.Kp], part);
+                sum += part;
+            }
         }
     return sum;
 }
 
-__device__ __forceinline__ bool finite4(const float4& v) {
-    return (fabsf(v.x) <= FLT_MAX) & (fabsf(v.y) <= FLT_MAX) & (fabsf(v.z) <= FLT_MAX) & (fabsf(v.w) <= FLT_MAX);
+// An output that has to be summed again: not finite, or so small that the lost ends of small operands may show in it.  (Zero is what most
+// zero sums are.)
+__device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) <= FLT_MAX) | ((fabsf(v) < 0x1p-100f) & (v != 0.f)); }
+// max(|a|, |b|), NaN if one of them is.
+__device__ __forceinline__ float max_abs(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(fabsf(a)), "f"(fabsf(b)));
+    return m;
 }
 // Four outputs of row m, from channel k on: bias, residual, activation, whatever the alignment.
 __device__ __forceinline__ void finish4(const OpArgs& a, int m, int k, float4 v, const float4& b, const float4& s, bool vec, bool vec_r) {
@@ -322,13 +334,14 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                 return v;
             };
             const float4 bias = *reinterpret_cast<const float4*>(s_bias + c), slope = *reinterpret_cast<const float4*>(s_slope + c);
-            // Row by row, whatever the alignment and the activation, and with values that are not finite.
+            // Row by row, whatever the alignment and the activation, and with values that are not finite or tiny.
             auto any_row = [&](int row) {
-                float4 x = sum4(row);
+                float4 x = sum4(row), b = bias;
 #pragma unroll 1
                 for (int j = 0; j < 4; ++j) {      // one of the four at a time, in x.x
-                    if (!(fabsf(x.x) <= FLT_MAX) && k + j < a.K) x.x = plain_dot(f, m_share + row, k + j);
+                    if (doubtful(x.x + b.x) && k + j < a.K) x.x = plain_dot(f, m_share + row, k + j);
                     x = make_float4(x.y, x.z, x.w, x.x);
+                    b = make_float4(b.y, b.z, b.w, b.x);
                 }
                 finish4(a, m_share + row, k, x, bias, slope, vec, vec_r);
             };
@@ -344,21 +357,22 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (residual && r + u * kStepR < r1) q[u] = *reinterpret_cast<const float4*>(res + (size_t)(u * kStepR) * a.res_Cs);
-                    bool plain = false;
+                    float top_abs = 0.f;
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (r + u * kStepR < r1) v[u] = sum4(r + u * kStepR);
-                        plain = plain | !finite4(v[u]);
+                        v[u] = make_float4(v[u].x + bias.x, v[u].y + bias.y, v[u].z + bias.z, v[u].w + bias.w);
+                        if (r + u * kStepR < r1) top_abs = max_abs(top_abs, max_abs(max_abs(v[u].x, v[u].y), max_abs(v[u].z, v[u].w)));
                     }
-                    if (plain) {
+                    if (doubtful(top_abs)) {       // one not finite, or all tiny (ResNet-18 x 2 images without the test of tiny ones 211 us, 214 with it, 217 with one per output)
 #pragma unroll 1
                         for (int u = 0; u < 4; ++u)
                             if (r + u * kStepR < r1) any_row(r + u * kStepR);
                     } else {
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
-                            float4 x = make_float4(v[u].x + bias.x, v[u].y + bias.y, v[u].z + bias.z, v[u].w + bias.w);
+                            float4 x = v[u];
                             if (residual) x = make_float4(x.x + q[u].x, x.y + q[u].y, x.z + q[u].z, x.w + q[u].w);
                             if (clamp) x = make_float4(fminf(fmaxf(x.x, 0.f), top), fminf(fmaxf(x.y, 0.f), top), fminf(fmaxf(x.z, 0.f), top), fminf(fmaxf(x.w, 0.f), top));
                             if (r + u * kStepR < r1) *reinterpret_cast<float4*>(y + (size_t)(u * kStepR) * a.Ks) = x;

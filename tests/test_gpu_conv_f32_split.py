@@ -148,6 +148,18 @@ def test_values_that_are_not_finite(case, monkeypatch):
     assert ((a[ok] - b[ok]).double().norm() <= 1e-5 * b[ok].double().norm())
 
 
+@pytest.mark.parametrize("act,k", [(0, 64), (3, 37)])
+@pytest.mark.parametrize("exponent", [-108, -114, -122])
+def test_operands_whose_parts_bf16_cannot_hold(exponent, act, k):
+    """No further off than a chain of fp32 multiply-adds, the steps of the least fp32 values included."""
+    import torch
+    p, t = _prepare((2, 64, 9, 9, k, 3, 3, 1, 1, 1, 1), act=act, x=torch.randn((2, 9, 9, 64), generator=torch.Generator(device="cuda").manual_seed(5), device="cuda") * 2.0 ** exponent)
+    t["b"][:k] = 0.0
+    _launch(p)
+    y, _, chain = _reference(p, t, False)
+    assert ((t["y"][..., :k].double() - y).abs() <= chain + 64 * 9 * 2.0 ** -149).all()
+
+
 @pytest.mark.parametrize("what", ["x", "w", "size", "narrow", "few", "stem"])
 def test_what_stays_on_the_fp32_units(what):
     import torch

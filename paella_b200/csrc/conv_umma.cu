@@ -20,7 +20,7 @@
 // device memory; conv_umma_pre_kernel also normalises its input tiles.  conv_umma_pair_kernel puts two blocks (cta_group::2)
 // on a tile of 256 rows where a lone launch is large.  conv_umma_gather_kernel (PB_CONV_GATHER=1) is the earlier design, kept for
 // comparison: 128 producer threads gather A with 16-byte cp.async copies (a lone Inception-v3 request
-// takes 1656 us with it, 297 without).
+// takes 1656 us with it, 266 without).
 //
 // Every wait is bounded: when a wait runs out the CTA raises a device-global error flag,
 // sets a shared abort flag that releases all other waits of the CTA, skips the epilogue,
@@ -1877,7 +1877,7 @@ int bn_limit() {
 }
 
 // PB_CONV_PERSIST=1: model launches run the persistent kernel (a CTA walks several tiles).  Off by default.
-// Measured on B200 with 3 tiles per CTA: a lone Inception-v3 request 342 -> 1119 us (297 today), the mix MNIST : Inception-v3 = 9 : 1 in a closed
+// Measured on B200 with 3 tiles per CTA: a lone Inception-v3 request 342 -> 1119 us (266 with the one-tile kernel today), the mix MNIST : Inception-v3 = 9 : 1 in a closed
 // loop of 192 clients 317 -> 166 thousand requests a second.  It has not followed the one-tile kernel: no split reductions, no
 // stores through TMA, multiplications and copies issued under `lane == 0` (390 clocks a k-block), and the tiles it walks are cut
 // for one tile per CTA.  (Against the one-tile kernel of its time it had a lone request at 604 us instead of 723.)

@@ -4,8 +4,9 @@
 //   D[m, n] = sum_k A[m, k] * B[k, n]     m = output pixel (all images back to back), n = output channel,
 //                                          k = (tap, input channel), taps of 32-channel chunks
 //
-// A = a0 + a1 + a2 and B = b0 + b1 + b2 exactly (8 bits of mantissa each, rounded to nearest, so 24 and the signs), and of the nine
-// products the six of weight 2^-18 and more are multiplied: what is left out is 2^-26 of a product at most and has no preferred sign.
+// Both are multiplied by 2^16 first, so that bf16 holds the ends of the least fp32 value, too; then A = a0 + a1 + a2 and B = b0 + b1 + b2 exactly (8 bits
+// of mantissa each, rounded to nearest, so 24 and the signs), and of the nine products the six of weight 2^-18 and more are multiplied.
+// The sums are multiplied by 2^-32 at the end.
 // Products of bf16 values are exact in fp32.  The tensor core's own additions do not round to nearest, so its sums are kept
 // short: an accumulator holds 64 values of k, and the products a0 b0 have one of their own, apart from the five small ones (whose
 // roundings are 2^-8 of theirs).  After every 64 k both are read from tensor memory and added to the sums in registers, which are
@@ -27,10 +28,9 @@
 // 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 214.  Error against 64 bits, relative, fp32 units / here:
 // 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
 //
-// Infinities, NaN and values that round to infinity in bf16 make 0 x inf of the parts: an output that is not finite is computed again,
-// as a plain fp32 sum.  So are outputs below 2^-100 whose neighbours (four channels of up to four pixels) are no larger: an operand below 2^-110
-// loses the ends that bf16 cannot hold, 2^-134 at most each, which shows where all is that small (64 -> 64 3x3, inputs of 2^-114 / 2^-118 /
-// 2^-122: relative error 5.6e-7 / 8.7e-6 / 1.4e-4 without the second sum, 1.3e-7 with it, 1.1e-7 on the fp32 units) and nowhere else.
+// Infinities, NaN and operands of 2^112 and more make 0 x inf of the parts, and sums of 2^96 and more overflow: an output that is not finite is computed again,
+// as a plain fp32 sum.  (64 -> 64 3x3, relative error against 64 bits here / on the fp32 units: inputs of 2^-122 and weights of 2^30 8.5e-8 / 1.1e-7, 2^-140 and
+// 2^100 7.0e-8 / 1.1e-7, results of 2^-134 3.3e-6 / 3.7e-5.  Without the scaling 1.4e-4, 1.0 and 5.8e-5.)
 //
 // This is the fp32 member of the kernel family the reference's TVM adapters launch
 // (jobs/tvm_<model>/tvm_<model>.cpp:24-47; generated fp32 kernels there).
@@ -63,6 +63,7 @@ constexpr uint32_t kBox = kTileRows * kChunk * 4;       // 16 KB
 constexpr int kWarpA = 8, kWarpB = 16, kWarpCopy = 24, kWarpMma = 25;
 constexpr int kThreadsF = 26 * 32;
 constexpr uint32_t kTmemCols = 512;
+constexpr uint64_t kUp = 0x4780000047800000ull, kDown = 0x2f8000002f800000ull;      // pairs of 2^16 and 2^-32
 
 struct SplitArgs {
     OpArgs op;
@@ -101,9 +102,9 @@ __device__ __forceinline__ void tcgen05_st8(uint32_t taddr, const uint32_t (&r)[
                  ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ uint64_t sub_f32x2(uint64_t x, uint64_t y) {
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t x, uint64_t y) {
     uint64_t r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return r;
 }
 // 16 bytes into another block's shared memory, counted by its barrier.
@@ -114,16 +115,22 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, const float4& v, uint
 }
 __device__ __forceinline__ void tcgen05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Two values to three pairs of bf16 that add up to them (the first in the low halves).
+// lo and hi less the bf16 values of the pair, exactly.  (The mixed multiply-add reads a half of a register: two instructions where widening the
+// halves and subtracting takes three.)
+__device__ __forceinline__ void less_bf16(uint32_t pair, float& lo, float& hi) {
+    asm("{\n\t.reg .b16 l, h, m;\n\tmov.b32 {l, h}, %2;\n\tmov.b16 m, 0xbf80;\n\t"
+        "fma.rn.f32.bf16 %0, l, m, %0;\n\tfma.rn.f32.bf16 %1, h, m, %1;\n\t}"
+        : "+f"(lo), "+f"(hi)
+        : "r"(pair));
+}
+// Two values, times 2^16, to three pairs of bf16 that add up to them (the first in the low halves).
 __device__ __forceinline__ void split2(uint32_t x0, uint32_t x1, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    uint64_t v = pack_f32x2(x0, x1);
-    float lo = __uint_as_float(x0), hi = __uint_as_float(x1);
+    float lo, hi;
+    unpack_f32x2(mul_f32x2(pack_f32x2(x0, x1), kUp), lo, hi);
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p0) : "f"(hi), "f"(lo));
-    v = sub_f32x2(v, pack_f32x2(p0 << 16, p0 & 0xffff0000u));
-    unpack_f32x2(v, lo, hi);
+    less_bf16(p0, lo, hi);
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(hi), "f"(lo));
-    v = sub_f32x2(v, pack_f32x2(p1 << 16, p1 & 0xffff0000u));
-    unpack_f32x2(v, lo, hi);
+    less_bf16(p1, lo, hi);
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(hi), "f"(lo));
 }
 
@@ -147,9 +154,8 @@ __device__ __forceinline__ float plain_dot(const SplitArgs& f, int m, int k) {
     return sum;
 }
 
-// An output that has to be summed again: not finite, or so small that the lost ends of small operands may show in it.  (Zero is what most
-// zero sums are.)
-__device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) <= FLT_MAX) | ((fabsf(v) < 0x1p-100f) & (v != 0.f)); }
+// An output that has to be summed again: not finite.
+__device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) <= FLT_MAX); }
 // max(|a|, |b|), NaN if one of them is.
 __device__ __forceinline__ float max_abs(float a, float b) {
     float m;
@@ -301,8 +307,8 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 #pragma unroll
             for (int c = 0; c < kCols; c += 4) {
                 float4 v;
-                unpack_f32x2(acc[c / 2], v.x, v.y);
-                unpack_f32x2(acc[c / 2 + 1], v.z, v.w);
+                unpack_f32x2(mul_f32x2(acc[c / 2], kDown), v.x, v.y);
+                unpack_f32x2(mul_f32x2(acc[c / 2 + 1], kDown), v.z, v.w);
                 const uint32_t off = (((uint32_t)(col0 + c) >> 2) ^ mix) << 4;
                 if (owner == rank) st_shared_v4(at + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
                 else st_async_v4(to + off, v, bar);
@@ -334,7 +340,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                 return v;
             };
             const float4 bias = *reinterpret_cast<const float4*>(s_bias + c), slope = *reinterpret_cast<const float4*>(s_slope + c);
-            // Row by row, whatever the alignment and the activation, and with values that are not finite or tiny.
+            // Row by row, whatever the alignment and the activation, and with values that are not finite.
             auto any_row = [&](int row) {
                 float4 x = sum4(row), b = bias;
 #pragma unroll 1
@@ -365,7 +371,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                         v[u] = make_float4(v[u].x + bias.x, v[u].y + bias.y, v[u].z + bias.z, v[u].w + bias.w);
                         if (r + u * kStepR < r1) top_abs = max_abs(top_abs, max_abs(max_abs(v[u].x, v[u].y), max_abs(v[u].z, v[u].w)));
                     }
-                    if (doubtful(top_abs)) {       // one not finite, or all tiny (ResNet-18 x 2 images without the test of tiny ones 211 us, 214 with it, 217 with one per output)
+                    if (doubtful(top_abs)) {       // one not finite
 #pragma unroll 1
                         for (int u = 0; u < 4; ++u)
                             if (r + u * kStepR < r1) any_row(r + u * kStepR);

@@ -160,6 +160,30 @@ def test_operands_whose_parts_bf16_cannot_hold(exponent, act, k):
     assert ((t["y"][..., :k].double() - y).abs() <= chain + 64 * 9 * 2.0 ** -149).all()
 
 
+@pytest.mark.parametrize("act,k", [(0, 64), (3, 37)])
+@pytest.mark.parametrize("where", ["all", "channel", "image"])
+@pytest.mark.parametrize("small,large", [(-118, 30), (-126, 60), (-140, 100)])
+def test_small_operands_that_meet_large_factors(small, large, where, act, k):
+    """Operands whose ends bf16 cannot hold, in results of any size: all of them, one output channel, one image of a batch.  The sums
+    are rounded to fp32 once a rank, to a multiple of 2^-149."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn((3, 9, 9, 64), generator=gen, device="cuda")
+    p, t = _prepare((3, 64, 9, 9, k, 3, 3, 1, 1, 1, 1), act=act, x=x)
+    if where == "channel":
+        x, t["w"][k // 2] = x * 2.0 ** large, t["w"][k // 2] * 2.0 ** small
+    else:
+        x[slice(None) if where == "all" else slice(1, 2)] *= 2.0 ** small
+        t["w"] *= 2.0 ** large
+    t["x"][..., :64] = x
+    t["wd"] = gu.pack_weights(capi.STAGE_CONV_SIMT, p, t["w"].cpu().numpy())
+    p.w = t["wd"].data_ptr()
+    t["b"][:k] = 0.0
+    _launch(p)
+    y, bound, _ = _reference(p, t, False)
+    assert ((t["y"][..., :k].double() - y).abs() <= bound + 8 * 2.0 ** -149).all()
+
+
 @pytest.mark.parametrize("what", ["x", "w", "size", "narrow", "few", "stem"])
 def test_what_stays_on_the_fp32_units(what):
     import torch

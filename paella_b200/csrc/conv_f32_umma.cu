@@ -28,9 +28,11 @@
 // 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 214.  Error against 64 bits, relative, fp32 units / here:
 // 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
 //
-// Infinities, NaN and operands of 2^112 and more make 0 x inf of the parts, and sums of 2^96 and more overflow: an output that is not finite is computed again,
-// as a plain fp32 sum.  (64 -> 64 3x3, relative error against 64 bits here / on the fp32 units: inputs of 2^-122 and weights of 2^30 8.5e-8 / 1.1e-7, 2^-140 and
-// 2^100 7.0e-8 / 1.1e-7, results of 2^-134 3.3e-6 / 3.7e-5.  Without the scaling 1.4e-4, 1.0 and 5.8e-5.)
+// Infinities, NaN and operands of 2^112 and more make 0 x inf of the parts, and sums of 2^96 and more overflow: a block that finds one of its sums not finite
+// makes them all again in a second pass, as plain fp32 multiply-adds of the same copies (28 TFLOP/s; one thread a poisoned output, as it was, took
+// 10.9 ms for 256 -> 256 on 16 of 28 x 28 where every pixel is NaN, 0.49 ms for 64 -> 64 on 2 of 56 x 56; this 0.56 ms and 34 us, the fp32 units 0.41 and 23).
+// What is small is exact (64 -> 64 3x3, relative error against 64 bits here / on the fp32 units: inputs of 2^-122 and weights of 2^30 8.5e-8 / 1.1e-7, 2^-140 and
+// 2^100 7.0e-8 / 1.1e-7, results of 2^-134 3.3e-6 / 3.7e-5; without the scaling 1.4e-4, 1.0 and 5.8e-5).
 //
 // This is the fp32 member of the kernel family the reference's TVM adapters launch
 // (jobs/tvm_<model>/tvm_<model>.cpp:24-47; generated fp32 kernels there).
@@ -38,7 +40,6 @@
 #include <llis/job/finished_block_notifier.h>
 
 #include <algorithm>
-#include <cfloat>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
@@ -61,7 +62,7 @@ constexpr int kTileRows = 128, kChunk = 32;             // pixels of a tile, cha
 constexpr int kMaxRing = 4;
 constexpr uint32_t kBox = kTileRows * kChunk * 4;       // 16 KB
 constexpr int kWarpA = 8, kWarpB = 16, kWarpCopy = 24, kWarpMma = 25;
-constexpr int kThreadsF = 26 * 32;
+constexpr int kThreadsF = 26 * 32;                      // 832
 constexpr uint32_t kTmemCols = 512;
 constexpr uint64_t kUp = 0x4780000047800000ull, kDown = 0x2f8000002f800000ull;      // pairs of 2^16 and 2^-32
 
@@ -107,6 +108,11 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t x, uint64_t y) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return r;
 }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
 // 16 bytes into another block's shared memory, counted by its barrier.
 __device__ __forceinline__ void st_async_v4(uint32_t addr, const float4& v, uint32_t bar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
@@ -134,34 +140,187 @@ __device__ __forceinline__ void split2(uint32_t x0, uint32_t x1, uint32_t& p0, u
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(hi), "f"(lo));
 }
 
-// One output as a plain fp32 sum.
-__device__ __forceinline__ float plain_dot(const SplitArgs& f, int m, int k) {
+// Where a summing thread's row of sums goes.  Rank z finishes rows [z, z + 1) x 128 / splits of the tile: every rank sends it its sums (st.async: the sums
+// go from registers into the owner's shared memory and count on its barrier), laid out as [rank][row][channel], 16-byte chunks in an order that
+// keeps both the writers (a row each) and the readers (a chunk each) free of bank conflicts.
+template <int BN>
+struct Meeting {
+    uint32_t at, to, bar, mix;
+    bool mine;
+    __device__ __forceinline__ Meeting(const SplitArgs& f, uint32_t smem, int row, int rank, uint64_t* s_sums) {
+        const int ranks_log2 = 31 - __clz(f.splits), share = kTileRows >> ranks_log2, owner = row >> (7 - ranks_log2), rl = row & (share - 1);
+        at = to = smem + Layout<BN>::meet + (uint32_t)((rank * share + rl) * (BN * 4));
+        mix = (uint32_t)rl & 7u;
+        bar = 0;
+        mine = owner == rank;
+        if (f.splits > 1) {
+            to = cluster_addr(at, (uint32_t)owner);
+            bar = cluster_addr(smem_u32(s_sums), (uint32_t)owner);
+        }
+    }
+    __device__ __forceinline__ void put(int col, const float4& v) const {      // columns col .. col + 3
+        const uint32_t off = (((uint32_t)col >> 2) ^ mix) << 4;
+        if (mine) st_shared_v4(at + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+        else st_async_v4(to + off, v, bar);
+    }
+};
+
+// Is `p` true anywhere in the summing warps?
+__device__ __forceinline__ bool sums_any(bool p) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(p ? 1u : 0u) : "memory");
+    return r != 0;
+}
+// The summing warps have decided whether there is a second pass (they go on at once); the others wait for that.
+__device__ __forceinline__ void block_arrive() { asm volatile("barrier.cta.arrive 2, 832;" ::: "memory"); }
+__device__ __forceinline__ void block_await() { asm volatile("barrier.cta.sync 2, 832;" ::: "memory"); }
+// Everybody: the second pass is complete.
+__device__ __forceinline__ void block_meet() { asm volatile("barrier.cta.sync 3, 832;" ::: "memory"); }
+
+// ---- a block's share of the reduction once more, as plain fp32 multiply-adds ----------------------------------------
+// The raw operands come again, through the ring's first two stages; its third takes the sums.  (Called with what is constant only: arguments that live
+// through the loops of the first pass for this cost it 5 %.)
+template <int BN>
+struct Share {          // the tile and the steps of this block
+    int m0, n0, kb0, n_kb;
+    uint32_t smem;
+    __device__ __forceinline__ Share(const SplitArgs& f, const uint8_t* smem_raw)
+        : m0((int)blockIdx.x * kTileRows), n0((int)blockIdx.y * BN), smem((smem_u32(smem_raw) + 1023u) & ~1023u) {
+        const int steps = (f.chunks + 1) / 2, ranks_log2 = 31 - __clz(f.splits), rank = (int)blockIdx.z;
+        kb0 = (steps * rank) >> ranks_log2;
+        n_kb = ((steps * (rank + 1)) >> ranks_log2) - kb0;
+    }
+};
+// How often stage st was used by the first pass:
+template <int BN>
+__device__ __forceinline__ uint32_t ring_uses(uint32_t st, int n_kb) { return ((uint32_t)n_kb + Layout<BN>::ring - 1u - st) / Layout<BN>::ring; }
+
+template <int BN, bool kRows>
+__device__ __noinline__ void copy_again(const CUtensorMap* tmap_x, const CUtensorMap* tmap_w, const SplitArgs& f, uint8_t* smem_raw, uint64_t* s_full, uint64_t* s_empty,
+                                        volatile uint32_t* s_abort) {
+    using L = Layout<BN>;
     const OpArgs& a = f.op;
-    const int img = m / f.PQ, pix = m - img * f.PQ, p = pix / a.Q, q = pix - p * a.Q;
-    float sum = 0.f;
-    for (int r = 0; r < a.R; ++r)
-        for (int s = 0; s < a.S; ++s) {
-            const int ih = p * a.stride_h - a.pad_h + r * a.dil_h, iw = q * a.stride_w - a.pad_w + s * a.dil_w;
-            if (ih < 0 || ih >= a.H || iw < 0 || iw >= a.W) continue;
-            const float* x = static_cast<const float*>(a.x) + (((size_t)img * a.H + ih) * a.W + iw) * a.Cs;
-            const float* w = static_cast<const float*>(a.w) + (size_t)(r * a.S + s) * a.Cs * f.Kp + k;
-            for (int c0 = 0; c0 < a.C; c0 += 16) {      // shorter chains round less
-                float part = 0.f;
-                for (int c = c0; c < min(c0 + 16, a.C); ++c) part = fmaf(x[c], w[(size_t)c * f.Kp], part);
-                sum += part;
+    const Share<BN> b(f, smem_raw);
+    const int m0 = b.m0, n0 = b.n0, kb0 = b.kb0, n_kb = b.n_kb;
+    const uint32_t smem = b.smem;
+    const int img = m0 / f.PQ, pix = m0 - img * f.PQ, p = pix / a.Q, w_org = (pix - p * a.Q) * a.stride_w - a.pad_w, h_org = p * a.stride_h - a.pad_h;
+    for (int kb = 0; kb < n_kb; ++kb) {
+        const uint32_t st = (uint32_t)kb & 1u, bar = smem_u32(&s_full[st]), to = smem + st * L::stage;
+        if (kb >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_empty[st]), (ring_uses<BN>(st, n_kb) + (uint32_t)(kb >> 1) - 1u) & 1u, s_abort, &g_f32_err_flag, 0x2au))) break;
+        const int chunk = 2 * (kb0 + kb), have = min(2, f.chunks - chunk);
+        if (elect_one()) {
+            mbar_arrive_expect_tx(bar, (uint32_t)have * ((kRows ? 0u : kBox) + L::w_box));
+            for (int h = 0; h < have; ++h) {
+                const int tap = (chunk + h) / f.cpt, c = (chunk + h - tap * f.cpt) * kChunk, r = tap / a.S;
+                tma_load_3d(to + L::raw_w + (uint32_t)h * L::w_box, tmap_w, n0, c, tap, bar);
+                if (kRows) continue;
+                if (f.a_tiled) tma_load_2d(to + (uint32_t)h * kBox, tmap_x, c, m0, bar);
+                else tma_load_im2col_4d(to + (uint32_t)h * kBox, tmap_x, c, w_org, h_org, img, (uint16_t)((tap - r * a.S) * a.dil_w), (uint16_t)(r * a.dil_h), bar);
             }
         }
-    return sum;
+        __syncwarp();
+    }
 }
 
-// An output that has to be summed again: not finite.
-__device__ __forceinline__ bool doubtful(float v) { return !(fabsf(v) <= FLT_MAX); }
-// max(|a|, |b|), NaN if one of them is.
-__device__ __forceinline__ float max_abs(float a, float b) {
-    float m;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(fabsf(a)), "f"(fabsf(b)));
-    return m;
+// Warps 8-23: two groups of 256 threads, a box of a step each; a thread has rows t / 8 + 32 i and columns 4 (t % 8) + 32 j, + 0 .. 3.  The sums of a box go
+// to shared memory, [group][i][j][t][4]: no chain is longer than 32.
+template <int BN, bool kRows>
+__device__ __noinline__ void sum_again(const SplitArgs& f, uint8_t* smem_raw, uint64_t* s_full, uint64_t* s_empty, volatile uint32_t* s_abort) {
+    using L = Layout<BN>;
+    constexpr int kWide = BN / 32;                 // column quads of a thread
+    const OpArgs& a = f.op;
+    const Share<BN> b(f, smem_raw);
+    const int m0 = b.m0, kb0 = b.kb0, n_kb = b.n_kb;
+    const uint32_t smem = b.smem;
+    const int t = (int)threadIdx.x & 255, h = ((int)threadIdx.x >> 8) - 1;
+    const uint32_t row = (uint32_t)t >> 3, swz = row & 7u, box = smem + (uint32_t)h * kBox, w_at = smem + L::raw_w + (uint32_t)h * L::w_box + ((uint32_t)t & 7u) * 16u;
+    const uint32_t sums = smem + 2 * L::stage + ((uint32_t)(h * 4 * kWide) * 256u + (uint32_t)t) * 16u;
+    // kRows: this thread brings four pixels of a row's window
+    const int m = m0 + (t & 127), img = m / f.PQ, pix = m - img * f.PQ, p = pix / a.Q, ih0 = p * a.stride_h - a.pad_h, px0 = (t >> 7) * 4;
+    const int iw0 = (pix - p * a.Q) * a.stride_w - a.pad_w + px0;
+#pragma unroll 1
+    for (int kb = 0; kb < n_kb; ++kb) {
+        const uint32_t st = (uint32_t)kb & 1u;
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), (ring_uses<BN>(st, n_kb) + (uint32_t)(kb >> 1)) & 1u, s_abort, &g_f32_err_flag, 0x2bu)) && !kRows) break;      // (kRows: the group meets below)
+        const bool have = 2 * (kb0 + kb) + h < f.chunks;
+        if constexpr (kRows) {
+            const int ih = ih0 + (2 * (kb0 + kb) + h) * a.dil_h;
+            const uint4* const from = static_cast<const uint4*>(a.x) + ((ptrdiff_t)img * a.H + ih) * a.W + iw0;
+            for (int c = 0; c < 4; ++c) {
+                uint4 v = make_uint4(0, 0, 0, 0);
+                if (have && m < f.M && px0 + c < a.S && ih >= 0 && ih < a.H && iw0 + c >= 0 && iw0 + c < a.W) v = from[c];
+                st_shared_v4(box + st * L::stage + (uint32_t)(t & 127) * 128u + ((uint32_t)((px0 + c) ^ (t & 7)) << 4), v.x, a.C > 1 ? v.y : 0u, a.C > 2 ? v.z : 0u, a.C > 3 ? v.w : 0u);
+            }
+            asm volatile("bar.sync %0, 256;" ::"r"(4 + h) : "memory");
+        }
+        float acc[4][4 * kWide];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4 * kWide; ++j) acc[i][j] = 0.f;
+        if (have) {
+#pragma unroll 1
+            for (uint32_t c = 0; c < 8; ++c) {
+                float x[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 v = ld_shared_v4(box + st * L::stage + (row + 32u * (uint32_t)i) * 128u + ((c ^ swz) << 4));
+                    x[i][0] = __uint_as_float(v.x); x[i][1] = __uint_as_float(v.y); x[i][2] = __uint_as_float(v.z); x[i][3] = __uint_as_float(v.w);
+                }
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {
+#pragma unroll
+                    for (int j = 0; j < kWide; ++j) {
+                        const uint4 w = ld_shared_v4(w_at + st * L::stage + (c * 4u + q) * (uint32_t)(BN * 4) + (uint32_t)j * 128u);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            acc[i][4 * j] = fmaf(x[i][q], __uint_as_float(w.x), acc[i][4 * j]);
+                            acc[i][4 * j + 1] = fmaf(x[i][q], __uint_as_float(w.y), acc[i][4 * j + 1]);
+                            acc[i][4 * j + 2] = fmaf(x[i][q], __uint_as_float(w.z), acc[i][4 * j + 2]);
+                            acc[i][4 * j + 3] = fmaf(x[i][q], __uint_as_float(w.w), acc[i][4 * j + 3]);
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (elect_one()) mbar_arrive(smem_u32(&s_empty[st]));
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < kWide; ++j) {
+                const uint32_t to = sums + (uint32_t)(i * kWide + j) * 4096u;
+                float4 v = make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
+                if (kb > 0) {
+                    const uint4 o = ld_shared_v4(to);
+                    v = make_float4(__uint_as_float(o.x) + v.x, __uint_as_float(o.y) + v.y, __uint_as_float(o.z) + v.z, __uint_as_float(o.w) + v.w);
+                }
+                st_shared_v4(to, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+            }
+    }
 }
+
+// Summing warps: the second pass's sums to where they meet.  (A call of its own: with the sums read back into the registers of the first pass every
+// launch pays 5 % for the copies.)
+template <int BN>
+__device__ __noinline__ void send_again(const SplitArgs& f, uint8_t* smem_raw, uint64_t* s_sums) {
+    using L = Layout<BN>;
+    constexpr int kCols = BN / 2;
+    constexpr uint32_t kGroup = (uint32_t)kTileRows * BN * 4;
+    block_meet();
+    const int row = (int)threadIdx.x & 127, col0 = ((int)threadIdx.x >> 7) * kCols;
+    const Share<BN> b(f, smem_raw);
+    const Meeting<BN> to(f, b.smem, row, (int)blockIdx.z, s_sums);
+    const uint32_t from = b.smem + 2 * L::stage + (uint32_t)(row >> 5) * (uint32_t)(BN / 32) * 4096u + (uint32_t)(row & 31) * 128u;
+    for (int c = col0; c < col0 + kCols; c += 4) {
+        const uint32_t at = from + (uint32_t)(c >> 5) * 4096u + (uint32_t)(c & 31) * 4u;
+        const uint4 v = ld_shared_v4(at), w = ld_shared_v4(at + kGroup);
+        to.put(c, make_float4(__uint_as_float(v.x) + __uint_as_float(w.x), __uint_as_float(v.y) + __uint_as_float(w.y), __uint_as_float(v.z) + __uint_as_float(w.z),
+                              __uint_as_float(v.w) + __uint_as_float(w.w)));
+    }
+}
+
 // Four outputs of row m, from channel k on: bias, residual, activation, whatever the alignment.
 __device__ __forceinline__ void finish4(const OpArgs& a, int m, int k, float4 v, const float4& b, const float4& s, bool vec, bool vec_r) {
     v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
@@ -203,9 +362,9 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[kMaxRing], s_empty[kMaxRing];      // raw operands
     __shared__ __align__(8) uint64_t s_ready[2], s_done[2], s_free[2];   // operands split; multiplied; accumulators read
-    __shared__ __align__(8) uint64_t s_sums;                             // the other ranks' sums have arrived
+    __shared__ __align__(8) uint64_t s_sums[1];                          // the other ranks' sums have arrived
     __shared__ uint32_t s_tmem_base;
-    __shared__ volatile uint32_t s_abort;
+    __shared__ volatile uint32_t s_abort, s_again;
     __shared__ __align__(16) float s_bias[BN], s_slope[BN];
     using L = Layout<BN>;
 
@@ -225,15 +384,16 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     if (warp == kWarpCopy) {            // a lane per barrier
         if (lane < (int)ring) {
             mbar_init(smem_u32(&s_full[lane]), 1);
-            mbar_init(smem_u32(&s_empty[lane]), kRows ? 8 : 16);
+            mbar_init(smem_u32(&s_empty[lane]), 16);
         } else if (lane >= 8 && lane < 10) {
             mbar_init(smem_u32(&s_ready[lane - 8]), 16);
             mbar_init(smem_u32(&s_done[lane - 8]), 1);
             mbar_init(smem_u32(&s_free[lane - 8]), 8);
         } else if (lane == 16) {
-            mbar_init(smem_u32(&s_sums), 1);
-            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(&s_sums), (uint32_t)((f.splits - 1) * (kTileRows >> ranks_log2) * BN * 4));
+            mbar_init(smem_u32(s_sums), 1);
+            if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(s_sums), (uint32_t)((f.splits - 1) * (kTileRows >> ranks_log2) * BN * 4));
             s_abort = 0;
+            s_again = 0;
         } else if (lane == 24) {
             if (!kRows) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
@@ -291,36 +451,42 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             if (elect_one()) mbar_arrive(smem_u32(&s_free[t]));
             __syncwarp();
         }
-        // Rank z finishes rows [z, z + 1) x 128 / splits of the tile: every rank sends it its sums (st.async: the sums go from registers into the
-        // owner's shared memory and count on its barrier), laid out as [rank][row][channel], 16-byte chunks in an order that keeps both the
-        // writers (a row each) and the readers (a chunk each) free of bank conflicts.
+        // Sums that are not finite - operands of 2^112 and more, infinities and NaN among them, or products that overflow - are made again in plain fp32, those
+        // of the block's whole share of the reduction.
+        uint64_t finite[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < kCols / 2; ++j) {
+            acc[j] = mul_f32x2(acc[j], kDown);
+            finite[j & 3] = fma_f32x2(acc[j], 0ull, finite[j & 3]);
+        }
+        float f0, f1;
+        unpack_f32x2(add_f32x2(add_f32x2(finite[0], finite[1]), add_f32x2(finite[2], finite[3])), f0, f1);
+        const bool again = sums_any(!(f0 == f1) && !s_abort);      // (zeros or NaN)
+        if (again && tid == 0) s_again = 1;
+        __syncwarp();
+        block_arrive();
         const uint32_t meet = smem + L::meet;
         const int share = kTileRows >> ranks_log2;
-        {
-            const int owner = row >> (7 - ranks_log2), rl = row & (share - 1);
-            const uint32_t at = meet + (uint32_t)((rank * share + rl) * (BN * 4)), mix = (uint32_t)rl & 7u;
-            uint32_t to = at, bar = 0;
-            if (f.splits > 1) {
-                to = cluster_addr(at, (uint32_t)owner);
-                bar = cluster_addr(smem_u32(&s_sums), (uint32_t)owner);
-            }
+        if (__builtin_expect(again, 0)) {
+            send_again<BN>(f, smem_raw, s_sums);
+        } else {
+            const Meeting<BN> to(f, smem, row, rank, s_sums);
 #pragma unroll
             for (int c = 0; c < kCols; c += 4) {
                 float4 v;
-                unpack_f32x2(mul_f32x2(acc[c / 2], kDown), v.x, v.y);
-                unpack_f32x2(mul_f32x2(acc[c / 2 + 1], kDown), v.z, v.w);
-                const uint32_t off = (((uint32_t)(col0 + c) >> 2) ^ mix) << 4;
-                if (owner == rank) st_shared_v4(at + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
-                else st_async_v4(to + off, v, bar);
+                unpack_f32x2(acc[c / 2], v.x, v.y);
+                unpack_f32x2(acc[c / 2 + 1], v.z, v.w);
+                to.put(col0 + c, v);
             }
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");
         if (f.splits > 1) {       // (also when this block gives up: it stays until the others have written to it)
             bool here = false;
-            for (uint32_t i = 0; i < kWaitLimit && !here; ++i) here = mbar_try_wait(smem_u32(&s_sums), 0u);
+            for (uint32_t i = 0; i < kWaitLimit && !here; ++i) here = mbar_try_wait(smem_u32(s_sums), 0u);
             if (!here) atomicExch(err, 0x28u);
             ok = __all_sync(0xffffffffu, here) && ok;
         }
+        ok = ok && !s_abort;           // (the second pass may have given up)
         if (ok) {
             const bool vec = ((a.Ks | a.out_c_off) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
             const bool vec_r = (a.res_Cs & 3) == 0 && (reinterpret_cast<uintptr_t>(a.residual) & 15) == 0;
@@ -340,17 +506,7 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                 return v;
             };
             const float4 bias = *reinterpret_cast<const float4*>(s_bias + c), slope = *reinterpret_cast<const float4*>(s_slope + c);
-            // Row by row, whatever the alignment and the activation, and with values that are not finite.
-            auto any_row = [&](int row) {
-                float4 x = sum4(row), b = bias;
-#pragma unroll 1
-                for (int j = 0; j < 4; ++j) {      // one of the four at a time, in x.x
-                    if (doubtful(x.x + b.x) && k + j < a.K) x.x = plain_dot(f, m_share + row, k + j);
-                    x = make_float4(x.y, x.z, x.w, x.x);
-                    b = make_float4(b.y, b.z, b.w, b.x);
-                }
-                finish4(a, m_share + row, k, x, bias, slope, vec, vec_r);
-            };
+            auto any_row = [&](int row) { finish4(a, m_share + row, k, sum4(row), bias, slope, vec, vec_r); };      // whatever the alignment and the activation
             // Branches cost a lone warp more than the arithmetic: rows four at a time, their loads together, nothing left to decide.
             auto rows4 = [&](auto with_residual, auto with_clamp) {
                 constexpr bool residual = decltype(with_residual)::value, clamp = decltype(with_clamp)::value;
@@ -363,26 +519,18 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (residual && r + u * kStepR < r1) q[u] = *reinterpret_cast<const float4*>(res + (size_t)(u * kStepR) * a.res_Cs);
-                    float top_abs = 0.f;
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (r + u * kStepR < r1) v[u] = sum4(r + u * kStepR);
                         v[u] = make_float4(v[u].x + bias.x, v[u].y + bias.y, v[u].z + bias.z, v[u].w + bias.w);
-                        if (r + u * kStepR < r1) top_abs = max_abs(top_abs, max_abs(max_abs(v[u].x, v[u].y), max_abs(v[u].z, v[u].w)));
                     }
-                    if (doubtful(top_abs)) {       // one not finite
-#pragma unroll 1
-                        for (int u = 0; u < 4; ++u)
-                            if (r + u * kStepR < r1) any_row(r + u * kStepR);
-                    } else {
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            float4 x = v[u];
-                            if (residual) x = make_float4(x.x + q[u].x, x.y + q[u].y, x.z + q[u].z, x.w + q[u].w);
-                            if (clamp) x = make_float4(fminf(fmaxf(x.x, 0.f), top), fminf(fmaxf(x.y, 0.f), top), fminf(fmaxf(x.z, 0.f), top), fminf(fmaxf(x.w, 0.f), top));
-                            if (r + u * kStepR < r1) *reinterpret_cast<float4*>(y + (size_t)(u * kStepR) * a.Ks) = x;
-                        }
+                    for (int u = 0; u < 4; ++u) {
+                        float4 x = v[u];
+                        if (residual) x = make_float4(x.x + q[u].x, x.y + q[u].y, x.z + q[u].z, x.w + q[u].w);
+                        if (clamp) x = make_float4(fminf(fmaxf(x.x, 0.f), top), fminf(fmaxf(x.y, 0.f), top), fminf(fmaxf(x.z, 0.f), top), fminf(fmaxf(x.w, 0.f), top));
+                        if (r + u * kStepR < r1) *reinterpret_cast<float4*>(y + (size_t)(u * kStepR) * a.Ks) = x;
                     }
                     res += (size_t)(4 * kStepR) * a.res_Cs;
                     y += (size_t)(4 * kStepR) * a.Ks;
@@ -420,7 +568,8 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         for (int kb = 0; kb < n_kb; ++kb) {
             const int t = kb & 1;
             const bool have = 2 * (kb0 + kb) + h < f.chunks;       // an odd number of chunks ends with half a step
-            uint4 v[8];
+            uint4 v[kRows ? 8 : 4];
+            const uint32_t from = smem + st * L::stage + (uint32_t)h * kBox + row * 128u;
             if constexpr (kRows) {
                 const int ih = ih0 + (2 * (kb0 + kb) + h) * a.dil_h;
                 const bool row_ok = have && ih >= 0 && ih < a.H;
@@ -438,18 +587,19 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                 }
             } else {
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[st]), parity, &s_abort, err, 0x22u))) break;
-                const uint32_t from = smem + st * L::stage + (uint32_t)h * kBox + row * 128u;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) v[c] = ld_shared_v4(from + (((uint32_t)c ^ swz) << 4));      // (without a second box: not used)
             }
             bool ok = true;
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
+                if constexpr (!kRows) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) v[c] = ld_shared_v4(from + (((uint32_t)(q * 4 + c) ^ swz) << 4));      // (without a second box: not used)
+                }
                 uint32_t p[3][8];
                 if (have) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        const uint4& x = v[q * 4 + c];
+                        const uint4& x = v[kRows ? q * 4 + c : c];
                         split2(x.x, x.y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
                         split2(x.z, x.w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
                     }
@@ -471,10 +621,15 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             __syncwarp();
             if (elect_one()) {
                 mbar_arrive(smem_u32(&s_ready[t]));
-                if (!kRows) mbar_arrive(smem_u32(&s_empty[st]));
+                mbar_arrive(smem_u32(&s_empty[st]));
             }
             __syncwarp();
             if (++st == ring) { st = 0; parity ^= 1u; }
+        }
+        block_await();
+        if (s_again) {
+            sum_again<BN, kRows>(f, smem_raw, s_full, s_empty, &s_abort);
+            block_meet();
         }
     } else if (warp < kWarpCopy) {
         // ===== weights to three parts, in shared memory: eight k of one channel at a time, lanes along the channels =====
@@ -517,6 +672,11 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             }
             __syncwarp();
             if (++st == ring) { st = 0; parity ^= 1u; }
+        }
+        block_await();
+        if (s_again) {
+            sum_again<BN, kRows>(f, smem_raw, s_full, s_empty, &s_abort);
+            block_meet();
         }
     } else if (warp == kWarpCopy) {
         // ===== copies =====
@@ -573,6 +733,11 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             chunk += 2;
             if (++st == ring) { st = 0; parity ^= 1u; }
         }
+        block_await();
+        if (s_again) {
+            copy_again<BN, kRows>(&tmap_x, &tmap_w, f, smem_raw, s_full, s_empty, &s_abort);
+            block_meet();
+        }
     } else {
         // ===== multiplications =====
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
@@ -602,6 +767,8 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             }
             __syncwarp();
         }
+        block_await();
+        if (s_again) block_meet();
     }
     tcgen05_fence_before();
     __syncthreads();

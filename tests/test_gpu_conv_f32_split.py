@@ -148,6 +148,64 @@ def test_values_that_are_not_finite(case, monkeypatch):
     assert ((a[ok] - b[ok]).double().norm() <= 1e-5 * b[ok].double().norm())
 
 
+@pytest.mark.parametrize("case", CASES)
+def test_second_pass(case):
+    """The same, and operands that are too large for the parts, at every tile, rank count and edge: not finite where the sums in 64 bits are
+    not, within the bound everywhere else."""
+    import torch
+    n, c, h, w = case[:4]
+    x = torch.randn((n, h, w, c), generator=torch.Generator(device="cuda").manual_seed(4), device="cuda")
+    for i, v in enumerate((float("inf"), -float("inf"), float("nan"), 2.0 ** 113, -3.4e37)):
+        x.view(-1)[(i + 1) * x.numel() // 7] = v
+    p, t = _prepare(case, act=0, residual=True, x=x)
+    _launch(p)
+    y, bound, _ = _reference(p, t, True)
+    out, want = t["y"][..., :p.K], y.float()
+    ok = torch.isfinite(want)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isposinf(out), torch.isposinf(want)) and torch.equal(torch.isneginf(out), torch.isneginf(want))
+    assert ((out.double() - y).abs()[ok] <= bound[ok]).all() and (t["y"][..., p.K:] == 7.0).all()
+
+
+@pytest.mark.parametrize("case", [CASES[2], CASES[10], CASES[15]])
+def test_infinite_weights_meet_the_padding(case, monkeypatch):
+    """Zeros beyond the edge times infinity, as on the fp32 units."""
+    import torch
+    outs = []
+    for on in "10":
+        monkeypatch.setenv("PB_F32_SPLIT", on)
+        p, t = _prepare(case, act=0)
+        t["w"][1, 0, 0, 0], t["w"][5, -1, -1, -1] = float("inf"), -float("inf")
+        t["wd"] = gu.pack_weights(capi.STAGE_CONV_SIMT, p, t["w"].cpu().numpy())
+        p.w = t["wd"].data_ptr()
+        _launch(p)
+        outs.append(t["y"][..., :p.K])
+    a, b = outs
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b)) and torch.isnan(b).any()
+
+
+@pytest.mark.parametrize("case", [CASES[10], CASES[13], CASES[15]])
+def test_poisoned_launches_take_no_longer_than_a_few_ordinary_ones(case, monkeypatch):
+    """Every pixel NaN: measured at 1.4 to 2 times the launch on the fp32 units (a serial sum per output took 20 to 50)."""
+    import torch
+    times = []
+    for on in "10":
+        monkeypatch.setenv("PB_F32_SPLIT", on)
+        p, t = _prepare(case, act=0)
+        t["x"].fill_(float("nan"))
+        _launch(p)
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        best = 1e9
+        for _ in range(5):
+            e[0].record()
+            for _ in range(10):
+                capi.load().pb_op_launch(capi.STAGE_CONV_SIMT, C.byref(p), None, 0, None)
+            e[1].record()
+            gu.sync()
+            best = min(best, e[0].elapsed_time(e[1]))
+        times.append(best)
+    assert times[0] < 4 * times[1]
+
+
 @pytest.mark.parametrize("act,k", [(0, 64), (3, 37)])
 @pytest.mark.parametrize("exponent", [-108, -114, -122])
 def test_operands_whose_parts_bf16_cannot_hold(exponent, act, k):

@@ -5,19 +5,21 @@
 //                                          k = (tap, input channel), taps of 32-channel chunks
 //
 // Both are multiplied by 2^16 first, so that bf16 holds the ends of the least fp32 value, too; then A = a0 + a1 + a2 and B = b0 + b1 + b2 exactly (8 bits
-// of mantissa each, rounded to nearest, so 24 and the signs), and of the nine products the six of weight 2^-18 and more are multiplied.
+// of mantissa each, rounded to nearest, so 24 and the signs).  a1 is 2^-8 of A at most and a2 2^-17, so of the nine products all are multiplied but a2 b2, 2^-34 of
+// a product.  (Without a1 b2 and a2 b1, up to 2^-24 of it, a sum of one product is 7.7e-8 off instead of 5.9e-8, its one rounding: 256 -> 256 channels on 16 maps
+// of 28 x 28 98.0 us, with them 103.8.)
 // The sums are multiplied by 2^-32 at the end.
 // Products of bf16 values are exact in fp32.  The tensor core's own additions do not round to nearest, so its sums are kept
-// short: an accumulator holds 64 values of k, and the products a0 b0 have one of their own, apart from the five small ones (whose
+// short: an accumulator holds 64 values of k, and the products a0 b0 have one of their own, apart from the seven small ones (whose
 // roundings are 2^-8 of theirs).  After every 64 k both are read from tensor memory and added to the sums in registers, which are
 // ordinary fp32.
 //
 // Block = 26 warps on a tile of 128 pixels x BN channels, in steps of 64 k:
 //   warp 24      copies, three or four steps ahead: two im2col boxes of 128 pixels x 32 channels and two of 32 x BN weights, fp32
 //   warps 8-15   split them: a thread has one box of a pixel, and leaves its three rows of bf16 in TENSOR memory, from where the tensor core
-//                takes operand A (shared memory then moves operand B only: six multiplications per 16 k read 6 x 2 KB there, not 6 x 6 KB)
+//                takes operand A (shared memory then moves operand B only: eight multiplications per 16 k read 8 x 2 KB there, not 8 x 6 KB)
 //   warps 16-23  split the weights, into shared memory
-//   warp 25      multiplies: 4 x 6 instructions of 128 x BN x 16 a step
+//   warp 25      multiplies: 4 x 8 instructions of 128 x BN x 16 a step
 //   warps 0-7    add up, half of the columns each, and finish the tile: bias, residual, activation
 // Tensor memory: two steps of operand A (192 columns) and two pairs of accumulators (4 BN).  A layer with few tiles splits its k range over
 // the blocks of a cluster, whose sums meet through distributed shared memory, in rank order: results do not depend on timing.
@@ -756,7 +758,9 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
                 for (int k = 0; k < 4; ++k) {
                     const uint32_t a0 = at + (uint32_t)(k * 8), a1 = a0 + 32u, a2 = a0 + 64u;
                     const uint64_t w0 = bt + (uint64_t)(k * 2), w1 = w0 + (L::part >> 4), w2 = w1 + (L::part >> 4);
-                    mma_ta(small, a0, w2, idesc, k > 0 ? 1u : 0u);
+                    mma_ta(small, a1, w2, idesc, k > 0 ? 1u : 0u);
+                    mma_ta(small, a2, w1, idesc, 1u);
+                    mma_ta(small, a0, w2, idesc, 1u);
                     mma_ta(small, a2, w0, idesc, 1u);
                     mma_ta(small, a1, w1, idesc, 1u);
                     mma_ta(small, a0, w1, idesc, 1u);

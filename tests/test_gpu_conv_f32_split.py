@@ -1,8 +1,8 @@
 """Dense fp32 convolutions on the tensor cores (operands split into three bf16 parts) at the sizes where they can go wrong, against
 torch in 64 bits.
 
-Bound: an output is sum(x w) over n = C*R*S products.  The parts reproduce the operands exactly; the products left out are at most
-3 * 2^-26 of each product.  A step of 64 products is four additions of 16 exact products each to an fp32 accumulator, every one of which
+Bound: an output is sum(x w) over n = C*R*S products.  The parts reproduce the operands exactly; the one product of parts that is left out is at
+most 2^-34 of each product.  A step of 64 products is four additions of 16 exact products each to an fp32 accumulator, every one of which
 may truncate (2^-23 of a partial sum, itself at most sum|x w| of the step), and one rounding to nearest adds it to the sums of the steps
 before it: together at most (8 + n / 64) * 2^-23 * sum|x w|.  Bias, residual and result add one rounding each."""
 import ctypes as C
@@ -216,6 +216,27 @@ def test_operands_whose_parts_bf16_cannot_hold(exponent, act, k):
     _launch(p)
     y, _, chain = _reference(p, t, False)
     assert ((t["y"][..., :k].double() - y).abs() <= chain + 64 * 9 * 2.0 ** -149).all()
+
+
+@pytest.mark.parametrize("case", [(2, 64, 9, 9, 64, 1, 1, 1, 0, 0, 1), (1, 512, 16, 16, 40, 1, 1, 1, 0, 0, 1), (2, 3, 32, 32, 64, 3, 3, 1, 1, 1, 1)])
+def test_a_sum_of_one_product_is_rounded_once(case):
+    """One channel of one pixel of the window is not zero: what is left out (2^-34) and lost in the sum of the small products (eight of
+    2^-8, truncated at 2^-23 each) is within 2^-27 of the result, besides the half unit, 2^-24, of its one rounding."""
+    import torch
+    n, c, h, w, k = case[:5]
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.zeros((n, h, w, c), device="cuda")
+    x[:, ::3, ::3, :] = torch.nn.functional.one_hot(torch.arange(x[:, ::3, ::3, 0].numel(), device="cuda") % c, c).view_as(x[:, ::3, ::3, :]) * 1.0
+    x *= 1 + torch.rand(x.shape, generator=gen, device="cuda")
+    x[x > 1.98] = 1 + 2.0 ** -8 - 2.0 ** -17         # the largest second and third parts
+    p, t = _prepare(case, act=0, x=x)
+    t["w"] = 1 + torch.rand(t["w"].shape, generator=gen, device="cuda")
+    t["w"].view(-1)[::3] = 1 + 2.0 ** -8 - 2.0 ** -17
+    t["wd"], p.bias = gu.pack_weights(capi.STAGE_CONV_SIMT, p, t["w"].cpu().numpy()), None
+    p.w = t["wd"].data_ptr()
+    _launch(p)
+    y = _reference(p, t, False)[0] - t["b"][:k].double()
+    assert ((t["y"][..., :k].double() - y).abs() <= (2.0 ** -24 + 2.0 ** -27) * y.abs()).all()
 
 
 @pytest.mark.parametrize("act,k", [(0, 64), (3, 37)])

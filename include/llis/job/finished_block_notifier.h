@@ -52,6 +52,30 @@ class FinishedBlockNotifier {
             }
         }
     }
+
+    // The same for a grid that was declared as `declared` blocks, whatever its size: this block's ticket stands for the tickets of that grid from
+    // declared * (ticket - 1) / blocks to declared * ticket / blocks, so the last of them is the last block's.
+    __device__ __forceinline__ void start_as(JobId job_id, unsigned declared) {
+        if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) records(InstrumentInfo::kStart, agg_counter_start_, job_id, declared, false);
+    }
+    __device__ __forceinline__ void end_as(JobId job_id, unsigned declared) {
+        __syncthreads();
+        if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
+            __threadfence();
+            records(InstrumentInfo::kEnd, agg_counter_end_, job_id, declared, true);
+        }
+    }
+    __device__ __forceinline__ void records(uint8_t kind, unsigned& counter, JobId job_id, unsigned declared, bool release) {
+        const unsigned g = gridDim.x * gridDim.y * gridDim.z;
+        const unsigned long long ticket = atomicInc(&counter, g - 1) + 1ull;
+        const unsigned last = (unsigned)(declared * ticket / g);
+        for (unsigned v = (unsigned)(declared * (ticket - 1) / g) + 1; v <= last; ++v) {
+            const unsigned batch = v % noti_batch_size_;
+            if (batch != 0 && v != declared) continue;
+            if (release) __threadfence();
+            channel_.write(kind, 0, (uint8_t)(batch == 0 ? noti_batch_size_ : batch), job_id, release);
+        }
+    }
 #endif
 
     // Host: n notifiers in device memory, all bound to `channel`.

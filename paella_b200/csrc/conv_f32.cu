@@ -41,6 +41,7 @@ struct F32Args {
     int Kp;              // channels of a row of packed weights (K rounded up to 4)
     int n_stages;        // k stages of the whole reduction
     int splits;          // cluster size
+    uint32_t declared;   // blocks this launch was declared as, where they are not the grid's (else 0)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -97,7 +98,10 @@ template <int BN, bool Aligned, bool Padded>
 __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, uint32_t job_id, FinishedBlockNotifier* nf) {
     griddep_wait();
     resolve_slot(job_id, nf);
-    if (nf) nf->start(job_id);
+    if (nf) {
+        if (f.declared) nf->start_as(job_id, f.declared);
+        else nf->start(job_id);
+    }
     constexpr int TJ = BN == 64 ? 8 : 4;           // channels per thread
     constexpr int kGroupThreads = 8 * BN / TJ, kGroups = kBlock / kGroupThreads, kGroupK = kTK / kGroups;
     constexpr int kStageFloats = kTK * kTM + kTK * BN;
@@ -269,7 +273,10 @@ __global__ void __launch_bounds__(kBlock, 2) conv_f32_kernel(const F32Args f, ui
         asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait.acquire;" ::: "memory");      // every rank has been read
     }
     griddep_launch();
-    if (nf) nf->end(job_id);
+    if (nf) {
+        if (f.declared) nf->end_as(job_id, f.declared);
+        else nf->end(job_id);
+    }
 }
 
 struct F32Geometry {
@@ -305,13 +312,15 @@ F32Geometry conv_f32_geometry(const pb_op_params* p) {
     const int groups = g.BN == 16 ? 8 : 4;
     const size_t pipe = (size_t)kDepth * (kTK * kTM + kTK * g.BN) * 4, red = (size_t)groups * kTM * (g.BN + 4) * 4;
     g.smem = (uint32_t)std::max(pipe, red);
-    const bool aligned = ((uintptr_t)p->w & 15) == 0, padded = p->C != p->Cs;
-#define PB_F32(BN_) (padded ? (aligned ? (const void*)conv_f32_kernel<BN_, true, true> : (const void*)conv_f32_kernel<BN_, false, true>) \
-                            : (aligned ? (const void*)conv_f32_kernel<BN_, true, false> : (const void*)conv_f32_kernel<BN_, false, false>))
+    const bool wide = ((uintptr_t)p->w & 15) == 0, padded = p->C != p->Cs;
+#define PB_F32(BN_) (padded ? (wide ? (const void*)conv_f32_kernel<BN_, true, true> : (const void*)conv_f32_kernel<BN_, false, true>) \
+                            : (wide ? (const void*)conv_f32_kernel<BN_, true, false> : (const void*)conv_f32_kernel<BN_, false, false>))
     g.fn = g.BN == 64 ? PB_F32(64) : (g.BN == 32 ? PB_F32(32) : PB_F32(16));
 #undef PB_F32
     return g;
 }
+
+bool aligned(const pb_op_params* p) { return (((uintptr_t)p->x | (uintptr_t)p->w) & 15) == 0; }
 
 }  // namespace
 
@@ -346,7 +355,13 @@ int conv_f32_info(const pb_op_params* p, pb_launch_info* out) {
     if (cudaFuncGetAttributes(&at, g.fn) == cudaSuccess) out->regs_per_thread = (uint32_t)at.numRegs;
     else cudaGetLastError();
     out->smem_per_block = g.smem;
-    if (conv_f32_split_takes(p)) conv_f32_split_info(p, out);
+    if (conv_f32_split_layer(p)) {
+        // The blocks do not depend on where the tensors are: the launch may be declared before that is known.
+        pb_launch_info split = *out;
+        conv_f32_split_info(p, &split);
+        if (aligned(p)) *out = split;
+        else out->num_blocks = split.num_blocks;
+    }
     const uint64_t nb = (uint64_t)batch_of(p), y = nb * p->K * p->P * p->Q;
     out->flops = 2ull * y * p->C * p->R * p->S;
     out->bytes = 4ull * (nb * p->C * p->H * p->W + (uint64_t)p->K * p->C * p->R * p->S + y + (p->residual ? y : 0)) + 4ull * p->K;
@@ -354,7 +369,8 @@ int conv_f32_info(const pb_op_params* p, pb_launch_info* out) {
 }
 
 int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl) {
-    if (conv_f32_split_takes(p)) return conv_f32_split_launch(p, op, st, job_id, notifier, pdl);
+    const bool split = conv_f32_split_layer(p);
+    if (split && aligned(p)) return conv_f32_split_launch(p, op, st, job_id, notifier, pdl);
     const F32Geometry g = conv_f32_geometry(p);
     F32Args f;
     f.op = op;
@@ -363,6 +379,12 @@ int conv_f32_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, ui
     f.Kp = round_up(p->K, 4);
     f.n_stages = g.n_stages;
     f.splits = g.splits;
+    f.declared = 0;
+    if (split) {
+        pb_launch_info li;
+        conv_f32_split_info(p, &li);
+        f.declared = li.num_blocks;
+    }
     PB_CUDA(cudaFuncSetAttribute(g.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)g.m_tiles, (unsigned)g.n_tiles, (unsigned)g.splits);

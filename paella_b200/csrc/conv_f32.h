@@ -6,8 +6,9 @@
 
 namespace pb {
 
-// Is this layer's launch the tensor-core kernel's?
-bool conv_f32_split_takes(const pb_op_params* p);
+// Is this layer the tensor-core kernel's?  (Its copies also want pixels and weights on 16-byte boundaries; a launch that has them elsewhere runs on the fp32
+// units and reports as many blocks as were declared.)
+bool conv_f32_split_layer(const pb_op_params* p);
 // Blocks and their resources (the rest of the record is the caller's).
 int conv_f32_split_info(const pb_op_params* p, pb_launch_info* out);
 int conv_f32_split_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);

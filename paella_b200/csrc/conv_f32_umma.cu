@@ -838,7 +838,7 @@ uint32_t* conv_f32_error_flag_ptr() {
     return static_cast<uint32_t*>(p);
 }
 
-// The layers that run here: what the copies can express - pixels and weights on 16-byte boundaries, the output size that follows from
+// The layers that run here: what the copies can express - the output size that follows from
 // padding, filter and stride (im2col boxes walk exactly those pixels), offsets within the descriptor's fields - and what gains.
 // - A box is 32 channels of one tap, so a layer of fewer than 24 would multiply zeros: 56 x 56, 3x3, 8 images, 8 / 16 / 24 / 32 channels -> 64 the
 //   fp32 units 18.7 / 24.5 / 30.7 / 36.1 us, here 19.1 / 19.1 / 19.2 / 19.1; one image 8.2 / 8.9 / 10.1 / 11.2 and 8.2 / 8.0 / 8.2 / 8.1.
@@ -847,11 +847,11 @@ uint32_t* conv_f32_error_flag_ptr() {
 // - Stems: 7 x 7, stride 2, 64 channels on 1 / 2 / 8 images of 224 x 224 22.4 / 32.3 / 110 and 9.7 / 17.9 / 51 us; 3 x 3, stride 2, 32 channels on 2
 //   and 8 10.6 / 31.2 and 10.1 / 28.1, 16 channels on 8 of 320 x 320 51.3 and 51.4, 8 channels 5 x 5 on one of 28 x 28 5.8 and 6.4.
 // PB_F32_SPLIT=0 (read at every use; for tests and comparisons) keeps every layer on the fp32 units.
-bool conv_f32_split_takes(const pb_op_params* p) {
+bool conv_f32_split_layer(const pb_op_params* p) {
     const char* e = getenv("PB_F32_SPLIT");
     if (e && e[0] == '0') return false;
     const int reach_h = (p->R - 1) * dil(p->dil_h), reach_w = (p->S - 1) * dil(p->dil_w);
-    return (p->C >= 24 || stem(p)) && (p->K > 32 || p->R * p->S > 1) && (((uintptr_t)p->x | (uintptr_t)p->w) & 15) == 0 && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
+    return (p->C >= 24 || stem(p)) && (p->K > 32 || p->R * p->S > 1) && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
            p->pad_w <= 100 && reach_h <= 100 && reach_w <= 100 && p->stride_h >= 1 && p->stride_w >= 1 && p->stride_h <= 8 && p->stride_w <= 8 &&
            p->P == (p->H + 2 * p->pad_h - reach_h - 1) / p->stride_h + 1 && p->Q == (p->W + 2 * p->pad_w - reach_w - 1) / p->stride_w + 1;
 }

@@ -283,3 +283,34 @@ def test_what_stays_on_the_fp32_units(what):
     _launch(p)
     y, _, chain = _reference(p, t, False)
     assert ((t["y"][..., :p.K].double() - y[:, :rows]).abs() <= chain[:, :rows]).all()
+
+
+@pytest.mark.parametrize("what", ["x", "w"])
+@pytest.mark.parametrize("case", [CASES[5], CASES[10], CASES[11], CASES[14], CASES[15]])
+def test_the_declared_blocks_do_not_depend_on_where_the_tensors_are(case, what):
+    """Declared before the tensors are known, launched with one off 16 bytes: as many starts and ends as declared, twice."""
+    import torch
+    from tests.test_gpu_ring import _drain, _unpack
+    from oracle import scheduler as osch
+    L, ring, nf = capi.load(), C.c_void_p(), C.c_void_p()
+    capi.check(L.pb_ring_create(0, 1 << 16, C.byref(ring)), "pb_ring_create")
+    capi.check(L.pb_notifier_create_array(ring, 1, C.byref(nf)), "pb_notifier_create_array")
+    p, t = _prepare(case)
+    x, w, p.x, p.w = p.x, p.w, None, None
+    li = capi.LaunchInfo()
+    capi.check(L.pb_op_info(capi.STAGE_CONV_SIMT, C.byref(p), C.byref(li)), "pb_op_info")
+    assert li.threads_per_block == 832
+    p.x, p.w = x, w
+    old = t["x"] if what == "x" else t["wd"].view(torch.float32)
+    t["moved"] = torch.zeros(old.numel() + 1, device="cuda")
+    t["moved"][1:] = old.reshape(-1)
+    setattr(p, what, t["moved"].data_ptr() + 4)
+    want = sorted(osch.notifier_records(li.num_blocks))
+    for job in (5, 6):
+        capi.check(L.pb_op_launch(capi.STAGE_CONV_SIMT, C.byref(p), None, job, nf), "pb_op_launch")
+        gu.sync()
+        recs = [_unpack(r) for r in _drain(L, ring, 2 * len(want), timeout=2.0)]
+        for kind in (0, 1):
+            assert sorted(r["num"] for r in recs if r["is_start"] == kind and r["job_id"] == job) == want
+    L.pb_notifier_free_array(nf)
+    L.pb_ring_destroy(ring)

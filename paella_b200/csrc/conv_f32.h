@@ -9,6 +9,8 @@ namespace pb {
 // Is this layer the tensor-core kernel's?  (Its copies also want pixels and weights on 16-byte boundaries; a launch that has them elsewhere runs on the fp32
 // units and reports as many blocks as were declared.)
 bool conv_f32_split_layer(const pb_op_params* p);
+// Modelled microseconds of a launch of up to 32 output channels on the fp32 units.
+double conv_f32_units_us(const pb_op_params* p);
 // Blocks and their resources (the rest of the record is the caller's).
 int conv_f32_split_info(const pb_op_params* p, pb_launch_info* out);
 int conv_f32_split_launch(const pb_op_params* p, const OpArgs& op, cudaStream_t st, uint32_t job_id, void* notifier, bool pdl);

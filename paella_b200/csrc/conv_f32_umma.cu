@@ -830,6 +830,13 @@ SplitGeometry split_geometry(const pb_op_params* p) {
     return g;
 }
 
+// Modelled microseconds of a launch of up to 32 output channels here (fitted as conv_f32_units_us is, 2.3 % off in the mean).
+double narrow_us(const pb_op_params* p) {
+    const SplitGeometry g = split_geometry(p);
+    const int waves = ceil_div(g.m_tiles * g.n_tiles * g.splits, g.splits == 8 ? 120 : g.splits == 4 ? 132 : 148);
+    return 0.3 + waves * (4.1 + 0.736 * ceil_div(ceil_div(g.chunks, 2), g.splits) + (g.splits == 1 ? 0.0 : g.splits == 2 ? 0.65 : g.splits == 4 ? 1.0 : 1.2));
+}
+
 }  // namespace
 
 uint32_t* conv_f32_error_flag_ptr() {
@@ -843,7 +850,10 @@ uint32_t* conv_f32_error_flag_ptr() {
 // - A box is 32 channels of one tap, so a layer of fewer than 24 would multiply zeros: 56 x 56, 3x3, 8 images, 8 / 16 / 24 / 32 channels -> 64 the
 //   fp32 units 18.7 / 24.5 / 30.7 / 36.1 us, here 19.1 / 19.1 / 19.2 / 19.1; one image 8.2 / 8.9 / 10.1 / 11.2 and 8.2 / 8.0 / 8.2 / 8.1.
 // - 1x1 layers of up to 32 output channels are short and store little: 256 -> 24 at 14 x 14 5.6 and 7.3, 128 -> 24 at 28 x 28 x 8 6.2 and 6.4 (36
-//   columns: 7.2 and 7.2, 9.1 and 6.7); 3x3 layers gain at any width (64 -> 8 at 56 x 56 8.5 and 8.6, x 8 images 28.5 and 23.1).
+//   columns: 7.2 and 7.2, 9.1 and 6.7).
+// - Larger filters of up to 32 output channels: whichever of two fitted times is less (narrow_us, conv_f32_units_us): 64 -> 16 3x3 on one of 28 x 28 5.6 and
+//   7.5, 1x7 on one of 7 x 7 5.3 and 7.9, 64 -> 8 3x3 on 8 of 56 x 56 28 and 23.  Over 381 such layers of 32 channels and more the units take 9.36 ms, this kernel
+//   6.16, the faster of the two 5.996, the modelled one 5.997.  (With 24 to 31 channels and in stems, below, this kernel takes them all.)
 // - Stems: 7 x 7, stride 2, 64 channels on 1 / 2 / 8 images of 224 x 224 22.4 / 32.3 / 110 and 9.7 / 17.9 / 51 us; 3 x 3, stride 2, 32 channels on 2
 //   and 8 10.6 / 31.2 and 10.1 / 28.1, 16 channels on 8 of 320 x 320 51.3 and 51.4, 8 channels 5 x 5 on one of 28 x 28 5.8 and 6.4.
 // PB_F32_SPLIT=0 (read at every use; for tests and comparisons) keeps every layer on the fp32 units.
@@ -851,7 +861,7 @@ bool conv_f32_split_layer(const pb_op_params* p) {
     const char* e = getenv("PB_F32_SPLIT");
     if (e && e[0] == '0') return false;
     const int reach_h = (p->R - 1) * dil(p->dil_h), reach_w = (p->S - 1) * dil(p->dil_w);
-    return (p->C >= 24 || stem(p)) && (p->K > 32 || p->R * p->S > 1) && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
+    return (p->C >= 24 || stem(p)) && (p->K > 32 || (p->R * p->S > 1 && (p->C < kChunk || narrow_us(p) < conv_f32_units_us(p)))) && p->pad_h >= 0 && p->pad_w >= 0 && p->pad_h <= 100 &&
            p->pad_w <= 100 && reach_h <= 100 && reach_w <= 100 && p->stride_h >= 1 && p->stride_w >= 1 && p->stride_h <= 8 && p->stride_w <= 8 &&
            p->P == (p->H + 2 * p->pad_h - reach_h - 1) / p->stride_h + 1 && p->Q == (p->W + 2 * p->pad_w - reach_w - 1) / p->stride_w + 1;
 }

@@ -1933,7 +1933,7 @@ static WinTile win_tile(int kind, const pb_op_params* p) {
 // or 2, and at least 100 blocks in the launch (all images).  Measured on Inception-v3 served in gangs of 8: thresholds of
 // 30, 100 and 300 blocks give the same +2 % requests/s over 592 (its two stem max pools then run here); below 100 a lone
 // request's pooling layers are a few dozen blocks and keep the strip kernels, which finish sooner on an idle GPU.
-// PB_WINDOW_TILE=0 switches it off; PB_WINDOW_TILE_MIN_BLOCKS sets another threshold (tests use 1).  Read at every call:
+// PB_WINDOW_TILE=0 switches it off (=1: see win_ring); PB_WINDOW_TILE_MIN_BLOCKS sets another threshold (tests use 1).  Read at every call:
 // this runs when a launch is built (graph capture, direct operator calls), never on the replay path.
 static uint32_t tile_blocks(int kind, const pb_op_params* p) {
     if (p->dtype != 1 || (p->Cs & 7) || (p->Ks & 3) || (p->out_c_off & 3) || p->act > 2 || strip_of(p) == 0) return 0;
@@ -1980,7 +1980,10 @@ static const void* tile_fn(int kind, const pb_op_params* p) {
 
 // Ring of a launch's window: depthwise windows of stride 1 whose column tiles have seven or eight strips (four walking warps; with five
 // strips, 256 maps of 64 x 40 x 16, 37 us become 47) and whose rows give every block 24 and more (a block's range starts with two rows of
-// no output; fewer blocks than the GPU holds lose more than the ring gains).  Tiles / ring: 64 maps of 112 x 112 x 128 86.0 / 82.0 us, 32 of
+// no output; fewer blocks than the GPU holds lose more than the ring gains), and where its walks are a tenth shorter than the tiles': one walk down a map of
+// P rows takes P + 2, in threes, a tile's two more than its own; a map that one tile holds gains nothing and pays for ranges that end inside of it
+// (tiles / ring: 100 MB of 14 x 28 x 64 maps 45.1 / 46.9 us, 10 x 32 36.7 / 40.7, 5 x 112 56.6 / 63.8, 20 x 112 42.1 / 45.9; 19 x 28 49.7 / 42.5, 28 x 28 43.7 / 41.7).
+// PB_WINDOW_TILE=1: wherever it can run (for tests).  Tiles / ring: 64 maps of 112 x 112 x 128 86.0 / 82.0 us, 32 of
 // 224 x 224 x 64 83.6 / 71.9, 4 of 300 x 500 x 96 63.4 / 55.5, 64 of 57 x 57 x 200 50.6 / 45.7, 2 of 200 x 200 x 640 45.3 / 44.8.
 static WinRing win_ring(int kind, const pb_op_params* p) {
     WinRing g = {};
@@ -1995,6 +1998,13 @@ static WinRing win_ring(int kind, const pb_op_params* p) {
     const int ranges = 3 * 148 / g.slabs;
     const long long rows = (long long)batch_of(p) * g.col_tiles * p->P;      // of a slab
     if (g.strips < 7 || ranges < 1 || rows < 24ll * ranges || rows > 0x3fffffff) return g;
+    const char* e = getenv("PB_WINDOW_TILE");
+    if (!e || e[0] != '1') {
+        const WinTile t = win_tile(kind, p);
+        const long long tile_walks = (long long)ceil_div(p->P, t.rows) * t.col_tiles * t.strips * t.bands * ceil_div(t.band_rows + 2, 3);
+        const long long ring_walks = (long long)g.col_tiles * g.strips * ceil_div(p->P + 2, 3);
+        if (t.rows >= p->P || 10 * tile_walks < 11 * ring_walks) return g;
+    }
     g.rows = (int)rows;
     g.blocks = ranges * g.slabs;
     return g;

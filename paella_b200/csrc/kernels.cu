@@ -867,7 +867,7 @@ struct WinLane {
 };
 
 template <int kMode, int kStride, int kAct, bool kCountPad, bool kWide>
-__global__ void __launch_bounds__(kTileMaxThreads, kMode == kWinDw ? 3 : 4) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
+__global__ void __launch_bounds__(kTileMaxThreads, kMode == kWinAvg ? 4 : 3) window3_tile_kernel(OpArgs a, WinTile g, const __grid_constant__ CUtensorMap tmap, uint32_t job_id,
                                                                         FinishedBlockNotifier* nf) {
     PB_NOTIFY_START();
     typedef WinLane<kMode, kStride, kAct, kCountPad, kWide> Lane;
@@ -1884,9 +1884,10 @@ static size_t strip_threads(const pb_op_params* p, int strip) {
 // for 256 images of 35 x 35 x 192 instead of 51), so their tiles are fitted to the map: as few column tiles as hold at most 40 columns
 // each, as many rows as keep the window (the rows a walk runs past the tile included) within 74 KB, so that three blocks fit an SM,
 // and bands of rows where a map has fewer strips than half-warps.
-// A pooling lane holds no filter, so four of its blocks fit an SM's registers, and a batch's windows are cut for four (average, 256 maps of
-// 35 x 35 x 192 49.2 -> 47.2 us, the smaller windows alone 53.1, five blocks 47.2; 256 of 17 x 17 x 256 25.0 -> 20.7; maximum 20.7 -> 17.5, stride 2 on
-// 64 of 35 x 35 x 288 14.3 -> 12.6).  Depthwise blocks, whose registers allow three, lose with them (256 of 35 x 35 x 192 55.7 -> 59.8).
+// A pooling lane holds no filter, so four of its blocks fit an SM's registers (maxima without asking: asked for, 26 of 71 x 71 x 192 take 17.4 us instead of
+// 17.2), and a batch's windows are cut for four (average, 256 maps of 35 x 35 x 192 49.2 -> 48.3 us, the smaller windows alone 53.1; 256 of
+// 17 x 17 x 256 25.0 -> 20.7; maximum 20.7 -> 17.5, stride 2 on 64 of 35 x 35 x 288 14.3 -> 12.6) - not where whole
+// waves of them read a quarter more (97 of 56 x 30 x 192 at stride 2, two waves of the larger or three 8.3 and 9.0; 78 of them, two and two, 7.4 and 7.0).  Depthwise blocks, whose registers allow three, lose with them (256 of 35 x 35 x 192 55.7 -> 59.8).
 constexpr int kTileWindowBytes = 74 * 1024, kTileWindowBytesPool = 54 * 1024;
 static WinTile win_tile_within(const pb_op_params* p, int limit) {
     const int st = p->stride_h, strip = st == 1 ? kTileStrip1 : kTileStrip2;
@@ -1926,7 +1927,11 @@ static size_t win_blocks(const pb_op_params* p, const WinTile& g) { return (size
 static WinTile win_tile(int kind, const pb_op_params* p) {
     const WinTile g = win_tile_within(p, kTileWindowBytes);
     const bool fills = win_blocks(p, g) * batch_of(p) >= 3 * 148;      // else more blocks are only more halo: 8 of 147 x 147 x 64 4.4 -> 4.8
-    return kind != PB_STAGE_DWCONV && batch_of(p) > 1 && fills ? win_tile_within(p, kTileWindowBytesPool) : g;
+    if (kind == PB_STAGE_DWCONV || batch_of(p) == 1 || !fills) return g;
+    const WinTile small = win_tile_within(p, kTileWindowBytesPool);
+    // whole waves of blocks, each as long as its windows
+    auto waves = [&](const WinTile& t, int per_sm) { return (double)ceil_div((int)std::min<size_t>(win_blocks(p, t) * batch_of(p), 1u << 30), 148 * per_sm) * per_sm * t.alloc_rows * t.in_cols; };
+    return waves(small, 4) > 1.25 * waves(g, 3) ? g : small;
 }
 
 // Blocks of window3_tile_kernel for one image, or 0 when the layer keeps the strip kernels: bf16, a 3x3 window of stride 1

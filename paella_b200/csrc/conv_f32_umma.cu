@@ -383,7 +383,11 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     constexpr uint32_t ring = L::ring;
     uint32_t* const err = &g_f32_err_flag;
 
-    if (warp == kWarpCopy) {            // a lane per barrier
+    if (warp == kWarpCopy) {            // the maps are on their way while the barriers are set up, a lane per barrier
+        if (elect_one()) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+            if (!kRows) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+        }
         if (lane < (int)ring) {
             mbar_init(smem_u32(&s_full[lane]), 1);
             mbar_init(smem_u32(&s_empty[lane]), 16);
@@ -396,9 +400,6 @@ conv_f32_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             if (f.splits > 1) mbar_arrive_expect_tx(smem_u32(s_sums), (uint32_t)((f.splits - 1) * (kTileRows >> ranks_log2) * BN * 4));
             s_abort = 0;
             s_again = 0;
-        } else if (lane == 24) {
-            if (!kRows) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();

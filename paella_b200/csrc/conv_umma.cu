@@ -121,14 +121,16 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Optional phase stamps for development builds (-DPB_CONV_TIMING): %globaltimer at eight points of
-// the first 64 CTAs, written to a device array the probe program reads back.
+// Optional phase stamps for development builds (-DPB_CONV_TIMING): %globaltimer at ten points of
+// the first 64 CTAs (8: sent to the other ranks, 9: their parts are here), written to a device array the probe program reads back.
 #ifdef PB_CONV_TIMING
-__device__ unsigned long long g_conv_t[64 * 8];
+constexpr int kConvStamps = 10;
+__device__ unsigned long long g_conv_t[64 * kConvStamps];
 #define PB_T(i)                                                                                         \
     do {                                                                                                \
+        static_assert((i) < kConvStamps, "a slot of its own for every stamp");                         \
         const unsigned b_ = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);             \
-        if (b_ < 64) g_conv_t[b_ * 8 + (i)] = globaltimer_ns();                                         \
+        if (b_ < 64) g_conv_t[b_ * kConvStamps + (i)] = globaltimer_ns();                                         \
     } while (0)
 // per-k-block SM-clock stamps of the first 8 CTAs: [cta][kb][0 = loads issued, 1 = operands landed, 2 = MMAs issued]
 __device__ unsigned long long g_conv_kb[8 * 64 * 3];
@@ -550,7 +552,7 @@ __device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_ba
             send(v1);
         }
     }
-    if (tid == 0) PB_T(10);
+    if (tid == 0) PB_T(8);
     // This rank's own first columns (zeros if it had no k-blocks), under the wait for the others' parts.
     tcgen05_wait_ld();
     const uint32_t own_addr = lane_addr + (uint32_t)(rank * w);
@@ -565,7 +567,7 @@ __device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_ba
 #pragma unroll
         for (int j = 0; j < 8; ++j) v0[j] = 0;
     }
-    if (tid == 0) PB_T(11);
+    if (tid == 0) PB_T(9);
     if (ok) {
         __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
         const uint32_t others = (active & ((1u << rank) - 1u)) | ((active >> (rank + 1)) << rank);

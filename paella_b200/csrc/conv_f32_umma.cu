@@ -115,12 +115,6 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t x, uint64_t y, uint64_t z
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
     return r;
 }
-// 16 bytes into another block's shared memory, counted by its barrier.
-__device__ __forceinline__ void st_async_v4(uint32_t addr, const float4& v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-                 ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
-                 : "memory");
-}
 __device__ __forceinline__ void tcgen05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // lo and hi less the bf16 values of the pair, exactly.  (The mixed multiply-add reads a half of a register: two instructions where widening the
@@ -163,7 +157,7 @@ struct Meeting {
     __device__ __forceinline__ void put(int col, const float4& v) const {      // columns col .. col + 3
         const uint32_t off = (((uint32_t)col >> 2) ^ mix) << 4;
         if (mine) st_shared_v4(at + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
-        else st_async_v4(to + off, v, bar);
+        else st_async_v4(to + off, __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w), bar);
     }
 };
 

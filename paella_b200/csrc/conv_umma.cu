@@ -170,10 +170,6 @@ __device__ unsigned long long g_conv_ns;             // sum of the CTAs' lifetim
 // folded in: cvt's .relu clamps negatives to zero, ReLU6 is one more packed min against 6.0.
 // Rounding is monotonic and 0 and 6 are bf16 values, so activation-after-rounding equals
 // rounding-after-activation.
-// The activation is chosen at run time, by branches all threads take alike: as a template parameter of the epilogues it made four
-// copies of each (and of each cluster size), 124 KB of code per kernel, and a launch whose copy had not run on its SM lately
-// spent 0.5 to 1.6 us of its epilogue fetching it.  The loops below are kept rolled for the same reason.  Two copies, ReLU and ReLU6 /
-// the others, are as fast as four where the arguments are constants (the lone launches): see EpiArgs.
 // n / d for n >= 0, with d's reciprocal: a few instructions where the integer division is a chain of twenty to forty (a block's set-up had five
 // of them in a row).  The estimate is off by one at most while the quotient is below 2^22; the loops make it right whatever it is.
 __device__ __forceinline__ int quotient(int n, int d, float inv, int& rem) {
@@ -205,6 +201,10 @@ __device__ __forceinline__ EpiArgs epi_args(const ConvArgs& a) {
     return {a.residual, a.bias, a.y, a.err_flag, a.M, a.K, a.Ks, a.out_c_off, a.res_Cs, a.act, a.BN, a.out_box, a.splits, a.nkb, a.meet};
 }
 
+// The activation is chosen at run time, by branches all threads take alike: as a template parameter of the epilogues it made four
+// copies of each (and of each cluster size), 124 KB of code per kernel, and a launch whose copy had not run on its SM lately
+// spent 0.5 to 1.6 us of its epilogue fetching it.  The loops below are kept rolled for the same reason.  Two copies, ReLU and ReLU6 /
+// the others, are as fast as four where the arguments are constants (the lone launches): see EpiArgs.
 // kAct: 0 = the activation is chosen here, 1 = it is ReLU or ReLU6, 2 = it is neither.
 // Eight accumulator columns of this thread's row, from channel k on: + bias (+ residual), activation, bf16.  The four epilogue
 // warps run one per scheduler with nothing to hide instruction latency behind, so this is kept to one packed add and one
@@ -395,19 +395,15 @@ __device__ __forceinline__ void epilogue(const Args& a, uint32_t tmem_base, bool
 // ---- split reduction: the thread blocks of a cluster share one output tile -----------------------------------
 // Rank z of the cluster multiplies its share of the k-blocks; then rank d finishes columns [d*w, (d+1)*w) of the
 // tile, w = BN / splits.  Every rank sends each owner its part straight from tensor memory (st.async: registers into the owner's
-// shared memory, counted by the owner's barrier), 16 bytes per lane and consecutive lanes (= rows) side by side; the owner adds the
-// parts in rank order, its own from its tensor memory, so the fp32 result does not depend on timing.  Where the pipeline leaves
+// shared memory, counted by the owner's barrier), 16 bytes per lane and consecutive lanes (= rows) side by side; the owner adds them
+// in rank order to its own part, from its tensor memory, so the fp32 result does not depend on timing (in rank order all told, with its own among
+// them, Inception-v3 alone takes 264 us instead of 262, ResNet-18 x 3 images 116.6 instead of 114.8).  Where the pipeline leaves
 // room the parts have a place of their own and a rank sends as soon as its accumulator is complete; else they land in
 // the owner's pipeline buffers, and every rank first tells the others that its multiplications are done with them.
 // Nobody waits for having been read: a block ends when the others' parts, and before them their messages, have arrived.
 // Bound by the way between SMs: with development probes 800 clocks and 20 bytes a clock per SM, however it is used; owners that pulled parked
 // tiles with loads saw 8 to 10 (48 KB at four ranks 5080 clocks, 28 KB at eight 5070; st.async 3110 and 2410), and two cluster barriers
 // besides.  (A global workspace under an atomic counter, before: +4 to +8 us per launch.)
-__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-                 ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar)
-                 : "memory");
-}
 // (Relaxed: it says that memory has been read, and a release takes 1500 clocks.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -435,7 +431,7 @@ __device__ __forceinline__ uint32_t meet_bytes(const Args& a, int rank) {
 }
 
 // The columns of this rank: its own part, then the others' in rank order.  `at` is this thread's row of those, [rank but this][4 columns][row].
-template <int kAct, class Args>
+template <class Args>
 __device__ __forceinline__ void cluster_finish(const Args& a, uint32_t own_addr, int k0, bool row_valid, __nv_bfloat16* yrow, const __nv_bfloat16* rrow,
                                                const float* bias, uint32_t others, uint32_t at, int w, bool mine, uint32_t (&own)[8], uint4 res) {
     const uint32_t step = (uint32_t)(w >> 2) * 2048u;      // between two ranks' parts
@@ -480,7 +476,7 @@ __device__ __forceinline__ void cluster_finish(const Args& a, uint32_t own_addr,
             uint32_t v[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) asm("mov.b64 {%0, %1}, %2;" : "=r"(v[2 * j]), "=r"(v[2 * j + 1]) : "l"(sum[j]));
-            *reinterpret_cast<uint4*>(yrow + k) = finish8<kAct>(a, v, res, rrow != nullptr, k, bias + c);
+            *reinterpret_cast<uint4*>(yrow + k) = finish8<0>(a, v, res, rrow != nullptr, k, bias + c);
         }
         res = next;
         tcgen05_wait_ld();
@@ -492,7 +488,7 @@ __device__ __forceinline__ void cluster_finish(const Args& a, uint32_t own_addr,
 }
 
 // Run by warps 0-3 of every rank.  s_go: the other ranks' pipelines are free (splits - 1 arrivals); s_parts: their parts are here.
-template <bool kByAct, class Args>
+template <class Args>
 __device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_base, int m0, int n0, int rank, uint32_t smem_base, const float* s_bias,
                                                  uint64_t* s_accum_p, uint64_t* s_go, uint64_t* s_parts, volatile uint32_t* s_abort_p) {
     const int tid = threadIdx.x;
@@ -572,9 +568,7 @@ __device__ __forceinline__ void epilogue_cluster(const Args& a, uint32_t tmem_ba
         __nv_bfloat16* yrow = a.y + (size_t)m * a.Ks + a.out_c_off;
         const uint32_t others = (active & ((1u << rank) - 1u)) | ((active >> (rank + 1)) << rank);
         const float* bias = s_bias + rank * w;
-        if constexpr (!kByAct) cluster_finish<0>(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
-        else if (a.act == 1 || a.act == 2) cluster_finish<1>(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
-        else cluster_finish<2>(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
+        cluster_finish(a, own_addr, k0, row_valid, yrow, rrow, bias, others, at, w, mine, v0, res);
     }
 }
 
@@ -967,13 +961,9 @@ __device__ __forceinline__ void conv_tile_tma(const CUtensorMap* tmap_w, const C
         griddep_wait();
         if (tid == 0) PB_S(2);
         griddep_launch();
-        if constexpr (kLone) {
-            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, smem_base, s_bias, s_accum, s_go, s_parts, s_abort);
-            else epilogue<true>(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
-        } else {
-            if (a.splits > 1) epilogue_cluster<false>(epi_args(a), tmem_base, m0, n0, bz, smem_base, s_bias, s_accum, s_go, s_parts, s_abort);
-            else epilogue<false>(epi_args(a), tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
-        }
+        if (a.splits > 1) epilogue_cluster(epi_args(a), tmem_base, m0, n0, bz, smem_base, s_bias, s_accum, s_go, s_parts, s_abort);
+        else if constexpr (kLone) epilogue<true>(a, tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
+        else epilogue<false>(epi_args(a), tmem_base, true, m0, n0, s_bias, s_accum, s_abort, 0u, a.out_box ? tmap_y : nullptr, smem_base, s_res, publish);
         if (tid == 0) { PB_T(6); PB_S(6); }
     } else if (warp == 4) {
         // ===== operand A =====

@@ -139,8 +139,9 @@ __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
     asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
-// Thread-block cluster: barrier halves (every thread of every block of the cluster takes part), the address of
-// this block's shared memory word in block `rank`, a 16-byte load from it.
+// Thread-block cluster: barrier halves, the address of this block's shared memory word in block `rank`.  Every thread of every block arrives
+// once its block's mbarriers are set up; only the warps that send to other blocks wait.  There is no second barrier: a block ends when everything
+// that the others send to it has arrived, which its own mbarriers count.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 // Orders nothing: for a rank that has only read.  (A release here would wait for the tile's stores to global memory.)
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
@@ -150,10 +151,11 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, uint32_t ra
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
+// 16 bytes from registers into another block's shared memory, counted by its barrier.
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ void tcgen05_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 

@@ -27,6 +27,7 @@ CASES = [
     (1, 256, 7, 64, 3, 64, 8, True),
     (1, 128, 17, 512, 3, 64, 4, True),
     (1, 512, 17, 512, 3, 128, 8, False),         # eight ranks that send into each other's buffers
+    (8, 256, 17, 160, 5, 64, 4, False),          # 25 k-blocks a rank: a stage more instead of a place beside the pipeline
     (1, 520, 8, 72, 3, 64, 8, True),             # channels and columns past whole boxes and tiles
 ]
 
@@ -37,7 +38,8 @@ def _check_route(li, n, c, h, k, r, columns, ranks, beside):
     assert li.num_blocks == -(-n * h * h // 128) * -(-k // columns) * ranks
     stage, parts, k_blocks = 16384 + columns * 128, (columns - columns // ranks) * 512, -(-r * r * -(-c // 64) // ranks)
     stages = (111616 - (parts if beside else 0)) // stage
-    assert beside == ((111616 - parts) // stage >= max(2, min(3, k_blocks)))
+    room = (111616 - parts) // stage
+    assert beside == (room >= max(2, min(3, k_blocks)) and (k_blocks <= 20 or room >= min(8, k_blocks, 111616 // stage)))
     pipe = max(2, min(8, k_blocks, stages)) * stage
     assert 1024 <= li.smem_per_block - (pipe + parts if beside else max(pipe, parts)) < 4096          # (alignment; barriers and biases)
 

@@ -3,7 +3,7 @@
 //   D[m, n] = sum_k A[m, k] * B[k, n]     m = output pixel (all images back to back), n = output channel,
 //                                          k = (r*S + s)*Cs + c   (filter tap, input channel)
 //
-// The layers that conv_f32_umma.cu leaves: five to 23 input channels, narrow 1x1 layers, unaligned tensors, output sizes of the caller's own.
+// The layers that conv_f32_umma.cu leaves: five to 23 input channels, short layers of few outputs, unaligned tensors, output sizes of the caller's own.
 // The ceiling is the fused multiply-add rate: 148 SMs x 128 x 2 x 1.9 GHz = 72 TFLOP/s.  The direct kernel this replaces for dense layers (conv_simt_kernel: one output per thread, every operand
 // through L1 for each multiplication) ran at 1.9 TFLOP/s.
 //

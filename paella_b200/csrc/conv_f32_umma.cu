@@ -24,15 +24,15 @@
 // Tensor memory: two steps of operand A (192 columns) and two pairs of accumulators (4 BN).  A layer with few tiles splits its k range over
 // the blocks of a cluster, whose sums meet through distributed shared memory, in rank order: results do not depend on timing.
 //
-// Bound by the instructions of the splitting warps (about 1250 issue slots a scheduler and step) and, where a launch has few steps, by the
-// latency of a step's chain: 0.76 us at 64 columns, 0.68 at 32.  Measured against the kernel on the fp32 units, us a launch in a chain:
-// 64 -> 64 3x3 on 2 maps of 56 x 56 23.1 -> 8.8, 128 -> 128 on 2 of 28 x 28 21.7 -> 9.5, 512 -> 512 on 2 of 7 x 7 29.2 -> 12.5, 256 -> 256 on 16 of
-// 28 x 28 408 -> 97 (152 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 214.  Error against 64 bits, relative, fp32 units / here:
+// Bound by the tensor pipe and the instructions of all warps together (59 % and 1120 issue slots a scheduler and step, 64 %, in a large layer) and, where a
+// launch has few steps, by the latency of a step's chain: 0.84 us at 64 columns, 0.74 at 32.  Measured against the kernel on the fp32 units, us a launch in a
+// row of equal ones: 64 -> 64 3x3 on 2 maps of 56 x 56 23.3 -> 10.6, 128 -> 128 on 2 of 28 x 28 22.1 -> 11.0, 512 -> 512 on 2 of 7 x 7 29.5 -> 14.6,
+// 256 -> 256 on 16 of 28 x 28 408 -> 103 (143 TFLOP/s of fp32 multiply-adds); ResNet-18 x 2 images 429 -> 213.  Error against 64 bits, relative, fp32 units / here:
 // 1.62e-7 / 8.3e-8, 1.14e-7 / 8.1e-8, 1.86e-7 / 9.8e-8, 3.03e-7 / 1.24e-7 (the layers above), 64 -> 64 1x1 7.1e-8 / 5.9e-8.
 //
 // Infinities, NaN and operands of 2^112 and more make 0 x inf of the parts, and sums of 2^96 and more overflow: a block that finds one of its sums not finite
-// makes them all again in a second pass, as plain fp32 multiply-adds of the same copies (28 TFLOP/s; one thread a poisoned output, as it was, took
-// 10.9 ms for 256 -> 256 on 16 of 28 x 28 where every pixel is NaN, 0.49 ms for 64 -> 64 on 2 of 56 x 56; this 0.56 ms and 34 us, the fp32 units 0.41 and 23).
+// makes them all again in a second pass, as plain fp32 multiply-adds of the same copies (32 TFLOP/s; one thread a poisoned output, as it was, took
+// 10.9 ms for 256 -> 256 on 16 of 28 x 28 where every pixel is NaN, 0.49 ms for 64 -> 64 on 2 of 56 x 56; this 0.57 ms and 34 us, the fp32 units 0.41 and 23).
 // What is small is exact (64 -> 64 3x3, relative error against 64 bits here / on the fp32 units: inputs of 2^-122 and weights of 2^30 8.5e-8 / 1.1e-7, 2^-140 and
 // 2^100 7.0e-8 / 1.1e-7, results of 2^-134 3.3e-6 / 3.7e-5; without the scaling 1.4e-4, 1.0 and 5.8e-5).
 //
@@ -806,7 +806,7 @@ SplitGeometry split_geometry(const pb_op_params* p) {
     g.m_tiles = ceil_div(batch_of(p) * p->P * p->Q, kTileRows);
     const int steps = ceil_div(g.chunks, 2);
     // Least modelled time: waves of one block an SM, each a block's fixed time (operand latency, the meeting of the ranks' sums, stores) and
-    // its steps.  Measured in chains of equal launches, tile width / ranks -> us: 256 -> 256 channels 3x3 on 2 maps of 14 x 14 64/1 31.4, 64/2 18.2,
+    // its steps.  Measured in chains of equal launches (with six products a step; eight take 0.74 and 0.84 us), tile width / ranks -> us: 256 -> 256 channels 3x3 on 2 maps of 14 x 14 64/1 31.4, 64/2 18.2,
     // 64/4 11.9, 64/8 17.5 (two waves), 32/1 27.6, 32/2 15.9, 32/4 11.1; 512 -> 512 on 2 of 7 x 7 58.6, 31.8, 18.6, 12.5, 52.2, 28.0, 16.1, 20.6; 512 -> 512
     // 1x1 on one of 14 x 14 9.9, 7.4, 6.2, -, 8.5, 6.2, 5.9.
     static const struct { int splits, blocks; double fixed[2]; } kRanks[] = {{1, 148, {3.2, 4.0}}, {2, 148, {3.7, 4.6}}, {4, 132, {4.2, 5.1}}, {8, 120, {4.6, 5.6}}};
@@ -866,7 +866,7 @@ int conv_f32_split_info(const pb_op_params* p, pb_launch_info* out) {
     out->num_blocks = (uint32_t)(g.m_tiles * g.n_tiles * g.splits);
     out->threads_per_block = kThreadsF;
     cudaFuncAttributes at;
-    out->regs_per_thread = 144;
+    out->regs_per_thread = 72;
     if (cudaFuncGetAttributes(&at, g.fn) == cudaSuccess) out->regs_per_thread = (uint32_t)at.numRegs;
     else cudaGetLastError();
     out->smem_per_block = g.smem;

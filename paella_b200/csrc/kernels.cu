@@ -986,9 +986,9 @@ __global__ void __launch_bounds__(kTileMaxThreads, kMode == kWinAvg ? 4 : 3) win
 // The depthwise walk (stride 1) over tensors of many rows, with the window in a ring: a fixed number of blocks share all rows of all
 // (image, column tile) units of their slab between them, each a contiguous range, and walk down it while one warp copies the next three window
 // rows.  A tile of window3_tile_kernel reads two rows more than the thirteen it writes; here that is once per unit or range, and the blocks
-// neither fill and walk in turn nor end in waves.  Bound by DRAM with reads and writes mixed: 128 x 1024 x 1024 104 -> 95.5 us (86 % of the copy
-// rate), and 98, 104 and 108 with rings of three, four and five stages - more rows under way are more places open at once; with the slabs of
-// a pixel in different ranges 113.  Average pooling gains nothing here (256 maps of 35 x 35 x 192: tiles 49.2, rings 49.4 to 55 us).
+// neither fill and walk in turn nor end in waves.  Bound by DRAM with reads and writes mixed: 128 x 1024 x 1024 104 -> 98.4 us (84 % of the copy
+// rate); rings of three, four and five stages take 2, 9 and 13 % more - more rows under way are more places open at once; with the slabs of
+// a pixel in different ranges 18 %.  Average pooling gains nothing here (256 maps of 35 x 35 x 192: tiles 49.2, rings 49.4 to 55 us).
 constexpr int kRingStages = 2;
 struct WinRing {
     int col_tiles, strips, in_cols, slabs;
